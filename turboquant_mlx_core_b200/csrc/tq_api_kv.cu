@@ -25,7 +25,7 @@ void launch_kv_encode(const void* x, bool x_is_f16, long n_vec, int head_dim, ui
 void launch_kv_decode_f16(const uint32_t* words, const float* norms, long n_vec, int head_dim, uint32_t wht_seed,
                           __half* out, cudaStream_t stream);
 size_t attn_scratch_bytes(int n_seqs, int q_heads, int head_dim, int n_splits);
-void launch_kv_attention(const void* d_seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads,
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads,
                          int head_dim, AttnPlan plan, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl,
                          void* scratch, __half* out, float* lse, unsigned int* status, cudaStream_t stream);
 AttnPlan attn_make_plan(int n_seqs, int q_heads, int kv_heads, int head_dim, int max_tok, int sm_count, int kernel);
@@ -36,19 +36,10 @@ namespace turboquant {
 using tq::DeviceBuffer;
 using tq::Error;
 
-// Device image of the kernel-side per-sequence descriptor (tq_kv_kernels.cu: AttnSeq).
-struct SeqDesc {
-    const uint32_t* k_words;
-    const uint32_t* v_words;
-    const float* k_norms;
-    const float* v_norms;
-    const uint32_t* qjl_words;
-    const float* qjl_norms;
-    int start, end;
-};
-
 struct LayerKVStorage {
-    DeviceBuffer k_words, v_words, k_norms, v_norms, qjl_words, qjl_norms;
+    DeviceBuffer slab;   // the six arrays, see tq::KvSlab
+    uint32_t *k_words = nullptr, *v_words = nullptr, *qjl_words = nullptr;
+    float *k_norms = nullptr, *v_norms = nullptr, *qjl_norms = nullptr;
     int num_tokens = 0;
     int capacity = 0;
 };
@@ -63,6 +54,7 @@ public:
                    "TQKVCache: head_dim must be a power of two in [32, 512]");
         device_ = tq::current_device();
         layers_.resize(static_cast<size_t>(num_layers));
+        for (DeviceBuffer* b : {&stage_k_, &stage_v_, &attn_scratch_, &attn_q_, &attn_out_, &attn_lse_}) b->owned_by(&use_);
     }
 
     int num_layers() const { return layers_n_; }
@@ -81,6 +73,7 @@ public:
         TQ_REQUIRE(tokens >= 0, "append: negative token count");
         if (tokens == 0) return;
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         reserve(L, L.num_tokens + tokens, st);
         const size_t es = dtype == TQ_F32 ? 4 : 2;
@@ -89,12 +82,12 @@ public:
         const void* d_k = keys;
         const void* d_v = values;
         if (!tq::is_device_pointer(keys)) {
-            stage_k_.reserve(bytes);
+            stage_k_.reserve(bytes, st);
             TQ_CUDA(cudaMemcpyAsync(stage_k_.as<void>(), keys, bytes, cudaMemcpyHostToDevice, st));
             d_k = stage_k_.as<void>();
         }
         if (!tq::is_device_pointer(values)) {
-            stage_v_.reserve(bytes);
+            stage_v_.reserve(bytes, st);
             TQ_CUDA(cudaMemcpyAsync(stage_v_.as<void>(), values, bytes, cudaMemcpyHostToDevice, st));
             d_v = stage_v_.as<void>();
         }
@@ -103,9 +96,9 @@ public:
         const uint32_t ks = tq::kv_layer_seed(static_cast<uint32_t>(layer), 1);  // src/kv_cache.cpp:40-42
         const uint32_t vs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 2);
         const uint32_t qs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 3);
-        const tq::KvEncodeSegment kseg{L.k_words.as<uint32_t>() + off * wph, L.k_norms.as<float>() + off,
-                                       L.qjl_words.as<uint32_t>() + off * qph, L.qjl_norms.as<float>() + off};
-        const tq::KvEncodeSegment vseg{L.v_words.as<uint32_t>() + off * wph, L.v_norms.as<float>() + off, nullptr, nullptr};
+        const tq::KvEncodeSegment kseg{L.k_words + off * wph, L.k_norms + off,
+                                       L.qjl_words + off * qph, L.qjl_norms + off};
+        const tq::KvEncodeSegment vseg{L.v_words + off * wph, L.v_norms + off, nullptr, nullptr};
         tq::launch_kv_encode_pair_segments(d_k, d_v, dtype == TQ_F16, static_cast<long>(n_vec), static_cast<long>(n_vec), dim_, ks, vs, qs,
                                            &kseg, &vseg, 1, st);
         L.num_tokens += tokens;
@@ -118,7 +111,11 @@ public:
         TQ_REQUIRE(tokens >= 0, "reserve: negative token count");
         TQ_CUDA(cudaSetDevice(device_));
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
-        if (tokens > L.capacity) reserve_exact(L, tokens, st);
+        if (tokens > L.capacity) {
+            use_.note(st);
+            reserve_exact(L, tokens, st, false);
+            TQ_CUDA(cudaStreamSynchronize(st));
+        }
     }
 
     // One decode step of a batch: token i of keys / values ([n, heads, dim], device memory) is
@@ -148,11 +145,12 @@ public:
                                c->layers_n_ == c0->layers_n_,
                            "append_batch: caches of one call must share shape and device");
                 LayerKVStorage& L = c->layers_[static_cast<size_t>(layer)];
+                c->use_.note(st);
                 c->reserve(L, L.num_tokens + 1, st);
                 const size_t off = static_cast<size_t>(L.num_tokens) * c->heads_;
-                kseg[i] = {L.k_words.as<uint32_t>() + off * wph, L.k_norms.as<float>() + off,
-                           L.qjl_words.as<uint32_t>() + off * qph, L.qjl_norms.as<float>() + off};
-                vseg[i] = {L.v_words.as<uint32_t>() + off * wph, L.v_norms.as<float>() + off, nullptr, nullptr};
+                kseg[i] = {L.k_words + off * wph, L.k_norms + off,
+                           L.qjl_words + off * qph, L.qjl_norms + off};
+                vseg[i] = {L.v_words + off * wph, L.v_norms + off, nullptr, nullptr};
             }
             const long n_vec = static_cast<long>(nb) * c0->heads_;
             const char* kp = static_cast<const char*>(keys) + static_cast<size_t>(b0) * vec_bytes;
@@ -174,23 +172,25 @@ public:
         TQ_REQUIRE(start >= 0 && end <= L.num_tokens && start < end, "Invalid token range for dequantization");
         TQ_REQUIRE(out, "get_fp16: NULL output");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         const size_t n_vec = static_cast<size_t>(end - start) * heads_;
         const size_t off = static_cast<size_t>(start) * heads_;
         const bool dev = tq::is_device_pointer(out);
         DeviceBuffer stage;
         __half* d_out = static_cast<__half*>(out);
         if (!dev) {
-            stage.reserve(n_vec * dim_ * sizeof(__half));
+            stage.reserve(n_vec * dim_ * sizeof(__half), st);
             d_out = stage.as<__half>();
         }
         const uint32_t seed = tq::kv_layer_seed(static_cast<uint32_t>(layer), values ? 2 : 1);
-        const DeviceBuffer& W = values ? L.v_words : L.k_words;
-        const DeviceBuffer& N = values ? L.v_norms : L.k_norms;
-        tq::launch_kv_decode_f16(W.as<uint32_t>() + off * words_per_head(), N.as<float>() + off,
+        const uint32_t* const words = values ? L.v_words : L.k_words;
+        const float* const norms = values ? L.v_norms : L.k_norms;
+        tq::launch_kv_decode_f16(words + off * words_per_head(), norms + off,
                                  static_cast<long>(n_vec), dim_, seed, d_out, st);
         if (!dev) {
             TQ_CUDA(cudaMemcpyAsync(out, d_out, n_vec * dim_ * sizeof(__half), cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));
+            stage.set_idle();
         }
     }
 
@@ -203,8 +203,8 @@ public:
         TQ_CUDA(cudaSetDevice(device_));
         TQ_CUDA(cudaDeviceSynchronize());
         const size_t n = static_cast<size_t>(L.num_tokens) * heads_;
-        auto copy = [&](void* dst, const DeviceBuffer& src, size_t bytes) {
-            if (dst && bytes) TQ_CUDA(cudaMemcpy(dst, src.as<void>(), bytes, cudaMemcpyDefault));
+        auto copy = [&](void* dst, const void* src, size_t bytes) {
+            if (dst && bytes) TQ_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDefault));
         };
         copy(k_words, L.k_words, n * words_per_head() * 4);
         copy(v_words, L.v_words, n * words_per_head() * 4);
@@ -246,9 +246,9 @@ public:
             put(static_cast<uint32_t>(layer_blob_bytes(L)));
             put(static_cast<uint32_t>(L.num_tokens));
             const size_t n = static_cast<size_t>(L.num_tokens) * heads_;
-            auto span = [&](const DeviceBuffer& src, size_t bytes) {
+            auto span = [&](const void* src, size_t bytes) {
                 put(static_cast<uint32_t>(bytes));
-                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, src.as<void>(), bytes, cudaMemcpyDeviceToHost));
+                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, src, bytes, cudaMemcpyDeviceToHost));
                 pos += bytes;
             };
             span(L.k_words, n * words_per_head() * 4);
@@ -302,10 +302,10 @@ public:
             LayerKVStorage& L = layers_[l];
             L.num_tokens = 0;
             reserve(L, static_cast<int>(tokens[l]), nullptr);
-            DeviceBuffer* dst[6] = {&L.k_words, &L.v_words, &L.k_norms, &L.v_norms, &L.qjl_words, &L.qjl_norms};
+            void* dst[6] = {L.k_words, L.v_words, L.k_norms, L.v_norms, L.qjl_words, L.qjl_norms};
             for (int i = 0; i < 6; ++i)
                 if (spans[l][i].bytes)
-                    TQ_CUDA(cudaMemcpy(dst[i]->as<void>(), data + spans[l][i].off, spans[l][i].bytes, cudaMemcpyHostToDevice));
+                    TQ_CUDA(cudaMemcpy(dst[i], data + spans[l][i].off, spans[l][i].bytes, cudaMemcpyHostToDevice));
             L.num_tokens = static_cast<int>(tokens[l]);
             seq_length_ = std::max(seq_length_, L.num_tokens);
         }
@@ -351,10 +351,10 @@ public:
             put(static_cast<uint32_t>(range_blob_bytes(b - a)));
             put(static_cast<uint32_t>(b - a));
             const size_t n = static_cast<size_t>(b - a) * heads_, first = static_cast<size_t>(a) * heads_;
-            auto span = [&](const DeviceBuffer& src, size_t elem_bytes) {
+            auto span = [&](const void* src, size_t elem_bytes) {
                 const size_t bytes = n * elem_bytes;
                 put(static_cast<uint32_t>(bytes));
-                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, src.as<uint8_t>() + first * elem_bytes, bytes, cudaMemcpyDeviceToHost));
+                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, static_cast<const uint8_t*>(src) + first * elem_bytes, bytes, cudaMemcpyDeviceToHost));
                 pos += bytes;
             };
             span(L.k_words, static_cast<size_t>(words_per_head()) * 4);
@@ -406,29 +406,27 @@ public:
             LayerKVStorage& L = layers_[l];
             reserve(L, L.num_tokens + static_cast<int>(tokens[l]), nullptr);
             const size_t first = static_cast<size_t>(L.num_tokens) * heads_;
-            DeviceBuffer* dst[6] = {&L.k_words, &L.v_words, &L.k_norms, &L.v_norms, &L.qjl_words, &L.qjl_norms};
+            void* dst[6] = {L.k_words, L.v_words, L.k_norms, L.v_norms, L.qjl_words, L.qjl_norms};
             const size_t elem[6] = {static_cast<size_t>(words_per_head()) * 4, static_cast<size_t>(words_per_head()) * 4, 4, 4,
                                     static_cast<size_t>(qjl_words_per_head()) * 4, 4};
             for (int i = 0; i < 6; ++i)
                 if (spans[l][i].bytes)
-                    TQ_CUDA(cudaMemcpy(dst[i]->as<uint8_t>() + first * elem[i], data + spans[l][i].off, spans[l][i].bytes,
+                    TQ_CUDA(cudaMemcpy(static_cast<uint8_t*>(dst[i]) + first * elem[i], data + spans[l][i].off, spans[l][i].bytes,
                                        cudaMemcpyHostToDevice));
             L.num_tokens += static_cast<int>(tokens[l]);
             seq_length_ = std::max(seq_length_, L.num_tokens);
         }
     }
 
-    SeqDesc describe(int layer, int start, int end) const {
+    tq::AttnSeq describe(int layer, int start, int end) const {
         TQ_REQUIRE(layer >= 0 && layer < layers_n_, "Layer index out of range");
         const LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         TQ_REQUIRE(start >= 0 && end <= L.num_tokens && start < end, "Invalid token range for attention");
-        return SeqDesc{L.k_words.as<uint32_t>(), L.v_words.as<uint32_t>(), L.k_norms.as<float>(), L.v_norms.as<float>(),
-                       L.qjl_words.as<uint32_t>(), L.qjl_norms.as<float>(), start, end};
+        return tq::AttnSeq{L.slab.as<unsigned char>(), start, end, L.capacity, 0};
     }
 
     int device() const { return device_; }
     DeviceBuffer& attn_scratch() { return attn_scratch_; }
-    DeviceBuffer& attn_desc() { return attn_desc_; }
     DeviceBuffer& attn_q() { return attn_q_; }
     DeviceBuffer& attn_out() { return attn_out_; }
     DeviceBuffer& attn_lse() { return attn_lse_; }
@@ -441,12 +439,11 @@ public:
     // directly (only when a bounded wait ran out), so reading it costs the host nothing.
     unsigned int* attn_status_device() {
         if (!h_attn_status_) {
-            TQ_CUDA(cudaMallocHost(&h_attn_status_, sizeof(unsigned int)));
-            *h_attn_status_ = 0u;
+            h_attn_status_ = tq::status_word_take(device_);
+            d_attn_status_ = static_cast<unsigned int*>(tq::pinned_host_device_alias(h_attn_status_));
+            TQ_REQUIRE(d_attn_status_ != nullptr, "attention: the status word is not mapped for the device");
         }
-        void* alias = tq::pinned_host_device_alias(h_attn_status_);
-        TQ_REQUIRE(alias != nullptr, "attention: the status word is not mapped for the device");
-        return static_cast<unsigned int*>(alias);
+        return d_attn_status_;
     }
     // Device copy of the descriptor table of `layer`; uploaded only when it differs from what is there.
     const void* upload_descriptors(int layer, const void* table, size_t bytes, cudaStream_t st) {
@@ -462,7 +459,8 @@ public:
         TQ_REQUIRE(cap == cudaStreamCaptureStatusNone,
                    "attention: the sequences or ranges of this call differ from the previous call for this layer; run it once "
                    "outside the stream capture first (the descriptor upload cannot be captured)");
-        dev.reserve(bytes);
+        dev.owned_by(&use_);
+        dev.reserve(bytes, st);
         // from pageable memory: staged by the driver before the call returns, so `table` may die
         TQ_CUDA(cudaMemcpyAsync(dev.as<void>(), table, bytes, cudaMemcpyHostToDevice, st));
         host.assign(static_cast<const uint8_t*>(table), static_cast<const uint8_t*>(table) + bytes);
@@ -470,8 +468,16 @@ public:
     }
     // Throws when an attention launch that has finished reported a failure (and clears the report).
     ~TQKVCache() {
-        if (h_attn_status_) cudaFreeHost(h_attn_status_);
+        if (!use_.only_legacy()) {   // the buffers below then find nothing pending
+            int cur = -1;
+            if (cudaGetDevice(&cur) == cudaSuccess && cur != device_) cudaSetDevice(device_);
+            cudaDeviceSynchronize();
+            if (cur >= 0 && cur != device_) cudaSetDevice(cur);
+        }
+        tq::status_word_return(h_attn_status_, device_);
     }
+    // Every stream that work on this cache's memory is put on (its release has to wait for that work).
+    void note_stream(cudaStream_t st) { use_.note(st); }
     TQKVCache(const TQKVCache&) = delete;
     TQKVCache& operator=(const TQKVCache&) = delete;
     void check_attention_status() {
@@ -487,35 +493,48 @@ private:
     // Grow a layer's buffers to hold `tokens` tokens (capacity doubles; old contents kept).
     void reserve(LayerKVStorage& L, int tokens, cudaStream_t st) {
         if (tokens <= L.capacity) return;
-        reserve_exact(L, std::max(L.capacity * 2, std::max(tokens, 256)), st);
+        reserve_exact(L, std::max(L.capacity * 2, std::max(tokens, 256)), st, true);
     }
-    void reserve_exact(LayerKVStorage& L, int cap, cudaStream_t st) {
+    // on_stream: the storage's first use is work on `st` (an append); otherwise it may be any stream's.
+    void reserve_exact(LayerKVStorage& L, int cap, cudaStream_t st, bool on_stream) {
         // whole 16-token tiles: the attention kernel fetches the cache a tile at a time
         cap = (cap + 15) / 16 * 16;
-        const size_t per = static_cast<size_t>(heads_);
-        const size_t old_n = static_cast<size_t>(L.num_tokens) * per;
-        auto grow = [&](DeviceBuffer& b, size_t elem_bytes_per_vec) {
-            DeviceBuffer nb(static_cast<size_t>(cap) * per * elem_bytes_per_vec);
-            if (old_n) TQ_CUDA(cudaMemcpyAsync(nb.as<void>(), b.as<void>(), old_n * elem_bytes_per_vec, cudaMemcpyDeviceToDevice, st));
-            TQ_CUDA(cudaStreamSynchronize(st));  // the old buffer is freed on return
-            b = std::move(nb);
+        const int wph = words_per_head(), qph = qjl_words_per_head();
+        DeviceBuffer slab;
+        slab.owned_by(&use_);
+        const size_t bytes = tq::KvSlab::bytes(cap, heads_, wph, qph);
+        if (on_stream) slab.reserve(bytes, st);
+        else slab.reserve(bytes);
+        const tq::AttnView v = tq::attn_view(tq::AttnSeq{slab.as<unsigned char>(), 0, 0, cap, 0}, heads_, wph, qph);
+        const size_t old_n = static_cast<size_t>(L.num_tokens) * heads_;
+        auto move = [&](const void* to, const void* from, size_t words_per_vec) {
+            if (old_n) TQ_CUDA(cudaMemcpyAsync(const_cast<void*>(to), from, old_n * words_per_vec * 4, cudaMemcpyDeviceToDevice, st));
         };
-        grow(L.k_words, static_cast<size_t>(words_per_head()) * 4);
-        grow(L.v_words, static_cast<size_t>(words_per_head()) * 4);
-        grow(L.k_norms, 4);
-        grow(L.v_norms, 4);
-        grow(L.qjl_words, static_cast<size_t>(qjl_words_per_head()) * 4);
-        grow(L.qjl_norms, 4);
+        move(v.k_words, L.k_words, wph);
+        move(v.v_words, L.v_words, wph);
+        move(v.k_norms, L.k_norms, 1);
+        move(v.v_norms, L.v_norms, 1);
+        move(v.qjl_words, L.qjl_words, qph);
+        move(v.qjl_norms, L.qjl_norms, 1);
+        L.k_words = const_cast<uint32_t*>(v.k_words);
+        L.v_words = const_cast<uint32_t*>(v.v_words);
+        L.k_norms = const_cast<float*>(v.k_norms);
+        L.v_norms = const_cast<float*>(v.v_norms);
+        L.qjl_words = const_cast<uint32_t*>(v.qjl_words);
+        L.qjl_norms = const_cast<float*>(v.qjl_norms);
+        L.slab = std::move(slab);   // the old storage goes back once the copies out of it have ended
         L.capacity = cap;
     }
 
     int layers_n_, heads_, dim_, kv_bits_, max_context_, decode_window_;
     int device_ = 0;
     int seq_length_ = 0;
+    tq::StreamUse use_;
     std::vector<LayerKVStorage> layers_;
     DeviceBuffer stage_k_, stage_v_;
-    DeviceBuffer attn_scratch_, attn_desc_, attn_q_, attn_out_, attn_lse_;
+    DeviceBuffer attn_scratch_, attn_q_, attn_out_, attn_lse_;
     unsigned int* h_attn_status_ = nullptr;
+    unsigned int* d_attn_status_ = nullptr;         // its address for kernels
     std::vector<DeviceBuffer> desc_dev_;            // per layer: the descriptor table of the last attention call
     std::vector<std::vector<uint8_t>> desc_host_;   // ... and its host copy, to tell whether an upload is needed
     int attention_kernel_ = 0;
@@ -534,49 +553,53 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
     TQ_REQUIRE(dim <= 256, "attention: head_dim above 256 is not supported");
     TQ_CUDA(cudaSetDevice(c0->device()));
     c0->check_attention_status();   // a failure of an earlier asynchronous call
-    std::vector<SeqDesc> desc(static_cast<size_t>(n_seqs));
+    tq::AttnSeqs seqs;
+    seqs.table = nullptr;
+    std::vector<tq::AttnSeq> many;   // more sequences than travel as parameters
+    if (n_seqs > tq::kAttnInlineSeqs) many.resize(static_cast<size_t>(n_seqs));
+    tq::AttnSeq* const desc = many.empty() ? seqs.inl : many.data();
     int max_tok = 0;
     for (int i = 0; i < n_seqs; ++i) {
         TQ_REQUIRE(caches[i] && caches[i]->num_heads() == heads && caches[i]->head_dim() == dim &&
                        caches[i]->device() == c0->device(),
                    "attention: caches of one call must share shape and device");
         desc[i] = caches[i]->describe(layer, starts[i], ends[i]);
+        caches[i]->note_stream(st);
         max_tok = std::max(max_tok, ends[i] - starts[i]);
     }
     const tq::AttnPlan plan = tq::attn_make_plan(n_seqs, q_heads, heads, dim, max_tok, tq::sm_count(c0->device()), c0->attention_kernel());
     const int n_splits = plan.n_splits;
 
-    // The descriptor table goes up only when it differs from the one already on the device: a call
-    // that repeats the previous ranges enqueues kernels only (and can then be captured in a graph).
-    const void* d_desc = c0->upload_descriptors(layer, desc.data(), desc.size() * sizeof(SeqDesc), st);
+    // A table goes up only when it differs from the one already on the device: a call that repeats the
+    // previous ranges enqueues kernels only (and can then be captured in a graph).
+    if (!many.empty())
+        seqs.table = static_cast<const tq::AttnSeq*>(c0->upload_descriptors(layer, many.data(), many.size() * sizeof(tq::AttnSeq), st));
     const size_t n_q = static_cast<size_t>(n_seqs) * q_heads * dim;
     const size_t q_es = q_dtype == TQ_F32 ? 4 : 2;
     const void* d_q = q;
     if (!tq::is_device_pointer(q)) {
-        c0->attn_q().reserve(n_q * q_es);
+        c0->attn_q().reserve(n_q * q_es, st);
         TQ_CUDA(cudaMemcpyAsync(c0->attn_q().as<void>(), q, n_q * q_es, cudaMemcpyHostToDevice, st));
         d_q = c0->attn_q().as<void>();
     }
     const bool out_dev = tq::is_device_pointer(out);
     __half* d_out = static_cast<__half*>(out);
     if (!out_dev) {
-        c0->attn_out().reserve(n_q * sizeof(__half));
+        c0->attn_out().reserve(n_q * sizeof(__half), st);
         d_out = c0->attn_out().as<__half>();
     }
     // optional log-sum-exp per (sequence, query head), fp32, host or device
     const size_t n_lse = static_cast<size_t>(n_seqs) * q_heads;
     float* d_lse = lse_out;
     if (lse_out != nullptr && !tq::is_device_pointer(lse_out)) {
-        c0->attn_lse().reserve(n_lse * sizeof(float));
+        c0->attn_lse().reserve(n_lse * sizeof(float), st);
         d_lse = c0->attn_lse().as<float>();
     }
-    c0->attn_scratch().reserve(tq::attn_scratch_bytes(n_seqs, q_heads, dim, n_splits));
-    tq::launch_kv_attention(d_desc, n_seqs, d_q, q_dtype == TQ_F16, q_heads, heads, dim, plan,
+    c0->attn_scratch().reserve(tq::attn_scratch_bytes(n_seqs, q_heads, dim, n_splits), st);
+    tq::launch_kv_attention(seqs, n_seqs, d_q, q_dtype == TQ_F16, q_heads, heads, dim, plan,
                             tq::kv_layer_seed(static_cast<uint32_t>(layer), 1), tq::kv_layer_seed(static_cast<uint32_t>(layer), 2),
                             tq::kv_layer_seed(static_cast<uint32_t>(layer), 3), use_qjl, c0->attn_scratch().as<void>(), d_out, d_lse,
                             c0->attn_status_device(), st);
-    // desc was copied from pageable host memory: the copy has been staged by the time
-    // cudaMemcpyAsync returned, so `desc` may die here.
     const bool lse_host = lse_out != nullptr && d_lse != lse_out;
     if (lse_host) TQ_CUDA(cudaMemcpyAsync(lse_out, d_lse, n_lse * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (!out_dev) TQ_CUDA(cudaMemcpyAsync(out, d_out, n_q * sizeof(__half), cudaMemcpyDeviceToHost, st));

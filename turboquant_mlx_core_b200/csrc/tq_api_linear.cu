@@ -37,6 +37,8 @@ public:
         else throw Error("TurboQuantLinear: packed_primary must have in/2 or in columns");
         device_ = tq::current_device();
         sm_count_ = tq::sm_count(device_);
+        for (DeviceBuffer* b : {&codes_, &norms_, &tables_, &scratch_, &staged_scratch_, &gemm_scratch_, &counter_, &x_f16_, &x_f32_, &y_f16_})
+            b->owned_by(&use_);
 
         cudaStream_t st = nullptr;
         uint32_t h_seeds[3];
@@ -105,8 +107,7 @@ public:
         TQ_CUDA(cudaMemset(counter_.as<void>(), 0, sizeof(unsigned int)));
         // The kernels' error word is page-locked host memory that they store to directly (only on
         // a failure), so the host checks it after a synchronisation without a copy.
-        TQ_CUDA(cudaMallocHost(&h_status_, sizeof(unsigned int)));
-        *h_status_ = 0;
+        h_status_ = tq::status_word_take(device_);
         d_status_ = static_cast<unsigned int*>(tq::pinned_host_device_alias(h_status_));
         TQ_REQUIRE(d_status_ != nullptr, "TurboQuantLinear: the status word is not mapped for the device");
 
@@ -115,8 +116,8 @@ public:
         DeviceBuffer x0(static_cast<size_t>(in_) * sizeof(__half)), y0(static_cast<size_t>(out_) * sizeof(__half));
         TQ_CUDA(cudaMemset(x0.as<void>(), 0, x0.bytes()));
         launch_forward(x0.as<__half>(), 1, y0.as<__half>(), nullptr);
-        TQ_CUDA(cudaDeviceSynchronize());
-        check_status();
+        check_status();   // waits for the device
+        for (DeviceBuffer* b : {&x0, &y0, &stage_p, &stage_r, &flags}) b->set_idle();
     }
 
     int in_features() const { return in_; }
@@ -131,6 +132,7 @@ public:
         TQ_REQUIRE(x_dtype == TQ_F32 || x_dtype == TQ_F16, "TurboQuantLinear::forward: x must be fp32 or fp16");
         if (batch == 0) return;
         make_current();
+        use_.note(st);
         const size_t nx = static_cast<size_t>(batch) * in_, ny = static_cast<size_t>(batch) * out_;
         const PointerKind kx = classify(x), ky = classify(y);
         const bool x_dev = kx.device, y_dev = ky.device;
@@ -139,7 +141,7 @@ public:
         if (x_dtype == TQ_F16) {
             if (x_dev) d_x = static_cast<const __half*>(x);
             else {
-                x_f16_.reserve(nx * sizeof(__half));
+                x_f16_.reserve(nx * sizeof(__half), st);
                 TQ_CUDA(cudaMemcpyAsync(x_f16_.as<void>(), x, nx * sizeof(__half), cudaMemcpyHostToDevice, st));
                 d_x = x_f16_.as<__half>();
             }
@@ -147,11 +149,11 @@ public:
             const float* d_xf;
             if (x_dev) d_xf = static_cast<const float*>(x);
             else {
-                x_f32_.reserve(nx * sizeof(float));
+                x_f32_.reserve(nx * sizeof(float), st);
                 TQ_CUDA(cudaMemcpyAsync(x_f32_.as<void>(), x, nx * sizeof(float), cudaMemcpyHostToDevice, st));
                 d_xf = x_f32_.as<float>();
             }
-            x_f16_.reserve(nx * sizeof(__half));
+            x_f16_.reserve(nx * sizeof(__half), st);
             tq::launch_f32_to_f16(d_xf, x_f16_.as<__half>(), static_cast<long>(nx), st);  // src/dequantizer.cpp:691
             d_x = x_f16_.as<__half>();
         }
@@ -162,7 +164,7 @@ public:
         if (y_dev) d_y = static_cast<__half*>(y);
         else if (y_alias) d_y = static_cast<__half*>(y_alias);
         else {
-            y_f16_.reserve(ny * sizeof(__half));
+            y_f16_.reserve(ny * sizeof(__half), st);
             d_y = y_f16_.as<__half>();
         }
         launch_forward(d_x, batch, d_y, st);
@@ -186,6 +188,7 @@ public:
                    "forward_scatter: rows [row_offset, row_offset + out) must fit the destination row stride");
         TQ_REQUIRE(tq::is_device_pointer(x), "forward_scatter: x must be a device pointer");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         __half* d[8];
         for (int i = 0; i < n_dst; ++i) {
             TQ_REQUIRE(dst[i] != nullptr, "forward_scatter: NULL destination");
@@ -203,7 +206,8 @@ public:
     }
 
     // This layer as one matrix of a grouped decode launch (see tq_linear_forward_group).
-    tq::GemvGroupItem group_item(void* y) const {
+    tq::GemvGroupItem group_item(void* y, cudaStream_t st) {
+        use_.note(st);
         tq::GemvGroupItem it{};
         it.codes = codes_.as<uint8_t>(); it.norms = norms_.as<float>(); it.table = tables_.as<float>();
         it.y = static_cast<__half*>(y);
@@ -213,9 +217,10 @@ public:
         return it;
     }
     // The same for batches that go to the tensor-memory GEMM (scratch for `batch` rows is reserved here).
-    tq::GemmGroupItem gemm_group_item(void* y, int batch) {
+    tq::GemmGroupItem gemm_group_item(void* y, int batch, cudaStream_t st) {
         const int planes = dual_ ? 2 : 1;
-        gemm_scratch_.reserve(tq::gemm_scratch_bytes(out_, in_, batch, planes, sm_count_));
+        use_.note(st);
+        gemm_scratch_.reserve(tq::gemm_scratch_bytes(out_, in_, batch, planes, sm_count_), st);
         tq::GemmGroupItem it{};
         it.codes = codes_.as<uint8_t>(); it.norms = norms_.as<float>(); it.table = tables_.as<float>();
         it.y = static_cast<__half*>(y);
@@ -237,6 +242,7 @@ public:
         TQ_REQUIRE(y_stride >= out_, "forward_strided: row stride smaller than out_features");
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y), "forward_strided: x and y must be device pointers");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         launch_forward(static_cast<const __half*>(x), batch, static_cast<__half*>(y), st, y_stride);
     }
 
@@ -252,6 +258,7 @@ public:
         TQ_REQUIRE(slot >= 0 && slot < 32, "forward_allgather: flag slot must be 0..31");
         TQ_REQUIRE(tq::is_device_pointer(x), "forward_allgather: x must be a device pointer");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         __half* d[8];
         for (int i = 0; i < n_dst; ++i) {
             TQ_REQUIRE(dst[i] != nullptr, "forward_allgather: NULL destination");
@@ -274,6 +281,7 @@ public:
         TQ_REQUIRE(y_stride >= out_, "forward_allgather_packets: row stride smaller than the layer's rows");
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y), "forward_allgather_packets: x and y must be device pointers");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         __half* d[1] = {static_cast<__half*>(y)};
         tq::GemvGather g{epoch, nullptr, wait ? 1 : 0, wait_epoch};
         g.ll_rank = rank;
@@ -286,6 +294,7 @@ public:
 
     void wait_peers(const void* flags, int n, unsigned int value, cudaStream_t st) {
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         tq::launch_peer_wait(static_cast<const unsigned int*>(flags), n, value, d_status_, st);
     }
 
@@ -300,13 +309,14 @@ public:
         TQ_REQUIRE(result, "dequantize: NULL result");
         TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16, "dequantize: result must be fp32 or fp16");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         const size_t n = static_cast<size_t>(out_) * in_;
         const size_t es = dtype == TQ_F32 ? 4 : 2;
         const bool dev = tq::is_device_pointer(result);
         DeviceBuffer stage;
         void* d_out = result;
         if (!dev) {
-            stage.reserve(n * es);
+            stage.reserve(n * es, st);
             d_out = stage.as<void>();
         }
         if (dtype == TQ_F32)
@@ -318,6 +328,7 @@ public:
         if (!dev) {
             TQ_CUDA(cudaMemcpyAsync(result, d_out, n * es, cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));
+            stage.set_idle();
         }
     }
 
@@ -329,6 +340,7 @@ public:
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y),
                    "allocation-free forward: x and y must be device pointers (copying host memory would need a staging allocation)");
         TQ_CUDA(cudaSetDevice(device_));
+        use_.note(st);
         // the kernel forward() would run, when its working set fits the array; else the other one
         if (decode_kernel_ == 2 && tq::gemv_staged_fits_static(out_, in_, batch, dual_ ? 2 : 1, sm_count_))
             tq::launch_tq8_gemv_staged_static(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(),
@@ -341,7 +353,13 @@ public:
     }
 
     ~TurboQuantLinear() {
-        if (h_status_) cudaFreeHost(h_status_);
+        if (!use_.only_legacy()) {   // the buffers then find nothing pending
+            int cur = -1;
+            if (cudaGetDevice(&cur) == cudaSuccess && cur != device_) cudaSetDevice(device_);
+            cudaDeviceSynchronize();
+            if (cur >= 0 && cur != device_) cudaSetDevice(cur);
+        }
+        tq::status_word_return(h_status_, device_);
     }
 
 private:
@@ -400,7 +418,7 @@ private:
         // activation tile is as narrow as the batch, in steps of 16 rows).
         if (batch > kGemmMinBatch && tq::gemm_supported(in_)) {
             const int planes = dual_ ? 2 : 1;
-            gemm_scratch_.reserve(tq::gemm_scratch_bytes(out_, in_, batch, planes, sm_count_));
+            gemm_scratch_.reserve(tq::gemm_scratch_bytes(out_, in_, batch, planes, sm_count_), st);
             tq::launch_tq8_gemm(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), d_x, d_y, out_, in_, batch,
                                 block_, planes, seed_p_, seed_r_, gemm_scratch_.as<void>(), d_status_,
                                 sm_count_, st, y_stride);
@@ -434,6 +452,7 @@ private:
 
     int in_, out_;
     uint32_t block_;
+    tq::StreamUse use_;
     int device_ = 0, sm_count_ = 0;
     bool primary_5bit_ = false, has_residual_ = false, shared_ = false, dual_ = false;
     uint32_t seed_p_ = 0, seed_r_ = 0;
@@ -504,7 +523,7 @@ int tq_linear_forward_group(const tq_linear_t* lins, int n, const void* x_fp16_d
         if (lins[0]->impl->gemm_path(batch)) {
             // 9 rows and up: one rotation launch, one tensor-memory GEMM launch and one split-K finish for the group
             tq::GemmGroupItem items[4];
-            for (int i = 0; i < n; ++i) items[i] = lins[i]->impl->gemm_group_item(y_fp16_device[i], batch);
+            for (int i = 0; i < n; ++i) items[i] = lins[i]->impl->gemm_group_item(y_fp16_device[i], batch, st);
             tq::launch_tq8_gemm_group(items, n, static_cast<const __half*>(x_fp16_device), batch, lins[0]->impl->sm_count(), st);
             return 0;
         }
@@ -513,7 +532,7 @@ int tq_linear_forward_group(const tq_linear_t* lins, int n, const void* x_fp16_d
             const int nb = batch - b0 < 8 ? batch - b0 : 8;
             tq::GemvGroupItem items[4];
             for (int i = 0; i < n; ++i)
-                items[i] = lins[i]->impl->group_item(static_cast<__half*>(y_fp16_device[i]) + static_cast<size_t>(b0) * lins[i]->impl->out_features());
+                items[i] = lins[i]->impl->group_item(static_cast<__half*>(y_fp16_device[i]) + static_cast<size_t>(b0) * lins[i]->impl->out_features(), st);
             tq::launch_tq8_gemv_group(items, n, static_cast<const __half*>(x_fp16_device) + static_cast<size_t>(b0) * lins[0]->impl->in_features(),
                                       nb, lins[0]->impl->sm_count(), st);
         }
@@ -582,6 +601,7 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         const uint32_t h_seeds[3] = {seed_p, (shared_rotation && residual_bits > 0) ? 0u : seed_r, block};
         TQ_CUDA(cudaMemcpyAsync(seeds, h_seeds, sizeof h_seeds, cudaMemcpyDefault, st));
         TQ_CUDA(cudaStreamSynchronize(st));  // scratch and staging buffers die here
+        for (DeviceBuffer* b : {&w_stage, &recon, &orig, &pp_stage, &pr_stage, &nm_stage}) b->set_idle();
         return 0;
     });
 }

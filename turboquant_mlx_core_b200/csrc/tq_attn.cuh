@@ -8,17 +8,55 @@
 
 namespace tq {
 
-// One sequence of an attention call: the layer's storage (token-major records, see
-// tq_kv_kernels.cu) and the token range [start, end) the query attends to.
+// A layer's storage is ONE allocation that holds its six token-major arrays (see tq_kv_kernels.cu) one after the
+// other, each sized for `cap` tokens; cap is a multiple of 16, so every array starts on a 64-byte boundary.
+struct KvSlab {
+    const unsigned char* base;
+    int cap;
+    __host__ __device__ static size_t bytes(int cap, int heads, int wph, int qph) {
+        return static_cast<size_t>(cap) * heads * (2 * wph + qph + 3) * 4;
+    }
+};
+
+// One sequence of an attention call: the layer's storage and the token range [start, end) the query attends to.
 struct AttnSeq {
+    const unsigned char* base;
+    int start, end, cap, pad;
+};
+// ... with the arrays' addresses spelled out.
+struct AttnView {
     const uint32_t* k_words;
     const uint32_t* v_words;
+    const uint32_t* qjl_words;
     const float* k_norms;
     const float* v_norms;
-    const uint32_t* qjl_words;
     const float* qjl_norms;
     int start, end;
 };
+__host__ __device__ __forceinline__ AttnView attn_view(const AttnSeq& s, int heads, int wph, int qph) {
+    const size_t n = static_cast<size_t>(s.cap) * heads;
+    const uint32_t* const w = reinterpret_cast<const uint32_t*>(s.base);
+    AttnView v;
+    v.k_words = w;
+    v.v_words = w + n * wph;
+    v.qjl_words = w + n * 2 * wph;
+    v.k_norms = reinterpret_cast<const float*>(w + n * (2 * wph + qph));
+    v.v_norms = v.k_norms + n;
+    v.qjl_norms = v.k_norms + 2 * n;
+    v.start = s.start;
+    v.end = s.end;
+    return v;
+}
+
+// The sequences of one attention call.  A decode step moves every range by a token, so the descriptors of up to
+// kAttnInlineSeqs sequences travel as kernel parameters (24 bytes each): a table in device memory cost an upload per
+// call, and the copy between two kernels a gap in the stream.  Larger batches use the table.
+constexpr int kAttnInlineSeqs = 32;
+struct AttnSeqs {
+    const AttnSeq* table;              // nullptr: the descriptors are in `inl`
+    AttnSeq inl[kAttnInlineSeqs];
+};
+__device__ __forceinline__ AttnSeq attn_seq(const AttnSeqs& s, int i) { return s.table != nullptr ? s.table[i] : s.inl[i]; }
 
 // The pair tables hold kAttnCentroidScale * centroid: with this factor all four centroid
 // magnitudes round to fp16 with a relative error below 1.4e-5 (unscaled: up to 3e-4, which the
@@ -29,7 +67,7 @@ constexpr float kAttnSoftmaxSlack = 2.0f;
 
 // Tensor-memory kernel (tq_attn_tc.cu): head_dim 128, four KV heads, up to 8 query heads per KV head
 // and CTA.  Partials in the layout attn_combine_kernel reads.
-void launch_attn_tc(const AttnSeq* seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads, int n_splits,
+void launch_attn_tc(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads, int n_splits,
                     uint32_t k_seed, uint32_t qjl_seed, bool use_qjl, float inv_sqrt, float inv_scale_d, float attn_scale,
                     float gamma, float* part_acc, float* part_ml, unsigned int* status, cudaStream_t stream);
 constexpr int kAttnTcCtasPerSm = 2;

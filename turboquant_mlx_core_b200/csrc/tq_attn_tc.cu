@@ -175,7 +175,7 @@ __device__ __forceinline__ bool tc_value_group_or(bool pred) {
 }
 
 template <typename QT>
-__global__ void __launch_bounds__(kTcThreads, kAttnTcCtasPerSm) attn_tc_kernel(const AttnSeq* __restrict__ seqs, const QT* __restrict__ qv,
+__global__ void __launch_bounds__(kTcThreads, kAttnTcCtasPerSm) attn_tc_kernel(const __grid_constant__ AttnSeqs seqs, const QT* __restrict__ qv,
                                                                               int q_heads, int n_splits, uint32_t k_seed,
                                                                               uint32_t qjl_seed, int use_qjl, float inv_sqrt,
                                                                               float inv_scale_d, float attn_scale, float gamma,
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kTcThreads, kAttnTcCtasPerSm) attn_tc_kernel(c
     const int g0 = gchunk * 8;
     const int ng = min(8, G - g0);
 
-    const AttnSeq S = seqs[seq];
+    const AttnView S = attn_view(attn_seq(seqs, seq), 4, 13, 4);
     const int first_tile = S.start >> 5, end_tile = (S.end + kTcTile - 1) >> 5;
     const int all_tiles = S.end > S.start ? end_tile - first_tile : 0;
     const int tile0 = first_tile + static_cast<int>(static_cast<long>(all_tiles) * split / n_splits);
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(kTcThreads, kAttnTcCtasPerSm) attn_tc_kernel(c
 
 }  // namespace
 
-void launch_attn_tc(const AttnSeq* seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads, int n_splits,
+void launch_attn_tc(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads, int n_splits,
                     uint32_t k_seed, uint32_t qjl_seed, bool use_qjl, float inv_sqrt, float inv_scale_d, float attn_scale,
                     float gamma, float* part_acc, float* part_ml, unsigned int* status, cudaStream_t stream) {
     TQ_REQUIRE(kv_heads == 4 && q_heads % 4 == 0, "tensor-memory attention kernel: four KV heads");

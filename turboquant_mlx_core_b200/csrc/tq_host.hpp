@@ -62,39 +62,93 @@ inline void* pinned_host_device_alias(const void* p) {
     return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
 }
 
+// ---- device memory (tq_memory.cu: released blocks are kept for the next owner) -----------------
+inline bool is_legacy_stream(cudaStream_t st) { return st == nullptr || st == cudaStreamLegacy; }
+size_t pool_size_class(size_t bytes);
+// A block on `device`, which must be current.  on_stream: its first use is work put on `st`; otherwise the block is
+// idle when the call returns.
+void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream);
+// idle: nothing queued anywhere uses the block; otherwise everything that does was put on the legacy default stream.
+void pool_release(void* p, size_t bytes, int device, bool idle);
+void pool_trim();
+// A zeroed word of page-locked host memory that the device can write.
+unsigned int* status_word_take(int device);
+// All work that could write the word was put on the legacy default stream, or has ended.
+void status_word_return(unsigned int* w, int device);
+
+// Which streams an object's memory has been used on: what its release has to wait for.
+class StreamUse {
+public:
+    void note(cudaStream_t st) { other_ = other_ || !is_legacy_stream(st); }
+    // True when only work on the legacy default stream can be pending.
+    bool only_legacy() const { return !other_; }
+
+private:
+    bool other_ = false;
+};
+
 class DeviceBuffer {
 public:
     DeviceBuffer() = default;
     explicit DeviceBuffer(size_t bytes) { resize(bytes); }
     DeviceBuffer(const DeviceBuffer&) = delete;
     DeviceBuffer& operator=(const DeviceBuffer&) = delete;
-    DeviceBuffer(DeviceBuffer&& o) noexcept : p_(o.p_), n_(o.n_) { o.p_ = nullptr; o.n_ = 0; }
+    DeviceBuffer(DeviceBuffer&& o) noexcept { take(o); }
     DeviceBuffer& operator=(DeviceBuffer&& o) noexcept {
-        if (this != &o) { release(); p_ = o.p_; n_ = o.n_; o.p_ = nullptr; o.n_ = 0; }
+        if (this != &o) { release(); take(o); }
         return *this;
     }
     ~DeviceBuffer() { release(); }
 
+    // Without an owner a release waits for the device; with one it follows the owner's record of streams.
+    void owned_by(const StreamUse* use) { use_ = use; }
+    // Nothing queued uses the contents any more: the release need not wait.
+    void set_idle() { idle_ = true; }
+
     // Grow-only: keeps the allocation when it is already large enough (contents kept
     // only in that case).
-    void reserve(size_t bytes) {
-        if (bytes <= n_) return;
-        release();
-        if (bytes) TQ_CUDA(cudaMalloc(&p_, bytes));
-        n_ = bytes;
-    }
+    void reserve(size_t bytes) { grow(bytes, nullptr, false); }
+    // ... for contents whose first use is work on `st`.
+    void reserve(size_t bytes, cudaStream_t st) { grow(bytes, st, true); }
     void resize(size_t bytes) { reserve(bytes); }
     void release() {
-        if (p_) cudaFree(p_);
+        if (p_) {
+            const bool legacy = use_ != nullptr && use_->only_legacy();
+            if (!idle_ && !legacy) {
+                int cur = -1;
+                if (cudaGetDevice(&cur) == cudaSuccess && cur != device_) cudaSetDevice(device_);
+                cudaDeviceSynchronize();
+                if (cur >= 0 && cur != device_) cudaSetDevice(cur);
+            }
+            pool_release(p_, n_, device_, idle_ || !legacy);
+        }
         p_ = nullptr;
         n_ = 0;
+        idle_ = false;
     }
     template <typename T = void> T* as() const { return static_cast<T*>(p_); }
     size_t bytes() const { return n_; }
 
 private:
+    void grow(size_t bytes, cudaStream_t st, bool on_stream) {
+        if (bytes <= n_) return;
+        release();
+        const int device = current_device();
+        p_ = pool_alloc(bytes, device, st, on_stream);
+        device_ = device;
+        n_ = bytes;
+    }
+    void take(DeviceBuffer& o) {
+        p_ = o.p_; n_ = o.n_; device_ = o.device_; use_ = o.use_; idle_ = o.idle_;
+        o.p_ = nullptr;
+        o.n_ = 0;
+        o.idle_ = false;
+    }
     void* p_ = nullptr;
     size_t n_ = 0;
+    int device_ = 0;
+    const StreamUse* use_ = nullptr;
+    bool idle_ = false;
 };
 
 // A read-only view of caller data on the device: device pointers are used in place,
@@ -103,7 +157,7 @@ template <typename T>
 const T* device_view(const T* p, size_t count, DeviceBuffer& staging, cudaStream_t stream) {
     if (count == 0) return p;
     if (is_device_pointer(p)) return p;
-    staging.reserve(count * sizeof(T));
+    staging.reserve(count * sizeof(T), stream);
     TQ_CUDA(cudaMemcpyAsync(staging.as<void>(), p, count * sizeof(T), cudaMemcpyHostToDevice, stream));
     return staging.as<T>();
 }

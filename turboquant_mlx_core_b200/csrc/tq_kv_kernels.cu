@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const uint32_t* __restri
 constexpr int kAttnGMax = 8;
 
 template <int E, typename QT>
-__global__ void __launch_bounds__(128) attn_partial_kernel(const AttnSeq* __restrict__ seqs, const QT* __restrict__ q,
+__global__ void __launch_bounds__(128) attn_partial_kernel(const __grid_constant__ AttnSeqs seqs, const QT* __restrict__ q,
                                                            int q_heads, int kv_heads, int n_splits, uint32_t k_seed,
                                                            uint32_t qjl_seed, int use_qjl, float inv_sqrt,
                                                            float inv_scale_d, float attn_scale, float gamma,
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(128) attn_partial_kernel(const AttnSeq* __rest
     const int G = q_heads / kv_heads;
     const int g0 = gchunk * kAttnGMax;
     const int ng = min(kAttnGMax, G - g0);
-    const AttnSeq S = seqs[seq];
+    const AttnView S = attn_view(attn_seq(seqs, seq), kv_heads, WPH, QPH);
     const int n_tok = S.end - S.start;
     const int t0 = S.start + static_cast<int>(static_cast<long>(n_tok) * split / n_splits);
     const int t1 = S.start + static_cast<int>(static_cast<long>(n_tok) * (split + 1) / n_splits);
@@ -537,7 +537,7 @@ __host__ __device__ __forceinline__ int attn_pair_dim(int q, int pidx) {
 }
 
 template <typename QT>
-__global__ void __launch_bounds__(kMmaThreads, 3) attn_mma_kernel(const AttnSeq* __restrict__ seqs, const QT* __restrict__ qv,
+__global__ void __launch_bounds__(kMmaThreads, 3) attn_mma_kernel(const __grid_constant__ AttnSeqs seqs, const QT* __restrict__ qv,
                                                                int q_heads, int kv_heads, int n_splits, uint32_t k_seed,
                                                                uint32_t qjl_seed, int use_qjl, float inv_sqrt,
                                                                float inv_scale_d, float attn_scale, float gamma,
@@ -555,6 +555,8 @@ __global__ void __launch_bounds__(kMmaThreads, 3) attn_mma_kernel(const AttnSeq*
     __shared__ float s_m[4][8], s_l[4][8];
     __shared__ float s_acc[4][8][D + 4];   // row stride 132: the publishing stores below hit 32 distinct banks
 
+    __shared__ AttnView s_view;   // in memory: recomputed from the parameters the addresses cost registers inside the tile loop
+
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, q = lane & 3;
     const int split = blockIdx.x, kvh = blockIdx.y % kv_heads, gchunk = blockIdx.y / kv_heads, seq = blockIdx.z;
@@ -562,6 +564,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3) attn_mma_kernel(const AttnSeq*
     const int g0 = gchunk * 8;
     const int ng = min(8, G - g0);
 
+    if (tid == 0) s_view = attn_view(attn_seq(seqs, seq), kv_heads, WPH, QPH);
     const uint32_t tab_addr = static_cast<uint32_t>(__cvta_generic_to_shared(s_tab));
     const uint32_t lut_addr = (tab_addr + 8191u) & ~8191u;           // pair table, [pair index][lane]
     uint32_t* const s_lut = s_tab + ((lut_addr - tab_addr) >> 2);
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3) attn_mma_kernel(const AttnSeq*
         bs[pidx] = pack_half2(s_q[g][q][pidx] * s0, s_q[g][q][pidx + 16] * s1);
     }
 
-    const AttnSeq S = seqs[seq];
+    const AttnView S = s_view;
     const int n_tok = S.end - S.start;
     const int t0 = S.start + static_cast<int>(static_cast<long>(n_tok) * split / n_splits);
     const int t1 = S.start + static_cast<int>(static_cast<long>(n_tok) * (split + 1) / n_splits);
@@ -880,7 +883,7 @@ struct PipeLayout {
 };
 
 template <int GH, typename QT>
-__global__ void __launch_bounds__(32 * GH, kPipeWarpsPerSm / GH) attn_pipe_kernel(const AttnSeq* __restrict__ seqs, const QT* __restrict__ qv,
+__global__ void __launch_bounds__(32 * GH, kPipeWarpsPerSm / GH) attn_pipe_kernel(const __grid_constant__ AttnSeqs seqs, const QT* __restrict__ qv,
                                                                     int q_heads, int kv_heads, int n_splits, uint32_t k_seed,
                                                                     uint32_t qjl_seed, int use_qjl, float inv_sqrt,
                                                                     float inv_scale_d, float attn_scale, float gamma,
@@ -910,7 +913,7 @@ __global__ void __launch_bounds__(32 * GH, kPipeWarpsPerSm / GH) attn_pipe_kerne
     const uint32_t stage_addr = raw_addr + LY::kOffStages;
     const uint32_t bar_full = raw_addr + LY::kOffBars, bar_empty = bar_full + 8u * kPipeStages;
 
-    const AttnSeq S = seqs[seq];
+    const AttnView S = attn_view(attn_seq(seqs, seq), kv_heads, 13, 4);
     const int first_tile = S.start >> 4, end_tile = (S.end + 15) >> 4;
     const int all_tiles = S.end > S.start ? end_tile - first_tile : 0;
     const int tile0 = first_tile + static_cast<int>(static_cast<long>(all_tiles) * split / n_splits);
@@ -1415,7 +1418,7 @@ AttnPlan attn_make_plan(int n_seqs, int q_heads, int kv_heads, int head_dim, int
 }
 
 template <int GH, typename QT>
-static void launch_attn_pipe(const AttnSeq* seqs, int n_seqs, const QT* q, int q_heads, int kv_heads, int n_splits, uint32_t k_seed,
+static void launch_attn_pipe(const AttnSeqs& seqs, int n_seqs, const QT* q, int q_heads, int kv_heads, int n_splits, uint32_t k_seed,
                              uint32_t qjl_seed, bool use_qjl, float inv_sqrt, float inv_scale_d, float attn_scale, float gamma,
                              float* part_acc, float* part_ml, unsigned int* status, cudaStream_t stream) {
     // the opt-in shared-memory size is a per-device attribute of each instantiation
@@ -1432,7 +1435,7 @@ static void launch_attn_pipe(const AttnSeq* seqs, int n_seqs, const QT* q, int q
                qjl_seed, use_qjl ? 1 : 0, inv_sqrt, inv_scale_d, attn_scale, gamma, part_acc, part_ml, status);
 }
 
-void launch_kv_attention(const void* d_seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads,
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads,
                          int head_dim, AttnPlan plan, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl,
                          void* scratch, __half* out, float* lse, unsigned int* status, cudaStream_t stream) {
     if (n_seqs == 0) return;
@@ -1450,19 +1453,19 @@ void launch_kv_attention(const void* d_seqs, int n_seqs, const void* q, bool q_i
     const long n_rows = static_cast<long>(n_seqs) * q_heads;
 #define TQ_ATT(EV)                                                                                                       \
     if (q_is_f16)                                                                                                        \
-        attn_partial_kernel<EV, __half><<<grid, 128, 0, stream>>>(static_cast<const AttnSeq*>(d_seqs),                    \
+        attn_partial_kernel<EV, __half><<<grid, 128, 0, stream>>>(seqs,                    \
                                                                   static_cast<const __half*>(q), q_heads, kv_heads,      \
                                                                   n_splits, k_seed, qjl_seed, use_qjl ? 1 : 0, inv_sqrt,  \
                                                                   inv_scale_d, attn_scale, gamma, part_acc, part_ml);    \
     else                                                                                                                 \
-        attn_partial_kernel<EV, float><<<grid, 128, 0, stream>>>(static_cast<const AttnSeq*>(d_seqs),                     \
+        attn_partial_kernel<EV, float><<<grid, 128, 0, stream>>>(seqs,                     \
                                                                  static_cast<const float*>(q), q_heads, kv_heads,        \
                                                                  n_splits, k_seed, qjl_seed, use_qjl ? 1 : 0, inv_sqrt,   \
                                                                  inv_scale_d, attn_scale, gamma, part_acc, part_ml);     \
     launch_pdl(attn_combine_kernel<EV>, dim3(static_cast<unsigned>((n_rows + 3) / 4)), dim3(128), 0, stream, part_acc, part_ml, n_rows, \
                n_splits, v_seed, inv_sqrt, inv_scale_d, out, lse);
     if (plan.tensor_memory) {
-        launch_attn_tc(static_cast<const AttnSeq*>(d_seqs), n_seqs, q, q_is_f16, q_heads, kv_heads, n_splits, k_seed, qjl_seed, use_qjl,
+        launch_attn_tc(seqs, n_seqs, q, q_is_f16, q_heads, kv_heads, n_splits, k_seed, qjl_seed, use_qjl,
                        inv_sqrt, inv_scale_d, attn_scale, gamma, part_acc, part_ml, status, stream);
         launch_pdl(attn_combine_kernel<4>, dim3(static_cast<unsigned>((n_rows + 3) / 4)), dim3(128), 0, stream, part_acc, part_ml, n_rows,
                    n_splits, v_seed, inv_sqrt, inv_scale_d, out, lse);
@@ -1471,7 +1474,6 @@ void launch_kv_attention(const void* d_seqs, int n_seqs, const void* q, bool q_i
     }
     if (const int gh = plan.pipe_heads) {
         TQ_REQUIRE(gh == attn_pipe_heads(head_dim, kv_heads), "attention: plan does not match the cache shape");
-        const AttnSeq* seqs = static_cast<const AttnSeq*>(d_seqs);
 #define TQ_PIPE(GHV)                                                                                                            \
     if (q_is_f16)                                                                                                               \
         launch_attn_pipe<GHV, __half>(seqs, n_seqs, static_cast<const __half*>(q), q_heads, kv_heads, n_splits, k_seed, qjl_seed, \
@@ -1494,11 +1496,11 @@ void launch_kv_attention(const void* d_seqs, int n_seqs, const void* q, bool q_i
     }
     if (head_dim == 128) {
         if (q_is_f16)
-            launch_pdl(attn_mma_kernel<__half>, grid, dim3(kMmaThreads), 0, stream, static_cast<const AttnSeq*>(d_seqs),
+            launch_pdl(attn_mma_kernel<__half>, grid, dim3(kMmaThreads), 0, stream, seqs,
                        static_cast<const __half*>(q), q_heads, kv_heads, n_splits, k_seed, qjl_seed, use_qjl ? 1 : 0, inv_sqrt,
                        inv_scale_d, attn_scale, gamma, part_acc, part_ml);
         else
-            launch_pdl(attn_mma_kernel<float>, grid, dim3(kMmaThreads), 0, stream, static_cast<const AttnSeq*>(d_seqs),
+            launch_pdl(attn_mma_kernel<float>, grid, dim3(kMmaThreads), 0, stream, seqs,
                        static_cast<const float*>(q), q_heads, kv_heads, n_splits, k_seed, qjl_seed, use_qjl ? 1 : 0, inv_sqrt,
                        inv_scale_d, attn_scale, gamma, part_acc, part_ml);
         launch_pdl(attn_combine_kernel<4>, dim3(static_cast<unsigned>((n_rows + 3) / 4)), dim3(128), 0, stream, part_acc, part_ml, n_rows,

@@ -18,6 +18,7 @@
 #include <cmath>
 
 #include "tq_common.cuh"
+#include "tq_host.hpp"
 #include "tq_kernels.cuh"
 
 namespace tq {
@@ -215,14 +216,14 @@ void derive_seeds(const float* d_weight, size_t n_elems, uint32_t* seed_primary,
     const int n = byte_count ? static_cast<int>((byte_count + stride - 1) / stride) : 0;
     std::vector<uint8_t> sample(n);
     if (n) {
-        uint8_t* d_sample = nullptr;
-        TQ_CUDA(cudaMalloc(&d_sample, n));
+        DeviceBuffer buf;
+        buf.reserve(n, stream);
+        uint8_t* const d_sample = buf.as<uint8_t>();
         gather_bytes_kernel<<<(n + 255) / 256, 256, 0, stream>>>(reinterpret_cast<const uint8_t*>(d_weight), byte_count,
                                                                  stride, d_sample, n);
-        cudaError_t e = cudaMemcpyAsync(sample.data(), d_sample, n, cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        cudaFree(d_sample);
-        TQ_CUDA(e);
+        TQ_CUDA(cudaMemcpyAsync(sample.data(), d_sample, n, cudaMemcpyDeviceToHost, stream));
+        TQ_CUDA(cudaStreamSynchronize(stream));
+        buf.set_idle();
     }
     *seed_primary = fnv1a(sample, 0u);
     *seed_residual = fnv1a(sample, 1u);
