@@ -20,7 +20,42 @@ from ._lib import TQ_F16, TQ_F32, TQError, check
 
 
 def _is_torch(x) -> bool:
-    return type(x).__module__.startswith("torch")
+    return hasattr(x, "data_ptr")
+
+
+# torch dtype -> tag and the torch module, filled in by the first tensor that comes by (the package works without torch)
+_torch = None
+_TORCH_TAGS: dict = {}
+
+
+def _load_torch():
+    global _torch
+    import torch
+    _TORCH_TAGS.update({torch.float32: TQ_F32, torch.float16: TQ_F16})
+    _torch = torch
+    return torch
+
+
+# The calls of a decode step move a few microseconds of work to the GPU each, so their Python side is kept to a handful
+# of attribute look-ups: a forward call took 14.7 us to enqueue, of which 4.2 us were the library's.
+def _tensor(x) -> int:
+    """Address of a contiguous torch tensor."""
+    if not x.is_contiguous():
+        raise ValueError("tensor must be contiguous")
+    return x.data_ptr()
+
+
+def _tensor_tag(x) -> int:
+    if _torch is None:
+        _load_torch()
+    tag = _TORCH_TAGS.get(x.dtype)
+    if tag is None:
+        raise TypeError(f"expected float32 or float16, got {x.dtype}")
+    return tag
+
+
+def _handles(items) -> "C.Array":
+    return (C.c_void_p * len(items))(*[i._h for i in items])
 
 
 def _ptr(x):
@@ -260,6 +295,7 @@ class TurboQuantLinear:
         if not self._h:
             raise TQError("TurboQuantLinear: " + _lib.last_error())
         self.in_features_, self.out_features_ = in_features, out_features
+        self._forward = L.tq_linear_forward
 
     def in_features(self) -> int:
         return self.in_features_
@@ -273,21 +309,30 @@ class TurboQuantLinear:
 
     def forward(self, x, out=None, stream=None):
         """[batch, in] fp32/fp16 -> fp16 [batch, out] (src/linear.cpp:20-26)."""
-        if not _is_torch(x):
-            x = np.ascontiguousarray(x)
-            if x.dtype not in (np.float32, np.float16):
-                x = x.astype(np.float32)
-        if x.shape[-1] != self.in_features_:
-            raise ValueError("input feature size mismatch")
-        batch = int(np.prod(x.shape[:-1])) if len(x.shape) > 1 else 1
-        if out is None:
-            if _is_torch(x):
-                import torch
-                out = torch.empty((batch, self.out_features_), dtype=torch.float16, device=x.device)
+        n_in = self.in_features_
+        if hasattr(x, "data_ptr"):
+            tag = _tensor_tag(x)
+            if x.size(-1) != n_in:
+                raise ValueError("input feature size mismatch")
+            xp, batch = _tensor(x), x.numel() // n_in
+            if out is None:
+                out = x.new_empty((batch, self.out_features_), dtype=_torch.float16)
+                yp = out.data_ptr()
             else:
+                yp = _ptr(out)
+        else:
+            x = np.ascontiguousarray(x)
+            if x.dtype != np.float32 and x.dtype != np.float16:
+                x = x.astype(np.float32)
+            if x.shape[-1] != n_in:
+                raise ValueError("input feature size mismatch")
+            tag = TQ_F32 if x.dtype == np.float32 else TQ_F16
+            xp, batch = x.ctypes.data, x.size // n_in
+            if out is None:
                 out = np.empty((batch, self.out_features_), np.float16)
-        check(self._L.tq_linear_forward(self._h, _ptr(x), _dtype_tag(x), batch, _ptr(out), _stream_ptr(stream)),
-              "TurboQuantLinear.forward")
+            yp = _ptr(out)
+        if self._forward(self._h, xp, tag, batch, yp, None if stream is None else _stream_ptr(stream)):
+            check(-1, "TurboQuantLinear.forward")
         return out
 
     def dequantize(self, dtype=np.float32, out=None, stream=None):
@@ -351,15 +396,19 @@ def forward_group(linears, x, outs=None, stream=None):
     """Several TurboQuantLinear layers on the same device activation x ([batch, in] fp16 torch tensor) in one launch
     of each kernel of the path (tq_linear_forward_group): returns the list of fp16 [batch, out_i] results, each bit-equal
     to linears[i].forward(x).  The layers must share in_features, the WHT block and the rotation mode (q / k / v, gate / up)."""
-    import torch
     if not linears or len(linears) > 4:
         raise ValueError("forward_group takes 1..4 layers")
-    batch = int(np.prod(x.shape[:-1])) if len(x.shape) > 1 else 1
+    first = linears[0]
+    batch = x.numel() // x.size(-1) if x.dim() > 1 else 1
     if outs is None:
-        outs = [torch.empty((batch, lin.out_features_), dtype=torch.float16, device=x.device) for lin in linears]
-    hs = (C.c_void_p * len(linears))(*[lin._h for lin in linears])
-    ys = (C.c_void_p * len(linears))(*[o.data_ptr() for o in outs])
-    check(linears[0]._L.tq_linear_forward_group(hs, len(linears), _ptr(x), batch, ys, _stream_ptr(stream)), "forward_group")
+        if _torch is None:
+            _load_torch()
+        f16 = _torch.float16
+        outs = [x.new_empty((batch, lin.out_features_), dtype=f16) for lin in linears]
+    ys = (C.c_void_p * len(outs))(*[o.data_ptr() for o in outs])
+    if first._L.tq_linear_forward_group(_handles(linears), len(linears), _tensor(x), batch, ys,
+                                        None if stream is None else _stream_ptr(stream)):
+        check(-1, "forward_group")
     return outs
 
 
@@ -523,10 +572,11 @@ class DecodeBuffer:
         return self._L.tq_decode_buffer_current_length(self._h)
 
     def _kv(self, keys, values, ndim):
-        if not _is_torch(keys):
+        if not hasattr(keys, "data_ptr"):
             keys = np.ascontiguousarray(keys)
             values = np.ascontiguousarray(values)
-        if tuple(keys.shape) != tuple(values.shape) or len(keys.shape) != ndim or tuple(keys.shape[-2:]) != (self.num_heads, self.head_dim):
+        shape = keys.shape
+        if shape != values.shape or len(shape) != ndim or shape[-2] != self.num_heads or shape[-1] != self.head_dim:
             raise ValueError("keys and values must both be [..., num_heads, head_dim]")
         return keys, values
 
@@ -581,31 +631,38 @@ def hybrid_attention(cache, buffer, layer: int, queries, out=None, stream=None):
     """hybrid_attention (src/attention_dispatch.cpp:21-74) for one query position: queries
     [q_heads, head_dim] -> fp16 [q_heads, head_dim].  Contexts that fit the decode window are attended
     there, longer ones over the compressed cache."""
-    L = _lib.load()
-    if not _is_torch(queries):
+    tensor = hasattr(queries, "data_ptr")
+    if not tensor:
         queries = np.ascontiguousarray(queries)
-    if len(queries.shape) != 2 or queries.shape[-1] != cache.head_dim:
+    shape = queries.shape
+    if len(shape) != 2 or shape[-1] != cache.head_dim:
         raise ValueError("queries must be [q_heads, head_dim]")
-    if out is None:
-        if _is_torch(queries):
-            import torch
-            out = torch.empty(tuple(queries.shape), dtype=torch.float16, device=queries.device)
-        else:
-            out = np.empty(queries.shape, np.float16)
-    check(L.tq_hybrid_attention(cache.handle, buffer.handle, layer, _ptr(queries), _dtype_tag(queries), int(queries.shape[0]),
-                                _ptr(out), _stream_ptr(stream)), "hybrid_attention")
+    if tensor:
+        qp, tag = _tensor(queries), _tensor_tag(queries)
+        if out is None:
+            out = _torch.empty_like(queries, dtype=_torch.float16)
+    else:
+        qp, tag = _ptr(queries), _dtype_tag(queries)
+        if out is None:
+            out = np.empty(shape, np.float16)
+    if cache._L.tq_hybrid_attention(cache._h, buffer._h, layer, qp, tag, int(shape[0]), _ptr(out),
+                                    None if stream is None else _stream_ptr(stream)):
+        check(-1, "hybrid_attention")
     return out
 
 
 def append_batch(caches, layer: int, keys, values, stream=None):
     """One decode step of a batch: row i of keys / values ([n_seqs, heads, head_dim], device
     tensors) is appended as one token to caches[i]; two kernel launches per 32 sequences."""
-    L = _lib.load()
     n = len(caches)
-    if int(keys.shape[0]) != n or int(values.shape[0]) != n:
+    if keys.shape[0] != n or values.shape[0] != n:
         raise ValueError("keys and values must have one row per cache")
-    arr = (C.c_void_p * n)(*[c.handle for c in caches])
-    check(L.tq_kv_append_batch(arr, n, layer, _ptr(keys), _ptr(values), _dtype_tag(keys), _stream_ptr(stream)), "append_batch")
+    if hasattr(keys, "data_ptr"):
+        kp, vp, tag = _tensor(keys), _tensor(values), _tensor_tag(keys)
+    else:
+        kp, vp, tag = _ptr(keys), _ptr(values), _dtype_tag(keys)
+    if caches[0]._L.tq_kv_append_batch(_handles(caches), n, layer, kp, vp, tag, None if stream is None else _stream_ptr(stream)):
+        check(-1, "append_batch")
 
 
 def compressed_attention(caches, layer: int, queries, start: int = 0, end: int = -1, use_qjl: bool = False,
@@ -615,31 +672,30 @@ def compressed_attention(caches, layer: int, queries, start: int = 0, end: int =
     queries: [n_seqs, q_heads, head_dim] -> fp16 of the same shape.  With return_lse the result
     is (out, lse): lse[n_seqs, q_heads] fp32 is the log of each row's softmax denominator, which
     lets results over disjoint token ranges be merged (sharding.merge_attention_parts)."""
-    L = _lib.load()
     if isinstance(caches, TQKVCache):
         caches = [caches]
-    n = len(caches)
-    if not _is_torch(queries):
+    n, L = len(caches), caches[0]._L
+    tensor = hasattr(queries, "data_ptr")
+    if not tensor:
         queries = np.ascontiguousarray(queries)
-    if queries.shape[0] != n or queries.shape[-1] != caches[0].head_dim:
+    shape = queries.shape
+    if shape[0] != n or shape[-1] != caches[0].head_dim:
         raise ValueError("queries must be [n_seqs, q_heads, head_dim]")
-    q_heads = int(queries.shape[1])
-    if out is None:
-        if _is_torch(queries):
-            import torch
-            out = torch.empty(tuple(queries.shape), dtype=torch.float16, device=queries.device)
-        else:
-            out = np.empty(queries.shape, np.float16)
-    arr = (C.c_void_p * n)(*[c.handle for c in caches])
-    if not return_lse:
-        check(L.tq_kv_attention(arr, n, layer, _ptr(queries), _dtype_tag(queries), q_heads, _ptr(out), start, end,
-                                int(use_qjl), _stream_ptr(stream)), "compressed_attention")
-        return out
-    if _is_torch(queries):
-        import torch
-        lse = torch.empty((n, q_heads), dtype=torch.float32, device=queries.device)
+    q_heads = int(shape[1])
+    lse = None
+    if tensor:
+        qp, tag = _tensor(queries), _tensor_tag(queries)
+        if out is None:
+            out = _torch.empty_like(queries, dtype=_torch.float16)
+        if return_lse:
+            lse = queries.new_empty((n, q_heads), dtype=_torch.float32)
     else:
-        lse = np.empty((n, q_heads), np.float32)
-    check(L.tq_kv_attention_lse(arr, n, layer, _ptr(queries), _dtype_tag(queries), q_heads, _ptr(out), _ptr(lse), start,
-                                end, int(use_qjl), _stream_ptr(stream)), "compressed_attention")
-    return out, lse
+        qp, tag = _ptr(queries), _dtype_tag(queries)
+        if out is None:
+            out = np.empty(shape, np.float16)
+        if return_lse:
+            lse = np.empty((n, q_heads), np.float32)
+    if L.tq_kv_attention_lse(_handles(caches), n, layer, qp, tag, q_heads, _ptr(out), None if lse is None else _ptr(lse), start, end,
+                             1 if use_qjl else 0, None if stream is None else _stream_ptr(stream)):
+        check(-1, "compressed_attention")
+    return (out, lse) if return_lse else out

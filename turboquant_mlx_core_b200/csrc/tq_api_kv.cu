@@ -72,7 +72,7 @@ public:
         TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16, "append: keys/values must be fp32 or fp16");
         TQ_REQUIRE(tokens >= 0, "append: negative token count");
         if (tokens == 0) return;
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         reserve(L, L.num_tokens + tokens, st);
@@ -109,7 +109,7 @@ public:
     void reserve_tokens(int layer, int tokens, cudaStream_t st) {
         TQ_REQUIRE(layer >= 0 && layer < layers_n_, "Layer index out of range");
         TQ_REQUIRE(tokens >= 0, "reserve: negative token count");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         if (tokens > L.capacity) {
             use_.note(st);
@@ -129,7 +129,7 @@ public:
         TQKVCache* c0 = caches[0];
         TQ_REQUIRE(c0, "append_batch: NULL cache");
         TQ_REQUIRE(layer >= 0 && layer < c0->layers_n_, "Layer index out of range");
-        TQ_CUDA(cudaSetDevice(c0->device_));
+        tq::ensure_device(c0->device_);
         const int wph = c0->words_per_head(), qph = c0->qjl_words_per_head();
         const uint32_t ks = tq::kv_layer_seed(static_cast<uint32_t>(layer), 1);
         const uint32_t vs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 2);
@@ -171,7 +171,7 @@ public:
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         TQ_REQUIRE(start >= 0 && end <= L.num_tokens && start < end, "Invalid token range for dequantization");
         TQ_REQUIRE(out, "get_fp16: NULL output");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         const size_t n_vec = static_cast<size_t>(end - start) * heads_;
         const size_t off = static_cast<size_t>(start) * heads_;
@@ -200,7 +200,7 @@ public:
                      uint32_t* qjl_words, float* qjl_norms) {
         TQ_REQUIRE(layer >= 0 && layer < layers_n_, "Layer index out of range");
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         const size_t n = static_cast<size_t>(L.num_tokens) * heads_;
         auto copy = [&](void* dst, const void* src, size_t bytes) {
@@ -230,7 +230,7 @@ public:
     }
     // Writes the stream into host memory `out` (snapshot_bytes() bytes).
     void snapshot_to(uint8_t* out, uint32_t model_hash, uint32_t codebook_hash) {
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         size_t pos = 0;
         auto put = [&](uint32_t v) { std::memcpy(out + pos, &v, 4); pos += 4; };
@@ -295,7 +295,7 @@ public:
             }
             TQ_REQUIRE(pos == end, "restore: trailing bytes in a layer blob");
         }
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         seq_length_ = 0;
         for (uint32_t l = 0; l < layers; ++l) {
@@ -337,7 +337,7 @@ public:
         return total;
     }
     void delta_to(uint8_t* out, uint32_t from, uint32_t to) {
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         size_t pos = 0;
         auto put = [&](uint32_t v) { std::memcpy(out + pos, &v, 4); pos += 4; };
@@ -400,7 +400,7 @@ public:
             }
             TQ_REQUIRE(pos == end, "apply_delta: trailing bytes in a layer blob");
         }
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         for (uint32_t l = 0; l < layers; ++l) {
             LayerKVStorage& L = layers_[l];
@@ -551,7 +551,7 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
     const int heads = c0->num_heads(), dim = c0->head_dim();
     TQ_REQUIRE(q_heads > 0 && q_heads % heads == 0, "attention: query heads must be a multiple of KV heads");
     TQ_REQUIRE(dim <= 256, "attention: head_dim above 256 is not supported");
-    TQ_CUDA(cudaSetDevice(c0->device()));
+    tq::ensure_device(c0->device());
     c0->check_attention_status();   // a failure of an earlier asynchronous call
     tq::AttnSeqs seqs;
     seqs.table = nullptr;
@@ -655,7 +655,7 @@ public:
         // src/decode_buffer.cpp:128-141
         TQ_REQUIRE(start >= 0 && end > start && end <= current_length_, "DecodeBuffer: requested range is out of bounds");
         TQ_REQUIRE(out != nullptr, "decode buffer: NULL output");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         const long n = end - start;
         const int row = heads_ * dim_;
         const bool dev = tq::is_device_pointer(out);
@@ -676,7 +676,7 @@ private:
         TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16, "decode buffer: keys and values must be fp32 or fp16");
         if (n == 0) return;
         TQ_REQUIRE(keys != nullptr && values != nullptr, "decode buffer: NULL keys or values");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         const int row = heads_ * dim_;
         const size_t bytes = static_cast<size_t>(n) * row * (dtype == TQ_F32 ? 4 : 2);
         const void* dk = keys;
@@ -714,7 +714,7 @@ void hybrid_attention(TQKVCache* cache, DecodeBuffer* buf, int layer, const void
     TQ_REQUIRE(q_heads > 0 && q_heads % heads == 0, "hybrid_attention: query heads must be a multiple of KV heads");
     const int seq_len = cache->seq_length();
     const size_t n_q = static_cast<size_t>(q_heads) * dim;
-    TQ_CUDA(cudaSetDevice(cache->device()));
+    tq::ensure_device(cache->device());
     if (seq_len == 0) {
         if (tq::is_device_pointer(out)) TQ_CUDA(cudaMemsetAsync(out, 0, n_q * sizeof(__half), st));
         else std::memset(out, 0, n_q * sizeof(__half));

@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <optional>
 
 #include "tq_host.hpp"
 #include "tq_kernels.cuh"
@@ -131,20 +132,34 @@ public:
         TQ_REQUIRE(batch >= 0, "TurboQuantLinear::forward: negative batch");
         TQ_REQUIRE(x_dtype == TQ_F32 || x_dtype == TQ_F16, "TurboQuantLinear::forward: x must be fp32 or fp16");
         if (batch == 0) return;
-        make_current();
+        tq::ensure_device(device_);
         use_.note(st);
         const size_t nx = static_cast<size_t>(batch) * in_, ny = static_cast<size_t>(batch) * out_;
         const PointerKind kx = classify(x), ky = classify(y);
         const bool x_dev = kx.device, y_dev = ky.device;
 
+        // Host memory, a decode call: a few rows travel as kernel parameters, more of them through page-locked staging
+        // (the call waits for its result, so the staging is free again when it returns); see tq_host_rows.cu.
+        const bool decode_call = batch <= 8 || nx * sizeof(__half) <= kHostStageBytes;
         const __half* d_x;
-        if (x_dtype == TQ_F16) {
-            if (x_dev) d_x = static_cast<const __half*>(x);
-            else {
-                x_f16_.reserve(nx * sizeof(__half), st);
-                TQ_CUDA(cudaMemcpyAsync(x_f16_.as<void>(), x, nx * sizeof(__half), cudaMemcpyHostToDevice, st));
-                d_x = x_f16_.as<__half>();
+        std::optional<tq::PinnedStage> x_stage, y_stage;
+        if (x_dev && x_dtype == TQ_F16) {
+            d_x = static_cast<const __half*>(x);
+        } else if (!x_dev && (nx * sizeof(__half) <= tq::kMaxParamRowBytes || (!y_dev && decode_call && kx.pinned_alias == nullptr))) {
+            x_f16_.reserve(nx * sizeof(__half) + 16, st);
+            d_x = x_f16_.as<__half>();
+            if (nx * sizeof(__half) <= tq::kMaxParamRowBytes) {
+                tq::launch_rows_from_params(x, x_dtype == TQ_F16, nx, x_f16_.as<__half>(), st);
+            } else {
+                x_stage.emplace(nx * sizeof(__half));
+                if (x_dtype == TQ_F16) std::memcpy(x_stage->host(), x, nx * sizeof(__half));
+                else tq::host_f32_to_f16(static_cast<const float*>(x), x_stage->host<uint16_t>(), nx);
+                TQ_CUDA(cudaMemcpyAsync(x_f16_.as<void>(), x_stage->host(), nx * sizeof(__half), cudaMemcpyHostToDevice, st));
             }
+        } else if (x_dtype == TQ_F16) {
+            x_f16_.reserve(nx * sizeof(__half), st);
+            TQ_CUDA(cudaMemcpyAsync(x_f16_.as<void>(), x, nx * sizeof(__half), cudaMemcpyHostToDevice, st));
+            d_x = x_f16_.as<__half>();
         } else {
             const float* d_xf;
             if (x_dev) d_xf = static_cast<const float*>(x);
@@ -157,20 +172,25 @@ public:
             tq::launch_f32_to_f16(d_xf, x_f16_.as<__half>(), static_cast<long>(nx), st);  // src/dequantizer.cpp:691
             d_x = x_f16_.as<__half>();
         }
-        // A few rows into page-locked host memory: the decode kernel stores them there itself
-        // (8 KB of posted writes cost less than a separate copy); anything larger or pageable is staged.
-        void* y_alias = (!y_dev && batch <= 8) ? ky.pinned_alias : nullptr;
+        // A few rows into page-locked host memory, the caller's or our staging: the decode kernel stores them there itself
+        // (8 KB of posted writes cost less than a separate copy).  Larger results are copied.
         __half* d_y;
-        if (y_dev) d_y = static_cast<__half*>(y);
-        else if (y_alias) d_y = static_cast<__half*>(y_alias);
-        else {
+        if (y_dev) {
+            d_y = static_cast<__half*>(y);
+        } else if (batch <= 8 && ky.pinned_alias != nullptr) {
+            d_y = static_cast<__half*>(ky.pinned_alias);
+        } else if (batch <= 8 && ny * sizeof(__half) <= kHostStageBytes) {
+            y_stage.emplace(ny * sizeof(__half));
+            d_y = y_stage->device<__half>();
+        } else {
             y_f16_.reserve(ny * sizeof(__half), st);
             d_y = y_f16_.as<__half>();
         }
         launch_forward(d_x, batch, d_y, st);
         if (!y_dev) {
-            if (!y_alias) TQ_CUDA(cudaMemcpyAsync(y, d_y, ny * sizeof(__half), cudaMemcpyDeviceToHost, st));
+            if (d_y == y_f16_.as<__half>()) TQ_CUDA(cudaMemcpyAsync(y, d_y, ny * sizeof(__half), cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));
+            if (y_stage) std::memcpy(y, y_stage->host(), ny * sizeof(__half));
             require_ok(*static_cast<volatile unsigned int*>(h_status_));
         }
     }
@@ -187,7 +207,7 @@ public:
         TQ_REQUIRE(row_offset >= 0 && row_offset + out_ <= dst_stride,
                    "forward_scatter: rows [row_offset, row_offset + out) must fit the destination row stride");
         TQ_REQUIRE(tq::is_device_pointer(x), "forward_scatter: x must be a device pointer");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         __half* d[8];
         for (int i = 0; i < n_dst; ++i) {
@@ -241,7 +261,7 @@ public:
         TQ_REQUIRE(batch >= 1, "forward_strided: batch must be positive");
         TQ_REQUIRE(y_stride >= out_, "forward_strided: row stride smaller than out_features");
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y), "forward_strided: x and y must be device pointers");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         launch_forward(static_cast<const __half*>(x), batch, static_cast<__half*>(y), st, y_stride);
     }
@@ -257,7 +277,7 @@ public:
                    "forward_allgather: rows [row_offset, row_offset + out) must fit the destination row stride");
         TQ_REQUIRE(slot >= 0 && slot < 32, "forward_allgather: flag slot must be 0..31");
         TQ_REQUIRE(tq::is_device_pointer(x), "forward_allgather: x must be a device pointer");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         __half* d[8];
         for (int i = 0; i < n_dst; ++i) {
@@ -280,7 +300,7 @@ public:
         TQ_REQUIRE(world >= 1 && world <= 8 && rank >= 0 && rank < world, "forward_allgather_packets: bad rank / world");
         TQ_REQUIRE(y_stride >= out_, "forward_allgather_packets: row stride smaller than the layer's rows");
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y), "forward_allgather_packets: x and y must be device pointers");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         __half* d[1] = {static_cast<__half*>(y)};
         tq::GemvGather g{epoch, nullptr, wait ? 1 : 0, wait_epoch};
@@ -293,13 +313,13 @@ public:
     }
 
     void wait_peers(const void* flags, int n, unsigned int value, cudaStream_t st) {
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         tq::launch_peer_wait(static_cast<const unsigned int*>(flags), n, value, d_status_, st);
     }
 
     void check_status() {
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
         require_ok(*static_cast<volatile unsigned int*>(h_status_));
     }
@@ -308,7 +328,7 @@ public:
     void dequantize(void* result, int dtype, cudaStream_t st) {
         TQ_REQUIRE(result, "dequantize: NULL result");
         TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16, "dequantize: result must be fp32 or fp16");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         const size_t n = static_cast<size_t>(out_) * in_;
         const size_t es = dtype == TQ_F32 ? 4 : 2;
@@ -339,7 +359,7 @@ public:
         TQ_REQUIRE(batch >= 1 && batch <= 8, "allocation-free forward: batch must be 1..8");
         TQ_REQUIRE(tq::is_device_pointer(x) && tq::is_device_pointer(y),
                    "allocation-free forward: x and y must be device pointers (copying host memory would need a staging allocation)");
-        TQ_CUDA(cudaSetDevice(device_));
+        tq::ensure_device(device_);
         use_.note(st);
         // the kernel forward() would run, when its working set fits the array; else the other one
         if (decode_kernel_ == 2 && tq::gemv_staged_fits_static(out_, in_, batch, dual_ ? 2 : 1, sm_count_))
@@ -389,11 +409,6 @@ private:
         next_kind_ = (next_kind_ + 1) & 3;
         return k;
     }
-    // cudaSetDevice only when another device is current (it is not free even as a no-op).
-    void make_current() {
-        int cur = -1;
-        if (cudaGetDevice(&cur) != cudaSuccess || cur != device_) TQ_CUDA(cudaSetDevice(device_));
-    }
     PointerKind kinds_[4];
     int next_kind_ = 0;
 
@@ -411,6 +426,7 @@ private:
     // Device pointers only.  More than kGemmMinBatch rows go to the tensor-core GEMM (when the
     // shape allows); otherwise batches above 8 rows are issued as passes of 8 through the GEMV.
     static constexpr int kGemmMinBatch = 8;
+    static constexpr size_t kHostStageBytes = size_t(4) << 20;   // rows of a host caller that go through page-locked staging
     // y_stride: elements between activation rows of y (0 = out_features: a dense [batch, out] result).
     void launch_forward(const __half* d_x, int batch, __half* d_y, cudaStream_t st, long y_stride = 0) {
         if (y_stride <= 0) y_stride = out_;
@@ -518,7 +534,7 @@ int tq_linear_forward_group(const tq_linear_t* lins, int n, const void* x_fp16_d
                        lins[i]->impl->block_size() == lins[0]->impl->block_size(),
                        "tq_linear_forward_group: the layers must share in_features, the WHT block and the rotation mode");
         }
-        TQ_CUDA(cudaSetDevice(lins[0]->impl->device()));
+        tq::ensure_device(lins[0]->impl->device());
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         if (lins[0]->impl->gemm_path(batch)) {
             // 9 rows and up: one rotation launch, one tensor-memory GEMM launch and one split-K finish for the group

@@ -36,6 +36,11 @@ R guarded(R ok_unused, R fail, F&& body) {
 // ---- device selection -------------------------------------------------------------------
 int current_device();
 int sm_count(int device);
+// cudaSetDevice only when another device is current (it is not free even as a no-op).
+inline void ensure_device(int device) {
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess || cur != device) TQ_CUDA(cudaSetDevice(device));
+}
 
 // ---- pointers ---------------------------------------------------------------------------
 // True when the CUDA driver knows `p` as device (or managed) memory.
@@ -75,6 +80,23 @@ void pool_trim();
 unsigned int* status_word_take(int device);
 // All work that could write the word was put on the legacy default stream, or has ended.
 void status_word_return(unsigned int* w, int device);
+
+
+// Page-locked host memory for the length of one call that waits for its result (kept for the next call).
+class PinnedStage {
+public:
+    explicit PinnedStage(size_t bytes);
+    ~PinnedStage();
+    PinnedStage(const PinnedStage&) = delete;
+    PinnedStage& operator=(const PinnedStage&) = delete;
+    template <typename T = void> T* host() const { return static_cast<T*>(p_); }
+    template <typename T = void> T* device() const { return static_cast<T*>(alias_); }   // its address for kernels
+
+private:
+    void* p_ = nullptr;
+    void* alias_ = nullptr;
+    size_t bytes_ = 0;
+};
 
 // Which streams an object's memory has been used on: what its release has to wait for.
 class StreamUse {

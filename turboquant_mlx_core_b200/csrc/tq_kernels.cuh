@@ -216,6 +216,10 @@ void launch_swiglu_f16(const __half* gate_up, __half* act, long rows, int inter,
 
 // tq_misc.cu — small element-wise helpers.
 void launch_f32_to_f16(const float* in, __half* out, long n, cudaStream_t stream);
+// Activation rows of a host caller (tq_host_rows.cu).
+constexpr size_t kMaxParamRowBytes = 31744;   // fp16 bytes that travel as kernel parameters (a launch takes 32 764)
+void host_f32_to_f16(const float* src, uint16_t* dst, size_t n);
+void launch_rows_from_params(const void* host_x, bool is_f16, size_t n, __half* dst, cudaStream_t stream);
 void launch_f16_to_f32(const __half* in, float* out, long n, cudaStream_t stream);
 
 }  // namespace tq

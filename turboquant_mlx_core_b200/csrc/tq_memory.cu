@@ -25,6 +25,7 @@ namespace {
 
 constexpr size_t kKeepBytes = size_t(512) << 20;
 constexpr double kKeepSeconds = 30.0;
+constexpr size_t kKeepPinnedBytes = size_t(32) << 20;
 constexpr size_t kStatusWords = 512;   // page-locked status words per page
 
 double now_s() {
@@ -45,8 +46,16 @@ struct Word {
     cudaEvent_t pending;
 };
 
+struct Pinned {
+    void* p;
+    void* alias;
+    size_t bytes;
+};
+
 struct Pool {
     std::mutex mu;
+    std::vector<Pinned> pinned;   // page-locked staging, the latest last
+    size_t pinned_kept = 0;
     std::list<Block> blocks;   // in order of release: the oldest first
     size_t kept[64] = {0};
     std::list<Word> words;
@@ -207,6 +216,45 @@ void status_word_return(unsigned int* w, int device) {
     cudaEvent_t e = device >= 0 && device < 64 ? mark_legacy_stream(P, device) : nullptr;
     if (!e) return;   // 4 bytes stay with the page
     P.words.push_back(Word{w, device, e});
+}
+
+PinnedStage::PinnedStage(size_t bytes) {
+    size_t want = size_t(64) << 10;
+    while (want < bytes) want *= 2;
+    Pool& P = pool();
+    {
+        std::lock_guard<std::mutex> lock(P.mu);
+        for (size_t i = P.pinned.size(); i-- > 0;) {
+            if (P.pinned[i].bytes != want) continue;
+            p_ = P.pinned[i].p;
+            alias_ = P.pinned[i].alias;
+            bytes_ = want;
+            P.pinned.erase(P.pinned.begin() + static_cast<long>(i));
+            P.pinned_kept -= want;
+            return;
+        }
+    }
+    TQ_CUDA(cudaHostAlloc(&p_, want, cudaHostAllocPortable | cudaHostAllocMapped));
+    bytes_ = want;
+    alias_ = pinned_host_device_alias(p_);
+    if (alias_ == nullptr) {
+        cudaFreeHost(p_);
+        throw Error("page-locked staging memory is not mapped for the device");
+    }
+}
+
+PinnedStage::~PinnedStage() {
+    if (!p_) return;
+    Pool& P = pool();
+    {
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (P.pinned_kept + bytes_ <= kKeepPinnedBytes) {
+            P.pinned.push_back(Pinned{p_, alias_, bytes_});
+            P.pinned_kept += bytes_;
+            return;
+        }
+    }
+    cudaFreeHost(p_);
 }
 
 }  // namespace tq
