@@ -494,9 +494,7 @@ class TQKVCache:
     ATTENTION_AUTO, ATTENTION_LOADS, ATTENTION_PIPELINE, ATTENTION_TENSOR_MEMORY = 0, 1, 2, 3
 
     def set_attention_kernel(self, kernel: int):
-        """Decode-attention kernel for calls that name this cache first: automatic (by job size),
-        the load-based kernel, the bulk-copy pipeline, or the tensor-memory kernel (head_dim 128, four KV
-        heads; other shapes fall back to the automatic choice)."""
+        """Accepts the four values above; one kernel serves them all."""
         check(self._L.tq_kv_set_attention_kernel(self._h, int(kernel)), "TQKVCache.set_attention_kernel")
 
     def check_attention_status(self):

@@ -17,31 +17,15 @@
 #include "turboquant_c/turboquant_b200.h"
 #include "turboquant_c/turboquant_c.h"
 
-namespace tq {
-// tq_kv_kernels.cu
-void launch_kv_encode(const void* x, bool x_is_f16, long n_vec, int head_dim, uint32_t wht_seed, uint32_t qjl_seed,
-                      bool with_qjl, uint32_t* words, float* norms, uint32_t* qjl_words, float* qjl_norms,
-                      cudaStream_t stream);
-void launch_kv_decode_f16(const uint32_t* words, const float* norms, long n_vec, int head_dim, uint32_t wht_seed,
-                          __half* out, cudaStream_t stream);
-size_t attn_scratch_bytes(int n_seqs, int q_heads, int head_dim, int n_splits);
-void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads,
-                         int head_dim, AttnPlan plan, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl,
-                         void* scratch, __half* out, float* lse, unsigned int* status, cudaStream_t stream);
-AttnPlan attn_make_plan(int n_seqs, int q_heads, int kv_heads, int head_dim, int max_tok, int sm_count, int kernel);
-}  // namespace tq
-
 namespace turboquant {
 
 using tq::DeviceBuffer;
 using tq::Error;
 
 struct LayerKVStorage {
-    DeviceBuffer slab;   // the six arrays, see tq::KvSlab
-    uint32_t *k_words = nullptr, *v_words = nullptr, *qjl_words = nullptr;
-    float *k_norms = nullptr, *v_norms = nullptr, *qjl_norms = nullptr;
+    DeviceBuffer slab;   // blocks of 16 tokens and one head (tq_attn.cuh)
     int num_tokens = 0;
-    int capacity = 0;
+    int capacity = 0;    // a multiple of 16
 };
 
 class TQKVCache {
@@ -54,7 +38,7 @@ public:
                    "TQKVCache: head_dim must be a power of two in [32, 512]");
         device_ = tq::current_device();
         layers_.resize(static_cast<size_t>(num_layers));
-        for (DeviceBuffer* b : {&stage_k_, &stage_v_, &attn_scratch_, &attn_q_, &attn_out_, &attn_lse_}) b->owned_by(&use_);
+        for (DeviceBuffer* b : {&stage_k_, &stage_v_, &attn_scratch_, &attn_q_, &attn_out_, &attn_lse_, &attn_counters_}) b->owned_by(&use_);
     }
 
     int num_layers() const { return layers_n_; }
@@ -91,16 +75,11 @@ public:
             TQ_CUDA(cudaMemcpyAsync(stage_v_.as<void>(), values, bytes, cudaMemcpyHostToDevice, st));
             d_v = stage_v_.as<void>();
         }
-        const size_t off = static_cast<size_t>(L.num_tokens) * heads_;
-        const int wph = words_per_head(), qph = qjl_words_per_head();
         const uint32_t ks = tq::kv_layer_seed(static_cast<uint32_t>(layer), 1);  // src/kv_cache.cpp:40-42
         const uint32_t vs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 2);
         const uint32_t qs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 3);
-        const tq::KvEncodeSegment kseg{L.k_words + off * wph, L.k_norms + off,
-                                       L.qjl_words + off * qph, L.qjl_norms + off};
-        const tq::KvEncodeSegment vseg{L.v_words + off * wph, L.v_norms + off, nullptr, nullptr};
-        tq::launch_kv_encode_pair_segments(d_k, d_v, dtype == TQ_F16, static_cast<long>(n_vec), static_cast<long>(n_vec), dim_, ks, vs, qs,
-                                           &kseg, &vseg, 1, st);
+        const tq::KvSegment seg{L.slab.as<unsigned char>(), L.num_tokens};
+        tq::launch_kv_encode(d_k, d_v, dtype == TQ_F16, tokens, heads_, dim_, ks, vs, qs, &seg, 1, st);
         L.num_tokens += tokens;
         seq_length_ = std::max(seq_length_, L.num_tokens);
     }
@@ -130,7 +109,6 @@ public:
         TQ_REQUIRE(c0, "append_batch: NULL cache");
         TQ_REQUIRE(layer >= 0 && layer < c0->layers_n_, "Layer index out of range");
         tq::ensure_device(c0->device_);
-        const int wph = c0->words_per_head(), qph = c0->qjl_words_per_head();
         const uint32_t ks = tq::kv_layer_seed(static_cast<uint32_t>(layer), 1);
         const uint32_t vs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 2);
         const uint32_t qs = tq::kv_layer_seed(static_cast<uint32_t>(layer), 3);
@@ -138,7 +116,7 @@ public:
         const size_t vec_bytes = static_cast<size_t>(c0->heads_) * c0->dim_ * es;
         for (int b0 = 0; b0 < n; b0 += 32) {
             const int nb = std::min(32, n - b0);
-            tq::KvEncodeSegment kseg[32], vseg[32];
+            tq::KvSegment seg[tq::kKvMaxSegments];
             for (int i = 0; i < nb; ++i) {
                 TQKVCache* c = caches[b0 + i];
                 TQ_REQUIRE(c && c->heads_ == c0->heads_ && c->dim_ == c0->dim_ && c->device_ == c0->device_ &&
@@ -147,15 +125,11 @@ public:
                 LayerKVStorage& L = c->layers_[static_cast<size_t>(layer)];
                 c->use_.note(st);
                 c->reserve(L, L.num_tokens + 1, st);
-                const size_t off = static_cast<size_t>(L.num_tokens) * c->heads_;
-                kseg[i] = {L.k_words + off * wph, L.k_norms + off,
-                           L.qjl_words + off * qph, L.qjl_norms + off};
-                vseg[i] = {L.v_words + off * wph, L.v_norms + off, nullptr, nullptr};
+                seg[i] = {L.slab.as<unsigned char>(), L.num_tokens};
             }
-            const long n_vec = static_cast<long>(nb) * c0->heads_;
             const char* kp = static_cast<const char*>(keys) + static_cast<size_t>(b0) * vec_bytes;
             const char* vp = static_cast<const char*>(values) + static_cast<size_t>(b0) * vec_bytes;
-            tq::launch_kv_encode_pair_segments(kp, vp, dtype == TQ_F16, n_vec, c0->heads_, c0->dim_, ks, vs, qs, kseg, vseg, nb, st);
+            tq::launch_kv_encode(kp, vp, dtype == TQ_F16, 1, c0->heads_, c0->dim_, ks, vs, qs, seg, nb, st);
             for (int i = 0; i < nb; ++i) {
                 TQKVCache* c = caches[b0 + i];
                 LayerKVStorage& L = c->layers_[static_cast<size_t>(layer)];
@@ -174,7 +148,6 @@ public:
         tq::ensure_device(device_);
         use_.note(st);
         const size_t n_vec = static_cast<size_t>(end - start) * heads_;
-        const size_t off = static_cast<size_t>(start) * heads_;
         const bool dev = tq::is_device_pointer(out);
         DeviceBuffer stage;
         __half* d_out = static_cast<__half*>(out);
@@ -183,10 +156,7 @@ public:
             d_out = stage.as<__half>();
         }
         const uint32_t seed = tq::kv_layer_seed(static_cast<uint32_t>(layer), values ? 2 : 1);
-        const uint32_t* const words = values ? L.v_words : L.k_words;
-        const float* const norms = values ? L.v_norms : L.k_norms;
-        tq::launch_kv_decode_f16(words + off * words_per_head(), norms + off,
-                                 static_cast<long>(n_vec), dim_, seed, d_out, st);
+        tq::launch_kv_decode_f16(L.slab.as<unsigned char>(), start, end - start, heads_, dim_, values, seed, d_out, st);
         if (!dev) {
             TQ_CUDA(cudaMemcpyAsync(out, d_out, n_vec * dim_ * sizeof(__half), cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));
@@ -202,16 +172,10 @@ public:
         LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         tq::ensure_device(device_);
         TQ_CUDA(cudaDeviceSynchronize());
-        const size_t n = static_cast<size_t>(L.num_tokens) * heads_;
-        auto copy = [&](void* dst, const void* src, size_t bytes) {
-            if (dst && bytes) TQ_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDefault));
-        };
-        copy(k_words, L.k_words, n * words_per_head() * 4);
-        copy(v_words, L.v_words, n * words_per_head() * 4);
-        copy(k_norms, L.k_norms, n * 4);
-        copy(v_norms, L.v_norms, n * 4);
-        copy(qjl_words, L.qjl_words, n * qjl_words_per_head() * 4);
-        copy(qjl_norms, L.qjl_norms, n * 4);
+        void* const dst[6] = {k_words, v_words, k_norms, v_norms, qjl_words, qjl_norms};
+        bool any = false;
+        for (void* d : dst) any = any || d != nullptr;
+        if (any) copy_arrays(L, 0, L.num_tokens, dst);
         return L.num_tokens;
     }
 
@@ -245,18 +209,7 @@ public:
         for (const LayerKVStorage& L : layers_) {
             put(static_cast<uint32_t>(layer_blob_bytes(L)));
             put(static_cast<uint32_t>(L.num_tokens));
-            const size_t n = static_cast<size_t>(L.num_tokens) * heads_;
-            auto span = [&](const void* src, size_t bytes) {
-                put(static_cast<uint32_t>(bytes));
-                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, src, bytes, cudaMemcpyDeviceToHost));
-                pos += bytes;
-            };
-            span(L.k_words, n * words_per_head() * 4);
-            span(L.v_words, n * words_per_head() * 4);
-            span(L.k_norms, n * 4);
-            span(L.v_norms, n * 4);
-            span(L.qjl_words, n * qjl_words_per_head() * 4);
-            span(L.qjl_norms, n * 4);
+            put_arrays(L, 0, L.num_tokens, out, pos);
         }
     }
     // Replaces the cache contents with a stream written by snapshot_to (or by the reference's
@@ -302,10 +255,9 @@ public:
             LayerKVStorage& L = layers_[l];
             L.num_tokens = 0;
             reserve(L, static_cast<int>(tokens[l]), nullptr);
-            void* dst[6] = {L.k_words, L.v_words, L.k_norms, L.v_norms, L.qjl_words, L.qjl_norms};
-            for (int i = 0; i < 6; ++i)
-                if (spans[l][i].bytes)
-                    TQ_CUDA(cudaMemcpy(dst[i], data + spans[l][i].off, spans[l][i].bytes, cudaMemcpyHostToDevice));
+            const uint8_t* src[6];
+            for (int i = 0; i < 6; ++i) src[i] = data + spans[l][i].off;
+            load_arrays(L, 0, static_cast<int>(tokens[l]), src);
             L.num_tokens = static_cast<int>(tokens[l]);
             seq_length_ = std::max(seq_length_, L.num_tokens);
         }
@@ -350,19 +302,7 @@ public:
             clamp_range(L, from, to, a, b);
             put(static_cast<uint32_t>(range_blob_bytes(b - a)));
             put(static_cast<uint32_t>(b - a));
-            const size_t n = static_cast<size_t>(b - a) * heads_, first = static_cast<size_t>(a) * heads_;
-            auto span = [&](const void* src, size_t elem_bytes) {
-                const size_t bytes = n * elem_bytes;
-                put(static_cast<uint32_t>(bytes));
-                if (bytes) TQ_CUDA(cudaMemcpy(out + pos, static_cast<const uint8_t*>(src) + first * elem_bytes, bytes, cudaMemcpyDeviceToHost));
-                pos += bytes;
-            };
-            span(L.k_words, static_cast<size_t>(words_per_head()) * 4);
-            span(L.v_words, static_cast<size_t>(words_per_head()) * 4);
-            span(L.k_norms, 4);
-            span(L.v_norms, 4);
-            span(L.qjl_words, static_cast<size_t>(qjl_words_per_head()) * 4);
-            span(L.qjl_norms, 4);
+            put_arrays(L, a, b - a, out, pos);
         }
     }
     // Appends a delta stream (ours or the reference's delta_serialize) to every layer.  The layer
@@ -405,14 +345,9 @@ public:
         for (uint32_t l = 0; l < layers; ++l) {
             LayerKVStorage& L = layers_[l];
             reserve(L, L.num_tokens + static_cast<int>(tokens[l]), nullptr);
-            const size_t first = static_cast<size_t>(L.num_tokens) * heads_;
-            void* dst[6] = {L.k_words, L.v_words, L.k_norms, L.v_norms, L.qjl_words, L.qjl_norms};
-            const size_t elem[6] = {static_cast<size_t>(words_per_head()) * 4, static_cast<size_t>(words_per_head()) * 4, 4, 4,
-                                    static_cast<size_t>(qjl_words_per_head()) * 4, 4};
-            for (int i = 0; i < 6; ++i)
-                if (spans[l][i].bytes)
-                    TQ_CUDA(cudaMemcpy(static_cast<uint8_t*>(dst[i]) + first * elem[i], data + spans[l][i].off, spans[l][i].bytes,
-                                       cudaMemcpyHostToDevice));
+            const uint8_t* src[6];
+            for (int i = 0; i < 6; ++i) src[i] = data + spans[l][i].off;
+            load_arrays(L, L.num_tokens, static_cast<int>(tokens[l]), src);
             L.num_tokens += static_cast<int>(tokens[l]);
             seq_length_ = std::max(seq_length_, L.num_tokens);
         }
@@ -422,7 +357,7 @@ public:
         TQ_REQUIRE(layer >= 0 && layer < layers_n_, "Layer index out of range");
         const LayerKVStorage& L = layers_[static_cast<size_t>(layer)];
         TQ_REQUIRE(start >= 0 && end <= L.num_tokens && start < end, "Invalid token range for attention");
-        return tq::AttnSeq{L.slab.as<unsigned char>(), start, end, L.capacity, 0};
+        return tq::AttnSeq{L.slab.as<unsigned char>(), start, end, 0, 0};
     }
 
     int device() const { return device_; }
@@ -430,10 +365,9 @@ public:
     DeviceBuffer& attn_q() { return attn_q_; }
     DeviceBuffer& attn_out() { return attn_out_; }
     DeviceBuffer& attn_lse() { return attn_lse_; }
-    int attention_kernel() const { return attention_kernel_; }
+    // One kernel serves every shape; the choice between the former ones is still accepted.
     void set_attention_kernel(int k) {
-        TQ_REQUIRE(k >= 0 && k <= 3, "attention kernel: 0 (automatic), 1 (load-based), 2 (bulk-copy pipeline) or 3 (tensor memory)");
-        attention_kernel_ = k;
+        TQ_REQUIRE(k >= 0 && k <= 3, "attention kernel: 0 .. 3");
     }
     // Status word of the attention kernels: page-locked host memory that the device writes
     // directly (only when a bounded wait ran out), so reading it costs the host nothing.
@@ -444,6 +378,15 @@ public:
             TQ_REQUIRE(d_attn_status_ != nullptr, "attention: the status word is not mapped for the device");
         }
         return d_attn_status_;
+    }
+    // Job counters of the attention kernel: zero before a launch, and left zero by it.
+    unsigned int* attn_job_counters(size_t n, cudaStream_t st) {
+        if (n > counters_zeroed_) {
+            attn_counters_.reserve(n * sizeof(unsigned int), st);
+            TQ_CUDA(cudaMemsetAsync(attn_counters_.as<void>(), 0, attn_counters_.bytes(), st));
+            counters_zeroed_ = attn_counters_.bytes() / sizeof(unsigned int);
+        }
+        return attn_counters_.as<unsigned int>();
     }
     // Device copy of the descriptor table of `layer`; uploaded only when it differs from what is there.
     const void* upload_descriptors(int layer, const void* table, size_t bytes, cudaStream_t st) {
@@ -484,12 +427,73 @@ public:
         if (h_attn_status_ && *static_cast<volatile unsigned int*>(h_attn_status_) != 0u) {
             const unsigned int code = *h_attn_status_;
             *h_attn_status_ = 0u;
+            counters_zeroed_ = 0;   // a job that was not finished left its counter behind
             throw Error("attention: a bounded wait in the kernel ran out (device status " + std::to_string(code) +
                         "); the output of that call is not valid");
         }
     }
 
 private:
+    // Bytes per vector of the reference's six arrays, in the streams' order.
+    std::array<size_t, 6> array_bytes() const {
+        const size_t w = static_cast<size_t>(words_per_head()) * 4, s = static_cast<size_t>(qjl_words_per_head()) * 4;
+        return {w, w, 4, 4, s, 4};
+    }
+    // Device memory for the six arrays of n vectors: {key words, value words, key norms, value norms, sign words, sign norms}.
+    tq::KvArrays stage_arrays(DeviceBuffer& buf, size_t n, void* (&at)[6]) const {
+        const std::array<size_t, 6> per = array_bytes();
+        size_t total = 0;
+        for (size_t b : per) total += (n * b + 255) / 256 * 256;
+        buf.reserve(total);
+        unsigned char* p = buf.as<unsigned char>();
+        for (int i = 0; i < 6; ++i) {
+            at[i] = p;
+            p += (n * per[i] + 255) / 256 * 256;
+        }
+        return tq::KvArrays{static_cast<uint32_t*>(at[0]), static_cast<uint32_t*>(at[1]), static_cast<float*>(at[2]),
+                            static_cast<float*>(at[3]), static_cast<uint32_t*>(at[4]), static_cast<float*>(at[5])};
+    }
+    // The reference's arrays of tokens [start, start + tokens) to dst[i] (host or device; NULL: not wanted).  The device
+    // is idle when this is called, and when it returns.
+    void copy_arrays(const LayerKVStorage& L, int start, int tokens, void* const (&dst)[6]) const {
+        const size_t n = static_cast<size_t>(tokens) * heads_;
+        if (n == 0) return;
+        DeviceBuffer buf;
+        void* at[6];
+        const tq::KvArrays arrays = stage_arrays(buf, n, at);
+        tq::launch_kv_unpack(L.slab.as<unsigned char>(), start, tokens, heads_, dim_, arrays, nullptr);
+        const std::array<size_t, 6> per = array_bytes();
+        for (int i = 0; i < 6; ++i)
+            if (dst[i]) TQ_CUDA(cudaMemcpy(dst[i], at[i], n * per[i], cudaMemcpyDefault));
+        TQ_CUDA(cudaDeviceSynchronize());
+        buf.set_idle();
+    }
+    // ... to a stream in host memory, each array behind its length.
+    void put_arrays(const LayerKVStorage& L, int start, int tokens, uint8_t* out, size_t& pos) const {
+        const std::array<size_t, 6> per = array_bytes();
+        void* dst[6];
+        for (int i = 0; i < 6; ++i) {
+            const uint32_t bytes = static_cast<uint32_t>(static_cast<size_t>(tokens) * heads_ * per[i]);
+            std::memcpy(out + pos, &bytes, 4);
+            dst[i] = out + pos + 4;
+            pos += 4 + bytes;
+        }
+        copy_arrays(L, start, tokens, dst);
+    }
+    // The other way: host arrays into tokens [start, start + tokens) of the (large enough) storage.
+    void load_arrays(LayerKVStorage& L, int start, int tokens, const uint8_t* const (&src)[6]) const {
+        const size_t n = static_cast<size_t>(tokens) * heads_;
+        if (n == 0) return;
+        DeviceBuffer buf;
+        void* at[6];
+        const tq::KvArrays arrays = stage_arrays(buf, n, at);
+        const std::array<size_t, 6> per = array_bytes();
+        for (int i = 0; i < 6; ++i) TQ_CUDA(cudaMemcpy(at[i], src[i], n * per[i], cudaMemcpyHostToDevice));
+        tq::launch_kv_pack(L.slab.as<unsigned char>(), start, tokens, heads_, dim_, arrays, nullptr);
+        TQ_CUDA(cudaDeviceSynchronize());
+        buf.set_idle();
+    }
+
     // Grow a layer's buffers to hold `tokens` tokens (capacity doubles; old contents kept).
     void reserve(LayerKVStorage& L, int tokens, cudaStream_t st) {
         if (tokens <= L.capacity) return;
@@ -499,29 +503,13 @@ private:
     void reserve_exact(LayerKVStorage& L, int cap, cudaStream_t st, bool on_stream) {
         // whole 16-token tiles: the attention kernel fetches the cache a tile at a time
         cap = (cap + 15) / 16 * 16;
-        const int wph = words_per_head(), qph = qjl_words_per_head();
         DeviceBuffer slab;
         slab.owned_by(&use_);
-        const size_t bytes = tq::KvSlab::bytes(cap, heads_, wph, qph);
+        const size_t bytes = tq::kv_layer_bytes(cap, heads_, dim_);
         if (on_stream) slab.reserve(bytes, st);
         else slab.reserve(bytes);
-        const tq::AttnView v = tq::attn_view(tq::AttnSeq{slab.as<unsigned char>(), 0, 0, cap, 0}, heads_, wph, qph);
-        const size_t old_n = static_cast<size_t>(L.num_tokens) * heads_;
-        auto move = [&](const void* to, const void* from, size_t words_per_vec) {
-            if (old_n) TQ_CUDA(cudaMemcpyAsync(const_cast<void*>(to), from, old_n * words_per_vec * 4, cudaMemcpyDeviceToDevice, st));
-        };
-        move(v.k_words, L.k_words, wph);
-        move(v.v_words, L.v_words, wph);
-        move(v.k_norms, L.k_norms, 1);
-        move(v.v_norms, L.v_norms, 1);
-        move(v.qjl_words, L.qjl_words, qph);
-        move(v.qjl_norms, L.qjl_norms, 1);
-        L.k_words = const_cast<uint32_t*>(v.k_words);
-        L.v_words = const_cast<uint32_t*>(v.v_words);
-        L.k_norms = const_cast<float*>(v.k_norms);
-        L.v_norms = const_cast<float*>(v.v_norms);
-        L.qjl_words = const_cast<uint32_t*>(v.qjl_words);
-        L.qjl_norms = const_cast<float*>(v.qjl_norms);
+        const size_t used = tq::kv_layer_bytes((L.num_tokens + 15) / 16 * 16, heads_, dim_);   // whole tiles: one contiguous piece
+        if (used) TQ_CUDA(cudaMemcpyAsync(slab.as<void>(), L.slab.as<void>(), used, cudaMemcpyDeviceToDevice, st));
         L.slab = std::move(slab);   // the old storage goes back once the copies out of it have ended
         L.capacity = cap;
     }
@@ -532,12 +520,12 @@ private:
     tq::StreamUse use_;
     std::vector<LayerKVStorage> layers_;
     DeviceBuffer stage_k_, stage_v_;
-    DeviceBuffer attn_scratch_, attn_q_, attn_out_, attn_lse_;
+    DeviceBuffer attn_scratch_, attn_q_, attn_out_, attn_lse_, attn_counters_;
+    size_t counters_zeroed_ = 0;   // words of attn_counters_ known to be zero between launches
     unsigned int* h_attn_status_ = nullptr;
     unsigned int* d_attn_status_ = nullptr;         // its address for kernels
     std::vector<DeviceBuffer> desc_dev_;            // per layer: the descriptor table of the last attention call
     std::vector<std::vector<uint8_t>> desc_host_;   // ... and its host copy, to tell whether an upload is needed
-    int attention_kernel_ = 0;
 };
 
 // Attention of one query position per sequence over [start, end) of each cache.
@@ -558,18 +546,15 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
     std::vector<tq::AttnSeq> many;   // more sequences than travel as parameters
     if (n_seqs > tq::kAttnInlineSeqs) many.resize(static_cast<size_t>(n_seqs));
     tq::AttnSeq* const desc = many.empty() ? seqs.inl : many.data();
-    int max_tok = 0;
     for (int i = 0; i < n_seqs; ++i) {
         TQ_REQUIRE(caches[i] && caches[i]->num_heads() == heads && caches[i]->head_dim() == dim &&
                        caches[i]->device() == c0->device(),
                    "attention: caches of one call must share shape and device");
         desc[i] = caches[i]->describe(layer, starts[i], ends[i]);
         caches[i]->note_stream(st);
-        max_tok = std::max(max_tok, ends[i] - starts[i]);
     }
-    const tq::AttnPlan plan = tq::attn_make_plan(n_seqs, q_heads, heads, dim, max_tok, tq::sm_count(c0->device()), c0->attention_kernel());
-    const int n_splits = plan.n_splits;
-
+    const int sms = tq::sm_count(c0->device());
+    const long tiles = tq::attn_number_tiles(desc, n_seqs);
     // A table goes up only when it differs from the one already on the device: a call that repeats the
     // previous ranges enqueues kernels only (and can then be captured in a graph).
     if (!many.empty())
@@ -595,11 +580,12 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
         c0->attn_lse().reserve(n_lse * sizeof(float), st);
         d_lse = c0->attn_lse().as<float>();
     }
-    c0->attn_scratch().reserve(tq::attn_scratch_bytes(n_seqs, q_heads, dim, n_splits), st);
-    tq::launch_kv_attention(seqs, n_seqs, d_q, q_dtype == TQ_F16, q_heads, heads, dim, plan,
+    c0->attn_scratch().reserve(tq::attn_scratch_bytes(dim, sms), st);
+    unsigned int* const counters = c0->attn_job_counters(tq::attn_counters(n_seqs, q_heads, heads), st);
+    tq::launch_kv_attention(seqs, n_seqs, tiles, d_q, q_dtype == TQ_F16, q_heads, heads, dim,
                             tq::kv_layer_seed(static_cast<uint32_t>(layer), 1), tq::kv_layer_seed(static_cast<uint32_t>(layer), 2),
-                            tq::kv_layer_seed(static_cast<uint32_t>(layer), 3), use_qjl, c0->attn_scratch().as<void>(), d_out, d_lse,
-                            c0->attn_status_device(), st);
+                            tq::kv_layer_seed(static_cast<uint32_t>(layer), 3), use_qjl, c0->attn_scratch().as<void>(), counters, d_out, d_lse,
+                            c0->attn_status_device(), sms, st);
     const bool lse_host = lse_out != nullptr && d_lse != lse_out;
     if (lse_host) TQ_CUDA(cudaMemcpyAsync(lse_out, d_lse, n_lse * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (!out_dev) TQ_CUDA(cudaMemcpyAsync(out, d_out, n_q * sizeof(__half), cudaMemcpyDeviceToHost, st));

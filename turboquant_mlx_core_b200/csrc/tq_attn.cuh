@@ -1,4 +1,4 @@
-// Shared by the decode-attention kernels (tq_kv_kernels.cu, tq_attn_tc.cu).
+// The compressed cache's storage and the kernels on it (tq_kv_kernels.cu, tq_attention.cu), and the fp16 decode window.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -8,49 +8,78 @@
 
 namespace tq {
 
-// A layer's storage is ONE allocation that holds its six token-major arrays (see tq_kv_kernels.cu) one after the
-// other, each sized for `cap` tokens; cap is a multiple of 16, so every array starts on a 64-byte boundary.
-struct KvSlab {
-    const unsigned char* base;
-    int cap;
-    __host__ __device__ static size_t bytes(int cap, int heads, int wph, int qph) {
-        return static_cast<size_t>(cap) * heads * (2 * wph + qph + 3) * 4;
-    }
+// ---- storage of the compressed cache -----------------------------------------------------------------
+// A layer's storage is one allocation of blocks [16-token tile][KV head].  A block holds the 16 tokens' records of one
+// head in the order the attention kernel consumes them, so a tile is ONE contiguous bulk copy whatever the head count
+// (the reference's token-major arrays took six copies per tile, or one per token and array beyond four heads):
+//   keys    16 tokens x D/2 bytes: dim 8 w + i in nibble i of word w, bits 0-2 the code, bit 3 the residual's sign bit
+//   values  D = 128: per token and quarter q of the dims three words of nibbles for the quarter's first 24 dims; the
+//           codes of its last eight dims are spread over the nibbles' spare bits (bit k of dim 24 + i in bit 3 of nibble i
+//           of word k).  Words 0 and 1 of all (token, quarter) first, then word 2.   48 bytes per token
+//           other D: nibbles like the keys, bit 3 zero
+//   norms   16 key norms, 16 value norms, 16 residual norms (fp32)
+// D = 128: 124 bytes per token and head (the reference's words of ten codes: 132), every byte of a nibble word a pair
+// of codes that one byte permutation turns into a table address.  Snapshots, deltas and exports convert to and from the
+// reference's arrays (tq_kv_kernels.cu).
+constexpr int kKvTile = 16;
+template <int D>
+struct KvBlock {
+    static constexpr int kKeyBytes = kKvTile * D / 2;
+    static constexpr int kValueBytes = D == 128 ? kKvTile * 48 : kKvTile * D / 2;
+    static constexpr int kValueOff = kKeyBytes, kNormOff = kKeyBytes + kValueBytes;
+    static constexpr int kBytes = kNormOff + 3 * kKvTile * 4;
+    static_assert(kBytes % 16 == 0, "a block is a bulk copy");
 };
+__host__ __device__ constexpr size_t kv_block_bytes(int dim) {
+    return static_cast<size_t>(kKvTile) * dim / 2 + (dim == 128 ? kKvTile * 48 : kKvTile * dim / 2) + 3 * kKvTile * 4;
+}
+// Bytes of a layer's storage for `cap` tokens (a multiple of 16).
+inline size_t kv_layer_bytes(int cap, int heads, int dim) { return static_cast<size_t>(cap / kKvTile) * heads * kv_block_bytes(dim); }
 
-// One sequence of an attention call: the layer's storage and the token range [start, end) the query attends to.
-struct AttnSeq {
-    const unsigned char* base;
-    int start, end, cap, pad;
-};
-// ... with the arrays' addresses spelled out.
-struct AttnView {
-    const uint32_t* k_words;
-    const uint32_t* v_words;
-    const uint32_t* qjl_words;
-    const float* k_norms;
-    const float* v_norms;
-    const float* qjl_norms;
-    int start, end;
-};
-__host__ __device__ __forceinline__ AttnView attn_view(const AttnSeq& s, int heads, int wph, int qph) {
-    const size_t n = static_cast<size_t>(s.cap) * heads;
-    const uint32_t* const w = reinterpret_cast<const uint32_t*>(s.base);
-    AttnView v;
-    v.k_words = w;
-    v.v_words = w + n * wph;
-    v.qjl_words = w + n * 2 * wph;
-    v.k_norms = reinterpret_cast<const float*>(w + n * (2 * wph + qph));
-    v.v_norms = v.k_norms + n;
-    v.qjl_norms = v.k_norms + 2 * n;
-    v.start = s.start;
-    v.end = s.end;
-    return v;
+// The value words of (token slot t of the tile, quarter q) of a D = 128 block.
+__device__ __forceinline__ uint32_t* kv_value01(unsigned char* block, int t, int q) {
+    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff) + (t * 4 + q) * 2;
+}
+__device__ __forceinline__ uint32_t* kv_value2(unsigned char* block, int t, int q) {
+    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff + 512) + t * 4 + q;
+}
+// The codes of a quarter's last eight dims, out of the spare bits of its three words.
+__device__ __forceinline__ uint32_t kv_value_spare(uint32_t w0, uint32_t w1, uint32_t w2) {
+    return ((w0 >> 3) & 0x11111111u) | ((w1 >> 2) & 0x22222222u) | ((w2 >> 1) & 0x44444444u);
 }
 
-// The sequences of one attention call.  A decode step moves every range by a token, so the descriptors of up to
-// kAttnInlineSeqs sequences travel as kernel parameters (24 bytes each): a table in device memory cost an upload per
-// call, and the copy between two kernels a gap in the stream.  Larger batches use the table.
+// One append: `tokens` tokens of a layer, from token `first` on, written to the storage at `base`.
+struct KvSegment {
+    unsigned char* base;
+    int first;
+};
+constexpr int kKvMaxSegments = 32;
+void launch_kv_encode(const void* keys, const void* values, bool is_f16, int tokens_per_seg, int heads, int dim, uint32_t k_seed,
+                      uint32_t v_seed, uint32_t qjl_seed, const KvSegment* segs, int n_segs, cudaStream_t stream);
+// fp16 [tokens, heads, dim] of tokens [start, start + tokens).
+void launch_kv_decode_f16(const unsigned char* base, int start, int tokens, int heads, int dim, bool values, uint32_t wht_seed,
+                          __half* out, cudaStream_t stream);
+// The reference's token-major arrays (src/kv_cache.cpp:119-128; ceil(D/10) words of ten codes, norms, sign words, sign
+// norms) of tokens [start, start + tokens), out of the storage or into it.
+struct KvArrays {
+    uint32_t *k_words, *v_words;
+    float *k_norms, *v_norms;
+    uint32_t* qjl_words;
+    float* qjl_norms;
+};
+void launch_kv_unpack(const unsigned char* base, int start, int tokens, int heads, int dim, const KvArrays& out, cudaStream_t stream);
+void launch_kv_pack(unsigned char* base, int start, int tokens, int heads, int dim, const KvArrays& in, cudaStream_t stream);
+
+// ---- decode attention over the compressed cache (tq_attention.cu) --------------------------------------
+// One sequence of a call: the layer's storage and the token range [start, end) the query attends to.  tile0 counts the
+// tiles of the sequences before it.
+struct AttnSeq {
+    const unsigned char* base;
+    int start, end, tile0, pad;
+};
+// A decode step moves every range by a token, so the descriptors of up to kAttnInlineSeqs sequences travel as kernel
+// parameters (24 bytes each): a table in device memory cost an upload per call, and the copy between two kernels a gap
+// in the stream.  Larger batches use the table.
 constexpr int kAttnInlineSeqs = 32;
 struct AttnSeqs {
     const AttnSeq* table;              // nullptr: the descriptors are in `inl`
@@ -58,19 +87,20 @@ struct AttnSeqs {
 };
 __device__ __forceinline__ AttnSeq attn_seq(const AttnSeqs& s, int i) { return s.table != nullptr ? s.table[i] : s.inl[i]; }
 
-// The pair tables hold kAttnCentroidScale * centroid: with this factor all four centroid
+// The pair table holds kAttnCentroidScale * centroid: with this factor all four centroid
 // magnitudes round to fp16 with a relative error below 1.4e-5 (unscaled: up to 3e-4, which the
 // softmax amplifies); the factor is divided out of the key and value norms.
 constexpr float kAttnCentroidScale = 1.1979075f;
 // Lazy softmax reference: it only moves when a score exceeds it by more than this.
 constexpr float kAttnSoftmaxSlack = 2.0f;
 
-// Tensor-memory kernel (tq_attn_tc.cu): head_dim 128, four KV heads, up to 8 query heads per KV head
-// and CTA.  Partials in the layout attn_combine_kernel reads.
-void launch_attn_tc(const AttnSeqs& seqs, int n_seqs, const void* q, bool q_is_f16, int q_heads, int kv_heads, int n_splits,
-                    uint32_t k_seed, uint32_t qjl_seed, bool use_qjl, float inv_sqrt, float inv_scale_d, float attn_scale,
-                    float gamma, float* part_acc, float* part_ml, unsigned int* status, cudaStream_t stream);
-constexpr int kAttnTcCtasPerSm = 2;
+// Sets the descriptors' tile0 and returns the tiles of all sequences.
+long attn_number_tiles(AttnSeq* seqs, int n_seqs);
+size_t attn_scratch_bytes(int dim, int sm_count);
+size_t attn_counters(int n_seqs, int q_heads, int kv_heads);   // zeroed words; every launch leaves them zero
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
+                         uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl, void* scratch, unsigned int* counters,
+                         __half* out, float* lse, unsigned int* status, int sm_count, cudaStream_t stream);
 
 // fp16 decode window (tq_attn_dense.cu): ring writes / reads and scaled-dot-product attention over a
 // contiguous run of ring slots.  `row` = heads * head_dim.

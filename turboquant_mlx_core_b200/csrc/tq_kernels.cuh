@@ -162,31 +162,6 @@ void launch_qjl_compress(const float* d_residual, int num_tokens, int num_heads,
 void launch_qjl_dot_correction(const uint32_t* d_signs_q, const uint32_t* d_signs_k, const float* d_norms_k, int num_queries, int num_keys,
                                int num_heads, int head_idx, int proj_dim, float* d_corrections, cudaStream_t stream);
 
-// tq_kv_kernels.cu — KV-cache encoder with several destinations: the n_vec input vectors
-// ([n_vec, head_dim], contiguous) are cut into segments of vec_per_seg vectors and segment s is
-// written to segs[s] (at most 32 segments per launch).  A decode step that appends one token to
-// many sequences' caches is one launch for the keys and one for the values.
-// How one decode-attention call runs (attn_make_plan in tq_kv_kernels.cu).
-struct AttnPlan {
-    int n_splits;     // context splits per sequence
-    int pipe_heads;   // KV heads per CTA of the bulk-copy pipeline kernel; 0: load-based kernels
-    int tensor_memory;   // 1: the tensor-memory kernel (tq_attn_tc.cu) instead of either
-};
-
-struct KvEncodeSegment {
-    uint32_t* words;
-    float* norms;
-    uint32_t* qjl_words;  // may be NULL when with_qjl is false
-    float* qjl_norms;
-};
-void launch_kv_encode_segments(const void* x, bool x_is_f16, long n_vec, long vec_per_seg, int head_dim, uint32_t wht_seed,
-                               uint32_t qjl_seed, bool with_qjl, const KvEncodeSegment* segs, int n_segs,
-                               cudaStream_t stream);
-// keys (with residual bits) and values of the same tokens: one launch when there are fewer than 512 vectors
-void launch_kv_encode_pair_segments(const void* k, const void* v, bool x_is_f16, long n_vec, long vec_per_seg, int head_dim,
-                                    uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, const KvEncodeSegment* ksegs,
-                                    const KvEncodeSegment* vsegs, int n_segs, cudaStream_t stream);
-
 // tq_peer.cu — exchange between ranks over peer-mapped memory (plain stores, flags with epochs).
 void launch_exchange_broadcast(const void* src, void* const* dst, int n_dst, int rows, long row_bytes, long src_stride,
                                long dst_stride, unsigned int* const* signal, int n_signal, int slot, unsigned int* done,
