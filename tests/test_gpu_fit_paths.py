@@ -1,0 +1,30 @@
+"""The two ways of the codebook fit: bucketed samples, and passes over all samples for data that repeats itself.  Centroids
+within the rounding of a mean (one part in 2^24, taken a few times over: the tolerance of tests/test_codebook_fit.py)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 255, 8193, 65537, 1_000_003])
+@pytest.mark.parametrize("kind", ["scaled", "outliers", "one value", "few values", "zeros"])
+def test_fit_against_the_checker(tq, oracle, n, kind):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n)
+    if kind == "scaled":                # far from the codebook it starts from
+        x = x * 1e-3 + 5e-4
+    elif kind == "outliers":            # the sums' unit follows the largest magnitude
+        x[:: max(1, n // 7)] *= 1e6
+    elif kind == "one value":
+        x[:] = 0.37
+    elif kind == "few values":          # more of each than a bucket may hold (from 65537 on)
+        x = np.array([-1.2, 0.1, 0.9])[rng.integers(0, 3, n)]
+    else:
+        x[: n // 2] = 0.0
+    x = x.astype(np.float32)
+    want, _ = oracle.fit_codebook(x, 4, 20)
+    got = tq.generate_codebook_from_data(x, 4, 20)
+    tol = 3e-6 * np.abs(want) + 3e-7
+    if kind == "outliers":
+        tol = tol + 3e-6 * np.abs(x).max() / 1e6      # both sides round sums that an outlier dominates
+    assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()

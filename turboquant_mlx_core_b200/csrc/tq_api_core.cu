@@ -207,7 +207,10 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
         TQ_REQUIRE(!need_residual || (cr0 && residual_centroids), "tq_fit_layer_codebooks: bad residual bit width or NULL output");
         auto st = static_cast<cudaStream_t>(stream);
         const size_t n = static_cast<size_t>(out_features) * in_features;
-        DeviceBuffer w_stage, norms(static_cast<size_t>(out_features) * 4), scaled(n * 4), resid(need_residual ? n * 4 : 0);
+        DeviceBuffer w_stage, norms, scaled, resid;
+        norms.reserve(static_cast<size_t>(out_features) * 4, st);
+        scaled.reserve(n * 4, st);
+        if (need_residual) resid.reserve(n * 4, st);
         const float* d_w = device_view(weight, n, w_stage, st);
         uint32_t seed_p = 0, seed_r = 0;
         derive_seeds(d_w, n, &seed_p, &seed_r, st);
@@ -220,6 +223,7 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
             launch_codebook_fit(resid.as<float>(), static_cast<long>(n), residual_bits, iterations, cr0, residual_centroids,
                                 residual_boundaries, st);
         TQ_CUDA(cudaStreamSynchronize(st));
+        for (DeviceBuffer* b : {&w_stage, &norms, &scaled, &resid}) b->set_idle();
         return 0;
     });
 }

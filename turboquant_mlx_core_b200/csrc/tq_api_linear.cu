@@ -589,7 +589,9 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         std::vector<float> cp(n_primary), cr(n_residual);
         TQ_CUDA(cudaMemcpy(cp.data(), primary_centroids, sizeof(float) * n_primary, cudaMemcpyDefault));
         TQ_CUDA(cudaMemcpy(cr.data(), residual_centroids, sizeof(float) * n_residual, cudaMemcpyDefault));
-        DeviceBuffer w_stage, recon(n * sizeof(float)), orig(static_cast<size_t>(out_features) * sizeof(float) + 4);
+        DeviceBuffer w_stage, recon, orig;
+        recon.reserve(n * sizeof(float), st);
+        orig.reserve(static_cast<size_t>(out_features) * sizeof(float) + 4, st);
         const float* d_w = device_view(weight, n, w_stage, st);
         const bool pp_dev = is_device_pointer(packed_primary), pr_dev = is_device_pointer(packed_residual),
                    nm_dev = is_device_pointer(norms);
@@ -597,9 +599,9 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         uint8_t* d_pp = packed_primary;
         uint8_t* d_pr = packed_residual;
         float* d_nm = norms;
-        if (!pp_dev) { pp_stage.reserve(pp_bytes + 4); d_pp = pp_stage.as<uint8_t>(); }
-        if (!pr_dev) { pr_stage.reserve(pr_bytes + 4); d_pr = pr_stage.as<uint8_t>(); }
-        if (!nm_dev) { nm_stage.reserve(static_cast<size_t>(out_features) * 4 + 4); d_nm = nm_stage.as<float>(); }
+        if (!pp_dev) { pp_stage.reserve(pp_bytes + 4, st); d_pp = pp_stage.as<uint8_t>(); }
+        if (!pr_dev) { pr_stage.reserve(pr_bytes + 4, st); d_pr = pr_stage.as<uint8_t>(); }
+        if (!nm_dev) { nm_stage.reserve(static_cast<size_t>(out_features) * 4 + 4, st); d_nm = nm_stage.as<float>(); }
         uint32_t seed_p = 0, seed_r = 0;
         if (given_seeds != nullptr) {
             seed_p = given_seeds[0];

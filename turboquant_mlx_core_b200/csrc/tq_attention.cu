@@ -7,22 +7,25 @@
 //   S^T [16 tokens x 8 heads]  = K [16 x D] . Qrot^T           centroids
 //   S2^T                        = Sgn [16 x D] . Qsgn^T         the residual's signs (use_qjl)
 //   O^T [D dims x 8 heads]     += V^T [D x 16] . P^T
-// A storage byte holds the codes of two neighbouring dims (tq_attn.cuh).  One byte permutation makes it a table address
-// (256 entries of 256 bytes at the fixed window address 0x10000, entry e at 0x10000 + 256 e, a private copy per lane, so
-// lookups meet no bank conflict), and the table's word is the fp16 pair the fragment needs: two instructions per pair,
-// where words of ten 3-bit codes took a shift, a mask and a load.  The order in which a thread takes its dims is the same
-// on both operands and undone at the end.  Value fragments are transposed in registers (movmatrix).
+// A storage byte holds a pair of codes (tq_attn.cuh): two dims of a key, or one dim of two tokens' values, as the two
+// products want them.  One dot-product instruction makes it the address of a table entry (256 entries of 128 bytes, a
+// private copy per lane, so lookups meet no bank conflict), and the entry is the fp16 pair the fragment needs: two
+// instructions per pair, where words of ten 3-bit codes took a shift, a mask and a load, and values a transposition
+// (movmatrix) on top, which the shared-memory pipe carries.  The order in which a thread takes its dims is the same on both
+// operands and undone at the end.
 //
 // Work split.  A job is (sequence, KV head, group of 8 query heads); its tiles are consecutive in a flat numbering of all
-// tiles of the call, which is cut into equal ranges, one per CTA - one CTA per SM, whatever the mix of lengths.  A CTA
-// walks its range job by job: its 16 warps take the job's tiles in turn, each through a ring of its own (one
-// cp.async.bulk per tile, no synchronisation between warps), and merge their (max, sum, accumulator) in shared memory.
-// A job that lies in one range is finished there; the parts of one that several ranges share go to scratch, and the CTA
-// that arrives last (a counter per job) adds them in range order - the result does not depend on timing - un-rotates
-// and writes.  One launch, no combine kernel.
+// tiles of the call, which is cut into equal ranges, two per SM, whatever the mix of lengths.  A CTA is two teams of
+// warps that share the table and nothing else, so that one team computes while the other is between jobs (with one team
+// of 16 warps 27 of 92 us went into the jobs' ends).  A team walks its range job by job: its warps take the job's tiles in
+// turn, each through a ring of its own (one cp.async.bulk per tile, no synchronisation between warps), and merge their
+// (max, sum, accumulator) in shared memory.  A job that lies in one range is finished there; the parts of one that several
+// ranges share go to scratch, and the team that arrives last (a counter per job) adds them in range order - the result
+// does not depend on timing - un-rotates and writes.  One launch, no combine kernel.  A job's start and end cost a team about
+// as much as `pad` tiles, so the flat numbering gives every job that many empty tiles in front: a range with two jobs gets
+// fewer tiles than one with a single one.
 //
-// Bound: issue slots and the shared-memory pipe (about 330 warp instructions and 90 shared wavefronts per tile) ahead of
-// DRAM.
+// The next job's first tiles are requested before the merge of the current one, which has shared memory of its own.
 #include <cmath>
 
 #include "tq_attn.cuh"
@@ -35,29 +38,35 @@ namespace {
 
 __constant__ float kC3[8] = {-2.152176f, -1.344318f, -0.756130f, -0.245379f, 0.245379f, 0.756130f, 1.344318f, 2.152176f};
 
-constexpr uint32_t kTabAddr = 0x10000u, kTabBytes = 0x10000u;   // window address and size of the pair table
-constexpr uint32_t kLowBase = 0x800u;                           // shared memory below is the runtime's and the statics'
+constexpr uint32_t kTabBytes = 256 * 128;                       // the pair table, at the start of shared memory
+constexpr float kNone = -1e30f;
 constexpr int kGroup = 8;                                       // query heads of a job
 constexpr unsigned long long kWaitLimitNs = 200ull * 1000 * 1000;
 
 template <int D>
 struct AttnCfg {
-    static constexpr int kWarps = D == 256 ? 8 : 16;            // 256 dims: 64 accumulator registers
+    static constexpr int kWarps = D == 256 ? 8 : 16;            // 256 dims: 64 accumulator registers, and one team
     static constexpr int kThreads = 32 * kWarps;
-    static constexpr int kStages = D == 256 ? 3 : 4;
-    static constexpr int kRing = kStages * KvBlock<D>::kBytes;  // bytes of a warp's ring
-    static constexpr int kLowRings = (kTabAddr - kLowBase) / kRing < static_cast<uint32_t>(kWarps) ? (kTabAddr - kLowBase) / kRing : kWarps;
+    static constexpr int kStages = 2;                           // of two tiles each: one wait and one refill per two tiles
+    static constexpr int kStageBytes = 2 * KvBlock<D>::kBytes;
+    static constexpr int kRing = kStages * kStageBytes;         // bytes of a warp's ring
+    static constexpr int kAccRegs = D / 4;                      // accumulators of a thread
     static constexpr int kAccStride = D + 4;                    // floats per head of a published accumulator
-    static constexpr uint32_t kHighBase = kTabAddr + kTabBytes;
+    static constexpr int kTeams = D == 256 ? 1 : 2, kTeam = kWarps / kTeams;   // teams, warps of a team
+    static constexpr int kHalf = kTeam / 2;                     // the upper half of a team hands over to the lower one
+    static constexpr int kPubBytes = 32 * (kAccRegs + 4) * 4;   // registers of a warp, or [8 heads][kAccStride]
     static constexpr int kQStride = D + 8;                      // halves per rotated query
-    static constexpr uint32_t kOffQ = kHighBase + (kWarps - kLowRings) * kRing;
-    static constexpr uint32_t kOffOut = kOffQ + kGroup * kQStride * 2;
-    static constexpr uint32_t kOffMl = kOffOut + kGroup * kAccStride * 4;      // [2][warps][8]
-    static constexpr uint32_t kEnd = kOffMl + 2 * kWarps * kGroup * 4;
+    static constexpr uint32_t kOffQ = kTabBytes + kWarps * kRing;                        // rotated queries
+    static constexpr uint32_t kOffQs = kOffQ + kGroup * kQStride * 2;                   // ... with the residual's signs
+    static constexpr uint32_t kOffPub = kOffQs + kGroup * kQStride * 2;
+    static constexpr uint32_t kOffOut = kOffPub + kHalf * kPubBytes;
+    static constexpr uint32_t kOffMl = kOffOut + kGroup * kAccStride * 4;               // [2][kHalf][8], then flags and the job
+    static constexpr uint32_t kTeamBytes = kOffMl + 2 * kHalf * kGroup * 4 + 80 - kOffQ;   // of one team, from kOffQ on
+    static constexpr uint32_t kEnd = kOffQ + kTeams * kTeamBytes;
     static constexpr int kPartFloats = kGroup * D + 2 * kGroup;                // a job part in scratch: accumulators, then (max, sum)
-    static_assert(kRing >= kGroup * kAccStride * 4, "a warp publishes its accumulator through its ring");
-    static_assert(kOffQ % 16 == 0 && kOffOut % 16 == 0, "alignment");
-    static_assert(kEnd <= 227u * 1024u + 1024u, "shared memory of an SM");
+    static_assert(kPubBytes >= kGroup * kAccStride * 4, "a warp's accumulator in head order fits its place");
+    static_assert(kOffQ % 16 == 0 && kOffPub % 16 == 0 && kOffOut % 16 == 0, "alignment");
+    static_assert(kEnd + 1024u <= 227u * 1024u, "shared memory of an SM");
 };
 
 struct AttnArgs {
@@ -65,10 +74,10 @@ struct AttnArgs {
     const void* q;
     __half* out;
     float* lse;
-    float* part;               // [CTA][2][kPartFloats]
+    float* part;               // [range][2][kPartFloats]
     unsigned int* counters;    // [job]
     unsigned int* status;
-    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units;
+    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units, ranges, pad;
     uint32_t k_seed, v_seed, qjl_seed;
     float inv_sqrt, inv_scale, score_scale, qscale;
 };
@@ -97,38 +106,42 @@ __device__ __forceinline__ unsigned long long timer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    return done != 0;
+}
 // False when the phase did not complete in time.
+__device__ __noinline__ bool bar_wait_long(uint32_t bar, uint32_t parity) {
+    const unsigned long long t0 = timer_ns();
+    for (uint32_t spin = 1; !bar_try(bar, parity); ++spin)
+        if ((spin & 63) == 0 && timer_ns() - t0 > kWaitLimitNs) return false;
+    return true;
+}
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    unsigned long long t0 = 0;
-    for (uint32_t spin = 0;; ++spin) {
-        uint32_t done;
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                     : "=r"(done)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (done) return true;
-        if (spin == 64) t0 = timer_ns();
-        if (spin > 64 && (spin & 63) == 0 && timer_ns() - t0 > kWaitLimitNs) return false;
-    }
+    return bar_try(bar, parity) || bar_try(bar, parity) || bar_wait_long(bar, parity);
 }
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
                  "r"(bar)
                  : "memory");
 }
-// The table word of byte BYTE of `word`: address = lane constant with its second byte replaced (byte 1 the entry,
-// byte 0 the lane's copy, bytes 2 and 3 the table's base).
+// Address of the table word of byte BYTE of `word`: byte * 128 + the address of this lane's copy of entry 0, one
+// dot-product instruction.  (A byte permutation would do with entries of 256 bytes, but the logic pipe it runs on also
+// carries the sign and mask operations and issues every other cycle.)
 template <int BYTE>
-__device__ __forceinline__ uint32_t pair_addr(uint32_t word, uint32_t lane_const) {
-    return __byte_perm(word, lane_const, 0x7604u | (static_cast<uint32_t>(BYTE) << 4));
+__device__ __forceinline__ uint32_t pair_addr(uint32_t word, uint32_t lane_base) {
+    return __dp4a(word, 128u << (8 * BYTE), lane_base);
 }
 __device__ __forceinline__ uint32_t table_load(uint32_t addr) {
     uint32_t v;
     asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-// Words of one token of a nibble array: word w of thread q's quarter.
+// W consecutive words.
 template <int W>
 __device__ __forceinline__ void load_words(uint32_t (&w)[W], uint32_t addr) {
     if constexpr (W % 4 == 0) {
@@ -151,85 +164,127 @@ template <int D, bool QJL>
 __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __grid_constant__ AttnArgs a) {
     using C = AttnCfg<D>;
     using B = KvBlock<D>;
-    constexpr int kSteps = D / 16;   // k steps of a score product = m tiles of the value product
+    constexpr int kSteps = D / 16;   // k steps of a score product, m tiles of the value product
     constexpr int W = D / 32;        // nibble words of a token that a thread takes
     extern __shared__ __align__(16) unsigned char attn_smem[];
     __shared__ __align__(8) unsigned long long s_bars[C::kWarps * C::kStages];
-    __shared__ unsigned int s_last;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lane = threadIdx.x & 31, cta_warp = threadIdx.x >> 5;
+    const int team = cta_warp / C::kTeam, warp = cta_warp - team * C::kTeam, tid = threadIdx.x - team * (C::kTeam * 32);   // in the team
     const int g = lane >> 2, q = lane & 3;
+    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(C::kTeam * 32) : "memory"); };
     const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem));
-    if (base > kLowBase) {   // layout assumption broken: refuse to run
-        if (tid == 0) raise_status(a.status, 1u);
-        return;
-    }
-    auto at = [&](uint32_t window) { return attn_smem + (window - base); };
-    const uint32_t ring = warp < C::kLowRings ? kLowBase + warp * C::kRing : C::kHighBase + (warp - C::kLowRings) * C::kRing;
-    const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(&s_bars[warp * C::kStages]));
-    __half* const s_q = reinterpret_cast<__half*>(at(C::kOffQ));
-    float* const s_out = reinterpret_cast<float*>(at(C::kOffOut));
-    float* const s_m = reinterpret_cast<float*>(at(C::kOffMl));
-    float* const s_l = s_m + C::kWarps * kGroup;
+    const uint32_t ring = base + kTabBytes + cta_warp * C::kRing;
+    const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(&s_bars[cta_warp * C::kStages]));
+    unsigned char* const mine = attn_smem + C::kOffQ + team * C::kTeamBytes;   // this team's shared memory
+    __half* const s_q = reinterpret_cast<__half*>(mine);
+    __half* const s_qs = reinterpret_cast<__half*>(mine + (C::kOffQs - C::kOffQ));
+    unsigned char* const s_pub = mine + (C::kOffPub - C::kOffQ);
+    float* const s_out = reinterpret_cast<float*>(mine + (C::kOffOut - C::kOffQ));
+    float* const s_m = reinterpret_cast<float*>(mine + (C::kOffMl - C::kOffQ));
+    float* const s_l = s_m + C::kHalf * kGroup;
+    volatile unsigned int* const s_flag = reinterpret_cast<volatile unsigned int*>(s_l + C::kHalf * kGroup);   // [0] last, [1] stop
+    // The job's fields that only its end needs, kept out of the tile loop's registers: two of them, the next job is located
+    // before the last one's end.
+    volatile int* const s_job = reinterpret_cast<volatile int*>(s_l + C::kHalf * kGroup) + 4;
+    int job_slot = 0;
 
     if (lane == 0) {
         for (int s = 0; s < C::kStages; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * s), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // The table does not depend on the kernels before this one.  Entry: [32 lanes] centroid pair, [32 lanes] sign pair.
-    for (int i = tid; i < 256 * 16; i += C::kThreads) {
-        const int e = i >> 4, part = i & 15;   // 4 copies per store
-        const uint32_t v = part < 8 ? pack_half2(kAttnCentroidScale * kC3[e & 7], kAttnCentroidScale * kC3[(e >> 4) & 7])
-                                    : ((e & 8) ? 0x3C00u : 0xBC00u) | ((e & 128) ? 0x3C000000u : 0xBC000000u);
-        *reinterpret_cast<uint4*>(at(kTabAddr + e * 256 + part * 16)) = make_uint4(v, v, v, v);
+    // The table does not depend on the kernels before this one.  (Bits 6 and 7 of a byte are not part of its codes.)
+    for (int i = threadIdx.x; i < 256 * 8; i += C::kThreads) {
+        const int e = i >> 3;
+        const uint32_t v = pack_half2(kAttnCentroidScale * kC3[e & 7], kAttnCentroidScale * kC3[(e >> 3) & 7]);
+        *reinterpret_cast<uint4*>(attn_smem + i * 16) = make_uint4(v, v, v, v);   // 4 copies per store
     }
-    pdl_wait_release();
+    if (tid == 0) s_flag[1] = 0u;
+    __syncthreads();
 
-    const uint32_t lane_const = kTabAddr | static_cast<uint32_t>(lane * 4);
-    const int cta = static_cast<int>(blockIdx.x), n_ctas = static_cast<int>(gridDim.x);
-    const int u_end = static_cast<int>(static_cast<long>(a.units) * (cta + 1) / n_ctas);
+    const uint32_t lane_base = base + static_cast<uint32_t>(lane * 4);
+    // the first teams of all CTAs come first: few ranges spread over the SMs
+    const int range = static_cast<int>(blockIdx.x + gridDim.x * static_cast<unsigned>(team));
+    if (range >= a.ranges) {
+        pdl_wait_release();
+        return;
+    }
+    const int u_end = static_cast<int>(static_cast<long>(a.units) * (range + 1) / a.ranges);
     const int jobs_per_seq = a.kv_heads * a.gchunks, G = a.q_heads / a.kv_heads;
-    uint32_t phase = 0;      // bit s: parity of the next completion of stage s
+    const size_t tile_stride = static_cast<size_t>(a.kv_heads) * B::kBytes;
+    uint32_t phase = 0;      // parity of the completion waited for next; flips every kStages = 2 stages
     int stage = 0;
     bool ok = true;
 
-    for (int u = static_cast<int>(static_cast<long>(a.units) * cta / n_ctas); u < u_end;) {
-        // ---- which job, which of its tiles ----
+    // The job of flat tile u, and this range's tiles of it.
+    struct Segment {
+        const unsigned char* src;   // block of the segment's first tile
+        int start, end, first_token;
+        int tiles, tile0, n_tiles;  // of the job; the segment's first; its count
+        int q_row0, ng, job, mine;
+        int next_u;
+    };
+    auto locate = [&](int u) {
         int lo = 0, hi = a.n_seqs - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (attn_seq(a.seqs, mid).tile0 * jobs_per_seq <= u) lo = mid;
+            if ((attn_seq(a.seqs, mid).tile0 + mid * a.pad) * jobs_per_seq <= u) lo = mid;
             else hi = mid - 1;
         }
         const AttnSeq S = attn_seq(a.seqs, lo);
-        const int first_tile = S.start / kKvTile, tiles = (S.end + kKvTile - 1) / kKvTile - first_tile;
-        const int in_seq = u - S.tile0 * jobs_per_seq;
-        const int hg = in_seq / tiles, tile0 = in_seq - hg * tiles;
-        const int n_tiles = min(u_end - u, tiles - tile0);
-        const int kvh = hg / a.gchunks, g0 = (hg - kvh * a.gchunks) * kGroup, ng = min(kGroup, G - g0);
-        const int q_row0 = lo * a.q_heads + kvh * G + g0;
-        const int job = lo * jobs_per_seq + hg, job_u0 = u - tile0;
-        u += n_tiles;
-
-        const unsigned char* const src = S.base + (static_cast<size_t>(first_tile + tile0) * a.kv_heads + kvh) * B::kBytes;
-        const size_t tile_stride = static_cast<size_t>(a.kv_heads) * B::kBytes;
-        const int mine = n_tiles > warp ? (n_tiles - warp + C::kWarps - 1) / C::kWarps : 0;   // tiles warp, warp + kWarps, ...
-        if (lane == 0) {
-            for (int i = 0; i < min(mine, C::kStages); ++i) {
-                const int s = (stage + i) % C::kStages;
-                bulk_copy(ring + s * B::kBytes, src + static_cast<size_t>(warp + i * C::kWarps) * tile_stride, B::kBytes, bars + 8u * s);
-            }
+        Segment g;
+        const int first_tile = S.start / kKvTile;
+        g.tiles = (S.end + kKvTile - 1) / kKvTile - first_tile;
+        const int in_seq = u - (S.tile0 + lo * a.pad) * jobs_per_seq, hg = in_seq / (g.tiles + a.pad);
+        const int at = in_seq - hg * (g.tiles + a.pad);          // position in the job, its empty tiles included
+        const int skip = max(a.pad - at, 0);
+        g.tile0 = at + skip - a.pad;
+        g.n_tiles = max(min(u_end - u - skip, g.tiles - g.tile0), 0);   // 0: the range ends in the job's empty tiles
+        g.next_u = u + skip + g.n_tiles;
+        const int kvh = hg / a.gchunks, g0 = (hg - kvh * a.gchunks) * kGroup;
+        g.ng = min(kGroup, G - g0);
+        g.q_row0 = lo * a.q_heads + kvh * G + g0;
+        g.job = lo * jobs_per_seq + hg;
+        g.start = S.start;
+        g.end = S.end;
+        g.first_token = (first_tile + g.tile0) * kKvTile;
+        g.src = S.base + static_cast<size_t>(first_tile + g.tile0) * tile_stride + static_cast<size_t>(kvh) * B::kBytes;
+        if (tid == 0) {
+            volatile int* const j = s_job + 7 * job_slot;
+            j[0] = g.tiles; j[1] = g.tile0; j[2] = g.n_tiles; j[3] = g.q_row0; j[4] = g.ng; j[5] = g.job; j[6] = g.next_u;
         }
+        g.mine = g.n_tiles > warp ? (g.n_tiles - warp + C::kTeam - 1) / C::kTeam : 0;   // tiles warp, warp + kTeam, ...
+        return g;
+    };
+    // One stage: this warp's next two tiles, or its last one.  (a lane)
+    auto request = [&](uint32_t dst, const unsigned char* src, int left, uint32_t bar) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(left > 1 ? 2 * B::kBytes : B::kBytes) : "memory");
+        bulk_copy(dst, src, B::kBytes, bar);
+        if (left > 1) bulk_copy(dst + B::kBytes, src + C::kTeam * tile_stride, B::kBytes, bar);
+    };
+    auto request_first = [&](const Segment& g) {
+        for (int i = 0; i < C::kStages && 2 * i < g.mine; ++i) {
+            const int s = stage ^ i;
+            request(ring + s * C::kStageBytes, g.src + static_cast<size_t>(warp + 2 * i * C::kTeam) * tile_stride, g.mine - 2 * i, bars + 8u * s);
+        }
+    };
+
+    int u = static_cast<int>(static_cast<long>(a.units) * range / a.ranges);
+    if (a.seqs.table != nullptr) pdl_wait_release();   // the table may have been uploaded just before
+    Segment seg = locate(u);
+    if (a.seqs.table == nullptr) pdl_wait_release();
+    if (lane == 0) request_first(seg);
+    for (;;) {
         // ---- rotated queries: fp16-round, sign, butterfly, 1 / sqrt(D), fp16-round (a warp per head) ----
-        if (warp < kGroup) {
+        for (int h = warp; h < kGroup; h += C::kTeam) {
             constexpr int E = D / 32;
             float v[E];
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 const int d = lane * E + j;
                 float t = 0.f;
-                if (warp < ng) {
-                    const size_t qi = static_cast<size_t>(q_row0 + warp) * D + d;
+                if (h < seg.ng) {
+                    const size_t qi = static_cast<size_t>(seg.q_row0 + h) * D + d;
                     t = a.q_is_f16 ? __half2float(static_cast<const __half*>(a.q)[qi])
                                    : __half2float(__float2half_rn(static_cast<const float*>(a.q)[qi]));
                 }
@@ -237,114 +292,145 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             }
             warp_fwht<E>(v, lane);
 #pragma unroll
-            for (int j = 0; j < E; ++j) s_q[warp * C::kQStride + lane * E + j] = __float2half_rn(v[j] * a.inv_sqrt);
+            for (int j = 0; j < E; ++j) {
+                const __half r = __float2half_rn(v[j] * a.inv_sqrt);
+                s_q[h * C::kQStride + lane * E + j] = r;
+                if constexpr (QJL)
+                    s_qs[h * C::kQStride + lane * E + j] = __float2half_rn(v[j] * (qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>(lane * E + j)) ? a.qscale : -a.qscale));
+            }
         }
-        __syncthreads();
+        team_sync();
         // B fragments of head g.  Pair p of thread q: dims (D/4) q + 2 p and the next.  Sign pair 4 w + r: dims 8 w + r
-        // and 8 w + r + 4 of the quarter, the sign of the residual's own rotation folded in.
+        // and 8 w + r + 4 of the quarter.
         uint32_t bq[2 * kSteps], bs[QJL ? 2 * kSteps : 1];
+        float c2_init[2] = {0.f, 0.f};
         {
             const __half* const sq = s_q + g * C::kQStride + (D / 4) * q;
 #pragma unroll
             for (int p = 0; p < 2 * kSteps; ++p) bq[p] = *reinterpret_cast<const uint32_t*>(sq + 2 * p);
             if constexpr (QJL) {
+                // Pairs 0 and 2 meet {0, 2} instead of {-1, 1} (one logic op less per pair, see below): the sum of their
+                // dims over the whole head is taken off the product up front.
+                const __half* const ss = s_qs + g * C::kQStride + (D / 4) * q;
+                float even = 0.f;
 #pragma unroll
                 for (int p = 0; p < 2 * kSteps; ++p) {
-                    const int d0 = 8 * (p / 4) + p % 4, d1 = d0 + 4;
-                    const uint32_t s0 = qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>((D / 4) * q + d0)) ? 0u : 0x8000u;
-                    const uint32_t s1 = qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>((D / 4) * q + d1)) ? 0u : 0x80000000u;
-                    bs[p] = (static_cast<uint32_t>(__half_as_ushort(sq[d0])) | (static_cast<uint32_t>(__half_as_ushort(sq[d1])) << 16)) ^ (s0 | s1);
+                    const int d0 = 8 * (p / 4) + p % 4;
+                    bs[p] = static_cast<uint32_t>(__half_as_ushort(ss[d0])) | (static_cast<uint32_t>(__half_as_ushort(ss[d0 + 4])) << 16);
+                    if ((p & 1) == 0) even += __half2float(ss[d0]) + __half2float(ss[d0 + 4]);
                 }
+                even += __shfl_xor_sync(0xffffffffu, even, 1);
+                even += __shfl_xor_sync(0xffffffffu, even, 2);
+                // an accumulator fragment holds heads 2q and 2q + 1
+                c2_init[0] = -__shfl_sync(0xffffffffu, even, 8 * q);
+                c2_init[1] = -__shfl_sync(0xffffffffu, even, 8 * q + 4);
             }
         }
 
-        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};   // heads 2q, 2q + 1; in units of log2
+        // Reference of heads 2q, 2q + 1 in units of log2, kNone before the first tile (finite: scores are taken relative to it).
+        float m_run[2] = {kNone, kNone}, l_run[2] = {0.f, 0.f};
         float acc[kSteps][4];
 #pragma unroll
         for (int mt = 0; mt < kSteps; ++mt)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[mt][k] = 0.f;
 
-        int token = (first_tile + tile0 + warp) * kKvTile + g;   // this thread's tokens of the tile: token, token + 8
-        for (int i = 0; i < mine; ++i, token += C::kWarps * kKvTile) {
-            if (!bar_wait(bars + 8u * stage, (phase >> stage) & 1u)) {
-                ok = false;
-                break;
+        // The values of a tile are multiplied one iteration late, beside the next tile's scores: the two are independent, and
+        // together they cover each other's shared-memory and tensor latencies.
+        uint32_t xa[W], xb[W], pb0 = 0u, pb1 = 0u;   // value words (token pairs q and q + 4, dim group g) and P^T of the last tile
+#pragma unroll
+        for (int w = 0; w < W; ++w) xa[w] = xb[w] = 0u;
+        // rows g and g + 8 of m tile 2 w + h are dims 4 w + 2 h and the next of group g
+        auto multiply_values = [&] {
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const uint32_t A = D == 128 && w == 3 ? kv_value_spare(xa[0], xa[1 % W], xa[2 % W]) : xa[w];
+                const uint32_t Bw = D == 128 && w == 3 ? kv_value_spare(xb[0], xb[1 % W], xb[2 % W]) : xb[w];
+                mma_f16(acc[2 * w], table_load(pair_addr<0>(A, lane_base)), table_load(pair_addr<1>(A, lane_base)),
+                        table_load(pair_addr<0>(Bw, lane_base)), table_load(pair_addr<1>(Bw, lane_base)), pb0, pb1);
+                mma_f16(acc[2 * w + 1], table_load(pair_addr<2>(A, lane_base)), table_load(pair_addr<3>(A, lane_base)),
+                        table_load(pair_addr<2>(Bw, lane_base)), table_load(pair_addr<3>(Bw, lane_base)), pb0, pb1);
             }
-            const uint32_t blk = ring + stage * B::kBytes;
+        };
+        // One tile: its block in shared memory, its first token.
+        auto take_tile = [&](uint32_t blk, int token) {
             // ---- scores ----
             float c1[4] = {0.f, 0.f, 0.f, 0.f}, c1b[4] = {0.f, 0.f, 0.f, 0.f};
+            float c2[4] = {c2_init[0], c2_init[1], c2_init[0], c2_init[1]}, c2b[4] = {0.f, 0.f, 0.f, 0.f};
             {
                 uint32_t ka[W], kb[W];
                 load_words<W>(ka, blk + g * (D / 2) + q * (D / 8));
                 load_words<W>(kb, blk + (g + 8) * (D / 2) + q * (D / 8));
 #pragma unroll
                 for (int w = 0; w < W; ++w) {
-                    mma_f16(c1, table_load(pair_addr<0>(ka[w], lane_const)), table_load(pair_addr<0>(kb[w], lane_const)),
-                            table_load(pair_addr<1>(ka[w], lane_const)), table_load(pair_addr<1>(kb[w], lane_const)), bq[4 * w], bq[4 * w + 1]);
-                    mma_f16(c1b, table_load(pair_addr<2>(ka[w], lane_const)), table_load(pair_addr<2>(kb[w], lane_const)),
-                            table_load(pair_addr<3>(ka[w], lane_const)), table_load(pair_addr<3>(kb[w], lane_const)), bq[4 * w + 2], bq[4 * w + 3]);
+                    mma_f16(c1, table_load(pair_addr<0>(ka[w], lane_base)), table_load(pair_addr<0>(kb[w], lane_base)),
+                            table_load(pair_addr<1>(ka[w], lane_base)), table_load(pair_addr<1>(kb[w], lane_base)), bq[4 * w], bq[4 * w + 1]);
+                    mma_f16(c1b, table_load(pair_addr<2>(ka[w], lane_base)), table_load(pair_addr<2>(kb[w], lane_base)),
+                            table_load(pair_addr<3>(ka[w], lane_base)), table_load(pair_addr<3>(kb[w], lane_base)), bq[4 * w + 2], bq[4 * w + 3]);
                 }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) c1[k] += c1b[k];
                 if constexpr (QJL) {
-                    float c2[4] = {0.f, 0.f, 0.f, 0.f}, c2b[4] = {0.f, 0.f, 0.f, 0.f};
-                    // sign bits of nibbles r and r + 4 -> fp16 pair (+-1, +-1): the shifted bits over the pattern of (-1, -1)
-                    auto sgn = [](uint32_t w, int r) { return ((w << (12 - 4 * r)) & 0x80008000u) ^ 0xBC00BC00u; };
+                    // Bits 14 and 30 (dims 2, 6 of a word) as they stand are fp16 {0, 2}; bits 15 and 31 (dims 3, 7) over the
+                    // pattern of (-1, -1) are {-1, 1}; the word shifted by a byte gives dims 0, 4 and 1, 5 the same way.
+                    auto two = [](uint32_t w) { return w & 0x40004000u; };
+                    auto one = [](uint32_t w) { return (w & 0x80008000u) ^ 0xBC00BC00u; };
 #pragma unroll
                     for (int w = 0; w < W; ++w) {
-                        mma_f16(c2, sgn(ka[w], 0), sgn(kb[w], 0), sgn(ka[w], 1), sgn(kb[w], 1), bs[4 * w], bs[4 * w + 1]);
-                        mma_f16(c2b, sgn(ka[w], 2), sgn(kb[w], 2), sgn(ka[w], 3), sgn(kb[w], 3), bs[4 * w + 2], bs[4 * w + 3]);
+                        const uint32_t la = ka[w] << 8, lb = kb[w] << 8;
+                        mma_f16(c2, two(la), two(lb), one(la), one(lb), bs[4 * w], bs[4 * w + 1]);
+                        mma_f16(c2b, two(ka[w]), two(kb[w]), one(ka[w]), one(kb[w]), bs[4 * w + 2], bs[4 * w + 3]);
                     }
-                    const float qa = load_f32(blk + B::kNormOff + 2 * kKvTile * 4 + g * 4) * a.qscale;
-                    const float qb = load_f32(blk + B::kNormOff + 2 * kKvTile * 4 + (g + 8) * 4) * a.qscale;
-                    c1[0] = fmaf(qa, c2[0] + c2b[0], c1[0]);
-                    c1[1] = fmaf(qa, c2[1] + c2b[1], c1[1]);
-                    c1[2] = fmaf(qb, c2[2] + c2b[2], c1[2]);
-                    c1[3] = fmaf(qb, c2[3] + c2b[3], c1[3]);
                 }
             }
-            const bool va = token >= S.start && token < S.end, vb = token + 8 >= S.start && token + 8 < S.end;
-            const float kna = load_f32(blk + B::kNormOff + g * 4) * a.score_scale, knb = load_f32(blk + B::kNormOff + (g + 8) * 4) * a.score_scale;
-            float vna = load_f32(blk + B::kNormOff + kKvTile * 4 + g * 4), vnb = load_f32(blk + B::kNormOff + kKvTile * 4 + (g + 8) * 4);
-            vna = va ? vna * (1.0f / kAttnCentroidScale) : 0.f;
-            vnb = vb ? vnb * (1.0f / kAttnCentroidScale) : 0.f;
-            const float s00 = va ? c1[0] * kna : -INFINITY, s01 = va ? c1[1] * kna : -INFINITY;
-            const float s10 = vb ? c1[2] * knb : -INFINITY, s11 = vb ? c1[3] * knb : -INFINITY;
-            // value words, then the stage can be refilled
-            uint32_t xa[W], xb[W];
+            multiply_values();   // of the tile before
+            // ---- this tile's norms and value words; then the stage can be refilled ----
+            float kna, knb, vna, vnb, qna = 0.f, qnb = 0.f;
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(kna), "=f"(vna) : "r"(blk + B::kNormOff + g * 8));
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(knb), "=f"(vnb) : "r"(blk + B::kNormOff + (g + 8) * 8));
+            if constexpr (QJL) {
+                qna = load_f32(blk + B::kNormOff + 2 * kKvTile * 4 + g * 4);
+                qnb = load_f32(blk + B::kNormOff + 2 * kKvTile * 4 + (g + 8) * 4);
+            }
             if constexpr (D == 128) {
-                uint32_t t[2];
-                load_words<2>(t, blk + B::kValueOff + g * 32 + q * 8);
+                uint32_t t[2], o[1];
+                load_words<2>(t, blk + B::kValueOff + (q * 8 + g) * 8);
                 xa[0] = t[0];
                 xa[1] = t[1];
-                load_words<2>(t, blk + B::kValueOff + (g + 8) * 32 + q * 8);
+                load_words<2>(t, blk + B::kValueOff + ((q + 4) * 8 + g) * 8);
                 xb[0] = t[0];
                 xb[1] = t[1];
-                uint32_t o[1];
-                load_words<1>(o, blk + B::kValueOff + 512 + g * 16 + q * 4);
+                load_words<1>(o, blk + B::kValueOff + 512 + (q * 8 + g) * 4);
                 xa[2] = o[0];
-                load_words<1>(o, blk + B::kValueOff + 512 + (g + 8) * 16 + q * 4);
+                load_words<1>(o, blk + B::kValueOff + 512 + ((q + 4) * 8 + g) * 4);
                 xb[2] = o[0];
-                xa[3] = kv_value_spare(xa[0], xa[1], xa[2]);
-                xb[3] = kv_value_spare(xb[0], xb[1], xb[2]);
             } else {
-                load_words<W>(xa, blk + B::kValueOff + g * (D / 2) + q * (D / 8));
-                load_words<W>(xb, blk + B::kValueOff + (g + 8) * (D / 2) + q * (D / 8));
+                load_words<W>(xa, blk + B::kValueOff + (q * 8 + g) * (D / 8));
+                load_words<W>(xb, blk + B::kValueOff + ((q + 4) * 8 + g) * (D / 8));
             }
-            __syncwarp();
-            if (lane == 0 && i + C::kStages < mine)
-                bulk_copy(blk, src + static_cast<size_t>(warp + (i + C::kStages) * C::kWarps) * tile_stride, B::kBytes, bars + 8u * stage);
-            phase ^= 1u << stage;
-            stage = stage + 1 == C::kStages ? 0 : stage + 1;
-
             // ---- online softmax with a lazy reference: it moves (and the sums are rescaled) only when some score exceeds
             // it by more than the slack, so the usual tile needs one vote instead of a reduction over the tokens.  Every
             // tile holds a token of [start, end), so the reference is finite from a warp's first tile on.
             constexpr float kSlack = kAttnSoftmaxSlack * 1.4426950408889634f;
-            const float tm0 = fmaxf(s00, s10), tm1 = fmaxf(s01, s11);
-            if (__any_sync(0xffffffffu, tm0 > m_run[0] + kSlack || tm1 > m_run[1] + kSlack)) {
-                float mx0 = tm0, mx1 = tm1;
+            float x0 = c1[0] + c1b[0], x1 = c1[1] + c1b[1], x2 = c1[2] + c1b[2], x3 = c1[3] + c1b[3];
+            if constexpr (QJL) {
+                x0 = fmaf(qna, c2[0] + c2b[0], x0);
+                x1 = fmaf(qna, c2[1] + c2b[1], x1);
+                x2 = fmaf(qnb, c2[2] + c2b[2], x2);
+                x3 = fmaf(qnb, c2[3] + c2b[3], x3);
+            }
+            kna *= a.score_scale;
+            knb *= a.score_scale;
+            // scores relative to the reference: (token g: heads 2q, 2q + 1), (token g + 8: the same)
+            float s00 = fmaf(x0, kna, -m_run[0]), s01 = fmaf(x1, kna, -m_run[1]), s10 = fmaf(x2, knb, -m_run[0]), s11 = fmaf(x3, knb, -m_run[1]);
+            if (token < seg.start || token + kKvTile > seg.end) {   // tokens outside the range, only in a job's end tiles
+                const int ta = token + g, tb = ta + 8;
+                if (ta < seg.start || ta >= seg.end) { s00 = s01 = -INFINITY; vna = 0.f; }
+                if (tb < seg.start || tb >= seg.end) { s10 = s11 = -INFINITY; vnb = 0.f; }
+            }
+            if (__any_sync(0xffffffffu, fmaxf(fmaxf(s00, s01), fmaxf(s10, s11)) > kSlack)) {
+                // absolute again: relative to the first tile's reference (kNone) a score has no bits left
+                const float t00 = s00 == -INFINITY ? s00 : x0 * kna, t01 = s01 == -INFINITY ? s01 : x1 * kna;
+                const float t10 = s10 == -INFINITY ? s10 : x2 * knb, t11 = s11 == -INFINITY ? s11 : x3 * knb;
+                float mx0 = fmaxf(t00, t10), mx1 = fmaxf(t01, t11);
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) {
                     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
@@ -356,6 +442,10 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 l_run[1] *= cr1;
                 m_run[0] = mn0;
                 m_run[1] = mn1;
+                s00 = t00 - mn0;
+                s01 = t01 - mn1;
+                s10 = t10 - mn0;
+                s11 = t11 - mn1;
 #pragma unroll
                 for (int mt = 0; mt < kSteps; ++mt) {
                     acc[mt][0] *= cr0;
@@ -364,149 +454,184 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                     acc[mt][3] *= cr1;
                 }
             }
-            const float p00 = exp2_approx(s00 - m_run[0]), p01 = exp2_approx(s01 - m_run[1]);
-            const float p10 = exp2_approx(s10 - m_run[0]), p11 = exp2_approx(s11 - m_run[1]);
+            const float p00 = exp2_approx(s00), p01 = exp2_approx(s01), p10 = exp2_approx(s10), p11 = exp2_approx(s11);
             l_run[0] += p00 + p10;
             l_run[1] += p01 + p11;
             // P^T fragment: (tokens 2q, 2q+1 | 2q+8, 2q+9 ; head g) from (token g | g+8 ; heads 2q, 2q+1)
-            const uint32_t pb0 = movmatrix_trans(pack_half2(p00 * vna, p01 * vna));
-            const uint32_t pb1 = movmatrix_trans(pack_half2(p10 * vnb, p11 * vnb));
-            // ---- values: V [token x dim] fragments -> V^T [dim x token] ----
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                mma_f16(acc[2 * w], movmatrix_trans(table_load(pair_addr<0>(xa[w], lane_const))), movmatrix_trans(table_load(pair_addr<1>(xa[w], lane_const))),
-                        movmatrix_trans(table_load(pair_addr<0>(xb[w], lane_const))), movmatrix_trans(table_load(pair_addr<1>(xb[w], lane_const))), pb0, pb1);
-                mma_f16(acc[2 * w + 1], movmatrix_trans(table_load(pair_addr<2>(xa[w], lane_const))), movmatrix_trans(table_load(pair_addr<3>(xa[w], lane_const))),
-                        movmatrix_trans(table_load(pair_addr<2>(xb[w], lane_const))), movmatrix_trans(table_load(pair_addr<3>(xb[w], lane_const))), pb0, pb1);
+            pb0 = movmatrix_trans(pack_half2(p00 * vna, p01 * vna));
+            pb1 = movmatrix_trans(pack_half2(p10 * vnb, p11 * vnb));
+        };
+        const unsigned char* next_src = seg.src + static_cast<size_t>(warp + 2 * C::kStages * C::kTeam) * tile_stride;
+        int token = seg.first_token + warp * kKvTile;
+        for (int left = seg.mine; left > 0; left -= 2, token += 2 * C::kTeam * kKvTile) {
+            if (!bar_wait(bars + 8u * stage, phase)) {
+                ok = false;
+                break;
             }
+            const uint32_t blk = ring + stage * C::kStageBytes;
+            take_tile(blk, token);
+            if (left > 1) take_tile(blk + B::kBytes, token + C::kTeam * kKvTile);
+            __syncwarp();
+            if (lane == 0 && left > 2 * C::kStages) request(blk, next_src, left - 2 * C::kStages, bars + 8u * stage);
+            next_src += 2 * C::kTeam * tile_stride;
+            phase ^= static_cast<uint32_t>(stage);
+            stage ^= 1;
+        }
+        multiply_values();   // of the last tile
+        struct { int tiles, tile0, n_tiles, q_row0, ng, job; } done;
+        {
+            const volatile int* const j = s_job + 7 * job_slot;
+            done.tiles = j[0]; done.tile0 = j[1]; done.n_tiles = j[2]; done.q_row0 = j[3]; done.ng = j[4]; done.job = j[5];
+        }
+        u = s_job[7 * job_slot + 6];
+        bool more = u < u_end;
+        job_slot ^= 1;
+        if (more) {
+            seg = locate(u);
+            more = seg.n_tiles > 0;
+            if (lane == 0 && ok) request_first(seg);   // every lane is past its last read of the ring
         }
 
-        // ---- merge the warps: every warp publishes through its ring, which is idle now ----
+        // ---- merge the warps: the upper half hands its registers to the lower half, which publishes in head order ----
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) {
             l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], o);
             l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], o);
         }
-        if (g == 0) {
-            s_m[warp * kGroup + 2 * q] = m_run[0];
-            s_m[warp * kGroup + 2 * q + 1] = m_run[1];
-            s_l[warp * kGroup + 2 * q] = l_run[0];
-            s_l[warp * kGroup + 2 * q + 1] = l_run[1];
-        }
-        {
-            float* const mine_acc = reinterpret_cast<float*>(at(ring));
-            // row slot of an m tile: slot = g + 8 half -> thread (slot & 7) / 2 of a quad, pair 2 mt + half, low or high code
-            const int d0 = (D / 4) * (g >> 1) + (g & 1);
+        float* const pub = reinterpret_cast<float*>(s_pub + (warp & (C::kHalf - 1)) * C::kPubBytes);
+        if (warp >= C::kHalf) {
 #pragma unroll
-            for (int mt = 0; mt < kSteps; ++mt)
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int d = d0 + 2 * (2 * mt + hf);
-                    mine_acc[(2 * q) * C::kAccStride + d] = acc[mt][2 * hf];
-                    mine_acc[(2 * q + 1) * C::kAccStride + d] = acc[mt][2 * hf + 1];
-                }
+            for (int mt = 0; mt < kSteps; ++mt) *reinterpret_cast<float4*>(pub + (mt * 32 + lane) * 4) = make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
+            *reinterpret_cast<float4*>(pub + (kSteps * 32 + lane) * 4) = make_float4(m_run[0], m_run[1], l_run[0], l_run[1]);
         }
-        __syncthreads();
-        const bool whole = n_tiles == tiles;
-        // which ranges share the job: the range of flat tile x is ((x + 1) n_ctas - 1) / units
-        const int c_first = whole ? cta : static_cast<int>((static_cast<long>(job_u0 + 1) * n_ctas - 1) / a.units);
-        const int c_last = whole ? cta : static_cast<int>((static_cast<long>(job_u0 + tiles) * n_ctas - 1) / a.units);
-        float* const my_part = a.part + static_cast<size_t>(2 * cta + (tile0 == 0 ? 1 : 0)) * C::kPartFloats;
-        for (int idx = tid; idx < kGroup * D; idx += C::kThreads) {
+        team_sync();
+        if (warp < C::kHalf) {
+            const float4 ml = *reinterpret_cast<const float4*>(pub + (kSteps * 32 + lane) * 4);
+            const float M0 = fmaxf(m_run[0], ml.x), M1 = fmaxf(m_run[1], ml.y);
+            // (a warp without tiles has the reference kNone and sums of zero)
+            const float f0 = exp2_approx(m_run[0] - M0), f1 = exp2_approx(m_run[1] - M1);
+            const float h0 = exp2_approx(ml.x - M0), h1 = exp2_approx(ml.y - M1);
+            l_run[0] = fmaf(l_run[0], f0, ml.z * h0);
+            l_run[1] = fmaf(l_run[1], f1, ml.w * h1);
+#pragma unroll
+            for (int mt = 0; mt < kSteps; ++mt) {
+                const float4 o = *reinterpret_cast<const float4*>(pub + (mt * 32 + lane) * 4);
+                acc[mt][0] = fmaf(acc[mt][0], f0, o.x * h0);
+                acc[mt][1] = fmaf(acc[mt][1], f1, o.y * h1);
+                acc[mt][2] = fmaf(acc[mt][2], f0, o.z * h0);
+                acc[mt][3] = fmaf(acc[mt][3], f1, o.w * h1);
+            }
+            __syncwarp();   // the place is this warp's own from here on
+            if (g == 0) {
+                s_m[warp * kGroup + 2 * q] = M0;
+                s_m[warp * kGroup + 2 * q + 1] = M1;
+                s_l[warp * kGroup + 2 * q] = l_run[0];
+                s_l[warp * kGroup + 2 * q + 1] = l_run[1];
+            }
+#pragma unroll
+            for (int mt = 0; mt < kSteps; ++mt) {
+                const int d = (D / 8) * g + 2 * mt;   // rows g and g + 8: dims d and d + 1; columns: heads 2q and 2q + 1
+                *reinterpret_cast<float2*>(pub + (2 * q) * C::kAccStride + d) = make_float2(acc[mt][0], acc[mt][2]);
+                *reinterpret_cast<float2*>(pub + (2 * q + 1) * C::kAccStride + d) = make_float2(acc[mt][1], acc[mt][3]);
+            }
+        }
+        team_sync();
+        const bool whole = done.n_tiles == done.tiles;
+        // which ranges share the job: the range of flat tile x is ((x + 1) ranges - 1) / units
+        const int job_u0 = u - done.n_tiles - done.tile0;   // the job's first tile
+        const int c_first = whole ? range : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
+        const int c_last = whole ? range : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
+        float* const my_part = a.part + static_cast<size_t>(2 * range + (done.tile0 == 0 ? 1 : 0)) * C::kPartFloats;
+        auto add4 = [](float4& x, float f0, const float4& y, float f1) {
+            x.x = fmaf(x.x, f0, y.x * f1);
+            x.y = fmaf(x.y, f0, y.y * f1);
+            x.z = fmaf(x.z, f0, y.z * f1);
+            x.w = fmaf(x.w, f0, y.w * f1);
+        };
+        for (int idx = tid * 4; idx < kGroup * D; idx += C::kTeam * 128) {
             const int h = idx / D, d = idx - h * D;
-            float M = -INFINITY;
+            float m[C::kHalf], M = kNone;
 #pragma unroll
-            for (int w = 0; w < C::kWarps; ++w) M = fmaxf(M, s_m[w * kGroup + h]);
-            float L = 0.f, A = 0.f;
+            for (int w = 0; w < C::kHalf; ++w) {
+                m[w] = s_m[w * kGroup + h];
+                M = fmaxf(M, m[w]);
+            }
+            float L = 0.f;
+            float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int w = 0; w < C::kWarps; ++w) {
-                const float m = s_m[w * kGroup + h];
-                const float f = m == -INFINITY ? 0.f : exp2_approx(m - M);
-                const float* const wa = reinterpret_cast<const float*>(at(w < C::kLowRings ? kLowBase + w * C::kRing : C::kHighBase + (w - C::kLowRings) * C::kRing));
+            for (int w = 0; w < C::kHalf; ++w) {
+                const float f = exp2_approx(m[w] - M);
                 L = fmaf(s_l[w * kGroup + h], f, L);
-                A = fmaf(wa[h * C::kAccStride + d], f, A);
+                add4(A, 1.f, *reinterpret_cast<const float4*>(s_pub + w * C::kPubBytes + (h * C::kAccStride + d) * 4), f);
             }
-            if (whole) {
-                s_out[h * C::kAccStride + d] = A;
-            } else {
-                my_part[idx] = A;
-                if (d == 0) {
-                    my_part[kGroup * D + 2 * h] = M;
-                    my_part[kGroup * D + 2 * h + 1] = L;
-                }
-            }
-            if (whole && d == 0) {
-                s_out[h * C::kAccStride + D] = M;
-                s_out[h * C::kAccStride + D + 1] = L;
-            }
+            *reinterpret_cast<float4*>((whole ? s_out + h * C::kAccStride : my_part + h * D) + d) = A;
+            if (d == 0) *reinterpret_cast<float2*>(whole ? s_out + h * C::kAccStride + D : my_part + kGroup * D + 2 * h) = make_float2(M, L);
         }
         bool finish = whole;
         if (!whole) {
             __threadfence();
-            __syncthreads();
+            team_sync();
             if (tid == 0) {
-                const unsigned int prev = atomicAdd(&a.counters[job], 1u);
-                s_last = prev == static_cast<unsigned int>(c_last - c_first) ? 1u : 0u;
-                if (s_last) a.counters[job] = 0u;   // ready for the next launch
+                const unsigned int prev = atomicAdd(&a.counters[done.job], 1u);
+                const bool last = prev == static_cast<unsigned int>(c_last - c_first);
+                s_flag[0] = last ? 1u : 0u;
+                if (last) a.counters[done.job] = 0u;   // ready for the next launch
             }
-            __syncthreads();
-            finish = s_last != 0u;
+            team_sync();
+            finish = s_flag[0] != 0u;
             if (finish) {
                 __threadfence();
                 auto part_of = [&](int c) {
                     // the first range's part of the job starts at its tile 0
                     return a.part + static_cast<size_t>(2 * c + (c == c_first ? 1 : 0)) * C::kPartFloats;
                 };
-                for (int idx = tid; idx < kGroup * D; idx += C::kThreads) {
+                for (int idx = tid * 4; idx < kGroup * D; idx += C::kTeam * 128) {
                     const int h = idx / D, d = idx - h * D;
-                    float M = -INFINITY, L = 0.f, A = 0.f;
-                    for (int c0 = c_first; c0 <= c_last; c0 += 4) {   // four parts at a time, added in order
-                        float pm[4], pl[4], pa[4];
+                    float M = kNone, L = 0.f;
+                    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int c0 = c_first; c0 <= c_last; c0 += 6) {   // six parts requested at a time, added in order
+                        float2 ml[6];
+                        float4 pa[6];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
+                        for (int k = 0; k < 6; ++k) {
                             const float* const p = part_of(min(c0 + k, c_last));
-                            pm[k] = c0 + k <= c_last ? __ldcg(p + kGroup * D + 2 * h) : -INFINITY;
-                            pl[k] = __ldcg(p + kGroup * D + 2 * h + 1);
-                            pa[k] = __ldcg(p + idx);
+                            ml[k] = __ldcg(reinterpret_cast<const float2*>(p + kGroup * D + 2 * h));
+                            pa[k] = __ldcg(reinterpret_cast<const float4*>(p + idx));
                         }
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            if (pm[k] == -INFINITY) continue;
-                            const float mn = fmaxf(M, pm[k]);
-                            const float f0 = exp2_approx(M - mn), f1 = exp2_approx(pm[k] - mn);
-                            L = fmaf(L, f0, pl[k] * f1);
-                            A = fmaf(A, f0, pa[k] * f1);
+                        for (int k = 0; k < 6; ++k) {
+                            if (c0 + k > c_last) break;
+                            const float mn = fmaxf(M, ml[k].x), f0 = exp2_approx(M - mn), f1 = exp2_approx(ml[k].x - mn);
+                            L = fmaf(L, f0, ml[k].y * f1);
+                            add4(A, f0, pa[k], f1);
                             M = mn;
                         }
                     }
-                    s_out[h * C::kAccStride + d] = A;
-                    if (d == 0) {
-                        s_out[h * C::kAccStride + D] = M;
-                        s_out[h * C::kAccStride + D + 1] = L;
-                    }
+                    *reinterpret_cast<float4*>(s_out + h * C::kAccStride + d) = A;
+                    if (d == 0) *reinterpret_cast<float2*>(s_out + h * C::kAccStride + D) = make_float2(M, L);
                 }
             }
         }
-        // generic accesses to the rings end here; the next job's bulk copies write them
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
+        if (!ok && lane == 0) s_flag[1] = 1u;
+        team_sync();   // (also: s_out is written, the publishing places are free)
+        const bool stop = s_flag[1] != 0u;
         // ---- un-rotate and write: out = (inv_sqrt * sign_v) o H(inv_scale * acc) / L, a warp per head ----
-        if (finish && warp < ng) {
+        for (int h = warp; finish && !stop && h < done.ng; h += C::kTeam) {
             constexpr int E = D / 32;
-            const float M = s_out[warp * C::kAccStride + D], L = s_out[warp * C::kAccStride + D + 1];
+            const float M = s_out[h * C::kAccStride + D], L = s_out[h * C::kAccStride + D + 1];
             float v[E];
 #pragma unroll
-            for (int j = 0; j < E; ++j) v[j] = s_out[warp * C::kAccStride + lane * E + j] * a.inv_scale;
+            for (int j = 0; j < E; ++j) v[j] = s_out[h * C::kAccStride + lane * E + j] * a.inv_scale;
             warp_fwht<E>(v, lane);
             const float invL = L > 0.f ? 1.0f / L : 0.f;
-            const size_t row = static_cast<size_t>(q_row0 + warp);
+            const size_t row = static_cast<size_t>(done.q_row0 + h);
             // log of the softmax denominator: lets a caller merge results over disjoint token ranges
             if (a.lse != nullptr && lane == 0) a.lse[row] = L > 0.f ? M * 0.6931471805599453f + __logf(L) : -INFINITY;
 #pragma unroll
             for (int j = 0; j < E; ++j)
                 a.out[row * D + lane * E + j] = __float2half_rn(v[j] * a.inv_sqrt * sign_value(a.v_seed, static_cast<uint32_t>(lane * E + j)) * invL);
         }
-        if (__syncthreads_or(!ok)) break;   // (also: s_out and s_q are free again)
+        if (stop || !more) break;
     }
     if (!ok && lane == 0) {
         // let whatever was requested land before the shared memory is released
@@ -519,8 +644,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
 template <int D, bool QJL>
 void launch_d(const AttnArgs& args, int grid, cudaStream_t stream) {
     using C = AttnCfg<D>;
-    // the window starts at the dynamic memory's base, at most kLowBase; asking up to the end of the map covers any base
-    constexpr int kSmem = static_cast<int>(C::kEnd - 0x400u);
+    constexpr int kSmem = static_cast<int>(C::kEnd);
     static bool configured[64] = {false};   // the opt-in size is a per-device attribute
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
@@ -542,7 +666,7 @@ long attn_number_tiles(AttnSeq* seqs, int n_seqs) {
     return total;
 }
 
-size_t attn_scratch_bytes(int dim, int sm_count) { return static_cast<size_t>(sm_count) * 2 * (kGroup * dim + 2 * kGroup) * sizeof(float); }
+size_t attn_scratch_bytes(int dim, int sm_count) { return static_cast<size_t>(2 * sm_count) * 2 * (kGroup * dim + 2 * kGroup) * sizeof(float); }
 
 size_t attn_counters(int n_seqs, int q_heads, int kv_heads) {
     return static_cast<size_t>(n_seqs) * kv_heads * ((q_heads / kv_heads + kGroup - 1) / kGroup);
@@ -566,21 +690,27 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, const voi
     a.q_heads = q_heads;
     a.kv_heads = kv_heads;
     a.gchunks = (q_heads / kv_heads + kGroup - 1) / kGroup;
-    const long units = tiles * kv_heads * a.gchunks;
-    TQ_REQUIRE(units > 0 && units < (1L << 31), "attention: too many tokens for one call");
-    a.units = static_cast<int>(units);
+    long units = tiles * kv_heads * a.gchunks;
+    TQ_REQUIRE(units > 0 && tiles > 0 && units < (1L << 31), "attention: too many tokens for one call");
     a.k_seed = k_seed;
     a.v_seed = v_seed;
     a.qjl_seed = qjl_seed;
     const double d = head_dim;
     a.inv_sqrt = 1.0f / std::sqrt(static_cast<float>(head_dim));
-    a.inv_scale = a.inv_sqrt;
+    a.inv_scale = a.inv_sqrt / kAttnCentroidScale;   // of the value sums, whose table is scaled as well
     // softmax scale 1 / sqrt(D) (src/attention_dispatch.cpp:35) and the rotation's 1 / sqrt(D), in units of log2
     a.score_scale = static_cast<float>(1.4426950408889634 / d / kAttnCentroidScale);
-    a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale);
-    // A CTA per SM while every CTA gets a tile per warp; fewer for short jobs, whose time is the merge of the parts.
-    const int warps = head_dim == 256 ? 8 : 16;
-    const int grid = static_cast<int>(std::min<long>(sm_count, std::max<long>(1, (units + warps - 1) / warps)));
+    // of the rotated query before its 1 / sqrt(D): the residual's reconstruction, in units of the scaled centroids
+    a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale / std::sqrt(d));
+    // Two ranges per SM while every range has a tile per warp; fewer for short jobs, whose time is the merge of the parts.
+    const int team = 8, teams = head_dim == 256 ? 1 : 2;
+    a.ranges = static_cast<int>(std::min<long>(static_cast<long>(teams) * sm_count, std::max<long>(1, (units + team - 1) / team)));
+    // 32: five rounds of the team's warps, about 6 us; less where ranges are short and every job ends in several of them
+    a.pad = static_cast<int>(std::min<long>(32, units / a.ranges / 8));
+    units += static_cast<long>(n_seqs) * kv_heads * a.gchunks * a.pad;
+    TQ_REQUIRE(units < (1L << 31), "attention: too many tokens for one call");
+    a.units = static_cast<int>(units);
+    const int grid = std::min(sm_count, a.ranges);
 #define TQ_ATT(DV)                                                   \
     case DV:                                                         \
         if (use_qjl) launch_d<DV, true>(a, grid, stream);            \

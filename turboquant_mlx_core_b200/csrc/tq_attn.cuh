@@ -11,16 +11,18 @@ namespace tq {
 // ---- storage of the compressed cache -----------------------------------------------------------------
 // A layer's storage is one allocation of blocks [16-token tile][KV head].  A block holds the 16 tokens' records of one
 // head in the order the attention kernel consumes them, so a tile is ONE contiguous bulk copy whatever the head count
-// (the reference's token-major arrays took six copies per tile, or one per token and array beyond four heads):
-//   keys    16 tokens x D/2 bytes: dim 8 w + i in nibble i of word w, bits 0-2 the code, bit 3 the residual's sign bit
-//   values  D = 128: per token and quarter q of the dims three words of nibbles for the quarter's first 24 dims; the
-//           codes of its last eight dims are spread over the nibbles' spare bits (bit k of dim 24 + i in bit 3 of nibble i
-//           of word k).  Words 0 and 1 of all (token, quarter) first, then word 2.   48 bytes per token
-//           other D: nibbles like the keys, bit 3 zero
-//   norms   16 key norms, 16 value norms, 16 residual norms (fp32)
-// D = 128: 124 bytes per token and head (the reference's words of ten codes: 132), every byte of a nibble word a pair
-// of codes that one byte permutation turns into a table address.  Snapshots, deltas and exports convert to and from the
-// reference's arrays (tq_kv_kernels.cu).
+// (the reference's token-major arrays took six copies per tile, or one per token and array beyond four heads).  A byte
+// is an entry of the kernel's table of code PAIRS:
+//   keys    16 tokens x D/2 bytes.  Byte b of a token: codes of dims 2b (bits 0-2) and 2b + 1 (bits 3-5), and the signs of
+//           their residuals in bits 6 and 7.
+//   values  8 token pairs x 8 groups of D/8 dims.  A byte holds one dim's codes of an even token (bits 0-2) and the odd
+//           token after it (bits 3-5): the operand of the value product wants two tokens side by side.  D = 128 packs a
+//           group's 16 dims into three words: bytes for the first 12, and the six bits of dim 12 + i's byte two by two in
+//           bits 6 and 7 of byte i of the three words - 48 bytes per token.  Words 0 and 1 of all (pair, group) come
+//           first, then word 2.  Other D: a byte per dim, bits 6 and 7 zero.
+//   norms   16 x (key norm, value norm), then 16 residual norms (fp32)
+// D = 128: 124 bytes per token and head (the reference's words of ten codes: 132).  Snapshots, deltas and exports convert
+// to and from the reference's arrays (tq_kv_kernels.cu).
 constexpr int kKvTile = 16;
 template <int D>
 struct KvBlock {
@@ -36,16 +38,30 @@ __host__ __device__ constexpr size_t kv_block_bytes(int dim) {
 // Bytes of a layer's storage for `cap` tokens (a multiple of 16).
 inline size_t kv_layer_bytes(int cap, int heads, int dim) { return static_cast<size_t>(cap / kKvTile) * heads * kv_block_bytes(dim); }
 
-// The value words of (token slot t of the tile, quarter q) of a D = 128 block.
-__device__ __forceinline__ uint32_t* kv_value01(unsigned char* block, int t, int q) {
-    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff) + (t * 4 + q) * 2;
+// The value words of (token pair p of the tile, dim group g): words 0 and 1, and word 2, of a D = 128 block; the first
+// of the D/32 words of other blocks.
+__host__ __device__ __forceinline__ uint32_t* kv_value01(unsigned char* block, int p, int g) {
+    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff) + (p * 8 + g) * 2;
 }
-__device__ __forceinline__ uint32_t* kv_value2(unsigned char* block, int t, int q) {
-    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff + 512) + t * 4 + q;
+__host__ __device__ __forceinline__ uint32_t* kv_value2(unsigned char* block, int p, int g) {
+    return reinterpret_cast<uint32_t*>(block + KvBlock<128>::kValueOff + 512) + p * 8 + g;
 }
-// The codes of a quarter's last eight dims, out of the spare bits of its three words.
-__device__ __forceinline__ uint32_t kv_value_spare(uint32_t w0, uint32_t w1, uint32_t w2) {
-    return ((w0 >> 3) & 0x11111111u) | ((w1 >> 2) & 0x22222222u) | ((w2 >> 1) & 0x44444444u);
+__host__ __device__ __forceinline__ uint32_t* kv_value_row(unsigned char* block, int dim, int p, int g) {
+    return reinterpret_cast<uint32_t*>(block + kKvTile * dim / 2) + (p * 8 + g) * (dim / 32);
+}
+// The bytes of a packed group's last four dims.
+__host__ __device__ __forceinline__ uint32_t kv_value_spare(uint32_t w0, uint32_t w1, uint32_t w2) {
+    return ((w0 >> 6) & 0x03030303u) | ((w1 >> 4) & 0x0C0C0C0Cu) | ((w2 >> 2) & 0x30303030u);
+}
+// Norms of a block: index into its floats from kNormOff on.
+__host__ __device__ constexpr int kv_key_norm(int slot) { return 2 * slot; }
+__host__ __device__ constexpr int kv_value_norm(int slot) { return 2 * slot + 1; }
+__host__ __device__ constexpr int kv_residual_norm(int slot) { return 2 * kKvTile + slot; }
+// ... and the other way, their bits for word k.
+__host__ __device__ __forceinline__ uint32_t kv_spare_bits(uint32_t spare, int k) { return ((spare >> (2 * k)) & 0x03030303u) << 6; }
+// The bits of value word k that belong to the odd token of its pair (the others: the even token's).
+__host__ __device__ __forceinline__ uint32_t kv_odd_bits(int dim, int k) {
+    return dim != 128 ? 0xF8F8F8F8u : (k == 0 ? 0x38383838u : (k == 1 ? 0xB8B8B8B8u : 0xF8F8F8F8u));
 }
 
 // One append: `tokens` tokens of a layer, from token `first` on, written to the storage at `base`.

@@ -1,23 +1,34 @@
 // Lloyd-Max codebook fit on the device (generate_codebook_from_data, src/codebook.cpp:99-143 and
 // 158-267) and the sample extraction of the converter's per-layer fit (src/converter.cpp:291-368).
 //
-// One iteration = two launches on the same stream, no host round trip:
-//   fit_partial_kernel   every thread bins its values by lower_bound over the current boundaries
-//                        (a value equal to a boundary goes to the lower bin, as the CPU path of the
-//                        reference and quantize() do) into a PRIVATE histogram in shared memory
-//                        ([bin][thread]: no atomics, no bank conflicts), sums in double as the
-//                        reference's CPU path; the block then folds its 256 histograms in a fixed order
-//                        and writes one (sum, count) pair per bin;
-//   fit_update_kernel    one warp folds the blocks' pairs in block order, moves each non-empty bin's
-//                        centroid to its mean, recomputes the midpoints and raises a "converged" flag
-//                        when no centroid moved by 1e-6 or more (src/codebook.cpp:68, 128-131).
-// All `iterations` pairs of launches are enqueued at once; launches after convergence return at
-// their first instruction.  Results are run-to-run identical (fixed summation orders).
+// An iteration needs, for every boundary, the count and the sum of the values at or below it.  Going over all samples for
+// that took 110 us per iteration at 16.8 M samples, a hundred times.  Instead the samples are bucketed ONCE by the leading
+// bits of their order-preserving key (sign, exponent, a few mantissa bits), with running counts and sums per bucket; a
+// boundary then only looks at the values of its own bucket, and all iterations run in one launch of one CTA, a warp per
+// boundary (about 1 us each).
+//   fit_count_kernel      bucket counts, largest magnitude            (one pass over the samples)
+//   fit_groups / fit_offsets   exclusive scan of the counts, 256 buckets per group
+//   fit_scatter_kernel    samples into their buckets                  (one pass)
+//   fit_sums_kernel       sum of every bucket
+//   fit_iterate_kernel    the iterations
+// A value equal to a boundary goes to the lower bin, as std::lower_bound in the reference's CPU path and quantize() have
+// it.  Sums are 64-bit integers in units of 2^-s, s chosen so that n values cannot overflow: exact up to the rounding of
+// values below 2^-37 of the largest, the accuracy of the reference's double sums, and independent of the order in which the
+// scatter placed the values - results are run-to-run identical.
+// A boundary whose bucket holds more than kFitMaxBucket values (samples with heavy repetition), or samples that are not
+// finite, stop fit_iterate_kernel; the remaining iterations then go over all samples:
+//   fit_partial_kernel   every thread bins its values by lower_bound over the current boundaries into a PRIVATE histogram in
+//                        shared memory ([bin][thread]: no atomics, no bank conflicts), sums in double; the block then folds
+//                        its 256 histograms in a fixed order and writes one (sum, count) pair per bin;
+//   fit_update_kernel    one warp folds the blocks' pairs in block order, moves each non-empty bin's centroid to its mean,
+//                        recomputes the midpoints and raises a "converged" flag when no centroid moved by 1e-6 or more
+//                        (src/codebook.cpp:68, 128-131).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 
 #include "tq_common.cuh"
+#include "tq_host.hpp"
 #include "tq_kernels.cuh"
 
 namespace tq {
@@ -34,7 +45,234 @@ struct FitState {
     int n;
     int converged;
     int iterations_run;
+    int go_over_all;                 // fit_iterate_kernel stopped: the remaining iterations go over all samples
+    unsigned int max_bits;           // bits of the largest magnitude
 };
+
+constexpr int kFitGroup = 256;              // buckets of a group
+constexpr unsigned int kFitMaxBucket = 32768;
+
+// Order-preserving key of a float: smaller values have smaller keys (-0 and +0 differ by one, which no sum notices).
+__device__ __forceinline__ unsigned int fit_key(float x) {
+    const unsigned int u = __float_as_uint(x);
+    return u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u);
+}
+// A sample in units of 2^-s.
+__device__ __forceinline__ long long fit_fixed(float x, double unit) { return __double2ll_rn(static_cast<double>(x) * unit); }
+// The unit for samples of magnitude up to max_bits: n of them stay below 2^62.
+__device__ __forceinline__ double fit_unit(unsigned int max_bits, int log2_n) {
+    const int e = static_cast<int>(max_bits >> 23) - 126;   // every magnitude is below 2^e
+    return exp2(static_cast<double>(62 - log2_n - e));
+}
+
+__global__ void __launch_bounds__(256) fit_count_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ count,
+                                                        FitState* __restrict__ state) {
+    unsigned int top = 0;
+    for (unsigned int i = blockIdx.x * 1024u + threadIdx.x; i < n; i += gridDim.x * 1024u) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned int at = i + 256u * k;
+            if (at < n && at >= i) {
+                const float x = __ldg(data + at);
+                top = max(top, __float_as_uint(x) & 0x7fffffffu);
+                atomicAdd(&count[fit_key(x) >> shift], 1u);
+            }
+        }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) atomicMax(&state->max_bits, top);
+}
+
+// Inclusive scan over the 256 threads of a block.
+__device__ __forceinline__ unsigned int block_scan256(unsigned int v, unsigned int* s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) v += s_warp[w];
+    __syncthreads();
+    return v;
+}
+__global__ void __launch_bounds__(256) fit_groups_kernel(const unsigned int* __restrict__ count, unsigned int* __restrict__ group) {
+    __shared__ unsigned int s_warp[8];
+    const unsigned int v = block_scan256(count[blockIdx.x * kFitGroup + threadIdx.x], s_warp);
+    if (threadIdx.x == 255) group[blockIdx.x] = v;
+}
+// Exclusive offsets of the buckets of a group; the groups before it are added up here (a few thousand at most).
+__global__ void __launch_bounds__(256) fit_offsets_kernel(const unsigned int* __restrict__ count, const unsigned int* __restrict__ group,
+                                                          unsigned int* __restrict__ offset, unsigned int* __restrict__ cursor) {
+    __shared__ unsigned int s_warp[8];
+    unsigned int before = 0;
+    for (unsigned int g = threadIdx.x; g < blockIdx.x; g += 256) before += group[g];
+    before = block_scan256(before, s_warp);
+    __shared__ unsigned int s_before;
+    if (threadIdx.x == 255) s_before = before;
+    __syncthreads();
+    const int b = blockIdx.x * kFitGroup + threadIdx.x;
+    const unsigned int c = count[b], at = s_before + block_scan256(c, s_warp) - c;
+    offset[b] = at;
+    cursor[b] = at;
+}
+__global__ void __launch_bounds__(256) fit_scatter_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ cursor,
+                                                          float* __restrict__ sorted) {
+    for (unsigned int i = blockIdx.x * 1024u + threadIdx.x; i < n; i += gridDim.x * 1024u) {
+        float x[4];
+        unsigned int pos[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned int at = i + 256u * k;
+            const bool in = at < n && at >= i;
+            x[k] = in ? __ldg(data + at) : 0.f;
+            pos[k] = in ? atomicAdd(&cursor[fit_key(x[k]) >> shift], 1u) : 0xffffffffu;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (pos[k] != 0xffffffffu) sorted[pos[k]] = x[k];
+    }
+}
+// One block per group, a warp per bucket: bucket sums and the group's.
+__global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__ sorted, const unsigned int* __restrict__ count,
+                                                       const unsigned int* __restrict__ offset, int log2_n, const FitState* __restrict__ state,
+                                                       long long* __restrict__ sum, long long* __restrict__ group_sum) {
+    __shared__ long long s_total[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double unit = fit_unit(state->max_bits, log2_n);
+    long long total = 0;
+    for (int k = warp; k < kFitGroup; k += 8) {
+        const int b = blockIdx.x * kFitGroup + k;
+        const unsigned int c = count[b], at = offset[b];
+        long long s = 0;
+        for (unsigned int i = lane; i < c; i += 32) s += fit_fixed(sorted[at + i], unit);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sum[b] = s;
+        total += s;
+    }
+    if (lane == 0) s_total[warp] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        long long t = 0;
+        for (int w = 0; w < 8; ++w) t += s_total[w];
+        group_sum[blockIdx.x] = t;
+    }
+}
+// All iterations: warp w follows boundary w.  `before_sum`: scratch for the exclusive scan of the groups' sums.
+__global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restrict__ sorted, unsigned int n, const unsigned int* __restrict__ count,
+                                                           const unsigned int* __restrict__ offset, const long long* __restrict__ sum,
+                                                           const long long* __restrict__ group_sum, int n_groups, long long* __restrict__ before_sum,
+                                                           int shift, int log2_n, int iterations, FitState* __restrict__ state) {
+    __shared__ float s_c[kFitMaxBins], s_b[kFitMaxBins];
+    __shared__ long long s_le_sum[kFitMaxBins + 1], s_part[33];
+    __shared__ unsigned int s_le[kFitMaxBins + 1];
+    __shared__ int s_stop, s_converged;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nc = state->n;
+    if (tid < nc) s_c[tid] = state->centroids[tid];
+    if (tid < nc - 1) s_b[tid] = state->boundaries[tid];
+    if (tid == 0) {
+        s_stop = state->max_bits >= 0x7f800000u ? 1 : 0;
+        s_converged = 0;
+    }
+    const double unit = fit_unit(state->max_bits, log2_n);
+    // exclusive scan of the groups' sums: a contiguous run of groups per thread
+    const int per = (n_groups + 1023) / 1024;
+    long long own = 0;
+    for (int k = 0; k < per; ++k) {
+        const int g = tid * per + k;
+        if (g < n_groups) own += group_sum[g];
+    }
+    long long scan = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, scan, o);
+        if (lane >= o) scan += t;
+    }
+    if (lane == 31) s_part[warp] = scan;
+    __syncthreads();
+    long long run = scan - own;
+    for (int w = 0; w < warp; ++w) run += s_part[w];
+    for (int k = 0; k < per; ++k) {
+        const int g = tid * per + k;
+        if (g < n_groups) {
+            before_sum[g] = run;
+            run += group_sum[g];
+        }
+    }
+    if (tid == 1023) s_part[32] = run;   // of all samples
+    __syncthreads();                     // (also makes before_sum visible within the block)
+    int bucket = -1;
+    unsigned int b_at = 0, b_count = 0;  // the boundary's bucket, and the sum of everything before it
+    long long b_sum = 0;
+    int it = 0;
+    for (; it < iterations && !s_stop && !s_converged; ++it) {
+        if (warp < nc - 1) {
+            const float bound = s_b[warp];
+            const int now = static_cast<int>(fit_key(bound) >> shift);
+            if (now != bucket) {
+                bucket = now;
+                b_at = offset[now];
+                b_count = count[now];
+                const int g = now / kFitGroup;
+                long long s = 0;
+                for (int b = g * kFitGroup + lane; b < now; b += 32) s += sum[b];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                b_sum = before_sum[g] + s;
+                if (b_count > kFitMaxBucket && lane == 0) s_stop = 1;
+            }
+            unsigned int c = 0;
+            long long s = 0;
+            if (b_count <= kFitMaxBucket) {
+#pragma unroll 4
+                for (unsigned int i = lane; i < b_count; i += 32) {
+                    const float x = sorted[b_at + i];
+                    const bool le = !(bound < x);
+                    c += le ? 1u : 0u;
+                    s += le ? fit_fixed(x, unit) : 0ll;
+                }
+            }
+            c = __reduce_add_sync(0xffffffffu, c);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) {
+                s_le[warp] = b_at + c;
+                s_le_sum[warp] = b_sum + s;
+            }
+        }
+        __syncthreads();
+        if (s_stop) break;   // nothing of this iteration has been applied
+        if (warp == 0) {
+            float shift_of = 0.f, c_new = lane < nc ? s_c[lane] : 0.f;
+            if (lane < nc) {
+                const unsigned int hi = lane < nc - 1 ? s_le[lane] : n, lo = lane > 0 ? s_le[lane - 1] : 0u;
+                const long long hs = lane < nc - 1 ? s_le_sum[lane] : s_part[32], ls = lane > 0 ? s_le_sum[lane - 1] : 0ll;
+                if (hi > lo) {   // an empty bin keeps its centroid
+                    const float mean = static_cast<float>(static_cast<double>(hs - ls) / unit / static_cast<double>(hi - lo));
+                    shift_of = fabsf(mean - c_new);
+                    c_new = mean;
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) shift_of = fmaxf(shift_of, __shfl_xor_sync(0xffffffffu, shift_of, o));
+            const float c_next = __shfl_down_sync(0xffffffffu, c_new, 1);
+            if (lane < nc) s_c[lane] = c_new;
+            if (lane + 1 < nc) s_b[lane] = __fmul_rn(__fadd_rn(c_new, c_next), 0.5f);
+            if (lane == 0 && shift_of < kFitShiftThreshold) s_converged = 1;
+        }
+        __syncthreads();
+    }
+    if (tid < nc) state->centroids[tid] = s_c[tid];
+    if (tid < nc - 1) state->boundaries[tid] = s_b[tid];
+    if (tid == 0) {
+        state->iterations_run += it;
+        state->converged = s_converged;
+        state->go_over_all = s_stop;
+    }
+}
 
 __global__ void __launch_bounds__(kFitThreads) fit_partial_kernel(const float* __restrict__ data, long n_values,
                                                                    const FitState* __restrict__ state, double* __restrict__ part_sum,
@@ -185,31 +423,71 @@ int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, c
         TQ_CUDA(cudaGetDevice(&dev));
         TQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         TQ_REQUIRE(n < (1L << 40), "tq_codebook_fit: at most 2^40 samples");
-        const long chunks = (n + (1L << 14) - 1) >> 14;
-        const int blocks = static_cast<int>(std::min<long>(chunks, 2L * sms));
-        const size_t smem = (sizeof(double) + sizeof(unsigned int)) * kFitMaxBins * kFitThreads;
-        static bool configured[64] = {false};
-        if (dev < 0 || dev >= 64 || !configured[dev]) {
-            TQ_CUDA(cudaFuncSetAttribute(fit_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            if (dev >= 0 && dev < 64) configured[dev] = true;
-        }
-        FitState* d_state = nullptr;
-        double* d_sum = nullptr;
-        unsigned long long* d_cnt = nullptr;
-        TQ_CUDA(cudaMallocAsync(&d_state, sizeof(FitState), stream));
-        TQ_CUDA(cudaMallocAsync(&d_sum, sizeof(double) * kFitMaxBins * blocks, stream));
-        TQ_CUDA(cudaMallocAsync(&d_cnt, sizeof(unsigned long long) * kFitMaxBins * blocks, stream));
+        DeviceBuffer state_buf;
+        state_buf.reserve(sizeof(FitState), stream);
+        FitState* const d_state = state_buf.as<FitState>();
         TQ_CUDA(cudaMemcpyAsync(d_state, &h, sizeof h, cudaMemcpyHostToDevice, stream));
-        for (int it = 0; it < iterations; ++it) {
-            fit_partial_kernel<<<blocks, kFitThreads, smem, stream>>>(d_data, n, d_state, d_sum, d_cnt);
-            fit_update_kernel<<<1, 32, 0, stream>>>(d_state, d_sum, d_cnt, blocks);
+        auto read_state = [&] {
+            TQ_CUDA(cudaMemcpyAsync(&h, d_state, sizeof h, cudaMemcpyDeviceToHost, stream));
+            TQ_CUDA(cudaStreamSynchronize(stream));
+        };
+        h.go_over_all = 1;
+        DeviceBuffer bucket_buf, sorted_buf;
+        if (n < (1L << 31)) {
+            // Mantissa bits of a bucket's key: a few hundred values in the buckets where boundaries lie (16.8 M normal samples:
+            // 11 bits, about 600), between 2^12 and 2^21 buckets.
+            int log2_n = 0;
+            while ((1L << log2_n) < n) ++log2_n;
+            const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13)), shift = 32 - key_bits, n_buckets = 1 << key_bits;
+            const int n_groups = n_buckets / kFitGroup;
+            bucket_buf.reserve(static_cast<size_t>(n_buckets) * (3 * 4 + 8) + static_cast<size_t>(n_groups) * (8 + 8 + 4), stream);
+            sorted_buf.reserve(static_cast<size_t>(n) * 4, stream);
+            long long* const d_sum = bucket_buf.as<long long>();
+            long long* const d_group_sum = d_sum + n_buckets;
+            long long* const d_before = d_group_sum + n_groups;
+            unsigned int* const d_count = reinterpret_cast<unsigned int*>(d_before + n_groups);
+            unsigned int* const d_offset = d_count + n_buckets;
+            unsigned int* const d_cursor = d_offset + n_buckets;
+            unsigned int* const d_group = d_cursor + n_buckets;
+            float* const d_sorted = sorted_buf.as<float>();
+            TQ_CUDA(cudaMemsetAsync(d_count, 0, static_cast<size_t>(n_buckets) * 4, stream));
+            const unsigned int un = static_cast<unsigned int>(n);
+            const int grid = static_cast<int>(std::min<long>((n + 1023) / 1024, 16L * sms));
+            fit_count_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_count, d_state);
+            fit_groups_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group);
+            fit_offsets_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group, d_offset, d_cursor);
+            fit_scatter_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_cursor, d_sorted);
+            fit_sums_kernel<<<n_groups, 256, 0, stream>>>(d_sorted, d_count, d_offset, log2_n, d_state, d_sum, d_group_sum);
+            fit_iterate_kernel<<<1, 1024, 0, stream>>>(d_sorted, un, d_count, d_offset, d_sum, d_group_sum, n_groups, d_before, shift, log2_n,
+                                                       iterations, d_state);
+            TQ_CUDA(cudaGetLastError());
+            read_state();
         }
-        TQ_CUDA(cudaGetLastError());
-        TQ_CUDA(cudaMemcpyAsync(&h, d_state, sizeof h, cudaMemcpyDeviceToHost, stream));
-        TQ_CUDA(cudaFreeAsync(d_state, stream));
-        TQ_CUDA(cudaFreeAsync(d_sum, stream));
-        TQ_CUDA(cudaFreeAsync(d_cnt, stream));
-        TQ_CUDA(cudaStreamSynchronize(stream));
+        if (h.go_over_all && !h.converged && h.iterations_run < iterations) {
+            const long chunks = (n + (1L << 14) - 1) >> 14;
+            const int blocks = static_cast<int>(std::min<long>(chunks, 2L * sms));
+            const size_t smem = (sizeof(double) + sizeof(unsigned int)) * kFitMaxBins * kFitThreads;
+            static bool configured[64] = {false};
+            if (dev < 0 || dev >= 64 || !configured[dev]) {
+                TQ_CUDA(cudaFuncSetAttribute(fit_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+                if (dev >= 0 && dev < 64) configured[dev] = true;
+            }
+            DeviceBuffer part_buf;
+            part_buf.reserve((sizeof(double) + sizeof(unsigned long long)) * kFitMaxBins * blocks, stream);
+            double* const d_psum = part_buf.as<double>();
+            unsigned long long* const d_pcnt = reinterpret_cast<unsigned long long*>(d_psum + kFitMaxBins * blocks);
+            // all pairs of launches are enqueued at once; those after convergence return at their first instruction
+            for (int it = h.iterations_run; it < iterations; ++it) {
+                fit_partial_kernel<<<blocks, kFitThreads, smem, stream>>>(d_data, n, d_state, d_psum, d_pcnt);
+                fit_update_kernel<<<1, 32, 0, stream>>>(d_state, d_psum, d_pcnt, blocks);
+            }
+            TQ_CUDA(cudaGetLastError());
+            read_state();
+            part_buf.set_idle();
+        }
+        state_buf.set_idle();
+        bucket_buf.set_idle();
+        sorted_buf.set_idle();
         run = h.iterations_run;
     }
     for (int i = 0; i < nc; ++i) centroids_out[i] = h.centroids[i];

@@ -429,9 +429,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
                 for (int h = 0; h < 16; ++h) {  // codes 2h, 2h + 1 -> column h
                     const uint32_t word = w[h >> 1];
                     const int b0 = (h & 1) * 2;  // bytes b0, b0 + 1 of the word
-                    const uint32_t i0 = b0 == 0 ? (word << 7) : (word >> 9);
-                    const uint32_t i1 = b0 == 0 ? (word >> 1) : (word >> 17);
-                    packed[h] = __byte_perm(lut_load((i0 & (255u << 7)) | lane_c), lut_load((i1 & (255u << 7)) | lane_c), 0x5410);
+                    // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
+                    packed[h] = __byte_perm(lut_load(__dp4a(word, 128u << (8 * b0), lane_c)), lut_load(__dp4a(word, 128u << (8 * b0 + 8), lane_c)), 0x5410);
                 }
                 // the slot must have been read by the MMAs of its previous stage
                 if (half == 0 && use > 0 && !bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag)) {

@@ -67,19 +67,42 @@ __device__ __forceinline__ float flip_unless(float v, uint32_t word, int j) {
     return __uint_as_float(__float_as_uint(v) ^ ((~word << (31 - j)) & 0x80000000u));
 }
 
+// The code of a rotated, scaled value x and the residual x - centroid.  The boundaries are the centroids' midpoints: +-t1,
+// +-t2, +-t3 and zero, and a code is the number of boundaries below the value.  For x > 0 that is 4 + #{t < |x|}, otherwise
+// 3 - #{t <= |x|}; one more unit in the last place on |x| turns the second comparison into the first.
+__device__ __forceinline__ uint32_t code_of(float x, float& residual) {
+    const uint32_t t1 = __float_as_uint(__fmul_rn(__fadd_rn(kMag0, kMag1), 0.5f));
+    const uint32_t t2 = __float_as_uint(__fmul_rn(__fadd_rn(kMag1, kMag2), 0.5f));
+    const uint32_t t3 = __float_as_uint(__fmul_rn(__fadd_rn(kMag2, kMag3), 0.5f));
+    const bool pos = x > 0.0f;
+    const uint32_t a = (__float_as_uint(x) & 0x7fffffffu) + (pos ? 0u : 1u);
+    const uint32_t m = (a > t1 ? 1u : 0u) + (a > t2 ? 1u : 0u) + (a > t3 ? 1u : 0u);
+    const float mag = a > t3 ? kMag3 : (a > t2 ? kMag2 : (a > t1 ? kMag1 : kMag0));
+    residual = __fsub_rn(x, pos ? mag : -mag);
+    return pos ? 4u + m : 3u - m;
+}
+
 struct KvSegments {
     KvSegment seg[kKvMaxSegments];
 };
 
+// Eight 3-bit fields at nibble positions (low or high half of a word) to four bytes.
+__device__ __forceinline__ uint32_t nibbles_to_bytes(uint32_t four) {
+    four = (four | (four << 8)) & 0x00FF00FFu;
+    return (four | (four << 4)) & 0x0F0F0F0Fu;
+}
+
 // ---- encoder (src/kv_cache.cpp:63-258) ---------------------------------------------------------------
-// Vectors 0 .. n - 1 are the keys, n .. 2 n - 1 the values; segment s takes vec_per_seg vectors.  Bit-exact: the sums of
-// squares run left to right, every other operation is element-wise or the shared butterfly.
+// Eight lanes take a pair of tokens (2p, 2p + 1) of one head, four lanes each; the first half of the units are the keys',
+// the second the values'.  A value byte holds both tokens' codes: the two quads exchange half of their words and each
+// writes four of the eight groups.  A pair of which only one token is appended keeps the other one's bits.
+// Bit-exact: the sums of squares run left to right, every other operation is element-wise or the shared butterfly.
 // Bound: issue slots (about 1100 instructions per lane and vector).  A warp per vector with one lane summing while 31
 // waited took 47 us for 2 x 32768 vectors of 128 (two launches), and a batched variant existed beside it for long
 // appends; four lanes per vector serve both.
 template <int D, typename InT>
-__global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ keys, const InT* __restrict__ values, int n, int heads,
-                                                        int vec_per_seg, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed,
+__global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ keys, const InT* __restrict__ values, int tokens, int n_segs,
+                                                        int heads, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed,
                                                         float scale, float inv_sqrt, int aligned,
                                                         const __grid_constant__ KvSegments tab) {
     constexpr int N = D / 4, W = N / 8;
@@ -96,12 +119,21 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     pdl_wait_release();
 
     const int lane = threadIdx.x & 31, q = lane & 3;
-    const long quad = (static_cast<long>(blockIdx.x) * 128 + threadIdx.x) >> 2;
-    const bool live = quad < 2L * n;
-    const long vec = live ? quad : 2L * n - 1;
-    const bool value = vec >= n;
-    const int gvec = static_cast<int>(value ? vec - n : vec);
-    const InT* const src = (value ? values : keys) + static_cast<size_t>(gvec) * D + q * N;
+    const bool odd = (lane & 4) != 0;
+    const int pairs = tokens / 2 + 1;                       // token pairs that `tokens` tokens can touch
+    const int per_tensor = n_segs * pairs * heads;
+    int unit = static_cast<int>((static_cast<long>(blockIdx.x) * 128 + threadIdx.x) >> 3);
+    const bool in_range = unit < 2 * per_tensor;
+    unit = in_range ? unit : 2 * per_tensor - 1;
+    const bool value = unit >= per_tensor;
+    const int u = value ? unit - per_tensor : unit;
+    const int sidx = u / (pairs * heads), rest = u - sidx * pairs * heads;
+    const int pair = rest / heads, head = rest - pair * heads;
+    const int first = tab.seg[sidx].first;
+    const int token = ((first >> 1) + pair) * 2 + (odd ? 1 : 0), tok = token - first;   // absolute, and within the call
+    const bool live = in_range && tok >= 0 && tok < tokens;
+    const int src_tok = tok < 0 ? 0 : (tok < tokens ? tok : tokens - 1);
+    const InT* const src = (value ? values : keys) + ((static_cast<size_t>(sidx) * tokens + src_tok) * heads + head) * D + q * N;
 
     float v[N];
     if (aligned) {
@@ -128,24 +160,14 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     }
     quad_fwht<N>(v, q);
 
-    // Codes.  The boundaries are the centroids' midpoints: +-t1, +-t2, +-t3 and zero, and a code is the number of
-    // boundaries below the value.  For v > 0 that is 4 + #{t < |v|}, otherwise 3 - #{t <= |v|}; one more unit in the last
-    // place on |v| turns the second comparison into the first.
-    const uint32_t t1 = __float_as_uint(__fmul_rn(__fadd_rn(kMag0, kMag1), 0.5f));
-    const uint32_t t2 = __float_as_uint(__fmul_rn(__fadd_rn(kMag1, kMag2), 0.5f));
-    const uint32_t t3 = __float_as_uint(__fmul_rn(__fadd_rn(kMag2, kMag3), 0.5f));
-    uint32_t words[W];
+    uint32_t words[W];   // nibbles: code, and for a key the residual's sign in bit 3
 #pragma unroll
     for (int w = 0; w < W; ++w) words[w] = 0u;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
         const float x = __fmul_rn(__fmul_rn(v[j], inv_sqrt), scale);
-        const bool pos = x > 0.0f;
-        const uint32_t a = (__float_as_uint(x) & 0x7fffffffu) + (pos ? 0u : 1u);
-        const uint32_t m = (a > t1 ? 1u : 0u) + (a > t2 ? 1u : 0u) + (a > t3 ? 1u : 0u);
-        uint32_t nib = pos ? 4u + m : 3u - m;
-        const float mag = a > t3 ? kMag3 : (a > t2 ? kMag2 : (a > t1 ? kMag1 : kMag0));
-        const float r = __fsub_rn(x, pos ? mag : -mag);
+        float r;
+        uint32_t nib = code_of(x, r);
         v[j] = r;
         if (!value) {
             const uint32_t w = sign_word(s_sign[2], j);
@@ -155,20 +177,48 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
         words[j / 8] |= nib << (4 * (j & 7));
     }
     const float rnorm = __fsqrt_rn(quad_square_sum<N>(v, lane));   // of the residual; only the keys keep it
-    if (!live) return;
 
-    const int sidx = gvec / vec_per_seg, rest = gvec - sidx * vec_per_seg;
-    const int tok = rest / heads, head = rest - tok * heads;
-    const int token = tab.seg[sidx].first + tok, slot = token & (kKvTile - 1);
+    // The half of the words that the other quad writes, for the half of its words that this one writes (values).  A
+    // group is N / 2 dims; D = 32 has half a word in it.
+    constexpr int GW = W >= 2 ? W / 2 : 1;   // nibble words of a group
+    uint32_t own[GW], other[GW];
+#pragma unroll
+    for (int w = 0; w < GW; ++w) {
+        const uint32_t lo = W >= 2 ? words[w] : words[0] & 0xFFFFu, hi = W >= 2 ? words[(GW + w) % W] : words[0] >> 16;
+        own[w] = odd ? hi : lo;
+        other[w] = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 4);
+    }
+    const bool other_live = __shfl_xor_sync(0xffffffffu, live ? 1 : 0, 4) != 0;
+    if (!live && !(value && other_live)) return;
+
+    const int slot = token & (kKvTile - 1);
     unsigned char* const block = tab.seg[sidx].base + (static_cast<size_t>(token / kKvTile) * heads + head) * B::kBytes;
-    if (value && D == 128) {
-        uint2 w01;
-        w01.x = words[0] | ((words[W - 1] & 0x11111111u) << 3);
-        w01.y = words[1 % W] | ((words[W - 1] & 0x22222222u) << 2);
-        *reinterpret_cast<uint2*>(kv_value01(block, slot, q)) = w01;
-        *kv_value2(block, slot, q) = words[2 % W] | ((words[W - 1] & 0x44444444u) << 1);
+    if (value) {
+        const bool even_live = odd ? other_live : live, odd_live = odd ? live : other_live;
+        const int g = 2 * q + (odd ? 1 : 0);
+        uint32_t bytes[2 * GW];   // a byte per dim: the even token's code, the odd one's above it
+#pragma unroll
+        for (int w = 0; w < GW; ++w) {
+            const uint32_t e = (even_live ? (odd ? other[w] : own[w]) : 0u), o = (odd_live ? (odd ? own[w] : other[w]) : 0u);
+            bytes[2 * w] = nibbles_to_bytes(e & 0xFFFFu) | (nibbles_to_bytes(o & 0xFFFFu) << 3);
+            bytes[2 * w + 1] = nibbles_to_bytes(e >> 16) | (nibbles_to_bytes(o >> 16) << 3);
+        }
+        auto put = [&](uint32_t* p, uint32_t w, int k) { *p = even_live ? w : (*p & ~kv_odd_bits(D, k)) | (w & kv_odd_bits(D, k)); };
+        if constexpr (D == 128) {
+            const uint32_t spare = bytes[3];
+            put(kv_value01(block, slot >> 1, g), bytes[0] | kv_spare_bits(spare, 0), 0);
+            put(kv_value01(block, slot >> 1, g) + 1, bytes[1] | kv_spare_bits(spare, 1), 1);
+            put(kv_value2(block, slot >> 1, g), bytes[2] | kv_spare_bits(spare, 2), 2);
+        } else {
+            uint32_t* const dst = kv_value_row(block, D, slot >> 1, g);
+#pragma unroll
+            for (int w = 0; w < (W >= 2 ? 2 * GW : 1); ++w) put(dst + w, bytes[w], 0);
+        }
     } else {
-        uint32_t* const dst = reinterpret_cast<uint32_t*>(block + (value ? B::kValueOff : 0)) + slot * (D / 8) + q * W;
+        uint32_t* const dst = reinterpret_cast<uint32_t*>(block) + slot * (D / 8) + q * W;
+#pragma unroll
+        for (int w = 0; w < W; ++w)   // code, sign, code, sign -> code, code, sign, sign
+            words[w] = (words[w] & 0x87878787u) | ((words[w] >> 1) & 0x38383838u) | ((words[w] << 3) & 0x40404040u);
         if constexpr (W % 4 == 0) {
 #pragma unroll
             for (int w = 0; w < W; w += 4) *reinterpret_cast<uint4*>(dst + w) = make_uint4(words[w], words[w + 1], words[w + 2], words[w + 3]);
@@ -177,10 +227,150 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
             for (int w = 0; w < W; ++w) dst[w] = words[w];
         }
     }
-    if (q == 0) {
+    if (q == 0 && live) {
         float* const norms = reinterpret_cast<float*>(block + B::kNormOff);
-        norms[(value ? kKvTile : 0) + slot] = norm;
-        if (!value) norms[2 * kKvTile + slot] = rnorm;
+        norms[value ? kv_value_norm(slot) : kv_key_norm(slot)] = norm;
+        if (!value) norms[kv_residual_norm(slot)] = rnorm;
+    }
+}
+
+// The same for a decode step's few vectors, where latency counts: eight dims per lane, so a warp (D = 128) takes one token
+// pair of a head.  The quad kernel's straight-line code for 32 dims per lane is 35 KB, which a kernel that runs once
+// fetches from L2 as it goes (8.7 us for 16 sequences of 4 heads); this one's is a quarter of it.  The running sums are one
+// lane's work, from shared memory.
+template <int D, typename InT>
+__global__ void __launch_bounds__(64) kv_encode_few_kernel(const InT* __restrict__ keys, const InT* __restrict__ values, int tokens, int n_segs,
+                                                           int heads, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, float scale,
+                                                           float inv_sqrt, int aligned, const __grid_constant__ KvSegments tab) {
+    constexpr int L = D / 8, kUnits = 64 / (2 * L);   // lanes of a vector, token pairs of a CTA
+    static_assert(2 * L <= 32, "both tokens of a pair in one warp");
+    using B = KvBlock<D>;
+    __shared__ __align__(16) float s_sq[2 * kUnits][D + 4];   // a row per vector, rows four banks apart
+    const int tid = threadIdx.x, l = tid & (L - 1);
+    const bool odd = (tid & L) != 0;
+    const int pairs = tokens / 2 + 1, per_tensor = n_segs * pairs * heads;
+    int unit = static_cast<int>(blockIdx.x) * kUnits + tid / (2 * L);
+    const bool in_range = unit < 2 * per_tensor;
+    unit = in_range ? unit : 2 * per_tensor - 1;
+    const bool value = unit >= per_tensor;
+    const int u = value ? unit - per_tensor : unit;
+    const int sidx = u / (pairs * heads), rest = u - sidx * pairs * heads;
+    const int pair = rest / heads, head = rest - pair * heads;
+    const int first = tab.seg[sidx].first;
+    const int token = ((first >> 1) + pair) * 2 + (odd ? 1 : 0), tok = token - first;   // absolute, and within the call
+    const bool live = in_range && tok >= 0 && tok < tokens;
+    const int src_tok = tok < 0 ? 0 : (tok < tokens ? tok : tokens - 1);
+    const InT* const src = (value ? values : keys) + ((static_cast<size_t>(sidx) * tokens + src_tok) * heads + head) * D + l * 8;
+    uint32_t flips = 0, qflips = 0;   // bit j: dim j's rotation sign, its residual sign (set = +1)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        flips |= sign_is_positive(value ? v_seed : k_seed, static_cast<uint32_t>(l * 8 + j)) ? 1u << j : 0u;
+        qflips |= qjl_sign_is_positive(qjl_seed, static_cast<uint32_t>(l * 8 + j)) ? 1u << j : 0u;
+    }
+    pdl_wait_release();
+
+    float v[8];
+    if (aligned) {
+        constexpr int kPer = 16 / static_cast<int>(sizeof(InT));
+#pragma unroll
+        for (int i = 0; i < 8 / kPer; ++i) {
+            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + i);
+            const InT* e = reinterpret_cast<const InT*>(&raw);
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) v[i * kPer + j] = as_f32<InT>(e[j]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = as_f32<InT>(src[j]);
+    }
+    float* const row = s_sq[tid / L];
+    const int lead = tid & 31 & ~(L - 1);   // the vector's first lane
+    auto square_sum = [&] {   // left to right, as in quad_square_sum
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(row + l * 8 + j) =
+                make_float4(__fmul_rn(v[j], v[j]), __fmul_rn(v[j + 1], v[j + 1]), __fmul_rn(v[j + 2], v[j + 2]), __fmul_rn(v[j + 3], v[j + 3]));
+        __syncwarp();
+        float acc = 0.0f;
+        if (l == 0) {
+#pragma unroll 4
+            for (int j = 0; j < D; j += 8) {
+                const float4 a = *reinterpret_cast<const float4*>(row + j), b = *reinterpret_cast<const float4*>(row + j + 4);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, a.x), a.y), a.z), a.w);
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, b.x), b.y), b.z), b.w);
+            }
+        }
+        __syncwarp();
+        return __shfl_sync(0xffffffffu, acc, lead);
+    };
+    const float norm = __fsqrt_rn(square_sum());
+    const float inv_norm = (norm > 1e-10f) ? __fdiv_rn(1.0f, norm) : 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = flip_unless(__fmul_rn(v[j], inv_norm), flips, j);
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2 * h)
+#pragma unroll
+            for (int j = i; j < i + h; ++j) {
+                const float a = v[j], b = v[j + h];
+                v[j] = __fadd_rn(a, b);
+                v[j + h] = __fsub_rn(a, b);
+            }
+#pragma unroll 1
+    for (int m = 1; m < L; m <<= 1) {
+        const bool upper = (l & m) != 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float other = __shfl_xor_sync(0xffffffffu, v[j], m);
+            v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
+        }
+    }
+    // the dims' bytes: keys two codes and their signs each, values one code
+    uint32_t kword = 0, bytes[2] = {0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        float r;
+        const uint32_t c = code_of(__fmul_rn(__fmul_rn(v[j], inv_sqrt), scale), r);
+        v[j] = r;
+        const bool bit = ((qflips >> j) & 1u) ? r > 0.0f : r < 0.0f;
+        kword |= ((c << (3 * (j & 1))) | (bit ? 64u << (j & 1) : 0u)) << (8 * (j >> 1));
+        bytes[j >> 2] |= c << (8 * (j & 3));
+    }
+    const float rnorm = __fsqrt_rn(square_sum());
+    // the other token's codes beside this one's
+    const bool other_live = __shfl_xor_sync(0xffffffffu, live ? 1 : 0, L) != 0;
+    const bool even_live = odd ? other_live : live, odd_live = odd ? live : other_live;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, bytes[w], L);
+        bytes[w] = (even_live ? (odd ? other : bytes[w]) : 0u) | (odd_live ? (odd ? bytes[w] : other) << 3 : 0u);
+    }
+    const uint32_t spare = __shfl_xor_sync(0xffffffffu, bytes[1], 1);   // D = 128: lanes 2g hold words 0 and 1, lanes 2g + 1 word 2 and the spare dims
+    if (!live && !(value && other_live)) return;
+
+    const int slot = token & (kKvTile - 1);
+    unsigned char* const block = tab.seg[sidx].base + (static_cast<size_t>(token / kKvTile) * heads + head) * B::kBytes;
+    if (value) {
+        auto put = [&](uint32_t* p, uint32_t w, int k) { *p = even_live ? w : (*p & ~kv_odd_bits(D, k)) | (w & kv_odd_bits(D, k)); };
+        if constexpr (D == 128) {
+            const int g = l >> 1;
+            if (l & 1) {
+                if (!odd) put(kv_value2(block, slot >> 1, g), bytes[0] | kv_spare_bits(bytes[1], 2), 2);
+            } else {
+                const int k = odd ? 1 : 0;
+                put(kv_value01(block, slot >> 1, g) + k, bytes[k] | kv_spare_bits(spare, k), k);
+            }
+        } else {
+            put(kv_value_row(block, D, slot >> 1, 0) + 2 * l + (odd ? 1 : 0), odd ? bytes[1] : bytes[0], 0);
+        }
+    } else {
+        reinterpret_cast<uint32_t*>(block)[slot * L + l] = kword;
+    }
+    if (l == 0 && live) {
+        float* const norms = reinterpret_cast<float*>(block + B::kNormOff);
+        norms[value ? kv_value_norm(slot) : kv_key_norm(slot)] = norm;
+        if (!value) norms[kv_residual_norm(slot)] = rnorm;
     }
 }
 
@@ -214,22 +404,36 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __r
     const long token = start + tok;
     const int slot = static_cast<int>(token & (kKvTile - 1));
     unsigned char* const block = const_cast<unsigned char*>(base) + (static_cast<size_t>(token / kKvTile) * heads + head) * B::kBytes;
-    uint32_t words[W];
-    if (values && D == 128) {
-        const uint2 w01 = *reinterpret_cast<const uint2*>(kv_value01(block, slot, q));
-        words[0] = w01.x;
-        words[1 % W] = w01.y;
-        words[2 % W] = *kv_value2(block, slot, q);
-        words[W - 1] = kv_value_spare(words[0], words[1 % W], words[2 % W]);
-    } else {
-        const uint32_t* const src = reinterpret_cast<const uint32_t*>(block + (values ? B::kValueOff : 0)) + slot * (D / 8) + q * W;
-#pragma unroll
-        for (int w = 0; w < W; ++w) words[w] = src[w];
-    }
-    const float norm = reinterpret_cast<const float*>(block + B::kNormOff)[(values ? kKvTile : 0) + slot];
     float v[N];
+    if (values) {
+        const int sh = (slot & 1) * 3;
 #pragma unroll
-    for (int j = 0; j < N; ++j) v[j] = s_cent[(words[j / 8] >> (4 * (j & 7))) & 7u][lane];
+        for (int h = 0; h < 2; ++h) {   // this lane's two groups of N / 2 dims
+            const int g = 2 * q + h;
+            if constexpr (D == 128) {
+                const uint2 w01 = *reinterpret_cast<const uint2*>(kv_value01(block, slot >> 1, g));
+                const uint32_t w[3] = {w01.x, w01.y, *kv_value2(block, slot >> 1, g)};
+#pragma unroll
+                for (int j = 0; j < 12; ++j) v[h * 16 + j] = s_cent[(w[j / 4] >> (8 * (j & 3) + sh)) & 7u][lane];
+                const uint32_t spare = kv_value_spare(w[0], w[1], w[2]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[(h * 16 + 12 + j) % N] = s_cent[(spare >> (8 * j + sh)) & 7u][lane];
+            } else {
+                const uint32_t* const src = kv_value_row(block, D, slot >> 1, g);
+#pragma unroll
+                for (int j = 0; j < N / 2; ++j) v[h * (N / 2) + j] = s_cent[(src[j / 4] >> (8 * (j & 3) + sh)) & 7u][lane];
+            }
+        }
+    } else {
+        const uint32_t* const src = reinterpret_cast<const uint32_t*>(block) + slot * (D / 8) + q * W;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const uint32_t x = src[w];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[8 * w + j] = s_cent[(x >> (8 * (j / 2) + 3 * (j & 1))) & 7u][lane];
+        }
+    }
+    const float norm = reinterpret_cast<const float*>(block + B::kNormOff)[values ? kv_value_norm(slot) : kv_key_norm(slot)];
     quad_fwht<N>(v, q);
     __align__(16) __half h[N];
 #pragma unroll
@@ -250,18 +454,19 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __r
 
 // ---- the reference's arrays ------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t stored_code(const unsigned char* block, int dim, int slot, int d, bool value, uint32_t* sign) {
-    const int key_bytes = kKvTile * dim / 2;
-    if (value && dim == 128) {
-        unsigned char* const b = const_cast<unsigned char*>(block);
-        const int q = d >> 5, r = d & 31;
-        const uint32_t w0 = kv_value01(b, slot, q)[0], w1 = kv_value01(b, slot, q)[1], w2 = *kv_value2(b, slot, q);
-        const uint32_t w = r < 8 ? w0 : (r < 16 ? w1 : (r < 24 ? w2 : kv_value_spare(w0, w1, w2)));
-        return (w >> (4 * (r & 7))) & 7u;
+    unsigned char* const b = const_cast<unsigned char*>(block);
+    if (value) {
+        const int per = dim / 8, g = d / per, r = d - g * per, odd = slot & 1;
+        if (dim == 128) {
+            const uint32_t w0 = kv_value01(b, slot >> 1, g)[0], w1 = kv_value01(b, slot >> 1, g)[1], w2 = *kv_value2(b, slot >> 1, g);
+            const uint32_t w = r < 4 ? w0 : (r < 8 ? w1 : (r < 12 ? w2 : kv_value_spare(w0, w1, w2)));
+            return (w >> (8 * (r & 3) + 3 * odd)) & 7u;
+        }
+        return (kv_value_row(b, dim, slot >> 1, g)[r >> 2] >> (8 * (r & 3) + 3 * odd)) & 7u;
     }
-    const uint32_t* const w = reinterpret_cast<const uint32_t*>(block + (value ? key_bytes : 0)) + slot * (dim / 8);
-    const uint32_t nib = w[d >> 3] >> (4 * (d & 7));
-    if (sign) *sign = (nib >> 3) & 1u;
-    return nib & 7u;
+    const uint32_t byte = block[slot * (dim / 2) + (d >> 1)];
+    if (sign) *sign = (byte >> (6 + (d & 1))) & 1u;
+    return (byte >> (3 * (d & 1))) & 7u;
 }
 
 // One thread per word of the reference's records: key words, value words, sign words, norms.
@@ -295,55 +500,68 @@ __global__ void __launch_bounds__(128) kv_unpack_kernel(const unsigned char* __r
         return;
     }
     const float* const norms = reinterpret_cast<const float*>(block + kv_block_bytes(dim) - 3 * kKvTile * 4);
-    if (out.k_norms) out.k_norms[vec] = norms[slot];
-    if (out.v_norms) out.v_norms[vec] = norms[kKvTile + slot];
-    if (out.qjl_norms) out.qjl_norms[vec] = norms[2 * kKvTile + slot];
+    if (out.k_norms) out.k_norms[vec] = norms[kv_key_norm(slot)];
+    if (out.v_norms) out.v_norms[vec] = norms[kv_value_norm(slot)];
+    if (out.qjl_norms) out.qjl_norms[vec] = norms[kv_residual_norm(slot)];
 }
 
 __device__ __forceinline__ uint32_t array_code(const uint32_t* words, long vec, int wph, int d) {
     return (words[vec * wph + d / 10] >> (3 * (d % 10))) & 7u;
 }
 
-// One thread per word of the storage: key nibbles, value words, and one for the norms.
-__global__ void __launch_bounds__(128) kv_pack_kernel(unsigned char* __restrict__ base, int start, long n_vec, int heads, int dim, KvArrays in) {
-    const int wph = (dim + 9) / 10, qph = dim / 32, kw = dim / 8, vw = dim == 128 ? 4 : dim / 8, per = kw + vw + 1;
+// One thread per (token pair, head) and word of the pair's records: the two tokens' key words, the value words, and one
+// for the norms.  A token outside [start, start + tokens) keeps its bits.
+__global__ void __launch_bounds__(128) kv_pack_kernel(unsigned char* __restrict__ base, int start, int tokens, int heads, int dim, KvArrays in) {
+    const int wph = (dim + 9) / 10, qph = dim / 32, kw = dim / 8, vw = dim == 128 ? 8 : dim / 4, per = 2 * kw + vw + 1;
     const long i = static_cast<long>(blockIdx.x) * 128 + threadIdx.x;
-    const long vec = i / per;
-    if (vec >= n_vec) return;
-    int item = static_cast<int>(i - vec * per);
-    const long tok = vec / heads, token = start + tok;
-    const int head = static_cast<int>(vec - tok * heads), slot = static_cast<int>(token & (kKvTile - 1));
-    unsigned char* const block = base + (static_cast<size_t>(token / kKvTile) * heads + head) * kv_block_bytes(dim);
-    const int key_bytes = kKvTile * dim / 2;
-    if (item < kw) {
+    const long unit = i / per;
+    const int pair0 = start >> 1, pairs = ((start + tokens - 1) >> 1) - pair0 + 1;
+    if (unit >= static_cast<long>(pairs) * heads) return;
+    int item = static_cast<int>(i - unit * per);
+    const int pair = pair0 + static_cast<int>(unit / heads), head = static_cast<int>(unit % heads);
+    auto inside = [&](int odd) { return 2 * pair + odd >= start && 2 * pair + odd < start + tokens; };
+    auto vec_of = [&](int odd) { return static_cast<long>(2 * pair + odd - start) * heads + head; };
+    const int slot = (2 * pair) & (kKvTile - 1);
+    unsigned char* const block = base + (static_cast<size_t>(2 * pair / kKvTile) * heads + head) * kv_block_bytes(dim);
+    if (item < 2 * kw) {
+        const int odd = item >= kw ? 1 : 0, w = item - odd * kw;
+        if (!inside(odd)) return;
+        const long vec = vec_of(odd);
         uint32_t word = 0;
         for (int k = 0; k < 8; ++k) {
-            const int d = item * 8 + k;
+            const int d = w * 8 + k;
             const uint32_t sign = (in.qjl_words[vec * qph + (d >> 5)] >> (d & 31)) & 1u;
-            word |= (array_code(in.k_words, vec, wph, d) | (sign << 3)) << (4 * k);
+            word |= ((array_code(in.k_words, vec, wph, d) << (3 * (k & 1))) | (sign << (6 + (k & 1)))) << (8 * (k >> 1));
         }
-        reinterpret_cast<uint32_t*>(block)[slot * kw + item] = word;
+        reinterpret_cast<uint32_t*>(block)[(slot + odd) * kw + w] = word;
         return;
     }
-    item -= kw;
+    item -= 2 * kw;
     if (item < vw) {
-        if (dim == 128) {
-            uint32_t w[4] = {0, 0, 0, 0};
-            for (int k = 0; k < 32; ++k) w[k >> 3] |= array_code(in.v_words, vec, wph, item * 32 + k) << (4 * (k & 7));
-            kv_value01(block, slot, item)[0] = w[0] | ((w[3] & 0x11111111u) << 3);
-            kv_value01(block, slot, item)[1] = w[1] | ((w[3] & 0x22222222u) << 2);
-            *kv_value2(block, slot, item) = w[2] | ((w[3] & 0x44444444u) << 1);
-        } else {
-            uint32_t word = 0;
-            for (int k = 0; k < 8; ++k) word |= array_code(in.v_words, vec, wph, item * 8 + k) << (4 * k);
-            reinterpret_cast<uint32_t*>(block + key_bytes)[slot * kw + item] = word;
+        // a packed group of 16 dims (three words), or four dims (one word)
+        const int d0 = dim == 128 ? item * 16 : item * 4, n_words = dim == 128 ? 3 : 1;
+        uint32_t w[4] = {0, 0, 0, 0};
+        for (int odd = 0; odd < 2; ++odd) {
+            if (!inside(odd)) continue;
+            for (int k = 0; k < (dim == 128 ? 16 : 4); ++k) w[k >> 2] |= array_code(in.v_words, vec_of(odd), wph, d0 + k) << (8 * (k & 3) + 3 * odd);
+        }
+        for (int k = 0; k < n_words; ++k) {
+            if (dim == 128) w[k] |= kv_spare_bits(w[3], k);
+            const uint32_t keep = (inside(1) ? 0u : kv_odd_bits(dim, k)) | (inside(0) ? 0u : ~kv_odd_bits(dim, k));
+            uint32_t* dst;
+            if (dim == 128) dst = k < 2 ? kv_value01(block, slot >> 1, item) + k : kv_value2(block, slot >> 1, item);
+            else dst = kv_value_row(block, dim, slot >> 1, 0) + item;
+            *dst = (*dst & keep) | (w[k] & ~keep);
         }
         return;
     }
     float* const norms = reinterpret_cast<float*>(block + kv_block_bytes(dim) - 3 * kKvTile * 4);
-    norms[slot] = in.k_norms[vec];
-    norms[kKvTile + slot] = in.v_norms[vec];
-    norms[2 * kKvTile + slot] = in.qjl_norms[vec];
+    for (int odd = 0; odd < 2; ++odd) {
+        if (!inside(odd)) continue;
+        norms[kv_key_norm(slot + odd)] = in.k_norms[vec_of(odd)];
+        norms[kv_value_norm(slot + odd)] = in.v_norms[vec_of(odd)];
+        norms[kv_residual_norm(slot + odd)] = in.qjl_norms[vec_of(odd)];
+    }
 }
 
 }  // namespace
@@ -361,23 +579,40 @@ __global__ void __launch_bounds__(128) kv_pack_kernel(unsigned char* __restrict_
 void launch_kv_encode(const void* keys, const void* values, bool is_f16, int tokens_per_seg, int heads, int dim, uint32_t k_seed,
                       uint32_t v_seed, uint32_t qjl_seed, const KvSegment* segs, int n_segs, cudaStream_t stream) {
     TQ_REQUIRE(n_segs >= 1 && n_segs <= kKvMaxSegments, "kv encode: 1..32 segments per launch");
-    const long n = static_cast<long>(tokens_per_seg) * heads * n_segs;
-    if (n == 0) return;
-    TQ_REQUIRE(n < (1L << 31), "kv encode: too many vectors for one call");
+    if (tokens_per_seg == 0) return;
+    const long units = 2L * n_segs * (tokens_per_seg / 2 + 1) * heads;   // token pairs of a head, keys and values
+    TQ_REQUIRE(units < (1L << 28), "kv encode: too many vectors for one call");
     KvSegments tab{};
     for (int i = 0; i < n_segs; ++i) tab.seg[i] = segs[i];
     const float scale = std::sqrt(static_cast<float>(dim));             // src/kv_cache.cpp:72
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(dim));   // src/rotation.cpp:301
     const int aligned = reinterpret_cast<uintptr_t>(keys) % 16 == 0 && reinterpret_cast<uintptr_t>(values) % 16 == 0 ? 1 : 0;
-    const dim3 grid(static_cast<unsigned>((2 * n * 4 + 127) / 128));
+    // Few vectors: eight dims per lane, while that still spreads over the SMs in one wave (measured at D = 128).
+    if (dim <= 128 && units <= 1184) {
+        const dim3 few(static_cast<unsigned>((units * 2 * (dim / 8) + 63) / 64));
+#define TQ_ENC_FEW(DV)                                                                                                                \
+    case DV:                                                                                                                          \
+        if (is_f16)                                                                                                                   \
+            launch_pdl(kv_encode_few_kernel<DV, __half>, few, dim3(64), 0, stream, static_cast<const __half*>(keys),                   \
+                       static_cast<const __half*>(values), tokens_per_seg, n_segs, heads, k_seed, v_seed, qjl_seed, scale, inv_sqrt,  \
+                       aligned, tab);                                                                                                 \
+        else                                                                                                                          \
+            launch_pdl(kv_encode_few_kernel<DV, float>, few, dim3(64), 0, stream, static_cast<const float*>(keys),                    \
+                       static_cast<const float*>(values), tokens_per_seg, n_segs, heads, k_seed, v_seed, qjl_seed, scale, inv_sqrt,   \
+                       aligned, tab);                                                                                                 \
+        return;
+        switch (dim) { TQ_ENC_FEW(32) TQ_ENC_FEW(64) TQ_ENC_FEW(128) }
+#undef TQ_ENC_FEW
+    }
+    const dim3 grid(static_cast<unsigned>((units * 8 + 127) / 128));
 #define TQ_ENC(DV)                                                                                                                    \
     if (is_f16)                                                                                                                       \
         launch_pdl(kv_encode_kernel<DV, __half>, grid, dim3(128), 0, stream, static_cast<const __half*>(keys),                        \
-                   static_cast<const __half*>(values), static_cast<int>(n), heads, tokens_per_seg * heads, k_seed, v_seed, qjl_seed,  \
+                   static_cast<const __half*>(values), tokens_per_seg, n_segs, heads, k_seed, v_seed, qjl_seed,           \
                    scale, inv_sqrt, aligned, tab);                                                                                    \
     else                                                                                                                              \
         launch_pdl(kv_encode_kernel<DV, float>, grid, dim3(128), 0, stream, static_cast<const float*>(keys),                          \
-                   static_cast<const float*>(values), static_cast<int>(n), heads, tokens_per_seg * heads, k_seed, v_seed, qjl_seed,   \
+                   static_cast<const float*>(values), tokens_per_seg, n_segs, heads, k_seed, v_seed, qjl_seed,           \
                    scale, inv_sqrt, aligned, tab);
     TQ_D_SWITCH(dim, TQ_ENC)
 #undef TQ_ENC
@@ -404,10 +639,10 @@ void launch_kv_unpack(const unsigned char* base, int start, int tokens, int head
 }
 
 void launch_kv_pack(unsigned char* base, int start, int tokens, int heads, int dim, const KvArrays& in, cudaStream_t stream) {
-    const long n = static_cast<long>(tokens) * heads;
-    if (n == 0) return;
-    const long threads = n * (dim / 8 + (dim == 128 ? 4 : dim / 8) + 1);
-    kv_pack_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, stream>>>(base, start, n, heads, dim, in);
+    if (tokens == 0) return;
+    const long pairs = ((start + tokens - 1) >> 1) - (start >> 1) + 1;
+    const long threads = pairs * heads * (2 * (dim / 8) + (dim == 128 ? 8 : dim / 4) + 1);
+    kv_pack_kernel<<<static_cast<unsigned>((threads + 127) / 128), 128, 0, stream>>>(base, start, tokens, heads, dim, in);
     TQ_CUDA(cudaGetLastError());
 }
 
