@@ -109,6 +109,39 @@ __host__ __device__ __forceinline__ size_t code_offset(long row, int col, size_t
            (static_cast<size_t>(row) & 15) * kCodeTileCols + (static_cast<size_t>(col) & 63);
 }
 
+// The butterfly stages of a WHT block that a warp holds in chunks of 256 columns, lane l the columns 8 l .. 8 l + 7 of
+// each: signs, the stages below 8 in the lane and those of 8 .. 128 (as far as the block goes) between lanes, in the order
+// and pairing of warp_fwht.  `col` = the lane's first column of the chunk.  The stages above 128 are the caller's, between
+// chunks.
+__device__ __forceinline__ void rotate_chunk(float (&v)[8], const uint4& raw, uint32_t seed, uint32_t col, int block, int lane, unsigned live) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __half2 h2 = *reinterpret_cast<const __half2*>(&w[j]);
+        v[2 * j] = __low2float(h2) * sign_value(seed, (col + 2 * j) & static_cast<uint32_t>(block - 1));
+        v[2 * j + 1] = __high2float(h2) * sign_value(seed, (col + 2 * j + 1) & static_cast<uint32_t>(block - 1));
+    }
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2 * h)
+#pragma unroll
+            for (int j = i; j < i + h; ++j) {
+                const float a = v[j], b = v[j + h];
+                v[j] = __fadd_rn(a, b);
+                v[j + h] = __fsub_rn(a, b);
+            }
+    const int lanes = block < 256 ? block >> 3 : 32;
+    for (int m = 1; m < lanes; m <<= 1) {
+        const bool upper = (lane & m) != 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float o = __shfl_xor_sync(live, v[j], m);
+            v[j] = upper ? __fsub_rn(o, v[j]) : __fadd_rn(v[j], o);
+        }
+    }
+}
+
 // Report a failure from a kernel.  The status word may live in page-locked HOST memory (so that
 // the host reads it without a copy): a plain store followed by a system-scope fence, no atomic.
 // Programmatic dependent launch for the small kernels of a decode step: launched with the attribute, a kernel's CTAs are

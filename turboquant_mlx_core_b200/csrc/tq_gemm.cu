@@ -18,8 +18,13 @@
 //   A pipeline stage is 128 K columns (two 64-column K blocks), the ring has up to four stages.
 //   warps 0-15 producers in two groups of eight; group g takes the stages g, g + 2, ...: codes HBM ->
 //              registers (two of the group's stages ahead) -> lookup (lane-private fp16 table in
-//              shared memory) -> weight tile in TENSOR memory (tcgen05.st; lane = row, 64 columns of
-//              fp16 pairs per stage)
+//              shared memory) -> weight tile in TENSOR memory (tcgen05.st, 64 columns of fp16 pairs per
+//              stage).  The store's 16x256b shape takes registers in the fragment order (lane / 4 = row,
+//              lane % 4 = columns), so a code load of a warp is 512 contiguous bytes; with a row per lane
+//              (32x32b) it touched 32 lines of 64 bytes, and the first-level cache, which the lookups
+//              also load with a wavefront per 32 weights, was the bound (5120 x 55296: 110 -> 89 us at 32
+//              rows, 644 -> 547 us at 1024).  The K order this gives is free: the rotation kernels write
+//              the activations in the same one (k_position).
 //   warp 17    activation tiles: the rotation kernel stores xrot in operand-tile order, so a K block
 //              of a tile is one contiguous bulk copy (cp.async.bulk, mbarrier complete_tx) of 128
 //              bytes per activation row of the tile
@@ -135,15 +140,22 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
         : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
-// 16 consecutive 32-bit columns of this thread's tensor-memory lane.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+// 16 lanes x 32 columns, four blocks of 8 columns side by side: registers 4 i + (0, 1) are row lane / 4, columns
+// 8 i + 2 (lane % 4) and the next; registers 4 i + (2, 3) the same columns of row lane / 4 + 8.
+__device__ __forceinline__ void tmem_st_16x256b(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], "
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         :
         : "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
           "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
+}
+// Codes are read once per 256 activation rows: they pass by the first-level cache.
+__device__ __forceinline__ uint4 load_codes16(const uint8_t* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 // Waits for this thread's tensor-memory stores and orders them before the barrier arrival that follows.
 __device__ __forceinline__ void tmem_st_publish() {
@@ -167,11 +179,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Where column c of a 64-column K block stands in the operands.  A producer lane holds 16 consecutive codes of a row
+// (columns 16 q .. of lane quarter q) and the tensor-memory store takes four fp16 of every lane for each block of 16: the
+// q-th four of block i are columns 16 q + 4 i and on.  Any order does as long as both operands share it.
+__host__ __device__ constexpr int k_position(int c) { return 16 * ((c >> 2) & 3) + 4 * (c >> 4) + (c & 3); }
+
 // ---- activation rotation to fp16, written in operand-tile order --------------------------------
 // One warp per (plane, row, WHT block): xrot = fp16( FWHT(sign o fp16(x)) / sqrt(bs) ).
 // Output layout: [plane][row tile of 256][K block of 64][32 KB tile], the tile being exactly the
 // shared-memory image the GEMM wants (8 x 8 core matrices: [row group 32][core column 8][row 8][8 fp16]),
-// so that a CTA fetches an activation tile with ONE contiguous bulk copy.  Rows past the last
+// so that a CTA fetches an activation tile with ONE contiguous bulk copy.  The order of the 64 columns of a K block is
+// the one in which the producers' tensor-memory store lays the weights down (k_position).  Rows past the last
 // one are left as they are: they only feed accumulator columns that are never stored.
 template <int E>
 __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
@@ -179,7 +197,7 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
                                                               uint32_t seed_r, float inv_sqrt) {
     pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
     constexpr int BS = 32 * E;
-    constexpr int V = E < 8 ? E : 8;  // halves per vector store (one core-matrix row holds 8)
+    constexpr int V = E < 4 ? E : 4;  // halves per vector store (k_position keeps groups of four together)
     const int lane = threadIdx.x & 31;
     const long blocks_per_row = in / BS;
     const long total = static_cast<long>(n_planes) * rows * blocks_per_row;
@@ -201,27 +219,27 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
 #pragma unroll
     for (int j0 = 0; j0 < E; j0 += V) {
         const long col = blk * BS + lane * E + j0;
-        const long kb = col / kBlockK, cin = col - kb * kBlockK;
+        const long kb = col / kBlockK, pos = k_position(static_cast<int>(col - kb * kBlockK));
         const long tile = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane + kb;
-        __half* dst = xrot + tile * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (cin >> 3)) * 8 + (rin & 7)) * 8 + (cin & 7);
-        __align__(16) __half h[V];
+        __half* dst = xrot + tile * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (pos >> 3)) * 8 + (rin & 7)) * 8 + (pos & 7);
+        __align__(8) __half h[V];
 #pragma unroll
         for (int j = 0; j < V; ++j) h[j] = __float2half_rn(v[j0 + j] * inv_sqrt);
-        if constexpr (V == 8) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
-        else if constexpr (V == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
+        if constexpr (V == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
         else if constexpr (V == 2) *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(h);
         else dst[0] = h[0];
     }
 }
 
-// The same for WHT blocks of up to 256 columns, with 16-byte accesses: a warp takes 256 columns
-// of one row, lane l the 8 columns 8l..8l+7 (one core-matrix row of the output tile); butterfly
-// stages below 8 stay in the lane, the rest are lane exchanges (the add tree of warp_fwht).  The
-// 8 warps of a CTA take 8 consecutive rows, so their stores complete whole 128-byte core matrices.
+// The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of one row (one block of 512 or
+// 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
+// the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
+// a CTA take 8 consecutive rows, so their stores complete whole 128-byte core matrices.
+template <int CHUNKS>
 __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows,
                                                       int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const long groups_per_row = (in + 255) / 256;
+    const long groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
     const long row_groups = (rows + 7) / 8;
     // blockIdx.x -> (plane, column group, group of 8 rows); warp -> row inside the group
     long b = blockIdx.x;
@@ -231,64 +249,72 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
     const int plane = static_cast<int>(b / groups_per_row);
     if (plane >= n_planes) return;
     const long row = rg * 8 + wib;
-    const int col = static_cast<int>(cg) * 256 + 8 * lane;
-    if (row >= rows || col >= in) return;  // in is a multiple of 32 >= block: whole lanes only; exchanges stay inside a block
+    const int col = static_cast<int>(cg) * 256 * CHUNKS + 8 * lane;
+    // in is a multiple of 32 >= block: whole lanes only; exchanges stay inside a block.  (A group of several chunks is a
+    // whole block, all of it inside the row.)
+    if (row >= rows || col >= in) return;
     const uint32_t seed = plane ? seed_r : seed_p;
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(x + row * in + col));
-    const uint32_t xw[4] = {raw.x, raw.y, raw.z, raw.w};
-    float v[8];
+    uint4 raw[CHUNKS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const __half2 h2 = *reinterpret_cast<const __half2*>(&xw[j]);
-        v[2 * j] = __low2float(h2) * sign_value(seed, static_cast<uint32_t>((col + 2 * j) & (block - 1)));
-        v[2 * j + 1] = __high2float(h2) * sign_value(seed, static_cast<uint32_t>((col + 2 * j + 1) & (block - 1)));
-    }
-#pragma unroll
-    for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-        for (int i = 0; i < 8; i += 2 * h)
-#pragma unroll
-            for (int j = i; j < i + h; ++j) {
-                const float a0 = v[j], b0 = v[j + h];
-                v[j] = __fadd_rn(a0, b0);
-                v[j + h] = __fsub_rn(a0, b0);
-            }
+    for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
     // lanes of an incomplete trailing group (in % 256 != 0) have returned: exchange only among the live ones
     const unsigned live = __activemask();
-    for (int m = 1; m < (block >> 3); m <<= 1) {
-        const bool upper = (lane & m) != 0;
+    float v[CHUNKS][8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float o = __shfl_xor_sync(live, v[j], m);
-            v[j] = upper ? __fsub_rn(o, v[j]) : __fadd_rn(v[j], o);
-        }
-    }
+    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], seed, static_cast<uint32_t>(col + 256 * c), block, lane, live);
+#pragma unroll
+    for (int h = 1; h < CHUNKS; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < CHUNKS; i += 2 * h)
+#pragma unroll
+            for (int c = i; c < i + h; ++c)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float a0 = v[c][j], b0 = v[c + h][j];
+                    v[c][j] = __fadd_rn(a0, b0);
+                    v[c + h][j] = __fsub_rn(a0, b0);
+                }
     const long n_row_tiles = (rows + kTileTok - 1) / kTileTok;
     const long kb_per_plane = in / kBlockK;
     const long rt = row / kTileTok, rin = row - rt * kTileTok;
-    const long kb = col / kBlockK, cin = col - kb * kBlockK;
-    const long tile = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane + kb;
-    __half* dst = xrot + tile * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (cin >> 3)) * 8 + (rin & 7)) * 8;
-    __align__(16) __half hv[8];
+    const long tile0 = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane;
+    // A lane's two groups of four columns are 16 positions apart; lane ^ 2 holds the ones next to them.  The lanes swap
+    // one group each, so that every lane stores a whole core-matrix row of 8.
+    const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
+    const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
+    __half* const dst = xrot + tile0 * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (pos >> 3)) * 8 + (rin & 7)) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) hv[j] = __float2half_rn(v[j] * inv_sqrt);
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(hv);
+    for (int c = 0; c < CHUNKS; ++c) {
+        uint2 group[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const __half2 lo = __floats2half2_rn(v[c][4 * j] * inv_sqrt, v[c][4 * j + 1] * inv_sqrt);
+            const __half2 hi = __floats2half2_rn(v[c][4 * j + 2] * inv_sqrt, v[c][4 * j + 3] * inv_sqrt);
+            group[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+        const uint2 keep = odd ? group[1] : group[0], give = odd ? group[0] : group[1];
+        const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
+        const uint4 row8 = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
+        *reinterpret_cast<uint4*>(dst + static_cast<long>((col + 256 * c) / kBlockK) * (kTileTok * kBlockK)) = row8;
+    }
 }
+template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
                                                                    int in, long rows, int n_planes, int block,
                                                                    uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
     pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
-    rotate_rows_wide_body(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt);
+    rotate_rows_wide_body<CHUNKS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt);
 }
 // The same rows rotated for several matrices at once (their own seeds and destinations): blockIdx.y = matrix.
 struct RotateGroupArgs {
     __half* xrot[4];
     uint32_t seed_p[4], seed_r[4];
 };
+template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const RotateGroupArgs g, int in,
                                                                          long rows, int n_planes, int block, float inv_sqrt) {
     pdl_wait_release();
-    rotate_rows_wide_body(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt);
+    rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt);
 }
 
 struct GemmArgs {
@@ -383,13 +409,16 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
         // column, 128 K columns).  A warp may touch lanes 32 * (warp % 4) .. + 31.  The 16 producer
         // warps form two groups of eight (warp / 8); inside a group warp w takes the rows of lane
         // quarter w % 4 and the K block (w / 4) % 2 of the stage; group g dequantises the stages g,
-        // g + 2, ...  A thread turns the 64 codes of its row and K block into 32 columns.
-        const int ar = 32 * (warp & 3) + lane;       // row inside the tile
+        // g + 2, ...  A thread turns 64 codes, 16 of each of four rows, into fp16 pairs.
         const int sub = (warp >> 2) & 1;             // which K block of the stage
         const int grp = warp >> 3;
-        const int grow = min(row0 + ar, p.out - 1);  // rows past the matrix repeat the last row (never stored)
-        // a row's 64 columns of K block kb are 64 contiguous bytes of code tile (row / 16, kb)
-        const uint8_t* code_ptr = p.codes + code_offset(grow, 0, code_tiles_per_row(p.in));
+        // The warp's rows are two code tiles of 16 x 64 bytes; lane (g, q) takes bytes 16 q .. of rows g and g + 8 of each:
+        // a load of the warp is 512 contiguous bytes.  Tiles past the matrix repeat the last one (never stored).
+        const int last_tile = (p.out - 1) >> 4, tile0 = (row0 >> 4) + 2 * (warp & 3);
+        const size_t tile_row_bytes = static_cast<size_t>(code_tiles_per_row(p.in)) * kCodeTileBytes;
+        const uint8_t* const code_lane = p.codes + (lane >> 2) * 64 + 16 * (lane & 3);
+        const uint8_t* const code_ptr[2] = {code_lane + static_cast<size_t>(min(tile0, last_tile)) * tile_row_bytes,
+                                            code_lane + static_cast<size_t>(min(tile0 + 1, last_tile)) * tile_row_bytes};
         const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemAColumn + kTmemASubCols * static_cast<uint32_t>(sub);
 
         // Codes are fetched two of the group's stages ahead into registers.  The second plane reads
@@ -398,10 +427,9 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
             const int kb = kSubPerStage * it + sub;
             if (kb < n_kb) {
                 const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
-                const uint4* src = reinterpret_cast<const uint4*>(
-                    code_ptr + static_cast<size_t>(kb_base + kb - plane * kb_per_plane) * kCodeTileBytes);
+                const size_t at = static_cast<size_t>(kb_base + kb - plane * kb_per_plane) * kCodeTileBytes;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = __ldg(src + i);
+                for (int i = 0; i < 4; ++i) c[i] = load_codes16(code_ptr[i >> 1] + at + 512 * (i & 1));
             }
         };
         uint4 c0[4], c1[4], c2[4];
@@ -421,13 +449,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
             const uint32_t st_addr = a_taddr + kTmemAStageCols * static_cast<uint32_t>(slot);
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                // 32 codes -> 32 fp16 -> 16 tensor-memory columns of this thread's lane
+                // code tile `half`: 16 codes of row g and of row g + 8 -> fp16 pairs, word i of a row's four in column block i
                 const uint32_t w[8] = {c0[2 * half].x, c0[2 * half].y, c0[2 * half].z, c0[2 * half].w,
                                        c0[2 * half + 1].x, c0[2 * half + 1].y, c0[2 * half + 1].z, c0[2 * half + 1].w};
                 uint32_t packed[16];
 #pragma unroll
-                for (int h = 0; h < 16; ++h) {  // codes 2h, 2h + 1 -> column h
-                    const uint32_t word = w[h >> 1];
+                for (int h = 0; h < 16; ++h) {
+                    const uint32_t word = w[4 * ((h >> 1) & 1) + (h >> 2)];
                     const int b0 = (h & 1) * 2;  // bytes b0, b0 + 1 of the word
                     // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
                     packed[h] = __byte_perm(lut_load(__dp4a(word, 128u << (8 * b0), lane_c)), lut_load(__dp4a(word, 128u << (8 * b0 + 8), lane_c)), 0x5410);
@@ -439,7 +467,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
                     alive = false;
                 }
                 if (!alive) break;
-                if (have) tmem_st16(st_addr + 16u * half, packed);
+                if (have) tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
             }
             if (!alive) break;
             // every lane waits for its own stores, then one arrival per warp
@@ -666,11 +694,13 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
         const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
         const long n_warps = static_cast<long>(n_planes) * m * (in / static_cast<int>(block));
         const unsigned int grid = static_cast<unsigned int>((n_warps + 3) / 4);
-        const long wide_blocks = static_cast<long>(n_planes) * ((in + 255) / 256) * ((m + 7) / 8);
-        if (block <= 256 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
-            launch_pdl(rotate_rows_f16_wide_kernel, dim3(static_cast<unsigned int>(wide_blocks)), dim3(256), 0, stream, x, xrot, in, m,
-                       n_planes, static_cast<int>(block), seed_p, seed_r, inv_sqrt);
-        } else
+        const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
+        const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8);
+        if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
+            auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_kernel<1> : (wide_cols == 512 ? rotate_rows_f16_wide_kernel<2> : rotate_rows_f16_wide_kernel<4>);
+            launch_pdl(wide, dim3(static_cast<unsigned int>(wide_blocks)), dim3(256), 0, stream, x, xrot, in, m, n_planes,
+                       static_cast<int>(block), seed_p, seed_r, inv_sqrt);
+        } else   // an activation that is not aligned
 #define TQ_ROT16_CASE(EV)                                                                                          \
     case 32 * EV:                                                                                                  \
         launch_pdl(rotate_rows_f16_kernel<EV>, dim3(grid), dim3(128), 0, stream, x, xrot, in, m, n_planes, seed_p, seed_r, inv_sqrt); \
@@ -753,9 +783,12 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     for (int i = n; i < kMaxGemmGroup; ++i) grp.tile_start[i + 1] = grp.tile_start[n];
     // 1. the rotations: one launch for the group where the wide kernel applies
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
-    const long wide_blocks = static_cast<long>(n_planes) * ((in + 255) / 256) * ((m + 7) / 8);
-    if (block <= 256 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
-        launch_pdl(rotate_rows_f16_wide_group_kernel, dim3(static_cast<unsigned int>(wide_blocks), static_cast<unsigned int>(n)), dim3(256), 0,
+    const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
+    const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8);
+    if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
+        auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_group_kernel<1>
+                                            : (wide_cols == 512 ? rotate_rows_f16_wide_group_kernel<2> : rotate_rows_f16_wide_group_kernel<4>);
+        launch_pdl(wide, dim3(static_cast<unsigned int>(wide_blocks), static_cast<unsigned int>(n)), dim3(256), 0,
                    stream, x, rot, in, m, n_planes, static_cast<int>(block), inv_sqrt);
     } else {
         const long n_warps = static_cast<long>(n_planes) * m * (in / static_cast<int>(block));
