@@ -127,6 +127,55 @@ __global__ void __launch_bounds__(128) rotate_x_kernel(const __half* __restrict_
     for (int j = 0; j < E; ++j) dst[j] = to_tf32(v[j] * inv_sqrt);
 }
 
+// The same with 16-byte accesses: a warp takes CHUNKS x 256 columns of a row (a WHT block of 512 or 1024 columns, or the
+// smaller blocks of 256 columns).  A lane of the kernel above reads E consecutive halves, 2 bytes at a time: 2 E accesses of
+// up to 32 lines each, and as all of its few CTAs land on the first SM that the kernel before it leaves (no other has room
+// yet), they serialised there: 13 us of the 31 us of a 3584 x 3584 layer with two rotations, block 512 and 4 rows.  For the
+// same reason the launch asks for shared memory it does not use: four CTAs per SM.
+template <int CHUNKS>
+__global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __restrict__ x, float* __restrict__ xrot, int in, int batch,
+                                                            int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
+    grid_launch_dependents();
+    grid_dependency_sync();
+    const int lane = threadIdx.x & 31;
+    const int groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= n_planes * batch * groups_per_row) return;
+    const int plane = warp / (batch * groups_per_row);
+    const int rem = warp - plane * batch * groups_per_row;
+    const int row = rem / groups_per_row, col = (rem - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
+    if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
+    const uint32_t seed = plane ? seed_r : seed_p;
+    const __half* const src = x + static_cast<size_t>(row) * in + col;
+    uint4 raw[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
+    const unsigned live = __activemask();
+    float v[CHUNKS][8];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], seed, static_cast<uint32_t>(col + 256 * c), block, lane, live);
+#pragma unroll
+    for (int h = 1; h < CHUNKS; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < CHUNKS; i += 2 * h)
+#pragma unroll
+            for (int c = i; c < i + h; ++c)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float a = v[c][j], b = v[c + h][j];
+                    v[c][j] = __fadd_rn(a, b);
+                    v[c + h][j] = __fsub_rn(a, b);
+                }
+    float* const dst = xrot + (static_cast<size_t>(plane) * batch + row) * in + col;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(dst + 256 * c + j) = make_float4(to_tf32(v[c][j] * inv_sqrt), to_tf32(v[c][j + 1] * inv_sqrt),
+                                                                        to_tf32(v[c][j + 2] * inv_sqrt), to_tf32(v[c][j + 3] * inv_sqrt));
+}
+constexpr size_t kRotateXSmem = 48 * 1024;
+
 struct GemvArgs {
     const uint8_t* codes;   // joint bytes in 16 x 64 tiles (code_offset)
     const float* norms;     // [out]
@@ -968,9 +1017,6 @@ static bool fill_gemv_args(GemvArgs& a, const __half* x, int out, int in, int ba
 
 // Shared-memory opt-in of every instantiation, once per device.
 static void configure_gemv_kernels();
-static void launch_rotate_x_pdl(const __half* x, float* xrot, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
-                                uint32_t seed_r, cudaStream_t stream);
-
 void launch_tq8_gemv(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
                      int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
                      void* scratch, unsigned int* status, int sm_count, cudaStream_t stream) {
@@ -1060,7 +1106,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     const int n_attr = 1;
 
     // 1. rotate the activation (one warp per plane x row x block)
-    if (!fused_rotation) launch_rotate_x_pdl(x, xrot, in, batch, block, n_planes, seed_p, seed_r, stream);
+    if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, n_planes, seed_p, seed_r, stream);
     // 2. the GEMV itself
     {
         const int n_units = a.n_row_units * a.n_slots;
@@ -1116,30 +1162,6 @@ static void configure_gemv_kernels() {
     if (dev < 64) configured[dev] = true;
 }
 
-static void launch_rotate_x_pdl(const __half* x, float* xrot, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
-                                uint32_t seed_r, cudaStream_t stream) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
-    const int n_warps = n_planes * batch * (in / static_cast<int>(block));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((n_warps + 3) / 4);
-    cfg.blockDim = dim3(128);
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-#define TQ_ROT_CASE(EV)                                                                                            \
-    case 32 * EV:                                                                                                  \
-        TQ_CUDA(cudaLaunchKernelEx(&cfg, rotate_x_kernel<EV>, x, xrot, in, batch, n_planes, seed_p, seed_r, inv_sqrt)); \
-        break;
-    switch (block) {
-        TQ_ROT_CASE(1) TQ_ROT_CASE(2) TQ_ROT_CASE(4) TQ_ROT_CASE(8) TQ_ROT_CASE(16) TQ_ROT_CASE(32)
-        default: throw Error("unsupported WHT block size");
-    }
-#undef TQ_ROT_CASE
-}
-
 void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, int batch, int sm_count, cudaStream_t stream) {
     TQ_REQUIRE(items != nullptr && n >= 1 && n <= kMaxGroup, "tq8_gemv group: 1..4 matrices");
     TQ_REQUIRE(x != nullptr && batch >= 1 && batch <= 8, "tq8_gemv group: 1..8 activation rows");
@@ -1188,7 +1210,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     configure_gemv_kernels();
     for (int i = 0; i < n; ++i)
         if (!fused[i])
-            launch_rotate_x_pdl(x, const_cast<float*>(grp.m[i].xrot), items[i].in, batch, items[i].block, items[i].n_planes,
+            launch_rotate_x(x, const_cast<float*>(grp.m[i].xrot), items[i].in, batch, items[i].block, items[i].n_planes,
                                 items[i].seed_p, items[i].seed_r, stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1214,21 +1236,29 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
 #undef TQ_GROUP_LAUNCH
 }
 
-// The activation rotation alone (the pre-kernel of WHT blocks above 256 columns), for the other
-// decode kernels: xrot = [n_planes, batch, in] fp32.
+// The activation rotation alone (the pre-kernel of several rows or WHT blocks above 256 columns), also for the other decode
+// kernels: xrot = [n_planes, batch, in] fp32.
 void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
                      uint32_t seed_r, cudaStream_t stream) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
-    const int n_warps = n_planes * batch * (in / static_cast<int>(block));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((n_warps + 3) / 4);
     cfg.blockDim = dim3(128);
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {   // (a row is a multiple of 32 halves)
+        const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
+        auto* const wide = wide_cols == 256 ? rotate_x_wide_kernel<1> : (wide_cols == 512 ? rotate_x_wide_kernel<2> : rotate_x_wide_kernel<4>);
+        cfg.gridDim = dim3((n_planes * batch * ((in + wide_cols - 1) / wide_cols) + 3) / 4);
+        cfg.dynamicSmemBytes = kRotateXSmem;
+        TQ_CUDA(cudaLaunchKernelEx(&cfg, wide, x, xrot, in, batch, n_planes, static_cast<int>(block), seed_p, seed_r, inv_sqrt));
+        return;
+    }
+    const int n_warps = n_planes * batch * (in / static_cast<int>(block));
+    cfg.gridDim = dim3((n_warps + 3) / 4);
 #define TQ_ROT_CASE(EV)                                                                                            \
     case 32 * EV:                                                                                                  \
         TQ_CUDA(cudaLaunchKernelEx(&cfg, rotate_x_kernel<EV>, x, xrot, in, batch, n_planes, seed_p, seed_r, inv_sqrt)); \
