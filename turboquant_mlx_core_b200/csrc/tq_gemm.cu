@@ -67,9 +67,11 @@ constexpr int kProducerWarps = 8 * kGroups;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kMmaWarp = kProducerWarps;       // issues the MMAs, owns the tensor-memory allocation
 constexpr int kCopyWarp = kProducerWarps + 1;  // issues the activation-tile bulk copies
-constexpr int kGemmThreads = kProducerThreads + 64;
+constexpr int kEpilogueWarp = kProducerWarps + 2;  // first of four warps that drain the accumulators
+constexpr int kEpilogueWarps = 4;
+constexpr int kGemmThreads = kProducerThreads + 64 + 32 * kEpilogueWarps;
 constexpr uint32_t kLutBytes = 256 * 32 * 4;           // one plane: 256 entries x 32 lane copies x (fp16, fp16)
-constexpr uint32_t kTmemCols = 512;   // accumulator: columns 0..255; weight tiles: 4 stages x 64 columns from 256 on
+constexpr uint32_t kTmemCols = 512;   // accumulators: columns 0..255 (two of up to 128 columns, or one); weight tiles: 4 stages x 64 columns from 256 on
 constexpr uint32_t kTmemAColumn = 256;
 constexpr uint32_t kTmemASubCols = kBlockK / 2;                    // one K block: two fp16 per 32-bit column
 constexpr uint32_t kTmemAStageCols = kSubPerStage * kTmemASubCols;
@@ -331,32 +333,34 @@ struct GemmArgs {
     float inv_scale;
 };
 
-// One CTA's work: output tile (row tile bx, token tile blockIdx.y), K split bz of matrix p.
-__device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const int bz) {
+// One CTA's work: K split bz of the output tiles t0, t0 + t_step, ... < t_end of matrix p.  Tile t is row tile t / n_tok,
+// token tile t % n_tok: CTAs that run side by side share the codes of a few row tiles, which then come from HBM once however
+// many token tiles there are.
+__device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const int t_step, const int t_end, const int bz) {
     extern __shared__ __align__(128) uint8_t gemm_smem[];
-    __shared__ __align__(8) unsigned long long s_full[kStagesMax], s_empty[kStagesMax], s_accum;
+    __shared__ __align__(8) unsigned long long s_full[kStagesMax], s_empty[kStagesMax], s_accum_full[2], s_accum_empty[2];
     __shared__ uint32_t s_tmem_base;
     __shared__ unsigned int s_abort;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row0 = bx * kTileRows;  // first weight row of the tile
-    const int tok0 = blockIdx.y * kTileTok;   // first activation row of the tile
-    // Activation rows this tile really has, rounded up to the MMA's granularity of 16: a short tile
-    // (a decode batch of 9..64 rows, or the tail of a prefill) costs a short MMA and a short copy.
-    const int n_tile = min(kTileTok, ((p.m - tok0) + 15) & ~15);
-    const uint32_t b_bytes = static_cast<uint32_t>(n_tile) * (kBlockK * 2);   // one 64-column piece: the tile's first n_tile rows are contiguous
-    const uint32_t idesc = instr_desc(static_cast<uint32_t>(n_tile));
+    const int n_tok = (p.m + kTileTok - 1) / kTileTok;
+    // Activation rows of a tile, rounded up to the MMA's granularity of 16: a short tile (a decode batch of 9..64 rows, or
+    // the tail of a prefill) costs a short MMA and a short copy.
+    auto tile_rows = [&](int t) { return min(kTileTok, ((p.m - (t % n_tok) * kTileTok) + 15) & ~15); };
+    const int n_max = min(kTileTok, (p.m + 15) & ~15);
+    const int n_acc = n_max <= kTileTok / 2 ? 2 : 1;   // accumulators: with two, a tile is drained beside the next one's products
+    const int n_local = t0 < t_end ? (t_end - t0 + t_step - 1) / t_step : 0;
 
     // ---- shared-memory map -------------------------------------------------------------------
     // [kLutWin, + 32 KB per plane)  lookup tables, at a fixed window address (it is an immediate of
     //                               the lookup's load instruction)
-    // [after the tables, end)       activation stages of 2 * b_bytes (two 64-column pieces), as many
-    //                               as fit, at most kStagesMax
+    // [after the tables, end)       activation stages of two 64-column pieces, as many as fit, at most kStagesMax
     const uint32_t raw = smem_addr(gemm_smem);
     uint32_t dyn_bytes;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
     const uint32_t stage0 = kLutWin + kLutBytes * static_cast<uint32_t>(p.n_planes);
-    const uint32_t stage_bytes = kSubPerStage * b_bytes;
+    const uint32_t piece_bytes = static_cast<uint32_t>(n_max) * (kBlockK * 2);   // a 64-column piece: a tile's first n_max rows are contiguous
+    const uint32_t stage_bytes = kSubPerStage * piece_bytes;
     const uint32_t smem_end = raw + dyn_bytes;
     int n_st = smem_end > stage0 ? static_cast<int>((smem_end - stage0) / stage_bytes) : 0;
     if (n_st > kStagesMax) n_st = kStagesMax;
@@ -364,14 +368,18 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
         if (tid == 0) raise_status(p.status, 9u);
         return;
     }
-    const uint32_t bar_full = smem_addr(&s_full[0]), bar_empty = smem_addr(&s_empty[0]), bar_accum = smem_addr(&s_accum);
+    const uint32_t bar_full = smem_addr(&s_full[0]), bar_empty = smem_addr(&s_empty[0]);
+    const uint32_t bar_acc_full = smem_addr(&s_accum_full[0]), bar_acc_empty = smem_addr(&s_accum_empty[0]);
 
     if (tid == 0) {
         for (int s = 0; s < kStagesMax; ++s) {
             bar_init(bar_full + 8u * s, kProducerWarps / kGroups + 1);   // one arrival per producer warp of the group + the copy thread
             bar_init(bar_empty + 8u * s, 1);
         }
-        bar_init(bar_accum, 1);
+        for (int s = 0; s < 2; ++s) {
+            bar_init(bar_acc_full + 8u * s, 1);
+            bar_init(bar_acc_empty + 8u * s, kEpilogueWarps);
+        }
         s_abort = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -396,7 +404,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
     volatile unsigned int* abort_flag = &s_abort;
 
     // K blocks (64 columns) of this CTA: a contiguous range of the (plane-major) list of all K blocks.
-    // A stage is two consecutive K blocks of the range (the last one may hold a single block).
+    // A stage is two consecutive K blocks of the range (the last one may hold a single block).  The stages of the CTA's
+    // tiles follow one another through the ring.
     const int kb_per_plane = p.in / kBlockK;
     const int n_kb_total = kb_per_plane * p.n_planes;
     const int kb_base = static_cast<int>(static_cast<long>(n_kb_total) * bz / p.k_splits);
@@ -414,35 +423,56 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
         const int grp = warp >> 3;
         // The warp's rows are two code tiles of 16 x 64 bytes; lane (g, q) takes bytes 16 q .. of rows g and g + 8 of each:
         // a load of the warp is 512 contiguous bytes.  Tiles past the matrix repeat the last one (never stored).
-        const int last_tile = (p.out - 1) >> 4, tile0 = (row0 >> 4) + 2 * (warp & 3);
+        const int last_tile = (p.out - 1) >> 4;
         const size_t tile_row_bytes = static_cast<size_t>(code_tiles_per_row(p.in)) * kCodeTileBytes;
         const uint8_t* const code_lane = p.codes + (lane >> 2) * 64 + 16 * (lane & 3);
-        const uint8_t* const code_ptr[2] = {code_lane + static_cast<size_t>(min(tile0, last_tile)) * tile_row_bytes,
-                                            code_lane + static_cast<size_t>(min(tile0 + 1, last_tile)) * tile_row_bytes};
         const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemAColumn + kTmemASubCols * static_cast<uint32_t>(sub);
+        const int n_stages = n_local * n_it;
 
-        // Codes are fetched two of the group's stages ahead into registers.  The second plane reads
-        // the same bytes again.
-        auto load_codes = [&](int it, uint4 (&c)[4]) {
-            const int kb = kSubPerStage * it + sub;
-            if (kb < n_kb) {
+        // The group's next stage to fetch.  Two of its stages are in registers or on their way; the second plane reads the
+        // same bytes again.
+        int f_it = grp, f_t = t0, f_left = n_stages - grp;
+        const uint8_t* f_ptr[2];
+        auto fetch_tile = [&] {
+            const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3);
+            f_ptr[0] = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes;
+            f_ptr[1] = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes;
+        };
+        auto carry = [&](int& it, int& t) {   // past the tile's last stage: the same place of the next tiles
+            bool moved = false;
+            while (it >= n_it) {
+                it -= n_it;
+                t += t_step;
+                moved = true;
+            }
+            return moved;
+        };
+        auto fetch = [&](uint4 (&c)[4]) {
+            const int kb = kSubPerStage * f_it + sub;
+            if (f_left > 0 && kb < n_kb) {
                 const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
                 const size_t at = static_cast<size_t>(kb_base + kb - plane * kb_per_plane) * kCodeTileBytes;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = load_codes16(code_ptr[i >> 1] + at + 512 * (i & 1));
+                for (int i = 0; i < 4; ++i) c[i] = load_codes16(f_ptr[i >> 1] + at + 512 * (i & 1));
             }
+            f_left -= kGroups;
+            f_it += kGroups;
+            if (f_it >= n_it && f_left > 0 && carry(f_it, f_t)) fetch_tile();
         };
-        uint4 c0[4], c1[4], c2[4];
+        uint4 buf0[4], buf1[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) c0[i] = c1[i] = c2[i] = make_uint4(0, 0, 0, 0);
-        load_codes(grp, c0);
-        load_codes(grp + kGroups, c1);
+        for (int i = 0; i < 4; ++i) buf0[i] = buf1[i] = make_uint4(0, 0, 0, 0);
+        carry(f_it, f_t);
+        fetch_tile();
+        fetch(buf0);
+        fetch(buf1);
+        int it = grp, unused_t = 0;
+        carry(it, unused_t);
         int slot = grp % n_st, use = grp / n_st;     // ring slot of stage `it` and how often it has been used before
-        bool alive = true;
-        for (int it = grp; alive && it < n_it; it += kGroups) {
-            load_codes(it + 2 * kGroups, c2);
+        // One stage; false once a wait has run out.
+        auto produce = [&](uint4 (&c0)[4]) {
             const int kb = kSubPerStage * it + sub;
-            const bool have = kb < n_kb;             // the last stage may lack its second K block
+            const bool have = kb < n_kb;             // the last stage of a tile may lack its second K block
             const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
             // lane offset, plus 32 KB for the second plane's table: bits outside the scaled code (7..14)
             const uint32_t lane_c = static_cast<uint32_t>(lane) * 4u + static_cast<uint32_t>(plane) * kLutBytes;
@@ -460,27 +490,29 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
                     // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
                     packed[h] = __byte_perm(lut_load(__dp4a(word, 128u << (8 * b0), lane_c)), lut_load(__dp4a(word, 128u << (8 * b0 + 8), lane_c)), 0x5410);
                 }
+                // the codes are used up: the stage after next into the same registers
+                if (half == 1) fetch(c0);
                 // the slot must have been read by the MMAs of its previous stage
-                if (half == 0 && use > 0 && !bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag)) {
+                if (half == 0 && use > 0 && !__all_sync(0xffffffffu, bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag))) {
                     raise_status(p.status, 6u);
                     atomicExch(&s_abort, 1u);
-                    alive = false;
+                    return false;
                 }
-                if (!alive) break;
                 if (have) tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
             }
-            if (!alive) break;
             // every lane waits for its own stores, then one arrival per warp
             tmem_st_publish();
             __syncwarp();
             if (lane == 0) bar_arrive(bar_full + 8u * slot);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                c0[i] = c1[i];
-                c1[i] = c2[i];
-            }
+            it += kGroups;
+            if (it >= n_it) carry(it, unused_t);
             slot += kGroups;
             if (slot >= n_st) { slot -= n_st; ++use; }
+            return true;
+        };
+        for (int left = n_stages - grp; left > 0; left -= 2 * kGroups) {
+            if (!produce(buf0)) break;
+            if (left > kGroups && !produce(buf1)) break;
         }
     } else if (warp == kCopyWarp) {
         // ---- activation tiles: one bulk copy per K block of the stage, as far ahead as the ring allows ----
@@ -491,95 +523,135 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
             // programmatic-dependency attribute, the CTA has set up its barriers, tensor memory and tables and the
             // producers are already streaming codes meanwhile): wait for that kernel here.
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            const size_t n_tok_tiles = (static_cast<size_t>(p.m) + kTileTok - 1) / kTileTok;
-            int slot = 0;
+            int slot = 0, filled = 0;
             uint32_t par = 1u;   // parity of the "empty" phase to wait for
-            for (int it = 0; it < n_it; ++it) {
-                if (it >= n_st && !bar_wait(bar_empty + 8u * slot, par, abort_flag)) {
-                    raise_status(p.status, 6u);
-                    atomicExch(&s_abort, 1u);
-                    break;
+            bool ok = true;
+            for (int t = t0; ok && t < t_end; t += t_step) {
+                const uint32_t b_bytes = static_cast<uint32_t>(tile_rows(t)) * (kBlockK * 2);
+                for (int it = 0; it < n_it; ++it) {
+                    if (filled >= n_st && !bar_wait(bar_empty + 8u * slot, par, abort_flag)) {
+                        raise_status(p.status, 6u);
+                        atomicExch(&s_abort, 1u);
+                        ok = false;
+                        break;
+                    }
+                    ++filled;
+                    const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
+                    const uint32_t bar = bar_full + 8u * slot;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(b_bytes * nsub) : "memory");
+                    for (int sb = 0; sb < nsub; ++sb) {
+                        const int kb = kSubPerStage * it + sb;
+                        const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
+                        const size_t tile = (static_cast<size_t>(plane) * n_tok + t % n_tok) * kb_per_plane + (kb_base + kb - plane * kb_per_plane);
+                        const __half* src = p.xrot + tile * (kTileTok * kBlockK);
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                         stage0 + static_cast<uint32_t>(slot) * stage_bytes + static_cast<uint32_t>(sb) * piece_bytes),
+                                     "l"(src), "r"(b_bytes), "r"(bar)
+                                     : "memory");
+                    }
+                    if (++slot == n_st) { slot = 0; par ^= 1u; }
                 }
-                const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
-                const uint32_t bar = bar_full + 8u * slot;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(b_bytes * nsub) : "memory");
-                for (int sb = 0; sb < nsub; ++sb) {
-                    const int kb = kSubPerStage * it + sb;
-                    const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
-                    const size_t tile = (static_cast<size_t>(plane) * n_tok_tiles + blockIdx.y) * kb_per_plane + (kb_base + kb - plane * kb_per_plane);
-                    const __half* src = p.xrot + tile * (kTileTok * kBlockK);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     stage0 + static_cast<uint32_t>(slot) * stage_bytes + static_cast<uint32_t>(sb) * b_bytes),
-                                 "l"(src), "r"(b_bytes), "r"(bar)
-                                 : "memory");
-                }
-                if (++slot == n_st) { slot = 0; par ^= 1u; }
             }
             // every activation tile of this CTA is on its way: the kernel after this one may start setting up
             asm volatile("griddepcontrol.launch_dependents;");
         }
         __syncwarp();
-    } else {
+    } else if (warp == kMmaWarp) {
         // ---- MMA issuer (one thread): one wait and one commit per stage ---------------------------------
         if (lane == 0) {
-            int slot = 0;
-            uint32_t par = 0u;
+            int slot = 0, acc = 0;
+            uint32_t par = 0u, acc_par = 1u;   // acc_par: parity of the "drained" phase to wait for
             bool ok = true;
-            for (int it = 0; it < n_it; ++it) {
-                if (!bar_wait(bar_full + 8u * slot, par, abort_flag)) {
-                    raise_status(p.status, 7u);
-                    atomicExch(&s_abort, 1u);
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
-                const uint32_t a_tmem = tmem_d + kTmemAColumn + kTmemAStageCols * static_cast<uint32_t>(slot);
-                const uint32_t b_stage = stage0 + static_cast<uint32_t>(slot) * stage_bytes;
-#pragma unroll
-                for (int sb = 0; sb < kSubPerStage; ++sb) {
-                    if (sb < nsub) {
-                        const uint64_t desc0 = smem_desc(b_stage + static_cast<uint32_t>(sb) * b_bytes);
-#pragma unroll
-                        for (int j = 0; j < kBlockK / 16; ++j)   // 256 bytes further along K per step: +16 in the address field
-                            umma_f16_ts(tmem_d, a_tmem + kTmemASubCols * sb + 8u * j, desc0 + static_cast<uint64_t>(16 * j), idesc,
-                                        (it | sb | j) != 0 ? 1u : 0u);
+            for (int j = 0; ok && j < n_local; ++j) {
+                const uint32_t idesc = instr_desc(static_cast<uint32_t>(tile_rows(t0 + j * t_step)));
+                const uint32_t d_tmem = tmem_d + static_cast<uint32_t>(acc * (kTileTok / 2));
+                if (j >= n_acc) {
+                    if (!bar_wait(bar_acc_empty + 8u * acc, acc_par, abort_flag)) {
+                        raise_status(p.status, 7u);
+                        atomicExch(&s_abort, 1u);
+                        break;
                     }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-                umma_commit(bar_empty + 8u * slot);   // the slot (weights and activation) may be refilled once these MMAs are done
-                if (++slot == n_st) { slot = 0; par ^= 1u; }
+                for (int it = 0; it < n_it; ++it) {
+                    if (!bar_wait(bar_full + 8u * slot, par, abort_flag)) {
+                        raise_status(p.status, 7u);
+                        atomicExch(&s_abort, 1u);
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
+                    const uint32_t a_tmem = tmem_d + kTmemAColumn + kTmemAStageCols * static_cast<uint32_t>(slot);
+                    const uint32_t b_stage = stage0 + static_cast<uint32_t>(slot) * stage_bytes;
+#pragma unroll
+                    for (int sb = 0; sb < kSubPerStage; ++sb) {
+                        if (sb < nsub) {
+                            const uint64_t desc0 = smem_desc(b_stage + static_cast<uint32_t>(sb) * piece_bytes);
+#pragma unroll
+                            for (int k = 0; k < kBlockK / 16; ++k)   // 256 bytes further along K per step: +16 in the address field
+                                umma_f16_ts(d_tmem, a_tmem + kTmemASubCols * sb + 8u * k, desc0 + static_cast<uint64_t>(16 * k), idesc,
+                                            (it | sb | k) != 0 ? 1u : 0u);
+                        }
+                    }
+                    umma_commit(bar_empty + 8u * slot);   // the slot (weights and activation) may be refilled once these MMAs are done
+                    if (++slot == n_st) { slot = 0; par ^= 1u; }
+                }
+                if (ok) umma_commit(bar_acc_full + 8u * acc);
+                if (++acc == n_acc) { acc = 0; acc_par ^= 1u; }
             }
-            if (ok) umma_commit(bar_accum);
         }
         __syncwarp();
-    }
-
-    // ---- epilogue (the producer warps): TMEM lanes 32 * (warp & 3), columns 64 * (warp >> 2) .. +63 ----
-    if (warp < kProducerWarps) {
-        const bool ok = !*abort_flag && bar_wait(bar_accum, 0, abort_flag);
-        if (!ok) {
-            raise_status(p.status, 8u);
-            atomicExch(&s_abort, 1u);
-        } else {
+    } else {
+        // ---- epilogue: TMEM lanes 32 * (warp & 3) .. + 31 (a lane = a weight row), 32 activation rows at a time ----
+        int acc = 0;
+        uint32_t par = 0u;
+        for (int j = 0; j < n_local; ++j) {
+            const int t = t0 + j * t_step;
+            if (!__all_sync(0xffffffffu, bar_wait(bar_acc_full + 8u * acc, par, abort_flag) && !*abort_flag)) {
+                raise_status(p.status, 8u);
+                atomicExch(&s_abort, 1u);
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int r = row0 + 32 * (warp & 3) + lane;
+            const int r = (t / n_tok) * kTileRows + 32 * (warp & 3) + lane;
+            const int tok0 = (t % n_tok) * kTileTok;
+            const int rows = min(kTileTok, p.m - tok0);
             const bool r_ok = r < p.out;
             const float scale = r_ok ? __ldg(p.norms + r) * p.inv_scale : 0.f;
+            const uint32_t d_tmem = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(acc * (kTileTok / 2));
+            __half* y = p.y + static_cast<size_t>(tok0) * p.y_stride + r;
+            float* part = p.partial + (static_cast<size_t>(bz) * p.m + tok0) * p.out + r;   // (only used with k_splits > 1)
 #pragma unroll 1
-            for (int cb = 0; cb < 2; ++cb) {
-                const int col0 = 64 * (warp >> 2) + 32 * cb;
-                if (col0 >= n_tile) break;   // warp-uniform: columns the MMA never wrote
+            for (int c0 = 0; c0 < rows; c0 += 32) {
                 uint32_t v[32];
-                tmem_ld32(tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(col0), v);
+                tmem_ld32(d_tmem + static_cast<uint32_t>(c0), v);
+                if (c0 + 32 >= rows) {   // the last read: the accumulator is free
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(bar_acc_empty + 8u * acc);
+                }
+                const int n = r_ok ? min(32, rows - c0) : 0;
+                if (p.k_splits == 1) {
+                    if (n == 32) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int tok = tok0 + col0 + j;
-                    if (r_ok && tok < p.m) {
-                        if (p.k_splits == 1) p.y[static_cast<size_t>(tok) * p.y_stride + r] = __float2half_rn(__uint_as_float(v[j]) * scale);
-                        else p.partial[(static_cast<size_t>(bz) * p.m + tok) * p.out + r] = __uint_as_float(v[j]);
+                        for (int k = 0; k < 32; ++k) {
+                            *y = __float2half_rn(__uint_as_float(v[k]) * scale);
+                            y += p.y_stride;
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k)
+                            if (k < n) y[k * p.y_stride] = __float2half_rn(__uint_as_float(v[k]) * scale);
                     }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; ++k)
+                        if (k < n) part[static_cast<size_t>(k) * p.out] = __uint_as_float(v[k]);
+                    part += static_cast<size_t>(32) * p.out;
                 }
             }
+            if (++acc == n_acc) { acc = 0; par ^= 1u; }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -590,8 +662,10 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int bx, const
     }
 }
 
+// gridDim.x CTAs walk the output tiles, gridDim.y = K splits.
 __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_kernel(const GemmArgs p) {
-    gemm_body(p, static_cast<int>(blockIdx.x), static_cast<int>(blockIdx.z));
+    const int n_tiles = ((p.out + kTileRows - 1) / kTileRows) * ((p.m + kTileTok - 1) / kTileTok);
+    gemm_body(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
 }
 
 // Several matrices that multiply the same activation rows (q / k / v, gate / up) in one launch: gridDim.x is cut into
@@ -608,7 +682,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const _
     int i = 0;
     while (i + 1 < grp.n && b >= grp.tile_start[i + 1]) ++i;
     if (static_cast<int>(blockIdx.z) >= grp.m[i].k_splits) return;
-    gemm_body(grp.m[i], b - grp.tile_start[i], static_cast<int>(blockIdx.z));
+    const int t = (b - grp.tile_start[i]) * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y);
+    gemm_body(grp.m[i], t, 1, t + 1, static_cast<int>(blockIdx.z));
 }
 
 // y = fp16(norm * inv_scale * sum over K splits, in split order) — fixed order, run-to-run identical.
@@ -729,8 +804,10 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
                                      static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
-    const dim3 grid(static_cast<unsigned int>((out + kTileRows - 1) / kTileRows),
-                    static_cast<unsigned int>((m + kTileTok - 1) / kTileTok), static_cast<unsigned int>(a.k_splits));
+    // a CTA per SM walks the tiles (with a K split there are fewer tiles x splits than SMs)
+    const long n_tiles = static_cast<long>((out + kTileRows - 1) / kTileRows) * ((m + kTileTok - 1) / kTileTok);
+    TQ_REQUIRE(n_tiles < (1L << 31), "tq8_gemm: too many output tiles");
+    const dim3 grid(static_cast<unsigned int>(std::min<long>(n_tiles, sm_count)), static_cast<unsigned int>(a.k_splits));
     launch_pdl(tq8_gemm_kernel, grid, dim3(kGemmThreads), smem, stream, a);
     TQ_CUDA(cudaGetLastError());
     if (a.k_splits > 1) {
