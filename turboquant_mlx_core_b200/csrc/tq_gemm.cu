@@ -106,9 +106,9 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile
     for (uint32_t spin = 0;; ++spin) {
         uint32_t done;
         asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
             : "=r"(done)
-            : "r"(bar), "r"(parity)
+            : "r"(bar), "r"(parity), "r"(20000u)   // ns that the thread may sleep
             : "memory");
         if (done) return true;
         if ((spin & 15) == 15 && *abort_flag) return false;
@@ -429,41 +429,48 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemAColumn + kTmemASubCols * static_cast<uint32_t>(sub);
         const int n_stages = n_local * n_it;
 
-        // The group's next stage to fetch.  Two of its stages are in registers or on their way; the second plane reads the
-        // same bytes again.
+        // The group's next stage to fetch: place in its tile, codes of its two code tiles, stages left.  Two of the group's
+        // stages are in registers or on their way; the second plane reads the same bytes again.
         int f_it = grp, f_t = t0, f_left = n_stages - grp;
-        const uint8_t* f_ptr[2];
-        auto fetch_tile = [&] {
-            const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3);
-            f_ptr[0] = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes;
-            f_ptr[1] = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes;
-        };
+        const uint8_t *f_ptr0, *f_ptr1;
         auto carry = [&](int& it, int& t) {   // past the tile's last stage: the same place of the next tiles
-            bool moved = false;
             while (it >= n_it) {
                 it -= n_it;
                 t += t_step;
-                moved = true;
             }
-            return moved;
+        };
+        auto fetch_place = [&] {
+            const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3);
+            int kb = kb_base + kSubPerStage * f_it + sub;
+            if (kb >= kb_per_plane) kb -= kb_per_plane;
+            f_ptr0 = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
+            f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
         };
         auto fetch = [&](uint4 (&c)[4]) {
             const int kb = kSubPerStage * f_it + sub;
             if (f_left > 0 && kb < n_kb) {
-                const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
-                const size_t at = static_cast<size_t>(kb_base + kb - plane * kb_per_plane) * kCodeTileBytes;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) c[i] = load_codes16(f_ptr[i >> 1] + at + 512 * (i & 1));
+                c[0] = load_codes16(f_ptr0);
+                c[1] = load_codes16(f_ptr0 + 512);
+                c[2] = load_codes16(f_ptr1);
+                c[3] = load_codes16(f_ptr1 + 512);
             }
             f_left -= kGroups;
             f_it += kGroups;
-            if (f_it >= n_it && f_left > 0 && carry(f_it, f_t)) fetch_tile();
+            f_ptr0 += kGroups * kSubPerStage * kCodeTileBytes;
+            f_ptr1 += kGroups * kSubPerStage * kCodeTileBytes;
+            // another tile, or possibly the second plane: place the pointers anew
+            if (f_it >= n_it || p.n_planes == 2) {
+                if (f_left > 0) {
+                    carry(f_it, f_t);
+                    fetch_place();
+                }
+            }
         };
         uint4 buf0[4], buf1[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) buf0[i] = buf1[i] = make_uint4(0, 0, 0, 0);
         carry(f_it, f_t);
-        fetch_tile();
+        fetch_place();
         fetch(buf0);
         fetch(buf1);
         int it = grp, unused_t = 0;
