@@ -109,39 +109,6 @@ __host__ __device__ __forceinline__ size_t code_offset(long row, int col, size_t
            (static_cast<size_t>(row) & 15) * kCodeTileCols + (static_cast<size_t>(col) & 63);
 }
 
-// The butterfly stages of a WHT block that a warp holds in chunks of 256 columns, lane l the columns 8 l .. 8 l + 7 of
-// each: signs, the stages below 8 in the lane and those of 8 .. 128 (as far as the block goes) between lanes, in the order
-// and pairing of warp_fwht.  `col` = the lane's first column of the chunk.  The stages above 128 are the caller's, between
-// chunks.
-__device__ __forceinline__ void rotate_chunk(float (&v)[8], const uint4& raw, uint32_t seed, uint32_t col, int block, int lane, unsigned live) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const __half2 h2 = *reinterpret_cast<const __half2*>(&w[j]);
-        v[2 * j] = __low2float(h2) * sign_value(seed, (col + 2 * j) & static_cast<uint32_t>(block - 1));
-        v[2 * j + 1] = __high2float(h2) * sign_value(seed, (col + 2 * j + 1) & static_cast<uint32_t>(block - 1));
-    }
-#pragma unroll
-    for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-        for (int i = 0; i < 8; i += 2 * h)
-#pragma unroll
-            for (int j = i; j < i + h; ++j) {
-                const float a = v[j], b = v[j + h];
-                v[j] = __fadd_rn(a, b);
-                v[j + h] = __fsub_rn(a, b);
-            }
-    const int lanes = block < 256 ? block >> 3 : 32;
-    for (int m = 1; m < lanes; m <<= 1) {
-        const bool upper = (lane & m) != 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float o = __shfl_xor_sync(live, v[j], m);
-            v[j] = upper ? __fsub_rn(o, v[j]) : __fadd_rn(v[j], o);
-        }
-    }
-}
-
 // Report a failure from a kernel.  The status word may live in page-locked HOST memory (so that
 // the host reads it without a copy): a plain store followed by a system-scope fence, no atomic.
 // Programmatic dependent launch for the small kernels of a decode step: launched with the attribute, a kernel's CTAs are
@@ -168,30 +135,129 @@ inline void launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaSt
 
 // Threads of a CTA that normalises one row (the RMSNorm kernel and the row-wise all-reduce tails: the same count, so the
 // same order of additions).  A decode step has a handful of rows: the row's latency, not the SM count, is what matters.
-constexpr int kRowNormThreads = 1024;
-
-// yr[:] = xr[:] * rsqrt(mean(xr[:]^2) + eps) * w for one row, by the whole CTA (up to 1024 threads, a multiple of 32;
-// cols even).  Shared by the RMSNorm kernel and the all-reduce tails that normalise the row they have just summed, so
-// the fused and the separate form give the same bits.
-__device__ __forceinline__ void rmsnorm_row(const __half* xr, const __half* __restrict__ w, __half* yr, int cols, float eps) {
-    float ss = 0.f;
-    for (int c = threadIdx.x * 2; c < cols; c += blockDim.x * 2) {
-        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(xr + c));
-        ss += v.x * v.x + v.y * v.y;
+// Up to 8 halves (n, even, at least 4-byte aligned) from or to memory, 16 bytes at once where they are all there and aligned;
+// missing ones read as zero.
+__device__ __forceinline__ uint4 load_halves(const __half* p, int n) {
+    if (n >= 8 && reinterpret_cast<uintptr_t>(p) % 16 == 0) return *reinterpret_cast<const uint4*>(p);
+    const uint32_t* const w = reinterpret_cast<const uint32_t*>(p);
+    return make_uint4(n > 0 ? w[0] : 0u, n > 2 ? w[1] : 0u, n > 4 ? w[2] : 0u, n > 6 ? w[3] : 0u);
+}
+__device__ __forceinline__ void store_halves(__half* p, int n, const uint4& v) {
+    if (n >= 8 && reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+        *reinterpret_cast<uint4*>(p) = v;
+        return;
     }
-    __shared__ float s_part[32];
+    uint32_t* const w = reinterpret_cast<uint32_t*>(p);
+    if (n > 0) w[0] = v.x;
+    if (n > 2) w[1] = v.y;
+    if (n > 4) w[2] = v.z;
+    if (n > 6) w[3] = v.w;
+}
+__device__ __forceinline__ void unpack_halves(const uint4& raw, float (&v)[8]) {
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+        v[2 * j] = f.x;
+        v[2 * j + 1] = f.y;
+    }
+}
+__device__ __forceinline__ uint4 pack_halves(const float (&v)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+        w[j] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Signs of eight columns of a WHT block, `col` and on, as the sign bits of their halves.
+__device__ __forceinline__ uint4 chunk_signs(uint32_t seed, uint32_t col, int block) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        w[j] = (sign_is_positive(seed, (col + 2 * j) & static_cast<uint32_t>(block - 1)) ? 0u : 0x8000u) |
+               (sign_is_positive(seed, (col + 2 * j + 1) & static_cast<uint32_t>(block - 1)) ? 0u : 0x80000000u);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// The butterfly stages of a WHT block that a warp holds in chunks of 256 columns, lane l the columns 8 l .. 8 l + 7 of
+// each: signs, the stages below 8 in the lane and those of 8 .. 128 (as far as the block goes) between lanes, in the order
+// and pairing of warp_fwht.  The stages above 128 are the caller's, between chunks.
+__device__ __forceinline__ void rotate_chunk(float (&v)[8], const uint4& raw, const uint4& signs, int block, int lane, unsigned live) {
+    unpack_halves(make_uint4(raw.x ^ signs.x, raw.y ^ signs.y, raw.z ^ signs.z, raw.w ^ signs.w), v);
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2 * h)
+#pragma unroll
+            for (int j = i; j < i + h; ++j) {
+                const float a = v[j], b = v[j + h];
+                v[j] = __fadd_rn(a, b);
+                v[j + h] = __fsub_rn(a, b);
+            }
+    const int lanes = block < 256 ? block >> 3 : 32;
+    for (int m = 1; m < lanes; m <<= 1) {
+        const float side = (lane & m) != 0 ? -1.0f : 1.0f;   // other + v or other - v, one exact multiply-add
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __fmaf_rn(v[j], side, __shfl_xor_sync(live, v[j], m));
+    }
+}
+
+// Threads of a CTA that normalises a row.  Eight columns per thread and step: 256 threads take 8192 columns in the four
+// steps that stay in registers, and eight rows run on an SM at a time (with 1024 threads and two columns per step a row's
+// barriers and reduction were most of its time).
+constexpr int kRowNormThreads = 256;
+constexpr int kRowNormKeep = 4;
+
+// yr[:] = xr[:] * rsqrt(mean(xr[:]^2) + eps) * w for one row, by the whole CTA (kRowNormThreads threads; cols even).  A
+// thread takes the columns 8 (threadIdx.x + k * kRowNormThreads) .. + 7, whatever the alignment, the first kRowNormKeep
+// steps of them in `keep`; the others are read from xr.  Shared by the RMSNorm kernel and the all-reduce tails that
+// normalise the row they have just summed, so the fused and the separate form give the same bits.
+__device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], const __half* xr, const __half* __restrict__ w, __half* yr, int cols,
+                                             float eps) {
+    constexpr int kStep = 8 * kRowNormThreads;
+    const int c0 = threadIdx.x * 8;
+    float ss = 0.f;
+    auto add = [&](const uint4& raw) {
+        float v[8];
+        unpack_halves(raw, v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+    };
+#pragma unroll
+    for (int k = 0; k < kRowNormKeep; ++k) add(keep[k]);   // (zero beyond the row)
+    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) add(load_halves(xr + c, cols - c));
+    __shared__ float s_part[kRowNormThreads / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
     __syncthreads();
     float tot = 0.f;
-    for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) tot += s_part[i];   // fixed order
+#pragma unroll
+    for (int i = 0; i < kRowNormThreads / 32; ++i) tot += s_part[i];   // fixed order
     const float scale = rsqrtf(tot / static_cast<float>(cols) + eps);
-    for (int c = threadIdx.x * 2; c < cols; c += blockDim.x * 2) {
-        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(xr + c));
-        const float2 g = __half22float2(*reinterpret_cast<const __half2*>(w + c));
-        *reinterpret_cast<__half2*>(yr + c) = __floats2half2_rn(v.x * scale * g.x, v.y * scale * g.y);
+    auto write = [&](int c, const uint4& raw) {
+        float v[8], g[8];
+        unpack_halves(raw, v);
+        unpack_halves(load_halves(w + c, cols - c), g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = v[j] * scale * g[j];
+        store_halves(yr + c, cols - c, pack_halves(v));
+    };
+#pragma unroll
+    for (int k = 0; k < kRowNormKeep; ++k)
+        if (c0 + k * kStep < cols) write(c0 + k * kStep, keep[k]);
+    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) write(c, load_halves(xr + c, cols - c));
+}
+__device__ __forceinline__ void rmsnorm_row(const __half* xr, const __half* __restrict__ w, __half* yr, int cols, float eps) {
+    uint4 keep[kRowNormKeep];
+#pragma unroll
+    for (int k = 0; k < kRowNormKeep; ++k) {
+        const int c = 8 * (threadIdx.x + k * kRowNormThreads);
+        keep[k] = c < cols ? load_halves(xr + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
     }
+    rmsnorm_kept(keep, xr, w, yr, cols, eps);
 }
 
 __device__ __forceinline__ void raise_status(unsigned int* status, unsigned int code) {

@@ -233,79 +233,82 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
     }
 }
 
-// The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of one row (one block of 512 or
+// The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of a row (one block of 512 or
 // 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
 // the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
-// a CTA take 8 consecutive rows, so their stores complete whole 128-byte core matrices.
+// a CTA take 8 consecutive rows, so their stores complete whole 128-byte core matrices, and `row_steps` such groups one after
+// the other: the hashes of the signs are a third of the instructions of a row, and they are the same for all rows (18944
+// columns: 67 us for 2048 rows with a group per CTA and signs multiplied in fp32, bound by instruction issue).
 template <int CHUNKS>
 __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows,
-                                                      int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
+                                                      int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const long groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
-    const long row_groups = (rows + 7) / 8;
-    // blockIdx.x -> (plane, column group, group of 8 rows); warp -> row inside the group
-    long b = blockIdx.x;
-    const long rg = b % row_groups;
+    const unsigned groups_per_row = (static_cast<unsigned>(in) + 256 * CHUNKS - 1) / (256 * CHUNKS);
+    const unsigned row_groups = static_cast<unsigned>((rows + 8 * row_steps - 1) / (8 * row_steps));
+    // blockIdx.x -> (plane, column group, rows); warp -> row inside a group of 8
+    unsigned b = blockIdx.x;
+    const unsigned rg = b % row_groups;
     b /= row_groups;
-    const long cg = b % groups_per_row;
+    const unsigned cg = b % groups_per_row;
     const int plane = static_cast<int>(b / groups_per_row);
     if (plane >= n_planes) return;
-    const long row = rg * 8 + wib;
     const int col = static_cast<int>(cg) * 256 * CHUNKS + 8 * lane;
-    // in is a multiple of 32 >= block: whole lanes only; exchanges stay inside a block.  (A group of several chunks is a
-    // whole block, all of it inside the row.)
-    if (row >= rows || col >= in) return;
-    const uint32_t seed = plane ? seed_r : seed_p;
-    uint4 raw[CHUNKS];
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
+    // in is a multiple of 64 and of the block: whole lanes only; exchanges stay inside a block.  (A group of several chunks
+    // is a whole block, all of it inside the row.)
+    if (col >= in) return;
     // lanes of an incomplete trailing group (in % 256 != 0) have returned: exchange only among the live ones
     const unsigned live = __activemask();
-    float v[CHUNKS][8];
+    const uint32_t seed = plane ? seed_r : seed_p;
+    uint4 signs[CHUNKS];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], seed, static_cast<uint32_t>(col + 256 * c), block, lane, live);
-#pragma unroll
-    for (int h = 1; h < CHUNKS; h <<= 1)
-#pragma unroll
-        for (int i = 0; i < CHUNKS; i += 2 * h)
-#pragma unroll
-            for (int c = i; c < i + h; ++c)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float a0 = v[c][j], b0 = v[c + h][j];
-                    v[c][j] = __fadd_rn(a0, b0);
-                    v[c + h][j] = __fsub_rn(a0, b0);
-                }
+    for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
     const long n_row_tiles = (rows + kTileTok - 1) / kTileTok;
     const long kb_per_plane = in / kBlockK;
-    const long rt = row / kTileTok, rin = row - rt * kTileTok;
-    const long tile0 = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane;
     // A lane's two groups of four columns are 16 positions apart; lane ^ 2 holds the ones next to them.  The lanes swap
     // one group each, so that every lane stores a whole core-matrix row of 8.
     const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
     const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
-    __half* const dst = xrot + tile0 * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (pos >> 3)) * 8 + (rin & 7)) * 8;
+    const long row0 = static_cast<long>(rg) * 8 * row_steps + wib, row_end = min(rows, row0 + 8L * row_steps);
+    for (long row = row0; row < row_end; row += 8) {
+        uint4 raw[CHUNKS];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        uint2 group[2];
+        for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
+        float v[CHUNKS][8];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const __half2 lo = __floats2half2_rn(v[c][4 * j] * inv_sqrt, v[c][4 * j + 1] * inv_sqrt);
-            const __half2 hi = __floats2half2_rn(v[c][4 * j + 2] * inv_sqrt, v[c][4 * j + 3] * inv_sqrt);
-            group[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
+#pragma unroll
+        for (int h = 1; h < CHUNKS; h <<= 1)
+#pragma unroll
+            for (int i = 0; i < CHUNKS; i += 2 * h)
+#pragma unroll
+                for (int c = i; c < i + h; ++c)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float a0 = v[c][j], b0 = v[c + h][j];
+                        v[c][j] = __fadd_rn(a0, b0);
+                        v[c + h][j] = __fsub_rn(a0, b0);
+                    }
+        const long rt = row / kTileTok, rin = row - rt * kTileTok;
+        const long tile0 = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane;
+        __half* const dst = xrot + tile0 * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (pos >> 3)) * 8 + (rin & 7)) * 8;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[c][j] *= inv_sqrt;
+            const uint4 h = pack_halves(v[c]);
+            const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
+            const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
+            const uint4 row8 = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
+            *reinterpret_cast<uint4*>(dst + static_cast<long>((col + 256 * c) / kBlockK) * (kTileTok * kBlockK)) = row8;
         }
-        const uint2 keep = odd ? group[1] : group[0], give = odd ? group[0] : group[1];
-        const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
-        const uint4 row8 = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
-        *reinterpret_cast<uint4*>(dst + static_cast<long>((col + 256 * c) / kBlockK) * (kTileTok * kBlockK)) = row8;
     }
 }
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
                                                                    int in, long rows, int n_planes, int block,
-                                                                   uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
+                                                                   uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
     pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
-    rotate_rows_wide_body<CHUNKS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt);
+    rotate_rows_wide_body<CHUNKS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt, row_steps);
 }
 // The same rows rotated for several matrices at once (their own seeds and destinations): blockIdx.y = matrix.
 struct RotateGroupArgs {
@@ -314,9 +317,9 @@ struct RotateGroupArgs {
 };
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const RotateGroupArgs g, int in,
-                                                                         long rows, int n_planes, int block, float inv_sqrt) {
+                                                                         long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
     pdl_wait_release();
-    rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt);
+    rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
 }
 
 struct GemmArgs {
@@ -731,6 +734,9 @@ __global__ void __launch_bounds__(256) gemm_finish_group_kernel(const FinishGrou
     }
 }
 
+// Groups of 8 rows that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
+int rotate_row_steps(long groups) { return static_cast<int>(std::max<long>(1, std::min<long>(8, groups / (148L * 8)))); }
+
 size_t xrot_bytes(int in, long m, int n_planes) {
     const size_t padded = (static_cast<size_t>(m) + kTileTok - 1) / kTileTok * kTileTok;  // whole operand tiles
     return (static_cast<size_t>(n_planes) * padded * static_cast<size_t>(in) * sizeof(__half) + 255) & ~static_cast<size_t>(255);
@@ -777,11 +783,12 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
         const long n_warps = static_cast<long>(n_planes) * m * (in / static_cast<int>(block));
         const unsigned int grid = static_cast<unsigned int>((n_warps + 3) / 4);
         const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
-        const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8);
+        const int row_steps = rotate_row_steps(static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8));
+        const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 8 * row_steps - 1) / (8 * row_steps));
         if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
             auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_kernel<1> : (wide_cols == 512 ? rotate_rows_f16_wide_kernel<2> : rotate_rows_f16_wide_kernel<4>);
             launch_pdl(wide, dim3(static_cast<unsigned int>(wide_blocks)), dim3(256), 0, stream, x, xrot, in, m, n_planes,
-                       static_cast<int>(block), seed_p, seed_r, inv_sqrt);
+                       static_cast<int>(block), seed_p, seed_r, inv_sqrt, row_steps);
         } else   // an activation that is not aligned
 #define TQ_ROT16_CASE(EV)                                                                                          \
     case 32 * EV:                                                                                                  \
@@ -868,12 +875,13 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     // 1. the rotations: one launch for the group where the wide kernel applies
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
     const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
-    const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8);
+    const int row_steps = rotate_row_steps(static_cast<long>(n) * n_planes * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8));
+    const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 8 * row_steps - 1) / (8 * row_steps));
     if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
         auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_group_kernel<1>
                                             : (wide_cols == 512 ? rotate_rows_f16_wide_group_kernel<2> : rotate_rows_f16_wide_group_kernel<4>);
         launch_pdl(wide, dim3(static_cast<unsigned int>(wide_blocks), static_cast<unsigned int>(n)), dim3(256), 0,
-                   stream, x, rot, in, m, n_planes, static_cast<int>(block), inv_sqrt);
+                   stream, x, rot, in, m, n_planes, static_cast<int>(block), inv_sqrt, row_steps);
     } else {
         const long n_warps = static_cast<long>(n_planes) * m * (in / static_cast<int>(block));
         const unsigned int grid = static_cast<unsigned int>((n_warps + 3) / 4);

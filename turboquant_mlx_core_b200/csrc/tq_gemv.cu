@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     const unsigned live = __activemask();
     float v[CHUNKS][8];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], seed, static_cast<uint32_t>(col + 256 * c), block, lane, live);
+    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block), block, lane, live);
 #pragma unroll
     for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll

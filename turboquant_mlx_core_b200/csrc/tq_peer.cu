@@ -110,28 +110,35 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_f16_kernel(const
                                                                float eps) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
-    const bool by_row = norm_w != nullptr;
-    const long first = by_row ? static_cast<long>(blockIdx.x) * cols + threadIdx.x * 2 : (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2;
-    const long last = by_row ? static_cast<long>(blockIdx.x + 1) * cols : count;
-    const long step = by_row ? static_cast<long>(blockDim.x) * 2 : static_cast<long>(gridDim.x) * blockDim.x * 2;
-    for (long i = first; i < last; i += step) {
-        float a = 0.f, b = 0.f;
-        if (residual != nullptr) {
-            const __half2 h = *reinterpret_cast<const __half2*>(residual + i);
-            a = __low2float(h);
-            b = __high2float(h);
+    // the sum of (up to) eight elements from i on, rounded and stored
+    auto sum8 = [&](long i, int n) {
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, h[8];
+        if (residual != nullptr) unpack_halves(load_halves(residual + i, n), a);
+        for (int s = 0; s < n_slots; ++s) {   // written by other GPUs: plain loads after the acquire of the wait kernel
+            unpack_halves(load_halves(slots + s * slot_stride + i, n), h);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[j] += h[j];
         }
-        for (int s = 0; s < n_slots; ++s) {
-            const __half2 h = *reinterpret_cast<const __half2*>(slots + s * slot_stride + i);   // written by other GPUs: plain loads after the acquire of the wait kernel
-            a += __low2float(h);
-            b += __high2float(h);
-        }
-        *reinterpret_cast<__half2*>(out + i) = __floats2half2_rn(a, b);
+        const uint4 r = pack_halves(a);
+        store_halves(out + i, n, r);
+        return r;
+    };
+    if (norm_w == nullptr) {
+        const long step = static_cast<long>(gridDim.x) * blockDim.x * 8;
+        for (long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8; i < count; i += step)
+            sum8(i, static_cast<int>(min(8L, count - i)));
+        return;
     }
-    if (by_row) {
-        __syncthreads();   // the row is complete (this CTA wrote all of it)
-        rmsnorm_row(out + static_cast<long>(blockIdx.x) * cols, norm_w, normed + static_cast<long>(blockIdx.x) * cols, cols, eps);
+    // a row per CTA; a thread sums the columns that it normalises afterwards (rmsnorm_kept's)
+    const long row = static_cast<long>(blockIdx.x) * cols;
+    uint4 keep[kRowNormKeep];
+#pragma unroll
+    for (int k = 0; k < kRowNormKeep; ++k) {
+        const int c = 8 * (threadIdx.x + k * kRowNormThreads);
+        keep[k] = c < cols ? sum8(row + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
     }
+    for (int c = 8 * (threadIdx.x + kRowNormKeep * kRowNormThreads); c < cols; c += 8 * kRowNormThreads) sum8(row + c, cols - c);
+    rmsnorm_kept(keep, out + row, norm_w, normed + row, cols, eps);
 }
 
 // Packets of the flag-in-data exchange {2 halves, epoch, 2 halves, epoch} -> contiguous fp16 (4 per packet).
@@ -333,8 +340,8 @@ void launch_exchange_sum_f16(const __half* slots, int n_slots, long slot_stride,
                    reinterpret_cast<uintptr_t>(out) % 4 == 0,
                "exchange sum: even element counts and 4-byte aligned buffers");
     if (count == 0) return;
-    long blocks = (count / 2 + 255) / 256;
-    if (blocks > 296) blocks = 296;
+    long blocks = (count / 8 + 255) / 256;
+    blocks = blocks < 1 ? 1 : (blocks > 1184 ? 1184 : blocks);
     if (norm_w != nullptr) {
         TQ_REQUIRE(normed != nullptr && cols > 0 && cols % 2 == 0 && count % cols == 0, "exchange sum + RMSNorm: whole rows of an even length");
         blocks = count / cols;
