@@ -1,0 +1,53 @@
+"""Decode attention against the oracle at the batches where the split of its work changes: jobs cut over many thread-block
+teams (one long sequence, few heads), whole jobs per team (one and several each), unequal lengths, more sequences than travel
+as kernel parameters.  Tolerance: the query is rounded to fp16, 2^-12 of a value in the root mean square, which moves a
+score s by up to 2^-12 |s| and its probability by as much relatively; with the inputs' outlier channels the scores that count
+reach about 8, so 2.0e-3; the result's rounding adds 2.4e-4 in squares."""
+import numpy as np
+import pytest
+
+from tests.conftest import rel_l2
+from tests.golden.make_golden import kv_inputs
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2.1e-3
+CASES = [
+    # tokens of each sequence, query heads, KV heads, head size
+    ([6000], 4, 1, 32),                       # hundreds of parts of one job
+    ([9000], 8, 1, 128),
+    ([5000, 17], 2, 1, 64),
+    ([1500], 3, 1, 256),
+    ([40] * 9, 8, 2, 128),                    # whole jobs, one per team
+    ([33, 1, 16, 90, 15, 47] * 6, 18, 2, 64),     # ... a group of 8 heads and one of a single head, lengths mixed
+    ([20, 5, 64] * 34, 4, 4, 128),            # ... two per team, descriptors from a table
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=[f"{len(c[0])}x{max(c[0])}_q{c[1]}_kv{c[2]}_d{c[3]}" for c in CASES])
+@pytest.mark.parametrize("qjl", [True, False], ids=["qjl", "plain"])
+def test_attention_work_split(tq, oracle, case, qjl):
+    lengths, q_heads, heads, dim = case
+    rng = np.random.default_rng(len(lengths) + dim)
+    q = rng.standard_normal((len(lengths), q_heads, dim)).astype(np.float16)
+    caches, want = [], []
+    for i, n in enumerate(lengths):
+        k, v = kv_inputs(100 + i, n, heads, dim)
+        c = tq.TQKVCache(1, heads, dim)
+        c.append(0, k, v)
+        caches.append(c)
+        if i < 8 or i >= len(lengths) - 4:    # the oracle's share of a large batch: its ends
+            kw, kn, qw, qn = oracle.kv_encode(k.astype(np.float32), oracle.kv_seed(0, 1), oracle.kv_seed(0, 3))
+            vw, vn, _, _ = oracle.kv_encode(v.astype(np.float32), oracle.kv_seed(0, 2))
+            want.append(oracle.attention(q[i].astype(np.float32), heads, kw, kn, vw, vn, qw, qn, layer=0, use_qjl=qjl))
+        else:
+            want.append(None)
+    got = tq.compressed_attention(caches, 0, q, use_qjl=qjl)
+    again = tq.compressed_attention(caches, 0, q, use_qjl=qjl)
+    for i, w in enumerate(want):
+        if w is not None:
+            assert rel_l2(got[i], w) < TOL, i
+        assert rel_l2(got[i], tq.compressed_attention([caches[i]], 0, q[i:i + 1], use_qjl=qjl)[0].astype(np.float32)) < TOL, i
+    assert np.array_equal(np.asarray(got).view(np.uint16), np.asarray(again).view(np.uint16))
+    for c in caches:
+        c.close()

@@ -21,11 +21,15 @@
 // turn, each through a ring of its own (one cp.async.bulk per tile, no synchronisation between warps), and merge their
 // (max, sum, accumulator) in shared memory.  A job that lies in one range is finished there; the parts of one that several
 // ranges share go to scratch, and the team that arrives last (a counter per job) adds them in range order - the result
-// does not depend on timing - un-rotates and writes.  One launch, no combine kernel.  A job's start and end cost a team about
+// does not depend on timing - un-rotates and writes.  One launch, no combine kernel.  Where a job has many parts their
+// weights are computed first, side by side, so that the accumulators stream: as a chain of rescaled sums, six parts a round
+// trip, 3 jobs of 2500 tiles spent 23 of 50 us there.  Where cutting the jobs costs more than it levels out, a range is a
+// number of whole jobs (launch_kv_attention).  A job's start and end cost a team about
 // as much as `pad` tiles, so the flat numbering gives every job that many empty tiles in front: a range with two jobs gets
 // fewer tiles than one with a single one.
 //
 // The next job's first tiles are requested before the merge of the current one, which has shared memory of its own.
+#include <algorithm>
 #include <cmath>
 
 #include "tq_attn.cuh"
@@ -41,6 +45,8 @@ __constant__ float kC3[8] = {-2.152176f, -1.344318f, -0.756130f, -0.245379f, 0.2
 constexpr uint32_t kTabBytes = 256 * 128;                       // the pair table, at the start of shared memory
 constexpr float kNone = -1e30f;
 constexpr int kGroup = 8;                                       // query heads of a job
+constexpr int kMaxRanges = 320;                                 // two per SM
+constexpr int kFewParts = 6;                                    // parts of a job that its last team adds in one round trip
 constexpr unsigned long long kWaitLimitNs = 200ull * 1000 * 1000;
 
 template <int D>
@@ -58,13 +64,22 @@ struct AttnCfg {
     static constexpr int kQStride = D + 8;                      // halves per rotated query
     static constexpr uint32_t kOffQ = kTabBytes + kWarps * kRing;                        // rotated queries
     static constexpr uint32_t kOffQs = kOffQ + kGroup * kQStride * 2;                   // ... with the residual's signs
-    static constexpr uint32_t kOffPub = kOffQs + kGroup * kQStride * 2;
+    // Rotated queries and probabilities as two fp16 numbers each, 22 bits, and two products: heads of other sizes than 128
+    // are multiplied as fp32 numbers would be.  (With one fp16 number the error against the oracle with QJL went from 2.0e-4,
+    // the rounding of the result, to 3.6e-4 for 64 dims.  128 dims have always been multiplied in fp16.)
+    static constexpr bool kSplit = D != 128;
+    static constexpr uint32_t kOffQl = kOffQs + kGroup * kQStride * 2;                  // what fp16 left of both, in fragment order
+    static constexpr uint32_t kOffQsl = kOffQl + (kSplit ? kGroup * kQStride * 2 : 0);
+    static constexpr uint32_t kOffPub = kOffQsl + (kSplit ? kGroup * kQStride * 2 : 0);
     static constexpr uint32_t kOffOut = kOffPub + kHalf * kPubBytes;
     static constexpr uint32_t kOffMl = kOffOut + kGroup * kAccStride * 4;               // [2][kHalf][8], then flags and the job
     static constexpr uint32_t kTeamBytes = kOffMl + 2 * kHalf * kGroup * 4 + 80 - kOffQ;   // of one team, from kOffQ on
     static constexpr uint32_t kEnd = kOffQ + kTeams * kTeamBytes;
     static constexpr int kPartFloats = kGroup * D + 2 * kGroup;                // a job part in scratch: accumulators, then (max, sum)
     static_assert(kPubBytes >= kGroup * kAccStride * 4, "a warp's accumulator in head order fits its place");
+    static constexpr int kMaxParts = kHalf * kPubBytes / (kGroup * 4);         // whose weights the publishing places hold
+    static_assert(kMaxParts >= kMaxRanges || D < 64, "parts of a job: up to all ranges");
+    static_assert(kGroup * kAccStride >= 2 * kTeam * kGroup, "the output's place holds two values per warp and head");
     static_assert(kOffQ % 16 == 0 && kOffPub % 16 == 0 && kOffOut % 16 == 0, "alignment");
     static_assert(kEnd + 1024u <= 227u * 1024u, "shared memory of an SM");
 };
@@ -77,7 +92,7 @@ struct AttnArgs {
     float* part;               // [range][2][kPartFloats]
     unsigned int* counters;    // [job]
     unsigned int* status;
-    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units, ranges, pad;
+    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units, ranges, pad, whole_jobs;
     uint32_t k_seed, v_seed, qjl_seed;
     float inv_sqrt, inv_scale, score_scale, qscale;
 };
@@ -166,6 +181,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     using B = KvBlock<D>;
     constexpr int kSteps = D / 16;   // k steps of a score product, m tiles of the value product
     constexpr int W = D / 32;        // nibble words of a token that a thread takes
+    constexpr bool kSplit = C::kSplit;
     extern __shared__ __align__(16) unsigned char attn_smem[];
     __shared__ __align__(8) unsigned long long s_bars[C::kWarps * C::kStages];
 
@@ -179,6 +195,8 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     unsigned char* const mine = attn_smem + C::kOffQ + team * C::kTeamBytes;   // this team's shared memory
     __half* const s_q = reinterpret_cast<__half*>(mine);
     __half* const s_qs = reinterpret_cast<__half*>(mine + (C::kOffQs - C::kOffQ));
+    [[maybe_unused]] __half* const s_ql = reinterpret_cast<__half*>(mine + (C::kOffQl - C::kOffQ));
+    [[maybe_unused]] __half* const s_qsl = reinterpret_cast<__half*>(mine + (C::kOffQsl - C::kOffQ));
     unsigned char* const s_pub = mine + (C::kOffPub - C::kOffQ);
     float* const s_out = reinterpret_cast<float*>(mine + (C::kOffOut - C::kOffQ));
     float* const s_m = reinterpret_cast<float*>(mine + (C::kOffMl - C::kOffQ));
@@ -209,8 +227,19 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         pdl_wait_release();
         return;
     }
-    const int u_end = static_cast<int>(static_cast<long>(a.units) * (range + 1) / a.ranges);
     const int jobs_per_seq = a.kv_heads * a.gchunks, G = a.q_heads / a.kv_heads;
+    // where range r starts: an equal share of the flat tiles, or of the jobs
+    auto range_start = [&](int r) {
+        if (!a.whole_jobs) return static_cast<int>(static_cast<long>(a.units) * r / a.ranges);
+        const int job = static_cast<int>(static_cast<long>(a.n_seqs) * jobs_per_seq * r / a.ranges);
+        if (job >= a.n_seqs * jobs_per_seq) return a.units;
+        const int seq = job / jobs_per_seq;
+        const AttnSeq S = attn_seq(a.seqs, seq);
+        return (S.tile0 + seq * a.pad) * jobs_per_seq + (job - seq * jobs_per_seq) * ((S.end + kKvTile - 1) / kKvTile - S.start / kKvTile + a.pad);
+    };
+    if (a.seqs.table != nullptr) pdl_wait_release();   // the table may have been uploaded just before
+    int u = range_start(range);
+    const int u_end = range_start(range + 1);
     const size_t tile_stride = static_cast<size_t>(a.kv_heads) * B::kBytes;
     uint32_t phase = 0;      // parity of the completion waited for next; flips every kStages = 2 stages
     int stage = 0;
@@ -269,8 +298,6 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         }
     };
 
-    int u = static_cast<int>(static_cast<long>(a.units) * range / a.ranges);
-    if (a.seqs.table != nullptr) pdl_wait_release();   // the table may have been uploaded just before
     Segment seg = locate(u);
     if (a.seqs.table == nullptr) pdl_wait_release();
     if (lane == 0) request_first(seg);
@@ -293,10 +320,16 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             warp_fwht<E>(v, lane);
 #pragma unroll
             for (int j = 0; j < E; ++j) {
-                const __half r = __float2half_rn(v[j] * a.inv_sqrt);
-                s_q[h * C::kQStride + lane * E + j] = r;
-                if constexpr (QJL)
-                    s_qs[h * C::kQStride + lane * E + j] = __float2half_rn(v[j] * (qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>(lane * E + j)) ? a.qscale : -a.qscale));
+                const int d = lane * E + j;
+                const float r = v[j] * a.inv_sqrt;
+                s_q[h * C::kQStride + d] = __float2half_rn(r);
+                if constexpr (kSplit) s_ql[h * C::kQStride + d] = __float2half_rn(r - __half2float(__float2half_rn(r)));
+                if constexpr (QJL) {
+                    const float rs = v[j] * (qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>(d)) ? a.qscale : -a.qscale);
+                    s_qs[h * C::kQStride + d] = __float2half_rn(rs);
+                    // dims 8 w + r and 8 w + r + 4 of a quarter side by side (sign pair 4 w + r)
+                    if constexpr (kSplit) s_qsl[h * C::kQStride + (d & ~7) + 2 * (d & 3) + ((d >> 2) & 1)] = __float2half_rn(rs - __half2float(__float2half_rn(rs)));
+                }
             }
         }
         team_sync();
@@ -318,6 +351,8 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                     const int d0 = 8 * (p / 4) + p % 4;
                     bs[p] = static_cast<uint32_t>(__half_as_ushort(ss[d0])) | (static_cast<uint32_t>(__half_as_ushort(ss[d0 + 4])) << 16);
                     if ((p & 1) == 0) even += __half2float(ss[d0]) + __half2float(ss[d0 + 4]);
+                    if constexpr (kSplit)
+                        if ((p & 1) == 0) even += __half2float(s_qsl[g * C::kQStride + (D / 4) * q + 2 * p]) + __half2float(s_qsl[g * C::kQStride + (D / 4) * q + 2 * p + 1]);
                 }
                 even += __shfl_xor_sync(0xffffffffu, even, 1);
                 even += __shfl_xor_sync(0xffffffffu, even, 2);
@@ -337,6 +372,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
 
         // The values of a tile are multiplied one iteration late, beside the next tile's scores: the two are independent, and
         // together they cover each other's shared-memory and tensor latencies.
+        [[maybe_unused]] uint32_t pl0 = 0u, pl1 = 0u;   // what fp16 left of P^T
         uint32_t xa[W], xb[W], pb0 = 0u, pb1 = 0u;   // value words (token pairs q and q + 4, dim group g) and P^T of the last tile
 #pragma unroll
         for (int w = 0; w < W; ++w) xa[w] = xb[w] = 0u;
@@ -346,12 +382,21 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             for (int w = 0; w < W; ++w) {
                 const uint32_t A = D == 128 && w == 3 ? kv_value_spare(xa[0], xa[1 % W], xa[2 % W]) : xa[w];
                 const uint32_t Bw = D == 128 && w == 3 ? kv_value_spare(xb[0], xb[1 % W], xb[2 % W]) : xb[w];
-                mma_f16(acc[2 * w], table_load(pair_addr<0>(A, lane_base)), table_load(pair_addr<1>(A, lane_base)),
-                        table_load(pair_addr<0>(Bw, lane_base)), table_load(pair_addr<1>(Bw, lane_base)), pb0, pb1);
-                mma_f16(acc[2 * w + 1], table_load(pair_addr<2>(A, lane_base)), table_load(pair_addr<3>(A, lane_base)),
-                        table_load(pair_addr<2>(Bw, lane_base)), table_load(pair_addr<3>(Bw, lane_base)), pb0, pb1);
+                const uint32_t v0 = table_load(pair_addr<0>(A, lane_base)), v1 = table_load(pair_addr<1>(A, lane_base));
+                const uint32_t v2 = table_load(pair_addr<0>(Bw, lane_base)), v3 = table_load(pair_addr<1>(Bw, lane_base));
+                const uint32_t v4 = table_load(pair_addr<2>(A, lane_base)), v5 = table_load(pair_addr<3>(A, lane_base));
+                const uint32_t v6 = table_load(pair_addr<2>(Bw, lane_base)), v7 = table_load(pair_addr<3>(Bw, lane_base));
+                mma_f16(acc[2 * w], v0, v1, v2, v3, pb0, pb1);
+                mma_f16(acc[2 * w + 1], v4, v5, v6, v7, pb0, pb1);
+                if constexpr (kSplit) {
+                    mma_f16(acc[2 * w], v0, v1, v2, v3, pl0, pl1);
+                    mma_f16(acc[2 * w + 1], v4, v5, v6, v7, pl0, pl1);
+                }
             }
         };
+        // This lane's fragments of the queries' remainders: words 4 w .. of quarter q, head g.
+        [[maybe_unused]] const uint32_t frag_ql = static_cast<uint32_t>(__cvta_generic_to_shared(s_ql)) + (g * C::kQStride + (D / 4) * q) * 2;
+        [[maybe_unused]] const uint32_t frag_qsl = static_cast<uint32_t>(__cvta_generic_to_shared(s_qsl)) + (g * C::kQStride + (D / 4) * q) * 2;
         // One tile: its block in shared memory, its first token.
         auto take_tile = [&](uint32_t blk, int token) {
             // ---- scores ----
@@ -363,10 +408,18 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 load_words<W>(kb, blk + (g + 8) * (D / 2) + q * (D / 8));
 #pragma unroll
                 for (int w = 0; w < W; ++w) {
-                    mma_f16(c1, table_load(pair_addr<0>(ka[w], lane_base)), table_load(pair_addr<0>(kb[w], lane_base)),
-                            table_load(pair_addr<1>(ka[w], lane_base)), table_load(pair_addr<1>(kb[w], lane_base)), bq[4 * w], bq[4 * w + 1]);
-                    mma_f16(c1b, table_load(pair_addr<2>(ka[w], lane_base)), table_load(pair_addr<2>(kb[w], lane_base)),
-                            table_load(pair_addr<3>(ka[w], lane_base)), table_load(pair_addr<3>(kb[w], lane_base)), bq[4 * w + 2], bq[4 * w + 3]);
+                    const uint32_t k0 = table_load(pair_addr<0>(ka[w], lane_base)), k1 = table_load(pair_addr<0>(kb[w], lane_base));
+                    const uint32_t k2 = table_load(pair_addr<1>(ka[w], lane_base)), k3 = table_load(pair_addr<1>(kb[w], lane_base));
+                    const uint32_t k4 = table_load(pair_addr<2>(ka[w], lane_base)), k5 = table_load(pair_addr<2>(kb[w], lane_base));
+                    const uint32_t k6 = table_load(pair_addr<3>(ka[w], lane_base)), k7 = table_load(pair_addr<3>(kb[w], lane_base));
+                    mma_f16(c1, k0, k1, k2, k3, bq[4 * w], bq[4 * w + 1]);
+                    mma_f16(c1b, k4, k5, k6, k7, bq[4 * w + 2], bq[4 * w + 3]);
+                    if constexpr (kSplit) {
+                        uint32_t lo[4];
+                        load_words<4>(lo, frag_ql + 16u * w);
+                        mma_f16(c1, k0, k1, k2, k3, lo[0], lo[1]);
+                        mma_f16(c1b, k4, k5, k6, k7, lo[2], lo[3]);
+                    }
                 }
                 if constexpr (QJL) {
                     // Bits 14 and 30 (dims 2, 6 of a word) as they stand are fp16 {0, 2}; bits 15 and 31 (dims 3, 7) over the
@@ -378,6 +431,12 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                         const uint32_t la = ka[w] << 8, lb = kb[w] << 8;
                         mma_f16(c2, two(la), two(lb), one(la), one(lb), bs[4 * w], bs[4 * w + 1]);
                         mma_f16(c2b, two(ka[w]), two(kb[w]), one(ka[w]), one(kb[w]), bs[4 * w + 2], bs[4 * w + 3]);
+                        if constexpr (kSplit) {
+                            uint32_t lo[4];
+                            load_words<4>(lo, frag_qsl + 16u * w);
+                            mma_f16(c2, two(la), two(lb), one(la), one(lb), lo[0], lo[1]);
+                            mma_f16(c2b, two(ka[w]), two(kb[w]), one(ka[w]), one(kb[w]), lo[2], lo[3]);
+                        }
                     }
                 }
             }
@@ -458,8 +517,14 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             l_run[0] += p00 + p10;
             l_run[1] += p01 + p11;
             // P^T fragment: (tokens 2q, 2q+1 | 2q+8, 2q+9 ; head g) from (token g | g+8 ; heads 2q, 2q+1)
-            pb0 = movmatrix_trans(pack_half2(p00 * vna, p01 * vna));
-            pb1 = movmatrix_trans(pack_half2(p10 * vnb, p11 * vnb));
+            const uint32_t pa = pack_half2(p00 * vna, p01 * vna), pb = pack_half2(p10 * vnb, p11 * vnb);
+            pb0 = movmatrix_trans(pa);
+            pb1 = movmatrix_trans(pb);
+            if constexpr (kSplit) {
+                const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&pa)), fb = __half22float2(*reinterpret_cast<const __half2*>(&pb));
+                pl0 = movmatrix_trans(pack_half2(fmaf(p00, vna, -fa.x), fmaf(p01, vna, -fa.y)));
+                pl1 = movmatrix_trans(pack_half2(fmaf(p10, vnb, -fb.x), fmaf(p11, vnb, -fb.y)));
+            }
         };
         const unsigned char* next_src = seg.src + static_cast<size_t>(warp + 2 * C::kStages * C::kTeam) * tile_stride;
         int token = seg.first_token + warp * kKvTile;
@@ -585,6 +650,58 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                     // the first range's part of the job starts at its tile 0
                     return a.part + static_cast<size_t>(2 * c + (c == c_first ? 1 : 0)) * C::kPartFloats;
                 };
+                const int n_parts = c_last - c_first + 1;
+                if (n_parts > kFewParts) {
+                    // Weights first: thread tid holds (max, sum) of head tid % 8 in parts tid / 8, tid / 8 + 32, ...
+                    constexpr int kHeld = (kMaxRanges * kGroup + C::kTeam * 32 - 1) / (C::kTeam * 32), kStep = C::kTeam * 32 / kGroup;
+                    const int h0 = tid & (kGroup - 1), p0 = tid / kGroup;
+                    float2 held[kHeld];
+                    float M = kNone;
+#pragma unroll
+                    for (int k = 0; k < kHeld; ++k) {
+                        const int c = p0 + k * kStep;
+                        held[k] = c < n_parts ? __ldcg(reinterpret_cast<const float2*>(part_of(c_first + c) + kGroup * D + 2 * h0)) : make_float2(kNone, 0.f);
+                    }
+#pragma unroll
+                    for (int k = 0; k < kHeld; ++k) M = fmaxf(M, held[k].x);
+                    M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 8));
+                    M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 16));
+                    float* const s_red = s_out;   // [warps][8] maxima, then the same of the sums; read before s_out is written
+                    if (lane < kGroup) s_red[warp * kGroup + lane] = M;
+                    team_sync();
+#pragma unroll
+                    for (int w = 0; w < C::kTeam; ++w) M = fmaxf(M, s_red[w * kGroup + h0]);
+                    float* const s_w = reinterpret_cast<float*>(s_pub);   // [parts][8]: the publishing places are free
+                    float L = 0.f;
+#pragma unroll
+                    for (int k = 0; k < kHeld; ++k) {
+                        const float f = exp2_approx(held[k].x - M);
+                        L = fmaf(held[k].y, f, L);
+                        if (p0 + k * kStep < n_parts) s_w[(p0 + k * kStep) * kGroup + h0] = f;
+                    }
+                    L += __shfl_xor_sync(0xffffffffu, L, 8);
+                    L += __shfl_xor_sync(0xffffffffu, L, 16);
+                    if (lane < kGroup) s_red[(C::kTeam + warp) * kGroup + lane] = L;
+                    team_sync();
+                    float sum = 0.f;
+#pragma unroll
+                    for (int w = 0; w < C::kTeam; ++w) sum += s_red[(C::kTeam + w) * kGroup + h0];
+                    team_sync();   // the reduction's place is read: s_out may be written
+                    if (p0 == 0) *reinterpret_cast<float2*>(s_out + h0 * C::kAccStride + D) = make_float2(M, sum);
+                    for (int idx = tid * 4; idx < kGroup * D; idx += C::kTeam * 128) {
+                        const int h = idx / D, d = idx - h * D;
+                        float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int c0 = 0; c0 < n_parts; c0 += 8) {
+                            float4 pa[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) pa[k] = __ldcg(reinterpret_cast<const float4*>(part_of(c_first + min(c0 + k, n_parts - 1)) + idx));
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                if (c0 + k < n_parts) add4(A, 1.f, pa[k], s_w[(c0 + k) * kGroup + h]);
+                        }
+                        *reinterpret_cast<float4*>(s_out + h * C::kAccStride + d) = A;
+                    }
+                } else
                 for (int idx = tid * 4; idx < kGroup * D; idx += C::kTeam * 128) {
                     const int h = idx / D, d = idx - h * D;
                     float M = kNone, L = 0.f;
@@ -657,11 +774,14 @@ void launch_d(const AttnArgs& args, int grid, cudaStream_t stream) {
 
 }  // namespace
 
-long attn_number_tiles(AttnSeq* seqs, int n_seqs) {
+long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest) {
     long total = 0;
+    *longest = 0;
     for (int i = 0; i < n_seqs; ++i) {
         seqs[i].tile0 = static_cast<int>(total);
-        total += (seqs[i].end + kKvTile - 1) / kKvTile - seqs[i].start / kKvTile;
+        const long tiles = (seqs[i].end + kKvTile - 1) / kKvTile - seqs[i].start / kKvTile;
+        *longest = std::max(*longest, tiles);
+        total += tiles;
     }
     return total;
 }
@@ -672,7 +792,7 @@ size_t attn_counters(int n_seqs, int q_heads, int kv_heads) {
     return static_cast<size_t>(n_seqs) * kv_heads * ((q_heads / kv_heads + kGroup - 1) / kGroup);
 }
 
-void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
                          uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl, void* scratch, unsigned int* counters,
                          __half* out, float* lse, unsigned int* status, int sm_count, cudaStream_t stream) {
     if (n_seqs == 0) return;
@@ -704,7 +824,20 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, const voi
     a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale / std::sqrt(d));
     // Two ranges per SM while every range has a tile per warp; fewer for short jobs, whose time is the merge of the parts.
     const int team = 8, teams = head_dim == 256 ? 1 : 2;
-    a.ranges = static_cast<int>(std::min<long>(static_cast<long>(teams) * sm_count, std::max<long>(1, (units + team - 1) / team)));
+    const long most = std::min<long>(static_cast<long>(teams) * sm_count, head_dim == 32 ? AttnCfg<32>::kMaxParts : kMaxRanges);
+    a.ranges = static_cast<int>(std::min<long>(most, std::max<long>(1, (units + team - 1) / team)));
+    // Or whole jobs per range.  An equal share of the tiles cuts most jobs, and the part of a job costs about 10 us more than
+    // a whole one (publish, fence, count, read back); against that stand the tiles that the longest range has more, 190 ns
+    // each with two teams on an SM and 100 ns with one (128 dims), and the end of every further job of a range, about 6 us.  Append +
+    // attention, cut against whole: 8 x 2000 tokens, 32 / 8 heads 25.1 / 16.8 us; 60 x 1500, 16 / 4 heads 46.0 / 35.1;
+    // 64 x 1000, 8 / 8 heads 56 / 49; 1 x 4096, 28 / 4 heads 18.0 / 34.0; 10 x 10539, 8 / 2 heads 27 / 54.
+    const long jobs = static_cast<long>(n_seqs) * kv_heads * a.gchunks;
+    const long jobs_per_range = (jobs + most - 1) / most, job_ranges = (jobs + jobs_per_range - 1) / jobs_per_range;
+    auto tile_ns = [&](long ranges) { return (ranges > sm_count ? 190L : 100L) * head_dim / 128; };
+    const long share = (units + a.ranges - 1) / a.ranges;
+    a.whole_jobs = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * 6000 <=
+                   share * tile_ns(a.ranges) + 10000 + 6000 * share * jobs / units;
+    if (a.whole_jobs) a.ranges = static_cast<int>(job_ranges);
     // 32: five rounds of the team's warps, about 6 us; less where ranges are short and every job ends in several of them
     a.pad = static_cast<int>(std::min<long>(32, units / a.ranges / 8));
     units += static_cast<long>(n_seqs) * kv_heads * a.gchunks * a.pad;
