@@ -236,9 +236,10 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
 // The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of a row (one block of 512 or
 // 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
 // the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
-// a CTA take 8 consecutive rows, so their stores complete whole 128-byte core matrices, and `row_steps` such groups one after
-// the other: the hashes of the signs are a third of the instructions of a row, and they are the same for all rows (18944
-// columns: 67 us for 2048 rows with a group per CTA and signs multiplied in fp32, bound by instruction issue).
+// a CTA take 8 consecutive rows, and `row_steps` such groups one after the other: the hashes of the signs are a third of the
+// instructions of a row, and they are the same for all rows.  The 8 rows of a K block are 1 KB of the operand tile: they
+// meet in shared memory (slots of a core matrix's rows permuted by its column: no bank conflicts) and leave as contiguous
+// stores; a lane's own 16-byte pieces of a row are 128 bytes apart.
 template <int CHUNKS>
 __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows,
                                                       int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
@@ -252,12 +253,12 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
     const unsigned cg = b % groups_per_row;
     const int plane = static_cast<int>(b / groups_per_row);
     if (plane >= n_planes) return;
+    __shared__ __align__(16) uint4 s_rows[2][256 * CHUNKS];   // [step parity][K block][core column][row slot]
     const int col = static_cast<int>(cg) * 256 * CHUNKS + 8 * lane;
-    // in is a multiple of 64 and of the block: whole lanes only; exchanges stay inside a block.  (A group of several chunks
-    // is a whole block, all of it inside the row.)
-    if (col >= in) return;
-    // lanes of an incomplete trailing group (in % 256 != 0) have returned: exchange only among the live ones
-    const unsigned live = __activemask();
+    // in is a multiple of 64 and of the block: whole lanes only, and exchanges stay inside a block.  (A group of several
+    // chunks is a whole block, all of it inside the row.)
+    const bool have = col < in;
+    const unsigned live = __ballot_sync(0xffffffffu, have);
     const uint32_t seed = plane ? seed_r : seed_p;
     uint4 signs[CHUNKS];
 #pragma unroll
@@ -268,38 +269,50 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
     // one group each, so that every lane stores a whole core-matrix row of 8.
     const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
     const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
-    const long row0 = static_cast<long>(rg) * 8 * row_steps + wib, row_end = min(rows, row0 + 8L * row_steps);
-    for (long row = row0; row < row_end; row += 8) {
-        uint4 raw[CHUNKS];
+    const int cc = pos >> 3;
+    int buf = 0;
+    const long first = static_cast<long>(rg) * 8 * row_steps, last = min(rows, first + 8L * row_steps);
+    for (long row8 = first; row8 < last; row8 += 8, buf ^= 1) {
+        const long row = row8 + wib;
+        if (have && row < rows) {
+            uint4 raw[CHUNKS];
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
-        float v[CHUNKS][8];
+            for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
+            float v[CHUNKS][8];
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
+            for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
 #pragma unroll
-        for (int h = 1; h < CHUNKS; h <<= 1)
+            for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll
-            for (int i = 0; i < CHUNKS; i += 2 * h)
+                for (int i = 0; i < CHUNKS; i += 2 * h)
 #pragma unroll
-                for (int c = i; c < i + h; ++c)
+                    for (int c = i; c < i + h; ++c)
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float a0 = v[c][j], b0 = v[c + h][j];
-                        v[c][j] = __fadd_rn(a0, b0);
-                        v[c + h][j] = __fsub_rn(a0, b0);
-                    }
-        const long rt = row / kTileTok, rin = row - rt * kTileTok;
+                        for (int j = 0; j < 8; ++j) {
+                            const float a0 = v[c][j], b0 = v[c + h][j];
+                            v[c][j] = __fadd_rn(a0, b0);
+                            v[c + h][j] = __fsub_rn(a0, b0);
+                        }
+#pragma unroll
+            for (int c = 0; c < CHUNKS; ++c) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[c][j] *= inv_sqrt;
+                const uint4 h = pack_halves(v[c]);
+                const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
+                const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
+                const uint4 piece = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
+                s_rows[buf][(4 * c + (lane >> 3)) * 64 + cc * 8 + (wib ^ cc)] = piece;
+            }
+        }
+        __syncthreads();   // (the other buffer's readers are past it when it is written again)
+        const long rt = row8 / kTileTok, rin = row8 - rt * kTileTok;
         const long tile0 = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane;
-        __half* const dst = xrot + tile0 * (kTileTok * kBlockK) + (((rin >> 3) * 8 + (pos >> 3)) * 8 + (rin & 7)) * 8;
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[c][j] *= inv_sqrt;
-            const uint4 h = pack_halves(v[c]);
-            const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
-            const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
-            const uint4 row8 = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
-            *reinterpret_cast<uint4*>(dst + static_cast<long>((col + 256 * c) / kBlockK) * (kTileTok * kBlockK)) = row8;
+            const int t = threadIdx.x & 63, kb = 4 * c + (threadIdx.x >> 6), tc = t >> 3, tr = t & 7;
+            const long kb_at = static_cast<long>(cg) * 4 * CHUNKS + kb;
+            if (kb_at < kb_per_plane && row8 + tr < rows)
+                *reinterpret_cast<uint4*>(xrot + (tile0 + kb_at) * (kTileTok * kBlockK) + ((rin >> 3) * 64 + t) * 8) = s_rows[buf][kb * 64 + tc * 8 + (tr ^ tc)];
         }
     }
 }
@@ -316,7 +329,7 @@ struct RotateGroupArgs {
     uint32_t seed_p[4], seed_r[4];
 };
 template <int CHUNKS>
-__global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const RotateGroupArgs g, int in,
+__global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
                                                                          long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
     pdl_wait_release();
     rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
