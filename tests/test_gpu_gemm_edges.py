@@ -1,4 +1,4 @@
-"""The many-row linear at the edges of its tiles: weight rows around the 16-row code tiles and the 128-row tile, activation
+"""The many-row linear at the edges of its tiles and of the tile loop: weight rows around the 16-row code tiles and the 128-row tile, activation
 rows around the 16-row MMA step and the 256-row tile, every WHT block size, K blocks that do not fill a stage, one and two
 rotations.  Tolerance: fp16 rounds the rotated activation, the table and the result by up to 2^-11 each, independently; the
 root mean square of three such errors over a row is below 2^-11 * sqrt(3 / 3) = 4.9e-4."""
@@ -19,6 +19,11 @@ CASES = [
     (257, 1024, 1024, 255, True),
     (113, 1536, 512, 257, True),
     (96, 2048, 1024, 10, False),
+    (200, 320, 64, 300, False),       # two rotations and full tiles: the shortest ring
+    # more tiles than SMs: the ring runs on from tile to tile
+    (57000, 64, 64, 20, True),        # one stage per tile, two accumulators in turn
+    (19100, 192, 64, 257, False),     # ... one accumulator, an odd number of K blocks, a short last token tile
+    (38000, 320, 64, 130, True),
 ]
 
 

@@ -32,7 +32,13 @@
 //              copies' bytes), issues its eight MMAs, commits to the stage's "empty" barrier.  The
 //              serial chain of this thread (wait, fence, issue, commit) is what bounds the kernel when
 //              the MMAs are short, hence few and long stages.
-//   warps 0-15 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16
+//   warps 18-21 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
+//              next tile's products (up to 128 activation rows: two accumulators in turn; above, the next
+//              tile's first MMA waits until this one is read)
+// A CTA per SM walks the output tiles and its ring of stages runs on from tile to tile: with a CTA per
+// tile, set-up, first loads and epilogue took 8 to 18 of 47 thousand cycles (5120 x 55296: 89 -> 76 us at
+// 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the producers bound it (about 500 cycles per 128 x 64
+// weights), at 256 the shared-memory pipe: lookups, code loads, the activation tile's write and its read.
 // The activation tile is as tall as the rows it really has (in steps of 16): a decode batch of 9..64
 // rows costs a short MMA and a short copy, so the codes are streamed once whatever the batch.
 // The dequantised weights never touch HBM; a weight tile is looked up once per 256 activation
