@@ -33,6 +33,56 @@ def test_host_rows_equal_device_rows(tq, rows, n_in, dtype):
     lin.close()
 
 
+@pytest.mark.parametrize("rows,n_in", [(1, 4096), (2, 4160), (5, 3200)])   # parameters and staging, as pageable rows
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+def test_page_locked_rows_are_read_in_stream_order(tq, rows, n_in, dtype):
+    """Work queued on the stream writes the page-locked rows: the forward that follows sees what it wrote."""
+    torch = pytest.importorskip("torch")
+    lin = make_linear(tq, n_in, 80)
+    x = torch.randn((rows, n_in), device="cuda").to(getattr(torch, dtype))
+    want = lin.forward(x)
+    a = torch.randn((8192, 8192), device="cuda")
+    pinned = torch.zeros((rows, n_in), dtype=x.dtype).pin_memory()
+    got = torch.empty_like(want)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for stream in (torch.cuda.default_stream(), side):
+        pinned.zero_()
+        with torch.cuda.stream(stream):
+            for _ in range(4):
+                a = a @ a * 1e-4                       # tens of milliseconds
+            pinned.copy_(x, non_blocking=True)
+            lin.forward(pinned, out=got, stream=stream)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    lin.close()
+
+
+@pytest.mark.parametrize("dtype", ["float16", "float32"])
+def test_a_captured_forward_reads_page_locked_rows_on_every_replay(tq, dtype):
+    torch = pytest.importorskip("torch")
+    lin = make_linear(tq, 1024, 80)
+    x = [torch.randn((3, 1024), device="cuda").to(getattr(torch, dtype)) for _ in range(3)]
+    want = [lin.forward(t) for t in x]
+    pinned = torch.zeros((3, 1024), dtype=x[0].dtype).pin_memory()
+    got = torch.empty_like(want[0])
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        lin.forward(pinned, out=got, stream=side)      # allocates what the capture must not
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        lin.forward(pinned, out=got, stream=side)
+    for t, w in zip(x, want):
+        pinned.copy_(t)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, w)
+    del graph
+    lin.close()
+
+
 def test_a_recycled_cache_waits_for_its_predecessor(tq):
     """Storage released with work still queued is reused behind that work, on the same stream and on another one."""
     torch = pytest.importorskip("torch")

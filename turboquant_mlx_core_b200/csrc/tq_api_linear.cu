@@ -139,16 +139,20 @@ public:
         const bool x_dev = kx.device, y_dev = ky.device;
 
         // Host memory, a decode call: a few rows travel as kernel parameters, more of them through page-locked staging
-        // (the call waits for its result, so the staging is free again when it returns); see tq_host_rows.cu.
+        // (the call waits for its result, so the staging is free again when it returns); see tq_host_rows.cu.  Both read the
+        // rows now, which is right for pageable memory only: page-locked rows may be written by work that is still queued
+        // on the stream, and a captured copy reads its source anew on every replay, so these stay copies on the stream.
         const bool decode_call = batch <= 8 || nx * sizeof(__half) <= kHostStageBytes;
+        const bool read_now = !x_dev && kx.pinned_alias == nullptr && !is_capturing(st);
+        const bool as_params = read_now && nx * sizeof(__half) <= tq::kMaxParamRowBytes;
         const __half* d_x;
         std::optional<tq::PinnedStage> x_stage, y_stage;
         if (x_dev && x_dtype == TQ_F16) {
             d_x = static_cast<const __half*>(x);
-        } else if (!x_dev && (nx * sizeof(__half) <= tq::kMaxParamRowBytes || (!y_dev && decode_call && kx.pinned_alias == nullptr))) {
+        } else if (as_params || (read_now && !y_dev && decode_call)) {
             x_f16_.reserve(nx * sizeof(__half) + 16, st);
             d_x = x_f16_.as<__half>();
-            if (nx * sizeof(__half) <= tq::kMaxParamRowBytes) {
+            if (as_params) {
                 tq::launch_rows_from_params(x, x_dtype == TQ_F16, nx, x_f16_.as<__half>(), st);
             } else {
                 x_stage.emplace(nx * sizeof(__half));
@@ -408,6 +412,12 @@ private:
         kinds_[next_kind_] = k;
         next_kind_ = (next_kind_ + 1) & 3;
         return k;
+    }
+    static bool is_capturing(cudaStream_t st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+        cudaGetLastError();
+        return true;   // the legacy stream while another one of the device is captured
     }
     PointerKind kinds_[4];
     int next_kind_ = 0;
