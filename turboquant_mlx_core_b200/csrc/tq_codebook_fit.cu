@@ -177,8 +177,9 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
     const int nc = state->n;
     if (tid < nc) s_c[tid] = state->centroids[tid];
     if (tid < nc - 1) s_b[tid] = state->boundaries[tid];
+    const bool finite = state->max_bits < 0x7f800000u;
     if (tid == 0) {
-        s_stop = state->max_bits >= 0x7f800000u ? 1 : 0;
+        s_stop = finite ? 0 : 1;
         s_converged = 0;
     }
     const double unit = fit_unit(state->max_bits, log2_n);
@@ -212,7 +213,8 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
     unsigned int b_at = 0, b_count = 0;  // the boundary's bucket, and the sum of everything before it
     long long b_sum = 0;
     int it = 0;
-    for (; it < iterations && !s_stop && !s_converged; ++it) {
+    // (s_stop is set between the barriers of an iteration, so only the check behind the first of them reads it)
+    for (; finite && it < iterations && !s_converged; ++it) {
         if (warp < nc - 1) {
             const float bound = s_b[warp];
             const int now = static_cast<int>(fit_key(bound) >> shift);
