@@ -7,14 +7,20 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [1, 255, 8193, 65537, 1_000_003])
-@pytest.mark.parametrize("kind", ["scaled", "outliers", "one value", "few values", "zeros"])
+@pytest.mark.parametrize("kind", ["scaled", "outliers", "1e9", "1e12", "-1e15", "lowest", "wide", "one value", "few values", "zeros"])
 def test_fit_against_the_checker(tq, oracle, n, kind):
     rng = np.random.default_rng(n)
     x = rng.standard_normal(n)
     if kind == "scaled":                # far from the codebook it starts from
         x = x * 1e-3 + 5e-4
-    elif kind == "outliers":            # the sums' unit follows the largest magnitude
+    elif kind == "outliers":            # other bins' values must not enter a bin's sum
         x[:: max(1, n // 7)] *= 1e6
+    elif kind in ("1e9", "1e12", "-1e15"):
+        x[n // 2] = float(kind)
+    elif kind == "lowest":              # masked samples
+        x[:: max(1, n // 5)] = np.finfo(np.float32).min
+    elif kind == "wide":                # 60 decades, and buckets of several exponents in a group
+        x = x * 10.0 ** rng.uniform(-30, 30, n)
     elif kind == "one value":
         x[:] = 0.37
     elif kind == "few values":          # more of each than a bucket may hold (from 65537 on)
@@ -25,6 +31,4 @@ def test_fit_against_the_checker(tq, oracle, n, kind):
     want, _ = oracle.fit_codebook(x, 4, 20)
     got = tq.generate_codebook_from_data(x, 4, 20)
     tol = 3e-6 * np.abs(want) + 3e-7
-    if kind == "outliers":
-        tol = tol + 3e-6 * np.abs(x).max() / 1e6      # both sides round sums that an outlier dominates
     assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()

@@ -3,18 +3,19 @@
 //
 // An iteration needs, for every boundary, the count and the sum of the values at or below it.  Going over all samples for
 // that took 110 us per iteration at 16.8 M samples, a hundred times.  Instead the samples are bucketed ONCE by the leading
-// bits of their order-preserving key (sign, exponent, a few mantissa bits), with running counts and sums per bucket; a
+// bits of their order-preserving key (sign, exponent, a few mantissa bits), with running counts and a sum per bucket; a
 // boundary then only looks at the values of its own bucket, and all iterations run in one launch of one CTA, a warp per
-// boundary (about 1 us each).
+// boundary and bin (about 1 us each).
 //   fit_count_kernel      bucket counts, largest magnitude            (one pass over the samples)
 //   fit_groups / fit_offsets   exclusive scan of the counts, 256 buckets per group
 //   fit_scatter_kernel    samples into their buckets                  (one pass)
 //   fit_sums_kernel       sum of every bucket
 //   fit_iterate_kernel    the iterations
 // A value equal to a boundary goes to the lower bin, as std::lower_bound in the reference's CPU path and quantize() have
-// it.  Sums are 64-bit integers in units of 2^-s, s chosen so that n values cannot overflow: exact up to the rounding of
-// values below 2^-37 of the largest, the accuracy of the reference's double sums, and independent of the order in which the
-// scatter placed the values - results are run-to-run identical.
+// it.  All values of a bucket have one sign and exponent, so a bucket's sum, and the sum of its values up to a boundary, is an
+// exact 64-bit integer of significands.  A bin is the double sum of the buckets between its boundaries and those two partial
+// ones, in a fixed order: only its own values enter, as in the reference's double sums, whatever the magnitudes of the
+// others (running sums over all buckets would lose a bin beside an outlier), and results are run-to-run identical.
 // A boundary whose bucket holds more than kFitMaxBucket values (samples with heavy repetition), or samples that are not
 // finite, stop fit_iterate_kernel; the remaining iterations then go over all samples:
 //   fit_partial_kernel   every thread bins its values by lower_bound over the current boundaries into a PRIVATE histogram in
@@ -59,12 +60,18 @@ __device__ __forceinline__ unsigned int fit_key(float x) {
     const unsigned int u = __float_as_uint(x);
     return u ^ ((u & 0x80000000u) ? 0xffffffffu : 0x80000000u);
 }
-// A sample in units of 2^-s.
-__device__ __forceinline__ long long fit_fixed(float x, double unit) { return __double2ll_rn(static_cast<double>(x) * unit); }
-// The unit for samples of magnitude up to max_bits: n of them stay below 2^62.
-__device__ __forceinline__ double fit_unit(unsigned int max_bits, int log2_n) {
-    const int e = static_cast<int>(max_bits >> 23) - 126;   // every magnitude is below 2^e
-    return exp2(static_cast<double>(62 - log2_n - e));
+// The values of a bucket agree in all bits above `shift` (the sign, the exponent, 3 of the mantissa at least), so a value is
+// (base + its bits below `shift`) units; the unit carries the sign.
+struct FitBucket {
+    unsigned int base;
+    double unit;
+};
+__device__ __forceinline__ FitBucket fit_bucket(int bucket, int shift) {
+    const unsigned int key = static_cast<unsigned int>(bucket) << shift;
+    const unsigned int u = (key & 0x80000000u) ? key ^ 0x80000000u : ~(key | ((1u << shift) - 1u));
+    const unsigned int e = (u >> 23) & 0xffu;
+    const double unit = __longlong_as_double(static_cast<long long>(max(e, 1u) - 150u + 1023u) << 52);
+    return FitBucket{(u & 0x7fffffu) | (e != 0u ? 0x800000u : 0u), (u & 0x80000000u) ? -unit : unit};
 }
 
 __global__ void __launch_bounds__(256) fit_count_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ count,
@@ -136,14 +143,15 @@ __global__ void __launch_bounds__(256) fit_scatter_kernel(const float* __restric
             if (pos[k] != 0xffffffffu) sorted[pos[k]] = x[k];
     }
 }
-// A block per kFitSumBuckets buckets, a warp per bucket: bucket sums, added up to the group's (integers: in any order).  The
-// samples lie in about a hundred of the groups; with a block per group those few blocks took 450 us for 16.8 M samples.
+// A block per kFitSumBuckets buckets, a warp per bucket: bucket sums, and the double sum of the block's.  The samples lie in
+// about a hundred groups of 256 buckets; with a block per group those few blocks took 450 us for 16.8 M samples.
 __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__ sorted, const unsigned int* __restrict__ count,
-                                                       const unsigned int* __restrict__ offset, int log2_n, const FitState* __restrict__ state,
-                                                       long long* __restrict__ sum, unsigned long long* __restrict__ group_sum) {
+                                                       const unsigned int* __restrict__ offset, int shift, double* __restrict__ sum,
+                                                       double* __restrict__ part) {
+    __shared__ double s_warp[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double unit = fit_unit(state->max_bits, log2_n);
-    long long total = 0;
+    const unsigned int below = (1u << shift) - 1u;
+    double total = 0.0;
     for (int k = warp; k < kFitSumBuckets; k += 8) {
         const int b = blockIdx.x * kFitSumBuckets + k;
         const unsigned int c = count[b], at = offset[b];
@@ -152,27 +160,44 @@ __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__
             float x[kFitBatch];
 #pragma unroll
             for (int j = 0; j < kFitBatch; ++j) x[j] = i + 32u * j < c ? sorted[at + i + 32u * j] : 0.f;
+            unsigned int t = 0;   // 8 x 2^20 at most
 #pragma unroll
-            for (int j = 0; j < kFitBatch; ++j) s += fit_fixed(x[j], unit);
+            for (int j = 0; j < kFitBatch; ++j) t += __float_as_uint(x[j]) & below;
+            s += t;
         }
+        double v = 0.0;
         if (c != 0) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const FitBucket k = fit_bucket(b, shift);
+            v = static_cast<double>(s + static_cast<long long>(c) * k.base) * k.unit;
+            total += v;
         }
-        if (lane == 0) sum[b] = s;
-        total += s;
+        if (lane == 0) sum[b] = v;
     }
-    if (lane == 0 && total != 0) atomicAdd(&group_sum[blockIdx.x / (kFitGroup / kFitSumBuckets)], static_cast<unsigned long long>(total));
+    if (lane == 0) s_warp[warp] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) total += s_warp[w];
+        part[blockIdx.x] = total;
+    }
 }
-// All iterations: warp w follows boundary w.  `before_sum`: scratch for the exclusive scan of the groups' sums.
+// All iterations: warp w follows boundary w, the upper one of bin w.  Bound by the latency of a chain of L2 reads and
+// reductions in one CTA, and by issue: 100 iterations over 16.8 M samples take 385 us.  (Significands as 64-bit sums of doubles'
+// conversions took 400 to 660 us; the bits below a bucket's prefix are 32-bit sums.)  `group_sum`: filled here from the parts.
 __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restrict__ sorted, unsigned int n, const unsigned int* __restrict__ count,
-                                                           const unsigned int* __restrict__ offset, const long long* __restrict__ sum,
-                                                           const long long* __restrict__ group_sum, int n_groups, long long* __restrict__ before_sum,
-                                                           int shift, int log2_n, int iterations, FitState* __restrict__ state) {
+                                                           const unsigned int* __restrict__ offset, const double* __restrict__ sum,
+                                                           const double* __restrict__ part, int n_groups, double* __restrict__ group_sum,
+                                                           int shift, int iterations, FitState* __restrict__ state) {
     __shared__ float s_c[kFitMaxBins], s_b[kFitMaxBins];
-    __shared__ long long s_le_sum[kFitMaxBins + 1], s_part[33];
-    __shared__ unsigned int s_le[kFitMaxBins + 1];
-    __shared__ int s_stop, s_converged;
+    // Per boundary: its bucket, that bucket's unit and sum, the sums of its group's buckets before and after it; the samples up
+    // to the boundary, those before the bucket included, and the significands of the ones in the bucket.
+    __shared__ int s_bucket[kFitMaxBins];
+    __shared__ double s_unit[kFitMaxBins], s_own[kFitMaxBins], s_before[kFitMaxBins], s_after[kFitMaxBins];
+    __shared__ unsigned int s_le[kFitMaxBins];
+    __shared__ long long s_low[kFitMaxBins];
+    __shared__ double s_mid[kFitMaxBins];      // per bin: the groups between its boundaries' (or the buckets, where they share one)
+    __shared__ int s_stop, s_converged, s_moved, s_near;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nc = state->n;
     if (tid < nc) s_c[tid] = state->centroids[tid];
@@ -180,58 +205,39 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
     const bool finite = state->max_bits < 0x7f800000u;
     if (tid == 0) {
         s_stop = finite ? 0 : 1;
-        s_converged = 0;
+        s_converged = s_moved = s_near = 0;
     }
-    const double unit = fit_unit(state->max_bits, log2_n);
-    // exclusive scan of the groups' sums: a contiguous run of groups per thread
-    const int per = (n_groups + 1023) / 1024;
-    long long own = 0;
-    for (int k = 0; k < per; ++k) {
-        const int g = tid * per + k;
-        if (g < n_groups) own += group_sum[g];
-    }
-    long long scan = own;
+    constexpr int kParts = kFitGroup / kFitSumBuckets;
+    for (int g = tid; g < n_groups; g += 1024) {
+        double v[kParts], s = 0.0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, scan, o);
-        if (lane >= o) scan += t;
+        for (int k = 0; k < kParts; ++k) v[k] = part[g * kParts + k];
+#pragma unroll
+        for (int k = 0; k < kParts; ++k) s += v[k];
+        group_sum[g] = s;
     }
-    if (lane == 31) s_part[warp] = scan;
-    __syncthreads();
-    long long run = scan - own;
-    for (int w = 0; w < warp; ++w) run += s_part[w];
-    for (int k = 0; k < per; ++k) {
-        const int g = tid * per + k;
-        if (g < n_groups) {
-            before_sum[g] = run;
-            run += group_sum[g];
-        }
-    }
-    if (tid == 1023) s_part[32] = run;   // of all samples
-    __syncthreads();                     // (also makes before_sum visible within the block)
-    int bucket = -1;
-    unsigned int b_at = 0, b_count = 0;  // the boundary's bucket, and the sum of everything before it
-    long long b_sum = 0;
+    __syncthreads();   // (also makes group_sum visible within the block)
+    int bucket = -1;                       // of the boundary, as of its last iteration
+    unsigned int b_at = 0, b_count = 0, base = 0;
     int it = 0;
     // (s_stop is set between the barriers of an iteration, so only the check behind the first of them reads it)
     for (; finite && it < iterations && !s_converged; ++it) {
         if (warp < nc - 1) {
-            const float bound = s_b[warp];
+            const float bound = s_b[warp] + 0.0f;   // -0 as +0: the two zeros lie in neighbouring buckets
             const int now = static_cast<int>(fit_key(bound) >> shift);
-            if (now != bucket) {
+            const bool changed = now != bucket;
+            bool moved = false;
+            double near[kFitGroup / 32];         // the group's buckets: requested before the bucket's samples, added up after them
+            if (changed) {
+                moved = bucket < 0 || now / kFitGroup != bucket / kFitGroup || s_near != 0;
                 bucket = now;
                 b_at = offset[now];
                 b_count = count[now];
-                const int g = now / kFitGroup;
-                long long s = 0;
-                for (int b = g * kFitGroup + lane; b < now; b += 32) s += sum[b];
+                base = fit_bucket(now, shift).base;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                b_sum = before_sum[g] + s;
-                if (b_count > kFitMaxBucket && lane == 0) s_stop = 1;
+                for (int k = 0; k < kFitGroup / 32; ++k) near[k] = sum[now / kFitGroup * kFitGroup + 32 * k + lane];
             }
-            unsigned int c = 0;
-            long long s = 0;
+            unsigned int c = 0, t = 0;   // t: 1024 x 2^20 at most
             if (b_count <= kFitMaxBucket) {
                 for (unsigned int i = lane; i < b_count; i += 32 * kFitBatch) {
                     float x[kFitBatch];
@@ -239,29 +245,94 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
                     for (int j = 0; j < kFitBatch; ++j) x[j] = i + 32u * j < b_count ? sorted[b_at + i + 32u * j] : INFINITY;
 #pragma unroll
                     for (int j = 0; j < kFitBatch; ++j) {
-                        const bool le = !(bound < x[j]) && i + 32u * j < b_count;
+                        const bool le = !(bound < x[j]);   // (the padding is not)
                         c += le ? 1u : 0u;
-                        s += le ? fit_fixed(x[j], unit) : 0ll;
+                        t += le ? __float_as_uint(x[j]) & ((1u << shift) - 1u) : 0u;
                     }
                 }
             }
             c = __reduce_add_sync(0xffffffffu, c);
+            const unsigned int t_high = __reduce_add_sync(0xffffffffu, t >> 16), t_low = __reduce_add_sync(0xffffffffu, t & 0xffffu);
+            if (changed) {
+                double low[kFitGroup / 32];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                for (int k = 0; k < kFitGroup / 32; ++k) {
+                    const int b = now / kFitGroup * kFitGroup + 32 * k + lane;
+                    if (b == now) s_own[warp] = near[k];
+                    low[k] = b < now ? near[k] : 0.0;
+                    near[k] = b > now ? near[k] : 0.0;
+                }
+#pragma unroll
+                for (int h = kFitGroup / 64; h > 0; h >>= 1)
+#pragma unroll
+                    for (int k = 0; k < h; ++k) {
+                        low[k] += low[k + h];
+                        near[k] += near[k + h];
+                    }
+                const double before = low[0], after = near[0];
+                // the lower half of the lanes adds up `before`, the upper half `after`
+                double v = (lane & 16) ? after : before;
+                v += __shfl_xor_sync(0xffffffffu, (lane & 16) ? before : after, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == 16) s_after[warp] = v;
+                if (lane == 0) {
+                    s_before[warp] = v;
+                    s_bucket[warp] = now;
+                    s_unit[warp] = fit_bucket(now, shift).unit;
+                    if (moved) s_moved = 1;
+                    if (b_count > kFitMaxBucket) s_stop = 1;
+                }
+            }
             if (lane == 0) {
                 s_le[warp] = b_at + c;
-                s_le_sum[warp] = b_sum + s;
+                s_low[warp] = (static_cast<long long>(t_high) << 16) + t_low + static_cast<long long>(c) * base;
             }
         }
         __syncthreads();
         if (s_stop) break;   // nothing of this iteration has been applied
+        if (s_moved) {       // a boundary is in another group than before: the sums of the groups in between
+            if (warp < nc) {
+                const int lo = warp > 0 ? s_bucket[warp - 1] : -1, hi = warp < nc - 1 ? s_bucket[warp] : n_groups * kFitGroup;
+                const int g_lo = warp > 0 ? lo / kFitGroup : -1, g_hi = hi / kFitGroup;
+                const bool groups = g_lo != g_hi;
+                const double* const from = groups ? group_sum : sum;
+                const int end = groups ? g_hi : hi;
+                double mid = 0.0;
+                for (int i = (groups ? g_lo : lo) + 1 + lane; i < end; i += 32 * kFitBatch) {
+                    double v[kFitBatch];
+#pragma unroll
+                    for (int j = 0; j < kFitBatch; ++j) v[j] = i + 32 * j < end ? from[i + 32 * j] : 0.0;
+#pragma unroll
+                    for (int j = 0; j < kFitBatch; ++j) mid += v[j];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) mid += __shfl_xor_sync(0xffffffffu, mid, o);
+                if (lane == 0) {
+                    s_mid[warp] = mid;
+                    if (!groups) s_near = 1;   // (stays: every further move counts then)
+                }
+            }
+            __syncthreads();
+        }
         if (warp == 0) {
             float shift_of = 0.f, c_new = lane < nc ? s_c[lane] : 0.f;
             if (lane < nc) {
-                const unsigned int hi = lane < nc - 1 ? s_le[lane] : n, lo = lane > 0 ? s_le[lane - 1] : 0u;
-                const long long hs = lane < nc - 1 ? s_le_sum[lane] : s_part[32], ls = lane > 0 ? s_le_sum[lane - 1] : 0ll;
-                if (hi > lo) {   // an empty bin keeps its centroid
-                    const float mean = static_cast<float>(static_cast<double>(hs - ls) / unit / static_cast<double>(hi - lo));
+                const bool has_lo = lane > 0, has_hi = lane < nc - 1;
+                const unsigned int above = has_hi ? s_le[lane] : n, below = has_lo ? s_le[lane - 1] : 0u;
+                if (above > below) {   // an empty bin keeps its centroid
+                    const int lo = has_lo ? s_bucket[lane - 1] : -1, hi = has_hi ? s_bucket[lane] : n_groups * kFitGroup;
+                    const bool groups = !has_lo || lo / kFitGroup != hi / kFitGroup;
+                    double total;
+                    if (lo == hi) {
+                        total = static_cast<double>(s_low[lane] - s_low[lane - 1]) * s_unit[lane];
+                    } else {
+                        total = s_mid[lane];
+                        // (both terms are whole numbers of the bucket's unit: exact)
+                        if (has_lo) total += s_own[lane - 1] - static_cast<double>(s_low[lane - 1]) * s_unit[lane - 1] + (groups ? s_after[lane - 1] : 0.0);
+                        if (has_hi) total += static_cast<double>(s_low[lane]) * s_unit[lane] + (groups ? s_before[lane] : 0.0);
+                    }
+                    const float mean = static_cast<float>(total / static_cast<double>(above - below));
                     shift_of = fabsf(mean - c_new);
                     c_new = mean;
                 }
@@ -271,7 +342,10 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
             const float c_next = __shfl_down_sync(0xffffffffu, c_new, 1);
             if (lane < nc) s_c[lane] = c_new;
             if (lane + 1 < nc) s_b[lane] = __fmul_rn(__fadd_rn(c_new, c_next), 0.5f);
-            if (lane == 0 && shift_of < kFitShiftThreshold) s_converged = 1;
+            if (lane == 0) {
+                s_moved = 0;   // (the others have read it, or read the zero that it still is)
+                if (shift_of < kFitShiftThreshold) s_converged = 1;
+            }
         }
         __syncthreads();
     }
@@ -450,12 +524,13 @@ int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, c
             while ((1L << log2_n) < n) ++log2_n;
             const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13)), shift = 32 - key_bits, n_buckets = 1 << key_bits;
             const int n_groups = n_buckets / kFitGroup;
-            bucket_buf.reserve(static_cast<size_t>(n_buckets) * (3 * 4 + 8) + static_cast<size_t>(n_groups) * (8 + 8 + 4), stream);
+            const int n_parts = n_buckets / kFitSumBuckets;
+            bucket_buf.reserve(static_cast<size_t>(n_buckets) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups) * 8 + static_cast<size_t>(n_groups) * 4, stream);
             sorted_buf.reserve(static_cast<size_t>(n) * 4, stream);
-            long long* const d_sum = bucket_buf.as<long long>();
-            long long* const d_group_sum = d_sum + n_buckets;
-            long long* const d_before = d_group_sum + n_groups;
-            unsigned int* const d_count = reinterpret_cast<unsigned int*>(d_before + n_groups);
+            double* const d_sum = bucket_buf.as<double>();
+            double* const d_part = d_sum + n_buckets;
+            double* const d_group_sum = d_part + n_parts;
+            unsigned int* const d_count = reinterpret_cast<unsigned int*>(d_group_sum + n_groups);
             unsigned int* const d_offset = d_count + n_buckets;
             unsigned int* const d_cursor = d_offset + n_buckets;
             unsigned int* const d_group = d_cursor + n_buckets;
@@ -467,11 +542,8 @@ int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, c
             fit_groups_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group);
             fit_offsets_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group, d_offset, d_cursor);
             fit_scatter_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_cursor, d_sorted);
-            TQ_CUDA(cudaMemsetAsync(d_group_sum, 0, static_cast<size_t>(n_groups) * 8, stream));
-            fit_sums_kernel<<<n_buckets / kFitSumBuckets, 256, 0, stream>>>(d_sorted, d_count, d_offset, log2_n, d_state, d_sum,
-                                                                           reinterpret_cast<unsigned long long*>(d_group_sum));
-            fit_iterate_kernel<<<1, 1024, 0, stream>>>(d_sorted, un, d_count, d_offset, d_sum, d_group_sum, n_groups, d_before, shift, log2_n,
-                                                       iterations, d_state);
+            fit_sums_kernel<<<n_parts, 256, 0, stream>>>(d_sorted, d_count, d_offset, shift, d_sum, d_part);
+            fit_iterate_kernel<<<1, 1024, 0, stream>>>(d_sorted, un, d_count, d_offset, d_sum, d_part, n_groups, d_group_sum, shift, iterations, d_state);
             TQ_CUDA(cudaGetLastError());
             read_state();
         }
