@@ -51,3 +51,48 @@ def test_attention_work_split(tq, oracle, case, qjl):
     assert np.array_equal(np.asarray(got).view(np.uint16), np.asarray(again).view(np.uint16))
     for c in caches:
         c.close()
+
+
+def encoded(tq, oracle, k, v):
+    heads, dim = k.shape[1:]
+    c = tq.TQKVCache(1, heads, dim)
+    c.append(0, k, v)
+    kw, kn, qw, qn = oracle.kv_encode(k, oracle.kv_seed(0, 1), oracle.kv_seed(0, 3))
+    vw, vn, _, _ = oracle.kv_encode(v, oracle.kv_seed(0, 2))
+    return c, (kw, kn, vw, vn, qw, qn)
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+@pytest.mark.parametrize("norm", [1e-6, 1e-3, 1e4, 5e4])
+def test_attention_takes_any_value_norm(tq, oracle, dim, norm):
+    """Value norms at both ends of what an fp16 result can hold, some of them zero: the largest weight times norm is brought
+    into fp16's range whatever it is."""
+    heads, q_heads, n = 2, 6, 700
+    k, v = (t.astype(np.float32) for t in kv_inputs(dim, n, heads, dim))
+    v *= norm / np.linalg.norm(v, axis=-1).mean()
+    v[5:9] = 0.0
+    v[40:60] *= 1e-3
+    c, codes = encoded(tq, oracle, k, v)
+    q = np.random.default_rng(dim).standard_normal((1, q_heads, dim)).astype(np.float16)
+    got, lse = tq.compressed_attention([c], 0, q, use_qjl=True, return_lse=True)
+    want = oracle.attention(q[0].astype(np.float32), heads, *codes, layer=0, use_qjl=True)
+    assert np.all(np.isfinite(got.astype(np.float32))) and np.all(np.isfinite(lse))
+    off = np.linalg.norm(got[0].astype(np.float64) - want)
+    assert off < TOL * np.linalg.norm(want) + 2.0 ** -25 * np.sqrt(want.size), off   # half of fp16's smallest step
+    c.close()
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128, 256])
+@pytest.mark.parametrize("scale", [1e-4, 1e4])
+def test_attention_takes_any_query_scale(tq, oracle, dim, scale):
+    """Queries near the ends of fp16's range against keys of the inverse scale: the rotated query, and the query with the
+    residual's signs, keep all their bits."""
+    heads, q_heads, n = 2, 6, 700
+    k, v = (t.astype(np.float32) for t in kv_inputs(dim, n, heads, dim))
+    c, codes = encoded(tq, oracle, (k / np.float32(scale)), v)
+    q = (np.random.default_rng(dim).standard_normal((1, q_heads, dim)) * scale).astype(np.float16)
+    got = tq.compressed_attention([c], 0, q, use_qjl=True)
+    want = oracle.attention(q[0].astype(np.float32), heads, *codes, layer=0, use_qjl=True)
+    # without the scaling 8e-4 at 128 dims and 4e-4 to 1.1e-3 at the others, with it what a scale of one has
+    assert rel_l2(got[0], want) < (7e-4 if dim == 128 else 4e-4)
+    c.close()

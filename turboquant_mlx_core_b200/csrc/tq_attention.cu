@@ -72,8 +72,8 @@ struct AttnCfg {
     static constexpr uint32_t kOffQsl = kOffQl + (kSplit ? kGroup * kQStride * 2 : 0);
     static constexpr uint32_t kOffPub = kOffQsl + (kSplit ? kGroup * kQStride * 2 : 0);
     static constexpr uint32_t kOffOut = kOffPub + kHalf * kPubBytes;
-    static constexpr uint32_t kOffMl = kOffOut + kGroup * kAccStride * 4;               // [2][kHalf][8], then flags and the job
-    static constexpr uint32_t kTeamBytes = kOffMl + 2 * kHalf * kGroup * 4 + 80 - kOffQ;   // of one team, from kOffQ on
+    static constexpr uint32_t kOffMl = kOffOut + kGroup * kAccStride * 4;               // [2][kHalf][8], then flags, the job and the queries' scales
+    static constexpr uint32_t kTeamBytes = kOffMl + 2 * kHalf * kGroup * 4 + 80 + kGroup * 4 - kOffQ;   // of one team, from kOffQ on
     static constexpr uint32_t kEnd = kOffQ + kTeams * kTeamBytes;
     static constexpr int kPartFloats = kGroup * D + 2 * kGroup;                // a job part in scratch: accumulators, then (max, sum)
     static_assert(kPubBytes >= kGroup * kAccStride * 4, "a warp's accumulator in head order fits its place");
@@ -115,6 +115,12 @@ __device__ __forceinline__ float exp2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+// The larger one, NaN where either is.
+__device__ __forceinline__ float max_or_nan(float x, float y) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(x), "f"(y));
+    return m;
 }
 __device__ __forceinline__ unsigned long long timer_ns() {
     unsigned long long t;
@@ -205,6 +211,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     // The job's fields that only its end needs, kept out of the tile loop's registers: two of them, the next job is located
     // before the last one's end.
     volatile int* const s_job = reinterpret_cast<volatile int*>(s_l + C::kHalf * kGroup) + 4;
+    float* const s_scale = reinterpret_cast<float*>(const_cast<int*>(s_job)) + 16;   // per query head: a product's weight in the score
     int job_slot = 0;
 
     if (lane == 0) {
@@ -302,10 +309,11 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     if (a.seqs.table == nullptr) pdl_wait_release();
     if (lane == 0) request_first(seg);
     for (;;) {
-        // ---- rotated queries: fp16-round, sign, butterfly, 1 / sqrt(D), fp16-round (a warp per head) ----
+        // ---- rotated queries: fp16-round, sign, butterfly, 1 / sqrt(D) (a warp per head), times the power of two that takes
+        // the largest to 2^13 .. 2^14, which the score's scale takes back: small and large queries keep all bits of fp16 ----
         for (int h = warp; h < kGroup; h += C::kTeam) {
             constexpr int E = D / 32;
-            float v[E];
+            float v[E], most = 0.f;
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 const int d = lane * E + j;
@@ -320,12 +328,23 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             warp_fwht<E>(v, lane);
 #pragma unroll
             for (int j = 0; j < E; ++j) {
+                v[j] *= a.inv_sqrt;
+                most = fmaxf(most, fabsf(v[j]));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+            const uint32_t e = __float_as_uint(most) >> 23;
+            const bool scaled = e >= 64 && e < 255;   // not zero, not infinite
+            const float up = scaled ? __uint_as_float((267 - e) << 23) : 1.f, down = scaled ? __uint_as_float((e - 13) << 23) : 1.f;
+            if (lane == 0) s_scale[h] = down * a.score_scale;
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
                 const int d = lane * E + j;
-                const float r = v[j] * a.inv_sqrt;
+                const float r = v[j] * up;
                 s_q[h * C::kQStride + d] = __float2half_rn(r);
                 if constexpr (kSplit) s_ql[h * C::kQStride + d] = __float2half_rn(r - __half2float(__float2half_rn(r)));
                 if constexpr (QJL) {
-                    const float rs = v[j] * (qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>(d)) ? a.qscale : -a.qscale);
+                    const float rs = r * (qjl_sign_is_positive(a.qjl_seed, static_cast<uint32_t>(d)) ? a.qscale : -a.qscale);
                     s_qs[h * C::kQStride + d] = __float2half_rn(rs);
                     // dims 8 w + r and 8 w + r + 4 of a quarter side by side (sign pair 4 w + r)
                     if constexpr (kSplit) s_qsl[h * C::kQStride + (d & ~7) + 2 * (d & 3) + ((d >> 2) & 1)] = __float2half_rn(rs - __half2float(__float2half_rn(rs)));
@@ -337,6 +356,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         // and 8 w + r + 4 of the quarter.
         uint32_t bq[2 * kSteps], bs[QJL ? 2 * kSteps : 1];
         float c2_init[2] = {0.f, 0.f};
+        const float scale0 = s_scale[2 * q], scale1 = s_scale[2 * q + 1];   // of the heads of an accumulator fragment
         {
             const __half* const sq = s_q + g * C::kQStride + (D / 4) * q;
 #pragma unroll
@@ -362,7 +382,8 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             }
         }
 
-        // Reference of heads 2q, 2q + 1 in units of log2, kNone before the first tile (finite: scores are taken relative to it).
+        // Reference of heads 2q, 2q + 1 in units of log2, kNone before the first tile (finite: scores are taken relative to it);
+        // sum of 2^(score - reference); sum of the values with those weights.
         float m_run[2] = {kNone, kNone}, l_run[2] = {0.f, 0.f};
         float acc[kSteps][4];
 #pragma unroll
@@ -465,10 +486,14 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 load_words<W>(xa, blk + B::kValueOff + (q * 8 + g) * (D / 8));
                 load_words<W>(xb, blk + B::kValueOff + ((q + 4) * 8 + g) * (D / 8));
             }
-            // ---- online softmax with a lazy reference: it moves (and the sums are rescaled) only when some score exceeds
-            // it by more than the slack, so the usual tile needs one vote instead of a reduction over the tokens.  Every
-            // tile holds a token of [start, end), so the reference is finite from a warp's first tile on.
-            constexpr float kSlack = kAttnSoftmaxSlack * 1.4426950408889634f;
+            // ---- online softmax.  What multiplies the values is w = 2^(score - reference) * value norm in fp16, so the
+            // reference follows the largest w, not the largest score: any norm fits, and a weight keeps all its bits down to
+            // 2^-27 of the largest.  It is lazy: it moves (and the sums are rescaled) only when some w no longer fits, so the
+            // usual tile needs one vote instead of a reduction over the tokens.  Every tile holds a token of [start, end), so
+            // the reference is finite from a warp's first tile on.  A norm of next to nothing counts as kLeastNorm (an
+            // output below fp16's range), which bounds the sum of 2^(score - reference) too.
+            constexpr float kMostWeight = 61440.f, kTopBits = 13.f;   // a new reference takes the largest w to 2^kTopBits
+            constexpr float kLeastNorm = 1e-18f, kMostNormBits = 100.f;
             float x0 = c1[0] + c1b[0], x1 = c1[1] + c1b[1], x2 = c1[2] + c1b[2], x3 = c1[3] + c1b[3];
             if constexpr (QJL) {
                 x0 = fmaf(qna, c2[0] + c2b[0], x0);
@@ -476,20 +501,24 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 x2 = fmaf(qnb, c2[2] + c2b[2], x2);
                 x3 = fmaf(qnb, c2[3] + c2b[3], x3);
             }
-            kna *= a.score_scale;
-            knb *= a.score_scale;
+            const float ka0 = kna * scale0, ka1 = kna * scale1, kb0 = knb * scale0, kb1 = knb * scale1;
             // scores relative to the reference: (token g: heads 2q, 2q + 1), (token g + 8: the same)
-            float s00 = fmaf(x0, kna, -m_run[0]), s01 = fmaf(x1, kna, -m_run[1]), s10 = fmaf(x2, knb, -m_run[0]), s11 = fmaf(x3, knb, -m_run[1]);
+            float s00 = fmaf(x0, ka0, -m_run[0]), s01 = fmaf(x1, ka1, -m_run[1]), s10 = fmaf(x2, kb0, -m_run[0]), s11 = fmaf(x3, kb1, -m_run[1]);
             if (token < seg.start || token + kKvTile > seg.end) {   // tokens outside the range, only in a job's end tiles
                 const int ta = token + g, tb = ta + 8;
                 if (ta < seg.start || ta >= seg.end) { s00 = s01 = -INFINITY; vna = 0.f; }
                 if (tb < seg.start || tb >= seg.end) { s10 = s11 = -INFINITY; vnb = 0.f; }
             }
-            if (__any_sync(0xffffffffu, fmaxf(fmaxf(s00, s01), fmaxf(s10, s11)) > kSlack)) {
+            vna = max_or_nan(vna, kLeastNorm);
+            vnb = max_or_nan(vnb, kLeastNorm);
+            float p00 = exp2_approx(s00), p01 = exp2_approx(s01), p10 = exp2_approx(s10), p11 = exp2_approx(s11);
+            float w00 = p00 * vna, w01 = p01 * vna, w10 = p10 * vnb, w11 = p11 * vnb;
+            if (__any_sync(0xffffffffu, fmaxf(fmaxf(w00, w01), fmaxf(w10, w11)) > kMostWeight)) {
                 // absolute again: relative to the first tile's reference (kNone) a score has no bits left
-                const float t00 = s00 == -INFINITY ? s00 : x0 * kna, t01 = s01 == -INFINITY ? s01 : x1 * kna;
-                const float t10 = s10 == -INFINITY ? s10 : x2 * knb, t11 = s11 == -INFINITY ? s11 : x3 * knb;
-                float mx0 = fmaxf(t00, t10), mx1 = fmaxf(t01, t11);
+                const float t00 = s00 == -INFINITY ? s00 : x0 * ka0, t01 = s01 == -INFINITY ? s01 : x1 * ka1;
+                const float t10 = s10 == -INFINITY ? s10 : x2 * kb0, t11 = s11 == -INFINITY ? s11 : x3 * kb1;
+                const float la = fminf(__log2f(vna), kMostNormBits) - kTopBits, lb = fminf(__log2f(vnb), kMostNormBits) - kTopBits;
+                float mx0 = fmaxf(t00 + la, t10 + lb), mx1 = fmaxf(t01 + la, t11 + lb);
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) {
                     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
@@ -501,10 +530,14 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 l_run[1] *= cr1;
                 m_run[0] = mn0;
                 m_run[1] = mn1;
-                s00 = t00 - mn0;
-                s01 = t01 - mn1;
-                s10 = t10 - mn0;
-                s11 = t11 - mn1;
+                p00 = exp2_approx(t00 - mn0);
+                p01 = exp2_approx(t01 - mn1);
+                p10 = exp2_approx(t10 - mn0);
+                p11 = exp2_approx(t11 - mn1);
+                w00 = p00 * vna;
+                w01 = p01 * vna;
+                w10 = p10 * vnb;
+                w11 = p11 * vnb;
 #pragma unroll
                 for (int mt = 0; mt < kSteps; ++mt) {
                     acc[mt][0] *= cr0;
@@ -513,17 +546,16 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                     acc[mt][3] *= cr1;
                 }
             }
-            const float p00 = exp2_approx(s00), p01 = exp2_approx(s01), p10 = exp2_approx(s10), p11 = exp2_approx(s11);
             l_run[0] += p00 + p10;
             l_run[1] += p01 + p11;
             // P^T fragment: (tokens 2q, 2q+1 | 2q+8, 2q+9 ; head g) from (token g | g+8 ; heads 2q, 2q+1)
-            const uint32_t pa = pack_half2(p00 * vna, p01 * vna), pb = pack_half2(p10 * vnb, p11 * vnb);
+            const uint32_t pa = pack_half2(w00, w01), pb = pack_half2(w10, w11);
             pb0 = movmatrix_trans(pa);
             pb1 = movmatrix_trans(pb);
             if constexpr (kSplit) {
                 const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&pa)), fb = __half22float2(*reinterpret_cast<const __half2*>(&pb));
-                pl0 = movmatrix_trans(pack_half2(fmaf(p00, vna, -fa.x), fmaf(p01, vna, -fa.y)));
-                pl1 = movmatrix_trans(pack_half2(fmaf(p10, vnb, -fb.x), fmaf(p11, vnb, -fb.y)));
+                pl0 = movmatrix_trans(pack_half2(w00 - fa.x, w01 - fa.y));
+                pl1 = movmatrix_trans(pack_half2(w10 - fb.x, w11 - fb.y));
             }
         };
         const unsigned char* next_src = seg.src + static_cast<size_t>(warp + 2 * C::kStages * C::kTeam) * tile_stride;
@@ -743,7 +775,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             const float invL = L > 0.f ? 1.0f / L : 0.f;
             const size_t row = static_cast<size_t>(done.q_row0 + h);
             // log of the softmax denominator: lets a caller merge results over disjoint token ranges
-            if (a.lse != nullptr && lane == 0) a.lse[row] = L > 0.f ? M * 0.6931471805599453f + __logf(L) : -INFINITY;
+            if (a.lse != nullptr && lane == 0) a.lse[row] = L > 0.f ? M * 0.6931471805599453f + logf(L) : -INFINITY;
 #pragma unroll
             for (int j = 0; j < E; ++j)
                 a.out[row * D + lane * E + j] = __float2half_rn(v[j] * a.inv_sqrt * sign_value(a.v_seed, static_cast<uint32_t>(lane * E + j)) * invL);
@@ -820,8 +852,8 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long long
     a.inv_scale = a.inv_sqrt / kAttnCentroidScale;   // of the value sums, whose table is scaled as well
     // softmax scale 1 / sqrt(D) (src/attention_dispatch.cpp:35) and the rotation's 1 / sqrt(D), in units of log2
     a.score_scale = static_cast<float>(1.4426950408889634 / d / kAttnCentroidScale);
-    // of the rotated query before its 1 / sqrt(D): the residual's reconstruction, in units of the scaled centroids
-    a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale / std::sqrt(d));
+    // of the rotated query: the residual's reconstruction, in units of the scaled centroids
+    a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale);
     // Two ranges per SM while every range has a tile per warp; fewer for short jobs, whose time is the merge of the parts.
     const int team = 8, teams = head_dim == 256 ? 1 : 2;
     const long most = std::min<long>(static_cast<long>(teams) * sm_count, head_dim == 32 ? AttnCfg<32>::kMaxParts : kMaxRanges);

@@ -107,7 +107,7 @@ __device__ __forceinline__ AttnSeq attn_seq(const AttnSeqs& s, int i) { return s
 // magnitudes round to fp16 with a relative error below 1.4e-5 (unscaled: up to 3e-4, which the
 // softmax amplifies); the factor is divided out of the key and value norms.
 constexpr float kAttnCentroidScale = 1.1979075f;
-// Lazy softmax reference: it only moves when a score exceeds it by more than this.
+// The decode window's lazy softmax reference (tq_attn_dense.cu): it only moves when a score exceeds it by more than this.
 constexpr float kAttnSoftmaxSlack = 2.0f;
 
 // Sets the descriptors' tile0 and returns the tiles of all sequences; `longest`: of the longest.
