@@ -298,6 +298,13 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         bulk_copy(dst, src, B::kBytes, bar);
         if (left > 1) bulk_copy(dst + B::kBytes, src + C::kTeam * tile_stride, B::kBytes, bar);
     };
+    // Before a place in the ring is filled again: every lane's reads of it have ended.  (A tile's value words are needed only
+    // beside the next tile's scores, and nothing else keeps their loads in front of the copy, which is of another proxy.
+    // The fence costs 2 of 92 us at 16 x 32768 tokens.)
+    auto end_reads = [] {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+    };
     auto request_first = [&](const Segment& g) {
         for (int i = 0; i < C::kStages && 2 * i < g.mine; ++i) {
             const int s = stage ^ i;
@@ -568,8 +575,10 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             const uint32_t blk = ring + stage * C::kStageBytes;
             take_tile(blk, token);
             if (left > 1) take_tile(blk + B::kBytes, token + C::kTeam * kKvTile);
-            __syncwarp();
-            if (lane == 0 && left > 2 * C::kStages) request(blk, next_src, left - 2 * C::kStages, bars + 8u * stage);
+            if (left > 2 * C::kStages) {
+                end_reads();
+                if (lane == 0) request(blk, next_src, left - 2 * C::kStages, bars + 8u * stage);
+            }
             next_src += 2 * C::kTeam * tile_stride;
             phase ^= static_cast<uint32_t>(stage);
             stage ^= 1;
@@ -586,7 +595,8 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         if (more) {
             seg = locate(u);
             more = seg.n_tiles > 0;
-            if (lane == 0 && ok) request_first(seg);   // every lane is past its last read of the ring
+            end_reads();
+            if (lane == 0 && ok) request_first(seg);
         }
 
         // ---- merge the warps: the upper half hands its registers to the lower half, which publishes in head order ----
