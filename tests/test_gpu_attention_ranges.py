@@ -96,3 +96,32 @@ def test_attention_takes_any_query_scale(tq, oracle, dim, scale):
     # without the scaling 8e-4 at 128 dims and 4e-4 to 1.1e-3 at the others, with it what a scale of one has
     assert rel_l2(got[0], want) < (7e-4 if dim == 128 else 4e-4)
     c.close()
+
+
+@pytest.mark.parametrize("dim", [32, 64, 256])
+@pytest.mark.parametrize("n", [40, 5000])
+def test_other_head_sizes_are_multiplied_as_fp32(tq, oracle, dim, n):
+    """The softmax denominator of head sizes other than 128 against double sums over the stored codes.  Scores reach 30: an
+    fp32 sum of them is good to 2^-24 x 30 per step, a few steps; centroids in plain fp16 left 1e-4."""
+    heads, q_heads = 2, 6
+    k, v = (t.astype(np.float32) for t in kv_inputs(n + dim, n, heads, dim))
+    q = np.random.default_rng(dim).standard_normal((1, q_heads, dim)).astype(np.float16)
+    k[n // 3] = 2.0 * q[0, ::q_heads // heads].astype(np.float32)          # one key that stands out
+    c, (kw, kn, vw, vn, qw, qn) = encoded(tq, oracle, k, v)
+    out, lse = tq.compressed_attention([c], 0, q, use_qjl=True, return_lse=True)
+    cents = oracle.codebook(3)[0].astype(np.float64)
+    d = np.arange(dim)
+    codes = (kw[:, d // 10] >> (3 * (d % 10)).astype(np.uint32)) & 7
+    signs = ((qw[:, d // 32] >> (d % 32).astype(np.uint32)) & 1) * 2.0 - 1.0
+    rot = oracle.wht(q[0].astype(np.float32), oracle.kv_seed(0, 1), dim).astype(np.float64)
+    flip = np.array([1.0 if (oracle.kv_seed(0, 3) * 2654435761 + j * 2246822519) >> 31 & 1 else -1.0 for j in range(dim)])
+    for h in range(q_heads):
+        own = slice(h // (q_heads // heads), None, heads)                  # records of the KV head
+        r = rot[h]
+        dot = cents[codes[own]] @ r + np.sqrt(2 / (np.pi * dim)) * qn[own].astype(np.float64) * (signs[own] @ (flip * r))
+        s = dot * kn[own].astype(np.float64) / dim
+        want = s.max() + np.log(np.exp(s - s.max()).sum())
+        assert abs(lse[0, h] - want) < 1e-5, (h, lse[0, h], want)
+    want = oracle.attention(q[0].astype(np.float32), heads, kw, kn, vw, vn, qw, qn, layer=0, use_qjl=True)
+    assert rel_l2(out[0], want) < 4e-4                                     # the result's rounding: 2^-12 in the mean
+    c.close()

@@ -53,8 +53,9 @@ template <int D>
 struct AttnCfg {
     static constexpr int kWarps = D == 256 ? 8 : 16;            // 256 dims: 64 accumulator registers, and one team
     static constexpr int kThreads = 32 * kWarps;
-    static constexpr int kStages = 2;                           // of two tiles each: one wait and one refill per two tiles
-    static constexpr int kStageBytes = 2 * KvBlock<D>::kBytes;
+    static constexpr int kPer = D == 256 ? 1 : 2;               // tiles of a stage: one wait and one refill per two tiles, where they fit
+    static constexpr int kStages = 2;
+    static constexpr int kStageBytes = kPer * KvBlock<D>::kBytes;
     static constexpr int kRing = kStages * kStageBytes;         // bytes of a warp's ring
     static constexpr int kAccRegs = D / 4;                      // accumulators of a thread
     static constexpr int kAccStride = D + 4;                    // floats per head of a published accumulator
@@ -62,12 +63,13 @@ struct AttnCfg {
     static constexpr int kHalf = kTeam / 2;                     // the upper half of a team hands over to the lower one
     static constexpr int kPubBytes = 32 * (kAccRegs + 4) * 4;   // registers of a warp, or [8 heads][kAccStride]
     static constexpr int kQStride = D + 8;                      // halves per rotated query
-    static constexpr uint32_t kOffQ = kTabBytes + kWarps * kRing;                        // rotated queries
-    static constexpr uint32_t kOffQs = kOffQ + kGroup * kQStride * 2;                   // ... with the residual's signs
-    // Rotated queries and probabilities as two fp16 numbers each, 22 bits, and two products: heads of other sizes than 128
-    // are multiplied as fp32 numbers would be.  (With one fp16 number the error against the oracle with QJL went from 2.0e-4,
-    // the rounding of the result, to 3.6e-4 for 64 dims.  128 dims have always been multiplied in fp16.)
+    // Heads of other sizes than 128 are multiplied as fp32 numbers would be: centroids, rotated queries and weights as two fp16
+    // numbers each, 22 bits (the centroids' second halves in a table of their own behind the first), and three products.  128
+    // dims have always been multiplied in fp16, with centroids scaled so that fp16 holds them to 1.4e-5.
     static constexpr bool kSplit = D != 128;
+    static constexpr uint32_t kTables = kSplit ? 2 * kTabBytes : kTabBytes;
+    static constexpr uint32_t kOffQ = kTables + kWarps * kRing;                         // rotated queries
+    static constexpr uint32_t kOffQs = kOffQ + kGroup * kQStride * 2;                   // ... with the residual's signs
     static constexpr uint32_t kOffQl = kOffQs + kGroup * kQStride * 2;                  // what fp16 left of both, in fragment order
     static constexpr uint32_t kOffQsl = kOffQl + (kSplit ? kGroup * kQStride * 2 : 0);
     static constexpr uint32_t kOffPub = kOffQsl + (kSplit ? kGroup * kQStride * 2 : 0);
@@ -101,6 +103,10 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void add4(float (&c)[4], const float (&t)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += t[i];
 }
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
     uint32_t d;
@@ -162,6 +168,13 @@ __device__ __forceinline__ uint32_t table_load(uint32_t addr) {
     asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
+// The second half of the same entry.
+__device__ __forceinline__ uint32_t table_load_low(uint32_t addr) {
+    uint32_t v;
+    asm("ld.shared.b32 %0, [%1 + 32768];" : "=r"(v) : "r"(addr));
+    return v;
+}
+static_assert(kTabBytes == 32768u, "table_load_low's immediate");
 // W consecutive words.
 template <int W>
 __device__ __forceinline__ void load_words(uint32_t (&w)[W], uint32_t addr) {
@@ -196,7 +209,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     const int g = lane >> 2, q = lane & 3;
     auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(C::kTeam * 32) : "memory"); };
     const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(attn_smem));
-    const uint32_t ring = base + kTabBytes + cta_warp * C::kRing;
+    const uint32_t ring = base + C::kTables + cta_warp * C::kRing;
     const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(&s_bars[cta_warp * C::kStages]));
     unsigned char* const mine = attn_smem + C::kOffQ + team * C::kTeamBytes;   // this team's shared memory
     __half* const s_q = reinterpret_cast<__half*>(mine);
@@ -221,8 +234,14 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
     // The table does not depend on the kernels before this one.  (Bits 6 and 7 of a byte are not part of its codes.)
     for (int i = threadIdx.x; i < 256 * 8; i += C::kThreads) {
         const int e = i >> 3;
-        const uint32_t v = pack_half2(kAttnCentroidScale * kC3[e & 7], kAttnCentroidScale * kC3[(e >> 3) & 7]);
+        const float c0 = kAttnCentroidScale * kC3[e & 7], c1 = kAttnCentroidScale * kC3[(e >> 3) & 7];
+        const uint32_t v = pack_half2(c0, c1);
         *reinterpret_cast<uint4*>(attn_smem + i * 16) = make_uint4(v, v, v, v);   // 4 copies per store
+        if constexpr (kSplit) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+            const uint32_t lo = pack_half2(c0 - f.x, c1 - f.y);
+            *reinterpret_cast<uint4*>(attn_smem + kTabBytes + i * 16) = make_uint4(lo, lo, lo, lo);
+        }
     }
     if (tid == 0) s_flag[1] = 0u;
     __syncthreads();
@@ -292,11 +311,12 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         g.mine = g.n_tiles > warp ? (g.n_tiles - warp + C::kTeam - 1) / C::kTeam : 0;   // tiles warp, warp + kTeam, ...
         return g;
     };
-    // One stage: this warp's next two tiles, or its last one.  (a lane)
+    // One stage: this warp's next kPer tiles, or its last one.  (a lane)
     auto request = [&](uint32_t dst, const unsigned char* src, int left, uint32_t bar) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(left > 1 ? 2 * B::kBytes : B::kBytes) : "memory");
+        const bool two = C::kPer == 2 && left > 1;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(two ? 2 * B::kBytes : B::kBytes) : "memory");
         bulk_copy(dst, src, B::kBytes, bar);
-        if (left > 1) bulk_copy(dst + B::kBytes, src + C::kTeam * tile_stride, B::kBytes, bar);
+        if (two) bulk_copy(dst + B::kBytes, src + C::kTeam * tile_stride, B::kBytes, bar);
     };
     // Before a place in the ring is filled again: every lane's reads of it have ended.  (A tile's value words are needed only
     // beside the next tile's scores, and nothing else keeps their loads in front of the copy, which is of another proxy.
@@ -306,9 +326,9 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         __syncwarp();
     };
     auto request_first = [&](const Segment& g) {
-        for (int i = 0; i < C::kStages && 2 * i < g.mine; ++i) {
+        for (int i = 0; i < C::kStages && C::kPer * i < g.mine; ++i) {
             const int s = stage ^ i;
-            request(ring + s * C::kStageBytes, g.src + static_cast<size_t>(warp + 2 * i * C::kTeam) * tile_stride, g.mine - 2 * i, bars + 8u * s);
+            request(ring + s * C::kStageBytes, g.src + static_cast<size_t>(warp + C::kPer * i * C::kTeam) * tile_stride, g.mine - C::kPer * i, bars + 8u * s);
         }
     };
 
@@ -410,15 +430,17 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             for (int w = 0; w < W; ++w) {
                 const uint32_t A = D == 128 && w == 3 ? kv_value_spare(xa[0], xa[1 % W], xa[2 % W]) : xa[w];
                 const uint32_t Bw = D == 128 && w == 3 ? kv_value_spare(xb[0], xb[1 % W], xb[2 % W]) : xb[w];
-                const uint32_t v0 = table_load(pair_addr<0>(A, lane_base)), v1 = table_load(pair_addr<1>(A, lane_base));
-                const uint32_t v2 = table_load(pair_addr<0>(Bw, lane_base)), v3 = table_load(pair_addr<1>(Bw, lane_base));
-                const uint32_t v4 = table_load(pair_addr<2>(A, lane_base)), v5 = table_load(pair_addr<3>(A, lane_base));
-                const uint32_t v6 = table_load(pair_addr<2>(Bw, lane_base)), v7 = table_load(pair_addr<3>(Bw, lane_base));
+                const uint32_t a0 = pair_addr<0>(A, lane_base), a1 = pair_addr<1>(A, lane_base), a2 = pair_addr<0>(Bw, lane_base), a3 = pair_addr<1>(Bw, lane_base);
+                const uint32_t a4 = pair_addr<2>(A, lane_base), a5 = pair_addr<3>(A, lane_base), a6 = pair_addr<2>(Bw, lane_base), a7 = pair_addr<3>(Bw, lane_base);
+                const uint32_t v0 = table_load(a0), v1 = table_load(a1), v2 = table_load(a2), v3 = table_load(a3);
+                const uint32_t v4 = table_load(a4), v5 = table_load(a5), v6 = table_load(a6), v7 = table_load(a7);
                 mma_f16(acc[2 * w], v0, v1, v2, v3, pb0, pb1);
                 mma_f16(acc[2 * w + 1], v4, v5, v6, v7, pb0, pb1);
                 if constexpr (kSplit) {
                     mma_f16(acc[2 * w], v0, v1, v2, v3, pl0, pl1);
                     mma_f16(acc[2 * w + 1], v4, v5, v6, v7, pl0, pl1);
+                    mma_f16(acc[2 * w], table_load_low(a0), table_load_low(a1), table_load_low(a2), table_load_low(a3), pb0, pb1);
+                    mma_f16(acc[2 * w + 1], table_load_low(a4), table_load_low(a5), table_load_low(a6), table_load_low(a7), pb0, pb1);
                 }
             }
         };
@@ -436,17 +458,27 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 load_words<W>(kb, blk + (g + 8) * (D / 2) + q * (D / 8));
 #pragma unroll
                 for (int w = 0; w < W; ++w) {
-                    const uint32_t k0 = table_load(pair_addr<0>(ka[w], lane_base)), k1 = table_load(pair_addr<0>(kb[w], lane_base));
-                    const uint32_t k2 = table_load(pair_addr<1>(ka[w], lane_base)), k3 = table_load(pair_addr<1>(kb[w], lane_base));
-                    const uint32_t k4 = table_load(pair_addr<2>(ka[w], lane_base)), k5 = table_load(pair_addr<2>(kb[w], lane_base));
-                    const uint32_t k6 = table_load(pair_addr<3>(ka[w], lane_base)), k7 = table_load(pair_addr<3>(kb[w], lane_base));
-                    mma_f16(c1, k0, k1, k2, k3, bq[4 * w], bq[4 * w + 1]);
-                    mma_f16(c1b, k4, k5, k6, k7, bq[4 * w + 2], bq[4 * w + 3]);
+                    const uint32_t a0 = pair_addr<0>(ka[w], lane_base), a1 = pair_addr<0>(kb[w], lane_base), a2 = pair_addr<1>(ka[w], lane_base), a3 = pair_addr<1>(kb[w], lane_base);
+                    const uint32_t a4 = pair_addr<2>(ka[w], lane_base), a5 = pair_addr<2>(kb[w], lane_base), a6 = pair_addr<3>(ka[w], lane_base), a7 = pair_addr<3>(kb[w], lane_base);
+                    const uint32_t k0 = table_load(a0), k1 = table_load(a1), k2 = table_load(a2), k3 = table_load(a3);
+                    const uint32_t k4 = table_load(a4), k5 = table_load(a5), k6 = table_load(a6), k7 = table_load(a7);
                     if constexpr (kSplit) {
+                        // the small products first, sums of 16 dims added up in fp32: the tensor cores' accumulation rounds toward
+                        // zero, which as one chain left 1e-6 of a score
+                        float t[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
                         uint32_t lo[4];
                         load_words<4>(lo, frag_ql + 16u * w);
-                        mma_f16(c1, k0, k1, k2, k3, lo[0], lo[1]);
-                        mma_f16(c1b, k4, k5, k6, k7, lo[2], lo[3]);
+                        mma_f16(t, table_load_low(a0), table_load_low(a1), table_load_low(a2), table_load_low(a3), bq[4 * w], bq[4 * w + 1]);
+                        mma_f16(tb, table_load_low(a4), table_load_low(a5), table_load_low(a6), table_load_low(a7), bq[4 * w + 2], bq[4 * w + 3]);
+                        mma_f16(t, k0, k1, k2, k3, lo[0], lo[1]);
+                        mma_f16(tb, k4, k5, k6, k7, lo[2], lo[3]);
+                        mma_f16(t, k0, k1, k2, k3, bq[4 * w], bq[4 * w + 1]);
+                        mma_f16(tb, k4, k5, k6, k7, bq[4 * w + 2], bq[4 * w + 3]);
+                        add4(c1, t);
+                        add4(c1b, tb);
+                    } else {
+                        mma_f16(c1, k0, k1, k2, k3, bq[4 * w], bq[4 * w + 1]);
+                        mma_f16(c1b, k4, k5, k6, k7, bq[4 * w + 2], bq[4 * w + 3]);
                     }
                 }
                 if constexpr (QJL) {
@@ -457,13 +489,21 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
 #pragma unroll
                     for (int w = 0; w < W; ++w) {
                         const uint32_t la = ka[w] << 8, lb = kb[w] << 8;
-                        mma_f16(c2, two(la), two(lb), one(la), one(lb), bs[4 * w], bs[4 * w + 1]);
-                        mma_f16(c2b, two(ka[w]), two(kb[w]), one(ka[w]), one(kb[w]), bs[4 * w + 2], bs[4 * w + 3]);
+                        const uint32_t s0 = two(la), s1 = two(lb), s2 = one(la), s3 = one(lb);
+                        const uint32_t s4 = two(ka[w]), s5 = two(kb[w]), s6 = one(ka[w]), s7 = one(kb[w]);
                         if constexpr (kSplit) {
+                            float t[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
                             uint32_t lo[4];
                             load_words<4>(lo, frag_qsl + 16u * w);
-                            mma_f16(c2, two(la), two(lb), one(la), one(lb), lo[0], lo[1]);
-                            mma_f16(c2b, two(ka[w]), two(kb[w]), one(ka[w]), one(kb[w]), lo[2], lo[3]);
+                            mma_f16(t, s0, s1, s2, s3, lo[0], lo[1]);
+                            mma_f16(tb, s4, s5, s6, s7, lo[2], lo[3]);
+                            mma_f16(t, s0, s1, s2, s3, bs[4 * w], bs[4 * w + 1]);
+                            mma_f16(tb, s4, s5, s6, s7, bs[4 * w + 2], bs[4 * w + 3]);
+                            add4(c2, t);
+                            add4(c2b, tb);
+                        } else {
+                            mma_f16(c2, s0, s1, s2, s3, bs[4 * w], bs[4 * w + 1]);
+                            mma_f16(c2b, s4, s5, s6, s7, bs[4 * w + 2], bs[4 * w + 3]);
                         }
                     }
                 }
@@ -565,21 +605,21 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                 pl1 = movmatrix_trans(pack_half2(w10 - fb.x, w11 - fb.y));
             }
         };
-        const unsigned char* next_src = seg.src + static_cast<size_t>(warp + 2 * C::kStages * C::kTeam) * tile_stride;
+        const unsigned char* next_src = seg.src + static_cast<size_t>(warp + C::kPer * C::kStages * C::kTeam) * tile_stride;
         int token = seg.first_token + warp * kKvTile;
-        for (int left = seg.mine; left > 0; left -= 2, token += 2 * C::kTeam * kKvTile) {
+        for (int left = seg.mine; left > 0; left -= C::kPer, token += C::kPer * C::kTeam * kKvTile) {
             if (!bar_wait(bars + 8u * stage, phase)) {
                 ok = false;
                 break;
             }
             const uint32_t blk = ring + stage * C::kStageBytes;
             take_tile(blk, token);
-            if (left > 1) take_tile(blk + B::kBytes, token + C::kTeam * kKvTile);
-            if (left > 2 * C::kStages) {
+            if (C::kPer == 2 && left > 1) take_tile(blk + B::kBytes, token + C::kTeam * kKvTile);
+            if (left > C::kPer * C::kStages) {
                 end_reads();
-                if (lane == 0) request(blk, next_src, left - 2 * C::kStages, bars + 8u * stage);
+                if (lane == 0) request(blk, next_src, left - C::kPer * C::kStages, bars + 8u * stage);
             }
-            next_src += 2 * C::kTeam * tile_stride;
+            next_src += C::kPer * C::kTeam * tile_stride;
             phase ^= static_cast<uint32_t>(stage);
             stage ^= 1;
         }
@@ -649,7 +689,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         const int c_first = whole ? range : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
         const int c_last = whole ? range : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
         float* const my_part = a.part + static_cast<size_t>(2 * range + (done.tile0 == 0 ? 1 : 0)) * C::kPartFloats;
-        auto add4 = [](float4& x, float f0, const float4& y, float f1) {
+        auto scale_add = [](float4& x, float f0, const float4& y, float f1) {
             x.x = fmaf(x.x, f0, y.x * f1);
             x.y = fmaf(x.y, f0, y.y * f1);
             x.z = fmaf(x.z, f0, y.z * f1);
@@ -669,7 +709,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
             for (int w = 0; w < C::kHalf; ++w) {
                 const float f = exp2_approx(m[w] - M);
                 L = fmaf(s_l[w * kGroup + h], f, L);
-                add4(A, 1.f, *reinterpret_cast<const float4*>(s_pub + w * C::kPubBytes + (h * C::kAccStride + d) * 4), f);
+                scale_add(A, 1.f, *reinterpret_cast<const float4*>(s_pub + w * C::kPubBytes + (h * C::kAccStride + d) * 4), f);
             }
             *reinterpret_cast<float4*>((whole ? s_out + h * C::kAccStride : my_part + h * D) + d) = A;
             if (d == 0) *reinterpret_cast<float2*>(whole ? s_out + h * C::kAccStride + D : my_part + kGroup * D + 2 * h) = make_float2(M, L);
@@ -739,7 +779,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                             for (int k = 0; k < 8; ++k) pa[k] = __ldcg(reinterpret_cast<const float4*>(part_of(c_first + min(c0 + k, n_parts - 1)) + idx));
 #pragma unroll
                             for (int k = 0; k < 8; ++k)
-                                if (c0 + k < n_parts) add4(A, 1.f, pa[k], s_w[(c0 + k) * kGroup + h]);
+                                if (c0 + k < n_parts) scale_add(A, 1.f, pa[k], s_w[(c0 + k) * kGroup + h]);
                         }
                         *reinterpret_cast<float4*>(s_out + h * C::kAccStride + d) = A;
                     }
@@ -762,7 +802,7 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
                             if (c0 + k > c_last) break;
                             const float mn = fmaxf(M, ml[k].x), f0 = exp2_approx(M - mn), f1 = exp2_approx(ml[k].x - mn);
                             L = fmaf(L, f0, ml[k].y * f1);
-                            add4(A, f0, pa[k], f1);
+                            scale_add(A, f0, pa[k], f1);
                             M = mn;
                         }
                     }
