@@ -144,13 +144,13 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     const int plane = warp / (batch * groups_per_row);
     const int rem = warp - plane * batch * groups_per_row;
     const int row = rem / groups_per_row, col = (rem - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
+    const unsigned live = __ballot_sync(0xffffffffu, col < in);   // the lanes that exchange values
     if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
     const uint32_t seed = plane ? seed_r : seed_p;
     const __half* const src = x + static_cast<size_t>(row) * in + col;
     uint4 raw[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
-    const unsigned live = __activemask();
     float v[CHUNKS][8];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block), block, lane, live);

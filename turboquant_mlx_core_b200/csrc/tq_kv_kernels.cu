@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
         const int which = i / D, d = i - which * D;
         const bool pos = which == 2 ? qjl_sign_is_positive(qjl_seed, static_cast<uint32_t>(d))
                                     : sign_is_positive(which ? v_seed : k_seed, static_cast<uint32_t>(d));
-        const uint32_t bits = __ballot_sync(__activemask(), pos);
+        const uint32_t bits = __ballot_sync(0xffffffffu, pos);
         if ((i & 31) == 0) s_sign[which][d >> 5] = bits;
     }
     __syncthreads();
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __r
         s_cent[c][i & 31] = __fmul_rn(c < 4 ? -mag : mag, inv_scale);
     }
     for (int i = threadIdx.x; i < D; i += 128) {
-        const uint32_t bits = __ballot_sync(__activemask(), sign_is_positive(wht_seed, static_cast<uint32_t>(i)));
+        const uint32_t bits = __ballot_sync(0xffffffffu, sign_is_positive(wht_seed, static_cast<uint32_t>(i)));
         if ((i & 31) == 0) s_sign[i >> 5] = bits;
     }
     __syncthreads();
