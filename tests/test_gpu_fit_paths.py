@@ -32,3 +32,16 @@ def test_fit_against_the_checker(tq, oracle, n, kind):
     got = tq.generate_codebook_from_data(x, 4, 20)
     tol = 3e-6 * np.abs(want) + 3e-7
     assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
+
+
+@pytest.mark.parametrize("n", [200_000, 1_000_003])
+@pytest.mark.parametrize("share", [0.05, 0.3, 1.0])
+def test_crowded_samples_are_fitted_in_passes_over_all(tq, oracle, n, share):
+    """One value in so many places that its bucket is not worth filling: seen beforehand, or when a boundary comes to it."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n).astype(np.float32)
+    x[rng.random(n) < share] = 0.0
+    want, _ = oracle.fit_codebook(x, 4, 20)
+    got, again = (tq.generate_codebook_from_data(x, 4, 20) for _ in range(2))
+    assert np.all(np.abs(got.centroids - want) <= 3e-6 * np.abs(want) + 3e-7)
+    assert np.array_equal(got.centroids.view(np.uint32), again.centroids.view(np.uint32))

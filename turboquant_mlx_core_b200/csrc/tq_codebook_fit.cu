@@ -6,6 +6,7 @@
 // bits of their order-preserving key (sign, exponent, a few mantissa bits), with running counts and a sum per bucket; a
 // boundary then only looks at the values of its own bucket, and all iterations run in one launch of one CTA, a warp per
 // boundary and bin (about 1 us each).
+//   fit_look_kernel       whether the samples repeat themselves (then as below)
 //   fit_count_kernel      bucket counts, largest magnitude            (one pass over the samples)
 //   fit_groups / fit_offsets   exclusive scan of the counts, 256 buckets per group
 //   fit_scatter_kernel    samples into their buckets                  (one pass)
@@ -16,8 +17,8 @@
 // exact 64-bit integer of significands.  A bin is the double sum of the buckets between its boundaries and those two partial
 // ones, in a fixed order: only its own values enter, as in the reference's double sums, whatever the magnitudes of the
 // others (running sums over all buckets would lose a bin beside an outlier), and results are run-to-run identical.
-// A boundary whose bucket holds more than kFitMaxBucket values (samples with heavy repetition), or samples that are not
-// finite, stop fit_iterate_kernel; the remaining iterations then go over all samples:
+// Samples that repeat themselves skip all that, and a boundary whose bucket holds more than kFitMaxBucket values, or samples
+// that are not finite, stop fit_iterate_kernel; the remaining iterations then go over all samples:
 //   fit_partial_kernel   every thread bins its values by lower_bound over the current boundaries into a PRIVATE histogram in
 //                        shared memory ([bin][thread]: no atomics, no bank conflicts), sums in double; the block then folds
 //                        its 256 histograms in a fixed order and writes one (sum, count) pair per bin;
@@ -53,7 +54,9 @@ struct FitState {
 constexpr int kFitGroup = 256;              // buckets of a group
 constexpr int kFitSumBuckets = 32;          // buckets whose sums a block takes
 constexpr int kFitBatch = 8;                // values of a bucket that a lane requests at once
-constexpr unsigned int kFitMaxBucket = 32768;
+constexpr unsigned int kFitMaxBucket = 32768;   // values of a bucket that the iterations look through
+constexpr int kFitLooked = 4096, kFitSlots = 8192;   // samples that fit_look_kernel looks at, its counters
+constexpr unsigned int kFitCrowd = 2 * kFitMaxBucket;
 
 // Order-preserving key of a float: smaller values have smaller keys (-0 and +0 differ by one, which no sum notices).
 __device__ __forceinline__ unsigned int fit_key(float x) {
@@ -74,8 +77,28 @@ __device__ __forceinline__ FitBucket fit_bucket(int bucket, int shift) {
     return FitBucket{(u & 0x7fffffu) | (e != 0u ? 0x800000u : 0u), (u & 0x80000000u) ? -unit : unit};
 }
 
+// Samples that repeat themselves: the atomic additions of a bucket's samples follow one another (3 ns each: 16.8 M equal
+// samples took 55 ms, half of them zero 39 ms, where the passes over all samples take 1 and 11), and the iterations stop
+// at such a bucket anyway.  One CTA looks at kFitLooked samples, evenly spread: where one bucket must hold more than
+// kFitCrowd, the kernels after it return at once.  (kFitSlots counters: two buckets that share one need twice the luck.)
+__global__ void __launch_bounds__(1024) fit_look_kernel(const float* __restrict__ data, unsigned int n, int shift, FitState* __restrict__ state) {
+    __shared__ unsigned int s_count[kFitSlots];
+    for (int i = threadIdx.x; i < kFitSlots; i += 1024) s_count[i] = 0u;
+    __syncthreads();
+    unsigned int most = 0;
+    const unsigned int step = n / kFitLooked;
+#pragma unroll
+    for (int k = 0; k < kFitLooked / 1024; ++k) {
+        const unsigned int bucket = fit_key(__ldg(data + static_cast<size_t>(k * 1024 + threadIdx.x) * step)) >> shift;
+        most = max(most, atomicAdd(&s_count[bucket % kFitSlots], 1u) + 1u);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most >= 16u && static_cast<unsigned long long>(most) * step > kFitCrowd) state->go_over_all = 1;
+}
+
 __global__ void __launch_bounds__(256) fit_count_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ count,
                                                         FitState* __restrict__ state) {
+    if (state->go_over_all) return;
     unsigned int top = 0;
     for (unsigned int i = blockIdx.x * 1024u + threadIdx.x; i < n; i += gridDim.x * 1024u) {
 #pragma unroll
@@ -127,7 +150,8 @@ __global__ void __launch_bounds__(256) fit_offsets_kernel(const unsigned int* __
     cursor[b] = at;
 }
 __global__ void __launch_bounds__(256) fit_scatter_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ cursor,
-                                                          float* __restrict__ sorted) {
+                                                          float* __restrict__ sorted, const FitState* __restrict__ state) {
+    if (state->go_over_all) return;
     for (unsigned int i = blockIdx.x * 1024u + threadIdx.x; i < n; i += gridDim.x * 1024u) {
         float x[4];
         unsigned int pos[4];
@@ -147,7 +171,8 @@ __global__ void __launch_bounds__(256) fit_scatter_kernel(const float* __restric
 // about a hundred groups of 256 buckets; with a block per group those few blocks took 450 us for 16.8 M samples.
 __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__ sorted, const unsigned int* __restrict__ count,
                                                        const unsigned int* __restrict__ offset, int shift, double* __restrict__ sum,
-                                                       double* __restrict__ part) {
+                                                       double* __restrict__ part, const FitState* __restrict__ state) {
+    if (state->go_over_all) return;
     __shared__ double s_warp[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned int below = (1u << shift) - 1u;
@@ -198,6 +223,7 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restri
     __shared__ long long s_low[kFitMaxBins];
     __shared__ double s_mid[kFitMaxBins];      // per bin: the groups between its boundaries' (or the buckets, where they share one)
     __shared__ int s_stop, s_converged, s_moved, s_near;
+    if (state->go_over_all) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nc = state->n;
     if (tid < nc) s_c[tid] = state->centroids[tid];
@@ -538,11 +564,12 @@ int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, c
             TQ_CUDA(cudaMemsetAsync(d_count, 0, static_cast<size_t>(n_buckets) * 4, stream));
             const unsigned int un = static_cast<unsigned int>(n);
             const int grid = static_cast<int>(std::min<long>((n + 1023) / 1024, 16L * sms));
+            if (un >= kFitCrowd) fit_look_kernel<<<1, 1024, 0, stream>>>(d_data, un, shift, d_state);
             fit_count_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_count, d_state);
             fit_groups_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group);
             fit_offsets_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group, d_offset, d_cursor);
-            fit_scatter_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_cursor, d_sorted);
-            fit_sums_kernel<<<n_parts, 256, 0, stream>>>(d_sorted, d_count, d_offset, shift, d_sum, d_part);
+            fit_scatter_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_cursor, d_sorted, d_state);
+            fit_sums_kernel<<<n_parts, 256, 0, stream>>>(d_sorted, d_count, d_offset, shift, d_sum, d_part, d_state);
             fit_iterate_kernel<<<1, 1024, 0, stream>>>(d_sorted, un, d_count, d_offset, d_sum, d_part, n_groups, d_group_sum, shift, iterations, d_state);
             TQ_CUDA(cudaGetLastError());
             read_state();
