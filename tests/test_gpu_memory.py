@@ -1,0 +1,49 @@
+"""Device memory kept between objects: what it must not make work, what it must give back."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+GROW_IN_CAPTURE = """
+import torch
+import turboquant_mlx_core_b200 as tq
+side = torch.cuda.Stream()
+kv = torch.randn((257, 2, 128), device="cuda").half()
+torch.cuda.synchronize()
+c = tq.TQKVCache(1, 2, 128)
+c.append(0, kv[:256], kv[:256], stream=side)          # full: the next token doubles the storage
+torch.cuda.synchronize()
+before = c.get_keys_fp16(0, 0, 256)
+other = tq.TQKVCache(1, 2, 128)
+other.reserve(0, 512)                                 # leaves a block of the doubled size behind, nothing pending on it
+other.append(0, kv[:1], kv[:1], stream=side)
+torch.cuda.synchronize()
+other.close()
+what = None
+try:
+    with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=side):
+        try:
+            c.append(0, kv[256:], kv[256:], stream=side)
+        except tq.TQError as e:
+            what = e
+except RuntimeError:
+    pass                                              # the capture that the refusal ended
+torch.cuda.synchronize()
+assert what is not None, "growing inside a capture was not refused"
+assert c.seq_length() == 256 and (c.get_keys_fp16(0, 0, 256).view("u2") == before.view("u2")).all()
+c.append(0, kv[256:], kv[256:])
+assert c.seq_length() == 257 and (c.get_keys_fp16(0, 0, 256).view("u2") == before.view("u2")).all()
+print("ok")
+"""
+
+
+def test_storage_does_not_grow_inside_a_capture():
+    """A kept block must not let an append inside a capture move the storage: the copy would run at replay, the host would
+    count on it now.  In a process of its own, which the broken capture ends with."""
+    r = subprocess.run([sys.executable, "-c", GROW_IN_CAPTURE], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr

@@ -384,7 +384,8 @@ public:
         if (n > counters_zeroed_) {
             attn_counters_.reserve(n * sizeof(unsigned int), st);
             TQ_CUDA(cudaMemsetAsync(attn_counters_.as<void>(), 0, attn_counters_.bytes(), st));
-            counters_zeroed_ = attn_counters_.bytes() / sizeof(unsigned int);
+            // (captured, they are zeroed by every replay and not now)
+            if (!tq::stream_is_capturing(st)) counters_zeroed_ = attn_counters_.bytes() / sizeof(unsigned int);
         }
         return attn_counters_.as<unsigned int>();
     }
@@ -506,8 +507,7 @@ private:
         DeviceBuffer slab;
         slab.owned_by(&use_);
         const size_t bytes = tq::kv_layer_bytes(cap, heads_, dim_);
-        if (on_stream) slab.reserve(bytes, st);
-        else slab.reserve(bytes);
+        slab.reserve(bytes, st, on_stream);
         const size_t used = tq::kv_layer_bytes((L.num_tokens + 15) / 16 * 16, heads_, dim_);   // whole tiles: one contiguous piece
         if (used) TQ_CUDA(cudaMemcpyAsync(slab.as<void>(), L.slab.as<void>(), used, cudaMemcpyDeviceToDevice, st));
         L.slab = std::move(slab);   // the old storage goes back once the copies out of it have ended
@@ -648,7 +648,7 @@ public:
         const bool dev = tq::is_device_pointer(out);
         __half* d_out = static_cast<__half*>(out);
         if (!dev) {
-            out_stage_.reserve(static_cast<size_t>(n) * row * sizeof(__half));
+            out_stage_.reserve(static_cast<size_t>(n) * row * sizeof(__half), st);
             d_out = out_stage_.as<__half>();
         }
         tq::launch_ring_read(values ? v_.as<__half>() : k_.as<__half>(), n, row, window_, start, d_out, st);
@@ -669,12 +669,12 @@ private:
         const void* dk = keys;
         const void* dv = values;
         if (!tq::is_device_pointer(keys)) {
-            k_stage_.reserve(bytes);
+            k_stage_.reserve(bytes, st);
             TQ_CUDA(cudaMemcpyAsync(k_stage_.as<void>(), keys, bytes, cudaMemcpyHostToDevice, st));
             dk = k_stage_.as<void>();
         }
         if (!tq::is_device_pointer(values)) {
-            v_stage_.reserve(bytes);
+            v_stage_.reserve(bytes, st);
             TQ_CUDA(cudaMemcpyAsync(v_stage_.as<void>(), values, bytes, cudaMemcpyHostToDevice, st));
             dv = v_stage_.as<void>();
         }
@@ -717,18 +717,18 @@ void hybrid_attention(TQKVCache* cache, DecodeBuffer* buf, int layer, const void
     const size_t q_es = q_dtype == TQ_F32 ? 4 : 2;
     const void* d_q = q;
     if (!tq::is_device_pointer(q)) {
-        buf->q_stage().reserve(n_q * q_es);
+        buf->q_stage().reserve(n_q * q_es, st);
         TQ_CUDA(cudaMemcpyAsync(buf->q_stage().as<void>(), q, n_q * q_es, cudaMemcpyHostToDevice, st));
         d_q = buf->q_stage().as<void>();
     }
     const bool out_dev = tq::is_device_pointer(out);
     __half* d_out = static_cast<__half*>(out);
     if (!out_dev) {
-        buf->out_stage().reserve(n_q * sizeof(__half));
+        buf->out_stage().reserve(n_q * sizeof(__half), st);
         d_out = buf->out_stage().as<__half>();
     }
     const int n_splits = tq::dense_attention_splits(seq_len, heads, q_heads, tq::sm_count(cache->device()));
-    buf->scratch().reserve(tq::dense_attention_scratch_bytes(q_heads, dim, n_splits));
+    buf->scratch().reserve(tq::dense_attention_scratch_bytes(q_heads, dim, n_splits), st);
     tq::launch_dense_attention(buf->key_ring(), buf->value_ring(), seq_len, heads, dim, d_q, q_dtype == TQ_F16, q_heads, n_splits,
                                buf->scratch().as<void>(), d_out, st);
     if (!out_dev) {

@@ -143,7 +143,7 @@ public:
         // rows now, which is right for pageable memory only: page-locked rows may be written by work that is still queued
         // on the stream, and a captured copy reads its source anew on every replay, so these stay copies on the stream.
         const bool decode_call = batch <= 8 || nx * sizeof(__half) <= kHostStageBytes;
-        const bool read_now = !x_dev && kx.pinned_alias == nullptr && !is_capturing(st);
+        const bool read_now = !x_dev && kx.pinned_alias == nullptr && !tq::stream_is_capturing(st);
         const bool as_params = read_now && nx * sizeof(__half) <= tq::kMaxParamRowBytes;
         const __half* d_x;
         std::optional<tq::PinnedStage> x_stage, y_stage;
@@ -412,12 +412,6 @@ private:
         kinds_[next_kind_] = k;
         next_kind_ = (next_kind_ + 1) & 3;
         return k;
-    }
-    static bool is_capturing(cudaStream_t st) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
-        cudaGetLastError();
-        return true;   // the legacy stream while another one of the device is captured
     }
     PointerKind kinds_[4];
     int next_kind_ = 0;

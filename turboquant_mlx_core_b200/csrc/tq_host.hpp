@@ -70,8 +70,10 @@ inline void* pinned_host_device_alias(const void* p) {
 // ---- device memory (tq_memory.cu: released blocks are kept for the next owner) -----------------
 inline bool is_legacy_stream(cudaStream_t st) { return st == nullptr || st == cudaStreamLegacy; }
 size_t pool_size_class(size_t bytes);
-// A block on `device`, which must be current.  on_stream: its first use is work put on `st`; otherwise the block is
-// idle when the call returns.
+// Whether work put on the stream is captured in a graph.
+bool stream_is_capturing(cudaStream_t st);
+// A block on `device`, which must be current, for an object that works on `st`.  on_stream: its first use is work put there;
+// otherwise the block is idle when the call returns.
 void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream);
 // idle: nothing queued anywhere uses the block; otherwise everything that does was put on the legacy default stream.
 void pool_release(void* p, size_t bytes, int device, bool idle);
@@ -130,8 +132,8 @@ public:
     // Grow-only: keeps the allocation when it is already large enough (contents kept
     // only in that case).
     void reserve(size_t bytes) { grow(bytes, nullptr, false); }
-    // ... for contents whose first use is work on `st`.
-    void reserve(size_t bytes, cudaStream_t st) { grow(bytes, st, true); }
+    // ... for contents whose first use is work on `st` (or, not on_stream, perhaps on another one after it).
+    void reserve(size_t bytes, cudaStream_t st, bool on_stream = true) { grow(bytes, st, on_stream); }
     void resize(size_t bytes) { reserve(bytes); }
     void release() {
         if (p_) {

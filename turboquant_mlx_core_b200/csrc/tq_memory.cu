@@ -13,6 +13,8 @@
 //              was put on the legacy default stream: then an event recorded there marks its end, and the next owner
 //              orders itself behind it - on its stream where it names one, on the host otherwise.  An owner that saw
 //              any other stream waits for the device before it releases, as cudaFree did.
+//   Capture    memory for work on a stream that is being captured comes from cudaMalloc, which the driver allows or refuses
+//              by the capture's mode: growing an object inside a capture is not something that a kept block makes work.
 #include <chrono>
 #include <list>
 #include <mutex>
@@ -68,8 +70,21 @@ Pool& pool() {
     return *p;
 }
 
+}  // namespace
+
+// (An error: the legacy stream while a blocking one of the device is captured.)
+bool stream_is_capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+namespace {
+
 // An event recorded on the current device's legacy default stream, nullptr when that failed (the caller then waits).
 cudaEvent_t mark_legacy_stream(Pool& P, int device) {
+    if (stream_is_capturing(nullptr)) return nullptr;   // an event there would break the capture of a blocking stream
     cudaEvent_t e = nullptr;
     if (!P.events[device].empty()) {
         e = P.events[device].back();
@@ -115,7 +130,7 @@ size_t pool_size_class(size_t bytes) {
 void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream) {
     const size_t want = pool_size_class(bytes);
     Pool& P = pool();
-    if (device >= 0 && device < 64) {
+    if (device >= 0 && device < 64 && !stream_is_capturing(st)) {
         std::lock_guard<std::mutex> lock(P.mu);
         // newest first: most likely still in the caches, and the oldest get the chance to age
         for (auto it = P.blocks.rbegin(); it != P.blocks.rend(); ++it) {
