@@ -109,7 +109,7 @@ tq_array_t tq_array_create(const void* data, int dtype, int ndim, const int* sha
         try {
             if (nb) {
                 TQ_REQUIRE(data, "tq_array_create: NULL data");
-                TQ_CUDA(cudaMalloc(&a->data, nb));
+                a->data = device_malloc(nb);
                 TQ_CUDA(cudaMemcpy(a->data, data, nb, cudaMemcpyDefault));
             }
         } catch (...) {

@@ -765,10 +765,11 @@ tq_array_s* new_f16_array(int ndim, const int* shape) {
     a->device = current_device();
     a->owns = true;
     if (a->nbytes()) {
-        cudaError_t e = cudaMalloc(&a->data, a->nbytes());
-        if (e != cudaSuccess) {
+        try {
+            a->data = device_malloc(a->nbytes());
+        } catch (...) {
             delete a;
-            throw Error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+            throw;
         }
     }
     return a;

@@ -712,8 +712,7 @@ int tq_linear_wait_peers(tq_linear_t lin, const void* local_flags, int n_flags, 
 void* tq_shared_alloc(size_t bytes) {
     return guarded<void*>(nullptr, nullptr, [&]() -> void* {
         TQ_REQUIRE(bytes > 0, "tq_shared_alloc: zero bytes");
-        void* p = nullptr;
-        TQ_CUDA(cudaMalloc(&p, bytes));
+        void* const p = device_malloc(bytes);
         TQ_CUDA(cudaMemset(p, 0, bytes));
         return p;
     });

@@ -78,6 +78,11 @@ void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream);
 // idle: nothing queued anywhere uses the block; otherwise everything that does was put on the legacy default stream.
 void pool_release(void* p, size_t bytes, int device, bool idle);
 void pool_trim();
+struct OutOfMemory : Error {
+    using Error::Error;
+};
+// cudaMalloc, after giving the unused blocks back where memory is short; OutOfMemory where it still is.
+void* device_malloc(size_t bytes);
 // A zeroed word of page-locked host memory that the device can write.
 unsigned int* status_word_take(int device);
 // All work that could write the word was put on the legacy default stream, or has ended.

@@ -153,12 +153,20 @@ void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream) {
             return p;
         }
     }
+    return device_malloc(want);
+}
+
+void* device_malloc(size_t bytes) {
     void* p = nullptr;
-    cudaError_t rc = cudaMalloc(&p, want);
+    cudaError_t rc = cudaMalloc(&p, bytes);
     if (rc == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         pool_trim();
-        rc = cudaMalloc(&p, want);
+        rc = cudaMalloc(&p, bytes);
+    }
+    if (rc == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        throw OutOfMemory("cudaMalloc of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(rc));
     }
     TQ_CUDA(rc);
     return p;
