@@ -3,6 +3,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +48,21 @@ def test_storage_does_not_grow_inside_a_capture():
     count on it now.  In a process of its own, which the broken capture ends with."""
     r = subprocess.run([sys.executable, "-c", GROW_IN_CAPTURE], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+def test_a_fit_needs_no_memory_that_is_not_there(tq):
+    """With less free memory than a copy of the samples takes, the fit goes over the samples where they are."""
+    torch = pytest.importorskip("torch")
+    x = torch.randn((1 << 28,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    want = tq.generate_codebook_from_data(x, 4, 3)
+    ones = tq.generate_codebook_from_data(torch.ones(100000, device="cuda"), 4, 3)   # the other path's kernels are loaded
+    assert ones is not None
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (768 << 20)), dtype=torch.uint8, device="cuda")
+    try:
+        got = tq.generate_codebook_from_data(x, 4, 3)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert np.all(np.abs(got.centroids - want.centroids) <= 3e-6 * np.abs(want.centroids) + 3e-7)

@@ -543,16 +543,22 @@ int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, c
         };
         h.go_over_all = 1;
         DeviceBuffer bucket_buf, sorted_buf;
-        if (n < (1L << 31)) {
-            // Mantissa bits of a bucket's key: a few hundred values in the buckets where boundaries lie (16.8 M normal samples:
-            // 11 bits, about 600), between 2^12 and 2^21 buckets.
-            int log2_n = 0;
-            while ((1L << log2_n) < n) ++log2_n;
-            const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13)), shift = 32 - key_bits, n_buckets = 1 << key_bits;
-            const int n_groups = n_buckets / kFitGroup;
-            const int n_parts = n_buckets / kFitSumBuckets;
-            bucket_buf.reserve(static_cast<size_t>(n_buckets) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups) * 8 + static_cast<size_t>(n_groups) * 4, stream);
-            sorted_buf.reserve(static_cast<size_t>(n) * 4, stream);
+        // Mantissa bits of a bucket's key: a few hundred values in the buckets where boundaries lie (16.8 M normal samples:
+        // 11 bits, about 600), between 2^12 and 2^21 buckets.
+        int log2_n = 0;
+        while ((1L << log2_n) < n) ++log2_n;
+        const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13)), shift = 32 - key_bits, n_buckets = 1 << key_bits;
+        const int n_groups = n_buckets / kFitGroup, n_parts = n_buckets / kFitSumBuckets;
+        bool bucketed = n < (1L << 31);
+        if (bucketed) {
+            try {
+                bucket_buf.reserve(static_cast<size_t>(n_buckets) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups) * 8 + static_cast<size_t>(n_groups) * 4, stream);
+                sorted_buf.reserve(static_cast<size_t>(n) * 4, stream);
+            } catch (const OutOfMemory&) {
+                bucketed = false;   // the passes over all samples need next to nothing
+            }
+        }
+        if (bucketed) {
             double* const d_sum = bucket_buf.as<double>();
             double* const d_part = d_sum + n_buckets;
             double* const d_group_sum = d_part + n_parts;
