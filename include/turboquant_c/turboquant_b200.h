@@ -41,6 +41,10 @@ const char* tq_last_error(void);
 int tq_device_count(void);
 /** Select the device used by this thread for subsequent calls and new handles. */
 int tq_set_device(int device);
+/** Device memory of freed objects is kept for the next ones, at most 512 MB per device, until something else is
+ *  freed half a minute later or an allocation of this library fails.  This call gives all of it back to the driver (for
+ *  another allocator in the process that needs it), waits for the work that may still use it, and returns the bytes. */
+size_t tq_release_cached_memory(void);
 
 /* ---- opaque tensor handle for the void* slots of turboquant_c.h ------------------
  * The reference passes `mlx::core::array*` through those slots

@@ -66,3 +66,55 @@ def test_a_fit_needs_no_memory_that_is_not_there(tq):
         del fill
         torch.cuda.empty_cache()
     assert np.all(np.abs(got.centroids - want.centroids) <= 3e-6 * np.abs(want.centroids) + 3e-7)
+
+
+def test_kept_memory_goes_back_on_request(tq):
+    torch = pytest.importorskip("torch")
+    tq.release_cached_memory()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    kv = torch.zeros((4096, 2, 128), device="cuda", dtype=torch.float16)
+    c = tq.TQKVCache(1, 2, 128)
+    c.reserve(0, 400_000)                                   # about 100 MB
+    c.append(0, kv, kv)
+    c.close()                                               # kept, with the append still queued
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] < before - (64 << 20)
+    assert tq.release_cached_memory() > (64 << 20)
+    assert torch.cuda.mem_get_info()[0] > before - (32 << 20)
+    assert tq.release_cached_memory() == 0
+
+
+def test_an_idle_block_comes_before_a_pending_one(tq):
+    """Storage that the host must be able to rely on at once does not wait for queued work while an idle block is there."""
+    torch = pytest.importorskip("torch")
+    tq.release_cached_memory()
+    kv = torch.randn((4096, 2, 128), device="cuda").half()
+    a = torch.randn((8192, 8192), device="cuda")
+    side = torch.cuda.Stream()
+
+    def make(stream=None):
+        c = tq.TQKVCache(1, 2, 128)
+        c.reserve(0, 4096, stream=stream)
+        return c
+
+    idle, pending = make(), make()
+    idle.close()
+    torch.cuda.synchronize()
+    for _ in range(6):
+        a = a @ a * 1e-4                                    # tens of milliseconds on the legacy stream
+    pending.append(0, kv, kv)
+    pending.close()
+    end = torch.cuda.Event()
+    end.record()
+    c = make(side)                                          # (the call waits for its stream, on which nothing is queued)
+    assert not end.query()
+    c.append(0, kv, kv, stream=side)
+    got = torch.empty((4096, 2, 128), dtype=torch.float16, device="cuda")
+    c.get_keys_fp16(0, 0, 4096, out=got, stream=side)
+    torch.cuda.synchronize()
+    other = make()                                          # the pending one, by now done
+    other.append(0, kv, kv)
+    assert np.array_equal(other.get_keys_fp16(0, 0, 4096).view(np.uint16), got.cpu().numpy().view(np.uint16))
+    c.close()
+    other.close()

@@ -57,6 +57,7 @@ def load() -> C.CDLL:
     sig("tq_version", C.c_char_p, [])
 
     sig("tq_array_create", vp, [vp, i, i, C.POINTER(C.c_int)])
+    sig("tq_release_cached_memory", C.c_size_t, [])
     sig("tq_array_wrap_device", vp, [vp, i, i, C.POINTER(C.c_int)])
     sig("tq_array_ndim", i, [vp])
     sig("tq_array_dim", i, [vp, i])

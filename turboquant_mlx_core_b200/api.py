@@ -102,6 +102,12 @@ class Codebook:
     bits: int
 
 
+def release_cached_memory() -> int:
+    """Gives the device memory that freed objects left for the next ones (at most 512 MB per device) back to the driver,
+    for another allocator in the process; returns the bytes."""
+    return int(_lib.load().tq_release_cached_memory())
+
+
 def generate_codebook(bits: int) -> Codebook:
     """generate_codebook (src/codebook.cpp:71-85); raises ValueError for bits outside 1..5."""
     L = _lib.load()

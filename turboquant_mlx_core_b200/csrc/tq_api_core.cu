@@ -92,6 +92,10 @@ int tq_set_device(int device) {
 
 // ---- tq_array ---------------------------------------------------------------------------
 
+size_t tq_release_cached_memory(void) {
+    return guarded<size_t>(0, 0, [&]() { return pool_trim(); });
+}
+
 tq_array_t tq_array_create(const void* data, int dtype, int ndim, const int* shape) {
     return guarded<tq_array_t>(nullptr, nullptr, [&]() -> tq_array_t {
         TQ_REQUIRE(ndim >= 0 && ndim <= 8 && dtype >= 0 && dtype <= 3, "tq_array_create: bad ndim or dtype");

@@ -77,7 +77,7 @@ bool stream_is_capturing(cudaStream_t st);
 void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream);
 // idle: nothing queued anywhere uses the block; otherwise everything that does was put on the legacy default stream.
 void pool_release(void* p, size_t bytes, int device, bool idle);
-void pool_trim();
+size_t pool_trim();   // the bytes that went back to the driver
 struct OutOfMemory : Error {
     using Error::Error;
 };

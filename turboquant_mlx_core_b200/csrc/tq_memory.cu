@@ -7,7 +7,8 @@
 //
 //   Bounded    at most kKeepBytes of unused memory per device; beyond it the blocks unused for longest go back to the
 //              driver first.  A block of more than half the bound is never kept.
-//   Given back blocks unused for kKeepSeconds at the next release, and everything unused when an allocation fails.
+//   Given back blocks unused for kKeepSeconds at the next release; everything unused when an allocation of the library fails,
+//              and when the program asks for it (tq_release_cached_memory), which it does for another allocator's sake.
 //   Threads    one mutex; a block belongs to one owner at a time.
 //   Streams    a block may be released while work that uses it is still queued.  The owner says whether all that work
 //              was put on the legacy default stream: then an event recorded there marks its end, and the next owner
@@ -72,19 +73,23 @@ Pool& pool() {
 
 }  // namespace
 
-// (An error: the legacy stream while a blocking one of the device is captured.)
 bool stream_is_capturing(cudaStream_t st) {
+    if (is_legacy_stream(st)) return false;   // it cannot be; asking takes 1.5 us
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
-    cudaGetLastError();
-    return true;
+    TQ_CUDA(cudaStreamIsCapturing(st, &cap));
+    return cap != cudaStreamCaptureStatusNone;
 }
 
 namespace {
 
 // An event recorded on the current device's legacy default stream, nullptr when that failed (the caller then waits).
 cudaEvent_t mark_legacy_stream(Pool& P, int device) {
-    if (stream_is_capturing(nullptr)) return nullptr;   // an event there would break the capture of a blocking stream
+    // While a blocking stream of the device is captured the question fails, and an event would break the capture.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
     cudaEvent_t e = nullptr;
     if (!P.events[device].empty()) {
         e = P.events[device].back();
@@ -130,30 +135,47 @@ size_t pool_size_class(size_t bytes) {
 void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream) {
     const size_t want = pool_size_class(bytes);
     Pool& P = pool();
-    if (device >= 0 && device < 64 && !stream_is_capturing(st)) {
+    if (device < 0 || device >= 64 || stream_is_capturing(st)) return device_malloc(want);
+    void* p = nullptr;
+    cudaEvent_t pending = nullptr;
+    {
         std::lock_guard<std::mutex> lock(P.mu);
-        // newest first: most likely still in the caches, and the oldest get the chance to age
-        for (auto it = P.blocks.rbegin(); it != P.blocks.rend(); ++it) {
+        // Newest first: most likely still in the caches, and the oldest get the chance to age.  Of those that the host would
+        // have to wait for (the newest, most likely) only if there is no other; work on the legacy stream waits by itself.
+        auto found = P.blocks.end();
+        for (auto it = P.blocks.end(); it != P.blocks.begin();) {
+            --it;
             if (it->bytes != want || it->device != device) continue;
-            void* const p = it->p;
-            const cudaEvent_t e = it->pending;
-            P.kept[device] -= want;
-            P.blocks.erase(std::next(it).base());
-            if (e) {
-                // work on the legacy stream is already behind the event
-                cudaError_t rc = cudaSuccess;
-                if (!on_stream) rc = cudaEventSynchronize(e);
-                else if (!is_legacy_stream(st)) rc = cudaStreamWaitEvent(st, e, 0);
-                P.events[device].push_back(e);
-                if (rc != cudaSuccess) {
-                    cudaFree(p);
-                    TQ_CUDA(rc);
-                }
+            if (found == P.blocks.end()) found = it;
+            if (it->pending == nullptr || (on_stream && is_legacy_stream(st)) || cudaEventQuery(it->pending) == cudaSuccess) {
+                found = it;
+                break;
             }
-            return p;
+            cudaGetLastError();
+        }
+        if (found != P.blocks.end()) {
+            p = found->p;
+            pending = found->pending;
+            P.kept[device] -= want;
+            P.blocks.erase(found);
         }
     }
-    return device_malloc(want);
+    if (p == nullptr) return device_malloc(want);
+    if (pending != nullptr) {
+        // work on the legacy stream is already behind the event
+        cudaError_t rc = cudaSuccess;
+        if (!on_stream) rc = cudaEventSynchronize(pending);
+        else if (!is_legacy_stream(st)) rc = cudaStreamWaitEvent(st, pending, 0);
+        {
+            std::lock_guard<std::mutex> lock(P.mu);
+            P.events[device].push_back(pending);
+        }
+        if (rc != cudaSuccess) {
+            cudaFree(p);
+            TQ_CUDA(rc);
+        }
+    }
+    return p;
 }
 
 void* device_malloc(size_t bytes) {
@@ -197,13 +219,16 @@ void pool_release(void* p, size_t bytes, int device, bool idle) {
     }
 }
 
-void pool_trim() {
+size_t pool_trim() {
     Pool& P = pool();
     std::lock_guard<std::mutex> lock(P.mu);
+    size_t freed = 0;
     while (!P.blocks.empty()) {
         DeviceGuard guard(P.blocks.front().device);
+        freed += P.blocks.front().bytes;
         free_block(P, P.blocks.begin());
     }
+    return freed;
 }
 
 unsigned int* status_word_take(int device) {
