@@ -147,6 +147,15 @@ public:
         const bool as_params = read_now && nx * sizeof(__half) <= tq::kMaxParamRowBytes;
         const __half* d_x;
         std::optional<tq::PinnedStage> x_stage, y_stage;
+        // A call that fails half-way has queued work that still reads or writes the staging: wait for it before it goes back.
+        struct StageUse {
+            const std::optional<tq::PinnedStage>&x, &y;
+            cudaStream_t st;
+            bool done = false;
+            ~StageUse() {
+                if (!done && (x || y)) cudaStreamSynchronize(st);
+            }
+        } stage_use{x_stage, y_stage, st};
         if (x_dev && x_dtype == TQ_F16) {
             d_x = static_cast<const __half*>(x);
         } else if (as_params || (read_now && !y_dev && decode_call)) {
@@ -194,6 +203,7 @@ public:
         if (!y_dev) {
             if (d_y == y_f16_.as<__half>()) TQ_CUDA(cudaMemcpyAsync(y, d_y, ny * sizeof(__half), cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));
+            stage_use.done = true;
             if (y_stage) std::memcpy(y, y_stage->host(), ny * sizeof(__half));
             require_ok(*static_cast<volatile unsigned int*>(h_status_));
         }
