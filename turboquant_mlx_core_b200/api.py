@@ -405,6 +405,8 @@ def forward_group(linears, x, outs=None, stream=None):
     if not linears or len(linears) > 4:
         raise ValueError("forward_group takes 1..4 layers")
     first = linears[0]
+    if not hasattr(x, "data_ptr"):
+        raise TQError("forward_group: x must be a device tensor")
     batch = x.numel() // x.size(-1) if x.dim() > 1 else 1
     if outs is None:
         if _torch is None:
@@ -661,11 +663,12 @@ def append_batch(caches, layer: int, keys, values, stream=None):
     n = len(caches)
     if keys.shape[0] != n or values.shape[0] != n:
         raise ValueError("keys and values must have one row per cache")
-    if hasattr(keys, "data_ptr"):
+    if hasattr(keys, "data_ptr") and hasattr(values, "data_ptr"):
         kp, vp, tag = _tensor(keys), _tensor(values), _tensor_tag(keys)
     else:
         kp, vp, tag = _ptr(keys), _ptr(values), _dtype_tag(keys)
-    if caches[0]._L.tq_kv_append_batch(_handles(caches), n, layer, kp, vp, tag, None if stream is None else _stream_ptr(stream)):
+    L = caches[0]._L if n else _lib.load()
+    if L.tq_kv_append_batch(_handles(caches), n, layer, kp, vp, tag, None if stream is None else _stream_ptr(stream)):
         check(-1, "append_batch")
 
 
@@ -678,7 +681,8 @@ def compressed_attention(caches, layer: int, queries, start: int = 0, end: int =
     lets results over disjoint token ranges be merged (sharding.merge_attention_parts)."""
     if isinstance(caches, TQKVCache):
         caches = [caches]
-    n, L = len(caches), caches[0]._L
+    n = len(caches)
+    L = caches[0]._L if n else _lib.load()
     tensor = hasattr(queries, "data_ptr")
     if not tensor:
         queries = np.ascontiguousarray(queries)
