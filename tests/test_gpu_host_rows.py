@@ -33,6 +33,22 @@ def test_host_rows_equal_device_rows(tq, rows, n_in, dtype):
     lin.close()
 
 
+@pytest.mark.parametrize("at", [0, 5, 63])
+@pytest.mark.parametrize("value", [np.nan, -np.nan, np.inf, -np.inf, 65519.99, 65520.0, -65520.0, 2.0 ** -25, -2.98e-8, 1e-45])
+def test_host_rounding_of_special_values(tq, at, value):
+    """Rows of 64: eight values at a time, and a NaN among them."""
+    torch = pytest.importorskip("torch")
+    lin = make_linear(tq, 64, 16)
+    x = np.random.default_rng(at).standard_normal((1, 64)).astype(np.float32)
+    x[0, at] = value
+    if np.isnan(value):
+        x.view(np.uint32)[0, at] = 0x7f800001 if np.signbit(value) else 0xffc12345      # signalling, and with a payload
+    got = lin.forward(x)
+    want = lin.forward(torch.from_numpy(x).cuda())
+    assert np.array_equal(got.view(np.uint16), want.cpu().numpy().view(np.uint16))
+    lin.close()
+
+
 @pytest.mark.parametrize("rows,n_in", [(1, 4096), (2, 4160), (5, 3200)])   # parameters and staging, as pageable rows
 @pytest.mark.parametrize("dtype", ["float16", "float32"])
 def test_page_locked_rows_are_read_in_stream_order(tq, rows, n_in, dtype):

@@ -5,15 +5,20 @@
 // parameters of a one-CTA kernel, which the launch delivers with no copy engine and no staging in between; the host
 // rounds fp32 to fp16 on the way (half the bytes, no conversion kernel).
 #include <cstring>
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
 
 #include "tq_common.cuh"
 #include "tq_kernels.cuh"
 
 namespace tq {
 
-// fp32 -> fp16, round to nearest even: the bits __float2half_rn gives.  Branch-free, so that the compiler vectorises it
-// (a call per element took longer than the layer's kernel).
-void host_f32_to_f16(const float* src, uint16_t* dst, size_t n) {
+// fp32 -> fp16, round to nearest even: the bits __float2half_rn gives.  (The steps are the well-known ones: rebias and add
+// half a unit less a tie's bit, add 0.5 for subnormal results; F. Giesen's public float_to_half collection has them.)  A loop
+// of one value at a time, as the compiler makes of this, takes 4 us for 4096 values, and where it came to lie moved a call by
+// 1.3 of 34 us; the processor's own conversion does eight at a time.
+static void f32_to_f16_portable(const float* src, uint16_t* dst, size_t n) {
     for (size_t i = 0; i < n; ++i) {
         uint32_t u;
         std::memcpy(&u, src + i, 4);
@@ -32,6 +37,24 @@ void host_f32_to_f16(const float* src, uint16_t* dst, size_t n) {
         h = a > 0x7f800000u ? 0x7fffu : h;    // NaN
         dst[i] = static_cast<uint16_t>(h > 0x7ffeu ? 0x7fffu : (h | sign));
     }
+}
+#if defined(__x86_64__)
+__attribute__((target("avx,f16c"))) static void f32_to_f16_eight(const float* src, uint16_t* dst, size_t n) {
+    size_t i = 0;
+    for (; i + 8 <= n; i += 8) {
+        const __m256 v = _mm256_loadu_ps(src + i);
+        if (_mm256_movemask_ps(_mm256_cmp_ps(v, v, _CMP_UNORD_Q)) != 0) f32_to_f16_portable(src + i, dst + i, 8);   // a NaN: 0x7fff, whatever its bits
+        else _mm_storeu_si128(reinterpret_cast<__m128i*>(dst + i), _mm256_cvtps_ph(v, _MM_FROUND_TO_NEAREST_INT));
+    }
+    f32_to_f16_portable(src + i, dst + i, n - i);
+}
+#endif
+void host_f32_to_f16(const float* src, uint16_t* dst, size_t n) {
+#if defined(__x86_64__)
+    static const bool eight = __builtin_cpu_supports("avx") && __builtin_cpu_supports("f16c");
+    if (eight) return f32_to_f16_eight(src, dst, n);
+#endif
+    f32_to_f16_portable(src, dst, n);
 }
 
 namespace {
