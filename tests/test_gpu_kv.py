@@ -51,9 +51,8 @@ def test_append_bits_and_decode(tq, golden, case, dtype):
 @pytest.mark.parametrize("heads,dim,tokens", [(4, 128, 300), (2, 64, 700), (1, 256, 530), (3, 32, 200), (1, 512, 515)])
 @pytest.mark.parametrize("dtype", [np.float16, np.float32])
 def test_bulk_append_bits_match_the_checker(tq, oracle, heads, dim, tokens, dtype):
-    """Appends of 512 vectors or more run the batched encoder (one thread per vector for the two
-    left-to-right sums of src/kv_cache.cpp:84-88, 226-231): every stored bit equals the CPU
-    restatement's, also when a later single-token append lands behind the bulk."""
+    """Bulk appends (four lanes per vector; the two sums of src/kv_cache.cpp:84-88, 226-231 run left to right): every stored
+    bit equals the CPU restatement's, also when a later single-token append lands behind the bulk."""
     k, v = kv_inputs(tokens + dim, tokens, heads, dim)
     c = tq.TQKVCache(1, heads, dim)
     c.append(0, k[:-1].astype(dtype), v[:-1].astype(dtype))
@@ -245,9 +244,8 @@ def test_snapshot_is_byte_identical_and_restores(tq, golden):
 
 @pytest.mark.parametrize("heads,q_heads", [(1, 4), (2, 14), (4, 28), (8, 32), (3, 6), (12, 12)])
 def test_attention_head_counts_and_ragged_ranges(tq, oracle, heads, q_heads):
-    """head_dim 128 over every way the cache is fetched: all heads of a 16-token tile as one slab
-    (1, 2, 4 KV heads), a group of four heads as per-token rows (8, 12), and the load-based kernel
-    (3); token ranges that start and end inside a tile, and shorter than one tile."""
+    """head_dim 128 for KV head counts that are and are not powers of two and groups of 1 to 7 query heads; token ranges that
+    start and end inside a 16-token tile, and shorter than one tile."""
     rng = np.random.default_rng(heads * 100 + q_heads)
     dim, n = 128, 333
     k, v = kv_inputs(int(rng.integers(1 << 30)), n, heads, dim)
@@ -256,33 +254,21 @@ def test_attention_head_counts_and_ragged_ranges(tq, oracle, heads, q_heads):
     ex = c.export(0)
     q = rng.standard_normal((1, q_heads, dim)).astype(np.float16)
     for start, end, use_qjl in [(0, n, True), (0, n, False), (5, 330, True), (17, 30, True), (32, 48, False), (331, 333, True)]:
-        # the automatic choice would run a job this small on the load-based kernel: ask for the pipeline
-        c.set_attention_kernel(c.ATTENTION_PIPELINE)
         out = tq.compressed_attention([c], 0, q, start=start, end=end, use_qjl=use_qjl)
-        c.set_attention_kernel(c.ATTENTION_LOADS)
-        other = tq.compressed_attention([c], 0, q, start=start, end=end, use_qjl=use_qjl)
-        assert rel_l2(out[0], other[0].astype(np.float32)) < ATTN_TOL
+        c.check_attention_status()
         want = oracle.attention(q[0].astype(np.float32), heads, ex["k_words"], ex["k_norms"], ex["v_words"], ex["v_norms"],
                                 ex["qjl_words"], ex["qjl_norms"], layer=0, start=start, end=end, use_qjl=use_qjl)
         assert np.all(np.isfinite(out.astype(np.float32)))
         assert rel_l2(out[0], want) < ATTN_TOL, (start, end, use_qjl, rel_l2(out[0], want))
-        if heads == 4:
-            # the tensor-memory kernel (tcgen05): tiles of 32 tokens, partial first and last tiles
-            c.set_attention_kernel(c.ATTENTION_TENSOR_MEMORY)
-            tm = tq.compressed_attention([c], 0, q, start=start, end=end, use_qjl=use_qjl)
-            c.check_attention_status()
-            assert np.all(np.isfinite(tm.astype(np.float32)))
-            assert rel_l2(tm[0], want) < ATTN_TOL, ("tensor memory", start, end, use_qjl, rel_l2(tm[0], want))
     c.close()
 
 
 @pytest.mark.parametrize("tokens", [4096, 32768])
 def test_attention_at_benchmark_contexts_matches_oracle(tq, oracle, tokens):
-    """One sequence, 4 KV / 28 query heads, at the context lengths the throughput figures are quoted
-    on: the three CUDA kernels (bulk-copy pipeline, load-based, tensor memory), residual bits off and on, each against
-    the CPU checker (mirrors src/attention_dispatch.cpp:58-73 over the fp16 keys and values that
-    src/kv_cache.cpp:292-365 would hand it).  At these lengths the context is cut into dozens of
-    splits, the softmax reference moves lazily and the parts are merged in fixed order."""
+    """One sequence, 4 KV / 28 query heads, at the context lengths the throughput figures are quoted on, residual bits off and
+    on, against the CPU checker (mirrors src/attention_dispatch.cpp:58-73 over the fp16 keys and values that
+    src/kv_cache.cpp:292-365 would hand it).  At these lengths a job is cut into dozens of parts, the softmax reference moves
+    lazily and the parts are merged in fixed order."""
     heads, dim, q_heads = 4, 128, 28
     k, v = kv_inputs(1000 + tokens, tokens, heads, dim)
     c = tq.TQKVCache(1, heads, dim)
@@ -292,34 +278,35 @@ def test_attention_at_benchmark_contexts_matches_oracle(tq, oracle, tokens):
     for use_qjl in (False, True):
         want = oracle.attention(q[0].astype(np.float32), heads, ex["k_words"], ex["k_norms"], ex["v_words"], ex["v_norms"],
                                 ex["qjl_words"], ex["qjl_norms"], layer=0, use_qjl=use_qjl)
-        for kernel in (c.ATTENTION_PIPELINE, c.ATTENTION_LOADS, c.ATTENTION_TENSOR_MEMORY):
-            c.set_attention_kernel(kernel)
-            out = tq.compressed_attention([c], 0, q, use_qjl=use_qjl)
-            c.check_attention_status()
-            assert np.all(np.isfinite(out.astype(np.float32)))
-            assert rel_l2(out[0], want) < ATTN_TOL, (tokens, use_qjl, kernel, rel_l2(out[0], want))
+        out = tq.compressed_attention([c], 0, q, use_qjl=use_qjl)
+        c.check_attention_status()
+        assert np.all(np.isfinite(out.astype(np.float32)))
+        assert rel_l2(out[0], want) < ATTN_TOL, (tokens, use_qjl, rel_l2(out[0], want))
     c.close()
 
 
-def test_attention_kernel_choice_is_automatic_for_long_batches(tq):
-    """40 sequences x 8192 tokens fill every CTA slot with 512 tokens or more: the automatic choice is the
-    pipeline kernel; it agrees with the load-based kernel, leaves the status clean, and the knob refuses
-    unknown values."""
+def test_attention_of_a_long_batch_matches_oracle(tq, oracle):
+    """40 sequences x 8192 tokens: descriptors from a table (more sequences than travel as parameters), several jobs per range.
+    Every sequence has queries of its own; the first, a middle and the last one are checked, to 2.1e-3: the checker rounds the
+    keys to fp16 and the kernel, at 128 dims, the rotated query, 2^-12 of a value in the mean each, which moves a score s by as
+    much relatively and its weight by 2^-12 |s|; scores that count reach 8 here.  The kernel choice takes its four values, which
+    mean the same, and refuses others."""
     heads, dim, q_heads, n, n_seqs = 4, 128, 28, 8192, 40
     rng = np.random.default_rng(21)
     k, v = kv_inputs(77, n, heads, dim)
     c = tq.TQKVCache(1, heads, dim)
     c.append(0, k, v)
+    ex = c.export(0)
     caches = [c] * n_seqs                      # the same storage read by every sequence of the batch
     q = rng.standard_normal((n_seqs, q_heads, dim)).astype(np.float16)
-    auto = tq.compressed_attention(caches, 0, q)
-    c.set_attention_kernel(c.ATTENTION_LOADS)
-    loads = tq.compressed_attention(caches, 0, q)
-    c.set_attention_kernel(c.ATTENTION_PIPELINE)
-    pipe = tq.compressed_attention(caches, 0, q)
+    out = tq.compressed_attention(caches, 0, q)
     c.check_attention_status()
-    assert rel_l2(auto, loads.astype(np.float32)) < ATTN_TOL
-    assert np.array_equal(auto.view(np.uint16), pipe.view(np.uint16))    # automatic == pipeline here
+    for i in (0, 17, n_seqs - 1):
+        want = oracle.attention(q[i].astype(np.float32), heads, ex["k_words"], ex["k_norms"], ex["v_words"], ex["v_norms"],
+                                ex["qjl_words"], ex["qjl_norms"], layer=0, use_qjl=False)
+        assert rel_l2(out[i], want) < 2.1e-3, i
+    for kernel in (c.ATTENTION_AUTO, c.ATTENTION_LOADS, c.ATTENTION_PIPELINE, c.ATTENTION_TENSOR_MEMORY):
+        c.set_attention_kernel(kernel)
     with pytest.raises(tq.TQError):
         c.set_attention_kernel(7)
     c.close()
