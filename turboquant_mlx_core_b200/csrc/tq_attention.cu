@@ -908,17 +908,26 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long long
     const int team = 8, teams = head_dim == 256 ? 1 : 2;
     const long most = std::min<long>(static_cast<long>(teams) * sm_count, head_dim == 32 ? AttnCfg<32>::kMaxParts : kMaxRanges);
     a.ranges = static_cast<int>(std::min<long>(most, std::max<long>(1, (units + team - 1) / team)));
-    // Or whole jobs per range.  An equal share of the tiles cuts most jobs, and the part of a job costs about 10 us more than
-    // a whole one (publish, fence, count, read back); against that stand the tiles that the longest range has more, 190 ns
-    // each with two teams on an SM and 100 ns with one (128 dims), and the end of every further job of a range, about 6 us.  Append +
-    // attention, cut against whole: 8 x 2000 tokens, 32 / 8 heads 25.1 / 16.8 us; 60 x 1500, 16 / 4 heads 46.0 / 35.1;
-    // 64 x 1000, 8 / 8 heads 56 / 49; 1 x 4096, 28 / 4 heads 18.0 / 34.0; 10 x 10539, 8 / 2 heads 27 / 54.
+    // Or whole jobs per range.  An equal share of the tiles cuts most jobs, and the part of a job costs more than a whole one
+    // (publish, fence, count, read back); against that stand the tiles that the longest range has more, and the end of every
+    // further job of a range.  Costs in ns by head size, from calls forced both ways (28 / 4 heads unless said, cut against
+    // whole, us): 32 dims 1 x 4096 tokens 8.2 / 18.0, 8 x 2000, 32 / 8 heads 10.6 / 11.0, 32 x 1000, 32 / 8 18.3 / 14.6;
+    // 64 dims 4 x 4096, 8 / 8 heads 17.2 / 27.6, 8 x 2000, 32 / 8 17.1 / 15.9, 64 x 1000, 8 / 8 35.0 / 30.5;
+    // 128 dims 1 x 4096 10.0 / 28.5, 8 x 2000, 32 / 8 19.4 / 16.6, 64 x 1000, 8 / 8 38.6 / 33.2, 10 x 10539, 8 / 2 22.4 / 68.3;
+    // 256 dims 16 x 2048, 14 / 2 31.1 / 57.2, 32 x 1000, 32 / 8 67.7 / 64.0, 64 x 1000, 8 / 8 124 / 128.
+    struct { int tile, tile_beside, part, job; } ns;   // a tile with one team on the SM, with two; a part; the end of a job
+    switch (head_dim) {
+        case 32: ns = {66, 143, 4000, 6000}; break;
+        case 64: ns = {100, 165, 7000, 6000}; break;
+        case 256: ns = {400, 400, 9000, 8000}; break;
+        default: ns = {100, 190, 10000, 6000}; break;
+    }
     const long jobs = static_cast<long>(n_seqs) * kv_heads * a.gchunks;
     const long jobs_per_range = (jobs + most - 1) / most, job_ranges = (jobs + jobs_per_range - 1) / jobs_per_range;
-    auto tile_ns = [&](long ranges) { return (ranges > sm_count ? 190L : 100L) * head_dim / 128; };
+    auto tile_ns = [&](long ranges) { return static_cast<long>(ranges > sm_count ? ns.tile_beside : ns.tile); };
     const long share = (units + a.ranges - 1) / a.ranges;
-    a.whole_jobs = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * 6000 <=
-                   share * tile_ns(a.ranges) + 10000 + 6000 * share * jobs / units;
+    a.whole_jobs = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * ns.job <=
+                   share * tile_ns(a.ranges) + ns.part + ns.job * share * jobs / units;
     if (a.whole_jobs) a.ranges = static_cast<int>(job_ranges);
     // 32: five rounds of the team's warps, about 6 us; less where ranges are short and every job ends in several of them
     a.pad = static_cast<int>(std::min<long>(32, units / a.ranges / 8));

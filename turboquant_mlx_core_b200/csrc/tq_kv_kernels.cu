@@ -587,8 +587,10 @@ void launch_kv_encode(const void* keys, const void* values, bool is_f16, int tok
     const float scale = std::sqrt(static_cast<float>(dim));             // src/kv_cache.cpp:72
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(dim));   // src/rotation.cpp:301
     const int aligned = reinterpret_cast<uintptr_t>(keys) % 16 == 0 && reinterpret_cast<uintptr_t>(values) % 16 == 0 ? 1 : 0;
-    // Few vectors: eight dims per lane, while that still spreads over the SMs in one wave (measured at D = 128).
-    if (dim <= 128 && units <= 1184) {
+    // Few vectors of 64 or 128 dims: eight dims per lane, up to 16 units per SM.  128 dims, 1040 / 2064 / 4112 units: 3.7 / 4.8 /
+    // 8.7 us against 5.4 / 5.6 / 5.9 us with four lanes per vector; 64 dims: 3.0 / 3.3 / 4.4 against 3.3 / 3.4 / 3.7.  (32 dims,
+    // 16 to 1040 units: 2.4 to 2.6 against 2.1 to 2.5.)
+    if ((dim == 64 || dim == 128) && units <= 16 * 148) {
         const dim3 few(static_cast<unsigned>((units * 2 * (dim / 8) + 63) / 64));
 #define TQ_ENC_FEW(DV)                                                                                                                \
     case DV:                                                                                                                          \
@@ -601,7 +603,7 @@ void launch_kv_encode(const void* keys, const void* values, bool is_f16, int tok
                        static_cast<const float*>(values), tokens_per_seg, n_segs, heads, k_seed, v_seed, qjl_seed, scale, inv_sqrt,   \
                        aligned, tab);                                                                                                 \
         return;
-        switch (dim) { TQ_ENC_FEW(32) TQ_ENC_FEW(64) TQ_ENC_FEW(128) }
+        switch (dim) { TQ_ENC_FEW(64) TQ_ENC_FEW(128) }
 #undef TQ_ENC_FEW
     }
     const dim3 grid(static_cast<unsigned>((units * 8 + 127) / 128));
