@@ -35,7 +35,7 @@
 //   warps 18-21 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
 //              next tile's products (up to 128 activation rows: two accumulators in turn; above, the next
 //              tile's first MMA waits until this one is read)
-// A CTA per SM walks the output tiles and its ring of stages runs on from tile to tile: with a CTA per
+// A CTA per SM walks the output tiles (of a single matrix; a group's matrices have a CTA per tile) and its ring of stages runs on from tile to tile: with a CTA per
 // tile, set-up, first loads and epilogue took 8 to 18 of 47 thousand cycles (5120 x 55296: 89 -> 76 us at
 // 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the producers bound it (about 500 cycles per 128 x 64
 // weights), at 256 the shared-memory pipe: lookups, code loads, the activation tile's write and its read.
@@ -65,7 +65,7 @@ namespace {
 
 constexpr int kTileRows = 128;  // weight rows per CTA (MMA M)
 constexpr int kTileTok = 256;   // activation rows per CTA (MMA N)
-constexpr int kBlockK = 64;     // K columns per stage
+constexpr int kBlockK = 64;     // columns of a K block
 constexpr int kSubPerStage = 2; // K blocks per pipeline stage: a stage is 128 K columns
 constexpr int kStagesMax = 4;   // ring of stages: weight tiles in tensor memory (4 x 64 columns), activation tiles in shared memory (as many as fit)
 constexpr int kGroups = 2;      // producer groups of eight warps: group g dequantises the stages g, g + 2, ...
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(256) gemm_finish_group_kernel(const FinishGrou
 }
 
 // Groups of 8 rows that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
-int rotate_row_steps(long groups) { return static_cast<int>(std::max<long>(1, std::min<long>(8, groups / (148L * 8)))); }
+int rotate_row_steps(long groups, int sm_count) { return static_cast<int>(std::max<long>(1, std::min<long>(8, groups / (8L * sm_count)))); }
 
 size_t xrot_bytes(int in, long m, int n_planes) {
     const size_t padded = (static_cast<size_t>(m) + kTileTok - 1) / kTileTok * kTileTok;  // whole operand tiles
@@ -802,7 +802,7 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
         const long n_warps = static_cast<long>(n_planes) * m * (in / static_cast<int>(block));
         const unsigned int grid = static_cast<unsigned int>((n_warps + 3) / 4);
         const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
-        const int row_steps = rotate_row_steps(static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8));
+        const int row_steps = rotate_row_steps(static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8), sm_count);
         const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 8 * row_steps - 1) / (8 * row_steps));
         if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
             auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_kernel<1> : (wide_cols == 512 ? rotate_rows_f16_wide_kernel<2> : rotate_rows_f16_wide_kernel<4>);
@@ -894,7 +894,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     // 1. the rotations: one launch for the group where the wide kernel applies
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
     const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
-    const int row_steps = rotate_row_steps(static_cast<long>(n) * n_planes * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8));
+    const int row_steps = rotate_row_steps(static_cast<long>(n) * n_planes * ((in + wide_cols - 1) / wide_cols) * ((m + 7) / 8), sm_count);
     const long wide_blocks = static_cast<long>(n_planes) * ((in + wide_cols - 1) / wide_cols) * ((m + 8 * row_steps - 1) / (8 * row_steps));
     if (reinterpret_cast<uintptr_t>(x) % 16 == 0 && wide_blocks < (1L << 31)) {
         auto* const wide = wide_cols == 256 ? rotate_rows_f16_wide_group_kernel<1>
