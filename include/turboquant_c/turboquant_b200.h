@@ -445,7 +445,7 @@ int tq_kv_apply_delta(tq_kv_cache_t cache, const void* data, size_t size);
  *  head size and length, so all four values mean the same. */
 int tq_kv_set_attention_kernel(tq_kv_cache_t cache, int kernel);
 /** Non-zero (message via tq_last_error) if an attention call on this cache that has finished
- *  reported a device-side failure (a bounded wait of the pipeline kernel ran out); clears the
+ *  reported a device-side failure (a bounded wait of the kernel ran out); clears the
  *  report.  Calls with host outputs check this themselves; callers with device outputs call it
  *  after synchronising their stream. */
 int tq_kv_attention_status(tq_kv_cache_t cache);

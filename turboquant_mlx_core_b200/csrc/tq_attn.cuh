@@ -53,12 +53,12 @@ __host__ __device__ __forceinline__ uint32_t* kv_value_row(unsigned char* block,
 __host__ __device__ __forceinline__ uint32_t kv_value_spare(uint32_t w0, uint32_t w1, uint32_t w2) {
     return ((w0 >> 6) & 0x03030303u) | ((w1 >> 4) & 0x0C0C0C0Cu) | ((w2 >> 2) & 0x30303030u);
 }
+// ... and the other way, their bits for word k.
+__host__ __device__ __forceinline__ uint32_t kv_spare_bits(uint32_t spare, int k) { return ((spare >> (2 * k)) & 0x03030303u) << 6; }
 // Norms of a block: index into its floats from kNormOff on.
 __host__ __device__ constexpr int kv_key_norm(int slot) { return 2 * slot; }
 __host__ __device__ constexpr int kv_value_norm(int slot) { return 2 * slot + 1; }
 __host__ __device__ constexpr int kv_residual_norm(int slot) { return 2 * kKvTile + slot; }
-// ... and the other way, their bits for word k.
-__host__ __device__ __forceinline__ uint32_t kv_spare_bits(uint32_t spare, int k) { return ((spare >> (2 * k)) & 0x03030303u) << 6; }
 // The bits of value word k that belong to the odd token of its pair (the others: the even token's).
 __host__ __device__ __forceinline__ uint32_t kv_odd_bits(int dim, int k) {
     return dim != 128 ? 0xF8F8F8F8u : (k == 0 ? 0x38383838u : (k == 1 ? 0xB8B8B8B8u : 0xF8F8F8F8u));

@@ -133,8 +133,6 @@ inline void launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaSt
     TQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
-// Threads of a CTA that normalises one row (the RMSNorm kernel and the row-wise all-reduce tails: the same count, so the
-// same order of additions).  A decode step has a handful of rows: the row's latency, not the SM count, is what matters.
 // Up to 8 halves (n, even, at least 4-byte aligned) from or to memory, 16 bytes at once where they are all there and aligned;
 // missing ones read as zero.
 __device__ __forceinline__ uint4 load_halves(const __half* p, int n) {
@@ -204,9 +202,10 @@ __device__ __forceinline__ void rotate_chunk(float (&v)[8], const uint4& raw, co
     }
 }
 
-// Threads of a CTA that normalises a row.  Eight columns per thread and step: 256 threads take 8192 columns in the four
-// steps that stay in registers, and eight rows run on an SM at a time (with 1024 threads and two columns per step a row's
-// barriers and reduction were most of its time).
+// Threads of a CTA that normalises a row (the RMSNorm kernel and the row-wise all-reduce tails: the same count, so the same
+// order of additions).  Eight columns per thread and step: 256 threads take 8192 columns in the four steps that stay in
+// registers, and eight rows run on an SM at a time (with 1024 threads and two columns per step a row's barriers and
+// reduction were most of its time).
 constexpr int kRowNormThreads = 256;
 constexpr int kRowNormKeep = 4;
 
