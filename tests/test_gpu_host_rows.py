@@ -33,6 +33,17 @@ def test_host_rows_equal_device_rows(tq, rows, n_in, dtype):
     lin.close()
 
 
+@pytest.mark.parametrize("rows,n_out", [(1, 32768), (1, 32769), (2, 16), (8, 4100), (9, 40)])   # stored by the kernel, and copied
+def test_host_results_equal_device_results(tq, rows, n_out):
+    torch = pytest.importorskip("torch")
+    lin = make_linear(tq, 64, n_out)
+    x = np.random.default_rng(n_out).standard_normal((rows, 64)).astype(np.float16)
+    want = lin.forward(torch.from_numpy(x).cuda()).cpu().numpy()
+    for _ in range(2):
+        assert np.array_equal(lin.forward(x).view(np.uint16), want.view(np.uint16))
+    lin.close()
+
+
 @pytest.mark.parametrize("at", [0, 5, 63])
 @pytest.mark.parametrize("value", [np.nan, -np.nan, np.inf, -np.inf, 65519.99, 65520.0, -65520.0, 2.0 ** -25, -2.98e-8, 1e-45])
 def test_host_rounding_of_special_values(tq, at, value):
