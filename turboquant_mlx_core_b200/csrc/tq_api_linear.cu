@@ -185,16 +185,16 @@ public:
             tq::launch_f32_to_f16(d_xf, x_f16_.as<__half>(), static_cast<long>(nx), st);  // src/dequantizer.cpp:691
             d_x = x_f16_.as<__half>();
         }
-        // A few rows into the caller's page-locked memory: the decode kernel stores them there itself.  One row of up to
-        // kHostStoreOutputs for pageable memory: the same through our staging.  A call of 4096 x 4096 takes 24.5 us so, 35.6 with
-        // a copy after the kernel, one of 1024 x 32768 36.9 / 40.2; but 3200 x 50694 94.7 / 80.4, four rows of 4096 x 4096
-        // 46.4 / 43.4 and eight 63.4 / 55.7: many small writes over PCIe.  Those are copied.
+        // A few rows into the caller's page-locked memory: the decode kernel stores them there itself.  Small results for pageable
+        // memory: the same through our staging, others are copied (many small writes over PCIe cost more).  Stored against
+        // copied, us a call: 4096 x 4096 at 1 / 2 / 4 / 8 rows 31 / 41 / 49 / 66 against 36 / 40 / 43 / 56; 1024 x 512 at 8 rows
+        // 33 / 39; 1024 x 2048 at 4 rows 28 / 37; 1024 x 16384 at 1 row 31 / 38, x 32768 41 / 41, x 65536 64 / 57.
         __half* d_y;
         if (y_dev) {
             d_y = static_cast<__half*>(y);
         } else if (batch <= 8 && ky.pinned_alias != nullptr) {
             d_y = static_cast<__half*>(ky.pinned_alias);
-        } else if (batch == 1 && out_ <= kHostStoreOutputs) {
+        } else if (batch <= 8 && ny <= (batch == 1 ? kHostStoreRow : kHostStoreRows)) {
             y_stage.emplace(ny * sizeof(__half));
             d_y = y_stage->device<__half>();
         } else {
@@ -442,7 +442,7 @@ private:
     // Device pointers only.  More than kGemmMinBatch rows go to the tensor-core GEMM (when the
     // shape allows); otherwise batches above 8 rows are issued as passes of 8 through the GEMV.
     static constexpr int kGemmMinBatch = 8;
-    static constexpr int kHostStoreOutputs = 32768;              // of one row that the decode kernel stores to host memory
+    static constexpr size_t kHostStoreRow = 16384, kHostStoreRows = 8192;   // results of one row, of several, that the decode kernel stores to host memory
     static constexpr size_t kHostStageBytes = size_t(4) << 20;   // rows of a host caller that go through page-locked staging
     // y_stride: elements between activation rows of y (0 = out_features: a dense [batch, out] result).
     void launch_forward(const __half* d_x, int batch, __half* d_y, cudaStream_t st, long y_stride = 0) {
