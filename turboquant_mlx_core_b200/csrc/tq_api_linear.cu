@@ -5,6 +5,7 @@
 // reference recomputes on every call — packing mode, "residual present" scan, the
 // 256-entry centroid-sum table (src/dequantizer.cpp:619-643, 674-688) — is decided once
 // when the handle is built.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -89,8 +90,26 @@ public:
                 tables[256 + b] = clamp_r(ri);
             }
         }
-        tables_.resize(512 * sizeof(float));
-        TQ_CUDA(cudaMemcpy(tables_.as<void>(), tables.data(), 512 * sizeof(float), cudaMemcpyHostToDevice));
+        // two rotations: both entries of a byte as a pair of fp16, the largest in [2^14, 2^15), rounded as the kernels round
+        // to TF32 (ten mantissa bits, ties away from zero)
+        float top = 0.0f;
+        for (const float t : tables) top = std::max(top, std::fabs(t));
+        if (dual_ && top > 0.0f && std::isfinite(top)) pair_unit_ = std::ldexp(1.0f, std::ilogb(top) - 14);
+        std::vector<float> words(tables);
+        words.resize(768);
+        for (int b = 0; b < 256; ++b) {
+            auto rounded = [&](float t) {
+                uint32_t u;
+                std::memcpy(&u, &t, sizeof u);
+                if (std::isfinite(t)) u = (u + 0x1000u) & ~0x1fffu;
+                std::memcpy(&t, &u, sizeof t);
+                return t / pair_unit_;
+            };
+            const __half2 pair = __floats2half2_rn(rounded(tables[b]), rounded(tables[256 + b]));
+            std::memcpy(&words[512 + b], &pair, sizeof pair);
+        }
+        tables_.resize(768 * sizeof(float));
+        TQ_CUDA(cudaMemcpy(tables_.as<void>(), words.data(), 768 * sizeof(float), cudaMemcpyHostToDevice));
 
         const size_t sb = tq::gemv_scratch_bytes(out_, in_, dual_ ? 2 : 1);
         if (sb) {
@@ -237,7 +256,7 @@ public:
         }
         tq::launch_tq8_gemv_scatter(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(),
                                     static_cast<const __half*>(x), d, n_dst, dst_stride, out_, in_, batch, block_,
-                                    dual_ ? 2 : 1, seed_p_, seed_r_, scratch_.as<void>(), d_status_,
+                                    dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, scratch_.as<void>(), d_status_,
                                     sm_count_, st, signal ? sig : nullptr, signal_slot, signal_value, counter_.as<unsigned int>());
     }
 
@@ -247,7 +266,7 @@ public:
         tq::GemvGroupItem it{};
         it.codes = codes_.as<uint8_t>(); it.norms = norms_.as<float>(); it.table = tables_.as<float>();
         it.y = static_cast<__half*>(y);
-        it.out = out_; it.in = in_; it.block = block_; it.n_planes = dual_ ? 2 : 1;
+        it.out = out_; it.in = in_; it.block = block_; it.n_planes = dual_ ? 2 : 1; it.pair_unit = pair_unit_;
         it.seed_p = seed_p_; it.seed_r = seed_r_;
         it.scratch = scratch_.as<void>(); it.status = d_status_;
         return it;
@@ -304,7 +323,7 @@ public:
         for (int i = 0; i < n_flags; ++i) sig[i] = static_cast<unsigned int*>(flags[i]);
         tq::GemvGather g{epoch, static_cast<const unsigned int*>(wait_flags), wait_flags ? n_wait : 0, wait_epoch};
         tq::launch_tq8_gemv_scatter(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), static_cast<const __half*>(x), d,
-                                    n_dst, dst_stride, out_, in_, batch, block_, dual_ ? 2 : 1, seed_p_, seed_r_, scratch_.as<void>(),
+                                    n_dst, dst_stride, out_, in_, batch, block_, dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, scratch_.as<void>(),
                                     d_status_, sm_count_, st, sig, slot, 0u, counter_.as<unsigned int>(), &g, n_flags);
     }
 
@@ -324,7 +343,7 @@ public:
         g.ll_world = world;
         for (int r = 0; r < world; ++r) g.ll_base[r] = packet_bufs[r];
         tq::launch_tq8_gemv_scatter(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), static_cast<const __half*>(x), d, 1,
-                                    y_stride, out_, in_, batch, block_, dual_ ? 2 : 1, seed_p_, seed_r_, scratch_.as<void>(), d_status_,
+                                    y_stride, out_, in_, batch, block_, dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, scratch_.as<void>(), d_status_,
                                     sm_count_, st, nullptr, 0, 0u, counter_.as<unsigned int>(), &g, 0);
     }
 
@@ -385,7 +404,7 @@ public:
         else
             tq::launch_tq8_gemv_static(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(),
                                        static_cast<const __half*>(x), static_cast<__half*>(y), out_, in_, batch, block_,
-                                       dual_ ? 2 : 1, seed_p_, seed_r_, d_status_, sm_count_, st);
+                                       dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, d_status_, sm_count_, st);
     }
 
     ~TurboQuantLinear() {
@@ -464,7 +483,7 @@ private:
                 __half* dst = d_y + static_cast<size_t>(b0) * y_stride;
                 tq::launch_tq8_gemv_scatter(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(),
                                             d_x + static_cast<size_t>(b0) * in_, &dst, 1, y_stride, out_, in_, nb, block_,
-                                            dual_ ? 2 : 1, seed_p_, seed_r_, scratch_.as<void>(), d_status_, sm_count_, st);
+                                            dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, scratch_.as<void>(), d_status_, sm_count_, st);
             }
             return;
         }
@@ -478,7 +497,7 @@ private:
             else
                 tq::launch_tq8_gemv(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(),
                                     d_x + static_cast<size_t>(b0) * in_, d_y + static_cast<size_t>(b0) * out_, out_, in_, nb,
-                                    block_, dual_ ? 2 : 1, seed_p_, seed_r_, scratch_.as<void>(),
+                                    block_, dual_ ? 2 : 1, pair_unit_, seed_p_, seed_r_, scratch_.as<void>(),
                                     d_status_, sm_count_, st);
         }
     }
@@ -488,6 +507,7 @@ private:
     tq::StreamUse use_;
     int device_ = 0, sm_count_ = 0;
     bool primary_5bit_ = false, has_residual_ = false, shared_ = false, dual_ = false;
+    float pair_unit_ = 1.0f;   // two rotations: unit of the fp16 pair table, a power of two
     uint32_t seed_p_ = 0, seed_r_ = 0;
     DeviceBuffer codes_, norms_, tables_, scratch_, staged_scratch_, gemm_scratch_, counter_;
     int decode_kernel_ = 0;               // 0 / 1: register-streamed kernel (the default), 2: bulk-copy staged kernel (TQ_DECODE_KERNEL=staged)

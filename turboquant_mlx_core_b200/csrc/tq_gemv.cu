@@ -44,10 +44,15 @@
 // the slots' partial sums in slot order (a fixed order, so results do not depend on scheduling), applies
 // norm*inv_scale and writes fp16.
 // Dual-rotation weights (separate sign seeds for the primary and residual planes,
-// src/dequantizer.cpp:214-246) run as two "planes": plane 0 looks up the primary
-// centroid of each joint byte against x rotated with the primary seed, plane 1 the
-// residual centroid against x rotated with the residual seed; planes are just further
-// partial-sum slots.
+// src/dequantizer.cpp:214-246): the activation is rotated with either seed, and a weight is the pair (primary centroid,
+// residual centroid) against the pair of rotated values.  A table word holds the pair as two fp16 numbers, and so does a
+// word of the activation: one lookup fetches both, and an m16n8k16 product takes eight columns of both planes where the
+// single-rotation kernel's m16n8k8 takes eight columns of one; everything else is the same.  (As further partial-sum slots
+// the planes took two lookups and a pass each: 3584 x 3584, block 512, 16.5 us at one row, 19.2 at four, 20.9 at eight; as
+// pairs 8.4, 11.0 and 12.7.)  fp16 has the ten mantissa bits of TF32, and powers of two bring its range to the values: one for the
+// table (its largest entry lies in [2^14, 2^15)) and one for every 256 columns of a rotated row, which rotate_x_pair_kernel
+// finds.  The operands are the TF32 numbers they were; what falls below fp16's normal numbers is 2^-28 of the largest beside it.
+// Relative error against 64-bit products, 12 draws of 8 rows: 3.772e-4 / 3.772e-4 (3584 columns), 3.633e-4 / 3.633e-4 (18944).
 #include <cmath>
 #include <cstdint>
 
@@ -176,22 +181,101 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
 }
 constexpr size_t kRotateXSmem = 48 * 1024;
 
+// The activation of weights with two rotations: a warp rotates CHUNKS x 256 columns of a row with either seed and writes pairs
+// of fp16 (primary, residual), [row][in], each 256 columns times a power of two that brings the largest value of the
+// two to [2^14, 2^15), and that power's inverse to xscale[row][columns / 256].  A row that is not 16-byte aligned (`aligned` = 0) is
+// read in halves: 2 KB at most per warp.
+template <int CHUNKS>
+__global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __restrict__ x, uint32_t* __restrict__ pairs, float* __restrict__ xscale,
+                                                            int in, int batch, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt,
+                                                            int aligned) {
+    grid_launch_dependents();
+    grid_dependency_sync();
+    const int lane = threadIdx.x & 31;
+    const int slices = (in + kSlice - 1) / kSlice, groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (warp >= batch * groups_per_row) return;
+    const int row = warp / groups_per_row, col = (warp - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
+    const unsigned live = __ballot_sync(0xffffffffu, col < in);   // the lanes that exchange values
+    if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
+    const __half* const src = x + static_cast<size_t>(row) * in + col;
+    uint4 raw[CHUNKS];
+    if (aligned) {
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
+    } else {
+        const unsigned short* const h = reinterpret_cast<const unsigned short*>(src);
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = __ldg(h + 256 * c + 2 * j) | (static_cast<uint32_t>(__ldg(h + 256 * c + 2 * j + 1)) << 16);
+            raw[c] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    float v[2][CHUNKS][8];
+#pragma unroll
+    for (int plane = 0; plane < 2; ++plane) {
+        const uint32_t seed = plane ? seed_r : seed_p;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[plane][c], raw[c], chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block), block, lane, live);
+#pragma unroll
+        for (int h = 1; h < CHUNKS; h <<= 1)
+#pragma unroll
+            for (int i = 0; i < CHUNKS; i += 2 * h)
+#pragma unroll
+                for (int c = i; c < i + h; ++c)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float a = v[plane][c][j], b = v[plane][c + h][j];
+                        v[plane][c][j] = __fadd_rn(a, b);
+                        v[plane][c + h][j] = __fsub_rn(a, b);
+                    }
+    }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+        unsigned int top = 0;
+#pragma unroll
+        for (int plane = 0; plane < 2; ++plane)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[plane][c][j] = to_tf32(v[plane][c][j] * inv_sqrt);
+                top = max(top, __float_as_uint(v[plane][c][j]) & 0x7fffffffu);
+            }
+        // 2^(14 - exponent), between 2^-113 and 2^126 (its inverse is a normal number); 1 beside an infinity or a NaN
+        const unsigned int e = __reduce_max_sync(live, top) >> 23;
+        const unsigned int f = e == 255u ? 127u : min(268u - e, 253u);
+        const float up = __uint_as_float(f << 23);
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const __half2 h = __floats2half2_rn(v[0][c][j] * up, v[1][c][j] * up);
+            w[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        uint4* const dst = reinterpret_cast<uint4*>(pairs + static_cast<size_t>(row) * in + col + 256 * c);
+        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        if (lane == 0) xscale[row * slices + col / kSlice + c] = __uint_as_float((254u - f) << 23);
+    }
+}
+
 struct GemvArgs {
     const uint8_t* codes;   // joint bytes in 16 x 64 tiles (code_offset)
     const float* norms;     // [out]
-    const float* table;     // [n_planes, 256] fp32
-    const float* xrot;      // [n_planes, batch, in] fp32 (TF32-rounded); used when x == nullptr
+    const float* table;     // [256] fp32; two rotations: [256] pairs of fp16
+    const float* xrot;      // [batch, in] fp32 (TF32-rounded), used when x == nullptr; two rotations: pairs of fp16
+    const float* xscale;    // two rotations: [8, ceil(in / 256)] what the pairs of a row's 256 columns are to be multiplied by
     const __half* x;        // [batch, in] fp16: rotate inside the kernel (WHT block <= 256), else nullptr
     __half* y;              // [batch, y_stride]: row r of activation row n at y[n * y_stride + r]
     float* partial;         // [n_slots, 8, out_pad] (only when n_slots > 1)
     unsigned int* counters; // [n_row_units][16 warps] (only when n_slots > 1)
     unsigned int* status;   // device error word (0 = ok)
     int out, in, batch;
-    int n_row_units, n_chunks, n_slots, out_pad;  // n_slots = n_planes * n_chunks
+    int n_row_units, n_slots, out_pad;  // n_slots = chunks of a row
     int wpt, tpu;           // warps per row tile, row tiles per unit (wpt * tpu = 16)
     float inv_scale;
-    uint32_t seed_p, seed_r;   // sign seeds of plane 0 / plane 1 (in-kernel rotation)
-    int block;                 // WHT block size                  (in-kernel rotation)
+    uint32_t seed_p;           // sign seed       (in-kernel rotation)
+    int block;                 // WHT block size  (in-kernel rotation)
     float inv_sqrt_block;
 };
 
@@ -314,6 +398,13 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---- flag-in-data exchange (see ScatterArgs) ----
 __device__ __forceinline__ void ll_wait_packets(const unsigned int* wait_epoch, const uint4* mine, int rank, int world, long packets,
                                                 unsigned int* status) {
@@ -362,7 +453,8 @@ __device__ __forceinline__ void ll_send_packets(const ScatterArgs& sc, const __h
 // geometry and the reduction need no runtime arithmetic).
 // MULTI = more than one slot (row units finished through partial sums in scratch); compile time, so that the
 // single-slot kernels carry none of that path's state in their 128 registers.
-template <int BP, bool SCATTER, bool LL, bool MULTI>
+// DUAL = weights with two rotations: table words and activation words are pairs of fp16.
+template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL>
 __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk) {
     // columns per chunk, derived here: one more field in GemvArgs made ptxas spill within the 128 registers
     const int chunk_cols = p.wpt * kSlice;
@@ -382,7 +474,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-    // ---- unit range of this CTA: unit = (slot, row unit), slot = plane * n_chunks + chunk ----
+    // ---- unit range of this CTA: unit = (slot, row unit), a slot is a chunk of columns ----
     // (the first `rem` CTAs take one unit more; one 32-bit division - the prologue runs once per launch on
     // instructions that are not cached yet, and cannot overlap the preceding kernel, whose CTA fills this SM)
     const int n_units = p.n_row_units * p.n_slots;
@@ -433,7 +525,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             u.slot = 0;
             u.ru = unit;
         }
-        const int c = (MULTI ? (u.slot % p.n_chunks) * chunk_cols : 0) + slice0;  // first column of this warp's slice
+        const int c = (MULTI ? u.slot * chunk_cols : 0) + slice0;  // first column of this warp's slice
         const int tile = u.ru * p.tpu + tile_in_unit;
         u.ptr = p.codes + (static_cast<size_t>(tile) * tiles_per_row + static_cast<size_t>(c >> 6)) * kCodeTileBytes + g * 64 + 16 * q;
         u.ok = 0;
@@ -472,22 +564,13 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         load_step(cur, s, true, blo[s], bhi[s]);
     }
 
-    auto build_table = [&](int plane) {
-        // 256 entries x 32 copies; a thread writes 4 consecutive copies per store
-        const int copy4 = (tid & 7) * 4;
-        for (int e = tid >> 3; e < 256; e += kConsumerThreads / 8) {
-            const float v = to_tf32(__ldg(p.table + plane * 256 + e));
-            sts_v4(kLutAddr + static_cast<uint32_t>(e) * 256u + static_cast<uint32_t>(copy4) * 4u, v, v, v, v);
-        }
-    };
     // Prologue order: table entries are fetched into registers (they do not depend on the
     // preceding kernel), then comes the dependency wait, then this warp's activation slice of
     // the first unit is requested, and only then are the table entries written to shared
     // memory - so the activation's latency hides behind the table build.
-    int staged_plane = MULTI ? cur.slot / p.n_chunks : 0;
     float tab_first[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) tab_first[k] = __ldg(p.table + staged_plane * 256 + (tid >> 3) + 64 * k);
+    for (int k = 0; k < 4; ++k) tab_first[k] = __ldg(p.table + (tid >> 3) + 64 * k);
 
     // Everything below reads or writes data the preceding kernels produce or still use.
     grid_dependency_sync();
@@ -518,13 +601,13 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         }
     }
     uint4 x_first = make_uint4(0, 0, 0, 0);
-    if (p.x != nullptr) {
-        const int cl0 = (MULTI ? (cur.slot - staged_plane * p.n_chunks) * chunk_cols : 0) + slice0 + 8 * lane;
+    if (!DUAL && p.x != nullptr) {
+        const int cl0 = (MULTI ? cur.slot * chunk_cols : 0) + slice0 + 8 * lane;
         if (cl0 < p.in) x_first = __ldg(reinterpret_cast<const uint4*>(p.x + cl0));
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float v = to_tf32(tab_first[k]);
+        const float v = DUAL ? tab_first[k] : to_tf32(tab_first[k]);
         sts_v4(kLutAddr + static_cast<uint32_t>((tid >> 3) + 64 * k) * 256u + static_cast<uint32_t>((tid & 7) * 4) * 4u, v, v, v, v);
     }
     __syncthreads();  // table and barriers visible
@@ -641,27 +724,20 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     uint32_t rpar = 0;      // parity of its "written" phase = ((i - kLag) / kRing) & 1
     Pos red = cur;          // position of the unit being summed
 
-    // Makes `slot` the current one: switches the table when the plane changes and rebuilds this
-    // warp's B fragments.  x0 is this lane's first-row activation when the caller has already
-    // requested it (have_x0).
+    // Makes `slot` the current one: rebuilds this warp's B fragments.  x0 is this lane's first-row activation when the
+    // caller has already requested it (have_x0).
+    float xs[2];   // two rotations: the scales of activation rows 2q and 2q + 1 in this warp's slice
     auto stage_slot = [&](int slot, const uint4& x0, bool have_x0) {
-        const int plane = MULTI ? slot / p.n_chunks : 0;
-            if (plane != staged_plane) {
-                named_barrier_sync(1, kConsumerThreads);  // nobody still reads the previous table
-                build_table(plane);
-                named_barrier_sync(1, kConsumerThreads);
-                staged_plane = plane;
-            }
             // B fragment of MMA (s, m): k = q -> column 64 s + 16 q + 2 m, k = q+4 -> the next column; n = g.
-            const int colw = (MULTI ? (slot - plane * p.n_chunks) * chunk_cols : 0) + slice0;  // first column of this warp's slice
+            const int colw = (MULTI ? slot * chunk_cols : 0) + slice0;  // first column of this warp's slice
             const int col0 = colw + 16 * q;
-            if (BP == 1 && p.x != nullptr) {
+            if (BP == 1 && !DUAL && p.x != nullptr) {
                 // One activation row (the launcher rotates in here only then): rotate this warp's 256 columns of it.
                 // Lane l holds columns 8l..8l+7 of the slice, stages below 8 stay in the lane, the rest are lane
                 // exchanges (same add tree as rotate_x_kernel).  A 1 KB strip of shared memory per warp turns the
                 // result into the fragment layout.  Every lane loads the row's fragment, so B columns 1..7 repeat
                 // column 0 and their results are never read: nothing to clear.
-                const uint32_t seed = plane ? p.seed_r : p.seed_p;
+                const uint32_t seed = p.seed_p;
                 const int cl = colw + 8 * lane;
                 uint4 xc = x0;
                 if (!have_x0) {
@@ -710,7 +786,15 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                                      : "r"(strip_addr + static_cast<uint32_t>(64 * s + 16 * q + k) * 4u));
                 __syncwarp();
             } else {
-            const float* xr = p.xrot + (static_cast<size_t>(plane) * p.batch + g) * p.in + col0;
+            const float* xr = p.xrot + static_cast<size_t>(g) * p.in + col0;
+            if constexpr (DUAL) {
+                const int slices = (p.in + kSlice - 1) / kSlice;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const int n = 2 * q + k;
+                    xs[k] = (n < BP && n < p.batch && colw < p.in) ? p.xscale[n * slices + colw / kSlice] : 0.f;
+                }
+            }
             const bool have_row = g < p.batch;
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
@@ -727,11 +811,9 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             }
         staged_slot = slot;
     };
-    stage_slot(cur.slot, x_first, p.x != nullptr);
+    stage_slot(cur.slot, x_first, !DUAL && p.x != nullptr);
 
     for (int i = 0; i < n_local; ++i) {
-        const int plane = cur.slot / p.n_chunks;
-        (void)plane;
         if (cur.slot != staged_slot) stage_slot(cur.slot, make_uint4(0, 0, 0, 0), false);
         const bool has_next = i + 1 < n_local;
 
@@ -763,8 +845,13 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 uint32_t av[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) av[k] = lut_load(ad[k]);
-                mma_tf32(acc0, av[0], av[1], av[2], av[3], bfrag[s][4 * w + 0], bfrag[s][4 * w + 1]);
-                mma_tf32(acc1, av[4], av[5], av[6], av[7], bfrag[s][4 * w + 2], bfrag[s][4 * w + 3]);
+                if constexpr (DUAL) {
+                    mma_f16(acc0, av[0], av[1], av[2], av[3], bfrag[s][4 * w + 0], bfrag[s][4 * w + 1]);
+                    mma_f16(acc1, av[4], av[5], av[6], av[7], bfrag[s][4 * w + 2], bfrag[s][4 * w + 3]);
+                } else {
+                    mma_tf32(acc0, av[0], av[1], av[2], av[3], bfrag[s][4 * w + 0], bfrag[s][4 * w + 1]);
+                    mma_tf32(acc1, av[4], av[5], av[6], av[7], bfrag[s][4 * w + 2], bfrag[s][4 * w + 3]);
+                }
             }
         }
         if (!has_next) grid_launch_dependents();  // the next kernel may start setting up
@@ -787,6 +874,13 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             // C fragment: (row g, columns 2q, 2q+1) and (row g+8, same columns)
             const uint32_t dst = red_addr + static_cast<uint32_t>(ws) * kSlotBytes + static_cast<uint32_t>(warp * kTileFloats) * 4u;
             const int n = 2 * q;
+            if constexpr (DUAL) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    acc0[k] *= xs[k & 1];
+                    acc1[k] *= xs[k & 1];
+                }
+            }
             if (n < BP) {
                 sts_f32(dst + static_cast<uint32_t>(g * BP + n) * 4u, acc0[0] + acc1[0]);
                 sts_f32(dst + static_cast<uint32_t>((g + 8) * BP + n) * 4u, acc0[2] + acc1[2]);
@@ -891,17 +985,17 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     }
 }
 
-template <int BP, bool MULTI>
+template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_kernel(const GemvArgs p) {
-    gemv_body<BP, false, false, MULTI>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    gemv_body<BP, false, false, MULTI, DUAL>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
 }
-template <int BP, bool MULTI>
+template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_packets_kernel(const GemvArgs p, const ScatterArgs sc) {
-    gemv_body<BP, true, true, MULTI>(p, sc, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    gemv_body<BP, true, true, MULTI, DUAL>(p, sc, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
 }
-template <int BP, bool MULTI>
+template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_scatter_kernel(const GemvArgs p, const ScatterArgs sc) {
-    gemv_body<BP, true, false, MULTI>(p, sc, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    gemv_body<BP, true, false, MULTI, DUAL>(p, sc, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
 }
 
 // Several matrices that multiply the same activation (q / k / v, gate / up) in one launch: the grid is cut into one
@@ -913,12 +1007,12 @@ struct GemvGroupArgs {
     int cta_start[kMaxGroup + 1];   // CTAs cta_start[i] .. cta_start[i + 1] - 1 work on matrix i
     int n;
 };
-template <int BP, bool MULTI>
+template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_group_kernel(const __grid_constant__ GemvGroupArgs grp) {
     const int b = static_cast<int>(blockIdx.x);
     int i = 0;
     while (i + 1 < grp.n && b >= grp.cta_start[i + 1]) ++i;
-    gemv_body<BP, false, false, MULTI>(grp.m[i], ScatterArgs{}, b - grp.cta_start[i], grp.cta_start[i + 1] - grp.cta_start[i]);
+    gemv_body<BP, false, false, MULTI, DUAL>(grp.m[i], ScatterArgs{}, b - grp.cta_start[i], grp.cta_start[i + 1] - grp.cta_start[i]);
 }
 
 // Waits (bounded) until flags[0..n) have all reached `value`: the receiving side of the completion
@@ -965,9 +1059,7 @@ int chunk_columns(int in) { return warps_per_tile(in) * kSlice; }
 }  // namespace
 
 // Scratch layout: [xrot: n_planes*8*in fp32][partials: n_slots*8*out_pad fp32][counters: n_row_tiles*16 u32]
-size_t gemv_scratch_bytes(int out, int in, int n_planes) {
-    const int chunk = chunk_columns(in);
-    const int n_slots = ((in + chunk - 1) / chunk) * n_planes;
+static size_t scratch_bytes(int out, int in, int n_planes, int n_slots) {
     const int n_row_tiles = (out + 15) / 16;
     const size_t out_pad = static_cast<size_t>(n_row_tiles) * 16;
     size_t bytes = align256(static_cast<size_t>(n_planes) * 8 * in * sizeof(float));
@@ -976,35 +1068,42 @@ size_t gemv_scratch_bytes(int out, int in, int n_planes) {
                  align256(static_cast<size_t>(n_row_tiles) * kWarps * sizeof(unsigned int));
     return bytes;
 }
+static int chunk_count(int in) { return (in + chunk_columns(in) - 1) / chunk_columns(in); }
+size_t gemv_scratch_bytes(int out, int in, int n_planes) { return scratch_bytes(out, in, n_planes, chunk_count(in)); }
 
 // Geometry, rotation mode and scratch pointers of one matrix (codes, norms, table, y and status are the caller's).
 // Returns whether the kernel rotates the activation itself; otherwise rotate_x_kernel fills a.xrot first.
-static bool fill_gemv_args(GemvArgs& a, const __half* x, int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
-                           uint32_t seed_r, void* scratch) {
+static bool fill_gemv_args(GemvArgs& a, const __half* x, int out, int in, int batch, uint32_t block, int n_planes, float pair_unit,
+                           uint32_t seed_p, void* scratch) {
     a.out = out; a.in = in; a.batch = batch;
     const int n_row_tiles = (out + 15) / 16;
     a.wpt = warps_per_tile(in);
     a.tpu = kWarps / a.wpt;
-    const int chunk = a.wpt * kSlice;  // columns per chunk
-    a.n_chunks = (in + chunk - 1) / chunk;
-    a.n_slots = a.n_chunks * n_planes;
+    a.n_slots = chunk_count(in);
     a.out_pad = n_row_tiles * 16;
     a.n_row_units = (n_row_tiles + a.tpu - 1) / a.tpu;
     a.inv_scale = 1.0f / std::sqrt(static_cast<float>(in));
+    if (n_planes == 2) {
+        a.table += 512;          // (the pairs, behind the two tables)
+        a.inv_scale *= pair_unit;
+    }
     // Blocks that fit a warp's 256-column slice are rotated inside the GEMV kernel (16-byte
     // activation loads); larger blocks, or an unaligned activation, go through rotate_x_kernel.
     // In-kernel rotation handles one activation row after the other (a chain of lane exchanges per row) in every
     // warp, which costs more than the pre-kernel from two rows on (4096 x 4096: 9.0 / 11.3 / 15.3 us in-kernel
     // against 8.3 / 9.2 / 10.8 us with the pre-kernel at 2 / 4 / 8 rows; the same at one row).
-    const bool fused_rotation = block <= static_cast<uint32_t>(kSlice) && in % 8 == 0 &&
+    // Two rotations always take the pre-kernel: a warp's strip in here would be two such chains, and the scales must be known
+    // before the first product (1024 x 512, block 128, one row: 7.3 us with two chains in every warp, 5.0 with the pre-kernel).
+    const bool fused_rotation = n_planes == 1 && block <= static_cast<uint32_t>(kSlice) && in % 8 == 0 &&
                                 reinterpret_cast<uintptr_t>(x) % 16 == 0 && batch == 1;
     a.x = fused_rotation ? x : nullptr;
-    a.seed_p = seed_p; a.seed_r = seed_r;
+    a.seed_p = seed_p;
     a.block = static_cast<int>(block);
     a.inv_sqrt_block = 1.0f / std::sqrt(static_cast<float>(block));
     uint8_t* sp = static_cast<uint8_t*>(scratch);
     float* xrot = reinterpret_cast<float*>(sp);
     a.xrot = xrot;
+    a.xscale = xrot + static_cast<size_t>(8) * in;   // (two rotations: the second plane's room)
     if (a.n_slots > 1) {
         sp += align256(static_cast<size_t>(n_planes) * 8 * in * sizeof(float));
         a.partial = reinterpret_cast<float*>(sp);
@@ -1015,12 +1114,14 @@ static bool fill_gemv_args(GemvArgs& a, const __half* x, int out, int in, int ba
     return fused_rotation;
 }
 
+static void launch_rotate_x_pair(const __half* x, float* xrot, int in, int batch, uint32_t block, uint32_t seed_p, uint32_t seed_r,
+                                 cudaStream_t stream);
 // Shared-memory opt-in of every instantiation, once per device.
 static void configure_gemv_kernels();
 void launch_tq8_gemv(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
-                     int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
-                     void* scratch, unsigned int* status, int sm_count, cudaStream_t stream) {
-    launch_tq8_gemv_scatter(codes, norms, table, x, &y, 1, out, out, in, batch, block, n_planes, seed_p, seed_r, scratch,
+                     int out, int in, int batch, uint32_t block, int n_planes, float pair_unit,
+                     uint32_t seed_p, uint32_t seed_r, void* scratch, unsigned int* status, int sm_count, cudaStream_t stream) {
+    launch_tq8_gemv_scatter(codes, norms, table, x, &y, 1, out, out, in, batch, block, n_planes, pair_unit, seed_p, seed_r, scratch,
                             status, sm_count, stream);
 }
 
@@ -1032,7 +1133,7 @@ void launch_peer_wait(const unsigned int* flags, int n, unsigned int value, unsi
 
 void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const float* table, const __half* x,
                              __half* const* dst, int n_dst, long dst_stride, int out, int in, int batch, uint32_t block,
-                             int n_planes, uint32_t seed_p, uint32_t seed_r, void* scratch, unsigned int* status,
+                             int n_planes, float pair_unit, uint32_t seed_p, uint32_t seed_r, void* scratch, unsigned int* status,
                              int sm_count, cudaStream_t stream, unsigned int* const* signal, int signal_slot,
                              unsigned int signal_value, unsigned int* done_counter, const GemvGather* gather, int n_signal) {
     TQ_REQUIRE(dst != nullptr && n_dst >= 1 && n_dst <= 8, "tq8_gemv: 1..8 destinations");
@@ -1094,7 +1195,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
         sa.n_wait = gather->n_wait;
         sa.wait_epoch = gather->wait_epoch;
     }
-    const bool fused_rotation = fill_gemv_args(a, x, out, in, batch, block, n_planes, seed_p, seed_r, scratch);
+    const bool fused_rotation = fill_gemv_args(a, x, out, in, batch, block, n_planes, pair_unit, seed_p, scratch);
     float* xrot = const_cast<float*>(a.xrot);
     const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));
 
@@ -1106,7 +1207,8 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     const int n_attr = 1;
 
     // 1. rotate the activation (one warp per plane x row x block)
-    if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, n_planes, seed_p, seed_r, stream);
+    if (n_planes == 2) launch_rotate_x_pair(x, xrot, in, batch, block, seed_p, seed_r, stream);
+    else if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, 1, seed_p, seed_r, stream);
     // 2. the GEMV itself
     {
         const int n_units = a.n_row_units * a.n_slots;
@@ -1119,10 +1221,13 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
         cfg.numAttrs = n_attr;
         // one destination with the layer's own row stride and no signal: the plain variant
         const bool scatter = sa.n_peer > 0 || sa.n_signal > 0 || sa.ll != 0 || sa.y_stride != a.out;
-#define TQ_GEMV_LAUNCH2(BPV, MV)                                                                  \
-    if (sa.ll) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_packets_kernel<BPV, MV>, a, sa));        \
-    else if (scatter) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_scatter_kernel<BPV, MV>, a, sa)); \
-    else TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_kernel<BPV, MV>, a));
+#define TQ_GEMV_LAUNCH3(BPV, MV, DV)                                                                  \
+    if (sa.ll) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_packets_kernel<BPV, MV, DV>, a, sa));        \
+    else if (scatter) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_scatter_kernel<BPV, MV, DV>, a, sa)); \
+    else TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_kernel<BPV, MV, DV>, a));
+#define TQ_GEMV_LAUNCH2(BPV, MV)                         \
+    if (n_planes == 2) { TQ_GEMV_LAUNCH3(BPV, MV, true) } \
+    else { TQ_GEMV_LAUNCH3(BPV, MV, false) }
 #define TQ_GEMV_LAUNCH(BPV)                           \
     if (a.n_slots > 1) { TQ_GEMV_LAUNCH2(BPV, true) } \
     else { TQ_GEMV_LAUNCH2(BPV, false) }
@@ -1134,6 +1239,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
         }
 #undef TQ_GEMV_LAUNCH
 #undef TQ_GEMV_LAUNCH2
+#undef TQ_GEMV_LAUNCH3
     }
 }
 
@@ -1144,20 +1250,24 @@ static void configure_gemv_kernels() {
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev < 64 && configured[dev]) return;
 #define TQ_GEMV_ATTR1(K) TQ_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemvSmem)));
-#define TQ_GEMV_ATTR(BPV)                                \
-    TQ_GEMV_ATTR1((tq8_gemv_kernel<BPV, false>))         \
-    TQ_GEMV_ATTR1((tq8_gemv_kernel<BPV, true>))          \
-    TQ_GEMV_ATTR1((tq8_gemv_scatter_kernel<BPV, false>)) \
-    TQ_GEMV_ATTR1((tq8_gemv_scatter_kernel<BPV, true>))  \
-    TQ_GEMV_ATTR1((tq8_gemv_packets_kernel<BPV, false>)) \
-    TQ_GEMV_ATTR1((tq8_gemv_packets_kernel<BPV, true>))  \
-    TQ_GEMV_ATTR1((tq8_gemv_group_kernel<BPV, false>))   \
-    TQ_GEMV_ATTR1((tq8_gemv_group_kernel<BPV, true>))
+#define TQ_GEMV_ATTR2(BPV, DV)                               \
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<BPV, false, DV>))         \
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<BPV, true, DV>))          \
+    TQ_GEMV_ATTR1((tq8_gemv_scatter_kernel<BPV, false, DV>)) \
+    TQ_GEMV_ATTR1((tq8_gemv_scatter_kernel<BPV, true, DV>))  \
+    TQ_GEMV_ATTR1((tq8_gemv_packets_kernel<BPV, false, DV>)) \
+    TQ_GEMV_ATTR1((tq8_gemv_packets_kernel<BPV, true, DV>))  \
+    TQ_GEMV_ATTR1((tq8_gemv_group_kernel<BPV, false, DV>))   \
+    TQ_GEMV_ATTR1((tq8_gemv_group_kernel<BPV, true, DV>))
+#define TQ_GEMV_ATTR(BPV)     \
+    TQ_GEMV_ATTR2(BPV, false) \
+    TQ_GEMV_ATTR2(BPV, true)
     TQ_GEMV_ATTR(1)
     TQ_GEMV_ATTR(2)
     TQ_GEMV_ATTR(4)
     TQ_GEMV_ATTR(8)
 #undef TQ_GEMV_ATTR
+#undef TQ_GEMV_ATTR2
 #undef TQ_GEMV_ATTR1
     if (dev < 64) configured[dev] = true;
 }
@@ -1179,7 +1289,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
         TQ_REQUIRE(it.in % static_cast<int>(it.block) == 0, "in_features must be divisible by block_size");
         GemvArgs& a = grp.m[i];
         a.codes = it.codes; a.norms = it.norms; a.table = it.table; a.y = it.y; a.status = it.status;
-        fused[i] = fill_gemv_args(a, x, it.out, it.in, batch, it.block, it.n_planes, it.seed_p, it.seed_r, it.scratch);
+        fused[i] = fill_gemv_args(a, x, it.out, it.in, batch, it.block, it.n_planes, it.pair_unit, it.seed_p, it.scratch);
         units[i] = a.n_row_units * a.n_slots;
         total_units += units[i];
     }
@@ -1209,9 +1319,11 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     for (int i = n; i < kMaxGroup; ++i) grp.cta_start[i + 1] = grp.cta_start[n];
     configure_gemv_kernels();
     for (int i = 0; i < n; ++i)
-        if (!fused[i])
-            launch_rotate_x(x, const_cast<float*>(grp.m[i].xrot), items[i].in, batch, items[i].block, items[i].n_planes,
-                                items[i].seed_p, items[i].seed_r, stream);
+        if (!fused[i]) {
+            float* const xrot = const_cast<float*>(grp.m[i].xrot);
+            if (items[i].n_planes == 2) launch_rotate_x_pair(x, xrot, items[i].in, batch, items[i].block, items[i].seed_p, items[i].seed_r, stream);
+            else launch_rotate_x(x, xrot, items[i].in, batch, items[i].block, 1, items[i].seed_p, items[i].seed_r, stream);
+        }
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1224,9 +1336,13 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     cfg.numAttrs = 1;
     const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));
     const bool multi = grp.m[0].n_slots > 1;   // the same for all: same in_features and planes
-#define TQ_GROUP_LAUNCH(BPV)                                                              \
-    if (multi) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_group_kernel<BPV, true>, grp)); \
-    else TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_group_kernel<BPV, false>, grp));
+    const bool dual = items[0].n_planes == 2;
+#define TQ_GROUP_LAUNCH2(BPV, DV)                                                             \
+    if (multi) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_group_kernel<BPV, true, DV>, grp)); \
+    else TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_group_kernel<BPV, false, DV>, grp));
+#define TQ_GROUP_LAUNCH(BPV)                    \
+    if (dual) { TQ_GROUP_LAUNCH2(BPV, true) } \
+    else { TQ_GROUP_LAUNCH2(BPV, false) }
     switch (bp) {
         case 1: TQ_GROUP_LAUNCH(1) break;
         case 2: TQ_GROUP_LAUNCH(2) break;
@@ -1234,6 +1350,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
         default: TQ_GROUP_LAUNCH(8) break;
     }
 #undef TQ_GROUP_LAUNCH
+#undef TQ_GROUP_LAUNCH2
 }
 
 // The activation rotation alone (the pre-kernel of several rows or WHT blocks above 256 columns), also for the other decode
@@ -1270,6 +1387,17 @@ void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t b
 #undef TQ_ROT_CASE
 }
 
+// The same for weights with two rotations: pairs of fp16 and their scales (see rotate_x_pair_kernel), in the room of
+// launch_rotate_x's two planes.
+static void launch_rotate_x_pair(const __half* x, float* xrot, int in, int batch, uint32_t block, uint32_t seed_p, uint32_t seed_r,
+                                 cudaStream_t stream) {
+    const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
+    auto* const kernel = wide_cols == 256 ? rotate_x_pair_kernel<1> : (wide_cols == 512 ? rotate_x_pair_kernel<2> : rotate_x_pair_kernel<4>);
+    launch_pdl(kernel, dim3((batch * ((in + wide_cols - 1) / wide_cols) + 3) / 4), dim3(128), kRotateXSmem, stream, x,
+               reinterpret_cast<uint32_t*>(xrot), xrot + static_cast<size_t>(8) * in, in, batch, static_cast<int>(block), seed_p, seed_r,
+               1.0f / std::sqrt(static_cast<float>(block)), reinterpret_cast<uintptr_t>(x) % 16 == 0 ? 1 : 0);
+}
+
 // ---- allocation-free variant ---------------------------------------------------------------
 // Same two kernels, but the scratch (rotated activation, split-K partial sums, arrival
 // counters) lives in a fixed array inside the library image instead of a buffer the handle
@@ -1298,11 +1426,13 @@ static void* static_scratch_address() {
 void* gemv_static_scratch_address() { return static_scratch_address(); }
 
 void launch_tq8_gemv_static(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
-                            int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
-                            unsigned int* status, int sm_count, cudaStream_t stream) {
-    const size_t need = gemv_scratch_bytes(out, in, n_planes);
-    if (need > kStaticScratchBytes)
-        throw Error("allocation-free forward: this layer needs " + std::to_string(need) +
+                            int out, int in, int batch, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p,
+                            uint32_t seed_r, unsigned int* status, int sm_count, cudaStream_t stream) {
+    // Which layers are taken: those whose planes would fit as partial-sum slots of their own (layers with two rotations need
+    // less than that).
+    const size_t asked = scratch_bytes(out, in, n_planes, chunk_count(in) * n_planes), need = gemv_scratch_bytes(out, in, n_planes);
+    if (asked > kStaticScratchBytes)
+        throw Error("allocation-free forward: this layer needs " + std::to_string(asked) +
                     " bytes of scratch, the built-in array holds " + std::to_string(kStaticScratchBytes));
     void* scratch = static_scratch_address();
     // The array is shared by every call and keeps what the last one left.  The arrival
@@ -1315,7 +1445,7 @@ void launch_tq8_gemv_static(const uint8_t* codes, const float* norms, const floa
         const size_t counter_bytes = align256(static_cast<size_t>(n_row_tiles) * kWarps * sizeof(unsigned int));
         TQ_CUDA(cudaMemsetAsync(static_cast<uint8_t*>(scratch) + need - counter_bytes, 0, counter_bytes, stream));
     }
-    launch_tq8_gemv(codes, norms, table, x, y, out, in, batch, block, n_planes, seed_p, seed_r, scratch, status, sm_count,
+    launch_tq8_gemv(codes, norms, table, x, y, out, in, batch, block, n_planes, pair_unit, seed_p, seed_r, scratch, status, sm_count,
                     stream);
 }
 

@@ -27,15 +27,16 @@ void launch_dequant_f32(const uint8_t* joint, const float* norms, const float* t
 void launch_dequant_f16(const uint8_t* joint, const float* norms, const float* tables, __half* out, long rows, int in,
                         uint32_t block, uint32_t seed_p, uint32_t seed_r, bool dual, cudaStream_t stream);
 
-// tq_gemv.cu — fused dequantise + GEMV, 1..8 activation rows.  table: [n_planes, 256] fp32
-// (one plane for shared rotation / primary only, two for dual rotation).
+// tq_gemv.cu — fused dequantise + GEMV, 1..8 activation rows.  table: 256 fp32 (shared rotation / primary only), or for
+// dual rotation 2 x 256 fp32 and then 256 words that hold a primary and a residual entry each, as fp16 divided by pair_unit
+// (a power of two).
 // scratch: gemv_scratch_bytes(out, in) bytes, zero-initialised once (the kernel leaves
 // its counters at zero); may be NULL when that size is 0.  status: one device word,
 // set non-zero by the kernel if its shared-memory layout assumption does not hold.
 size_t gemv_scratch_bytes(int out, int in, int n_planes);
 void launch_tq8_gemv(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
-                     int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
-                     void* scratch, unsigned int* status, int sm_count, cudaStream_t stream);
+                     int out, int in, int batch, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p,
+                     uint32_t seed_r, void* scratch, unsigned int* status, int sm_count, cudaStream_t stream);
 
 // The same with the fp16 result written to n_dst (1..8) buffers at once: destination d receives
 // activation row n, output row r at dst[d][n * dst_stride + r].  Destinations may be other GPUs'
@@ -56,7 +57,7 @@ struct GemvGather {
 };
 void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const float* table, const __half* x,
                              __half* const* dst, int n_dst, long dst_stride, int out, int in, int batch, uint32_t block,
-                             int n_planes, uint32_t seed_p, uint32_t seed_r, void* scratch, unsigned int* status,
+                             int n_planes, float pair_unit, uint32_t seed_p, uint32_t seed_r, void* scratch, unsigned int* status,
                              int sm_count, cudaStream_t stream, unsigned int* const* signal = nullptr, int signal_slot = 0,
                              unsigned int signal_value = 0, unsigned int* done_counter = nullptr,
                              const GemvGather* gather = nullptr, int n_signal = 0);
@@ -71,6 +72,7 @@ struct GemvGroupItem {
     int out, in;
     uint32_t block;
     int n_planes;
+    float pair_unit;
     uint32_t seed_p, seed_r;
     void* scratch;
     unsigned int* status;
@@ -106,8 +108,8 @@ void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t b
 // (gemv_static_scratch_capacity() bytes); throws if the layer needs more.
 size_t gemv_static_scratch_capacity();
 void launch_tq8_gemv_static(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
-                            int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
-                            unsigned int* status, int sm_count, cudaStream_t stream);
+                            int out, int in, int batch, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p,
+                            uint32_t seed_r, unsigned int* status, int sm_count, cudaStream_t stream);
 
 // tq_gemm.cu — fused dequantise + GEMM on tcgen05 / tensor memory for many activation rows
 // (prefill).  x: [m, in] fp16, y: [m, out] fp16.  scratch: gemm_scratch_bytes(...) bytes (the
