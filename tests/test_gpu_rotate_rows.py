@@ -1,0 +1,46 @@
+"""The activation rotation of the many-row linear at the edges of its tiles: blocks of 32 to 512 columns (and 1024, which has a
+kernel of its own), a last group of columns that is not full, rows around the groups of 8 and 32, several steps per CTA.
+Tolerance as in test_gpu_gemm_edges: three roundings to fp16, root mean square below 4.9e-4; a row on its own may reach 1.5 of that."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_in,block,shared", [
+    (64, 32, True), (192, 64, False), (320, 64, True), (3584, 128, True), (384, 128, False), (768, 256, True), (1536, 512, False),
+    (512, 512, True), (2048, 1024, False),
+])
+@pytest.mark.parametrize("rows", [9, 31, 33, 257])
+def test_rotation_of_many_rows(tq, n_in, block, shared, rows):
+    check(tq, n_in, block, shared, rows)
+
+
+@pytest.mark.parametrize("n_in,block,rows", [(8192, 64, 1300), (16384, 128, 2050), (16384, 512, 2077)])
+def test_rotation_with_several_steps(tq, n_in, block, rows):
+    check(tq, n_in, block, True, rows)
+
+
+def check(tq, n_in, block, shared, rows):
+    torch = pytest.importorskip("torch")
+    n_out = 144
+    g = torch.Generator(device="cuda").manual_seed(n_in + block + rows)
+    w = torch.randn((n_out, n_in), generator=g, device="cuda") * 0.02
+    c = tq.generate_codebook(4)
+    layers = []
+    for _ in range(2):
+        qw = tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, block, shared))
+        layers.append(tq.TurboQuantLinear(n_in, n_out, qw, c, c, block))
+        w = torch.randn((n_out, n_in), generator=g, device="cuda") * 0.02
+    x = torch.randn((rows, n_in), generator=g, device="cuda").half()
+    alone = [lin.forward(x) for lin in layers]
+    for lin, y in zip(layers, alone):
+        back = torch.empty((n_out, n_in), device="cuda")
+        lin.dequantize(out=back)
+        want = x.double() @ back.double().T
+        err = (y.double() - want).norm(dim=1) / want.norm(dim=1)
+        assert float(err.square().mean().sqrt()) < 4.9e-4
+        assert float(err.max()) < 1.5 * 4.9e-4
+        lin.check_status()
+    for y, got in zip(alone, tq.forward_group(layers, x)):
+        assert torch.equal(y, got)
