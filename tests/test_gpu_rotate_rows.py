@@ -44,3 +44,28 @@ def check(tq, n_in, block, shared, rows):
         lin.check_status()
     for y, got in zip(alone, tq.forward_group(layers, x)):
         assert torch.equal(y, got)
+
+
+@pytest.mark.parametrize("n_in,n_out,rows,stride", [
+    (3584, 1024, 64, 0), (4096, 130, 40, 0), (4096, 126, 9, 0), (2048, 128, 300, 0),   # rows of four outputs, and not
+    (4096, 128, 17, 131), (4096, 128, 17, 136),                                        # rows of a wider buffer
+    (8192, 16, 65, 0),                                                                 # more than eight splits
+])
+def test_sums_over_the_splits_of_k(tq, n_in, n_out, rows, stride):
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(n_in + n_out + rows)
+    w = torch.randn((n_out, n_in), generator=g, device="cuda") * 0.02
+    c = tq.generate_codebook(4)
+    lin = tq.TurboQuantLinear(n_in, n_out, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, 128, True)), c, c, 128)
+    back = torch.empty((n_out, n_in), device="cuda")
+    lin.dequantize(out=back)
+    x = torch.randn((rows, n_in), generator=g, device="cuda").half()
+    y = lin.forward(x)
+    want = x.double() @ back.double().T
+    assert float((y.double() - want).norm() / want.norm()) < 4.9e-4
+    if stride:
+        wide = torch.full((rows, stride), 7.0, device="cuda", dtype=torch.float16)
+        lin.forward_strided(x, wide.data_ptr() + 2 * 3, stride)
+        torch.cuda.synchronize()
+        assert torch.equal(wide[:, 3:3 + n_out], y) and bool((wide[:, :3] == 7).all()) and bool((wide[:, 3 + n_out:] == 7).all())
+    lin.check_status()
