@@ -45,3 +45,39 @@ def test_crowded_samples_are_fitted_in_passes_over_all(tq, oracle, n, share):
     got, again = (tq.generate_codebook_from_data(x, 4, 20) for _ in range(2))
     assert np.all(np.abs(got.centroids - want) <= 3e-6 * np.abs(want) + 3e-7)
     assert np.array_equal(got.centroids.view(np.uint32), again.centroids.view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["normal", "wide", "small", "one sign", "two magnitudes"])
+def test_fit_counts_outside_of_the_window(tq, oracle, kind):
+    """From 2 M samples on the counters on the SM hold 48 exponents: samples below them, of one sign, and nowhere near the codebook."""
+    n = 2_200_003
+    rng = np.random.default_rng(7)
+    x = rng.standard_normal(n)
+    if kind == "wide":
+        x = x * 10.0 ** rng.uniform(-30, 30, n)
+    elif kind == "small":
+        x = x * 1e-39                       # subnormal numbers
+    elif kind == "one sign":
+        x = -np.abs(x)
+    elif kind == "two magnitudes":
+        x[: n // 2] *= 1e-20
+        rng.shuffle(x)
+    x = x.astype(np.float32)
+    want, _ = oracle.fit_codebook(x, 4, 3)
+    got, again = (tq.generate_codebook_from_data(x, 4, 3) for _ in range(2))
+    assert np.all(np.abs(got.centroids - want) <= 3e-6 * np.abs(want) + 3e-7)
+    assert np.array_equal(got.centroids.view(np.uint32), again.centroids.view(np.uint32))
+
+
+@pytest.mark.parametrize("rows,cols,block", [(40, 64, 64), (300, 512, 512), (1024, 2048, 128)])
+def test_layer_fits_side_by_side(tq, rows, cols, block):
+    """The two fits of a layer in one launch: each as it is alone."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = torch.randn((rows, cols), generator=g, device="cuda") * 0.02
+    both = tq.fit_layer_codebooks(w, block, 4, 3, 40)
+    alone, _ = tq.fit_layer_codebooks(w, block, 4, 0, 40)
+    assert np.array_equal(both[0].centroids.view(np.uint32), alone.centroids.view(np.uint32))
+    host = tq.fit_layer_codebooks(w.cpu().numpy(), block, 4, 3, 40)
+    assert all(np.array_equal(a.centroids.view(np.uint32), b.centroids.view(np.uint32)) for a, b in zip(both, host))
+    assert both[1].centroids.size == 8 and np.all(np.diff(both[1].centroids) > 0)

@@ -190,7 +190,7 @@ int tq_codebook_fit(const float* data, long n, int bits, int iterations, float* 
         auto st = static_cast<cudaStream_t>(stream);
         DeviceBuffer stage;
         const float* d_data = n ? device_view(data, static_cast<size_t>(n), stage, st) : nullptr;
-        const int run = launch_codebook_fit(d_data, n, bits, iterations, c0, centroids, boundaries, st);
+        const int run = launch_codebook_fit(FitRequest{d_data, n, bits, iterations, c0, centroids, boundaries}, st);
         if (iterations_run) *iterations_run = run;
         return 0;
     });
@@ -221,11 +221,11 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
         launch_row_norms(d_w, norms.as<float>(), out_features, in_features, st);
         launch_layer_samples(d_w, norms.as<float>(), out_features, in_features, block, seed_p, cp0, 1 << primary_bits,
                              scaled.as<float>(), need_residual ? resid.as<float>() : nullptr, st);
-        launch_codebook_fit(scaled.as<float>(), static_cast<long>(n), primary_bits, iterations, cp0, primary_centroids,
-                            primary_boundaries, st);
+        const FitRequest primary{scaled.as<float>(), static_cast<long>(n), primary_bits, iterations, cp0, primary_centroids, primary_boundaries};
         if (need_residual)
-            launch_codebook_fit(resid.as<float>(), static_cast<long>(n), residual_bits, iterations, cr0, residual_centroids,
-                                residual_boundaries, st);
+            launch_codebook_fits(primary, FitRequest{resid.as<float>(), static_cast<long>(n), residual_bits, iterations, cr0, residual_centroids, residual_boundaries}, st);
+        else
+            launch_codebook_fit(primary, st);
         TQ_CUDA(cudaStreamSynchronize(st));
         for (DeviceBuffer* b : {&w_stage, &norms, &scaled, &resid}) b->set_idle();
         return 0;

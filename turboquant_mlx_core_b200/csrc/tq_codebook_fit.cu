@@ -5,11 +5,11 @@
 // that took 110 us per iteration at 16.8 M samples, a hundred times.  Instead the samples are bucketed ONCE by the leading
 // bits of their order-preserving key (sign, exponent, a few mantissa bits), with running counts and a sum per bucket; a
 // boundary then only looks at the values of its own bucket, and all iterations run in one launch of one CTA, a warp per
-// boundary and bin (about 1 us each).
+// boundary and bin (3 to 6 us each).
 //   fit_look_kernel       whether the samples repeat themselves (then as below)
-//   fit_count_kernel      bucket counts, largest magnitude            (one pass over the samples)
+//   fit_count_window_kernel    bucket counts, largest magnitude       (one pass over the samples; fit_count_kernel for few of them)
 //   fit_groups / fit_offsets   exclusive scan of the counts, 256 buckets per group
-//   fit_scatter_kernel    samples into their buckets                  (one pass)
+//   fit_scatter_window_kernel  samples into their buckets             (one pass; fit_scatter_kernel)
 //   fit_sums_kernel       sum of every bucket
 //   fit_iterate_kernel    the iterations
 // A value equal to a boundary goes to the lower bin, as std::lower_bound in the reference's CPU path and quantize() have
@@ -49,6 +49,7 @@ struct FitState {
     int iterations_run;
     int go_over_all;                 // fit_iterate_kernel stopped: the remaining iterations go over all samples
     unsigned int max_bits;           // bits of the largest magnitude
+    int window_low;                  // lowest exponent of the window (fit_count_window_kernel)
 };
 
 constexpr int kFitGroup = 256;              // buckets of a group
@@ -81,19 +82,116 @@ __device__ __forceinline__ FitBucket fit_bucket(int bucket, int shift) {
 // samples took 55 ms, half of them zero 39 ms, where the passes over all samples take 1 and 11), and the iterations stop
 // at such a bucket anyway.  One CTA looks at kFitLooked samples, evenly spread: where one bucket must hold more than
 // kFitCrowd, the kernels after it return at once.  (kFitSlots counters: two buckets that share one need twice the luck.)
-__global__ void __launch_bounds__(1024) fit_look_kernel(const float* __restrict__ data, unsigned int n, int shift, FitState* __restrict__ state) {
-    __shared__ unsigned int s_count[kFitSlots];
+// It also chooses the window of the two kernels behind it: `window` exponents down from the largest one of which it sees two samples.
+__global__ void __launch_bounds__(1024) fit_look_kernel(const float* __restrict__ data, unsigned int n, int shift, int window, FitState* __restrict__ state) {
+    __shared__ unsigned int s_count[kFitSlots], s_exp[256];
     for (int i = threadIdx.x; i < kFitSlots; i += 1024) s_count[i] = 0u;
+    if (threadIdx.x < 256) s_exp[threadIdx.x] = 0u;
     __syncthreads();
     unsigned int most = 0;
     const unsigned int step = n / kFitLooked;
 #pragma unroll
     for (int k = 0; k < kFitLooked / 1024; ++k) {
-        const unsigned int bucket = fit_key(__ldg(data + static_cast<size_t>(k * 1024 + threadIdx.x) * step)) >> shift;
+        const float x = __ldg(data + static_cast<size_t>(k * 1024 + threadIdx.x) * step);
+        const unsigned int bucket = fit_key(x) >> shift;
+        atomicAdd(&s_exp[(__float_as_uint(x) >> 23) & 0xffu], 1u);
         most = max(most, atomicAdd(&s_count[bucket % kFitSlots], 1u) + 1u);
     }
     most = __reduce_max_sync(0xffffffffu, most);
     if ((threadIdx.x & 31) == 0 && most >= 16u && static_cast<unsigned long long>(most) * step > kFitCrowd) state->go_over_all = 1;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int top = -1;
+        for (int e = threadIdx.x; e < 256; e += 32)
+            if (s_exp[e] >= 2u) top = e;
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (threadIdx.x == 0) state->window_low = max(0, min(top, 254) - window + 1);
+    }
+}
+
+// Counting and scattering with most of the counters on the SM.  An atomic addition in L2 for every sample took 250 to 420 us per
+// pass over 16.8 M of them (the scatter waits for its answer), of which reading them is 10.  A CTA per SM keeps counters for
+// the buckets of a window, 2^(shift - 23) .. of `window` exponents and both signs (all but 0.1 % of normal samples), and
+// adds a bucket's count up in L2 once; what that addition returns is where the CTA's samples of the bucket begin, so
+// the scatter, which deals the samples to CTAs in the same way, needs no other word from the CTAs around it.  Samples outside of
+// the window are counted in L2.
+constexpr int kWindowSlots = 49152;           // counters of a CTA: 192 KB
+constexpr unsigned int kWindowTile = 8192;    // samples that a CTA takes at a time
+// Used wherever the samples are looked at first (from kFitCrowd on): 262144 / 1 M / 4.2 M / 16.8 M normal samples are counted in
+// 5 / 8 / 14 / 40 us (37 / 104 / 135 / 186 in L2) and scattered in 9 / 13 / 30 / 142 (39 / 113 / 143 / 299).
+struct FitWindow {
+    unsigned int low, slots;   // magnitudes (shifted) from `low` on, `slots` of them, of either sign
+    int shift;
+    __device__ __forceinline__ FitWindow(const FitState* state, int shift_, int window)
+        : low(static_cast<unsigned int>(state->window_low) << (23 - shift_)), slots(static_cast<unsigned int>(window) << (23 - shift_)), shift(shift_) {}
+    // The slot of a sample, or 0xffffffff.
+    __device__ __forceinline__ unsigned int slot(float x) const {
+        const unsigned int u = __float_as_uint(x), m = ((u & 0x7fffffffu) >> shift) - low;
+        return m < slots ? m + ((u >> 31) ? slots : 0u) : 0xffffffffu;
+    }
+    __device__ __forceinline__ unsigned int bucket(unsigned int slot) const {
+        const bool negative = slot >= slots;
+        const unsigned int m = (negative ? slot - slots : slot) + low + (0x80000000u >> shift);
+        return negative ? (0xffffffffu >> shift) - m : m;
+    }
+};
+__global__ void __launch_bounds__(1024) fit_count_window_kernel(const float* __restrict__ data, unsigned int n, int shift, int window,
+                                                                unsigned int* __restrict__ count, unsigned int* __restrict__ begin, FitState* __restrict__ state) {
+    if (state->go_over_all) return;
+    extern __shared__ unsigned int s_counter[];
+    const FitWindow w(state, shift, window);
+    for (unsigned int i = threadIdx.x; i < 2 * w.slots; i += 1024) s_counter[i] = 0u;
+    __syncthreads();
+    unsigned int top = 0;
+    for (unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * kWindowTile; i0 < n; i0 += static_cast<unsigned long long>(gridDim.x) * kWindowTile) {
+        float x[kWindowTile / 1024];
+        const unsigned int i = static_cast<unsigned int>(i0) + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < static_cast<int>(kWindowTile / 1024); ++k)
+            if (i + 1024u * k < n) x[k] = __ldcs(data + i + 1024u * k);
+#pragma unroll
+        for (int k = 0; k < static_cast<int>(kWindowTile / 1024); ++k)
+            if (i + 1024u * k < n) {
+                top = max(top, __float_as_uint(x[k]) & 0x7fffffffu);
+                const unsigned int slot = w.slot(x[k]);
+                if (slot != 0xffffffffu) atomicAdd(&s_counter[slot], 1u);
+                else atomicAdd(&count[fit_key(x[k]) >> shift], 1u);
+            }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) atomicMax(&state->max_bits, top);
+    __syncthreads();
+    unsigned int* const mine = begin + static_cast<size_t>(blockIdx.x) * 2 * w.slots;
+#pragma unroll 4
+    for (unsigned int i = threadIdx.x; i < 2 * w.slots; i += 1024) {
+        const unsigned int c = s_counter[i];
+        if (c != 0u) mine[i] = atomicAdd(&count[w.bucket(i)], c);
+    }
+}
+__global__ void __launch_bounds__(1024) fit_scatter_window_kernel(const float* __restrict__ data, unsigned int n, int shift, int window,
+                                                                  const unsigned int* __restrict__ offset, const unsigned int* __restrict__ begin,
+                                                                  unsigned int* __restrict__ cursor, float* __restrict__ sorted,
+                                                                  const FitState* __restrict__ state) {
+    if (state->go_over_all) return;
+    extern __shared__ unsigned int s_counter[];
+    const FitWindow w(state, shift, window);
+    const unsigned int* const mine = begin + static_cast<size_t>(blockIdx.x) * 2 * w.slots;   // (not set where the CTA has no sample)
+#pragma unroll 4
+    for (unsigned int i = threadIdx.x; i < 2 * w.slots; i += 1024) s_counter[i] = mine[i] + offset[w.bucket(i)];
+    __syncthreads();
+    for (unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * kWindowTile; i0 < n; i0 += static_cast<unsigned long long>(gridDim.x) * kWindowTile) {
+        float x[kWindowTile / 1024];
+        const unsigned int i = static_cast<unsigned int>(i0) + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < static_cast<int>(kWindowTile / 1024); ++k)
+            if (i + 1024u * k < n) x[k] = __ldcs(data + i + 1024u * k);
+#pragma unroll
+        for (int k = 0; k < static_cast<int>(kWindowTile / 1024); ++k)
+            if (i + 1024u * k < n) {
+                const unsigned int slot = w.slot(x[k]);
+                sorted[atomicAdd(slot != 0xffffffffu ? &s_counter[slot] : &cursor[fit_key(x[k]) >> shift], 1u)] = x[k];
+            }
+    }
 }
 
 __global__ void __launch_bounds__(256) fit_count_kernel(const float* __restrict__ data, unsigned int n, int shift, unsigned int* __restrict__ count,
@@ -207,13 +305,33 @@ __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__
         part[blockIdx.x] = total;
     }
 }
-// All iterations: warp w follows boundary w, the upper one of bin w.  Bound by the latency of a chain of L2 reads and
-// reductions in one CTA, and by issue: 100 iterations over 16.8 M samples take 385 us.  (Significands as 64-bit sums of doubles'
-// conversions took 400 to 660 us; the bits below a bucket's prefix are 32-bit sums.)  `group_sum`: filled here from the parts.
-__global__ void __launch_bounds__(1024) fit_iterate_kernel(const float* __restrict__ sorted, unsigned int n, const unsigned int* __restrict__ count,
-                                                           const unsigned int* __restrict__ offset, const double* __restrict__ sum,
-                                                           const double* __restrict__ part, int n_groups, double* __restrict__ group_sum,
-                                                           int shift, int iterations, FitState* __restrict__ state) {
+// All iterations of a fit in one CTA, a CTA per fit: warp w follows boundary w, the upper one of bin w.  Bound by the latency of a
+// chain of L2 reads, reductions and barriers: 100 iterations over 16.8 M samples take 340 to 600 us, those of a layer's two
+// fits, side by side, 570 (one after the other 890).  (Significands as 64-bit sums of doubles' conversions took 400 to 660 us; the bits
+// below a bucket's prefix are 32-bit sums.  Two warps per boundary that keep their bucket's samples in registers: no change.)
+// `group_sum`: filled here from the parts.
+struct FitJob {
+    const float* sorted;
+    const unsigned int *count, *offset;
+    const double *sum, *part;
+    double* group_sum;
+    FitState* state;
+    unsigned int n;
+    int n_groups, shift, iterations;
+};
+constexpr int kFitJobs = 2;
+struct FitJobs {
+    FitJob job[kFitJobs];
+};
+__global__ void __launch_bounds__(1024) fit_iterate_kernel(const __grid_constant__ FitJobs jobs) {
+    const FitJob& f = jobs.job[blockIdx.x];
+    const float* __restrict__ sorted = f.sorted;
+    const unsigned int *__restrict__ count = f.count, *__restrict__ offset = f.offset;
+    const double *__restrict__ sum = f.sum, *__restrict__ part = f.part;
+    double* __restrict__ group_sum = f.group_sum;
+    FitState* __restrict__ state = f.state;
+    const unsigned int n = f.n;
+    const int n_groups = f.n_groups, shift = f.shift, iterations = f.iterations;
     __shared__ float s_c[kFitMaxBins], s_b[kFitMaxBins];
     // Per boundary: its bucket, that bucket's unit and sum, the sums of its group's buckets before and after it; the samples up
     // to the boundary, those before the bucket included, and the significands of the ones in the bucket.
@@ -517,100 +635,180 @@ __global__ void __launch_bounds__(128) layer_samples_kernel(const float* __restr
 
 }  // namespace
 
-// Fits `bits`-bit centroids to d_data[n] starting from init_centroids (2^bits values, ascending).
-// centroids_out / boundaries_out: host arrays of 2^bits and 2^bits - 1 floats.  Returns the iterations run.
-int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, const float* init_centroids, float* centroids_out,
-                        float* boundaries_out, cudaStream_t stream) {
-    TQ_REQUIRE(bits >= 1 && bits <= 5, "Unsupported bit width; must be 1-5");
-    const int nc = 1 << bits;
-    FitState h{};
-    h.n = nc;
-    for (int i = 0; i < nc; ++i) h.centroids[i] = init_centroids[i];
-    for (int i = 0; i + 1 < nc; ++i) h.boundaries[i] = (init_centroids[i] + init_centroids[i + 1]) * 0.5f;
-    int run = 0;
-    if (n > 0 && iterations > 0) {
-        int dev = 0, sms = 148;
-        TQ_CUDA(cudaGetDevice(&dev));
-        TQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        TQ_REQUIRE(n < (1L << 40), "tq_codebook_fit: at most 2^40 samples");
-        DeviceBuffer state_buf;
-        state_buf.reserve(sizeof(FitState), stream);
-        FitState* const d_state = state_buf.as<FitState>();
-        TQ_CUDA(cudaMemcpyAsync(d_state, &h, sizeof h, cudaMemcpyHostToDevice, stream));
-        auto read_state = [&] {
-            TQ_CUDA(cudaMemcpyAsync(&h, d_state, sizeof h, cudaMemcpyDeviceToHost, stream));
-            TQ_CUDA(cudaStreamSynchronize(stream));
-        };
-        h.go_over_all = 1;
-        DeviceBuffer bucket_buf, sorted_buf;
+namespace {
+
+// One fit on its way: what is queued on the stream, and the memory that it uses.
+class FitRun {
+public:
+    FitRun(const FitRequest& r, cudaStream_t stream) : r_(r), stream_(stream), nc_(1 << r.bits) {
+        TQ_REQUIRE(r.bits >= 1 && r.bits <= 5, "Unsupported bit width; must be 1-5");
+        h_.n = nc_;
+        for (int i = 0; i < nc_; ++i) h_.centroids[i] = r.init_centroids[i];
+        for (int i = 0; i + 1 < nc_; ++i) h_.boundaries[i] = (r.init_centroids[i] + r.init_centroids[i + 1]) * 0.5f;
+        active_ = r.n > 0 && r.iterations > 0;
+        if (!active_) return;
+        TQ_CUDA(cudaGetDevice(&dev_));
+        sms_ = sm_count(dev_);
+        TQ_REQUIRE(r.n < (1L << 40), "tq_codebook_fit: at most 2^40 samples");
+        state_buf_.reserve(sizeof(FitState), stream);
+        TQ_CUDA(cudaMemcpyAsync(state(), &h_, sizeof h_, cudaMemcpyHostToDevice, stream));
+        h_.go_over_all = 1;
         // Mantissa bits of a bucket's key: a few hundred values in the buckets where boundaries lie (16.8 M normal samples:
         // 11 bits, about 600), between 2^12 and 2^21 buckets.
         int log2_n = 0;
-        while ((1L << log2_n) < n) ++log2_n;
-        const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13)), shift = 32 - key_bits, n_buckets = 1 << key_bits;
-        const int n_groups = n_buckets / kFitGroup, n_parts = n_buckets / kFitSumBuckets;
-        bool bucketed = n < (1L << 31);
-        if (bucketed) {
+        while ((1L << log2_n) < r.n) ++log2_n;
+        const int key_bits = 9 + std::min(12, std::max(3, log2_n - 13));
+        shift_ = 32 - key_bits;
+        n_buckets_ = 1 << key_bits;
+        n_groups_ = n_buckets_ / kFitGroup;
+        const int n_parts = n_buckets_ / kFitSumBuckets;
+        bucketed_ = r.n < (1L << 31);
+        if (bucketed_) {
             try {
-                bucket_buf.reserve(static_cast<size_t>(n_buckets) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups) * 8 + static_cast<size_t>(n_groups) * 4, stream);
-                sorted_buf.reserve(static_cast<size_t>(n) * 4, stream);
+                bucket_buf_.reserve(static_cast<size_t>(n_buckets_) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups_) * 8 + static_cast<size_t>(n_groups_) * 4, stream);
+                sorted_buf_.reserve(static_cast<size_t>(r.n) * 4, stream);
             } catch (const OutOfMemory&) {
-                bucketed = false;   // the passes over all samples need next to nothing
+                bucketed_ = false;   // the passes over all samples need next to nothing
             }
         }
-        if (bucketed) {
-            double* const d_sum = bucket_buf.as<double>();
-            double* const d_part = d_sum + n_buckets;
-            double* const d_group_sum = d_part + n_parts;
-            unsigned int* const d_count = reinterpret_cast<unsigned int*>(d_group_sum + n_groups);
-            unsigned int* const d_offset = d_count + n_buckets;
-            unsigned int* const d_cursor = d_offset + n_buckets;
-            unsigned int* const d_group = d_cursor + n_buckets;
-            float* const d_sorted = sorted_buf.as<float>();
-            TQ_CUDA(cudaMemsetAsync(d_count, 0, static_cast<size_t>(n_buckets) * 4, stream));
-            const unsigned int un = static_cast<unsigned int>(n);
-            const int grid = static_cast<int>(std::min<long>((n + 1023) / 1024, 16L * sms));
-            if (un >= kFitCrowd) fit_look_kernel<<<1, 1024, 0, stream>>>(d_data, un, shift, d_state);
-            fit_count_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_count, d_state);
-            fit_groups_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group);
-            fit_offsets_kernel<<<n_groups, 256, 0, stream>>>(d_count, d_group, d_offset, d_cursor);
-            fit_scatter_kernel<<<grid, 256, 0, stream>>>(d_data, un, shift, d_cursor, d_sorted, d_state);
-            fit_sums_kernel<<<n_parts, 256, 0, stream>>>(d_sorted, d_count, d_offset, shift, d_sum, d_part, d_state);
-            fit_iterate_kernel<<<1, 1024, 0, stream>>>(d_sorted, un, d_count, d_offset, d_sum, d_part, n_groups, d_group_sum, shift, iterations, d_state);
-            TQ_CUDA(cudaGetLastError());
-            read_state();
-        }
-        if (h.go_over_all && !h.converged && h.iterations_run < iterations) {
-            const long chunks = (n + (1L << 14) - 1) >> 14;
-            const int blocks = static_cast<int>(std::min<long>(chunks, 2L * sms));
-            const size_t smem = (sizeof(double) + sizeof(unsigned int)) * kFitMaxBins * kFitThreads;
-            static bool configured[64] = {false};
-            if (dev < 0 || dev >= 64 || !configured[dev]) {
-                TQ_CUDA(cudaFuncSetAttribute(fit_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-                if (dev >= 0 && dev < 64) configured[dev] = true;
+        // exponents of the window; without memory for the CTAs' places all counters are in L2
+        window_ = std::min(254, kWindowSlots >> (24 - shift_));
+        windowed_ = bucketed_ && r.n >= static_cast<long>(kFitCrowd);
+        if (windowed_) {
+            try {
+                begin_buf_.reserve(window_bytes() * sms_, stream);
+            } catch (const OutOfMemory&) {
+                windowed_ = false;
             }
-            DeviceBuffer part_buf;
-            part_buf.reserve((sizeof(double) + sizeof(unsigned long long)) * kFitMaxBins * blocks, stream);
-            double* const d_psum = part_buf.as<double>();
-            unsigned long long* const d_pcnt = reinterpret_cast<unsigned long long*>(d_psum + kFitMaxBins * blocks);
-            // all pairs of launches are enqueued at once; those after convergence return at their first instruction
-            for (int it = h.iterations_run; it < iterations; ++it) {
-                fit_partial_kernel<<<blocks, kFitThreads, smem, stream>>>(d_data, n, d_state, d_psum, d_pcnt);
-                fit_update_kernel<<<1, 32, 0, stream>>>(d_state, d_psum, d_pcnt, blocks);
-            }
-            TQ_CUDA(cudaGetLastError());
-            read_state();
-            part_buf.set_idle();
         }
-        state_buf.set_idle();
-        bucket_buf.set_idle();
-        sorted_buf.set_idle();
-        run = h.iterations_run;
     }
-    for (int i = 0; i < nc; ++i) centroids_out[i] = h.centroids[i];
-    if (boundaries_out)
-        for (int i = 0; i + 1 < nc; ++i) boundaries_out[i] = (h.centroids[i] + h.centroids[i + 1]) * 0.5f;   // src/codebook.cpp:135-139
-    return run;
+    bool short_of_memory() const { return active_ && (!bucketed_ || (!windowed_ && r_.n >= static_cast<long>(kFitCrowd))) && r_.n < (1L << 31); }
+
+    // Queues what comes before the iterations; fills in the job and returns true where there are buckets to iterate on.
+    bool enqueue_buckets(FitJob& job) {
+        if (!active_ || !bucketed_) return false;
+        const int n_parts = n_buckets_ / kFitSumBuckets;
+        double* const d_sum = bucket_buf_.as<double>();
+        double* const d_part = d_sum + n_buckets_;
+        double* const d_group_sum = d_part + n_parts;
+        unsigned int* const d_count = reinterpret_cast<unsigned int*>(d_group_sum + n_groups_);
+        unsigned int* const d_offset = d_count + n_buckets_;
+        unsigned int* const d_cursor = d_offset + n_buckets_;
+        unsigned int* const d_group = d_cursor + n_buckets_;
+        float* const d_sorted = sorted_buf_.as<float>();
+        const unsigned int un = static_cast<unsigned int>(r_.n);
+        const int grid = static_cast<int>(std::min<long>((r_.n + 1023) / 1024, 16L * sms_));
+        TQ_CUDA(cudaMemsetAsync(d_count, 0, static_cast<size_t>(n_buckets_) * 4, stream_));
+        if (windowed_) {
+            static bool configured[64] = {false};
+            if (dev_ < 0 || dev_ >= 64 || !configured[dev_]) {
+                TQ_CUDA(cudaFuncSetAttribute(fit_count_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowSlots * 4));
+                TQ_CUDA(cudaFuncSetAttribute(fit_scatter_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindowSlots * 4));
+                if (dev_ >= 0 && dev_ < 64) configured[dev_] = true;
+            }
+        }
+        if (un >= kFitCrowd) fit_look_kernel<<<1, 1024, 0, stream_>>>(r_.data, un, shift_, window_, state());
+        unsigned int* const d_begin = begin_buf_.as<unsigned int>();
+        if (windowed_) fit_count_window_kernel<<<sms_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_count, d_begin, state());
+        else fit_count_kernel<<<grid, 256, 0, stream_>>>(r_.data, un, shift_, d_count, state());
+        fit_groups_kernel<<<n_groups_, 256, 0, stream_>>>(d_count, d_group);
+        fit_offsets_kernel<<<n_groups_, 256, 0, stream_>>>(d_count, d_group, d_offset, d_cursor);
+        if (windowed_) fit_scatter_window_kernel<<<sms_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_offset, d_begin, d_cursor, d_sorted, state());
+        else fit_scatter_kernel<<<grid, 256, 0, stream_>>>(r_.data, un, shift_, d_cursor, d_sorted, state());
+        fit_sums_kernel<<<n_parts, 256, 0, stream_>>>(d_sorted, d_count, d_offset, shift_, d_sum, d_part, state());
+        TQ_CUDA(cudaGetLastError());
+        job = FitJob{d_sorted, d_count, d_offset, d_sum, d_part, d_group_sum, state(), un, n_groups_, shift_, r_.iterations};
+        iterated_ = true;
+        return true;
+    }
+
+    // Waits for the iterations, makes those that are left over all samples, and hands the results out; the iterations run.
+    int finish() {
+        if (active_) {
+            if (iterated_) read_state();
+            if (h_.go_over_all && !h_.converged && h_.iterations_run < r_.iterations) go_over_all();
+            for (DeviceBuffer* b : {&state_buf_, &bucket_buf_, &sorted_buf_, &begin_buf_}) b->set_idle();
+        }
+        for (int i = 0; i < nc_; ++i) r_.centroids_out[i] = h_.centroids[i];
+        if (r_.boundaries_out)
+            for (int i = 0; i + 1 < nc_; ++i) r_.boundaries_out[i] = (h_.centroids[i] + h_.centroids[i + 1]) * 0.5f;   // src/codebook.cpp:135-139
+        return h_.iterations_run;
+    }
+
+private:
+    FitState* state() { return state_buf_.as<FitState>(); }
+    size_t window_bytes() const { return (static_cast<size_t>(window_) << (24 - shift_)) * sizeof(unsigned int); }
+    void read_state() {
+        TQ_CUDA(cudaMemcpyAsync(&h_, state(), sizeof h_, cudaMemcpyDeviceToHost, stream_));
+        TQ_CUDA(cudaStreamSynchronize(stream_));
+    }
+    void go_over_all() {
+        const long chunks = (r_.n + (1L << 14) - 1) >> 14;
+        const int blocks = static_cast<int>(std::min<long>(chunks, 2L * sms_));
+        const size_t smem = (sizeof(double) + sizeof(unsigned int)) * kFitMaxBins * kFitThreads;
+        static bool configured[64] = {false};
+        if (dev_ < 0 || dev_ >= 64 || !configured[dev_]) {
+            TQ_CUDA(cudaFuncSetAttribute(fit_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            if (dev_ >= 0 && dev_ < 64) configured[dev_] = true;
+        }
+        DeviceBuffer part_buf;
+        part_buf.reserve((sizeof(double) + sizeof(unsigned long long)) * kFitMaxBins * blocks, stream_);
+        double* const d_psum = part_buf.as<double>();
+        unsigned long long* const d_pcnt = reinterpret_cast<unsigned long long*>(d_psum + kFitMaxBins * blocks);
+        // all pairs of launches are enqueued at once; those after convergence return at their first instruction
+        for (int it = h_.iterations_run; it < r_.iterations; ++it) {
+            fit_partial_kernel<<<blocks, kFitThreads, smem, stream_>>>(r_.data, r_.n, state(), d_psum, d_pcnt);
+            fit_update_kernel<<<1, 32, 0, stream_>>>(state(), d_psum, d_pcnt, blocks);
+        }
+        TQ_CUDA(cudaGetLastError());
+        read_state();
+        part_buf.set_idle();
+    }
+
+    const FitRequest r_;
+    const cudaStream_t stream_;
+    const int nc_;
+    FitState h_{};
+    DeviceBuffer state_buf_, bucket_buf_, sorted_buf_, begin_buf_;
+    bool active_ = false, bucketed_ = false, windowed_ = false, iterated_ = false;
+    int dev_ = 0, sms_ = 148, shift_ = 0, n_buckets_ = 0, n_groups_ = 0, window_ = 0;
+};
+
+}  // namespace
+
+// Fits `bits`-bit centroids to data[n] starting from init_centroids (2^bits values, ascending).
+// centroids_out / boundaries_out: host arrays of 2^bits and 2^bits - 1 floats.  Returns the iterations run.
+int launch_codebook_fit(const FitRequest& r, cudaStream_t stream) {
+    FitRun run(r, stream);
+    FitJobs jobs{};
+    if (run.enqueue_buckets(jobs.job[0])) {
+        fit_iterate_kernel<<<1, 1024, 0, stream>>>(jobs);
+        TQ_CUDA(cudaGetLastError());
+    }
+    return run.finish();
+}
+
+// Two fits; their iterations run side by side (a CTA each, in one launch), as long as the device has memory for both.
+void launch_codebook_fits(const FitRequest& a, const FitRequest& b, cudaStream_t stream) {
+    constexpr long kTogether = 1L << 25;   // samples: up to there the memory is kept for the next call (tq_memory.cu)
+    if (std::max(a.n, b.n) <= kTogether) {
+        FitRun first(a, stream), second(b, stream);
+        if (!first.short_of_memory() && !second.short_of_memory()) {
+            FitJobs jobs{};
+            int n = 0;
+            if (first.enqueue_buckets(jobs.job[n])) ++n;
+            if (second.enqueue_buckets(jobs.job[n])) ++n;
+            if (n != 0) {
+                fit_iterate_kernel<<<n, 1024, 0, stream>>>(jobs);
+                TQ_CUDA(cudaGetLastError());
+            }
+            first.finish();
+            second.finish();
+            return;
+        }
+    }
+    launch_codebook_fit(a, stream);
+    launch_codebook_fit(b, stream);
 }
 
 void launch_layer_samples(const float* d_weight, const float* d_row_norms, long rows, int in, uint32_t block, uint32_t seed_p,

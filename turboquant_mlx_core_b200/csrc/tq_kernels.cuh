@@ -153,8 +153,15 @@ void launch_quantize_weight(const float* d_weight, long out, int in, const float
 void launch_row_norms(const float* d_matrix, float* d_out, long rows, int cols, cudaStream_t stream);
 
 // tq_codebook_fit.cu — Lloyd-Max fit on the device and the per-layer sample extraction.
-int launch_codebook_fit(const float* d_data, long n, int bits, int iterations, const float* init_centroids, float* centroids_out,
-                        float* boundaries_out, cudaStream_t stream);
+struct FitRequest {
+    const float* data;            // n samples, on the device
+    long n;
+    int bits, iterations;
+    const float* init_centroids;  // host: 2^bits, ascending
+    float *centroids_out, *boundaries_out;   // host; boundaries may be NULL
+};
+int launch_codebook_fit(const FitRequest& r, cudaStream_t stream);   // the iterations run
+void launch_codebook_fits(const FitRequest& a, const FitRequest& b, cudaStream_t stream);
 void launch_layer_samples(const float* d_weight, const float* d_row_norms, long rows, int in, uint32_t block, uint32_t seed_p,
                           const float* primary_centroids, int n_primary, float* d_scaled, float* d_residual, cudaStream_t stream);
 
