@@ -1,0 +1,62 @@
+"""Large copies between the device and host memory, in pieces: whatever their number, with a short last piece, several at once, and
+from several threads."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+# bytes of the fp32 result around the bounds of 8 and 32 MB and of a piece; rows that end inside a piece
+@pytest.mark.parametrize("rows,cols", [(64, 64), (2047, 1024), (2048, 1024), (2049, 1024), (8192, 1024), (8193, 1088), (20011, 1024)])
+def test_host_results_equal_device_results(tq, rows, cols):
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = torch.randn((rows, cols), generator=g, device="cuda") * 0.02
+    c = tq.generate_codebook(4)
+    cfg = tq.QuantizerConfig(4, 4, 64, True)
+    device, host = tq.quantize_weight(w, c, c, cfg), tq.quantize_weight(w.cpu().numpy(), c, c, cfg)
+    for name in ("packed_primary", "packed_residual", "norms", "seeds"):
+        assert np.array_equal(getattr(device, name), getattr(host, name)), name
+    lin = tq.TurboQuantLinear(cols, rows, host, c, c, 64)
+    back = torch.empty((rows, cols), device="cuda")
+    lin.dequantize(out=back)
+    assert np.array_equal(lin.dequantize(np.float32).view(np.uint32), back.cpu().numpy().view(np.uint32))
+    lin.close()
+
+
+def test_five_bit_and_primary_only_planes_are_written_whole(tq, oracle):
+    rng = np.random.default_rng(1)
+    w = (rng.standard_normal((48, 256)) * 0.02).astype(np.float32)
+    cb5, cb3 = tq.generate_codebook(5), tq.generate_codebook(3)
+    for bits, res, shared in ((5, 3, True), (4, 0, False), (5, 0, False)):
+        cb = cb5 if bits == 5 else tq.generate_codebook(4)
+        for _ in range(3):   # (memory that held something else before)
+            junk = np.full((48, 256), 0xA5, np.uint8)
+            del junk
+            qw = tq.quantize_weight(w, cb, cb3, tq.QuantizerConfig(bits, res, 128, shared))
+            pp, pr, norms, _ = oracle.quantize_weight(w, cb.centroids, cb3.centroids, bits, res, 128, shared)
+            assert np.array_equal(qw.packed_primary, pp) and np.array_equal(qw.packed_residual, pr)
+            assert np.array_equal(qw.norms.view(np.uint32), norms.view(np.uint32))
+
+
+def test_copies_from_several_threads(tq):
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    c = tq.generate_codebook(4)
+    weights = [torch.randn((3000, 1024), generator=g, device="cuda") * 0.02 for _ in range(4)]
+    layers = [tq.TurboQuantLinear(1024, 3000, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, 128, True)), c, c, 128) for w in weights]
+    alone = [lin.dequantize(np.float32) for lin in layers]
+    got = [None] * 4
+
+    def run(i):
+        for _ in range(3):
+            got[i] = layers[i].dequantize(np.float32)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(alone, got))

@@ -267,9 +267,9 @@ def quantize_weight(weight, primary_codebook: Codebook, residual_codebook: Codeb
     out_f, in_f = int(w.shape[0]), int(w.shape[1])
     if in_f % config.block_size:
         raise ValueError("in_features must be divisible by block_size")
-    pp = np.zeros((out_f, in_f // 2 if config.primary_bits <= 4 else in_f), np.uint8)
-    pr = np.zeros((out_f, in_f // 2), np.uint8)
-    norms = np.zeros(out_f, np.float32)
+    pp = np.empty((out_f, in_f // 2 if config.primary_bits <= 4 else in_f), np.uint8)
+    pr = np.empty((out_f, in_f // 2), np.uint8)
+    norms = np.empty(out_f, np.float32)
     cp, cr = _np(primary_codebook.centroids, np.float32), _np(residual_codebook.centroids, np.float32)
     out_seeds = np.zeros(3, np.uint32)
     if seeds is None:

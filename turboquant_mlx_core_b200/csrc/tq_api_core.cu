@@ -215,7 +215,13 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
         norms.reserve(static_cast<size_t>(out_features) * 4, st);
         scaled.reserve(n * 4, st);
         if (need_residual) resid.reserve(n * 4, st);
-        const float* d_w = device_view(weight, n, w_stage, st);
+        const float* d_w = weight;
+        if (!is_device_pointer(weight)) {
+            w_stage.reserve(n * sizeof(float), st);
+            const HostCopy copy{w_stage.as<void>(), weight, n * sizeof(float)};
+            copies_to_device(&copy, 1, st);
+            d_w = w_stage.as<float>();
+        }
         uint32_t seed_p = 0, seed_r = 0;
         derive_seeds(d_w, n, &seed_p, &seed_r, st);
         launch_row_norms(d_w, norms.as<float>(), out_features, in_features, st);

@@ -44,15 +44,25 @@ public:
 
         cudaStream_t st = nullptr;
         uint32_t h_seeds[3];
-        TQ_CUDA(cudaMemcpy(h_seeds, seeds, sizeof h_seeds, cudaMemcpyDefault));
+        tq::read_values(h_seeds, seeds, sizeof h_seeds);
         seed_p_ = h_seeds[0];
         seed_r_ = h_seeds[1];
 
         // codes: reference planes -> joint bytes
         const size_t n_w = static_cast<size_t>(out_) * in_;
         DeviceBuffer stage_p, stage_r, flags(2 * sizeof(unsigned int));
-        const uint8_t* d_pp = tq::device_view(packed_primary, static_cast<size_t>(out_) * primary_cols, stage_p, st);
-        const uint8_t* d_pr = tq::device_view(packed_residual, n_w / 2, stage_r, st);
+        const uint8_t *d_pp = packed_primary, *d_pr = packed_residual;
+        tq::HostCopy planes[2];
+        int n_planes = 0;
+        auto on_device = [&](const uint8_t*& plane, size_t bytes, DeviceBuffer& stage) {
+            if (tq::is_device_pointer(plane)) return;
+            stage.reserve(bytes, st);
+            planes[n_planes++] = tq::HostCopy{stage.as<void>(), plane, bytes};
+            plane = stage.as<uint8_t>();
+        };
+        on_device(d_pp, static_cast<size_t>(out_) * primary_cols, stage_p);
+        on_device(d_pr, n_w / 2, stage_r);
+        if (n_planes != 0) tq::copies_to_device(planes, n_planes, st);
         codes_.resize(tq::code_bytes(out_, in_));
         TQ_CUDA(cudaMemsetAsync(flags.as<void>(), 0, 2 * sizeof(unsigned int), st));
         tq::launch_relayout(d_pp, d_pr, codes_.as<uint8_t>(), out_, in_, primary_5bit_, flags.as<unsigned int>(), st);
@@ -68,8 +78,8 @@ public:
 
         // lookup tables over the joint byte
         std::vector<float> cp(n_p), cr(n_r);
-        TQ_CUDA(cudaMemcpy(cp.data(), cb_p, sizeof(float) * n_p, cudaMemcpyDefault));
-        TQ_CUDA(cudaMemcpy(cr.data(), cb_r, sizeof(float) * n_r, cudaMemcpyDefault));
+        tq::read_values(cp.data(), cb_p, sizeof(float) * n_p);
+        tq::read_values(cr.data(), cb_r, sizeof(float) * n_r);
         std::vector<float> tables(512, 0.0f);
         const int p_bits = primary_5bit_ ? 5 : 4;
         const int p_mask = (1 << p_bits) - 1;
@@ -381,8 +391,8 @@ public:
             tq::launch_dequant_f16(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), static_cast<__half*>(d_out),
                                    out_, in_, block_, seed_p_, seed_r_, dual_, st);
         if (!dev) {
-            TQ_CUDA(cudaMemcpyAsync(result, d_out, n * es, cudaMemcpyDeviceToHost, st));
-            TQ_CUDA(cudaStreamSynchronize(st));
+            const tq::HostCopy copy{result, d_out, n * es};
+            tq::copies_to_host(&copy, 1, st);
             stage.set_idle();
         }
     }
@@ -624,12 +634,18 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         const size_t n = static_cast<size_t>(out_features) * in_features;
         const size_t pp_bytes = primary_bits <= 4 ? n / 2 : n, pr_bytes = n / 2;
         std::vector<float> cp(n_primary), cr(n_residual);
-        TQ_CUDA(cudaMemcpy(cp.data(), primary_centroids, sizeof(float) * n_primary, cudaMemcpyDefault));
-        TQ_CUDA(cudaMemcpy(cr.data(), residual_centroids, sizeof(float) * n_residual, cudaMemcpyDefault));
+        read_values(cp.data(), primary_centroids, sizeof(float) * n_primary);
+        read_values(cr.data(), residual_centroids, sizeof(float) * n_residual);
         DeviceBuffer w_stage, recon, orig;
         recon.reserve(n * sizeof(float), st);
         orig.reserve(static_cast<size_t>(out_features) * sizeof(float) + 4, st);
-        const float* d_w = device_view(weight, n, w_stage, st);
+        const float* d_w = weight;
+        if (n != 0 && !is_device_pointer(weight)) {
+            w_stage.reserve(n * sizeof(float), st);
+            const HostCopy copy{w_stage.as<void>(), weight, n * sizeof(float)};
+            copies_to_device(&copy, 1, st);
+            d_w = w_stage.as<float>();
+        }
         const bool pp_dev = is_device_pointer(packed_primary), pr_dev = is_device_pointer(packed_residual),
                    nm_dev = is_device_pointer(norms);
         DeviceBuffer pp_stage, pr_stage, nm_stage;
@@ -649,13 +665,15 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         launch_quantize_weight(d_w, out_features, in_features, cp.data(), n_primary, cr.data(), n_residual, primary_bits,
                                residual_bits, block, shared_rotation != 0, seed_p, seed_r, d_pp, d_pr, d_nm,
                                orig.as<float>(), recon.as<float>(), st);
-        if (!pp_dev && pp_bytes) TQ_CUDA(cudaMemcpyAsync(packed_primary, d_pp, pp_bytes, cudaMemcpyDeviceToHost, st));
-        if (!pr_dev && pr_bytes) TQ_CUDA(cudaMemcpyAsync(packed_residual, d_pr, pr_bytes, cudaMemcpyDeviceToHost, st));
-        if (!nm_dev && out_features) TQ_CUDA(cudaMemcpyAsync(norms, d_nm, static_cast<size_t>(out_features) * 4, cudaMemcpyDeviceToHost, st));
+        HostCopy results[3];
+        int n_results = 0;
+        if (!pp_dev) results[n_results++] = HostCopy{packed_primary, d_pp, pp_bytes};
+        if (!pr_dev) results[n_results++] = HostCopy{packed_residual, d_pr, pr_bytes};
+        if (!nm_dev) results[n_results++] = HostCopy{norms, d_nm, static_cast<size_t>(out_features) * 4};
         // seeds = {primary, residual or 0 under shared rotation, block}  (src/quantizer.cpp:255-258)
         const uint32_t h_seeds[3] = {seed_p, (shared_rotation && residual_bits > 0) ? 0u : seed_r, block};
         TQ_CUDA(cudaMemcpyAsync(seeds, h_seeds, sizeof h_seeds, cudaMemcpyDefault, st));
-        TQ_CUDA(cudaStreamSynchronize(st));  // scratch and staging buffers die here
+        copies_to_host(results, n_results, st);   // (waits in any case: scratch and staging buffers die here)
         for (DeviceBuffer* b : {&w_stage, &recon, &orig, &pp_stage, &pr_stage, &nm_stage}) b->set_idle();
         return 0;
     });

@@ -180,6 +180,18 @@ private:
     bool idle_ = false;
 };
 
+// ---- host memory (tq_host_copy.cu) ---------------------------------------------------------------
+struct HostCopy {
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+// From device memory, behind the work queued on `st`, into host memory of any kind and back; the calls wait for the copies.
+void copies_to_host(const HostCopy* copies, int n, cudaStream_t st);
+void copies_to_device(const HostCopy* copies, int n, cudaStream_t st);
+// A few values that may be in device or in host memory.
+void read_values(void* dst, const void* src, size_t bytes);
+
 // A read-only view of caller data on the device: device pointers are used in place,
 // host pointers are copied into `staging` on `stream`.
 template <typename T>
