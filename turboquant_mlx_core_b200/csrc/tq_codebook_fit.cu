@@ -589,14 +589,16 @@ __global__ void __launch_bounds__(32) fit_update_kernel(FitState* __restrict__ s
 // Rotated, scaled samples of a weight matrix and the residuals the shared primary codebook leaves
 // (src/converter.cpp:303-357; the arithmetic is the quantiser's, src/quantizer.cpp:43-62, 117-120).
 // One warp per (row, WHT block).  residual may be NULL.
+// Bound by instruction issue: 4096 x 4096, block 512, 184 us with 4-byte accesses 64 bytes apart and the boundaries compared one
+// after the other, 62 here.
 struct SampleTables {
-    float cp[32], bp[31];
+    float cp[32], bp[31];   // the shared codebook's, ascending; boundaries padded with +infinity
     int n_p;
 };
 
 template <int E>
 __global__ void __launch_bounds__(128) layer_samples_kernel(const float* __restrict__ w, const float* __restrict__ orig_norm, long rows,
-                                                            int blocks_per_row, uint32_t seed_p, float scale, float inv_sqrt,
+                                                            int blocks_per_row, uint32_t seed_p, float scale, float inv_sqrt, int wide,
                                                             const SampleTables tb, float* __restrict__ scaled,
                                                             float* __restrict__ residual) {
     __shared__ SampleTables t;
@@ -617,18 +619,17 @@ __global__ void __launch_bounds__(128) layer_samples_kernel(const float* __restr
         const size_t base = static_cast<size_t>(row) * in + bcol;
         const float safe = fmaxf(orig_norm[row], 1e-10f);
         float v[E];
+        load_lane<E>(v, w + base, wide != 0);
 #pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = __fmul_rn(__fdiv_rn(w[base + j], safe), sp[j]);
+        for (int j = 0; j < E; ++j) v[j] = __fmul_rn(__fdiv_rn(v[j], safe), sp[j]);
         warp_fwht<E>(v, lane);
 #pragma unroll
-        for (int j = 0; j < E; ++j) {
-            v[j] = __fmul_rn(__fmul_rn(v[j], inv_sqrt), scale);
-            scaled[base + j] = v[j];
-            if (residual != nullptr) {
-                int idx = 0;
-                for (int i = 0; i < t.n_p - 1; ++i) idx += (t.bp[i] < v[j]) ? 1 : 0;
-                residual[base + j] = __fsub_rn(v[j], t.cp[idx]);
-            }
+        for (int j = 0; j < E; ++j) v[j] = __fmul_rn(__fmul_rn(v[j], inv_sqrt), scale);
+        store_lane<E>(scaled + base, v, wide != 0);
+        if (residual != nullptr) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) v[j] = __fsub_rn(v[j], t.cp[bin_of_sorted(v[j], t.bp, t.n_p > 16)]);
+            store_lane<E>(residual + base, v, wide != 0);
         }
     }
 }
@@ -820,6 +821,7 @@ void launch_layer_samples(const float* d_weight, const float* d_row_norms, long 
     SampleTables tb{};
     tb.n_p = n_primary;
     for (int i = 0; i < n_primary; ++i) tb.cp[i] = primary_centroids[i];
+    for (float& b : tb.bp) b = INFINITY;
     for (int i = 0; i + 1 < n_primary; ++i) tb.bp[i] = (primary_centroids[i] + primary_centroids[i + 1]) * 0.5f;
     const float scale = std::sqrt(static_cast<float>(in));
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
@@ -827,9 +829,10 @@ void launch_layer_samples(const float* d_weight, const float* d_row_norms, long 
     const long total = rows * bpr;
     const long want = (total + 3) / 4;
     const int grid = static_cast<int>(want < 148L * 16 ? want : 148L * 16);
+    const int wide = (reinterpret_cast<uintptr_t>(d_weight) | reinterpret_cast<uintptr_t>(d_scaled) | reinterpret_cast<uintptr_t>(d_residual)) % 16 == 0 ? 1 : 0;
 #define TQ_S_CASE(EV)                                                                                                              \
     case 32 * EV:                                                                                                                  \
-        layer_samples_kernel<EV><<<grid, 128, 0, stream>>>(d_weight, d_row_norms, rows, bpr, seed_p, scale, inv_sqrt, tb, d_scaled, \
+        layer_samples_kernel<EV><<<grid, 128, 0, stream>>>(d_weight, d_row_norms, rows, bpr, seed_p, scale, inv_sqrt, wide, tb, d_scaled, \
                                                            d_residual);                                                            \
         break;
     switch (block) {

@@ -61,8 +61,8 @@ __host__ __device__ __forceinline__ uint32_t kv_layer_seed(uint32_t layer, uint3
 // One warp transforms one block of 32*E values; lane l holds elements [l*E, (l+1)*E).
 // The add tree is the reference's (src/rotation.cpp:14-25): for h = 1, 2, 4, ... the
 // pair (j, j+h) becomes (a+b, a-b) with a the lower index.  Stages h < E stay in
-// registers; stages h >= E exchange with lane ^ (h/E).  Only __fadd_rn/__fsub_rn are
-// used so nothing can be contracted into an FMA: results are bit-identical to the
+// registers; stages h >= E exchange with lane ^ (h/E).  Only __fadd_rn/__fsub_rn, and multiply-adds with +-1, which
+// round as they do, are used so nothing else can be contracted into an FMA: results are bit-identical to the
 // scalar loop.
 template <int E>
 __device__ __forceinline__ void warp_fwht(float (&v)[E], int lane) {
@@ -80,14 +80,52 @@ __device__ __forceinline__ void warp_fwht(float (&v)[E], int lane) {
     }
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) {
-        const bool upper = (lane & m) != 0;
+        // lower lane: mine + other; upper lane: other - mine  (a is the lower index)
+        const float side = (lane & m) != 0 ? -1.0f : 1.0f;
 #pragma unroll
-        for (int j = 0; j < E; ++j) {
-            float other = __shfl_xor_sync(0xffffffffu, v[j], m);
-            // lower lane: mine + other; upper lane: other - mine  (a is the lower index)
-            v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
+        for (int j = 0; j < E; ++j) v[j] = __fmaf_rn(v[j], side, __shfl_xor_sync(0xffffffffu, v[j], m));
+    }
+}
+
+// E consecutive values of a lane, in 16-byte accesses where `wide` (all addresses are multiples of 16 bytes then).
+template <int E>
+__device__ __forceinline__ void load_lane(float (&v)[E], const float* __restrict__ p, bool wide) {
+    if constexpr (E % 4 == 0) {
+        if (wide) {
+#pragma unroll
+            for (int j = 0; j < E; j += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(p + j);
+                v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+            }
+            return;
         }
     }
+#pragma unroll
+    for (int j = 0; j < E; ++j) v[j] = p[j];
+}
+template <int E>
+__device__ __forceinline__ void store_lane(float* __restrict__ p, const float (&v)[E], bool wide) {
+    if constexpr (E % 4 == 0) {
+        if (wide) {
+#pragma unroll
+            for (int j = 0; j < E; j += 4) *reinterpret_cast<float4*>(p + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            return;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < E; ++j) p[j] = v[j];
+}
+
+// Number of the sorted boundaries below v, as std::lower_bound finds it: `b` holds 31 (more than 15: `five`) or 15 of
+// them, +infinity where there are fewer.
+__device__ __forceinline__ int bin_of_sorted(float v, const float* b, bool five) {
+    int i = 0;
+    if (five && b[15] < v) i = 16;
+    if (b[i + 7] < v) i += 8;
+    if (b[i + 3] < v) i += 4;
+    if (b[i + 1] < v) i += 2;
+    if (b[i] < v) i += 1;
+    return i;
 }
 
 __host__ __device__ __forceinline__ bool is_pow2(uint32_t v) { return v && !(v & (v - 1)); }

@@ -26,33 +26,64 @@ namespace tq {
 namespace {
 
 // sum_j m[r][j]^2, accumulated strictly left to right in fp32; out[r] = sqrt(sum).
-// One warp per row: lanes read 32 consecutive columns (coalesced, four such pieces in flight) and
-// square them; the running sum then takes the 32 squares in column order through lane
-// broadcasts, every lane carrying the same sum.  Columns past the end contribute +0.0, which
-// leaves a non-negative sum unchanged.  All rows run at once, so the matrix streams from HBM
-// while each row's add chain (the order that makes the result bit-exact) stays serial.
-__global__ void __launch_bounds__(256) row_norm_seq_kernel(const float* __restrict__ m, float* __restrict__ out,
-                                                           long rows, int cols) {
-    const int lane = threadIdx.x & 31;
-    const long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= rows) return;
-    const float* src = m + row * cols;
-    float acc = 0.0f;
-    for (int c0 = 0; c0 < cols; c0 += 128) {
-        float sq[4];
+// The order makes the result bit-exact, and it is a chain of additions per row.  A lane takes a row, so that a warp's
+// instruction adds for 32 rows at once (with a warp per row, the squares passed from lane to lane, 4096 x 4096 took 86 us,
+// bound by those exchanges; here 24).  The rows come through shared memory: the CTA's warps fetch tiles of 32 rows x
+// kNormCols columns, kNormStages - 1 of them ahead, while the first warp adds the current one up.  Bound: the chain, four cycles
+// per column, and HBM.
+constexpr int kNormRows = 32, kNormCols = 128, kNormStages = 4, kNormThreads = 128;
+constexpr int kNormPitch = kNormCols + 4;   // floats: rows four banks apart
+constexpr size_t kNormSmem = sizeof(float) * kNormStages * kNormRows * kNormPitch;
+__device__ __forceinline__ void norm_fetch(float* dst, const float* src, bool have, bool wide) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if (wide) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(have ? 16 : 0) : "memory");
+    } else {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c = c0 + 32 * u + lane;
-            const float v = c < cols ? __ldg(src + c) : 0.0f;
-            sq[u] = __fmul_rn(v, v);
+        for (int k = 0; k < 4; ++k) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * k), "l"(src + k), "r"(have ? 4 : 0) : "memory");
+    }
+}
+// cols is a multiple of four.  Missing rows and columns read as zero (no address beyond the matrix is formed); they add +0.0
+// to sums that are not negative.
+__global__ void __launch_bounds__(kNormThreads) row_norm_seq_kernel(const float* __restrict__ m, float* __restrict__ out, long rows, int cols, int wide) {
+    extern __shared__ __align__(16) float s_tile[];   // [stage][row][kNormPitch]
+    const int tid = threadIdx.x;
+    const long row0 = static_cast<long>(blockIdx.x) * kNormRows;
+    const int n_tiles = (cols + kNormCols - 1) / kNormCols;
+    constexpr int kPieces = kNormRows * kNormCols / 4;   // of four columns
+    auto fetch = [&](int tile) {
+        if (tile < n_tiles) {
+            float* const stage = s_tile + (tile % kNormStages) * (kNormRows * kNormPitch);
+#pragma unroll
+            for (int k = 0; k < kPieces / kNormThreads; ++k) {
+                const int i = k * kNormThreads + tid, r = i / (kNormCols / 4), c = 4 * (i % (kNormCols / 4));
+                const int col = tile * kNormCols + c;
+                const bool have = row0 + r < rows && col < cols;
+                norm_fetch(stage + r * kNormPitch + c, have ? m + (row0 + r) * cols + col : m, have, wide != 0);
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc = __fadd_rn(acc, __shfl_sync(0xffffffffu, sq[u], j));
+    for (int t = 0; t < kNormStages - 1; ++t) fetch(t);
+    float acc = 0.0f;
+    for (int t = 0; t < n_tiles; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kNormStages - 2) : "memory");
+        __syncthreads();   // the tile is there for all, and the one before it has been added up
+        fetch(t + kNormStages - 1);
+        if (tid < 32) {
+            const float* const row = s_tile + (t % kNormStages) * (kNormRows * kNormPitch) + tid * kNormPitch;
+#pragma unroll 8
+            for (int c = 0; c < kNormCols; c += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(row + c);
+                acc = __fadd_rn(acc, __fmul_rn(v.x, v.x));
+                acc = __fadd_rn(acc, __fmul_rn(v.y, v.y));
+                acc = __fadd_rn(acc, __fmul_rn(v.z, v.z));
+                acc = __fadd_rn(acc, __fmul_rn(v.w, v.w));
+            }
         }
     }
-    if (lane == 0) out[row] = __fsqrt_rn(acc);
+    if (tid < 32 && row0 + tid < rows) out[row0 + tid] = __fsqrt_rn(acc);
 }
 
 __global__ void corrected_norm_kernel(const float* __restrict__ orig, float* __restrict__ recon_inout, long rows) {
@@ -67,23 +98,27 @@ __global__ void gather_bytes_kernel(const uint8_t* __restrict__ bytes, size_t by
     if (i < n) out[i] = bytes[static_cast<size_t>(i) * stride];
 }
 
+// Boundaries are padded with +infinity.  `sorted`: both codebooks ascend, so a code is found in four or five steps; the
+// comparisons are counted one by one otherwise.
 struct QuantTables {
     float cp[32], bp[31], cr[16], br[15];
-    int n_p, n_r;
+    int n_p, n_r, sorted;
 };
 
 __device__ __forceinline__ int bin_of(float v, const float* bounds, int n_bounds) {
     int idx = 0;
-    for (int i = 0; i < n_bounds; ++i) idx += (bounds[i] < v) ? 1 : 0;  // sorted, so this equals lower_bound
+    for (int i = 0; i < n_bounds; ++i) idx += (bounds[i] < v) ? 1 : 0;
     return idx;
 }
 
+// Bound by instruction issue.  4096 x 4096, block 512, one rotation: 297 us with 4-byte accesses 64 bytes apart, boundaries
+// compared one after the other and bytes stored one at a time (273 instructions per weight), 89 here.
 template <int E>
 __global__ void __launch_bounds__(128) quantize_rows_kernel(
     const float* __restrict__ w, const float* __restrict__ orig_norm, uint8_t* __restrict__ packed_primary,
     uint8_t* __restrict__ packed_residual, float* __restrict__ recon, long rows, int blocks_per_row, uint32_t seed_p,
     uint32_t seed_r, int primary_bits, int residual_bits, int shared_rotation, float scale, float inv_scale,
-    float inv_sqrt, const QuantTables tb) {
+    float inv_sqrt, int wide, const QuantTables tb) {
     __shared__ QuantTables t;
     if (threadIdx.x == 0) t = tb;
     __syncthreads();
@@ -107,17 +142,23 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(
         const size_t base = static_cast<size_t>(row) * in + bcol;
         const float safe = fmaxf(orig_norm[row], 1e-10f);
         float v[E];
+        load_lane<E>(v, w + base, wide != 0);
 #pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = __fmul_rn(__fdiv_rn(w[base + j], safe), sp[j]);
+        for (int j = 0; j < E; ++j) v[j] = __fmul_rn(__fdiv_rn(v[j], safe), sp[j]);
         warp_fwht<E>(v, lane);
         int cp_idx[E], cr_idx[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             v[j] = __fmul_rn(__fmul_rn(v[j], inv_sqrt), scale);
-            int idx = bin_of(v[j], t.bp, t.n_p - 1);
-            if (idx >= t.n_p) idx = t.n_p - 1;
-            cp_idx[j] = idx;
             cr_idx[j] = 0;
+        }
+        // (at most n_p - 1 boundaries are below a value)
+        if (t.sorted) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) cp_idx[j] = bin_of_sorted(v[j], t.bp, t.n_p > 16);
+        } else {
+#pragma unroll
+            for (int j = 0; j < E; ++j) cp_idx[j] = bin_of(v[j], t.bp, t.n_p - 1);
         }
         if (residual_bits > 0) {
             float r[E];
@@ -133,11 +174,13 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(
 #pragma unroll
                 for (int j = 0; j < E; ++j) r[j] = __fmul_rn(__fmul_rn(r[j], inv_sqrt), scale);
             }
+            // (a nibble: the reconstruction re-reads the packed one, :179-183)
+            if (t.sorted) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                int idx = bin_of(r[j], t.br, t.n_r - 1);
-                if (idx >= t.n_r) idx = t.n_r - 1;
-                cr_idx[j] = idx & 0x0F;  // the reconstruction re-reads the packed nibble (:179-183)
+                for (int j = 0; j < E; ++j) cr_idx[j] = bin_of_sorted(r[j], t.br, false);
+            } else {
+#pragma unroll
+                for (int j = 0; j < E; ++j) cr_idx[j] = bin_of(r[j], t.br, t.n_r - 1);
             }
         }
 
@@ -146,7 +189,31 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(
 #pragma unroll
             for (int j = 0; j < E; ++j) packed_primary[base + j] = static_cast<uint8_t>(cp_idx[j]);
         }
-        if constexpr (E >= 2) {
+        if constexpr (E >= 8) {
+            // eight nibbles to a word
+            uint32_t pw[E / 8], rw[E / 8];
+#pragma unroll
+            for (int k = 0; k < E / 8; ++k) {
+                pw[k] = rw[k] = 0u;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    pw[k] |= static_cast<uint32_t>(cp_idx[8 * k + j] & 0x0F) << (4 * j);
+                    rw[k] |= static_cast<uint32_t>(cr_idx[8 * k + j]) << (4 * j);
+                }
+            }
+            auto put = [&](uint8_t* plane, const uint32_t (&word)[E / 8]) {
+                uint8_t* const dst = plane + (base >> 1);
+                if (wide) {
+#pragma unroll
+                    for (int k = 0; k < E / 8; ++k) reinterpret_cast<uint32_t*>(dst)[k] = word[k];
+                } else {
+#pragma unroll
+                    for (int i = 0; i < E / 2; ++i) dst[i] = static_cast<uint8_t>(word[i / 4] >> (8 * (i & 3)));
+                }
+            };
+            if (primary_bits <= 4) put(packed_primary, pw);
+            put(packed_residual, rw);
+        } else if constexpr (E >= 2) {
 #pragma unroll
             for (int j = 0; j < E; j += 2) {
                 if (primary_bits <= 4)
@@ -187,8 +254,7 @@ __global__ void __launch_bounds__(128) quantize_rows_kernel(
                 for (int j = 0; j < E; ++j) u[j] = __fadd_rn(u[j], __fmul_rn(z[j], __fmul_rn(inv_sqrt, sr[j])));
             }
         }
-#pragma unroll
-        for (int j = 0; j < E; ++j) recon[base + j] = u[j];
+        store_lane<E>(recon + base, u, wide != 0);
     }
 }
 
@@ -205,7 +271,16 @@ uint32_t fnv1a(const std::vector<uint8_t>& bytes, uint32_t salt) {
 
 void launch_row_norms(const float* d_matrix, float* d_out, long rows, int cols, cudaStream_t stream) {
     if (rows == 0) return;
-    row_norm_seq_kernel<<<static_cast<int>((rows + 7) / 8), 256, 0, stream>>>(d_matrix, d_out, rows, cols);
+    TQ_REQUIRE(cols % 4 == 0, "row norms: columns in fours");   // (whole WHT blocks)
+    static bool configured[64] = {false};
+    int dev = 0;
+    TQ_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev]) {
+        TQ_CUDA(cudaFuncSetAttribute(row_norm_seq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kNormSmem)));
+        if (dev < 64) configured[dev] = true;
+    }
+    const int wide = reinterpret_cast<uintptr_t>(d_matrix) % 16 == 0 ? 1 : 0;
+    row_norm_seq_kernel<<<static_cast<unsigned int>((rows + kNormRows - 1) / kNormRows), kNormThreads, kNormSmem, stream>>>(d_matrix, d_out, rows, cols, wide);
     TQ_CUDA(cudaGetLastError());
 }
 
@@ -242,19 +317,28 @@ void launch_quantize_weight(const float* d_weight, long out, int in, const float
     QuantTables tb{};
     tb.n_p = n_p;
     tb.n_r = n_r;
+    tb.sorted = 1;
+    for (float& b : tb.bp) b = INFINITY;
+    for (float& b : tb.br) b = INFINITY;
     for (int i = 0; i < n_p; ++i) tb.cp[i] = cb_p[i];
     for (int i = 0; i < n_r; ++i) tb.cr[i] = cb_r[i];
     for (int i = 0; i + 1 < n_p; ++i) tb.bp[i] = (cb_p[i] + cb_p[i + 1]) * 0.5f;  // src/codebook.cpp:49-57
     for (int i = 0; i + 1 < n_r; ++i) tb.br[i] = (cb_r[i] + cb_r[i + 1]) * 0.5f;
+    for (int i = 1; i + 1 < n_p; ++i)
+        if (!(tb.bp[i - 1] <= tb.bp[i])) tb.sorted = 0;
+    for (int i = 1; i + 1 < n_r; ++i)
+        if (!(tb.br[i - 1] <= tb.br[i])) tb.sorted = 0;
+    if (std::isnan(tb.bp[0]) || std::isnan(tb.br[0])) tb.sorted = 0;
+    // 16-byte accesses: a lane's weights are a multiple of 16 bytes apart from four on, its codes whole words from eight on
+    const int wide = (reinterpret_cast<uintptr_t>(d_weight) | reinterpret_cast<uintptr_t>(d_recon_tmp) | reinterpret_cast<uintptr_t>(d_packed_primary) |
+                      reinterpret_cast<uintptr_t>(d_packed_residual)) % 16 == 0 ? 1 : 0;
     const float scale = std::sqrt(static_cast<float>(in));  // src/quantizer.cpp:51-52
     const float inv_scale = 1.0f / scale;
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
     const int bpr = in / static_cast<int>(block);
     const long total = out * bpr;
 
-    const int norm_grid = static_cast<int>((out + 7) / 8);  // 8 warps (rows) per CTA
-    row_norm_seq_kernel<<<norm_grid, 256, 0, stream>>>(d_weight, d_orig_norm_tmp, out, in);
-    TQ_CUDA(cudaGetLastError());
+    launch_row_norms(d_weight, d_orig_norm_tmp, out, in, stream);
     if (residual_bits == 0) TQ_CUDA(cudaMemsetAsync(d_packed_residual, 0, static_cast<size_t>(out) * (in / 2), stream));
     long want = (total + 3) / 4;
     const int grid = static_cast<int>(want < 148L * 16 ? want : 148L * 16);
@@ -263,7 +347,7 @@ void launch_quantize_weight(const float* d_weight, long out, int in, const float
         quantize_rows_kernel<EV><<<grid, 128, 0, stream>>>(d_weight, d_orig_norm_tmp, d_packed_primary,               \
                                                            d_packed_residual, d_recon_tmp, out, bpr, seed_p, seed_r,  \
                                                            primary_bits, residual_bits, shared_rotation ? 1 : 0,      \
-                                                           scale, inv_scale, inv_sqrt, tb);                           \
+                                                           scale, inv_scale, inv_sqrt, wide, tb);                     \
         break;
     switch (block) {
         TQ_Q_CASE(1) TQ_Q_CASE(2) TQ_Q_CASE(4) TQ_Q_CASE(8) TQ_Q_CASE(16) TQ_Q_CASE(32)
@@ -271,8 +355,7 @@ void launch_quantize_weight(const float* d_weight, long out, int in, const float
     }
 #undef TQ_Q_CASE
     TQ_CUDA(cudaGetLastError());
-    row_norm_seq_kernel<<<norm_grid, 256, 0, stream>>>(d_recon_tmp, d_norms, out, in);
-    TQ_CUDA(cudaGetLastError());
+    launch_row_norms(d_recon_tmp, d_norms, out, in, stream);
     corrected_norm_kernel<<<static_cast<int>((out + 255) / 256), 256, 0, stream>>>(d_orig_norm_tmp, d_norms, out);
     TQ_CUDA(cudaGetLastError());
 }
