@@ -250,21 +250,10 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
 // A warp takes 8 rows x COLS columns, `row_steps` times; the four warps of a CTA take neighbouring groups of 8 rows.  With the butterflies as
 // lane exchanges (as the kernel below has them) a value took 34 instructions, four of five issue slots: 2048 x 18944 in 52 us
 // against 23 of its bytes, three rotations of 2048 x 3584 in 37; here 30 and 20 (two rotations, block 512, of 2048 x 17920: 101 -> 59).
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // Two fp32 numbers times `scale`, as halves.
 __device__ __forceinline__ uint32_t scaled_halves(unsigned long long v, unsigned long long scale) {
-    float lo, hi;
-    asm("{ .reg .b64 t; mul.rn.f32x2 t, %2, %3; mov.b64 {%0, %1}, t; }" : "=f"(lo), "=f"(hi) : "l"(v), "l"(scale));
-    const __half2 h = __floats2half2_rn(lo, hi);
+    const float2 t = unpack2(mul2(v, scale));
+    const __half2 h = __floats2half2_rn(t.x, t.y);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 constexpr int kRotateWarps = 4;
@@ -309,8 +298,7 @@ __device__ __forceinline__ void rotate_rows_mma_body(const __half* __restrict__ 
         const uint32_t lo = odd ? 0xBC00u : 0x3C00u;
         h[i] = lo | ((lo ^ ((m & 1) ? 0x8000u : 0u)) << 16);
     }
-    unsigned long long scale;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(scale) : "f"(inv_sqrt));
+    const unsigned long long scale = pack2(inv_sqrt, inv_sqrt);
     const long n_row_tiles = (rows + kTileTok - 1) / kTileTok;
     const long kb_per_plane = in / kBlockK;
     uint4* const out = s_out[warp];

@@ -47,16 +47,84 @@ __device__ __forceinline__ void quad_fwht(float (&v)[N], int q) {
     }
 }
 
-// sum over the vector of v[j]^2, accumulated left to right in fp32 (src/kv_cache.cpp:84-88, 226-231: the order is part of
-// the result): the running sum goes through the quad's lanes in turn.
+// The same on pairs of neighbouring dims.
 template <int N>
-__device__ __forceinline__ float quad_square_sum(const float (&v)[N], int lane) {
+__device__ __forceinline__ void quad_fwht2(unsigned long long (&v)[N / 2], int q) {
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const float2 t = unpack2(v[i]);
+        v[i] = pack2(__fadd_rn(t.x, t.y), __fsub_rn(t.x, t.y));
+    }
+#pragma unroll
+    for (int h = 1; h < N / 2; h <<= 1) {
+#pragma unroll
+        for (int i = 0; i < N / 2; i += 2 * h) {
+#pragma unroll
+            for (int j = i; j < i + h; ++j) {
+                const unsigned long long a = v[j], b = v[j + h];
+                v[j] = add2(a, b);
+                v[j + h] = sub2(a, b);
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+        // other + v, or other - v in the upper lane: multiply-adds with +-1 round as they do
+        const float side = (q & m) != 0 ? -1.0f : 1.0f;
+        const unsigned long long side2 = pack2(side, side);
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) {
+            const float2 t = unpack2(v[j]);
+            v[j] = fma2(v[j], side2, pack2(__shfl_xor_sync(0xffffffffu, t.x, m), __shfl_xor_sync(0xffffffffu, t.y, m)));
+        }
+    }
+}
+
+// Sums over a vector of v[j]^2, accumulated left to right in fp32 (src/kv_cache.cpp:84-88, 226-231: the order is part of the
+// result).  The 32 vectors of a CTA put their squares into shared memory and one warp adds them up, a lane per vector; a
+// vector's quarters are kQuarter floats apart and vectors kPitch, so that neither side's 16-byte accesses meet in a bank.
+template <int D>
+struct SquareSums {
+    static constexpr int kQuarter = (D / 4 + 23) / 32 * 32 + 8, kPitch = 4 * kQuarter + 4;
+    static constexpr bool kShared = D <= 256;   // (beyond, the running sum goes through the quad's lanes in turn: 32 vectors take 70 KB)
+    __align__(16) float sq[kShared ? 32 * kPitch : 4];
+    float sum[32];
+};
+template <int D>
+__device__ __forceinline__ void put_squares(const unsigned long long (&v)[D / 8], SquareSums<D>& s) {
+    using S = SquareSums<D>;
+    float* const mine = s.sq + (threadIdx.x >> 2) * S::kPitch + (threadIdx.x & 3) * S::kQuarter;
+#pragma unroll
+    for (int j = 0; j < D / 4; j += 4) {
+        const float2 a = unpack2(mul2(v[j / 2], v[j / 2])), b = unpack2(mul2(v[j / 2 + 1], v[j / 2 + 1]));
+        *reinterpret_cast<float4*>(mine + j) = make_float4(a.x, a.y, b.x, b.y);
+    }
+}
+template <int D>
+__device__ __forceinline__ float add_squares(const SquareSums<D>& s, int vector) {
+    using S = SquareSums<D>;
+    const float* const row = s.sq + vector * S::kPitch;
+    float acc = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll 8
+        for (int j = 0; j < D / 4; j += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(row + k * S::kQuarter + j);
+            acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, t.x), t.y), t.z), t.w);
+        }
+    return acc;
+}
+template <int N>
+__device__ __forceinline__ float quad_square_sum(const unsigned long long (&v)[N / 2], int lane) {
     float acc = 0.0f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         float t = acc;
 #pragma unroll
-        for (int j = 0; j < N; ++j) t = __fadd_rn(t, __fmul_rn(v[j], v[j]));
+        for (int j = 0; j < N / 2; ++j) {
+            const float2 x = unpack2(mul2(v[j], v[j]));
+            t = __fadd_rn(__fadd_rn(t, x.x), x.y);
+        }
         acc = __shfl_sync(0xffffffffu, t, (lane & 28) + k);
     }
     return acc;
@@ -82,6 +150,19 @@ __device__ __forceinline__ uint32_t code_of(float x, float& residual) {
     return pos ? 4u + m : 3u - m;
 }
 
+// The code alone: 4 + m, or 7 - (4 + m) = (4 + m) ^ 7 for x <= 0, as in code_of, with a comparison less.
+__device__ __forceinline__ uint32_t code_only(float x) {
+    const uint32_t t1 = __float_as_uint(__fmul_rn(__fadd_rn(kMag0, kMag1), 0.5f));
+    const uint32_t t2 = __float_as_uint(__fmul_rn(__fadd_rn(kMag1, kMag2), 0.5f));
+    const uint32_t t3 = __float_as_uint(__fmul_rn(__fadd_rn(kMag2, kMag3), 0.5f));
+    const bool pos = x > 0.0f;
+    const uint32_t a = (__float_as_uint(x) & 0x7fffffffu) + (pos ? 0u : 1u);
+    const bool far = a > t2;
+    uint32_t c = far ? 6u : 4u;
+    if (a > (far ? t3 : t1)) c += 1u;
+    return pos ? c : c ^ 7u;
+}
+
 struct KvSegments {
     KvSegment seg[kKvMaxSegments];
 };
@@ -97,23 +178,44 @@ __device__ __forceinline__ uint32_t nibbles_to_bytes(uint32_t four) {
 // the second the values'.  A value byte holds both tokens' codes: the two quads exchange half of their words and each
 // writes four of the eight groups.  A pair of which only one token is appended keeps the other one's bits.
 // Bit-exact: the sums of squares run left to right, every other operation is element-wise or the shared butterfly.
-// Bound: issue slots (about 1100 instructions per lane and vector).  A warp per vector with one lane summing while 31
-// waited took 47 us for 2 x 32768 vectors of 128 (two launches), and a batched variant existed beside it for long
-// appends; four lanes per vector serve both.
+// Bound: issue slots.  2 x 32768 vectors of 128, fp16: 26 us under the profiler with 2175 instructions for a warp's eight
+// vectors (a quarter of them for sums that each lane of a quad repeated, and values had residuals that nothing reads);
+// 20 with 1445, pairs of dims in one instruction, signs flipped on the halves, the sums as above and
+// residuals for keys alone.
 template <int D, typename InT>
-__global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ keys, const InT* __restrict__ values, int tokens, int n_segs,
+__global__ void __launch_bounds__(128, D <= 128 ? 7 : (D == 256 ? 3 : 2)) kv_encode_kernel(const InT* __restrict__ keys, const InT* __restrict__ values, int tokens, int n_segs,
                                                         int heads, uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed,
                                                         float scale, float inv_sqrt, int aligned,
                                                         const __grid_constant__ KvSegments tab) {
     constexpr int N = D / 4, W = N / 8;
+    constexpr int kPer = 16 / static_cast<int>(sizeof(InT));   // elements of a 16-byte access
     using B = KvBlock<D>;
-    __shared__ uint32_t s_sign[3][D / 32];   // key rotation, value rotation, residual signs: bit set = +1
-    for (int i = threadIdx.x; i < 3 * D; i += 128) {
-        const int which = i / D, d = i - which * D;
-        const bool pos = which == 2 ? qjl_sign_is_positive(qjl_seed, static_cast<uint32_t>(d))
-                                    : sign_is_positive(which ? v_seed : k_seed, static_cast<uint32_t>(d));
-        const uint32_t bits = __ballot_sync(0xffffffffu, pos);
-        if ((i & 31) == 0) s_sign[which][d >> 5] = bits;
+    constexpr int kFlips = N / kPer + 1;                   // 16-byte words of a quarter's signs, and one so that the quarters lie in other banks
+    __shared__ __align__(16) uint4 s_flip[2][4 * kFlips];  // rotation signs of keys and values, as the elements' sign bits
+    __shared__ uint32_t s_qjl[D / 32];                    // residual signs: bit set = +1
+    __shared__ float s_cent[8][32];                       // a copy per lane
+    __shared__ SquareSums<D> s_sums;
+    __shared__ float* s_norm_at[32];                      // where a vector's residual norm goes
+    for (int i = threadIdx.x; i < D; i += 128) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, qjl_sign_is_positive(qjl_seed, static_cast<uint32_t>(i)));
+        if ((i & 31) == 0) s_qjl[i >> 5] = bits;
+    }
+    {
+        constexpr int kPerWord = 4 / static_cast<int>(sizeof(InT));
+        for (int i = threadIdx.x; i < 2 * D / kPerWord; i += 128) {
+            const int which = i / (D / kPerWord), d = (i - which * (D / kPerWord)) * kPerWord;
+            uint32_t m = 0;
+#pragma unroll
+            for (int k = 0; k < kPerWord; ++k)
+                if (!sign_is_positive(which ? v_seed : k_seed, static_cast<uint32_t>(d + k))) m |= 0x80000000u >> (16 * (kPerWord - 1 - k));
+            const int word = d / kPerWord, quarter = word / (N / kPerWord);
+            reinterpret_cast<uint32_t*>(&s_flip[which][quarter * kFlips])[word - quarter * (N / kPerWord)] = m;
+        }
+        for (int i = threadIdx.x; i < 256; i += 128) {
+            const int c = i >> 5, m = c < 4 ? 3 - c : c - 4;
+            const float mag = m == 3 ? kMag3 : (m == 2 ? kMag2 : (m == 1 ? kMag1 : kMag0));
+            s_cent[c][i & 31] = c < 4 ? -mag : mag;
+        }
     }
     __syncthreads();
     pdl_wait_release();
@@ -122,6 +224,7 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     const bool odd = (lane & 4) != 0;
     const int pairs = tokens / 2 + 1;                       // token pairs that `tokens` tokens can touch
     const int per_tensor = n_segs * pairs * heads;
+    const bool keys_here = static_cast<long>(blockIdx.x) * 16 < per_tensor;   // whether the CTA has a key (16 pairs per CTA)
     int unit = static_cast<int>((static_cast<long>(blockIdx.x) * 128 + threadIdx.x) >> 3);
     const bool in_range = unit < 2 * per_tensor;
     unit = in_range ? unit : 2 * per_tensor - 1;
@@ -135,48 +238,88 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     const int src_tok = tok < 0 ? 0 : (tok < tokens ? tok : tokens - 1);
     const InT* const src = (value ? values : keys) + ((static_cast<size_t>(sidx) * tokens + src_tok) * heads + head) * D + q * N;
 
-    float v[N];
-    if (aligned) {
-        constexpr int kPer = 16 / static_cast<int>(sizeof(InT));
+    unsigned long long v[N / 2];   // pairs of dims; the signs are flipped here (squares do not see them)
 #pragma unroll
-        for (int i = 0; i < N / kPer; ++i) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + i);
-            const InT* e = reinterpret_cast<const InT*>(&raw);
+    for (int i = 0; i < N / kPer; ++i) {
+        uint4 raw;
+        if (aligned) {
+            raw = __ldg(reinterpret_cast<const uint4*>(src) + i);
+        } else {
+            InT* const e = reinterpret_cast<InT*>(&raw);
 #pragma unroll
-            for (int j = 0; j < kPer; ++j) v[i * kPer + j] = as_f32<InT>(e[j]);
+            for (int j = 0; j < kPer; ++j) e[j] = src[i * kPer + j];
         }
+        const uint4 m = s_flip[value ? 1 : 0][q * kFlips + i];
+        raw = make_uint4(raw.x ^ m.x, raw.y ^ m.y, raw.z ^ m.z, raw.w ^ m.w);
+        const InT* const e = reinterpret_cast<const InT*>(&raw);
+#pragma unroll
+        for (int j = 0; j < kPer; j += 2) v[(i * kPer + j) / 2] = pack2(as_f32<InT>(e[j]), as_f32<InT>(e[j + 1]));
+    }
+    float norm;
+    if constexpr (SquareSums<D>::kShared) {
+        put_squares<D>(v, s_sums);
+        __syncthreads();
+        if (threadIdx.x < 32) s_sums.sum[lane] = add_squares<D>(s_sums, lane);
+        __syncthreads();
+        norm = __fsqrt_rn(s_sums.sum[threadIdx.x >> 2]);
     } else {
-#pragma unroll
-        for (int j = 0; j < N; ++j) v[j] = as_f32<InT>(src[j]);
+        norm = __fsqrt_rn(quad_square_sum<N>(v, lane));
     }
-    const float norm = __fsqrt_rn(quad_square_sum<N>(v, lane));
     const float inv_norm = (norm > 1e-10f) ? __fdiv_rn(1.0f, norm) : 0.0f;
-    const uint32_t* const signs = s_sign[value ? 1 : 0];
-    auto sign_word = [&](const uint32_t* s, int j) { return s[(q * N + j) >> 5]; };   // of this lane's dim j (N >= 8)
+    const unsigned long long inv_norm2 = pack2(inv_norm, inv_norm);
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-        const uint32_t w = sign_word(signs, j);
-        v[j] = flip_unless(__fmul_rn(v[j], inv_norm), N >= 32 ? w : w >> ((q * N) & 31), j & 31);
-    }
-    quad_fwht<N>(v, q);
+    for (int j = 0; j < N / 2; ++j) v[j] = mul2(v[j], inv_norm2);
+    quad_fwht2<N>(v, q);
+    const unsigned long long inv_sqrt2 = pack2(inv_sqrt, inv_sqrt), scale2 = pack2(scale, scale);
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) v[j] = mul2(mul2(v[j], inv_sqrt2), scale2);
 
-    uint32_t words[W];   // nibbles: code, and for a key the residual's sign in bit 3
+    uint32_t words[W];   // codes as nibbles
 #pragma unroll
     for (int w = 0; w < W; ++w) words[w] = 0u;
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-        const float x = __fmul_rn(__fmul_rn(v[j], inv_sqrt), scale);
-        float r;
-        uint32_t nib = code_of(x, r);
-        v[j] = r;
-        if (!value) {
-            const uint32_t w = sign_word(s_sign[2], j);
-            const bool qpos = ((N >= 32 ? w : w >> ((q * N) & 31)) >> (j & 31)) & 1u;
-            if (qpos ? r > 0.0f : r < 0.0f) nib |= 8u;
-        }
-        words[j / 8] |= nib << (4 * (j & 7));
+    for (int j = 0; j < N / 2; ++j) {
+        const float2 x = unpack2(v[j]);
+        words[j / 4] |= (code_only(x.x) | (code_only(x.y) << 4)) << (8 * (j & 3));
     }
-    const float rnorm = __fsqrt_rn(quad_square_sum<N>(v, lane));   // of the residual; only the keys keep it
+    uint32_t signs[W];   // a key's residual signs, eight bits of a word's dims
+    float rnorm = 0.f;   // the residual's norm; only the keys keep it
+    if (keys_here) {
+        bool plain = true;   // no residual is zero or not a number
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            signs[w] = 0u;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                const int i = 4 * w + j;
+                const float2 x = unpack2(v[i]);
+                const uint32_t two = words[w] >> (8 * j);
+                const float r0 = __fsub_rn(x.x, s_cent[two & 7u][lane]), r1 = __fsub_rn(x.y, s_cent[(two >> 4) & 7u][lane]);
+                plain = plain && fabsf(r0) > 0.0f && fabsf(r1) > 0.0f;
+                signs[w] = __funnelshift_l(__float_as_uint(r1), signs[w], 1);
+                signs[w] = __funnelshift_l(__float_as_uint(r0), signs[w], 1);
+                v[i] = pack2(r0, r1);
+            }
+        }
+        // a bit is set where the residual's sign is the dim's: r > 0 or r < 0
+        auto dims_signs = [&](int w) { return (s_qjl[(q * N + 8 * w) >> 5] >> ((q * N + 8 * w) & 31)) & 0xffu; };
+#pragma unroll
+        for (int w = 0; w < W; ++w) signs[w] ^= dims_signs(w);
+        if (!plain) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 r = unpack2(v[4 * w + j]);
+                    if (!(fabsf(r.x) > 0.0f)) signs[w] &= ~(1u << (2 * j));
+                    if (!(fabsf(r.y) > 0.0f)) signs[w] &= ~(2u << (2 * j));
+                }
+            }
+        }
+        // The last warp adds these up and stores the norms while the others write the codes.
+        if constexpr (SquareSums<D>::kShared) put_squares<D>(v, s_sums);
+        else rnorm = __fsqrt_rn(quad_square_sum<N>(v, lane));
+    }
 
     // The half of the words that the other quad writes, for the half of its words that this one writes (values).  A
     // group is N / 2 dims; D = 32 has half a word in it.
@@ -189,10 +332,21 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
         other[w] = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 4);
     }
     const bool other_live = __shfl_xor_sync(0xffffffffu, live ? 1 : 0, 4) != 0;
-    if (!live && !(value && other_live)) return;
-
     const int slot = token & (kKvTile - 1);
     unsigned char* const block = tab.seg[sidx].base + (static_cast<size_t>(token / kKvTile) * heads + head) * B::kBytes;
+    if constexpr (SquareSums<D>::kShared) {
+        if (keys_here) {
+            if (q == 0) s_norm_at[threadIdx.x >> 2] = live && !value ? reinterpret_cast<float*>(block + B::kNormOff) + kv_residual_norm(slot) : nullptr;
+            __syncthreads();
+            if (threadIdx.x >= 96) {
+                float* const at = s_norm_at[lane];
+                const float sum = add_squares<D>(s_sums, lane);
+                if (at != nullptr) *at = __fsqrt_rn(sum);
+            }
+        }
+    }
+    if (!live && !(value && other_live)) return;
+
     if (value) {
         const bool even_live = odd ? other_live : live, odd_live = odd ? live : other_live;
         const int g = 2 * q + (odd ? 1 : 0);
@@ -217,8 +371,9 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     } else {
         uint32_t* const dst = reinterpret_cast<uint32_t*>(block) + slot * (D / 8) + q * W;
 #pragma unroll
-        for (int w = 0; w < W; ++w)   // code, sign, code, sign -> code, code, sign, sign
-            words[w] = (words[w] & 0x87878787u) | ((words[w] >> 1) & 0x38383838u) | ((words[w] << 3) & 0x40404040u);
+        for (int w = 0; w < W; ++w)   // a byte: two codes, their two signs
+            words[w] = (words[w] & 0x07070707u) | ((words[w] >> 1) & 0x38383838u) | ((signs[w] & 0x03u) << 6) | ((signs[w] & 0x0Cu) << 12) |
+                       ((signs[w] & 0x30u) << 18) | ((signs[w] & 0xC0u) << 24);
         if constexpr (W % 4 == 0) {
 #pragma unroll
             for (int w = 0; w < W; w += 4) *reinterpret_cast<uint4*>(dst + w) = make_uint4(words[w], words[w + 1], words[w + 2], words[w + 3]);
@@ -230,7 +385,7 @@ __global__ void __launch_bounds__(128) kv_encode_kernel(const InT* __restrict__ 
     if (q == 0 && live) {
         float* const norms = reinterpret_cast<float*>(block + B::kNormOff);
         norms[value ? kv_value_norm(slot) : kv_key_norm(slot)] = norm;
-        if (!value) norms[kv_residual_norm(slot)] = rnorm;
+        if (!SquareSums<D>::kShared && !value) norms[kv_residual_norm(slot)] = rnorm;
     }
 }
 
