@@ -39,3 +39,28 @@ def test_long_appends_store_what_short_ones_do(tq, dim, dtype, first, tokens, he
     for name in a:
         if name != "tokens":
             assert np.array_equal(a[name], b[name], equal_nan=a[name].dtype == np.float32), name
+
+
+@pytest.mark.parametrize("dim", [32, 64, 128, 256, 512])
+@pytest.mark.parametrize("heads", [1, 3])
+def test_decoded_ranges_of_any_length_and_place(tq, dim, heads):
+    """Results that do not fill a warp's eight vectors, and ones that are not on a 16-byte boundary: the same bits."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    k = torch.randn((101, heads, dim), generator=g, device="cuda").half()
+    v = torch.randn((101, heads, dim), generator=g, device="cuda").half()
+    cache = tq.TQKVCache(1, heads, dim)
+    cache.append(0, k, v)
+    for get, src in ((cache.get_keys_fp16, k), (cache.get_values_fp16, v)):
+        whole = torch.empty((101, heads, dim), device="cuda", dtype=torch.float16)
+        get(0, 0, 101, out=whole)
+        assert float((whole.double() - src.double()).norm() / src.double().norm()) < 0.25   # three bits
+        for start, end in ((0, 1), (5, 6), (3, 12), (16, 33), (100, 101), (1, 100)):
+            n = (end - start) * heads * dim
+            room = torch.full((n + 16,), 3.0, device="cuda", dtype=torch.float16)
+            for at in (0, 1, 8):
+                room.fill_(3.0)
+                out = room[at:at + n].view(end - start, heads, dim)
+                get(0, start, end, out=out)
+                assert torch.equal(out, whole[start:end])
+                assert bool((room[:at] == 3).all()) and bool((room[at + n:] == 3).all())

@@ -21,33 +21,7 @@ template <>
 __device__ __forceinline__ float as_f32<__half>(__half v) { return __half2float(v); }
 
 // A vector is handled by four neighbouring lanes, lane q holding dims [q N, (q + 1) N), N = D / 4: the quarter whose
-// storage words are its own too, so nothing but two butterfly stages and the running sums crosses lanes.
-template <int N>
-__device__ __forceinline__ void quad_fwht(float (&v)[N], int q) {
-#pragma unroll
-    for (int h = 1; h < N; h <<= 1) {
-#pragma unroll
-        for (int i = 0; i < N; i += 2 * h) {
-#pragma unroll
-            for (int j = i; j < i + h; ++j) {
-                const float a = v[j], b = v[j + h];
-                v[j] = __fadd_rn(a, b);
-                v[j + h] = __fsub_rn(a, b);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-        const bool upper = (q & m) != 0;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[j], m);
-            v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
-        }
-    }
-}
-
-// The same on pairs of neighbouring dims.
+// storage words are its own too, so nothing but two butterfly stages crosses lanes.  Pairs of neighbouring dims.
 template <int N>
 __device__ __forceinline__ void quad_fwht2(unsigned long long (&v)[N / 2], int q) {
 #pragma unroll
@@ -531,22 +505,28 @@ __global__ void __launch_bounds__(64) kv_encode_few_kernel(const InT* __restrict
 
 // ---- range decoder (src/kv_cache.cpp:292-365) ----------------------------------------------------------
 // Four lanes per vector as in the encoder.  The centroids sit in shared memory once per lane: as a constant array they
-// were read one lane at a time (86 us for 65536 tokens of 4 heads).
+// were read one lane at a time (86 us for 65536 tokens of 4 heads).  A warp's eight vectors are contiguous in the result: they
+// leave through shared memory, in pieces of 16 bytes whose places within a lane's are turned by the lane and the vector
+// (no bank conflicts at 128 dims).  8192 tokens of 4 heads of 128: 6.7 us with a dim per instruction and stores 64 bytes apart,
+// 5.4 so; heads of 256 17.4 and 6.6.
 template <int D>
 __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __restrict__ base, int start, long n_vec, int heads, int values,
                                                         uint32_t wht_seed, float inv_scale, float inv_sqrt, __half* __restrict__ out) {
     constexpr int N = D / 4, W = N / 8;
     using B = KvBlock<D>;
+    constexpr int kPieces = N / 8, kFlips = kPieces + 1;    // 16-byte pieces of a lane's result; of a quarter's signs, and one for the banks' sake
     __shared__ float s_cent[8][32];
-    __shared__ uint32_t s_sign[D / 32];
+    __shared__ __align__(16) uint4 s_flip[4 * kFlips];      // rotation signs, as the halves' sign bits
+    __shared__ __align__(16) uint4 s_out[4][32 * kPieces];
     for (int i = threadIdx.x; i < 256; i += 128) {
         const int c = i >> 5, m = c < 4 ? 3 - c : c - 4;
         const float mag = m == 3 ? kMag3 : (m == 2 ? kMag2 : (m == 1 ? kMag1 : kMag0));
         s_cent[c][i & 31] = __fmul_rn(c < 4 ? -mag : mag, inv_scale);
     }
-    for (int i = threadIdx.x; i < D; i += 128) {
-        const uint32_t bits = __ballot_sync(0xffffffffu, sign_is_positive(wht_seed, static_cast<uint32_t>(i)));
-        if ((i & 31) == 0) s_sign[i >> 5] = bits;
+    for (int i = threadIdx.x; i < D / 2; i += 128) {
+        const int quarter = i / (N / 2);
+        reinterpret_cast<uint32_t*>(&s_flip[quarter * kFlips])[i - quarter * (N / 2)] =
+            (sign_is_positive(wht_seed, static_cast<uint32_t>(2 * i)) ? 0u : 0x8000u) | (sign_is_positive(wht_seed, static_cast<uint32_t>(2 * i + 1)) ? 0u : 0x80000000u);
     }
     __syncthreads();
     pdl_wait_release();
@@ -589,21 +569,43 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __r
         }
     }
     const float norm = reinterpret_cast<const float*>(block + B::kNormOff)[values ? kv_value_norm(slot) : kv_key_norm(slot)];
-    quad_fwht<N>(v, q);
-    __align__(16) __half h[N];
+    unsigned long long p[N / 2];
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-        const uint32_t w = s_sign[(q * N + j) >> 5];
-        h[j] = __float2half_rn(__fmul_rn(flip_unless(__fmul_rn(v[j], inv_sqrt), N >= 32 ? w : w >> ((q * N) & 31), j & 31), norm));
+    for (int j = 0; j < N / 2; ++j) p[j] = pack2(v[2 * j], v[2 * j + 1]);
+    quad_fwht2<N>(p, q);
+    const unsigned long long inv_sqrt2 = pack2(inv_sqrt, inv_sqrt), norm2 = pack2(norm, norm);
+    uint4 h[kPieces];
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 t = unpack2(mul2(mul2(p[4 * c + j], inv_sqrt2), norm2));
+            const __half2 r = __floats2half2_rn(t.x, t.y);
+            w[j] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        const uint4 m = s_flip[q * kFlips + c];
+        h[c] = make_uint4(w[0] ^ m.x, w[1] ^ m.y, w[2] ^ m.z, w[3] ^ m.w);
     }
-    if (!live) return;
-    __half* const dst = out + static_cast<size_t>(vec) * D + q * N;
+    const int in_warp = lane >> 2;   // which of the warp's vectors
+    auto place = [](int vector, int quarter, int piece) { return (vector * 4 + quarter) * kPieces + ((piece + quarter + vector) & (kPieces - 1)); };
     if (reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+        uint4* const mine = s_out[threadIdx.x >> 5];
 #pragma unroll
-        for (int c = 0; c < N / 8; ++c) reinterpret_cast<uint4*>(dst)[c] = reinterpret_cast<const uint4*>(h)[c];
-    } else {
+        for (int c = 0; c < kPieces; ++c) mine[place(in_warp, q, c)] = h[c];
+        __syncwarp();
+        const long first = quad - in_warp;
+        uint4* const dst = reinterpret_cast<uint4*>(out) + first * (4 * kPieces);
 #pragma unroll
-        for (int j = 0; j < N; ++j) dst[j] = h[j];
+        for (int k = 0; k < kPieces; ++k) {
+            const int i = 32 * k + lane, vector = i / (4 * kPieces), r = i - vector * (4 * kPieces);
+            if (first + vector < n_vec) dst[i] = mine[place(vector, r / kPieces, r & (kPieces - 1))];
+        }
+    } else if (live) {
+        const __half* const e = reinterpret_cast<const __half*>(h);
+        __half* const dst = out + static_cast<size_t>(vec) * D + q * N;
+#pragma unroll
+        for (int j = 0; j < N; ++j) dst[j] = e[j];
     }
 }
 
