@@ -289,7 +289,7 @@ public:
         tq::GemmGroupItem it{};
         it.codes = codes_.as<uint8_t>(); it.norms = norms_.as<float>(); it.table = tables_.as<float>();
         it.y = static_cast<__half*>(y);
-        it.out = out_; it.in = in_; it.block = block_; it.n_planes = planes;
+        it.out = out_; it.in = in_; it.block = block_; it.n_planes = planes; it.pair_unit = pair_unit_;
         it.seed_p = seed_p_; it.seed_r = seed_r_;
         it.scratch = gemm_scratch_.as<void>(); it.status = d_status_;
         return it;
@@ -482,7 +482,7 @@ private:
             const int planes = dual_ ? 2 : 1;
             gemm_scratch_.reserve(tq::gemm_scratch_bytes(out_, in_, batch, planes, sm_count_), st);
             tq::launch_tq8_gemm(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), d_x, d_y, out_, in_, batch,
-                                block_, planes, seed_p_, seed_r_, gemm_scratch_.as<void>(), d_status_,
+                                block_, planes, pair_unit_, seed_p_, seed_r_, gemm_scratch_.as<void>(), d_status_,
                                 sm_count_, st, y_stride);
             return;
         }

@@ -8,8 +8,8 @@
 // Same algebra as the decode kernel: the activation is rotated once (forward WHT of every block
 // of every row, written as fp16 by rotate_rows_f16_kernel), and the weight side is a table
 // lookup per code:   y[m, r] = norm[r] * inv_scale * sum_j table[code[r, j]] * xrot[m, j].
-// Dual-rotation weights run as two passes over K into the same accumulator (primary table
-// against x rotated with the primary seed, residual table against x rotated with the residual
+// Dual-rotation weights run as twice the K into the same accumulator (primary centroids
+// against x rotated with the primary seed, residual centroids against x rotated with the residual
 // seed).
 //
 // One CTA computes a 128 (weight rows) x 256 (activation rows, or fewer) tile of y^T:
@@ -76,14 +76,12 @@ constexpr int kCopyWarp = kProducerWarps + 1;  // issues the activation-tile bul
 constexpr int kEpilogueWarp = kProducerWarps + 2;  // first of four warps that drain the accumulators
 constexpr int kEpilogueWarps = 4;
 constexpr int kGemmThreads = kProducerThreads + 64 + 32 * kEpilogueWarps;
-constexpr uint32_t kLutBytes = 256 * 32 * 4;           // one plane: 256 entries x 32 lane copies x (fp16, fp16)
+constexpr uint32_t kLutBytes = 256 * 32 * 4;           // 256 entries x 32 lane copies x two fp16
 constexpr uint32_t kTmemCols = 512;   // accumulators: columns 0..255 (two of up to 128 columns, or one); weight tiles: 4 stages x 64 columns from 256 on
 constexpr uint32_t kTmemAColumn = 256;
 constexpr uint32_t kTmemASubCols = kBlockK / 2;                    // one K block: two fp16 per 32-bit column
 constexpr uint32_t kTmemAStageCols = kSubPerStage * kTmemASubCols;
 constexpr uint32_t kLutWin = 0x800u;  // window address of the lookup tables (an immediate of the lookup's load)
-// rings + tables (4 activation stages with one table plane, 3 with two) + worst-case padding in
-// front of the 32 KB-aligned tables
 // Everything an SM can give one CTA: tables at kLutWin, then three 64 KB stages for a 256-row tile.
 constexpr size_t kGemmSmemBytes = 232448 - 512;
 constexpr unsigned long long kGemmWaitLimitNs = 200ull * 1000 * 1000;
@@ -129,7 +127,7 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
            (static_cast<uint64_t>(1024u >> 4) << 32) | (1ull << 46);
 }
 
-// Table lookup: `offset` = scaled code | lane offset | plane offset; the table's window address is the immediate.
+// Table lookup: `offset` = scaled code | lane offset; the table's window address is the immediate.
 __device__ __forceinline__ uint32_t lut_load(uint32_t offset) {
     uint32_t v;
     asm("ld.shared.b32 %0, [%1 + 2048];" : "=r"(v) : "r"(offset));
@@ -158,6 +156,13 @@ __device__ __forceinline__ void tmem_st_16x256b(uint32_t taddr, const uint32_t (
         : "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
           "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
+}
+// The same, two blocks of 8 columns.
+__device__ __forceinline__ void tmem_st_16x256b(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :
+                 : "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 // Codes are read once per 256 activation rows: they pass by the first-level cache.
 __device__ __forceinline__ uint4 load_codes16(const uint8_t* p) {
@@ -481,7 +486,7 @@ __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const _
 struct GemmArgs {
     const uint8_t* codes;   // joint bytes in 16 x 64 tiles (code_offset)
     const float* norms;     // [out]
-    const float* table;     // [n_planes, 256] fp32
+    const float* table;     // [256] fp32; two rotations: [256] pairs of fp16
     const __half* xrot;     // rotated activation in operand-tile order (see rotate_rows_f16_kernel)
     __half* y;              // [m, out], activation rows y_stride elements apart
     long y_stride;
@@ -495,6 +500,13 @@ struct GemmArgs {
 // One CTA's work: K split bz of the output tiles t0, t0 + t_step, ... < t_end of matrix p.  Tile t is row tile t / n_tok,
 // token tile t % n_tok: CTAs that run side by side share the codes of a few row tiles, which then come from HBM once however
 // many token tiles there are.
+//
+// DUAL: weights with two rotations.  A table word holds both centroids of a byte as a pair of fp16, divided by the unit that inv_scale
+// carries, and a stage is ONE 64-column block of codes: its first K block are the primary centroids, against x rotated with the
+// primary seed, its second the residual ones.  A lookup serves both (as two planes one after the other the codes were read and looked up
+// twice: 3584 x 3584, block 512, 20.2 us at 64 rows, 31.6 at 256 and 116 at 2048; 16.7, 24.8 and 93 so.  18944 x 3584 at 64 rows 50.7
+// and 39.6.)
+template <bool DUAL>
 __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const int t_step, const int t_end, const int bz) {
     extern __shared__ __align__(128) uint8_t gemm_smem[];
     __shared__ __align__(8) unsigned long long s_full[kStagesMax], s_empty[kStagesMax], s_accum_full[2], s_accum_empty[2];
@@ -511,13 +523,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     const int n_local = t0 < t_end ? (t_end - t0 + t_step - 1) / t_step : 0;
 
     // ---- shared-memory map -------------------------------------------------------------------
-    // [kLutWin, + 32 KB per plane)  lookup tables, at a fixed window address (it is an immediate of
+    // [kLutWin, + 32 KB)            lookup table, at a fixed window address (it is an immediate of
     //                               the lookup's load instruction)
-    // [after the tables, end)       activation stages of two 64-column pieces, as many as fit, at most kStagesMax
+    // [after the table, end)        activation stages of two 64-column pieces, as many as fit, at most kStagesMax
     const uint32_t raw = smem_addr(gemm_smem);
     uint32_t dyn_bytes;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
-    const uint32_t stage0 = kLutWin + kLutBytes * static_cast<uint32_t>(p.n_planes);
+    const uint32_t stage0 = kLutWin + kLutBytes;
     const uint32_t piece_bytes = static_cast<uint32_t>(n_max) * (kBlockK * 2);   // a 64-column piece: a tile's first n_max rows are contiguous
     const uint32_t stage_bytes = kSubPerStage * piece_bytes;
     const uint32_t smem_end = raw + dyn_bytes;
@@ -548,11 +560,11 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // lookup tables: entry e, lane copy l at kLutWin + plane * 32 KB + e * 128 + l * 4, value (t, t) as fp16
-    for (int i = tid; i < 256 * 8 * p.n_planes; i += kGemmThreads) {
-        const int e = i >> 3, c4 = (i & 7) * 4;  // e counts across planes
-        const __half h = __float2half_rn(__ldg(p.table + e));
-        const uint32_t v = static_cast<uint32_t>(__half_as_ushort(h)) * 0x00010001u;
+    // lookup table: entry e, lane copy l at kLutWin + e * 128 + l * 4, value (t, t) or (primary, residual) as fp16
+    for (int i = tid; i < 256 * 8; i += kGemmThreads) {
+        const int e = i >> 3, c4 = (i & 7) * 4;
+        const float t = __ldg(p.table + e);
+        const uint32_t v = DUAL ? __float_as_uint(t) : static_cast<uint32_t>(__half_as_ushort(__float2half_rn(t))) * 0x00010001u;
         asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kLutWin + static_cast<uint32_t>(e) * 128u + c4 * 4u), "r"(v)
                      : "memory");
     }
@@ -562,14 +574,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     const uint32_t tmem_d = s_tmem_base;
     volatile unsigned int* abort_flag = &s_abort;
 
-    // K blocks (64 columns) of this CTA: a contiguous range of the (plane-major) list of all K blocks.
-    // A stage is two consecutive K blocks of the range (the last one may hold a single block).  The stages of the CTA's
-    // tiles follow one another through the ring.
+    // Blocks of 64 columns of this CTA: a contiguous range.  A stage is two consecutive ones (the last one may be alone; with
+    // two rotations one block and both its K blocks).  The stages of the CTA's tiles follow one another through the ring.
     const int kb_per_plane = p.in / kBlockK;
-    const int n_kb_total = kb_per_plane * p.n_planes;
-    const int kb_base = static_cast<int>(static_cast<long>(n_kb_total) * bz / p.k_splits);
-    const int n_kb = static_cast<int>(static_cast<long>(n_kb_total) * (bz + 1) / p.k_splits) - kb_base;
-    const int n_it = (n_kb + kSubPerStage - 1) / kSubPerStage;
+    constexpr int kBlocksPerStage = DUAL ? 1 : kSubPerStage;
+    const int kb_base = static_cast<int>(static_cast<long>(kb_per_plane) * bz / p.k_splits);
+    const int n_kb = static_cast<int>(static_cast<long>(kb_per_plane) * (bz + 1) / p.k_splits) - kb_base;
+    const int n_it = (n_kb + kBlocksPerStage - 1) / kBlocksPerStage;
 
     if (warp < kProducerWarps) {
         // ---- producers ------------------------------------------------------------------------
@@ -577,19 +588,22 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         // column, 128 K columns).  A warp may touch lanes 32 * (warp % 4) .. + 31.  The 16 producer
         // warps form two groups of eight (warp / 8); inside a group warp w takes the rows of lane
         // quarter w % 4 and the K block (w / 4) % 2 of the stage; group g dequantises the stages g,
-        // g + 2, ...  A thread turns 64 codes, 16 of each of four rows, into fp16 pairs.
-        const int sub = (warp >> 2) & 1;             // which K block of the stage
+        // g + 2, ...  A thread turns 64 codes, 16 of each of four rows, into fp16 pairs.  (With two rotations the two warps
+        // of a lane quarter take 16 of its rows each, and 32 codes a thread make as many pairs.)
+        const int sub = (warp >> 2) & 1;             // which K block of the stage, or which 16 rows
+        constexpr int kLoads = DUAL ? 2 : 4;
         const int grp = warp >> 3;
         // The warp's rows are two code tiles of 16 x 64 bytes; lane (g, q) takes bytes 16 q .. of rows g and g + 8 of each:
         // a load of the warp is 512 contiguous bytes.  Tiles past the matrix repeat the last one (never stored).
         const int last_tile = (p.out - 1) >> 4;
         const size_t tile_row_bytes = static_cast<size_t>(code_tiles_per_row(p.in)) * kCodeTileBytes;
         const uint8_t* const code_lane = p.codes + (lane >> 2) * 64 + 16 * (lane & 3);
-        const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + kTmemAColumn + kTmemASubCols * static_cast<uint32_t>(sub);
+        const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3) + (DUAL ? 16 * sub : 0)) << 16) + kTmemAColumn +
+                                 (DUAL ? 0u : kTmemASubCols * static_cast<uint32_t>(sub));
         const int n_stages = n_local * n_it;
 
         // The group's next stage to fetch: place in its tile, codes of its two code tiles, stages left.  Two of the group's
-        // stages are in registers or on their way; the second plane reads the same bytes again.
+        // stages are in registers or on their way.
         int f_it = grp, f_t = t0, f_left = n_stages - grp;
         const uint8_t *f_ptr0, *f_ptr1;
         auto carry = [&](int& it, int& t) {   // past the tile's last stage: the same place of the next tiles
@@ -599,35 +613,36 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             }
         };
         auto fetch_place = [&] {
-            const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3);
-            int kb = kb_base + kSubPerStage * f_it + sub;
-            if (kb >= kb_per_plane) kb -= kb_per_plane;
+            const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3) + (DUAL ? sub : 0);
+            const int kb = kb_base + kBlocksPerStage * f_it + (DUAL ? 0 : sub);
             f_ptr0 = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
-            f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
+            if constexpr (!DUAL) f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
         };
-        auto fetch = [&](uint4 (&c)[4]) {
-            const int kb = kSubPerStage * f_it + sub;
+        auto fetch = [&](uint4 (&c)[kLoads]) {
+            const int kb = kBlocksPerStage * f_it + (DUAL ? 0 : sub);
             if (f_left > 0 && kb < n_kb) {
                 c[0] = load_codes16(f_ptr0);
                 c[1] = load_codes16(f_ptr0 + 512);
-                c[2] = load_codes16(f_ptr1);
-                c[3] = load_codes16(f_ptr1 + 512);
+                if constexpr (!DUAL) {
+                    c[2] = load_codes16(f_ptr1);
+                    c[3] = load_codes16(f_ptr1 + 512);
+                }
             }
             f_left -= kGroups;
             f_it += kGroups;
-            f_ptr0 += kGroups * kSubPerStage * kCodeTileBytes;
-            f_ptr1 += kGroups * kSubPerStage * kCodeTileBytes;
-            // another tile, or possibly the second plane: place the pointers anew
-            if (f_it >= n_it || p.n_planes == 2) {
+            f_ptr0 += kGroups * kBlocksPerStage * kCodeTileBytes;
+            if constexpr (!DUAL) f_ptr1 += kGroups * kBlocksPerStage * kCodeTileBytes;
+            // another tile: place the pointers anew
+            if (f_it >= n_it) {
                 if (f_left > 0) {
                     carry(f_it, f_t);
                     fetch_place();
                 }
             }
         };
-        uint4 buf0[4], buf1[4];
+        uint4 buf0[kLoads], buf1[kLoads];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) buf0[i] = buf1[i] = make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < kLoads; ++i) buf0[i] = buf1[i] = make_uint4(0, 0, 0, 0);
         carry(f_it, f_t);
         fetch_place();
         fetch(buf0);
@@ -636,35 +651,57 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         carry(it, unused_t);
         int slot = grp % n_st, use = grp / n_st;     // ring slot of stage `it` and how often it has been used before
         // One stage; false once a wait has run out.
-        auto produce = [&](uint4 (&c0)[4]) {
-            const int kb = kSubPerStage * it + sub;
-            const bool have = kb < n_kb;             // the last stage of a tile may lack its second K block
-            const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
-            // lane offset, plus 32 KB for the second plane's table: bits outside the scaled code (7..14)
-            const uint32_t lane_c = static_cast<uint32_t>(lane) * 4u + static_cast<uint32_t>(plane) * kLutBytes;
+        auto produce = [&](uint4 (&c0)[kLoads]) {
+            const bool have = DUAL || kSubPerStage * it + sub < n_kb;   // the last stage of a tile may lack its second K block
+            const uint32_t lane_c = static_cast<uint32_t>(lane) * 4u;   // bits outside the scaled code (7..14)
             const uint32_t st_addr = a_taddr + kTmemAStageCols * static_cast<uint32_t>(slot);
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                // code tile `half`: 16 codes of row g and of row g + 8 -> fp16 pairs, word i of a row's four in column block i
-                const uint32_t w[8] = {c0[2 * half].x, c0[2 * half].y, c0[2 * half].z, c0[2 * half].w,
-                                       c0[2 * half + 1].x, c0[2 * half + 1].y, c0[2 * half + 1].z, c0[2 * half + 1].w};
-                uint32_t packed[16];
-#pragma unroll
-                for (int h = 0; h < 16; ++h) {
-                    const uint32_t word = w[4 * ((h >> 1) & 1) + (h >> 2)];
-                    const int b0 = (h & 1) * 2;  // bytes b0, b0 + 1 of the word
-                    // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
-                    packed[h] = __byte_perm(lut_load(__dp4a(word, 128u << (8 * b0), lane_c)), lut_load(__dp4a(word, 128u << (8 * b0 + 8), lane_c)), 0x5410);
-                }
-                // the codes are used up: the stage after next into the same registers
-                if (half == 1) fetch(c0);
-                // the slot must have been read by the MMAs of its previous stage
-                if (half == 0 && use > 0 && !__all_sync(0xffffffffu, bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag))) {
+            // the slot must have been read by the MMAs of its previous stage
+            auto slot_free = [&] {
+                if (use > 0 && !__all_sync(0xffffffffu, bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag))) {
                     raise_status(p.status, 6u);
                     atomicExch(&s_abort, 1u);
                     return false;
                 }
-                if (have) tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
+                return true;
+            };
+            // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
+            auto entry = [&](uint32_t word, int byte) { return lut_load(__dp4a(word, 128u << (8 * byte), lane_c)); };
+            if constexpr (DUAL) {
+                // half a block's columns at a time: words i = 2 half and 2 half + 1 of either row, both planes
+                const uint32_t w[8] = {c0[0].x, c0[0].y, c0[0].z, c0[0].w, c0[1].x, c0[1].y, c0[1].z, c0[1].w};
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t first[8], second[8];
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) {
+                        const uint32_t word = w[4 * ((h >> 1) & 1) + 2 * half + (h >> 2)];
+                        const int b0 = (h & 1) * 2;
+                        const uint32_t e0 = entry(word, b0), e1 = entry(word, b0 + 1);
+                        first[h] = __byte_perm(e0, e1, 0x5410);
+                        second[h] = __byte_perm(e0, e1, 0x7632);
+                    }
+                    if (half == 1) fetch(c0);   // the codes are used up: the stage after next into the same registers
+                    if (half == 0 && !slot_free()) return false;
+                    tmem_st_16x256b(st_addr + 16u * half, first);
+                    tmem_st_16x256b(st_addr + kTmemASubCols + 16u * half, second);
+                }
+            } else {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    // code tile `half`: 16 codes of row g and of row g + 8 -> fp16 pairs, word i of a row's four in column block i
+                    const uint32_t w[8] = {c0[2 * half].x, c0[2 * half].y, c0[2 * half].z, c0[2 * half].w,
+                                           c0[2 * half + 1].x, c0[2 * half + 1].y, c0[2 * half + 1].z, c0[2 * half + 1].w};
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int h = 0; h < 16; ++h) {
+                        const uint32_t word = w[4 * ((h >> 1) & 1) + (h >> 2)];
+                        const int b0 = (h & 1) * 2;  // bytes b0, b0 + 1 of the word
+                        packed[h] = __byte_perm(entry(word, b0), entry(word, b0 + 1), 0x5410);
+                    }
+                    if (half == 1) fetch(c0);   // the codes are used up: the stage after next into the same registers
+                    if (half == 0 && !slot_free()) return false;
+                    if (have) tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
+                }
             }
             // every lane waits for its own stores, then one arrival per warp
             tmem_st_publish();
@@ -702,13 +739,12 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                         break;
                     }
                     ++filled;
-                    const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
+                    const int nsub = DUAL ? kSubPerStage : min(kSubPerStage, n_kb - kSubPerStage * it);
                     const uint32_t bar = bar_full + 8u * slot;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(b_bytes * nsub) : "memory");
                     for (int sb = 0; sb < nsub; ++sb) {
-                        const int kb = kSubPerStage * it + sb;
-                        const int plane = (kb_base + kb) >= kb_per_plane ? 1 : 0;
-                        const size_t tile = (static_cast<size_t>(plane) * n_tok + t % n_tok) * kb_per_plane + (kb_base + kb - plane * kb_per_plane);
+                        const size_t tile = DUAL ? (static_cast<size_t>(sb) * n_tok + t % n_tok) * kb_per_plane + (kb_base + it)
+                                                 : static_cast<size_t>(t % n_tok) * kb_per_plane + (kb_base + kSubPerStage * it + sb);
                         const __half* src = p.xrot + tile * (kTileTok * kBlockK);
                         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                                          stage0 + static_cast<uint32_t>(slot) * stage_bytes + static_cast<uint32_t>(sb) * piece_bytes),
@@ -747,7 +783,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const int nsub = min(kSubPerStage, n_kb - kSubPerStage * it);
+                    const int nsub = DUAL ? kSubPerStage : min(kSubPerStage, n_kb - kSubPerStage * it);
                     const uint32_t a_tmem = tmem_d + kTmemAColumn + kTmemAStageCols * static_cast<uint32_t>(slot);
                     const uint32_t b_stage = stage0 + static_cast<uint32_t>(slot) * stage_bytes;
 #pragma unroll
@@ -829,9 +865,10 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
 }
 
 // gridDim.x CTAs walk the output tiles, gridDim.y = K splits.
+template <bool DUAL>
 __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_kernel(const GemmArgs p) {
     const int n_tiles = ((p.out + kTileRows - 1) / kTileRows) * ((p.m + kTileTok - 1) / kTileTok);
-    gemm_body(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
+    gemm_body<DUAL>(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
 }
 
 // Several matrices that multiply the same activation rows (q / k / v, gate / up) in one launch: gridDim.x is cut into
@@ -843,13 +880,14 @@ struct GemmGroupArgs {
     int tile_start[kMaxGemmGroup + 1];   // row tiles tile_start[i] .. tile_start[i + 1] - 1 belong to matrix i
     int n;
 };
+template <bool DUAL>
 __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const __grid_constant__ GemmGroupArgs grp) {
     const int b = static_cast<int>(blockIdx.x);
     int i = 0;
     while (i + 1 < grp.n && b >= grp.tile_start[i + 1]) ++i;
     if (static_cast<int>(blockIdx.z) >= grp.m[i].k_splits) return;
     const int t = (b - grp.tile_start[i]) * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y);
-    gemm_body(grp.m[i], t, 1, t + 1, static_cast<int>(blockIdx.z));
+    gemm_body<DUAL>(grp.m[i], t, 1, t + 1, static_cast<int>(blockIdx.z));
 }
 
 // y = fp16(norm * inv_scale * sum over K splits, in split order) - fixed order, run-to-run identical - for the matrices of a call
@@ -995,7 +1033,7 @@ size_t gemm_scratch_bytes(int out, int in, long m, int n_planes, int sm_count) {
 bool gemm_supported(int in) { return in % kBlockK == 0; }
 
 void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y, int out,
-                     int in, long m, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r, void* scratch,
+                     int in, long m, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p, uint32_t seed_r, void* scratch,
                      unsigned int* status, int sm_count, cudaStream_t stream, long y_stride) {
     if (y_stride <= 0) y_stride = out;
     TQ_REQUIRE(y_stride >= out, "tq8_gemm: output row stride smaller than the layer's rows");
@@ -1019,6 +1057,10 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     a.codes = codes; a.norms = norms; a.table = table; a.xrot = xrot; a.y = y; a.y_stride = y_stride; a.status = status;
     a.out = out; a.in = in; a.m = static_cast<int>(m); a.n_planes = n_planes;
     a.inv_scale = 1.0f / std::sqrt(static_cast<float>(in));
+    if (n_planes == 2) {
+        a.table += 512;   // (the pairs, behind the two tables)
+        a.inv_scale *= pair_unit;
+    }
     a.k_splits = gemm_k_splits(out, in, m, n_planes, sm_count);
     a.partial = a.k_splits > 1 ? reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + xrot_bytes(in, m, n_planes)) : nullptr;
     // stages + tables + worst-case padding in front of the 32 KB-aligned tables
@@ -1027,15 +1069,15 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kGemmSmemBytes)));
+        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
+        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
     // a CTA per SM walks the tiles (with a K split there are fewer tiles x splits than SMs)
     const long n_tiles = static_cast<long>((out + kTileRows - 1) / kTileRows) * ((m + kTileTok - 1) / kTileTok);
     TQ_REQUIRE(n_tiles < (1L << 31), "tq8_gemm: too many output tiles");
     const dim3 grid(static_cast<unsigned int>(std::min<long>(n_tiles, sm_count)), static_cast<unsigned int>(a.k_splits));
-    launch_pdl(tq8_gemm_kernel, grid, dim3(kGemmThreads), smem, stream, a);
+    launch_pdl(n_planes == 2 ? tq8_gemm_kernel<true> : tq8_gemm_kernel<false>, grid, dim3(kGemmThreads), smem, stream, a);
     TQ_CUDA(cudaGetLastError());
     FinishArgs fin{};
     int n_fin = 0;
@@ -1069,6 +1111,10 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         a.xrot = static_cast<__half*>(it.scratch);
         a.out = it.out; a.in = in; a.m = static_cast<int>(m); a.n_planes = n_planes;
         a.inv_scale = 1.0f / std::sqrt(static_cast<float>(in));
+        if (n_planes == 2) {
+            a.table += 512;
+            a.inv_scale *= it.pair_unit;
+        }
         // the split a matrix would get alone, not one for the group as a whole: with fewer splits the group ran 7-9 %
         // faster (16 / 64 rows) but the fp32 sums changed their order, and results would no longer be bit-equal to
         // separate calls
@@ -1088,12 +1134,13 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
+        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
+        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
     const dim3 grid(static_cast<unsigned int>(grp.tile_start[n]), static_cast<unsigned int>((m + kTileTok - 1) / kTileTok),
                     static_cast<unsigned int>(max_splits));
-    launch_pdl(tq8_gemm_group_kernel, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, grp);
+    launch_pdl(n_planes == 2 ? tq8_gemm_group_kernel<true> : tq8_gemm_group_kernel<false>, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, grp);
     // 3. the split-K sums
     launch_finish(fin, n_fin, static_cast<int>(m), sm_count, stream);
 }

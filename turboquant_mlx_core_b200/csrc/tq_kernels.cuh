@@ -120,7 +120,7 @@ int gemm_k_splits(int out, int in, long m, int n_planes, int sm_count);
 size_t gemm_scratch_bytes(int out, int in, long m, int n_planes, int sm_count);
 // y_stride: elements between consecutive activation rows of y (0 = out).
 void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y, int out,
-                     int in, long m, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r, void* scratch,
+                     int in, long m, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p, uint32_t seed_r, void* scratch,
                      unsigned int* status, int sm_count, cudaStream_t stream, long y_stride = 0);
 // Several matrices against the same activation rows in one rotation launch, one GEMM launch and one split-K finish:
 // y of matrix i = its own [m, out_i] buffer.  The matrices share in_features, the WHT block and the rotation mode; each
@@ -133,6 +133,7 @@ struct GemmGroupItem {
     int out, in;
     uint32_t block;
     int n_planes;
+    float pair_unit;
     uint32_t seed_p, seed_r;
     void* scratch;
     unsigned int* status;
