@@ -1032,6 +1032,24 @@ __global__ void peer_wait_kernel(const unsigned int* __restrict__ flags, int n, 
     }
 }
 
+// The wait that the decode kernel makes before it reads an activation that comes out of an exchange (see ScatterArgs), for a
+// rotation that runs in front of it: bounded, and the epoch stays for the decode kernel to advance.
+__global__ void gather_wait_kernel(const unsigned int* __restrict__ flags, int n, const unsigned int* __restrict__ wait_epoch, unsigned int* status) {
+    const int lane = threadIdx.x;
+    if (lane >= n) return;
+    const unsigned int want = *reinterpret_cast<const volatile unsigned int*>(wait_epoch) + 1u;
+    const unsigned long long t0 = global_timer_ns();
+    for (unsigned int spin = 0;; ++spin) {
+        unsigned int v;
+        asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(flags + lane) : "memory");
+        if (static_cast<int>(v - want) >= 0) return;
+        if ((spin & 255u) == 255u && global_timer_ns() - t0 > 5ull * kWaitLimitNs) {   // 1 s: a peer is gone
+            raise_status(status, 10u);
+            return;
+        }
+    }
+}
+
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
 // Warps that share one 16-row tile (a power of two up to 16); a chunk is that many 256-column slices, and
@@ -1206,7 +1224,11 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     const int n_attr = 1;
 
-    // 1. rotate the activation (one warp per plane x row x block)
+    // 1. rotate the activation, once the exchange that it may come from is complete
+    if (!fused_rotation && sa.n_wait > 0 && !sa.ll) {
+        gather_wait_kernel<<<1, 32, 0, stream>>>(sa.wait_flags, sa.n_wait, sa.wait_epoch, status);
+        TQ_CUDA(cudaGetLastError());
+    }
     if (n_planes == 2) launch_rotate_x_pair(x, xrot, in, batch, block, seed_p, seed_r, stream);
     else if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, 1, seed_p, seed_r, stream);
     // 2. the GEMV itself
