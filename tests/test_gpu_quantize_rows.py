@@ -1,4 +1,4 @@
-"""The quantiser's row norms, codes and planes at the edges of their kernels: bit for bit the checker's."""
+"""The quantiser's row norms, codes and planes at the edges of their kernels: bit for bit the oracle's."""
 import numpy as np
 import pytest
 
@@ -14,7 +14,7 @@ def same(a, b):
     (1, 32, 32), (31, 96, 32), (32, 128, 128), (33, 160, 32), (65, 448, 64), (7, 640, 128), (40, 768, 256), (3, 1536, 512), (130, 1024, 1024),
 ])
 @pytest.mark.parametrize("bits", [(4, 4, True), (4, 4, False), (5, 3, True), (3, 2, False)], ids=["shared", "dual", "five", "few"])
-def test_quantised_rows_match_the_checker(tq, oracle, rows, cols, block, bits):
+def test_quantised_rows_match_the_oracle(tq, oracle, rows, cols, block, bits):
     torch = pytest.importorskip("torch")
     pb, rb, shared = bits
     rng = np.random.default_rng(rows * cols)
