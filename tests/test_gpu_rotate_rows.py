@@ -1,5 +1,5 @@
-"""The activation rotation of the many-row linear at the edges of its tiles: blocks of 32 to 512 columns (and 1024, which has a
-kernel of its own), a last group of columns that is not full, rows around the groups of 8 and 32, several steps per CTA.
+"""The activation rotation of the many-row linear at the edges of its tiles: blocks of 32 to 1024 columns, a last group of columns
+that is not full, rows around the groups of 8 and 32, several steps per CTA.
 Tolerance as in test_gpu_gemm_edges: three roundings to fp16, root mean square below 4.9e-4; a row on its own may reach 1.5 of that."""
 import numpy as np
 import pytest
@@ -19,6 +19,28 @@ def test_rotation_of_many_rows(tq, n_in, block, shared, rows):
 @pytest.mark.parametrize("n_in,block,rows", [(8192, 64, 1300), (16384, 128, 2050), (16384, 512, 2077)])
 def test_rotation_with_several_steps(tq, n_in, block, rows):
     check(tq, n_in, block, True, rows)
+
+
+@pytest.mark.parametrize("n_in,block,shared", [
+    (64, 32, True), (192, 64, False), (128, 128, True), (3584, 128, True), (768, 256, False), (512, 512, True), (1536, 512, False), (1024, 1024, True),
+])
+def test_alignment_does_not_show(tq, n_in, block, shared):
+    """An activation that is not 16-byte aligned is rotated by another kernel, which adds in the same order: the same bits, also
+    where the sums of a block have to be rounded (values of very different size)."""
+    torch = pytest.importorskip("torch")
+    rows, n_out = 300, 256
+    g = torch.Generator(device="cuda").manual_seed(n_in + block)
+    c = tq.generate_codebook(4)
+    w = torch.randn((n_out, n_in), generator=g, device="cuda") * 0.02
+    lin = tq.TurboQuantLinear(n_in, n_out, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, block, shared)), c, c, block)
+    x = torch.randn((rows, n_in), generator=g, device="cuda")
+    x = (x * 2.0 ** torch.randint(-16, 6, x.shape, generator=g, device="cuda")).half()
+    shifted = torch.empty(rows * n_in + 1, device="cuda", dtype=torch.float16)[1:].view(rows, n_in).copy_(x)
+    y = lin.forward(x)
+    assert torch.isfinite(y).all()
+    assert torch.equal(lin.forward(shifted), y)
+    lin.check_status()
+    lin.close()
 
 
 def check(tq, n_in, block, shared, rows):

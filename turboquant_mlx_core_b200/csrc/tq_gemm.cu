@@ -244,140 +244,6 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
     }
 }
 
-// The rotation on the tensor cores, for WHT blocks up to 512 columns.  A Walsh-Hadamard transform is a product over the bits of
-// the column number, in any order; m16n8k16 with a matrix of +-1 takes four of them (the signed halves go in as they are, the sums
-// are fp32), the accumulators of a lane the others.  Of column c = (.. c6 c5 c4 c3 c2 c1 c0) the product takes c0, c1, c3, c4:
-//   B (activations, 8 rows): lane (g, q) holds row g; k = (c1 c4 c3 c0), so q = (c4 c3) and a 16-byte load of the columns
-//     32 j + 8 q .. + 7 is the operands of two tiles, c2 = 0 and 1
-//   A (+-1): k as above, m = (c3 c4 c1 c0)
-//   C: lane (g, q) holds (c4 c1 c0) = g, c3 = 0 / 1 and rows 2 q, 2 q + 1: an 8 x 8 matrix per c3 whose transpose is the core matrix
-//     4 c3 + 2 c2 + c5 of the operand tile's K block c6.. (k_position), 128 contiguous bytes
-// A warp takes 8 rows x COLS columns, `row_steps` times; the four warps of a CTA take neighbouring groups of 8 rows.  With the butterflies as
-// lane exchanges (as the kernel below has them) a value took 34 instructions, four of five issue slots: 2048 x 18944 in 52 us
-// against 23 of its bytes, three rotations of 2048 x 3584 in 37; here 30 and 20 (two rotations, block 512, of 2048 x 17920: 101 -> 59).
-// Two fp32 numbers times `scale`, as halves.
-__device__ __forceinline__ uint32_t scaled_halves(unsigned long long v, unsigned long long scale) {
-    const float2 t = unpack2(mul2(v, scale));
-    const __half2 h = __floats2half2_rn(t.x, t.y);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-constexpr int kRotateWarps = 4;
-template <int COLS>
-__device__ __forceinline__ void rotate_rows_mma_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows, int n_planes,
-                                                     int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
-    constexpr int kGroups32 = COLS / 32, kBlocks64 = COLS / 64;
-    __shared__ uint32_t s_sign[kGroups32];                                          // bit set: -1
-    __shared__ __align__(16) uint4 s_out[kRotateWarps][kBlocks64 * 64];             // a K block's eight core matrices: 1 KB
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-    const unsigned groups_per_row = (static_cast<unsigned>(in) + COLS - 1) / COLS;
-    const unsigned rows_per_cta = 8u * kRotateWarps * static_cast<unsigned>(row_steps);
-    const unsigned row_groups = static_cast<unsigned>((rows + rows_per_cta - 1) / rows_per_cta);
-    unsigned b = blockIdx.x;
-    const unsigned rg = b % row_groups;
-    b /= row_groups;
-    const unsigned cg = b % groups_per_row;
-    const int plane = static_cast<int>(b / groups_per_row);
-    if (plane >= n_planes) return;
-    const int col0 = static_cast<int>(cg) * COLS;
-    const uint32_t seed = plane ? seed_r : seed_p;
-    for (int i = tid; i < COLS; i += 32 * kRotateWarps) {
-        const uint32_t bits = __ballot_sync(0xffffffffu, !sign_is_positive(seed, static_cast<uint32_t>((col0 + i) & (block - 1))));
-        if (lane == 0) s_sign[i >> 5] = bits;
-    }
-    __syncthreads();
-    pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
-    uint32_t signs[kGroups32][4];   // of this lane's columns, at the halves' sign bits
-#pragma unroll
-    for (int j = 0; j < kGroups32; ++j) {
-        const uint32_t byte = s_sign[j] >> (8 * q);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) signs[j][w] = ((byte << (15 - 2 * w)) & 0x8000u) | ((byte << (30 - 2 * w)) & 0x80000000u);
-    }
-    // A: rows m = g and g + 8, columns k = 2 q, 2 q + 1 and those + 8
-    uint32_t h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = g + 8 * (i & 1), k = 2 * q + 8 * (i >> 1);
-        // common bits: c4 (m2, k2), c3 (m3, k1), c1 (m1, k3); and c0 (m0, k0) for the second half
-        const int odd = (((m >> 2) & (k >> 2)) ^ ((m >> 3) & (k >> 1)) ^ ((m >> 1) & (k >> 3))) & 1;
-        const uint32_t lo = odd ? 0xBC00u : 0x3C00u;
-        h[i] = lo | ((lo ^ ((m & 1) ? 0x8000u : 0u)) << 16);
-    }
-    const unsigned long long scale = pack2(inv_sqrt, inv_sqrt);
-    const long n_row_tiles = (rows + kTileTok - 1) / kTileTok;
-    const long kb_per_plane = in / kBlockK;
-    uint4* const out = s_out[warp];
-    const uint32_t out_addr = smem_addr(out) + static_cast<uint32_t>(lane) * 16u;
-    const long first = static_cast<long>(rg) * rows_per_cta;
-#pragma unroll 1
-    for (int step = 0; step < row_steps; ++step) {
-        const long row8 = first + 8L * (step * kRotateWarps + warp), row = row8 + g;
-        if (row8 >= rows) return;   // (no barrier of the CTA follows)
-        const __half* const src = x + row * in + col0 + 8 * q;
-        uint4 raw[kGroups32];
-#pragma unroll
-        for (int j = 0; j < kGroups32; ++j)
-            raw[j] = row < rows && col0 + 32 * j < in ? __ldg(reinterpret_cast<const uint4*>(src + 32 * j)) : make_uint4(0u, 0u, 0u, 0u);
-        unsigned long long v[kGroups32][2][2];   // [32 columns][c2][c3], two rows each
-#pragma unroll
-        for (int j = 0; j < kGroups32; ++j) {
-            const uint32_t w[4] = {raw[j].x ^ signs[j][0], raw[j].y ^ signs[j][1], raw[j].z ^ signs[j][2], raw[j].w ^ signs[j][3]};
-#pragma unroll
-            for (int c2 = 0; c2 < 2; ++c2)
-                asm("{ .reg .f32 d0, d1, d2, d3;\n"
-                    "  mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {d0, d1, d2, d3}, {%2, %3, %4, %5}, {%6, %7}, {%8, %8, %8, %8};\n"
-                    "  mov.b64 %0, {d0, d1};  mov.b64 %1, {d2, d3}; }"
-                    : "=l"(v[j][c2][0]), "=l"(v[j][c2][1])
-                    : "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]), "r"(w[2 * c2]), "r"(w[2 * c2 + 1]), "f"(0.0f));
-        }
-        auto butterfly = [](unsigned long long& a, unsigned long long& b) {
-            const unsigned long long s = add2(a, b);
-            b = sub2(a, b);
-            a = s;
-        };
-#pragma unroll
-        for (int j = 0; j < kGroups32; ++j)
-#pragma unroll
-            for (int c3 = 0; c3 < 2; ++c3) butterfly(v[j][0][c3], v[j][1][c3]);
-#pragma unroll
-        for (int bit = 1; bit < kGroups32; bit <<= 1) {
-            if (64 * bit <= block) {
-#pragma unroll
-                for (int j = 0; j < kGroups32; ++j)
-                    if ((j & bit) == 0) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) butterfly(v[j][c >> 1][c & 1], v[j | bit][c >> 1][c & 1]);
-                    }
-            }
-        }
-        __syncwarp();   // the step before has read its image
-#pragma unroll
-        for (int kb = 0; kb < kBlocks64; ++kb)
-#pragma unroll
-            for (int c3 = 0; c3 < 2; ++c3)   // matrices 4 c3 + 2 c2 + c5
-                asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(out_addr + 1024u * kb + 512u * c3),
-                             "r"(scaled_halves(v[2 * kb][0][c3], scale)), "r"(scaled_halves(v[2 * kb + 1][0][c3], scale)),
-                             "r"(scaled_halves(v[2 * kb][1][c3], scale)), "r"(scaled_halves(v[2 * kb + 1][1][c3], scale))
-                             : "memory");
-        __syncwarp();
-        const long rt = row8 / kTileTok, rin = row8 - rt * kTileTok;
-        const long kb0 = col0 / kBlockK;
-        uint4* const dst = reinterpret_cast<uint4*>(xrot + ((static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane + kb0) * (kTileTok * kBlockK) + rin * kBlockK) + lane;
-#pragma unroll
-        for (int kb = 0; kb < kBlocks64; ++kb)
-            if (kb0 + kb < kb_per_plane) {
-                dst[kb * (kTileTok * kBlockK / 8)] = out[64 * kb + lane];
-                dst[kb * (kTileTok * kBlockK / 8) + 32] = out[64 * kb + 32 + lane];
-            }
-    }
-}
-template <int COLS>
-__global__ void __launch_bounds__(32 * kRotateWarps, COLS == 128 ? 5 : (COLS == 256 ? 3 : 2)) rotate_rows_mma_kernel(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows,
-                                                                          int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt,
-                                                                          int row_steps) {
-    rotate_rows_mma_body<COLS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt, row_steps);
-}
-
 // The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of a row (one block of 512 or
 // 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
 // the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
@@ -461,26 +327,23 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
         }
     }
 }
+template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
                                                                    int in, long rows, int n_planes, int block,
                                                                    uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
     pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
-    rotate_rows_wide_body<4>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt, row_steps);
+    rotate_rows_wide_body<CHUNKS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt, row_steps);
 }
 // The same rows rotated for several matrices at once (their own seeds and destinations): blockIdx.y = matrix.
 struct RotateGroupArgs {
     __half* xrot[4];
     uint32_t seed_p[4], seed_r[4];
 };
-template <int COLS>
-__global__ void __launch_bounds__(32 * kRotateWarps, COLS == 128 ? 5 : (COLS == 256 ? 3 : 2)) rotate_rows_mma_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g,
-                                                                                int in, long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
-    rotate_rows_mma_body<COLS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
-}
+template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
                                                                          long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
     pdl_wait_release();
-    rotate_rows_wide_body<4>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
+    rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
 }
 
 struct GemmArgs {
@@ -972,33 +835,32 @@ void launch_finish(const FinishArgs& f, int n, int m, int sm_count, cudaStream_t
     else launch_pdl(gemm_finish_group_kernel, grid, dim3(threads), 0, stream, f, m);
 }
 
-// Steps that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
-int rotate_row_steps(long ctas, int sm_count) { return static_cast<int>(std::max<long>(1, std::min<long>(8, ctas / (8L * sm_count)))); }
+// Groups of 8 rows that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
+int rotate_row_steps(long groups, int sm_count) { return static_cast<int>(std::max<long>(1, std::min<long>(8, groups / (8L * sm_count)))); }
 
 // The activation rows rotated for n matrices (their own seeds and destinations): one launch, except for an activation that is
-// not aligned.
+// not aligned.  Both kernels add in the order of warp_fwht, in fp32: the operand does not depend on the alignment.  (With four of the
+// butterflies as products with +-1 on the tensor cores a 7B layer's projections of 2048 rows took 1100 us instead of 1120, of 64 rows
+// 119 instead of 121; but the sums were rounded elsewhere, and the results of the two kernels differed.)
 void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int in, long m, int n_planes, uint32_t block, int sm_count, cudaStream_t stream) {
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
     const int bs = static_cast<int>(block);
     if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {
-        const int cols = block <= 512 ? std::max(128, bs) : 1024, step_rows = block <= 512 ? 8 * kRotateWarps : 8;
+        const int cols = std::max(256, bs);
         const long groups = static_cast<long>(n_planes) * ((in + cols - 1) / cols);
-        const int row_steps = rotate_row_steps(n * groups * ((m + step_rows - 1) / step_rows), sm_count);
-        const long ctas = groups * ((m + static_cast<long>(step_rows) * row_steps - 1) / (static_cast<long>(step_rows) * row_steps));
+        const int row_steps = rotate_row_steps(n * groups * ((m + 7) / 8), sm_count);
+        const long ctas = groups * ((m + 8L * row_steps - 1) / (8L * row_steps));
         if (ctas < (1L << 31)) {
-            const dim3 grid(static_cast<unsigned int>(ctas), static_cast<unsigned int>(n)), mma_threads(32 * kRotateWarps);
-#define TQ_ROTATE_MMA(COLS)                                                                                                                         \
-    if (n == 1) launch_pdl(rotate_rows_mma_kernel<COLS>, grid, mma_threads, 0, stream, x, rot.xrot[0], in, m, n_planes, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
-    else launch_pdl(rotate_rows_mma_group_kernel<COLS>, grid, mma_threads, 0, stream, x, rot, in, m, n_planes, bs, inv_sqrt, row_steps);
+            const dim3 grid(static_cast<unsigned int>(ctas), static_cast<unsigned int>(n));
+#define TQ_ROTATE_WIDE(CHUNKS)                                                                                                                         \
+    if (n == 1) launch_pdl(rotate_rows_f16_wide_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot.xrot[0], in, m, n_planes, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
+    else launch_pdl(rotate_rows_f16_wide_group_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot, in, m, n_planes, bs, inv_sqrt, row_steps);
             switch (cols) {
-                case 128: TQ_ROTATE_MMA(128) break;
-                case 256: TQ_ROTATE_MMA(256) break;
-                case 512: TQ_ROTATE_MMA(512) break;
-                default:
-                    if (n == 1) launch_pdl(rotate_rows_f16_wide_kernel, grid, dim3(256), 0, stream, x, rot.xrot[0], in, m, n_planes, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps);
-                    else launch_pdl(rotate_rows_f16_wide_group_kernel, grid, dim3(256), 0, stream, x, rot, in, m, n_planes, bs, inv_sqrt, row_steps);
+                case 256: TQ_ROTATE_WIDE(1) break;
+                case 512: TQ_ROTATE_WIDE(2) break;
+                default: TQ_ROTATE_WIDE(4) break;
             }
-#undef TQ_ROTATE_MMA
+#undef TQ_ROTATE_WIDE
             return;
         }
     }
