@@ -60,3 +60,45 @@ def test_copies_from_several_threads(tq):
     for t in threads:
         t.join()
     assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(alone, got))
+
+
+@pytest.mark.parametrize("kind", ["per_thread", "non_blocking"])
+def test_host_weights_on_other_streams(tq, kind):
+    """Weights of more than 32 MB in host memory, on a stream whose handle means another stream in every thread (cudaStreamPerThread = 2)
+    and on one that does not wait for the default stream: the bits of device weights, call after call and beside a second thread."""
+    torch = pytest.importorskip("torch")
+    L = tq.load()
+    c = tq.generate_codebook(4)
+    cb = np.ascontiguousarray(c.centroids, np.float32)
+    cols = 1024
+
+    def quantize(w, rows, stream):
+        planes = [np.empty((rows, cols // 2), np.uint8) for _ in range(2)]
+        norms, seeds = np.empty(rows, np.float32), np.zeros(3, np.uint32)
+        p = w.ctypes.data if isinstance(w, np.ndarray) else w.data_ptr()
+        rc = L.tq_quantize_weight(p, rows, cols, cb.ctypes.data, cb.size, cb.ctypes.data, cb.size, 4, 4, 64, 1, planes[0].ctypes.data,
+                                  planes[1].ctypes.data, norms.ctypes.data, seeds.ctypes.data, stream)
+        assert rc == 0, L.tq_last_error().decode()
+        return planes + [norms.view(np.uint32), seeds]
+
+    def fit(w, stream):
+        return [x for b in tq.fit_layer_codebooks(w, 64, 4, 4, 10, stream=stream) for x in (b.centroids, b.boundaries)]
+
+    failures = []
+
+    def work(rows):
+        stream = 2 if kind == "per_thread" else torch.cuda.Stream().cuda_stream
+        g = torch.Generator(device="cuda").manual_seed(rows)
+        for _ in range(3):   # other weights each time: what an earlier call left in the staging is wrong
+            w = torch.randn((rows, cols), generator=g, device="cuda") * 0.02
+            torch.cuda.synchronize()
+            host = w.cpu().numpy()
+            for want, got in ((quantize(w, rows, None), quantize(host, rows, stream)), (fit(w, None), fit(host, stream))):
+                failures.extend((rows, i) for i, (a, b) in enumerate(zip(want, got)) if not np.array_equal(a, b))
+
+    threads = [threading.Thread(target=work, args=(rows,)) for rows in (8449, 20480)]   # 34.6 and 83.9 MB
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures

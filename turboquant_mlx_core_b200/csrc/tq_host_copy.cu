@@ -2,14 +2,16 @@
 // layer, a host caller's weights.
 //
 // The driver copies pageable memory on one thread, through staging of its own, and takes the faults of new pages on the way.  From
-// a size on, up to four threads move pieces of 1 MB between the caller's memory and a ring of page-locked ones, each behind its
-// own event, while the copy engine is at the next.  The threads live as long as the call.  On a host of 16 cores: 67 MB into
-// new pages 13.7 -> 4.8 ms, into old ones 3.2 -> 2.2, out of host memory 4.4 -> 2.4; two planes of 8.4 MB out of the quantiser
-// 2.2 -> 0.9 (half of it no longer clearing the pages first).  Smaller copies gain nothing: 17 MB to the device 0.8 and 0.8, 4 MB
-// from it 0.2 and 0.2 to 0.5.
+// a size on, up to five threads move pieces of 1 MB between the caller's memory and a ring of page-locked ones, while the copy
+// engine is at the next.  The calling thread alone talks to the driver: it queues the pieces' device copies, each with an event
+// behind it, and asks those events how far the engine has come, between pieces of its own.  The other threads live as long as the
+// call and do nothing but memcpy (a stream handle need not mean the same stream in another thread: cudaStreamPerThread does
+// not).  On a host of 16 cores: 67 MB into new pages 13.7 -> 4.8 ms, into old ones 3.2 -> 2.2, out of host memory 4.4 -> 2.2; two planes
+// of 8.4 MB out of the quantiser 2.2 -> 0.9 (half of it no longer clearing the pages first).  With half as large a ring, or pieces of
+// half the size, the calling thread's look comes too late: 5.6 ms into new pages.  Smaller copies gain nothing: 17 MB to the device 0.8
+// and 0.8, 4 MB from it 0.2 and 0.2 to 0.5.
 #include <algorithm>
 #include <atomic>
-#include <system_error>
 #include <thread>
 
 #include "tq_host.hpp"
@@ -19,9 +21,12 @@ namespace tq {
 namespace {
 
 constexpr size_t kPiece = size_t(1) << 20;
-constexpr int kRing = 8;                                // pieces of staging
+constexpr size_t kRing = 16;                            // pieces of staging at most
 constexpr size_t kThreadsToHost = size_t(8) << 20, kThreadsToDevice = size_t(32) << 20;   // bytes from which on threads are used
-constexpr int kThreads = 4;
+constexpr size_t kThreads = 5;                           // with the calling one
+// Another thread for every eight pieces: what other cores have in their caches is slower to read for the caller afterwards (16 MB of
+// planes out of the quantiser and into a layer: 2490 us with five threads, 2200 with three, 2300 with one).
+constexpr size_t kPiecesPerThread = 8;
 
 struct Piece {
     uint8_t* dst;
@@ -29,85 +34,108 @@ struct Piece {
     size_t bytes;
 };
 
-struct Ring {
-    PinnedStage stage{kRing * kPiece};
-    cudaEvent_t event[kRing] = {};
-    cudaStream_t st;
-    explicit Ring(cudaStream_t s) : st(s) {
-        for (cudaEvent_t& e : event) TQ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    ~Ring() {
-        cudaStreamSynchronize(st);   // (queued copies still read or write the staging)
-        for (cudaEvent_t e : event)
-            if (e) cudaEventDestroy(e);
-    }
-    uint8_t* place(size_t i) const { return stage.host<uint8_t>() + (i % kRing) * kPiece; }
+struct CopyEvent {
+    cudaEvent_t e = nullptr;
+    CopyEvent() { TQ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~CopyEvent() { cudaEventDestroy(e); }
+    CopyEvent(const CopyEvent&) = delete;
+    CopyEvent& operator=(const CopyEvent&) = delete;
 };
 
-// All pieces, by the calling thread and as many others as there is use for.
-void move_pieces(const std::vector<Piece>& pieces, bool to_device, cudaStream_t st) {
-    const size_t n = pieces.size();
-    Ring ring(st);
-    const int device = current_device();
-    std::vector<std::atomic<bool>> issued(n);   // the piece's device copy is queued, its event recorded behind it
-    for (auto& f : issued) f.store(false, std::memory_order_relaxed);
-    std::atomic<size_t> next{0};
-    std::atomic<int> failed{cudaSuccess};
-    auto issue = [&](size_t i) {
-        const Piece& p = pieces[i];
-        cudaError_t rc = to_device ? cudaMemcpyAsync(p.dst, ring.place(i), p.bytes, cudaMemcpyHostToDevice, st)
-                                   : cudaMemcpyAsync(ring.place(i), p.src, p.bytes, cudaMemcpyDeviceToHost, st);
-        if (rc == cudaSuccess) rc = cudaEventRecord(ring.event[i % kRing], st);
-        if (rc != cudaSuccess) failed.store(rc);
-        issued[i].store(true, std::memory_order_release);
-        return rc == cudaSuccess;
-    };
-    // Waits until piece i's device copy has ended.  (Its place belongs to whoever does: pieces are taken in order, and the one that
-    // issues a copy does so before it takes another piece.)
-    auto arrived = [&](size_t i) {
-        while (!issued[i].load(std::memory_order_acquire)) {
-            if (failed.load() != cudaSuccess) return false;
-            std::this_thread::yield();
-        }
-        const cudaError_t rc = cudaEventSynchronize(ring.event[i % kRing]);
-        if (rc != cudaSuccess) failed.store(rc);
-        return rc == cudaSuccess;
-    };
-    auto work = [&] {
-        for (size_t i; failed.load() == cudaSuccess && (i = next.fetch_add(1)) < n;) {
-            if (to_device) {
-                if (i >= kRing && !arrived(i - kRing)) return;
-                std::memcpy(ring.place(i), pieces[i].src, pieces[i].bytes);
-                if (!issue(i)) return;
-            } else {
-                if (!arrived(i)) return;
-                std::memcpy(pieces[i].dst, ring.place(i), pieces[i].bytes);
-                if (i + kRing < n && !issue(i + kRing)) return;
-            }
-        }
-    };
-    if (!to_device)
-        for (size_t i = 0; i < n && i < kRing; ++i)
-            if (!issue(i)) break;
-    std::vector<std::thread> helpers;
-    const size_t want = std::min<size_t>(std::min<size_t>(kThreads, std::max(1u, std::thread::hardware_concurrency())), n);
-    helpers.reserve(want);
-    for (size_t t = 1; t < want; ++t) {
+// The pieces of a call on their way.  Piece i uses place i % ring_ of the staging; pieces are taken up, queued and found done in order.
+class PieceMover {
+public:
+    PieceMover(const std::vector<Piece>& pieces, bool to_device, cudaStream_t st)
+        : pieces_(pieces), n_(pieces.size()), ring_(std::min(kRing, n_ / 2)), to_device_(to_device), st_(st), moved_(pieces.size()) {
+        for (auto& f : moved_) f.store(false, std::memory_order_relaxed);
+        if (to_device_) ready_.store(ring_);
+    }
+    ~PieceMover() {
+        stop_.store(true);
+        for (std::thread& t : helpers_) t.join();
+        if (arrived_ < queued_) cudaStreamSynchronize(st_);   // (a failure: queued copies still read or write the staging)
+    }
+
+    void run() {
+        if (!to_device_) queue_copies();
+        const size_t want = std::min(std::min(kThreads, static_cast<size_t>(std::max(1u, std::thread::hardware_concurrency()))), 1 + n_ / kPiecesPerThread);
         try {
-            helpers.emplace_back([&] {
-                const cudaError_t rc = cudaSetDevice(device);
-                if (rc != cudaSuccess) failed.store(rc);
-                else work();
-            });
-        } catch (const std::system_error&) {
-            break;   // fewer threads, then
+            helpers_.reserve(want);
+            while (helpers_.size() + 1 < want)
+                helpers_.emplace_back([this] {
+                    while (!stop_.load(std::memory_order_relaxed) && next_.load(std::memory_order_relaxed) < n_)
+                        if (!move_one()) std::this_thread::yield();
+                });
+        } catch (...) {   // fewer threads, then
+        }
+        // done: to the device, the last copy has arrived; from it, the last piece is with the caller
+        while (to_device_ ? arrived_ < n_ : moved_in_order_ < n_) {
+            const bool news = queue_copies() | find_arrived();
+            if (!move_one() && !news) std::this_thread::yield();
+            while (moved_in_order_ < n_ && moved_[moved_in_order_].load(std::memory_order_acquire)) ++moved_in_order_;
         }
     }
-    work();
-    for (std::thread& t : helpers) t.join();
-    TQ_CUDA(static_cast<cudaError_t>(failed.load()));
-    TQ_CUDA(cudaStreamSynchronize(st));
-}
+
+private:
+    uint8_t* place(size_t i) const { return stage_.host<uint8_t>() + (i % ring_) * kPiece; }
+
+    // Moves the next piece between the caller's memory and its place, if there is one whose place is ready.
+    bool move_one() {
+        size_t i = next_.load(std::memory_order_relaxed);
+        do {
+            if (i >= ready_.load(std::memory_order_acquire)) return false;
+        } while (!next_.compare_exchange_weak(i, i + 1, std::memory_order_relaxed));
+        const Piece& p = pieces_[i];
+        if (to_device_) std::memcpy(place(i), p.src, p.bytes);
+        else std::memcpy(p.dst, place(i), p.bytes);
+        moved_[i].store(true, std::memory_order_release);
+        return true;
+    }
+    // Queues the device copies that can be: to the device those of the pieces in their places, from it those whose place the piece
+    // before has left.
+    bool queue_copies() {
+        const size_t before = queued_;
+        for (; queued_ < n_; ++queued_) {
+            if (to_device_ ? !moved_[queued_].load(std::memory_order_acquire)
+                           : queued_ >= ring_ && !moved_[queued_ - ring_].load(std::memory_order_acquire))
+                break;
+            const Piece& p = pieces_[queued_];
+            if (to_device_) TQ_CUDA(cudaMemcpyAsync(p.dst, place(queued_), p.bytes, cudaMemcpyHostToDevice, st_));
+            else TQ_CUDA(cudaMemcpyAsync(place(queued_), p.src, p.bytes, cudaMemcpyDeviceToHost, st_));
+            TQ_CUDA(cudaEventRecord(events_[queued_ % ring_].e, st_));
+        }
+        return queued_ != before;
+    }
+    // Looks how many device copies have ended.  (A place's event is recorded anew only behind a copy that was found ended.)
+    bool find_arrived() {
+        const size_t before = arrived_;
+        while (arrived_ < queued_) {
+            const cudaError_t rc = cudaEventQuery(events_[arrived_ % ring_].e);
+            if (rc == cudaErrorNotReady) {
+                cudaGetLastError();
+                break;
+            }
+            TQ_CUDA(rc);
+            ++arrived_;
+        }
+        if (arrived_ != before) ready_.store(to_device_ ? std::min(n_, arrived_ + ring_) : arrived_, std::memory_order_release);
+        return arrived_ != before;
+    }
+
+    const std::vector<Piece>& pieces_;
+    const size_t n_;
+    const size_t ring_;   // (half the pieces: of a few megabytes the caller's copy stays in its caches, not the staging)
+    const bool to_device_;
+    const cudaStream_t st_;
+    PinnedStage stage_{ring_ * kPiece};
+    CopyEvent events_[kRing];
+    std::vector<std::atomic<bool>> moved_;   // the piece's memcpy is done
+    std::atomic<size_t> next_{0};            // pieces taken up
+    std::atomic<size_t> ready_{0};           // pieces that may be: their place is free, or holds them
+    std::atomic<bool> stop_{false};
+    size_t queued_ = 0, arrived_ = 0, moved_in_order_ = 0;   // (the calling thread's)
+    std::vector<std::thread> helpers_;
+};
 
 void copy_host(const HostCopy* copies, int n, bool to_device, cudaStream_t st) {
     std::vector<Piece> pieces;
@@ -126,11 +154,12 @@ void copy_host(const HostCopy* copies, int n, bool to_device, cudaStream_t st) {
         for (size_t at = 0; at < c.bytes; at += kPiece)
             pieces.push_back(Piece{static_cast<uint8_t*>(c.dst) + at, static_cast<const uint8_t*>(c.src) + at, std::min(kPiece, c.bytes - at)});
     }
-    if (total >= (to_device ? kThreadsToDevice : kThreadsToHost)) {
-        move_pieces(pieces, to_device, st);
-        return;
+    // (on a stream that is being captured the driver's own copy gives the error)
+    if (total >= (to_device ? kThreadsToDevice : kThreadsToHost) && !stream_is_capturing(st)) {
+        PieceMover(pieces, to_device, st).run();
+    } else {
+        for (const HostCopy& c : large) TQ_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st));
     }
-    for (const HostCopy& c : large) TQ_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st));
     TQ_CUDA(cudaStreamSynchronize(st));
 }
 
