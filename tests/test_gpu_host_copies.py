@@ -102,3 +102,45 @@ def test_host_weights_on_other_streams(tq, kind):
     for t in threads:
         t.join()
     assert not failures
+
+
+def test_page_locked_values_are_read_in_stream_order(tq):
+    """Codebooks and seeds in page-locked memory that work queued on the default stream still writes."""
+    torch = pytest.importorskip("torch")
+    L = tq.load()
+    rows, cols, block = 64, 256, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = torch.randn((rows, cols), generator=g, device="cuda") * 0.02
+    c = tq.generate_codebook(4)
+    cb = np.ascontiguousarray(c.centroids, np.float32)
+    want = tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, block, False))
+
+    def queued(values):
+        """Page-locked memory that holds other values until a copy behind some milliseconds of work has run."""
+        late = torch.full(values.shape, 1, dtype=values.dtype).pin_memory()
+        on_device = values.cuda()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)
+        late.copy_(on_device, non_blocking=True)
+        return late
+
+    planes = [np.empty((rows, cols // 2), np.uint8) for _ in range(2)]
+    norms, seeds = np.empty(rows, np.float32), np.zeros(3, np.uint32)
+    late = queued(torch.from_numpy(cb))
+    rc = L.tq_quantize_weight(w.data_ptr(), rows, cols, late.data_ptr(), cb.size, late.data_ptr(), cb.size, 4, 4, block, 0, planes[0].ctypes.data,
+                              planes[1].ctypes.data, norms.ctypes.data, seeds.ctypes.data, None)
+    assert rc == 0, L.tq_last_error().decode()
+    assert np.array_equal(planes[0], want.packed_primary) and np.array_equal(planes[1], want.packed_residual)
+    assert np.array_equal(norms, want.norms) and np.array_equal(seeds, want.seeds)
+
+    layer = tq.TurboQuantLinear(cols, rows, want, c, c, block)
+    late = queued(torch.from_numpy(want.seeds.view(np.int32)))
+    h = L.tq_linear_create(cols, rows, want.packed_primary.ctypes.data, cols // 2, want.packed_residual.ctypes.data, want.norms.ctypes.data,
+                           late.data_ptr(), cb.ctypes.data, cb.size, cb.ctypes.data, cb.size, block)
+    assert h, L.tq_last_error().decode()
+    back = torch.empty((rows, cols), device="cuda")
+    assert L.tq_linear_dequantize(h, back.data_ptr(), 0, None) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(back.cpu().numpy(), layer.dequantize(np.float32))
+    L.tq_linear_free(h)
+    layer.close()

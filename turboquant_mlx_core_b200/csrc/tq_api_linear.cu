@@ -44,7 +44,7 @@ public:
 
         cudaStream_t st = nullptr;
         uint32_t h_seeds[3];
-        tq::read_values(h_seeds, seeds, sizeof h_seeds);
+        TQ_CUDA(cudaMemcpy(h_seeds, seeds, sizeof h_seeds, cudaMemcpyDefault));
         seed_p_ = h_seeds[0];
         seed_r_ = h_seeds[1];
 
@@ -78,8 +78,8 @@ public:
 
         // lookup tables over the joint byte
         std::vector<float> cp(n_p), cr(n_r);
-        tq::read_values(cp.data(), cb_p, sizeof(float) * n_p);
-        tq::read_values(cr.data(), cb_r, sizeof(float) * n_r);
+        TQ_CUDA(cudaMemcpy(cp.data(), cb_p, sizeof(float) * n_p, cudaMemcpyDefault));
+        TQ_CUDA(cudaMemcpy(cr.data(), cb_r, sizeof(float) * n_r, cudaMemcpyDefault));
         std::vector<float> tables(512, 0.0f);
         const int p_bits = primary_5bit_ ? 5 : 4;
         const int p_mask = (1 << p_bits) - 1;
@@ -634,8 +634,8 @@ static int quantize_weight_impl(const float* weight, int out_features, int in_fe
         const size_t n = static_cast<size_t>(out_features) * in_features;
         const size_t pp_bytes = primary_bits <= 4 ? n / 2 : n, pr_bytes = n / 2;
         std::vector<float> cp(n_primary), cr(n_residual);
-        read_values(cp.data(), primary_centroids, sizeof(float) * n_primary);
-        read_values(cr.data(), residual_centroids, sizeof(float) * n_residual);
+        TQ_CUDA(cudaMemcpy(cp.data(), primary_centroids, sizeof(float) * n_primary, cudaMemcpyDefault));
+        TQ_CUDA(cudaMemcpy(cr.data(), residual_centroids, sizeof(float) * n_residual, cudaMemcpyDefault));
         DeviceBuffer w_stage, recon, orig;
         recon.reserve(n * sizeof(float), st);
         orig.reserve(static_cast<size_t>(out_features) * sizeof(float) + 4, st);

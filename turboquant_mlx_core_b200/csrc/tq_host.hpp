@@ -189,8 +189,6 @@ struct HostCopy {
 // From device memory, behind the work queued on `st`, into host memory of any kind and back; the calls wait for the copies.
 void copies_to_host(const HostCopy* copies, int n, cudaStream_t st);
 void copies_to_device(const HostCopy* copies, int n, cudaStream_t st);
-// A few values that may be in device or in host memory.
-void read_values(void* dst, const void* src, size_t bytes);
 
 // A read-only view of caller data on the device: device pointers are used in place,
 // host pointers are copied into `staging` on `stream`.

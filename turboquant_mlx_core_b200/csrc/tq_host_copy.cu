@@ -168,9 +168,4 @@ void copy_host(const HostCopy* copies, int n, bool to_device, cudaStream_t st) {
 void copies_to_host(const HostCopy* copies, int n, cudaStream_t st) { copy_host(copies, n, false, st); }
 void copies_to_device(const HostCopy* copies, int n, cudaStream_t st) { copy_host(copies, n, true, st); }
 
-void read_values(void* dst, const void* src, size_t bytes) {
-    if (is_device_pointer(src)) TQ_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
-    else std::memcpy(dst, src, bytes);
-}
-
 }  // namespace tq
