@@ -49,7 +49,7 @@ def test_crowded_samples_are_fitted_in_passes_over_all(tq, oracle, n, share):
 
 @pytest.mark.parametrize("kind", ["normal", "wide", "small", "one sign", "two magnitudes"])
 def test_fit_counts_outside_of_the_window(tq, oracle, kind):
-    """From 2 M samples on the counters on the SM hold 48 exponents: samples below them, of one sign, and nowhere near the codebook."""
+    """The counters on the SM hold 32 exponents at most: samples below them, of one sign, and nowhere near the codebook."""
     n = 2_200_003
     rng = np.random.default_rng(7)
     x = rng.standard_normal(n)
@@ -81,3 +81,66 @@ def test_layer_fits_side_by_side(tq, rows, cols, block):
     host = tq.fit_layer_codebooks(w.cpu().numpy(), block, 4, 3, 40)
     assert all(np.array_equal(a.centroids.view(np.uint32), b.centroids.view(np.uint32)) for a, b in zip(both, host))
     assert both[1].centroids.size == 8 and np.all(np.diff(both[1].centroids) > 0)
+
+
+def test_samples_are_there_again_for_the_passes_over_all(tq):
+    """The second fit's samples take the place of the first one's; where that one then has to go over all of its own after all
+    (magnitudes in one or two buckets, their residuals in many), it finds them there."""
+    torch = pytest.importorskip("torch")
+    rows, cols = 40_000, 64
+    g = torch.Generator(device="cuda").manual_seed(11)
+    w = torch.randn((rows, cols), generator=g, device="cuda") * (2e-3 / 8)
+    w[:, 5] += 1.0                                          # its transform: +-1 in every column
+    both = tq.fit_layer_codebooks(w, cols, 4, 4, 15)
+    alone, _ = tq.fit_layer_codebooks(w, cols, 4, 0, 15)
+    assert np.array_equal(both[0].centroids.view(np.uint32), alone.centroids.view(np.uint32))
+    assert abs(np.abs(both[0].centroids - 1.0).min()) < 1e-2   # (the samples are what the test takes them for)
+
+
+@pytest.mark.parametrize("rows,cols,log2_buckets", [(1024, 1024, 16), (4096, 4096, 20)])
+def test_memory_kept_after_a_layer_fit(tq, rows, cols, log2_buckets):
+    """Three arrays of samples, two sets of buckets, one of the CTAs' places (32 exponents or 48 K counters, for 8192 samples and more), in
+    size classes an eighth wide."""
+    torch = pytest.importorskip("torch")
+    w = torch.randn((rows, cols), device="cuda") * 0.02
+    n = rows * cols
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    places = min(sms, -(-n // 8192)) * 4 * min(49152, 64 << (log2_buckets - 9))
+    tq.fit_layer_codebooks(w, 64, 4, 4, 2)
+    tq.release_cached_memory()
+    tq.fit_layer_codebooks(w, 64, 4, 4, 2)
+    assert tq.release_cached_memory() <= 1.125 * (3 * 4 * n + 2 * 21 * 2 ** log2_buckets + places) + (1 << 20)
+
+
+def test_a_fit_leaves_other_kept_memory_alone(tq):
+    """What a layer's two fits hold beyond those of one does not push other objects' memory out."""
+    torch = pytest.importorskip("torch")
+    w = torch.randn((4096, 4096), device="cuda") * 0.02
+    kv = torch.zeros((16, 2, 128), device="cuda", dtype=torch.float16)
+
+    def caches(n):
+        made = [tq.TQKVCache(1, 2, 128) for _ in range(n)]
+        for c in made:
+            c.reserve(0, 400_000)
+            c.append(0, kv, kv)
+        torch.cuda.synchronize()
+        return made
+
+    def close(made):
+        for c in made:
+            c.close()
+        torch.cuda.synchronize()
+
+    tq.fit_layer_codebooks(w, 128, 4, 4, 2)
+    tq.release_cached_memory()
+    close(caches(1))
+    each = tq.release_cached_memory()
+    n = (290 << 20) // each                                 # one fit's memory is 212 MB of the 512 that are kept, a layer's two 260
+    close(caches(n))
+    tq.fit_layer_codebooks(w, 128, 4, 4, 2)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    made = caches(n)
+    assert torch.cuda.mem_get_info()[0] > free - (32 << 20)
+    close(made)
+    tq.release_cached_memory()

@@ -225,13 +225,19 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
         uint32_t seed_p = 0, seed_r = 0;
         derive_seeds(d_w, n, &seed_p, &seed_r, st);
         launch_row_norms(d_w, norms.as<float>(), out_features, in_features, st);
-        launch_layer_samples(d_w, norms.as<float>(), out_features, in_features, block, seed_p, cp0, 1 << primary_bits,
-                             scaled.as<float>(), need_residual ? resid.as<float>() : nullptr, st);
+        auto samples = [&] {
+            launch_layer_samples(d_w, norms.as<float>(), out_features, in_features, block, seed_p, cp0, 1 << primary_bits,
+                                 scaled.as<float>(), need_residual ? resid.as<float>() : nullptr, st);
+        };
+        samples();
         const FitRequest primary{scaled.as<float>(), static_cast<long>(n), primary_bits, iterations, cp0, primary_centroids, primary_boundaries};
-        if (need_residual)
-            launch_codebook_fits(primary, FitRequest{resid.as<float>(), static_cast<long>(n), residual_bits, iterations, cr0, residual_centroids, residual_boundaries}, st);
-        else
+        if (need_residual) {
+            FitRequest residual{resid.as<float>(), static_cast<long>(n), residual_bits, iterations, cr0, residual_centroids, residual_boundaries};
+            residual.room = scaled.as<float>();
+            launch_codebook_fits(primary, residual, samples, st);
+        } else {
             launch_codebook_fit(primary, st);
+        }
         TQ_CUDA(cudaStreamSynchronize(st));
         for (DeviceBuffer* b : {&w_stage, &norms, &scaled, &resid}) b->set_idle();
         return 0;

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <functional>
 
 #include "tq_common.cuh"
 #include "tq_host.hpp"
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(1024) fit_look_kernel(const float* __restrict_
 // the scatter, which deals the samples to CTAs in the same way, needs no other word from the CTAs around it.  Samples outside of
 // the window are counted in L2.
 constexpr int kWindowSlots = 49152;           // counters of a CTA: 192 KB
+constexpr int kWindowExponents = 32;          // no more exponents than that: below 2^-31 of the largest there is next to nothing
 constexpr unsigned int kWindowTile = 8192;    // samples that a CTA takes at a time
 // Used wherever the samples are looked at first (from kFitCrowd on): 262144 / 1 M / 4.2 M / 16.8 M normal samples are counted in
 // 5 / 8 / 14 / 40 us (37 / 104 / 135 / 186 in L2) and scattered in 9 / 13 / 30 / 142 (39 / 113 / 143 / 299).
@@ -641,7 +643,8 @@ namespace {
 // One fit on its way: what is queued on the stream, and the memory that it uses.
 class FitRun {
 public:
-    FitRun(const FitRequest& r, cudaStream_t stream) : r_(r), stream_(stream), nc_(1 << r.bits) {
+    // lender: a fit that is queued before this one on the same stream; its memory for the CTAs' places serves both.
+    FitRun(const FitRequest& r, cudaStream_t stream, const FitRun* lender = nullptr) : r_(r), stream_(stream), nc_(1 << r.bits) {
         TQ_REQUIRE(r.bits >= 1 && r.bits <= 5, "Unsupported bit width; must be 1-5");
         h_.n = nc_;
         for (int i = 0; i < nc_; ++i) h_.centroids[i] = r.init_centroids[i];
@@ -667,22 +670,29 @@ public:
         if (bucketed_) {
             try {
                 bucket_buf_.reserve(static_cast<size_t>(n_buckets_) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups_) * 8 + static_cast<size_t>(n_groups_) * 4, stream);
-                sorted_buf_.reserve(static_cast<size_t>(r.n) * 4, stream);
+                if (r.room == nullptr) sorted_buf_.reserve(static_cast<size_t>(r.n) * 4, stream);
             } catch (const OutOfMemory&) {
                 bucketed_ = false;   // the passes over all samples need next to nothing
             }
         }
         // exponents of the window; without memory for the CTAs' places all counters are in L2
-        window_ = std::min(254, kWindowSlots >> (24 - shift_));
+        window_ = std::min(kWindowExponents, kWindowSlots >> (24 - shift_));
+        window_ctas_ = static_cast<int>(std::min<long>(sms_, (r.n + kWindowTile - 1) / kWindowTile));
         windowed_ = bucketed_ && r.n >= static_cast<long>(kFitCrowd);
-        if (windowed_) {
+        if (windowed_ && lender != nullptr && lender->windowed_ && lender->begin_bytes() >= begin_bytes()) {
+            begin_ = lender->begin_;
+        } else if (windowed_) {
+            begin_buf_.set_first_to_go();
             try {
-                begin_buf_.reserve(window_bytes() * sms_, stream);
+                begin_buf_.reserve(begin_bytes(), stream);
             } catch (const OutOfMemory&) {
                 windowed_ = false;
             }
+            begin_ = begin_buf_.as<unsigned int>();
         }
+        if (lender != nullptr) bucket_buf_.set_first_to_go();   // (fits one after the other make do with the lender's)
     }
+    bool iterated() const { return iterated_; }
     bool short_of_memory() const { return active_ && (!bucketed_ || (!windowed_ && r_.n >= static_cast<long>(kFitCrowd))) && r_.n < (1L << 31); }
 
     // Queues what comes before the iterations; fills in the job and returns true where there are buckets to iterate on.
@@ -696,7 +706,7 @@ public:
         unsigned int* const d_offset = d_count + n_buckets_;
         unsigned int* const d_cursor = d_offset + n_buckets_;
         unsigned int* const d_group = d_cursor + n_buckets_;
-        float* const d_sorted = sorted_buf_.as<float>();
+        float* const d_sorted = r_.room != nullptr ? r_.room : sorted_buf_.as<float>();
         const unsigned int un = static_cast<unsigned int>(r_.n);
         const int grid = static_cast<int>(std::min<long>((r_.n + 1023) / 1024, 16L * sms_));
         TQ_CUDA(cudaMemsetAsync(d_count, 0, static_cast<size_t>(n_buckets_) * 4, stream_));
@@ -709,12 +719,11 @@ public:
             }
         }
         if (un >= kFitCrowd) fit_look_kernel<<<1, 1024, 0, stream_>>>(r_.data, un, shift_, window_, state());
-        unsigned int* const d_begin = begin_buf_.as<unsigned int>();
-        if (windowed_) fit_count_window_kernel<<<sms_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_count, d_begin, state());
+        if (windowed_) fit_count_window_kernel<<<window_ctas_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_count, begin_, state());
         else fit_count_kernel<<<grid, 256, 0, stream_>>>(r_.data, un, shift_, d_count, state());
         fit_groups_kernel<<<n_groups_, 256, 0, stream_>>>(d_count, d_group);
         fit_offsets_kernel<<<n_groups_, 256, 0, stream_>>>(d_count, d_group, d_offset, d_cursor);
-        if (windowed_) fit_scatter_window_kernel<<<sms_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_offset, d_begin, d_cursor, d_sorted, state());
+        if (windowed_) fit_scatter_window_kernel<<<window_ctas_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_offset, begin_, d_cursor, d_sorted, state());
         else fit_scatter_kernel<<<grid, 256, 0, stream_>>>(r_.data, un, shift_, d_cursor, d_sorted, state());
         fit_sums_kernel<<<n_parts, 256, 0, stream_>>>(d_sorted, d_count, d_offset, shift_, d_sum, d_part, state());
         TQ_CUDA(cudaGetLastError());
@@ -724,10 +733,14 @@ public:
     }
 
     // Waits for the iterations, makes those that are left over all samples, and hands the results out; the iterations run.
-    int finish() {
+    // samples_again: queues what fills the samples in once more, where they have been overwritten.
+    int finish(const std::function<void()>* samples_again = nullptr) {
         if (active_) {
             if (iterated_) read_state();
-            if (h_.go_over_all && !h_.converged && h_.iterations_run < r_.iterations) go_over_all();
+            if (h_.go_over_all && !h_.converged && h_.iterations_run < r_.iterations) {
+                if (samples_again != nullptr) (*samples_again)();
+                go_over_all();
+            }
             for (DeviceBuffer* b : {&state_buf_, &bucket_buf_, &sorted_buf_, &begin_buf_}) b->set_idle();
         }
         for (int i = 0; i < nc_; ++i) r_.centroids_out[i] = h_.centroids[i];
@@ -739,6 +752,7 @@ public:
 private:
     FitState* state() { return state_buf_.as<FitState>(); }
     size_t window_bytes() const { return (static_cast<size_t>(window_) << (24 - shift_)) * sizeof(unsigned int); }
+    size_t begin_bytes() const { return window_bytes() * window_ctas_; }
     void read_state() {
         TQ_CUDA(cudaMemcpyAsync(&h_, state(), sizeof h_, cudaMemcpyDeviceToHost, stream_));
         TQ_CUDA(cudaStreamSynchronize(stream_));
@@ -772,7 +786,8 @@ private:
     FitState h_{};
     DeviceBuffer state_buf_, bucket_buf_, sorted_buf_, begin_buf_;
     bool active_ = false, bucketed_ = false, windowed_ = false, iterated_ = false;
-    int dev_ = 0, sms_ = 148, shift_ = 0, n_buckets_ = 0, n_groups_ = 0, window_ = 0;
+    int dev_ = 0, sms_ = 148, shift_ = 0, n_buckets_ = 0, n_groups_ = 0, window_ = 0, window_ctas_ = 0;
+    unsigned int* begin_ = nullptr;   // where each CTA's samples of a bucket begin
 };
 
 }  // namespace
@@ -789,22 +804,24 @@ int launch_codebook_fit(const FitRequest& r, cudaStream_t stream) {
     return run.finish();
 }
 
-// Two fits; their iterations run side by side (a CTA each, in one launch), as long as the device has memory for both.
-void launch_codebook_fits(const FitRequest& a, const FitRequest& b, cudaStream_t stream) {
+// Two fits; their iterations run side by side (a CTA each, in one launch), as long as the device has memory for both.  Beyond what
+// one fit takes that is the second one's buckets, and what it holds of the first one's samples (b.room).
+void launch_codebook_fits(const FitRequest& a, const FitRequest& b, const std::function<void()>& samples_again, cudaStream_t stream) {
     constexpr long kTogether = 1L << 25;   // samples: up to there the memory is kept for the next call (tq_memory.cu)
     if (std::max(a.n, b.n) <= kTogether) {
-        FitRun first(a, stream), second(b, stream);
+        FitRun first(a, stream), second(b, stream, &first);
         if (!first.short_of_memory() && !second.short_of_memory()) {
             FitJobs jobs{};
             int n = 0;
             if (first.enqueue_buckets(jobs.job[n])) ++n;
-            if (second.enqueue_buckets(jobs.job[n])) ++n;
+            const bool overwritten = second.enqueue_buckets(jobs.job[n]) && b.room != nullptr;
+            if (second.iterated()) ++n;
             if (n != 0) {
                 fit_iterate_kernel<<<n, 1024, 0, stream>>>(jobs);
                 TQ_CUDA(cudaGetLastError());
             }
-            first.finish();
-            second.finish();
+            second.finish();   // (its samples in the room that they share, if any, are not needed any more)
+            first.finish(overwritten ? &samples_again : nullptr);
             return;
         }
     }

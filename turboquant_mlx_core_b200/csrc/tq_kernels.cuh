@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 namespace tq {
@@ -160,9 +161,11 @@ struct FitRequest {
     int bits, iterations;
     const float* init_centroids;  // host: 2^bits, ascending
     float *centroids_out, *boundaries_out;   // host; boundaries may be NULL
+    float* room = nullptr;        // n floats on the device that the fit may overwrite, instead of memory of its own
 };
 int launch_codebook_fit(const FitRequest& r, cudaStream_t stream);   // the iterations run
-void launch_codebook_fits(const FitRequest& a, const FitRequest& b, cudaStream_t stream);
+// b.room may be a's samples: `samples_again` then queues what fills them in once more, should the fit a need them after that.
+void launch_codebook_fits(const FitRequest& a, const FitRequest& b, const std::function<void()>& samples_again, cudaStream_t stream);
 void launch_layer_samples(const float* d_weight, const float* d_row_norms, long rows, int in, uint32_t block, uint32_t seed_p,
                           const float* primary_centroids, int n_primary, float* d_scaled, float* d_residual, cudaStream_t stream);
 
