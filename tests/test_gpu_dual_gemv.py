@@ -79,3 +79,30 @@ def test_two_rotations_zero_and_infinite_rows(tq):
     assert torch.equal(y[0], torch.zeros_like(y[0]))
     assert rel_l2(y[1].double().cpu(), (x[1].double() @ w.T).cpu()) < TOL
     assert not torch.isfinite(y[2]).any()
+
+
+@pytest.mark.parametrize("rows", [1, 5, 40])
+@pytest.mark.parametrize("odd", [float("inf"), float("nan")])
+def test_two_rotations_beside_a_centroid_that_is_not_finite(tq, rows, odd):
+    """A codebook entry that no weight uses, or one row alone, does not change the other rows, however small their centroids are."""
+    torch = pytest.importorskip("torch")
+    n_in, n_out, block = 512, 48, 128
+    rng = np.random.default_rng(rows)
+    primary = (np.sort(rng.standard_normal(16)) * 1e-6).astype(np.float32)
+    residual = (np.sort(rng.standard_normal(16)) * 1e-7).astype(np.float32)
+    primary[15] = odd
+    code = rng.integers(0, 15, (n_out, n_in))
+    code[7] = 15
+    other = rng.integers(0, 16, (n_out, n_in))
+    pack = lambda c: (c[:, 0::2] | (c[:, 1::2] << 4)).astype(np.uint8)
+    qw = tq.QuantizedWeight(pack(code), pack(other), np.full(n_out, 1e6, np.float32), np.array([11, 12, block], np.uint32))
+    lin = tq.TurboQuantLinear(n_in, n_out, qw, tq.codebook_from_centroids(primary), tq.codebook_from_centroids(residual), block)
+    back = torch.empty((n_out, n_in), device="cuda")
+    lin.dequantize(out=back)
+    x = torch.randn((rows, n_in), generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").half()
+    y = lin.forward(x)
+    keep = torch.arange(n_out, device="cuda") != 7
+    want = x.double() @ back[keep].double().T
+    assert rel_l2(y[:, keep].double().cpu(), want.cpu()) < TOL
+    assert not torch.isfinite(y[:, 7]).any()
+    lin.close()

@@ -103,8 +103,9 @@ public:
         // two rotations: both entries of a byte as a pair of fp16, the largest in [2^14, 2^15), rounded as the kernels round
         // to TF32 (ten mantissa bits, ties away from zero)
         float top = 0.0f;
-        for (const float t : tables) top = std::max(top, std::fabs(t));
-        if (dual_ && top > 0.0f && std::isfinite(top)) pair_unit_ = std::ldexp(1.0f, std::ilogb(top) - 14);
+        for (const float t : tables)
+            if (std::isfinite(t)) top = std::max(top, std::fabs(t));   // (an entry that is not finite stays what it is)
+        if (dual_ && top > 0.0f) pair_unit_ = std::ldexp(1.0f, std::ilogb(top) - 14);
         std::vector<float> words(tables);
         words.resize(768);
         for (int b = 0; b < 256; ++b) {
