@@ -1,5 +1,5 @@
-"""The sums over the splits of K, at the widths and row counts where the CTAs change from 32 to 64 and 128 threads and where
-the last one is not full."""
+"""The sums over the splits of K, at widths where the last CTA, warp or thread is not full, with fewer and with more splits than are
+requested at once."""
 import pytest
 
 pytestmark = pytest.mark.gpu

@@ -755,9 +755,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const _
 
 // y = fp16(norm * inv_scale * sum over K splits, in split order) - fixed order, run-to-run identical - for the matrices of a call
 // that were split (a group's by blockIdx.z).  Latency counts, it follows every split product of a decode batch: a thread takes four weight
-// rows, has their norms before the kernel in front has ended, and requests up to eight splits' sums at once.  (With one
+// rows, requests their norms before the kernel in front has ended, and then up to kBatch splits' sums at once.  (With one
 // element per thread, a 64-bit division for its place and the splits in turn: 7.9 us for 64 x 3584 in five splits under the
-// profiler, 4.7 here; 2048 x 512 twice in four splits 20.8, 15.4 here.)
+// profiler, 4.7 here; 2048 x 512 twice in four splits 20.8, 15.4 here.)  Calls in a graph, with one element per thread and here:
+// 4096 x 1024 at 16 rows 10.02 and 10.03 us, 2048 x 600 at 100 rows 11.1 and 11.1, 4096 x 4096 at 16 rows 13.34 and 13.33, 3584 x 512 at 64
+// rows 10.53 and 10.07, 8192 x 2048 at 9 rows 13.86 and 13.86.  With the norms' products in front of the wait and eight splits
+// at once the last two were 9.9 and 14.38, 4096 x 4096 13.61; with an early release of the kernel behind and CTAs of 32
+// threads on top of that, up to a microsecond more.
 struct FinishOne {
     const float* partial;
     const float* norms;
@@ -770,16 +774,13 @@ struct FinishArgs { FinishOne m[kMaxGemmGroup]; };
 constexpr int kFinishThreads = 128;
 __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m) {
     const int out = f.out, k_splits = f.k_splits;
-    const int c = 4 * static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    const int c = 4 * static_cast<int>(blockIdx.x * kFinishThreads + threadIdx.x);
     if (c >= out) return;
-    // The kernel behind is set up beside the product in front: it waits for this one, and so for that one, before it touches
-    // anything (0.2 us a call; the CTAs here are small and leave it room).
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    float scale[4];
+    float norm[4];   // (used behind the wait only: a product with it in front of the wait would wait for it there)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) scale[k] = c + k < out ? __ldg(f.norms + c + k) * f.inv_scale : 0.f;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr int kBatch = 8;
+    for (int k = 0; k < 4; ++k) norm[k] = c + k < out ? __ldg(f.norms + c + k) : 0.f;
+    pdl_wait_release();
+    constexpr int kBatch = 12;
     const size_t split = static_cast<size_t>(m) * out;
     for (int row = blockIdx.y; row < m; row += gridDim.y) {
         const float* const src = f.partial + static_cast<size_t>(row) * out + c;
@@ -797,7 +798,8 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m) {
                         acc[0] += v[z].x; acc[1] += v[z].y; acc[2] += v[z].z; acc[3] += v[z].w;
                     }
             }
-            const __half2 lo = __floats2half2_rn(acc[0] * scale[0], acc[1] * scale[1]), hi = __floats2half2_rn(acc[2] * scale[2], acc[3] * scale[3]);
+            const __half2 lo = __floats2half2_rn(acc[0] * (norm[0] * f.inv_scale), acc[1] * (norm[1] * f.inv_scale));
+            const __half2 hi = __floats2half2_rn(acc[2] * (norm[2] * f.inv_scale), acc[3] * (norm[3] * f.inv_scale));
             *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
         } else {
             for (int z = 0; z < k_splits; ++z)
@@ -806,7 +808,7 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m) {
                     if (c + k < out) acc[k] += __ldcg(src + z * split + k);
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (c + k < out) y[k] = __float2half_rn(acc[k] * scale[k]);
+                if (c + k < out) y[k] = __float2half_rn(acc[k] * (norm[k] * f.inv_scale));
         }
     }
 }
@@ -823,16 +825,11 @@ void launch_finish(const FinishArgs& f, int n, int m, int sm_count, cudaStream_t
     if (n == 0) return;
     int widest = 0;
     for (int i = 0; i < n; ++i) widest = std::max(widest, f.m[i].out);
-    // Sums of a few rows by CTAs of fewer threads, until every SM reads a share of them.  With that, the parameters of a single
-    // matrix and the early release: a call of 4096 x 1024 at 16 rows 10.85 -> 10.64 us (9.73 -> 9.35 in a graph), of 2048 x 600 at
-    // 100 rows 11.48 -> 11.03 (10.63 -> 10.09).
-    int threads = kFinishThreads;
-    while (threads > 32 && static_cast<long>((widest + 4 * threads - 1) / (4 * threads)) * m * n < sm_count) threads >>= 1;
-    const int gx = (widest + 4 * threads - 1) / (4 * threads);
+    const int gx = (widest + 4 * kFinishThreads - 1) / (4 * kFinishThreads);
     const int gy = std::max(1, std::min(m, 16 * sm_count / (gx * n)));   // sixteen CTAs per SM: one wave
     const dim3 grid(static_cast<unsigned int>(gx), static_cast<unsigned int>(gy), static_cast<unsigned int>(n));
-    if (n == 1) launch_pdl(gemm_finish_kernel, grid, dim3(threads), 0, stream, f.m[0], m);
-    else launch_pdl(gemm_finish_group_kernel, grid, dim3(threads), 0, stream, f, m);
+    if (n == 1) launch_pdl(gemm_finish_kernel, grid, dim3(kFinishThreads), 0, stream, f.m[0], m);
+    else launch_pdl(gemm_finish_group_kernel, grid, dim3(kFinishThreads), 0, stream, f, m);
 }
 
 // Groups of 8 rows that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
