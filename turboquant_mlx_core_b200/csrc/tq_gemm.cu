@@ -477,7 +477,11 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         };
         auto fetch_place = [&] {
             const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3) + (DUAL ? sub : 0);
-            const int kb = kb_base + kBlocksPerStage * f_it + (DUAL ? 0 : sub);
+            int kb = kb_base + kBlocksPerStage * f_it + (DUAL ? 0 : sub);
+            // A last stage without a second block: an address inside the row all the same (it is not read).  The bound also has the
+            // compiler order the producers' loop better: 5120 x 55296 at 16 rows 69.7 us without it, 68.8 with it, 3584 x 37888 at
+            // 64 rows 40.7 and 40.0.
+            if (!DUAL && kb >= kb_per_plane) kb -= kb_per_plane;
             f_ptr0 = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
             if constexpr (!DUAL) f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
         };
