@@ -50,3 +50,64 @@ def test_all_gather_of_layers_rotated_in_front(tq, block, shared, batch):
         lins[r].check_status()
         L.tq_exchange_free(ex[r])
         lins[r].close()
+
+
+def waiting_layer(tq, torch, L, block, shared, batch):
+    """A layer, its exchange, a gathered buffer with flags, and two flags to wait for in page-locked memory, not raised."""
+    rows, cols = 144, 1024
+    g = torch.Generator(device="cuda").manual_seed(batch + block)
+    c = tq.generate_codebook(4)
+    w = torch.randn((rows, cols), generator=g, device="cuda") * 0.02
+    lin = tq.TurboQuantLinear(cols, rows, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, block, shared)), c, c, block)
+    ex = L.tq_exchange_create(0, 2)
+    buf = torch.zeros(batch * 2 * rows * 2 + 256, dtype=torch.uint8, device="cuda")
+    x, late = (torch.randn((batch, cols), generator=g, device="cuda").half() for _ in range(2))
+    raised = torch.zeros(32, dtype=torch.int32).pin_memory()
+
+    def forward():
+        flags = buf.data_ptr() + batch * 2 * rows * 2
+        return L.tq_linear_forward_allgather(lin.handle, ex, C.c_void_p(x.data_ptr()), batch, pointers([buf.data_ptr()]), 1, 2 * rows, 0,
+                                             pointers([flags]), 1, C.c_void_p(raised.data_ptr()), 2, None)
+
+    def result():
+        return buf[:batch * 2 * rows * 2].view(torch.float16).view(batch, 2 * rows)[:, :rows]
+
+    return lin, ex, x, late, raised, forward, result
+
+
+@pytest.mark.parametrize("block,shared", [(512, True), (128, False), (512, False)], ids=["wide", "dual", "wide_dual"])
+@pytest.mark.parametrize("batch", [1, 3, 8])
+def test_the_rotation_reads_what_arrives_before_the_flags(tq, block, shared, batch):
+    """The forward is queued while its flags are low; then the copy engine brings another activation, and the host raises the flags (well
+    within the second that the kernel waits)."""
+    torch = pytest.importorskip("torch")
+    L = tq.load()
+    lin, ex, x, late, raised, forward, result = waiting_layer(tq, torch, L, block, shared, batch)
+    old, want = lin.forward(x), lin.forward(late)
+    assert not torch.equal(old, want)
+    arriving = late.cpu().pin_memory()
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    assert forward() == 0, L.tq_last_error().decode()
+    with torch.cuda.stream(side):
+        x.copy_(arriving, non_blocking=True)
+    side.synchronize()
+    raised.fill_(1)
+    torch.cuda.synchronize()
+    lin.check_status()
+    assert torch.equal(result(), want)
+    L.tq_exchange_free(ex)
+    lin.close()
+
+
+def test_flags_that_are_never_raised(tq):
+    """The wait in front of the rotation ends after a second, with the status of a lost peer."""
+    torch = pytest.importorskip("torch")
+    L = tq.load()
+    lin, ex, x, _, _, forward, _ = waiting_layer(tq, torch, L, 512, False, 3)
+    torch.cuda.synchronize()
+    assert forward() == 0, L.tq_last_error().decode()
+    with pytest.raises(tq.TQError, match="peer wait"):
+        lin.check_status()
+    L.tq_exchange_free(ex)
+    lin.close()
