@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __
 
 // Adds the splits' partial results of one query head.  Bound by latency, a few hundred KB from L2: with a thread per dim that went
 // through the splits in turn, weights and all, 28 heads of 111 splits took 21 us after the attention kernel's 46.  Here the
-// splits' weights are found once, a thread each (at most kMaxSplits), and kCombineRows rows of sixteen-byte loads run side
+// splits' weights are found once, a thread each (at most kMaxSplits), and kRows rows of sixteen-byte loads run side
 // by side, added up in a fixed order: 2 to 3 us.
 constexpr int kMaxSplits = 256;
 constexpr int kCombineThreads = 256;

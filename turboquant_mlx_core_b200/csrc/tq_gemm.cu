@@ -355,7 +355,7 @@ struct GemmArgs {
     long y_stride;
     float* partial;         // [k_splits, m, out] fp32 un-scaled partial sums (only when k_splits > 1)
     unsigned int* status;   // device error word (0 = ok)
-    int out, in, m, n_planes;
+    int out, in, m;
     int k_splits;           // CTAs along K per output tile (gridDim.z)
     float inv_scale;
 };
@@ -762,8 +762,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const _
 // rows, requests their norms before the kernel in front has ended, and then up to kBatch splits' sums at once.  (With one
 // element per thread, a 64-bit division for its place and the splits in turn: 7.9 us for 64 x 3584 in five splits under the
 // profiler, 4.7 here; 2048 x 512 twice in four splits 20.8, 15.4 here.)  Calls in a graph, with one element per thread and here:
-// 4096 x 1024 at 16 rows 10.02 and 10.03 us, 2048 x 600 at 100 rows 11.1 and 11.1, 4096 x 4096 at 16 rows 13.34 and 13.33, 3584 x 512 at 64
-// rows 10.53 and 10.07, 8192 x 2048 at 9 rows 13.86 and 13.86.  With the norms' products in front of the wait and eight splits
+// 4096 x 1024 at 16 rows 10.0 and 10.1 us, 2048 x 600 at 100 rows 11.2 and 11.2, 4096 x 4096 at 16 rows 13.35 and 13.35, 3584 x 512 at 64
+// rows 10.5 and 10.1, 8192 x 2048 at 9 rows 13.87 and 13.87.  With the norms' products in front of the wait and eight splits
 // at once the last two were 9.9 and 14.38, 4096 x 4096 13.61; with an early release of the kernel behind and CTAs of 32
 // threads on top of that, up to a microsecond more.
 struct FinishOne {
@@ -930,7 +930,7 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     // 2. the GEMM
     GemmArgs a{};
     a.codes = codes; a.norms = norms; a.table = table; a.xrot = xrot; a.y = y; a.y_stride = y_stride; a.status = status;
-    a.out = out; a.in = in; a.m = static_cast<int>(m); a.n_planes = n_planes;
+    a.out = out; a.in = in; a.m = static_cast<int>(m);
     a.inv_scale = 1.0f / std::sqrt(static_cast<float>(in));
     if (n_planes == 2) {
         a.table += 512;   // (the pairs, behind the two tables)
@@ -938,7 +938,6 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     }
     a.k_splits = gemm_k_splits(out, in, m, n_planes, sm_count);
     a.partial = a.k_splits > 1 ? reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + xrot_bytes(in, m, n_planes)) : nullptr;
-    // stages + tables + worst-case padding in front of the 32 KB-aligned tables
     const size_t smem = kGemmSmemBytes;
     static bool configured[64] = {false};
     int dev = 0;
@@ -984,7 +983,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         GemmArgs& a = grp.m[i];
         a.codes = it.codes; a.norms = it.norms; a.table = it.table; a.y = it.y; a.y_stride = it.out; a.status = it.status;
         a.xrot = static_cast<__half*>(it.scratch);
-        a.out = it.out; a.in = in; a.m = static_cast<int>(m); a.n_planes = n_planes;
+        a.out = it.out; a.in = in; a.m = static_cast<int>(m);
         a.inv_scale = 1.0f / std::sqrt(static_cast<float>(in));
         if (n_planes == 2) {
             a.table += 512;

@@ -376,10 +376,6 @@ __device__ __forceinline__ void ldg_stream_if(uint4& v, const uint8_t* p, bool p
         : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
         : "l"(p), "r"(static_cast<uint32_t>(pred)));
 }
-__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -1450,8 +1446,8 @@ void* gemv_static_scratch_address() { return static_scratch_address(); }
 void launch_tq8_gemv_static(const uint8_t* codes, const float* norms, const float* table, const __half* x, __half* y,
                             int out, int in, int batch, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p,
                             uint32_t seed_r, unsigned int* status, int sm_count, cudaStream_t stream) {
-    // Which layers are taken: those whose planes would fit as partial-sum slots of their own (layers with two rotations need
-    // less than that).
+    // Which layers are taken, and what an error counts: those whose planes would fit as partial-sum slots of their own.  (Layers with
+    // two rotations need less by now; a layer that was refused here still is.)
     const size_t asked = scratch_bytes(out, in, n_planes, chunk_count(in) * n_planes), need = gemv_scratch_bytes(out, in, n_planes);
     if (asked > kStaticScratchBytes)
         throw Error("allocation-free forward: this layer needs " + std::to_string(asked) +
