@@ -666,31 +666,30 @@ public:
         n_buckets_ = 1 << key_bits;
         n_groups_ = n_buckets_ / kFitGroup;
         const int n_parts = n_buckets_ / kFitSumBuckets;
-        bucketed_ = r.n < (1L << 31);
-        if (bucketed_) {
-            try {
-                bucket_buf_.reserve(static_cast<size_t>(n_buckets_) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups_) * 8 + static_cast<size_t>(n_groups_) * 4, stream);
-                if (r.room == nullptr) sorted_buf_.reserve(static_cast<size_t>(r.n) * 4, stream);
-            } catch (const OutOfMemory&) {
-                bucketed_ = false;   // the passes over all samples need next to nothing
-            }
-        }
+        const size_t bucket_bytes = static_cast<size_t>(n_buckets_) * (8 + 3 * 4) + static_cast<size_t>(n_parts + n_groups_) * 8 + static_cast<size_t>(n_groups_) * 4;
         // exponents of the window; without memory for the CTAs' places all counters are in L2
         window_ = std::min(kWindowExponents, kWindowSlots >> (24 - shift_));
         window_ctas_ = static_cast<int>(std::min<long>(sms_, (r.n + kWindowTile - 1) / kWindowTile));
+        bucketed_ = r.n < (1L << 31);
         windowed_ = bucketed_ && r.n >= static_cast<long>(kFitCrowd);
-        if (windowed_ && lender != nullptr && lender->windowed_ && lender->begin_bytes() >= begin_bytes()) {
-            begin_ = lender->begin_;
-        } else if (windowed_) {
-            begin_buf_.set_first_to_go();
+        const bool lent = windowed_ && lender != nullptr && lender->windowed_ && lender->begin_bytes() >= begin_bytes();
+        bucket_buf_.set_first_to_go();
+        for (;;) {
+            // (one block for the buckets and the places behind them: a cudaMalloc less in a first call)
+            const size_t places_at = (bucket_bytes + 255) / 256 * 256;
             try {
-                begin_buf_.reserve(begin_bytes(), stream);
+                if (bucketed_) bucket_buf_.reserve(windowed_ && !lent ? places_at + begin_bytes() : bucket_bytes, stream);
+                if (bucketed_ && r.room == nullptr) sorted_buf_.reserve(static_cast<size_t>(r.n) * 4, stream);
             } catch (const OutOfMemory&) {
-                windowed_ = false;
+                bucket_buf_.set_idle();
+                bucket_buf_.release();
+                if (windowed_) windowed_ = false;
+                else bucketed_ = false;   // the passes over all samples need next to nothing
+                continue;
             }
-            begin_ = begin_buf_.as<unsigned int>();
+            if (windowed_) begin_ = lent ? lender->begin_ : reinterpret_cast<unsigned int*>(bucket_buf_.as<uint8_t>() + places_at);
+            break;
         }
-        if (lender != nullptr) bucket_buf_.set_first_to_go();   // (fits one after the other make do with the lender's)
     }
     bool iterated() const { return iterated_; }
     bool short_of_memory() const { return active_ && (!bucketed_ || (!windowed_ && r_.n >= static_cast<long>(kFitCrowd))) && r_.n < (1L << 31); }
@@ -741,7 +740,7 @@ public:
                 if (samples_again != nullptr) (*samples_again)();
                 go_over_all();
             }
-            for (DeviceBuffer* b : {&state_buf_, &bucket_buf_, &sorted_buf_, &begin_buf_}) b->set_idle();
+            for (DeviceBuffer* b : {&state_buf_, &bucket_buf_, &sorted_buf_}) b->set_idle();
         }
         for (int i = 0; i < nc_; ++i) r_.centroids_out[i] = h_.centroids[i];
         if (r_.boundaries_out)
@@ -784,7 +783,7 @@ private:
     const cudaStream_t stream_;
     const int nc_;
     FitState h_{};
-    DeviceBuffer state_buf_, bucket_buf_, sorted_buf_, begin_buf_;
+    DeviceBuffer state_buf_, bucket_buf_, sorted_buf_;
     bool active_ = false, bucketed_ = false, windowed_ = false, iterated_ = false;
     int dev_ = 0, sms_ = 148, shift_ = 0, n_buckets_ = 0, n_groups_ = 0, window_ = 0, window_ctas_ = 0;
     unsigned int* begin_ = nullptr;   // where each CTA's samples of a bucket begin
