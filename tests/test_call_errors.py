@@ -18,6 +18,13 @@ def test_no_caches():
         tq.compressed_attention([], 0, rows(1))
 
 
+@pytest.mark.parametrize("columns,block,what", [(34, 32, "divisible"), (66, 64, "divisible"), (48, 48, "power of two"), (64, 16, "power of two")])
+def test_layer_fits_of_odd_shapes(columns, block, what):
+    """The reason is the shape's, whatever the kernels in front of it want."""
+    with pytest.raises(tq.TQError, match=what):
+        tq.fit_layer_codebooks(np.ones((4, columns), np.float32), block)
+
+
 @pytest.mark.gpu
 def test_host_rows_where_device_rows_are_needed():
     torch = pytest.importorskip("torch")

@@ -209,6 +209,8 @@ int tq_fit_layer_codebooks(const float* weight, int out_features, int in_feature
         const bool need_residual = residual_bits > 0;
         const float* cr0 = need_residual ? analytic_centroids(residual_bits) : nullptr;
         TQ_REQUIRE(!need_residual || (cr0 && residual_centroids), "tq_fit_layer_codebooks: bad residual bit width or NULL output");
+        TQ_REQUIRE(is_pow2(block) && block >= 32 && block <= 1024, "block_size must be a power of two in [32, 1024]");
+        TQ_REQUIRE(in_features % static_cast<int>(block) == 0, "in_features must be divisible by block_size");
         auto st = static_cast<cudaStream_t>(stream);
         const size_t n = static_cast<size_t>(out_features) * in_features;
         DeviceBuffer w_stage, norms, scaled, resid;
