@@ -673,7 +673,6 @@ public:
         bucketed_ = r.n < (1L << 31);
         windowed_ = bucketed_ && r.n >= static_cast<long>(kFitCrowd);
         const bool lent = windowed_ && lender != nullptr && lender->windowed_ && lender->begin_bytes() >= begin_bytes();
-        bucket_buf_.set_first_to_go();
         for (;;) {
             // (one block for the buckets and the places behind them: a cudaMalloc less in a first call)
             const size_t places_at = (bucket_bytes + 255) / 256 * 256;

@@ -76,8 +76,7 @@ bool stream_is_capturing(cudaStream_t st);
 // otherwise the block is idle when the call returns.
 void* pool_alloc(size_t bytes, int device, cudaStream_t st, bool on_stream);
 // idle: nothing queued anywhere uses the block; otherwise everything that does was put on the legacy default stream.
-// first_to_go: the block gives way before all others when too much is kept.
-void pool_release(void* p, size_t bytes, int device, bool idle, bool first_to_go = false);
+void pool_release(void* p, size_t bytes, int device, bool idle);
 size_t pool_trim();   // the bytes that went back to the driver
 struct OutOfMemory : Error {
     using Error::Error;
@@ -134,8 +133,6 @@ public:
     void owned_by(const StreamUse* use) { use_ = use; }
     // Nothing queued uses the contents any more: the release need not wait.
     void set_idle() { idle_ = true; }
-    // Scratch that makes a call faster but is not worth another object's kept memory.
-    void set_first_to_go() { first_to_go_ = true; }
 
     // Grow-only: keeps the allocation when it is already large enough (contents kept
     // only in that case).
@@ -152,7 +149,7 @@ public:
                 cudaDeviceSynchronize();
                 if (cur >= 0 && cur != device_) cudaSetDevice(cur);
             }
-            pool_release(p_, n_, device_, idle_ || !legacy, first_to_go_);
+            pool_release(p_, n_, device_, idle_ || !legacy);
         }
         p_ = nullptr;
         n_ = 0;
@@ -171,7 +168,7 @@ private:
         n_ = bytes;
     }
     void take(DeviceBuffer& o) {
-        p_ = o.p_; n_ = o.n_; device_ = o.device_; use_ = o.use_; idle_ = o.idle_; first_to_go_ = o.first_to_go_;
+        p_ = o.p_; n_ = o.n_; device_ = o.device_; use_ = o.use_; idle_ = o.idle_;
         o.p_ = nullptr;
         o.n_ = 0;
         o.idle_ = false;
@@ -180,7 +177,7 @@ private:
     size_t n_ = 0;
     int device_ = 0;
     const StreamUse* use_ = nullptr;
-    bool idle_ = false, first_to_go_ = false;
+    bool idle_ = false;
 };
 
 // ---- host memory (tq_host_copy.cu) ---------------------------------------------------------------

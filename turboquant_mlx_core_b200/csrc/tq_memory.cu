@@ -6,7 +6,7 @@
 // kept here instead, by device and size class, and handed out again.
 //
 //   Bounded    at most kKeepBytes of unused memory per device; beyond it the blocks unused for longest go back to the
-//              driver first, before them those whose owner said so.  A block of more than half the bound is never kept.
+//              driver first.  A block of more than half the bound is never kept.
 //   Given back blocks unused for kKeepSeconds at the next release; everything unused when an allocation of the library fails,
 //              and when the program asks for it (tq_release_cached_memory), which it does for another allocator's sake.
 //   Threads    one mutex; a block belongs to one owner at a time.
@@ -59,7 +59,7 @@ struct Pool {
     std::mutex mu;
     std::vector<Pinned> pinned;   // page-locked staging, the latest last
     size_t pinned_kept = 0;
-    std::list<Block> blocks;   // in the order in which they go back: the first to go, then by release, the oldest first
+    std::list<Block> blocks;   // in order of release: the oldest first
     size_t kept[64] = {0};
     std::list<Word> words;
     std::vector<cudaEvent_t> events[64];   // spare events of each device
@@ -194,7 +194,7 @@ void* device_malloc(size_t bytes) {
     return p;
 }
 
-void pool_release(void* p, size_t bytes, int device, bool idle, bool first_to_go) {
+void pool_release(void* p, size_t bytes, int device, bool idle) {
     if (!p) return;
     const size_t size = pool_size_class(bytes);
     Pool& P = pool();
@@ -209,11 +209,12 @@ void pool_release(void* p, size_t bytes, int device, bool idle, bool first_to_go
         return;
     }
     const double now = now_s();
-    P.blocks.insert(first_to_go ? P.blocks.begin() : P.blocks.end(), Block{p, size, device, e, now});
+    P.blocks.push_back(Block{p, size, device, e, now});
     P.kept[device] += size;
-    for (auto it = P.blocks.begin(); it != P.blocks.end();) {
+    while (!P.blocks.empty() && now - P.blocks.front().since > kKeepSeconds) free_block(P, P.blocks.begin());
+    for (auto it = P.blocks.begin(); P.kept[device] > kKeepBytes && it != P.blocks.end();) {
         auto next = std::next(it);
-        if (now - it->since > kKeepSeconds || (it->device == device && P.kept[device] > kKeepBytes)) free_block(P, it);
+        if (it->device == device) free_block(P, it);
         it = next;
     }
 }
