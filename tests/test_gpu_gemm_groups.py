@@ -1,0 +1,29 @@
+"""The many-row linear's three groups of dequantising warps: fewer stages (128 columns each, 64 with two rotations) than groups, one and two
+more than a multiple of three, a last stage of one K block, and the stages of several tiles running on through the ring.  Tolerance: as at
+the tile edges, three independent roundings to fp16, 2^-11 * sqrt(3 / 3)."""
+import numpy as np
+import pytest
+
+from tests.conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# columns, weight rows, activation rows, shared rotation
+CASES = [(64 * k, 130, 9 + 60 * k, k % 3 != 0) for k in range(1, 12)]
+CASES += [(128, 38000, 9, True), (192, 38000, 65, True), (448, 19100, 129, True), (128, 19100, 40, False), (320, 19100, 256, True)]
+
+
+@pytest.mark.parametrize("cols,rows,m,shared", CASES)
+def test_stages_and_groups(tq, oracle, cols, rows, m, shared):
+    import torch
+    rng = np.random.default_rng(rows + cols + m)
+    cb = oracle.codebook(4)[0]
+    w = (rng.standard_normal((rows, cols)) * 0.02).astype(np.float16).astype(np.float32)
+    pp, pr, norms, seeds = oracle.quantize_weight(w, cb, cb, 4, 4, 64, shared)
+    x = rng.standard_normal((m, cols)).astype(np.float16)
+    c = tq.codebook_from_centroids(cb)
+    lin = tq.TurboQuantLinear(cols, rows, tq.QuantizedWeight(pp, pr, norms, seeds), c, c, 64)
+    y = lin.forward(torch.from_numpy(x).cuda()).cpu().numpy()
+    assert rel_l2(y, oracle.linear_from_dequant(oracle.dequantize_weight(pp, pr, norms, seeds, cb, cb, 64), x.astype(np.float32))) < 4.9e-4
+    lin.check_status()
+    lin.close()

@@ -16,8 +16,8 @@
 //   D[128 x 256] (TMEM, fp32) += A[128 x 64] (weights, fp16, TMEM) . B[256 x 64]^T (xrot, fp16, smem)
 // per 64-column K block, as four tcgen05.mma (M 128, N 256, K 16) issued by one thread.
 //   A pipeline stage is 128 K columns (two 64-column K blocks), the ring has up to four stages.
-//   warps 0-15 producers in two groups of eight; group g takes the stages g, g + 2, ...: codes HBM ->
-//              registers (two of the group's stages ahead) -> lookup (lane-private fp16 table in
+//   warps 0-23 producers in three groups of eight; group g takes the stages g, g + 3, ...: codes HBM ->
+//              registers (the group's next stage, as the present one's are used up) -> lookup (lane-private fp16 table in
 //              shared memory) -> weight tile in TENSOR memory (tcgen05.st, 64 columns of fp16 pairs per
 //              stage).  The store's 16x256b shape takes registers in the fragment order (lane / 4 = row,
 //              lane % 4 = columns), so a code load of a warp is 512 contiguous bytes; with a row per lane
@@ -25,20 +25,22 @@
 //              also load with a wavefront per 32 weights, was the bound (5120 x 55296: 110 -> 89 us at 32
 //              rows, 644 -> 547 us at 1024).  The K order this gives is free: the rotation kernels write
 //              the activations in the same one (k_position).
-//   warp 17    activation tiles: the rotation kernel stores xrot in operand-tile order, so a K block
+//   warp 25    activation tiles: the rotation kernel stores xrot in operand-tile order, so a K block
 //              of a tile is one contiguous bulk copy (cp.async.bulk, mbarrier complete_tx) of 128
 //              bytes per activation row of the tile
-//   warp 16    one thread: waits for a stage (ONE barrier collects the producers' arrivals and the
-//              copies' bytes), issues its eight MMAs, commits to the stage's "empty" barrier.  The
-//              serial chain of this thread (wait, fence, issue, commit) is what bounds the kernel when
-//              the MMAs are short, hence few and long stages.
-//   warps 18-21 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
+//   warp 24    waits for a stage (ONE barrier collects the producers' arrivals and the copies' bytes); one
+//              elected lane issues its eight MMAs and commits to the stage's "empty" barrier.  This serial
+//              chain (wait, fence, issue, commit) bounds the kernel when the MMAs are short, hence few and
+//              long stages.
+//   warps 26-29 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
 //              next tile's products (up to 128 activation rows: two accumulators in turn; above, the next
 //              tile's first MMA waits until this one is read)
 // A CTA per SM walks the output tiles (of a single matrix; a group's matrices have a CTA per tile) and its ring of stages runs on from tile to tile: with a CTA per
 // tile, set-up, first loads and epilogue took 8 to 18 of 47 thousand cycles (5120 x 55296: 89 -> 76 us at
-// 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the producers bound it (about 500 cycles per 128 x 64
-// weights), at 256 the shared-memory pipe: lookups, code loads, the activation tile's write and its read.
+// 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the shared-memory pipe bounds it: 256 cycles of lookups and 64 of code loads
+// per 128 x 64 weights, 32 to 128 more for the activation tile, of the 400 to 450 that they take; at 16 rows that is 86 % of what the
+// memory delivers.  At 256 it is the same pipe: lookups, code loads, the activation tile's write and its read.  What a call costs besides
+// its stages is some 8 us: the rotation in front and its end, the CTA's set-up, the first codes, the epilogue.
 // The activation tile is as tall as the rows it really has (in steps of 16): a decode batch of 9..64
 // rows costs a short MMA and a short copy, so the codes are streamed once whatever the batch.
 // The dequantised weights never touch HBM; a weight tile is looked up once per 256 activation
@@ -68,7 +70,7 @@ constexpr int kTileTok = 256;   // activation rows per CTA (MMA N)
 constexpr int kBlockK = 64;     // columns of a K block
 constexpr int kSubPerStage = 2; // K blocks per pipeline stage: a stage is 128 K columns
 constexpr int kStagesMax = 4;   // ring of stages: weight tiles in tensor memory (4 x 64 columns), activation tiles in shared memory (as many as fit)
-constexpr int kGroups = 2;      // producer groups of eight warps: group g dequantises the stages g, g + 2, ...
+constexpr int kGroups = 3;      // producer groups of eight warps: group g dequantises the stages g, g + 3, ...
 constexpr int kProducerWarps = 8 * kGroups;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kMmaWarp = kProducerWarps;       // issues the MMAs, owns the tensor-memory allocation
@@ -84,6 +86,10 @@ constexpr uint32_t kTmemAStageCols = kSubPerStage * kTmemASubCols;
 constexpr uint32_t kLutWin = 0x800u;  // window address of the lookup tables (an immediate of the lookup's load)
 // Everything an SM can give one CTA: tables at kLutWin, then three 64 KB stages for a 256-row tile.
 constexpr size_t kGemmSmemBytes = 232448 - 512;
+// What a launch of m activation rows needs of it (an SM is set up faster for less: 3584 x 37888 at 16 rows 32.9 us with all of it, 32.4 so).
+size_t gemm_smem_bytes(long m) {
+    return std::min(kGemmSmemBytes, kLutWin + kLutBytes + kStagesMax * kSubPerStage * static_cast<size_t>(std::min<long>(kTileTok, (m + 15) / 16 * 16)) * kBlockK * 2);
+}
 constexpr unsigned long long kGemmWaitLimitNs = 200ull * 1000 * 1000;
 
 // instruction descriptor: D fp32, A and B fp16, both K-major, M = 128, N = n (a multiple of 16 up to 256)
@@ -104,15 +110,16 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait; gives up at once when another thread has already flagged a failure.
+// Bounded wait; gives up at once when another thread has already flagged a failure.  (Without a time to sleep: with 20 us of it
+// 3584 x 37888 at 16 rows took 35.3 us instead of 34.2.)
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile unsigned int* abort_flag) {
     unsigned long long t0 = 0;
     for (uint32_t spin = 0;; ++spin) {
         uint32_t done;
         asm volatile(
-            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+            "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
             : "=r"(done)
-            : "r"(bar), "r"(parity), "r"(20000u)   // ns that the thread may sleep
+            : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
         if ((spin & 15) == 15 && *abort_flag) return false;
@@ -164,11 +171,18 @@ __device__ __forceinline__ void tmem_st_16x256b(uint32_t taddr, const uint32_t (
                  : "r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-// Codes are read once per 256 activation rows: they pass by the first-level cache.
-__device__ __forceinline__ uint4 load_codes16(const uint8_t* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
+// 16 bytes of codes where `want`, in place: the registers are neither copied nor chosen between.  Codes are read once per 256
+// activation rows: they pass by the first-level cache.
+__device__ __forceinline__ void load_codes16_if(uint4& v, const uint8_t* p, bool want) {
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %5, 0; @p ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4]; }"
+                 : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(p), "r"(static_cast<uint32_t>(want)));
+}
+// One lane of a converged warp.  The compiler knows that it is one, so that the operands of the tensor and copy instructions behind
+// it are uniform; behind `lane == 0` each MMA took some hundred cycles to issue (3584 x 37888 at 16 rows 38.3 us, 35.4 with this).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+    return p != 0;
 }
 // Waits for this thread's tensor-memory stores and orders them before the barrier arrival that follows.
 __device__ __forceinline__ void tmem_st_publish() {
@@ -398,13 +412,18 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     const uint32_t smem_end = raw + dyn_bytes;
     int n_st = smem_end > stage0 ? static_cast<int>((smem_end - stage0) / stage_bytes) : 0;
     if (n_st > kStagesMax) n_st = kStagesMax;
-    if (raw > kLutWin || n_st < 2) {  // layout does not fit: refuse to run (nothing allocated yet)
+    if (raw > kLutWin || n_st < kGroups) {  // layout does not fit: refuse to run (nothing allocated yet)
         if (tid == 0) raise_status(p.status, 9u);
         return;
     }
     const uint32_t bar_full = smem_addr(&s_full[0]), bar_empty = smem_addr(&s_empty[0]);
     const uint32_t bar_acc_full = smem_addr(&s_accum_full[0]), bar_acc_empty = smem_addr(&s_accum_empty[0]);
 
+    // the table's entries are asked for first: they come while the barriers and the tensor memory are set up
+    constexpr int kTableSteps = (256 * 8 + kGemmThreads - 1) / kGemmThreads;
+    float table_entry[kTableSteps];
+#pragma unroll
+    for (int k = 0; k < kTableSteps; ++k) table_entry[k] = __ldg(p.table + min(255, (tid + k * kGemmThreads) >> 3));
     if (tid == 0) {
         for (int s = 0; s < kStagesMax; ++s) {
             bar_init(bar_full + 8u * s, kProducerWarps / kGroups + 1);   // one arrival per producer warp of the group + the copy thread
@@ -424,12 +443,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // lookup table: entry e, lane copy l at kLutWin + e * 128 + l * 4, value (t, t) or (primary, residual) as fp16
-    for (int i = tid; i < 256 * 8; i += kGemmThreads) {
-        const int e = i >> 3, c4 = (i & 7) * 4;
-        const float t = __ldg(p.table + e);
-        const uint32_t v = DUAL ? __float_as_uint(t) : static_cast<uint32_t>(__half_as_ushort(__float2half_rn(t))) * 0x00010001u;
-        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kLutWin + static_cast<uint32_t>(e) * 128u + c4 * 4u), "r"(v)
-                     : "memory");
+#pragma unroll
+    for (int k = 0; k < kTableSteps; ++k) {
+        const int i = tid + k * kGemmThreads, e = i >> 3, c4 = (i & 7) * 4;
+        const uint32_t v = DUAL ? __float_as_uint(table_entry[k]) : static_cast<uint32_t>(__half_as_ushort(__float2half_rn(table_entry[k]))) * 0x00010001u;
+        if (i < 256 * 8)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(kLutWin + static_cast<uint32_t>(e) * 128u + c4 * 4u), "r"(v)
+                         : "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -448,11 +468,14 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     if (warp < kProducerWarps) {
         // ---- producers ------------------------------------------------------------------------
         // Weight tile in tensor memory: lane = row of the tile, 64 columns per stage (two fp16 per
-        // column, 128 K columns).  A warp may touch lanes 32 * (warp % 4) .. + 31.  The 16 producer
-        // warps form two groups of eight (warp / 8); inside a group warp w takes the rows of lane
+        // column, 128 K columns).  A warp may touch lanes 32 * (warp % 4) .. + 31.  The 24 producer
+        // warps form three groups of eight (warp / 8); inside a group warp w takes the rows of lane
         // quarter w % 4 and the K block (w / 4) % 2 of the stage; group g dequantises the stages g,
-        // g + 2, ...  A thread turns 64 codes, 16 of each of four rows, into fp16 pairs.  (With two rotations the two warps
+        // g + 3, ...  A thread turns 64 codes, 16 of each of four rows, into fp16 pairs.  (With two rotations the two warps
         // of a lane quarter take 16 of its rows each, and 32 codes a thread make as many pairs.)
+        // Three groups with one stage in registers each, not two with two: all warps share the pipe of the lookups, and a stage
+        // costs a warp some 700 cycles beside them (its turn at the barriers, the tensor-memory stores, the next loads), in which
+        // with two groups the pipe was idle half of the time.  5120 x 55296 at 32 rows 66.2 -> 61.6 us, 4096 x 4096 at 16 12.4 -> 12.1.
         const int sub = (warp >> 2) & 1;             // which K block of the stage, or which 16 rows
         constexpr int kLoads = DUAL ? 2 : 4;
         const int grp = warp >> 3;
@@ -465,77 +488,66 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                                  (DUAL ? 0u : kTmemASubCols * static_cast<uint32_t>(sub));
         const int n_stages = n_local * n_it;
 
-        // The group's next stage to fetch: place in its tile, codes of its two code tiles, stages left.  Two of the group's
-        // stages are in registers or on their way.
-        int f_it = grp, f_t = t0, f_left = n_stages - grp;
-        const uint8_t *f_ptr0, *f_ptr1;
-        auto carry = [&](int& it, int& t) {   // past the tile's last stage: the same place of the next tiles
-            while (it >= n_it) {
-                it -= n_it;
-                t += t_step;
+        // The group's next stage to fetch: its place in its tile, where its codes are, stages left.
+        const int full_it = n_it - ((!DUAL && sub != 0 && (n_kb & 1)) ? 1 : 0);   // stages of a tile that have a block for this warp
+        int f_it = grp, f_t = t0, left = (n_local * n_it - grp + kGroups - 1) / kGroups, f_lim = left > 0 ? full_it : 0;
+        const uint8_t *f_ptr0 = code_lane, *f_ptr1 = code_lane;
+        auto fetch_place = [&] {   // past the tile's last stage: the same place of the next tiles
+            while (f_it >= n_it) {
+                f_it -= n_it;
+                f_t += t_step;
             }
-        };
-        auto fetch_place = [&] {
             const int tile = (f_t / n_tok) * (kTileRows / 16) + 2 * (warp & 3) + (DUAL ? sub : 0);
-            int kb = kb_base + kBlocksPerStage * f_it + (DUAL ? 0 : sub);
-            // A last stage without a second block: an address inside the row all the same (it is not read).  The bound also has the
-            // compiler order the producers' loop better: 5120 x 55296 at 16 rows 69.7 us without it, 68.8 with it, 3584 x 37888 at
-            // 64 rows 40.7 and 40.0.
-            if (!DUAL && kb >= kb_per_plane) kb -= kb_per_plane;
-            f_ptr0 = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
-            if constexpr (!DUAL) f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + static_cast<size_t>(kb) * kCodeTileBytes;
+            const size_t at = static_cast<size_t>(kb_base + kBlocksPerStage * f_it + (DUAL ? 0 : sub)) * kCodeTileBytes;
+            f_ptr0 = code_lane + static_cast<size_t>(min(tile, last_tile)) * tile_row_bytes + at;
+            if constexpr (!DUAL) f_ptr1 = code_lane + static_cast<size_t>(min(tile + 1, last_tile)) * tile_row_bytes + at;
         };
-        auto fetch = [&](uint4 (&c)[kLoads]) {
-            const int kb = kBlocksPerStage * f_it + (DUAL ? 0 : sub);
-            if (f_left > 0 && kb < n_kb) {
-                c[0] = load_codes16(f_ptr0);
-                c[1] = load_codes16(f_ptr0 + 512);
-                if constexpr (!DUAL) {
-                    c[2] = load_codes16(f_ptr1);
-                    c[3] = load_codes16(f_ptr1 + 512);
-                }
+        uint4 c[kLoads];
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) c[i] = make_uint4(0, 0, 0, 0);
+        if (left > 0) {
+            fetch_place();
+            const bool want = f_it < f_lim;
+            load_codes16_if(c[0], f_ptr0, want);
+            load_codes16_if(c[1], f_ptr0 + 512, want);
+            if constexpr (!DUAL) {
+                load_codes16_if(c[2], f_ptr1, want);
+                load_codes16_if(c[3], f_ptr1 + 512, want);
             }
-            f_left -= kGroups;
+        }
+        const uint32_t lane_c = static_cast<uint32_t>(lane) * 4u;   // bits outside the scaled code (7..14)
+        // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
+        auto entry = [&](uint32_t word, int byte) { return lut_load(__dp4a(word, 128u << (8 * byte), lane_c)); };
+        int slot = grp;                                             // ring slot of the stage, and the parity of its "empty" phase
+        uint32_t par = 1u;
+        bool ok = true;
+        for (; left > 0; --left) {
+            // The slot must have been read by the MMAs of its previous stage.  Asked for in front of the lookups and used behind them:
+            // the answer queues behind the other warps' lookups.
+            const uint32_t bar_e = bar_empty + 8u * slot;
+            uint32_t ready;
+            asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                         : "=r"(ready) : "r"(bar_e), "r"(par) : "memory");
+            auto slot_free = [&] {
+                if (__all_sync(0xffffffffu, ready)) return true;
+                if (__all_sync(0xffffffffu, bar_wait(bar_e, par, abort_flag))) return true;
+                raise_status(p.status, 6u);
+                atomicExch(&s_abort, 1u);
+                return false;
+            };
+            // where the group's next stage is
             f_it += kGroups;
             f_ptr0 += kGroups * kBlocksPerStage * kCodeTileBytes;
             if constexpr (!DUAL) f_ptr1 += kGroups * kBlocksPerStage * kCodeTileBytes;
-            // another tile: place the pointers anew
             if (f_it >= n_it) {
-                if (f_left > 0) {
-                    carry(f_it, f_t);
-                    fetch_place();
-                }
+                if (left > 1) fetch_place();
+                else f_lim = 0;
             }
-        };
-        uint4 buf0[kLoads], buf1[kLoads];
-#pragma unroll
-        for (int i = 0; i < kLoads; ++i) buf0[i] = buf1[i] = make_uint4(0, 0, 0, 0);
-        carry(f_it, f_t);
-        fetch_place();
-        fetch(buf0);
-        fetch(buf1);
-        int it = grp, unused_t = 0;
-        carry(it, unused_t);
-        int slot = grp % n_st, use = grp / n_st;     // ring slot of stage `it` and how often it has been used before
-        // One stage; false once a wait has run out.
-        auto produce = [&](uint4 (&c0)[kLoads]) {
-            const bool have = DUAL || kSubPerStage * it + sub < n_kb;   // the last stage of a tile may lack its second K block
-            const uint32_t lane_c = static_cast<uint32_t>(lane) * 4u;   // bits outside the scaled code (7..14)
+            const bool want = f_it < f_lim;
             const uint32_t st_addr = a_taddr + kTmemAStageCols * static_cast<uint32_t>(slot);
-            // the slot must have been read by the MMAs of its previous stage
-            auto slot_free = [&] {
-                if (use > 0 && !__all_sync(0xffffffffu, bar_wait(bar_empty + 8u * slot, static_cast<uint32_t>(use - 1) & 1u, abort_flag))) {
-                    raise_status(p.status, 6u);
-                    atomicExch(&s_abort, 1u);
-                    return false;
-                }
-                return true;
-            };
-            // byte * 128 + lane offset in one dot-product instruction (a shift and a mask each on the logic pipe before)
-            auto entry = [&](uint32_t word, int byte) { return lut_load(__dp4a(word, 128u << (8 * byte), lane_c)); };
             if constexpr (DUAL) {
                 // half a block's columns at a time: words i = 2 half and 2 half + 1 of either row, both planes
-                const uint32_t w[8] = {c0[0].x, c0[0].y, c0[0].z, c0[0].w, c0[1].x, c0[1].y, c0[1].z, c0[1].w};
+                const uint32_t w[8] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w};
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     uint32_t first[8], second[8];
@@ -547,8 +559,14 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                         first[h] = __byte_perm(e0, e1, 0x5410);
                         second[h] = __byte_perm(e0, e1, 0x7632);
                     }
-                    if (half == 1) fetch(c0);   // the codes are used up: the stage after next into the same registers
-                    if (half == 0 && !slot_free()) return false;
+                    if (half == 1) {
+                        load_codes16_if(c[0], f_ptr0, want);
+                        load_codes16_if(c[1], f_ptr0 + 512, want);
+                    }
+                    if (half == 0 && !slot_free()) {
+                        ok = false;
+                        break;
+                    }
                     tmem_st_16x256b(st_addr + 16u * half, first);
                     tmem_st_16x256b(st_addr + kTmemASubCols + 16u * half, second);
                 }
@@ -556,8 +574,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     // code tile `half`: 16 codes of row g and of row g + 8 -> fp16 pairs, word i of a row's four in column block i
-                    const uint32_t w[8] = {c0[2 * half].x, c0[2 * half].y, c0[2 * half].z, c0[2 * half].w,
-                                           c0[2 * half + 1].x, c0[2 * half + 1].y, c0[2 * half + 1].z, c0[2 * half + 1].w};
+                    const uint32_t w[8] = {c[2 * half].x, c[2 * half].y, c[2 * half].z, c[2 * half].w,
+                                           c[2 * half + 1].x, c[2 * half + 1].y, c[2 * half + 1].z, c[2 * half + 1].w};
                     uint32_t packed[16];
 #pragma unroll
                     for (int h = 0; h < 16; ++h) {
@@ -565,30 +583,33 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                         const int b0 = (h & 1) * 2;  // bytes b0, b0 + 1 of the word
                         packed[h] = __byte_perm(entry(word, b0), entry(word, b0 + 1), 0x5410);
                     }
-                    if (half == 1) fetch(c0);   // the codes are used up: the stage after next into the same registers
-                    if (half == 0 && !slot_free()) return false;
-                    if (have) tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
+                    // used up: the group's next stage into the same registers
+                    load_codes16_if(c[2 * half], half ? f_ptr1 : f_ptr0, want);
+                    load_codes16_if(c[2 * half + 1], (half ? f_ptr1 : f_ptr0) + 512, want);
+                    if (half == 0 && !slot_free()) {
+                        ok = false;
+                        break;
+                    }
+                    // (a tile's last stage may lack its second K block: what its warps store is not read)
+                    tmem_st_16x256b(st_addr + (static_cast<uint32_t>(16 * half) << 16), packed);
                 }
             }
+            if (!ok) break;
             // every lane waits for its own stores, then one arrival per warp
             tmem_st_publish();
             __syncwarp();
             if (lane == 0) bar_arrive(bar_full + 8u * slot);
-            it += kGroups;
-            if (it >= n_it) carry(it, unused_t);
             slot += kGroups;
-            if (slot >= n_st) { slot -= n_st; ++use; }
-            return true;
-        };
-        for (int left = n_stages - grp; left > 0; left -= 2 * kGroups) {
-            if (!produce(buf0)) break;
-            if (left > kGroups && !produce(buf1)) break;
+            if (slot >= n_st) {
+                slot -= n_st;
+                par ^= 1u;
+            }
         }
     } else if (warp == kCopyWarp) {
         // ---- activation tiles: one bulk copy per K block of the stage, as far ahead as the ring allows ----
         // One thread runs the whole loop; ring slot and phase are kept incrementally (no divisions on
         // this serial path).
-        if (lane == 0) {
+        if (elect_one()) {
             // The rotated activations are the only input the kernel before this one produces (launched with the
             // programmatic-dependency attribute, the CTA has set up its barriers, tensor memory and tables and the
             // producers are already streaming codes meanwhile): wait for that kernel here.
@@ -626,8 +647,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
-        // ---- MMA issuer (one thread): one wait and one commit per stage ---------------------------------
-        if (lane == 0) {
+        // ---- MMA issuer: the warp waits for a stage, one lane issues its MMAs and one commit ------------------------
+        {
             int slot = 0, acc = 0;
             uint32_t par = 0u, acc_par = 1u;   // acc_par: parity of the "drained" phase to wait for
             bool ok = true;
@@ -635,7 +656,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                 const uint32_t idesc = instr_desc(static_cast<uint32_t>(tile_rows(t0 + j * t_step)));
                 const uint32_t d_tmem = tmem_d + static_cast<uint32_t>(acc * (kTileTok / 2));
                 if (j >= n_acc) {
-                    if (!bar_wait(bar_acc_empty + 8u * acc, acc_par, abort_flag)) {
+                    if (!__all_sync(0xffffffffu, bar_wait(bar_acc_empty + 8u * acc, acc_par, abort_flag))) {
                         raise_status(p.status, 7u);
                         atomicExch(&s_abort, 1u);
                         break;
@@ -643,7 +664,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 for (int it = 0; it < n_it; ++it) {
-                    if (!bar_wait(bar_full + 8u * slot, par, abort_flag)) {
+                    if (!__all_sync(0xffffffffu, bar_wait(bar_full + 8u * slot, par, abort_flag))) {
                         raise_status(p.status, 7u);
                         atomicExch(&s_abort, 1u);
                         ok = false;
@@ -653,20 +674,24 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                     const int nsub = DUAL ? kSubPerStage : min(kSubPerStage, n_kb - kSubPerStage * it);
                     const uint32_t a_tmem = tmem_d + kTmemAColumn + kTmemAStageCols * static_cast<uint32_t>(slot);
                     const uint32_t b_stage = stage0 + static_cast<uint32_t>(slot) * stage_bytes;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int sb = 0; sb < kSubPerStage; ++sb) {
-                        if (sb < nsub) {
-                            const uint64_t desc0 = smem_desc(b_stage + static_cast<uint32_t>(sb) * piece_bytes);
+                        for (int sb = 0; sb < kSubPerStage; ++sb) {
+                            if (sb < nsub) {
+                                const uint64_t desc0 = smem_desc(b_stage + static_cast<uint32_t>(sb) * piece_bytes);
 #pragma unroll
-                            for (int k = 0; k < kBlockK / 16; ++k)   // 256 bytes further along K per step: +16 in the address field
-                                umma_f16_ts(d_tmem, a_tmem + kTmemASubCols * sb + 8u * k, desc0 + static_cast<uint64_t>(16 * k), idesc,
-                                            (it | sb | k) != 0 ? 1u : 0u);
+                                for (int k = 0; k < kBlockK / 16; ++k)   // 256 bytes further along K per step: +16 in the address field
+                                    umma_f16_ts(d_tmem, a_tmem + kTmemASubCols * sb + 8u * k, desc0 + static_cast<uint64_t>(16 * k), idesc,
+                                                (it | sb | k) != 0 ? 1u : 0u);
+                            }
                         }
+                        umma_commit(bar_empty + 8u * slot);   // the slot (weights and activation) may be refilled once these MMAs are done
                     }
-                    umma_commit(bar_empty + 8u * slot);   // the slot (weights and activation) may be refilled once these MMAs are done
+                    __syncwarp();
                     if (++slot == n_st) { slot = 0; par ^= 1u; }
                 }
-                if (ok) umma_commit(bar_acc_full + 8u * acc);
+                if (ok && elect_one()) umma_commit(bar_acc_full + 8u * acc);
+                __syncwarp();
                 if (++acc == n_acc) { acc = 0; acc_par ^= 1u; }
             }
         }
@@ -938,7 +963,7 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     }
     a.k_splits = gemm_k_splits(out, in, m, n_planes, sm_count);
     a.partial = a.k_splits > 1 ? reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + xrot_bytes(in, m, n_planes)) : nullptr;
-    const size_t smem = kGemmSmemBytes;
+    const size_t smem = gemm_smem_bytes(m);
     static bool configured[64] = {false};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
@@ -1014,7 +1039,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     }
     const dim3 grid(static_cast<unsigned int>(grp.tile_start[n]), static_cast<unsigned int>((m + kTileTok - 1) / kTileTok),
                     static_cast<unsigned int>(max_splits));
-    launch_pdl(n_planes == 2 ? tq8_gemm_group_kernel<true> : tq8_gemm_group_kernel<false>, grid, dim3(kGemmThreads), kGemmSmemBytes, stream, grp);
+    launch_pdl(n_planes == 2 ? tq8_gemm_group_kernel<true> : tq8_gemm_group_kernel<false>, grid, dim3(kGemmThreads), gemm_smem_bytes(m), stream, grp);
     // 3. the split-K sums
     launch_finish(fin, n_fin, static_cast<int>(m), sm_count, stream);
 }
