@@ -271,6 +271,26 @@ __device__ __forceinline__ void rotate_chunk(float (&v)[8], const uint4& raw, co
         for (int j = 0; j < 8; ++j) v[j] = __fmaf_rn(v[j], side, __shfl_xor_sync(live, v[j], m));
     }
 }
+// The same with the number of lane exchanges known and their signs at hand (side[k]: -1 where bit k of the lane is set): half of the
+// instructions where many rows follow one another.
+template <int STAGES>
+__device__ __forceinline__ void rotate_chunk_fixed(float (&v)[8], const uint4& raw, const uint4& signs, const float (&side)[STAGES], unsigned live) {
+    unpack_halves(make_uint4(raw.x ^ signs.x, raw.y ^ signs.y, raw.z ^ signs.z, raw.w ^ signs.w), v);
+#pragma unroll
+    for (int h = 1; h < 8; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2 * h)
+#pragma unroll
+            for (int j = i; j < i + h; ++j) {
+                const float a = v[j], b = v[j + h];
+                v[j] = __fadd_rn(a, b);
+                v[j + h] = __fsub_rn(a, b);
+            }
+#pragma unroll
+    for (int k = 0; k < STAGES; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __fmaf_rn(v[j], side[k], __shfl_xor_sync(live, v[j], 1 << k));
+}
 
 // Threads of a CTA that normalises a row (the RMSNorm kernel and the row-wise all-reduce tails: the same count, so the same
 // order of additions).  Eight columns per thread and step: 256 threads take 8192 columns in the four steps that stay in

@@ -261,51 +261,66 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
 // The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of a row (one block of 512 or
 // 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
 // the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
-// a CTA take 8 consecutive rows, and `row_steps` such groups one after the other: the hashes of the signs are a third of the
-// instructions of a row, and they are the same for all rows.  The 8 rows of a K block are 1 KB of the operand tile: they
-// meet in shared memory (slots of a core matrix's rows permuted by its column: no bank conflicts) and leave as contiguous
-// stores; a lane's own 16-byte pieces of a row are 128 bytes apart.
-template <int CHUNKS>
-__device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows,
-                                                      int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
+// a CTA take 8 consecutive rows, and `row_steps` such groups one after the other: the signs are the same for all rows.  The 8
+// rows of a K block are 1 KB of the operand tile: they meet in shared memory (slots of a core matrix's rows permuted by its column: no
+// bank conflicts) and leave as contiguous stores; a lane's own 16-byte pieces of a row are 128 bytes apart.
+// Instructions bound it, a third of the time the lane exchanges alone: 286 per 256 columns of a row with the exchanges in a loop, 64-bit places
+// and the signs of the lanes found anew for every row; 218 so, and the signs are made in front of the wait.  2048 x 18944: 53 -> 44 us under the
+// profiler, 64 x 18944 with the product behind it 27.5 -> 25.2.  With two columns an instruction (fp32 pairs): 302, the pairs have to be made.
+template <int CHUNKS, int STAGES>
+__device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, int rows, int block, uint32_t seed,
+                                                      unsigned col_group, unsigned row_group, float inv_sqrt, int row_steps, uint4 (*s_rows)[256 * CHUNKS]) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const unsigned groups_per_row = (static_cast<unsigned>(in) + 256 * CHUNKS - 1) / (256 * CHUNKS);
-    const unsigned row_groups = static_cast<unsigned>((rows + 8 * row_steps - 1) / (8 * row_steps));
-    // blockIdx.x -> (plane, column group, rows); warp -> row inside a group of 8
-    unsigned b = blockIdx.x;
-    const unsigned rg = b % row_groups;
-    b /= row_groups;
-    const unsigned cg = b % groups_per_row;
-    const int plane = static_cast<int>(b / groups_per_row);
-    if (plane >= n_planes) return;
-    __shared__ __align__(16) uint4 s_rows[2][256 * CHUNKS];   // [step parity][K block][core column][row slot]
-    const int col = static_cast<int>(cg) * 256 * CHUNKS + 8 * lane;
+    const int col = static_cast<int>(col_group) * 256 * CHUNKS + 8 * lane;
     // in is a multiple of 64 and of the block: whole lanes only, and exchanges stay inside a block.  (A group of several
     // chunks is a whole block, all of it inside the row.)
     const bool have = col < in;
     const unsigned live = __ballot_sync(0xffffffffu, have);
-    const uint32_t seed = plane ? seed_r : seed_p;
     uint4 signs[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
-    const long n_row_tiles = (rows + kTileTok - 1) / kTileTok;
-    const long kb_per_plane = in / kBlockK;
+    float side[STAGES];
+#pragma unroll
+    for (int k = 0; k < STAGES; ++k) side[k] = (lane & (1 << k)) != 0 ? -1.0f : 1.0f;
+    const int kb_per_plane = in / kBlockK;
     // A lane's two groups of four columns are 16 positions apart; lane ^ 2 holds the ones next to them.  The lanes swap
     // one group each, so that every lane stores a whole core-matrix row of 8.
     const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
     const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
     const int cc = pos >> 3;
-    int buf = 0;
-    const long first = static_cast<long>(rg) * 8 * row_steps, last = min(rows, first + 8L * row_steps);
-    for (long row8 = first; row8 < last; row8 += 8, buf ^= 1) {
-        const long row = row8 + wib;
-        if (have && row < rows) {
+    uint4* put = &s_rows[0][(lane >> 3) * 64 + cc * 8 + (wib ^ cc)];
+    // in the other direction: thread -> K block (of four per chunk), core column and row
+    const int t = threadIdx.x & 63, tc = t >> 3, tr = t & 7;
+    const uint4* get = &s_rows[0][(threadIdx.x >> 6) * 64 + tc * 8 + (tr ^ tc)];
+    constexpr int kOther = 256 * CHUNKS;   // to the buffer of the next step
+    int flip = kOther;
+    const int first = static_cast<int>(row_group) * 8 * row_steps, last = min(rows, first + 8 * row_steps);
+    const __half* src = x + static_cast<size_t>(first + wib) * in + col;
+    const size_t src_step = static_cast<size_t>(in) * 8;
+    const int kb_at = static_cast<int>(col_group) * 4 * CHUNKS + static_cast<int>(threadIdx.x >> 6);
+    auto place = [&](int row8) {
+        return xrot + (static_cast<size_t>(row8 / kTileTok) * kb_per_plane + kb_at) * (kTileTok * kBlockK) + ((row8 % kTileTok >> 3) * 64 + t) * 8;
+    };
+    __half* dst = place(first);
+    pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
+    // a row's loads are on their way while the one before it is worked on (not of blocks of 1024, which fill the registers)
+    constexpr bool kAhead = CHUNKS <= 2;
+    uint4 next[CHUNKS];
+    auto load = [&](const __half* from, bool there) {
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) next[c] = there ? __ldg(reinterpret_cast<const uint4*>(from + 256 * c)) : make_uint4(0, 0, 0, 0);
+    };
+    if (kAhead) load(src, have && first + wib < rows);
+    for (int row8 = first; row8 < last; row8 += 8) {
+        if (have && row8 + wib < rows) {
+            if (!kAhead) load(src, true);
             uint4 raw[CHUNKS];
 #pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(x + row * in + col + 256 * c));
+            for (int c = 0; c < CHUNKS; ++c) raw[c] = next[c];
+            if (kAhead) load(src + src_step, row8 + 8 + wib < last);
             float v[CHUNKS][8];
 #pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
+            for (int c = 0; c < CHUNKS; ++c) rotate_chunk_fixed<STAGES>(v[c], raw[c], signs[c], side, live);
 #pragma unroll
             for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll
@@ -325,19 +340,43 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
                 const uint4 h = pack_halves(v[c]);
                 const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
                 const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
-                const uint4 piece = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
-                s_rows[buf][(4 * c + (lane >> 3)) * 64 + cc * 8 + (wib ^ cc)] = piece;
+                put[256 * c] = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
             }
         }
         __syncthreads();   // (the other buffer's readers are past it when it is written again)
-        const long rt = row8 / kTileTok, rin = row8 - rt * kTileTok;
-        const long tile0 = (static_cast<long>(plane) * n_row_tiles + rt) * kb_per_plane;
+        if (row8 + tr < rows) {
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) {
-            const int t = threadIdx.x & 63, kb = 4 * c + (threadIdx.x >> 6), tc = t >> 3, tr = t & 7;
-            const long kb_at = static_cast<long>(cg) * 4 * CHUNKS + kb;
-            if (kb_at < kb_per_plane && row8 + tr < rows)
-                *reinterpret_cast<uint4*>(xrot + (tile0 + kb_at) * (kTileTok * kBlockK) + ((rin >> 3) * 64 + t) * 8) = s_rows[buf][kb * 64 + tc * 8 + (tr ^ tc)];
+            for (int c = 0; c < CHUNKS; ++c)
+                if (kb_at + 4 * c < kb_per_plane) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(4 * c) * (kTileTok * kBlockK)) = get[256 * c];
+        }
+        put += flip;
+        get += flip;
+        flip = -flip;
+        src += src_step;
+        dst += 64 * 8;
+        if ((row8 + 8) % kTileTok == 0) dst = place(row8 + 8);
+    }
+}
+// The lane exchanges of a block as a constant of the loop over rows.
+template <int CHUNKS>
+__device__ __forceinline__ void rotate_rows_wide(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows, int block, uint32_t seed_p,
+                                                 uint32_t seed_r, float inv_sqrt, int row_steps) {
+    __shared__ __align__(16) uint4 s_rows[2][256 * CHUNKS];   // [step parity][K block][core column][row slot]
+    const unsigned groups_per_row = (static_cast<unsigned>(in) + 256 * CHUNKS - 1) / (256 * CHUNKS);
+    const unsigned row_groups = static_cast<unsigned>((rows + 8 * row_steps - 1) / (8 * row_steps));
+    // blockIdx.x -> (plane, column group, rows); warp -> row inside a group of 8
+    const unsigned rg = blockIdx.x % row_groups, b = blockIdx.x / row_groups, cg = b % groups_per_row, plane = b / groups_per_row;
+    const uint32_t seed = plane ? seed_r : seed_p;
+    __half* const to = xrot + plane * ((static_cast<size_t>(rows) + kTileTok - 1) / kTileTok * (in / kBlockK) * (kTileTok * kBlockK));
+    const int m = static_cast<int>(rows);
+    if constexpr (CHUNKS > 1) {
+        rotate_rows_wide_body<CHUNKS, 5>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows);
+    } else {
+        switch (block) {
+            case 32: rotate_rows_wide_body<1, 2>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
+            case 64: rotate_rows_wide_body<1, 3>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
+            case 128: rotate_rows_wide_body<1, 4>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
+            default: rotate_rows_wide_body<1, 5>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
         }
     }
 }
@@ -345,8 +384,7 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
                                                                    int in, long rows, int n_planes, int block,
                                                                    uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
-    pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
-    rotate_rows_wide_body<CHUNKS>(x, xrot, in, rows, n_planes, block, seed_p, seed_r, inv_sqrt, row_steps);
+    rotate_rows_wide<CHUNKS>(x, xrot, in, rows, block, seed_p, seed_r, inv_sqrt, row_steps);
 }
 // The same rows rotated for several matrices at once (their own seeds and destinations): blockIdx.y = matrix.
 struct RotateGroupArgs {
@@ -356,8 +394,7 @@ struct RotateGroupArgs {
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
                                                                          long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
-    pdl_wait_release();
-    rotate_rows_wide_body<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, n_planes, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
+    rotate_rows_wide<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
 }
 
 struct GemmArgs {
