@@ -74,3 +74,26 @@ def test_rope(tq, heads, kv_heads, dim, offset):
         lo, hi = a[..., :half].astype(np.float64), a[..., half:].astype(np.float64)
         want = np.concatenate([lo * np.cos(ang) - hi * np.sin(ang), hi * np.cos(ang) + lo * np.sin(ang)], axis=-1)
         assert rel_l2(got.cpu().numpy(), want) < TOL
+
+
+@pytest.mark.parametrize("n_slots,residual", [(1, False), (1, True), (3, False), (3, True)])
+@pytest.mark.parametrize("cols,offset", [(8, 0), (2056, 0), (16400, 0), (2056, 2)])
+def test_sum_of_slots_and_rmsnorm(tq, n_slots, residual, cols, offset):
+    """One CTA a row, with and without whole 16-byte pieces, against the sum and the norm on their own."""
+    import torch
+    L = tq.load()
+    rng = np.random.default_rng(cols + n_slots)
+    rows, n = 3, 3 * cols
+    slots = _at(torch, rng.standard_normal((n_slots, rows, cols)).astype(np.float16), offset)
+    res = _at(torch, rng.standard_normal((rows, cols)).astype(np.float16), offset) if residual else None
+    w = _at(torch, (1 + 0.1 * rng.standard_normal(cols)).astype(np.float16), offset)
+    outs = [_at(torch, np.zeros((rows, cols), np.float16), offset) for _ in range(4)]
+    r = _p(res) if residual else None
+    assert L.tq_exchange_sum_f16(_p(slots), n_slots, n, n, r, _p(outs[0]), None) == 0
+    assert L.tq_rmsnorm_f16(_p(outs[0]), _p(w), _p(outs[1]), rows, cols, 1e-6, None) == 0
+    assert L.tq_exchange_sum_f16_rmsnorm(_p(slots), n_slots, n, rows, cols, r, _p(outs[2]), _p(w), _p(outs[3]), 1e-6, None) == 0
+    torch.cuda.synchronize()
+    want = res.float() if residual else torch.zeros((rows, cols), device="cuda")
+    for s in range(n_slots):
+        want = want + slots[s].float()
+    assert torch.equal(outs[0], want.half()) and torch.equal(outs[2], outs[0]) and torch.equal(outs[3], outs[1])

@@ -299,14 +299,35 @@ __device__ __forceinline__ void rotate_chunk_fixed(float (&v)[8], const uint4& r
 constexpr int kRowNormThreads = 256;
 constexpr int kRowNormKeep = 4;
 
+// Eight halves of a row; WIDE: all rows are multiples of eight and 16-byte aligned.
+template <bool WIDE>
+__device__ __forceinline__ uint4 load_row8(const __half* p, int n) {
+    if constexpr (WIDE) return *reinterpret_cast<const uint4*>(p);
+    else return load_halves(p, n);
+}
+template <bool WIDE>
+__device__ __forceinline__ void store_row8(__half* p, int n, const uint4& v) {
+    if constexpr (WIDE) *reinterpret_cast<uint4*>(p) = v;
+    else store_halves(p, n, v);
+}
+__device__ __forceinline__ bool rows_wide(int cols, const void* a, const void* b, const void* c) {
+    return cols % 8 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+
 // yr[:] = xr[:] * rsqrt(mean(xr[:]^2) + eps) * w for one row, by the whole CTA (kRowNormThreads threads; cols even).  A
 // thread takes the columns 8 (threadIdx.x + k * kRowNormThreads) .. + 7, whatever the alignment, the first kRowNormKeep
 // steps of them in `keep`; the others are read from xr.  Shared by the RMSNorm kernel and the all-reduce tails that
-// normalise the row they have just summed, so the fused and the separate form give the same bits.
+// normalise the row they have just summed, so the fused and the separate form give the same bits.  The weights are asked for
+// in front of the sum of squares, whose barrier they would otherwise be waited for behind.
+template <bool WIDE>
 __device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], const __half* xr, const __half* __restrict__ w, __half* yr, int cols,
                                              float eps) {
     constexpr int kStep = 8 * kRowNormThreads;
     const int c0 = threadIdx.x * 8;
+    uint4 gain[kRowNormKeep];
+#pragma unroll
+    for (int k = 0; k < kRowNormKeep; ++k)
+        gain[k] = c0 + k * kStep < cols ? load_row8<WIDE>(w + c0 + k * kStep, cols - c0 - k * kStep) : make_uint4(0u, 0u, 0u, 0u);
     float ss = 0.f;
     auto add = [&](const uint4& raw) {
         float v[8];
@@ -316,7 +337,7 @@ __device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], 
     };
 #pragma unroll
     for (int k = 0; k < kRowNormKeep; ++k) add(keep[k]);   // (zero beyond the row)
-    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) add(load_halves(xr + c, cols - c));
+    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) add(load_row8<WIDE>(xr + c, cols - c));
     __shared__ float s_part[kRowNormThreads / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -326,27 +347,28 @@ __device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], 
 #pragma unroll
     for (int i = 0; i < kRowNormThreads / 32; ++i) tot += s_part[i];   // fixed order
     const float scale = rsqrtf(tot / static_cast<float>(cols) + eps);
-    auto write = [&](int c, const uint4& raw) {
+    auto write = [&](int c, const uint4& raw, const uint4& weight) {
         float v[8], g[8];
         unpack_halves(raw, v);
-        unpack_halves(load_halves(w + c, cols - c), g);
+        unpack_halves(weight, g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = v[j] * scale * g[j];
-        store_halves(yr + c, cols - c, pack_halves(v));
+        store_row8<WIDE>(yr + c, cols - c, pack_halves(v));
     };
 #pragma unroll
     for (int k = 0; k < kRowNormKeep; ++k)
-        if (c0 + k * kStep < cols) write(c0 + k * kStep, keep[k]);
-    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) write(c, load_halves(xr + c, cols - c));
+        if (c0 + k * kStep < cols) write(c0 + k * kStep, keep[k], gain[k]);
+    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) write(c, load_row8<WIDE>(xr + c, cols - c), load_row8<WIDE>(w + c, cols - c));
 }
+template <bool WIDE>
 __device__ __forceinline__ void rmsnorm_row(const __half* xr, const __half* __restrict__ w, __half* yr, int cols, float eps) {
     uint4 keep[kRowNormKeep];
 #pragma unroll
     for (int k = 0; k < kRowNormKeep; ++k) {
         const int c = 8 * (threadIdx.x + k * kRowNormThreads);
-        keep[k] = c < cols ? load_halves(xr + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
+        keep[k] = c < cols ? load_row8<WIDE>(xr + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
     }
-    rmsnorm_kept(keep, xr, w, yr, cols, eps);
+    rmsnorm_kept<WIDE>(keep, xr, w, yr, cols, eps);
 }
 
 __device__ __forceinline__ void raise_status(unsigned int* status, unsigned int code) {

@@ -23,7 +23,10 @@ __device__ __forceinline__ void ops_dependency_sync() {
 __global__ void __launch_bounds__(kRowNormThreads) rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
                                                       int cols, float eps) {
     ops_dependency_sync();
-    rmsnorm_row(x + static_cast<size_t>(blockIdx.x) * cols, w, y + static_cast<size_t>(blockIdx.x) * cols, cols, eps);
+    const __half* const xr = x + static_cast<size_t>(blockIdx.x) * cols;
+    __half* const yr = y + static_cast<size_t>(blockIdx.x) * cols;
+    if (rows_wide(cols, x, w, y)) rmsnorm_row<true>(xr, w, yr, cols, eps);
+    else rmsnorm_row<false>(xr, w, yr, cols, eps);
 }
 
 // Rotary embedding, "rotate half" convention: element i of a head pairs with element i + d/2;
