@@ -69,7 +69,10 @@ constexpr int kSlice = 256;               // columns per warp
 constexpr int kChunk = kWarps * kSlice;   // widest chunk: columns one unit covers with all 16 warps on one row tile
 constexpr uint32_t kLutAddr = 0x10000u;   // shared-window address of the table
 constexpr uint32_t kLutBytes = 0x10000u;  // 256 entries * 256 B
-constexpr int kRedBytes = 32768;           // partial-sum ring: ring * 16 warps * (16 rows * bp + 4) floats
+// Partial-sum ring: ring * 16 warps * (16 rows * bp + 4) floats.  Eight rows take three slots of 32 KB, which tied the warps to each
+// other's pace: seven of 60 KB, 151936 x 2048 75.4 -> 73.9 us, 37888 x 3584 41.1 -> 40.1.  (Fewer rows have seven to sixteen slots as it is, and
+// gained nothing from more.)
+__host__ __device__ constexpr int red_bytes(int bp) { return bp == 8 ? 61440 : 32768; }
 constexpr int kMaxRing = 16;
 constexpr int kFlushUnits = 8;             // units a warp finishes between two arrival counts (several slots only)
 
@@ -141,7 +144,6 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __restrict__ x, float* __restrict__ xrot, int in, int batch,
                                                             int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
     grid_launch_dependents();
-    grid_dependency_sync();
     const int lane = threadIdx.x & 31;
     const int groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -153,12 +155,16 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
     const uint32_t seed = plane ? seed_r : seed_p;
     const __half* const src = x + static_cast<size_t>(row) * in + col;
+    uint4 signs[CHUNKS];   // in front of the wait: 4096 x 4096 at eight rows 9.9 -> 9.6 us with the product
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
+    grid_dependency_sync();
     uint4 raw[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
     float v[CHUNKS][8];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block), block, lane, live);
+    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
 #pragma unroll
     for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll
@@ -457,6 +463,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     // A warp's partial tile is [16 rows][BP] floats plus 4 floats of padding: the 16 tiles a
     // reduction reads side by side then start 4 banks apart instead of in the same bank.
     constexpr int kTileFloats = 16 * BP + 4;
+    constexpr int kRedBytes = red_bytes(BP);
     constexpr int kRing = (kRedBytes / (kWarps * kTileFloats * 4)) > kMaxRing ? kMaxRing : (kRedBytes / (kWarps * kTileFloats * 4));
     static_assert(kRing >= 2, "the ring needs a slot to write while another is summed");
     constexpr int kLag = kRing / 2;                       // how many units behind the sums run
@@ -483,7 +490,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     const uint32_t base = smem_u32(smem_raw);
     const uint32_t red_addr = (base + 127u) & ~127u;
     const uint32_t strip_addr = red_addr + kRedBytes + static_cast<uint32_t>(warp) * (kSlice * 4u);
-    if (red_addr + kRedBytes + kWarps * kSlice * 4u > kLutAddr) {  // layout assumption broken: refuse to run
+    if (red_addr + kRedBytes + (BP == 1 ? kWarps * kSlice * 4u : 0u) > kLutAddr) {  // layout assumption broken: refuse to run
         if (tid == 0) raise_status(p.status, 1u);
         return;
     }
