@@ -567,6 +567,19 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         load_step(cur, s, true, blo[s], bhi[s]);
     }
 
+    if constexpr (DUAL) {
+        // The rest of this unit and the next one on their way into the L2 cache, a line a lane, while the rotation in front is
+        // waited for: 3584 x 3584, four rows, 11.1 -> 9.8 us, one row 9.0 -> 8.2; further units in advance gain no more.  (One row of one
+        // rotation is rotated in here, and its loads would queue behind this: 7.5 -> 7.6 for 4096 x 4096 even so late as behind them.)
+        auto prefetch = [&](const Pos& u, int first, int steps) {
+            const int s = first + (lane >> 3);
+            if ((lane >> 3) < steps && ((u.ok >> s) & 1u) && (u.ok & 16u))
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(u.ptr - (g * 64 + 16 * q) + kCodeTileBytes * s + 128 * (lane & 7)));
+        };
+        prefetch(cur, 2, 2);
+        if (n_local > 1) prefetch(nxt, 0, 4);
+    }
+
     // Prologue order: table entries are fetched into registers (they do not depend on the
     // preceding kernel), then comes the dependency wait, then this warp's activation slice of
     // the first unit is requested, and only then are the table entries written to shared
