@@ -554,8 +554,8 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
         caches[i]->note_stream(st);
     }
     const int sms = tq::sm_count(c0->device());
-    long longest = 0;
-    const long tiles = tq::attn_number_tiles(desc, n_seqs, &longest);
+    long longest = 0, shortest = 0;
+    const long tiles = tq::attn_number_tiles(desc, n_seqs, &longest, &shortest);
     // A table goes up only when it differs from the one already on the device: a call that repeats the
     // previous ranges enqueues kernels only (and can then be captured in a graph).
     if (!many.empty())
@@ -583,7 +583,7 @@ void attention_batched(TQKVCache* const* caches, int n_seqs, int layer, const vo
     }
     c0->attn_scratch().reserve(tq::attn_scratch_bytes(dim, sms), st);
     unsigned int* const counters = c0->attn_job_counters(tq::attn_counters(n_seqs, q_heads, heads), st);
-    tq::launch_kv_attention(seqs, n_seqs, tiles, longest, d_q, q_dtype == TQ_F16, q_heads, heads, dim,
+    tq::launch_kv_attention(seqs, n_seqs, tiles, longest, shortest, d_q, q_dtype == TQ_F16, q_heads, heads, dim,
                             tq::kv_layer_seed(static_cast<uint32_t>(layer), 1), tq::kv_layer_seed(static_cast<uint32_t>(layer), 2),
                             tq::kv_layer_seed(static_cast<uint32_t>(layer), 3), use_qjl, c0->attn_scratch().as<void>(), counters, d_out, d_lse,
                             c0->attn_status_device(), sms, st);

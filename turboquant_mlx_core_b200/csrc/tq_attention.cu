@@ -24,12 +24,13 @@
 // does not depend on timing - un-rotates and writes.  One launch, no combine kernel.  Where a job has many parts their
 // weights are computed first, side by side, so that the accumulators stream: as a chain of rescaled sums, six parts a round
 // trip, 3 jobs of 2500 tiles spent 23 of 50 us there.  Where cutting the jobs costs more than it levels out, a range is a
-// number of whole jobs (launch_kv_attention).  A job's start and end cost a team about
+// number of whole jobs, or each job is cut into as many parts (launch_kv_attention).  A job's start and end cost a team about
 // as much as `pad` tiles, so the flat numbering gives every job that many empty tiles in front: a range with two jobs gets
 // fewer tiles than one with a single one.
 //
 // The next job's first tiles are requested before the merge of the current one, which has shared memory of its own.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "tq_attn.cuh"
@@ -94,7 +95,7 @@ struct AttnArgs {
     float* part;               // [range][2][kPartFloats]
     unsigned int* counters;    // [job]
     unsigned int* status;
-    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units, ranges, pad, whole_jobs;
+    int q_is_f16, n_seqs, q_heads, kv_heads, gchunks, units, ranges, pad, whole_jobs, parts;
     uint32_t k_seed, v_seed, qjl_seed;
     float inv_sqrt, inv_scale, score_scale, qscale;
 };
@@ -254,14 +255,16 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         return;
     }
     const int jobs_per_seq = a.kv_heads * a.gchunks, G = a.q_heads / a.kv_heads;
-    // where range r starts: an equal share of the flat tiles, or of the jobs
+    // where range r starts: an equal share of the flat tiles, or of the jobs, or of a job's tiles
     auto range_start = [&](int r) {
-        if (!a.whole_jobs) return static_cast<int>(static_cast<long>(a.units) * r / a.ranges);
-        const int job = static_cast<int>(static_cast<long>(a.n_seqs) * jobs_per_seq * r / a.ranges);
+        if (!a.whole_jobs && a.parts == 0) return static_cast<int>(static_cast<long>(a.units) * r / a.ranges);
+        const int job = a.parts != 0 ? r / a.parts : static_cast<int>(static_cast<long>(a.n_seqs) * jobs_per_seq * r / a.ranges);
         if (job >= a.n_seqs * jobs_per_seq) return a.units;
         const int seq = job / jobs_per_seq;
         const AttnSeq S = attn_seq(a.seqs, seq);
-        return (S.tile0 + seq * a.pad) * jobs_per_seq + (job - seq * jobs_per_seq) * ((S.end + kKvTile - 1) / kKvTile - S.start / kKvTile + a.pad);
+        const int tiles = (S.end + kKvTile - 1) / kKvTile - S.start / kKvTile;
+        const int start = (S.tile0 + seq * a.pad) * jobs_per_seq + (job - seq * jobs_per_seq) * (tiles + a.pad);
+        return a.parts != 0 ? start + static_cast<int>(static_cast<long>(tiles) * (r - job * a.parts) / a.parts) : start;   // (parts: no empty tiles)
     };
     if (a.seqs.table != nullptr) pdl_wait_release();   // the table may have been uploaded just before
     int u = range_start(range);
@@ -686,8 +689,9 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         const bool whole = done.n_tiles == done.tiles;
         // which ranges share the job: the range of flat tile x is ((x + 1) ranges - 1) / units
         const int job_u0 = u - done.n_tiles - done.tile0;   // the job's first tile
-        const int c_first = whole ? range : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
-        const int c_last = whole ? range : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
+        const int c_first = whole ? range : a.parts != 0 ? done.job * a.parts : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
+        const int c_last = whole ? range
+                                 : a.parts != 0 ? c_first + a.parts - 1 : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
         float* const my_part = a.part + static_cast<size_t>(2 * range + (done.tile0 == 0 ? 1 : 0)) * C::kPartFloats;
         auto scale_add = [](float4& x, float f0, const float4& y, float f1) {
             x.x = fmaf(x.x, f0, y.x * f1);
@@ -856,13 +860,15 @@ void launch_d(const AttnArgs& args, int grid, cudaStream_t stream) {
 
 }  // namespace
 
-long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest) {
+long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest, long* shortest) {
     long total = 0;
     *longest = 0;
+    *shortest = LONG_MAX;
     for (int i = 0; i < n_seqs; ++i) {
         seqs[i].tile0 = static_cast<int>(total);
         const long tiles = (seqs[i].end + kKvTile - 1) / kKvTile - seqs[i].start / kKvTile;
         *longest = std::max(*longest, tiles);
+        *shortest = std::min(*shortest, tiles);
         total += tiles;
     }
     return total;
@@ -874,7 +880,7 @@ size_t attn_counters(int n_seqs, int q_heads, int kv_heads) {
     return static_cast<size_t>(n_seqs) * kv_heads * ((q_heads / kv_heads + kGroup - 1) / kGroup);
 }
 
-void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, long shortest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
                          uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl, void* scratch, unsigned int* counters,
                          __half* out, float* lse, unsigned int* status, int sm_count, cudaStream_t stream) {
     if (n_seqs == 0) return;
@@ -915,22 +921,49 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long long
     // 64 dims 4 x 4096, 8 / 8 heads 17.2 / 27.6, 8 x 2000, 32 / 8 17.1 / 15.9, 64 x 1000, 8 / 8 35.0 / 30.5;
     // 128 dims 1 x 4096 10.0 / 28.5, 8 x 2000, 32 / 8 19.4 / 16.6, 64 x 1000, 8 / 8 38.6 / 33.2, 10 x 10539, 8 / 2 22.4 / 68.3;
     // 256 dims 16 x 2048, 14 / 2 31.1 / 57.2, 32 x 1000, 32 / 8 67.7 / 64.0, 64 x 1000, 8 / 8 124 / 128.
-    struct { int tile, tile_beside, part, job; } ns;   // a tile with one team on the SM, with two; a part; the end of a job
+    // Or, few jobs, each in as many parts: a range has one job, so that the parts are as long as each other, end together and are few
+    // (an equal share's ranges span two jobs each, and it takes all the ranges there are).  With one team an SM a tile takes half as
+    // long, so one part an SM is often the best.  Equal shares or whole jobs against as many parts as the rule takes, us: 128 dims,
+    // 28 / 4 heads, 1 x 1024 tokens 10.5 / 7.9, 1 x 4096 10.2 / 9.5, 1 x 8192 14.4 / 10.9, 1 x 32768 20.6 / 15.6, 8 x 1024 10.7 / 9.1; 40 / 8
+    // heads, 1 x 8192 14.8 / 11.6, 8 x 4096 23.7 / 18.8; 8 / 1 heads, 1 x 100000 30.7 / 18.6; 64 dims 1 x 16384 15.0 / 12.5, 16 x 4096, 8 / 8
+    // 29.4 / 26.1; 32 dims 1 x 16384 11.7 / 9.8; 256 dims 1 x 512 19.9 / 14.6, 4 x 2048 25.2 / 18.6.  16 x 32768, whose 64 jobs would be four
+    // parts each of the 4.6 that the SMs have room for, 80.3 in equal shares, 85.5 so.
+    struct {
+        int tile, tile_beside;   // a tile with one team on the SM, with two
+        int part, job;           // equal shares: a part; the end of a job
+        int merge, each;         // equal parts: cut at all; for each part of a job that its last one adds (many cost more each)
+    } ns;
     switch (head_dim) {
-        case 32: ns = {66, 143, 4000, 6000}; break;
-        case 64: ns = {100, 165, 7000, 6000}; break;
-        case 256: ns = {400, 400, 9000, 8000}; break;
-        default: ns = {100, 190, 10000, 6000}; break;
+        case 32: ns = {66, 143, 4000, 6000, 2000, 40}; break;
+        case 64: ns = {100, 155, 7000, 6000, 2300, 44}; break;
+        case 256: ns = {400, 400, 9000, 8000, 3500, 75}; break;
+        default: ns = {100, 176, 10000, 6000, 2500, 48}; break;
     }
+    constexpr long kSecondTeam = 1000;   // the start of a second team beside the first
     const long jobs = static_cast<long>(n_seqs) * kv_heads * a.gchunks;
     const long jobs_per_range = (jobs + most - 1) / most, job_ranges = (jobs + jobs_per_range - 1) / jobs_per_range;
     auto tile_ns = [&](long ranges) { return static_cast<long>(ranges > sm_count ? ns.tile_beside : ns.tile); };
     const long share = (units + a.ranges - 1) / a.ranges;
-    a.whole_jobs = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * ns.job <=
-                   share * tile_ns(a.ranges) + ns.part + ns.job * share * jobs / units;
-    if (a.whole_jobs) a.ranges = static_cast<int>(job_ranges);
+    const long whole_ns = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * ns.job;
+    const long share_ns = share * tile_ns(a.ranges) + ns.part + ns.each * a.ranges / jobs + ns.job * share * jobs / units;
+    a.whole_jobs = whole_ns <= share_ns;
+    a.parts = 0;
+    long best = std::min(whole_ns, share_ns);
+    for (long p = 2; p <= std::min(most / jobs, shortest); ++p) {   // (a part has a tile of every job)
+        const long ranges = jobs * p, part = std::max<long>(team, (longest + p - 1) / p);
+        const long cost = part * tile_ns(ranges) + ns.merge + (ns.each + p / 4) * p + (ranges > sm_count ? kSecondTeam : 0);
+        if (cost >= best) continue;
+        best = cost;
+        a.parts = static_cast<int>(p);
+    }
+    if (a.parts != 0) {
+        a.whole_jobs = 0;
+        a.ranges = static_cast<int>(jobs * a.parts);
+    } else if (a.whole_jobs) {
+        a.ranges = static_cast<int>(job_ranges);
+    }
     // 32: five rounds of the team's warps, about 6 us; less where ranges are short and every job ends in several of them
-    a.pad = static_cast<int>(std::min<long>(32, units / a.ranges / 8));
+    a.pad = a.parts != 0 ? 0 : static_cast<int>(std::min<long>(32, units / a.ranges / 8));
     units += static_cast<long>(n_seqs) * kv_heads * a.gchunks * a.pad;
     TQ_REQUIRE(units < (1L << 31), "attention: too many tokens for one call");
     a.units = static_cast<int>(units);

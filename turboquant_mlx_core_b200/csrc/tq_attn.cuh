@@ -110,11 +110,11 @@ constexpr float kAttnCentroidScale = 1.1979075f;
 // The decode window's lazy softmax reference (tq_attn_dense.cu): it only moves when a score exceeds it by more than this.
 constexpr float kAttnSoftmaxSlack = 2.0f;
 
-// Sets the descriptors' tile0 and returns the tiles of all sequences; `longest`: of the longest.
-long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest);
+// Sets the descriptors' tile0 and returns the tiles of all sequences; `longest`, `shortest`: of the longest, of the shortest.
+long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest, long* shortest);
 size_t attn_scratch_bytes(int dim, int sm_count);
 size_t attn_counters(int n_seqs, int q_heads, int kv_heads);   // zeroed words; every launch leaves them zero
-void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
+void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, long shortest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
                          uint32_t k_seed, uint32_t v_seed, uint32_t qjl_seed, bool use_qjl, void* scratch, unsigned int* counters,
                          __half* out, float* lse, unsigned int* status, int sm_count, cudaStream_t stream);
 
