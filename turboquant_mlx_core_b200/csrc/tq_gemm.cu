@@ -800,23 +800,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_kernel(const GemmArg
     gemm_body<DUAL>(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
 }
 
-// Several matrices that multiply the same activation rows (q / k / v, gate / up) in one launch: gridDim.x is cut into
-// one range of row tiles per matrix, gridDim.z is the largest K split of the group (CTAs beyond a matrix's own split
-// count leave at once).  Every matrix brings its own rotated activations (its own seeds), scratch and status word.
+// Several matrices that multiply the same activation rows (q / k / v, gate / up) in one launch, a CTA per tile and K split.  Every
+// matrix brings its own rotated activations (its own seeds), scratch and status word.  Matrices of one K split: gridDim.x is cut into one
+// range of row tiles per matrix, gridDim.y are the token tiles, gridDim.z the splits.  Otherwise (`flat`) the CTAs of a matrix, split by split,
+// follow one another in gridDim.x, the matrices with the longest ones first, so that short ones fill what is left of the last wave.  (With
+// the largest split as gridDim.z the CTAs beyond a matrix's own left at once, but each took its place on an SM first: 3584 -> 3584 +
+// 512 + 512 at 64 rows 20.1 -> 19.6 us, at 2048 96.5 -> 91.3, 5120 -> 5120 + 1024 + 1024 at 32 25.2 -> 22.7.  Matrices of one split in that order, and with
+// its division: 3 x 4096 -> 4096 at 16 rows 27.3 -> 27.8.)
 constexpr int kMaxGemmGroup = 4;
 struct GemmGroupArgs {
     GemmArgs m[kMaxGemmGroup];
-    int tile_start[kMaxGemmGroup + 1];   // row tiles tile_start[i] .. tile_start[i + 1] - 1 belong to matrix i
-    int n;
+    int start[kMaxGemmGroup + 1];   // row tiles, or CTAs, start[i] .. start[i + 1] - 1 belong to matrix i
+    int n_tiles[kMaxGemmGroup];     // (flat)
+    int n, flat;
 };
 template <bool DUAL>
 __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const __grid_constant__ GemmGroupArgs grp) {
     const int b = static_cast<int>(blockIdx.x);
     int i = 0;
-    while (i + 1 < grp.n && b >= grp.tile_start[i + 1]) ++i;
-    if (static_cast<int>(blockIdx.z) >= grp.m[i].k_splits) return;
-    const int t = (b - grp.tile_start[i]) * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y);
-    gemm_body<DUAL>(grp.m[i], t, 1, t + 1, static_cast<int>(blockIdx.z));
+    while (i + 1 < grp.n && b >= grp.start[i + 1]) ++i;
+    int t = (b - grp.start[i]) * static_cast<int>(gridDim.y) + static_cast<int>(blockIdx.y), bz = static_cast<int>(blockIdx.z);
+    if (grp.flat) {
+        bz = t / grp.n_tiles[i];
+        t -= bz * grp.n_tiles[i];
+    }
+    gemm_body<DUAL>(grp.m[i], t, 1, t + 1, bz);
 }
 
 // y = fp16(norm * inv_scale * sum over K splits, in split order) - fixed order, run-to-run identical - for the matrices of a call
@@ -1035,10 +1043,20 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     FinishArgs fin{};
     int n_fin = 0;
     grp.n = n;
-    grp.tile_start[0] = 0;
-    int max_splits = 1;
+    long n_ctas = 0;
+    int order[kMaxGemmGroup], splits[kMaxGemmGroup];
+    const long tok_tiles = (m + kTileTok - 1) / kTileTok;
     for (int i = 0; i < n; ++i) {
-        const GemmGroupItem& it = items[i];
+        // the split a matrix would get alone, not one for the group as a whole: with fewer splits the group ran 7-9 %
+        // faster (16 / 64 rows) but the fp32 sums changed their order, and results would no longer be bit-equal to
+        // separate calls
+        splits[i] = gemm_k_splits(items[i].out, in, m, n_planes, sm_count);
+        order[i] = i;
+        grp.flat |= splits[i] != splits[0] ? 1 : 0;
+    }
+    std::stable_sort(order, order + n, [&](int a, int b) { return splits[a] < splits[b]; });
+    for (int i = 0; i < n; ++i) {
+        const GemmGroupItem& it = items[order[i]];
         TQ_REQUIRE(it.codes && it.norms && it.table && it.y && it.scratch && it.out >= 1, "tq8_gemm group: NULL argument");
         TQ_REQUIRE(it.in == in && it.n_planes == n_planes && it.block == block,
                    "tq8_gemm group: the matrices must share in_features, the WHT block and the rotation mode");
@@ -1051,18 +1069,18 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
             a.table += 512;
             a.inv_scale *= it.pair_unit;
         }
-        // the split a matrix would get alone, not one for the group as a whole: with fewer splits the group ran 7-9 %
-        // faster (16 / 64 rows) but the fp32 sums changed their order, and results would no longer be bit-equal to
-        // separate calls
-        a.k_splits = gemm_k_splits(it.out, in, m, n_planes, sm_count);
+        a.k_splits = splits[order[i]];
         a.partial = a.k_splits > 1 ? reinterpret_cast<float*>(static_cast<uint8_t*>(it.scratch) + xrot_bytes(in, m, n_planes)) : nullptr;
-        grp.tile_start[i + 1] = grp.tile_start[i] + (it.out + kTileRows - 1) / kTileRows;
-        max_splits = std::max(max_splits, a.k_splits);
+        const long row_tiles = (it.out + kTileRows - 1) / kTileRows, n_tiles = row_tiles * tok_tiles;
+        grp.n_tiles[i] = static_cast<int>(n_tiles);
+        grp.start[i] = static_cast<int>(n_ctas);
+        n_ctas += grp.flat ? n_tiles * a.k_splits : row_tiles;
+        TQ_REQUIRE(n_tiles < (1L << 31) && n_ctas < (1L << 31), "tq8_gemm group: too many output tiles");
         rot.xrot[i] = static_cast<__half*>(it.scratch);
         rot.seed_p[i] = it.seed_p; rot.seed_r[i] = it.seed_r;
         finish_add(fin, n_fin, a);
     }
-    for (int i = n; i < kMaxGemmGroup; ++i) grp.tile_start[i + 1] = grp.tile_start[n];
+    for (int i = n; i <= kMaxGemmGroup; ++i) grp.start[i] = static_cast<int>(n_ctas);
     // 1. the rotations
     launch_rotate_rows(x, rot, n, in, m, n_planes, block, sm_count, stream);
     // 2. the GEMMs
@@ -1074,8 +1092,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
-    const dim3 grid(static_cast<unsigned int>(grp.tile_start[n]), static_cast<unsigned int>((m + kTileTok - 1) / kTileTok),
-                    static_cast<unsigned int>(max_splits));
+    const dim3 grid(static_cast<unsigned int>(n_ctas), grp.flat ? 1u : static_cast<unsigned int>(tok_tiles), grp.flat ? 1u : static_cast<unsigned int>(splits[0]));
     launch_pdl(n_planes == 2 ? tq8_gemm_group_kernel<true> : tq8_gemm_group_kernel<false>, grid, dim3(kGemmThreads), gemm_smem_bytes(m), stream, grp);
     // 3. the split-K sums
     launch_finish(fin, n_fin, static_cast<int>(m), sm_count, stream);
