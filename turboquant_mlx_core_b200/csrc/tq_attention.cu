@@ -949,13 +949,22 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long long
     a.whole_jobs = whole_ns <= share_ns;
     a.parts = 0;
     long best = std::min(whole_ns, share_ns);
-    for (long p = 2; p <= std::min(most / jobs, shortest); ++p) {   // (a part has a tile of every job)
+    // (powers of two, three times them, and as many as there are SMs or ranges: a call's host time is microseconds)
+    const long most_parts = std::min(most / jobs, shortest);   // (a part has a tile of every job)
+    auto consider = [&](long p) {
+        if (p < 2 || p > most_parts) return;
         const long ranges = jobs * p, part = std::max<long>(team, (longest + p - 1) / p);
         const long cost = part * tile_ns(ranges) + ns.merge + (ns.each + p / 4) * p + (ranges > sm_count ? kSecondTeam : 0);
-        if (cost >= best) continue;
+        if (cost >= best) return;
         best = cost;
         a.parts = static_cast<int>(p);
+    };
+    for (long p = 2; p <= most_parts; p *= 2) {
+        consider(p);
+        consider(p + p / 2);
     }
+    consider(sm_count / jobs);
+    consider(most_parts);
     if (a.parts != 0) {
         a.whole_jobs = 0;
         a.ranges = static_cast<int>(jobs * a.parts);
