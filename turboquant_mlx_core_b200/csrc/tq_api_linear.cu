@@ -175,7 +175,9 @@ public:
         const bool decode_call = batch <= 8 || nx * sizeof(__half) <= kHostStageBytes;
         const bool read_now = !x_dev && kx.pinned_alias == nullptr && !tq::stream_is_capturing(st);
         const bool as_params = read_now && nx * sizeof(__half) <= tq::kMaxParamRowBytes;
-        const __half* d_x;
+        // one row of one rotation: a parameter of the decode kernel itself
+        const bool row_inside = as_params && batch == 1 && decode_kernel_ != 2 && tq::gemv_takes_host_row(in_, block_, dual_ ? 2 : 1);
+        const __half* d_x = nullptr;
         std::optional<tq::PinnedStage> x_stage, y_stage;
         // A call that fails half-way has queued work that still reads or writes the staging: wait for it before it goes back.
         struct StageUse {
@@ -186,7 +188,8 @@ public:
                 if (!done && (x || y)) cudaStreamSynchronize(st);
             }
         } stage_use{x_stage, y_stage, st};
-        if (x_dev && x_dtype == TQ_F16) {
+        if (row_inside) {
+        } else if (x_dev && x_dtype == TQ_F16) {
             d_x = static_cast<const __half*>(x);
         } else if (as_params || (read_now && !y_dev && decode_call)) {
             x_f16_.reserve(nx * sizeof(__half) + 16, st);
@@ -231,7 +234,11 @@ public:
             y_f16_.reserve(ny * sizeof(__half), st);
             d_y = y_f16_.as<__half>();
         }
-        launch_forward(d_x, batch, d_y, st);
+        if (row_inside)
+            tq::launch_tq8_gemv_host_row(codes_.as<uint8_t>(), norms_.as<float>(), tables_.as<float>(), x, x_dtype == TQ_F16, d_y, out_, in_, block_,
+                                         seed_p_, scratch_.as<void>(), d_status_, sm_count_, st);
+        else
+            launch_forward(d_x, batch, d_y, st);
         if (!y_dev) {
             if (d_y == y_f16_.as<__half>()) TQ_CUDA(cudaMemcpyAsync(y, d_y, ny * sizeof(__half), cudaMemcpyDeviceToHost, st));
             TQ_CUDA(cudaStreamSynchronize(st));

@@ -56,6 +56,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include <cstring>
+
 #include "tq_common.cuh"
 #include "tq_kernels.cuh"
 
@@ -456,8 +458,13 @@ __device__ __forceinline__ void ll_send_packets(const ScatterArgs& sc, const __h
 // MULTI = more than one slot (row units finished through partial sums in scratch); compile time, so that the
 // single-slot kernels carry none of that path's state in their 128 registers.
 // DUAL = weights with two rotations: table words and activation words are pairs of fp16.
-template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL>
-__device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk) {
+// ROW = the activation row is a kernel parameter, `row` its generic address.
+template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false>
+__device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk, const __half* row = nullptr) {
+    auto load_x = [&](int col) {   // eight columns of the row that is rotated in here
+        if constexpr (ROW) return *reinterpret_cast<const uint4*>(row + col);
+        else return __ldg(reinterpret_cast<const uint4*>(p.x + col));
+    };
     // columns per chunk, derived here: one more field in GemvArgs made ptxas spill within the 128 registers
     const int chunk_cols = p.wpt * kSlice;
     // A warp's partial tile is [16 rows][BP] floats plus 4 floats of padding: the 16 tiles a
@@ -617,9 +624,9 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         }
     }
     uint4 x_first = make_uint4(0, 0, 0, 0);
-    if (!DUAL && p.x != nullptr) {
+    if (ROW || (!DUAL && p.x != nullptr)) {
         const int cl0 = (MULTI ? cur.slot * chunk_cols : 0) + slice0 + 8 * lane;
-        if (cl0 < p.in) x_first = __ldg(reinterpret_cast<const uint4*>(p.x + cl0));
+        if (cl0 < p.in) x_first = load_x(cl0);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -747,7 +754,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             // B fragment of MMA (s, m): k = q -> column 64 s + 16 q + 2 m, k = q+4 -> the next column; n = g.
             const int colw = (MULTI ? slot * chunk_cols : 0) + slice0;  // first column of this warp's slice
             const int col0 = colw + 16 * q;
-            if (BP == 1 && !DUAL && p.x != nullptr) {
+            if (ROW || (BP == 1 && !DUAL && p.x != nullptr)) {
                 // One activation row (the launcher rotates in here only then): rotate this warp's 256 columns of it.
                 // Lane l holds columns 8l..8l+7 of the slice, stages below 8 stay in the lane, the rest are lane
                 // exchanges (same add tree as rotate_x_kernel).  A 1 KB strip of shared memory per warp turns the
@@ -758,7 +765,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 uint4 xc = x0;
                 if (!have_x0) {
                     xc = make_uint4(0, 0, 0, 0);
-                    if (cl < p.in) xc = __ldg(reinterpret_cast<const uint4*>(p.x + cl));
+                    if (cl < p.in) xc = load_x(cl);
                 }
                 const uint32_t xw[4] = {xc.x, xc.y, xc.z, xc.w};
                 float v[8];
@@ -827,7 +834,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             }
         staged_slot = slot;
     };
-    stage_slot(cur.slot, x_first, !DUAL && p.x != nullptr);
+    stage_slot(cur.slot, x_first, ROW || (!DUAL && p.x != nullptr));
 
     for (int i = 0; i < n_local; ++i) {
         if (cur.slot != staged_slot) stage_slot(cur.slot, make_uint4(0, 0, 0, 0), false);
@@ -1004,6 +1011,17 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
 template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_kernel(const GemvArgs p) {
     gemv_body<BP, false, false, MULTI, DUAL>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+}
+// The one activation row of a host caller, which rides in the launch (16 N bytes of fp16): as a kernel of its own in front, which wrote it to
+// device memory, it cost a launch and its end.  4096 x 4096 from and to host memory 31.3 us, 29.7 so, 512 x 14336 39.8 and 33.5.
+template <int N>
+struct GemvRow {
+    uint4 v[N];
+};
+template <int N, bool MULTI>
+__global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_row_kernel(const GemvArgs p, const __grid_constant__ GemvRow<N> row) {
+    gemv_body<1, false, false, MULTI, false, true>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x),
+                                                   reinterpret_cast<const __half*>(row.v));
 }
 template <int BP, bool MULTI, bool DUAL>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_packets_kernel(const GemvArgs p, const ScatterArgs sc) {
@@ -1278,6 +1296,55 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
 #undef TQ_GEMV_LAUNCH
 #undef TQ_GEMV_LAUNCH2
 #undef TQ_GEMV_LAUNCH3
+    }
+}
+
+bool gemv_takes_host_row(int in, uint32_t block, int n_planes) {
+    return n_planes == 1 && block <= static_cast<uint32_t>(kSlice) && in % 8 == 0 && static_cast<size_t>(in) * 2 <= kMaxParamRowBytes;
+}
+template <int N, bool MULTI>
+static void launch_gemv_row(const GemvArgs& a, const void* host_x, bool is_f16, int sm_count, cudaStream_t stream) {
+    GemvRow<N> row;
+    if (is_f16) std::memcpy(row.v, host_x, static_cast<size_t>(a.in) * 2);
+    else host_f32_to_f16(static_cast<const float*>(host_x), reinterpret_cast<uint16_t*>(row.v), static_cast<size_t>(a.in));
+    static bool configured[64] = {false};   // the opt-in shared-memory size is a per-device function attribute
+    int dev = 0;
+    TQ_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !configured[dev]) {
+        TQ_CUDA(cudaFuncSetAttribute((tq8_gemv_row_kernel<N, MULTI>), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemvSmem)));
+        if (dev < 64) configured[dev] = true;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    const int n_units = a.n_row_units * a.n_slots;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(n_units < sm_count ? n_units : sm_count);
+    cfg.blockDim = dim3(kCtaThreads);
+    cfg.dynamicSmemBytes = kGemvSmem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void* args[] = {const_cast<GemvArgs*>(&a), &row};   // by address: the row is copied once, into the launch
+    TQ_CUDA(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(tq8_gemv_row_kernel<N, MULTI>), args));
+}
+void launch_tq8_gemv_host_row(const uint8_t* codes, const float* norms, const float* table, const void* host_x, bool is_f16, __half* y, int out,
+                              int in, uint32_t block, uint32_t seed_p, void* scratch, unsigned int* status, int sm_count, cudaStream_t stream) {
+    TQ_REQUIRE(gemv_takes_host_row(in, block, 1), "tq8_gemv: the activation row does not fit a launch's parameters");
+    TQ_REQUIRE(is_pow2(block) && block >= 32, "WHT block size must be a power of two in [32, 1024]");
+    TQ_REQUIRE(in % static_cast<int>(block) == 0, "in_features must be divisible by block_size");
+    TQ_REQUIRE(scratch != nullptr, "tq8_gemv needs its scratch buffer");
+    if (out == 0) return;
+    GemvArgs a{};
+    a.codes = codes; a.norms = norms; a.table = table; a.y = y; a.status = status;
+    fill_gemv_args(a, nullptr, out, in, 1, block, 1, 1.0f, seed_p, scratch);
+    // the launch copies its whole parameter block: sizes in steps of two
+    if (a.n_slots == 1) {   // 4096 columns at most
+        if (in <= 2048) launch_gemv_row<256, false>(a, host_x, is_f16, sm_count, stream);
+        else launch_gemv_row<512, false>(a, host_x, is_f16, sm_count, stream);
+    } else {
+        if (in <= 8192) launch_gemv_row<1024, true>(a, host_x, is_f16, sm_count, stream);
+        else launch_gemv_row<kMaxParamRowBytes / 16, true>(a, host_x, is_f16, sm_count, stream);
     }
 }
 

@@ -39,6 +39,12 @@ void launch_tq8_gemv(const uint8_t* codes, const float* norms, const float* tabl
                      int out, int in, int batch, uint32_t block, int n_planes, float pair_unit, uint32_t seed_p,
                      uint32_t seed_r, void* scratch, unsigned int* status, int sm_count, cudaStream_t stream);
 
+// One activation row of a host caller, which travels as a kernel parameter: fp32 or fp16 in host memory, read before the call returns.  For
+// weights with one rotation, WHT blocks up to 256 columns and rows of up to kMaxParamRowBytes of fp16.
+bool gemv_takes_host_row(int in, uint32_t block, int n_planes);
+void launch_tq8_gemv_host_row(const uint8_t* codes, const float* norms, const float* table, const void* host_x, bool is_f16, __half* y, int out,
+                              int in, uint32_t block, uint32_t seed_p, void* scratch, unsigned int* status, int sm_count, cudaStream_t stream);
+
 // The same with the fp16 result written to n_dst (1..8) buffers at once: destination d receives
 // activation row n, output row r at dst[d][n * dst_stride + r].  Destinations may be other GPUs'
 // memory mapped into this process (peer access / CUDA IPC): plain stores, no multicast.
