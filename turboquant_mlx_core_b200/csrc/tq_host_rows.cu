@@ -2,8 +2,9 @@
 //
 // A decode call hands over 8 KB and waits for 8 KB.  Through cudaMemcpyAsync from pageable memory, a conversion kernel and
 // a copy back the 4096 x 4096 layer took 45 us, 8 of them in the layer's kernel.  Up to 31 KB of rows now ride in the
-// parameters of a one-CTA kernel, which the launch delivers with no copy engine and no staging in between; the host
-// rounds fp32 to fp16 on the way (half the bytes, no conversion kernel).
+// parameters of a kernel, which the launch delivers with no copy engine and no staging in between; the host
+// rounds fp32 to fp16 on the way (half the bytes, no conversion kernel).  One row that the decode kernel rotates itself is a
+// parameter of that kernel (gemv_takes_host_row); several rows and other blocks go through the one-CTA kernel here.
 #include <cstring>
 #if defined(__x86_64__)
 #include <immintrin.h>
