@@ -34,6 +34,21 @@ def test_fit_against_the_checker(tq, oracle, n, kind):
     assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
 
 
+@pytest.mark.parametrize("n", [3000, 70_001])
+@pytest.mark.parametrize("eighths", [[0], [7], [3, 4], [0, 3, 4, 6], [1, 2, 5, 7], list(range(8))])
+def test_samples_in_some_eighths_of_the_bucket_keys(tq, oracle, n, eighths):
+    """A block of the bucket sums looks at a range of buckets in every eighth of the keys: ranges with and without samples in one."""
+    rng = np.random.default_rng(n)
+    e = rng.choice(eighths, n)                                   # sign and two bits of the exponent, in the order of the keys
+    exponent = (np.where(e >= 4, e - 4, 3 - e) * 64 + rng.integers(1, 60, n)).astype(np.uint32)
+    bits = (exponent << 23) | rng.integers(0, 1 << 23, n).astype(np.uint32) | np.where(e < 4, np.uint32(1) << 31, 0).astype(np.uint32)
+    x = bits.view(np.float32)
+    want, _ = oracle.fit_codebook(x, 4, 20)
+    got = tq.generate_codebook_from_data(x, 4, 20)
+    tol = 3e-6 * np.abs(want) + 3e-7
+    assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
+
+
 @pytest.mark.parametrize("n", [200_000, 1_000_003])
 @pytest.mark.parametrize("share", [0.05, 0.3, 1.0])
 def test_crowded_samples_are_fitted_in_passes_over_all(tq, oracle, n, share):
