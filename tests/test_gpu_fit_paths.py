@@ -34,10 +34,10 @@ def test_fit_against_the_checker(tq, oracle, n, kind):
     assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
 
 
-@pytest.mark.parametrize("n", [3000, 70_001])
-@pytest.mark.parametrize("eighths", [[0], [7], [3, 4], [0, 3, 4, 6], [1, 2, 5, 7], list(range(8))])
+@pytest.mark.parametrize("n,eighths", [(n, e) for n in (3000, 300_000, 2_100_000) for e in ([0], [7], [3, 4], [0, 3, 4, 6], [1, 2, 5, 7], list(range(8)))]
+                         + [(17_000_000, [0, 3, 4, 6])])
 def test_samples_in_some_eighths_of_the_bucket_keys(tq, oracle, n, eighths):
-    """A block of the bucket sums looks at a range of buckets in every eighth of the keys: ranges with and without samples in one."""
+    """A block of the bucket sums looks at up to eight ranges of buckets, evenly spread over the keys: with and without samples in one block."""
     rng = np.random.default_rng(n)
     e = rng.choice(eighths, n)                                   # sign and two bits of the exponent, in the order of the keys
     exponent = (np.where(e >= 4, e - 4, 3 - e) * 64 + rng.integers(1, 60, n)).astype(np.uint32)
@@ -45,6 +45,16 @@ def test_samples_in_some_eighths_of_the_bucket_keys(tq, oracle, n, eighths):
     x = bits.view(np.float32)
     want, _ = oracle.fit_codebook(x, 4, 20)
     got = tq.generate_codebook_from_data(x, 4, 20)
+    tol = 3e-6 * np.abs(want) + 3e-7
+    assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 511, 512, 513, 768, 769, 1023, 1280, 1281, 2305, 8192])
+def test_a_boundary_in_a_bucket_of_this_many_samples(tq, oracle, n):
+    """The iterations read a bucket in steps of 512 and of 256 values; all samples lie in one bucket, and so does a boundary."""
+    x = np.random.default_rng(n).uniform(0.88, 0.995, n).astype(np.float32)
+    want, _ = oracle.fit_codebook(x, 2, 20)
+    got = tq.generate_codebook_from_data(x, 2, 20)
     tol = 3e-6 * np.abs(want) + 3e-7
     assert np.all(np.abs(got.centroids - want) <= tol), np.abs(got.centroids - want).max()
 

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include <functional>
 
 #include "tq_common.cuh"
@@ -56,6 +57,7 @@ struct FitState {
 constexpr int kFitGroup = 256;              // buckets of a group
 constexpr int kFitSumBuckets = 32;          // buckets whose sums a block takes
 constexpr int kFitBatch = 8;                // values of a bucket that a lane requests at once
+constexpr int kFitLongBatch = 16;           // ... of a long one, in the iterations
 constexpr unsigned int kFitMaxBucket = 32768;   // values of a bucket that the iterations look through
 constexpr int kFitLooked = 4096, kFitSlots = 8192;   // samples that fit_look_kernel looks at, its counters
 constexpr unsigned int kFitCrowd = 2 * kFitMaxBucket;
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(256) fit_scatter_kernel(const float* __restric
             if (pos[k] != 0xffffffffu) sorted[pos[k]] = x[k];
     }
 }
-// Bucket sums, and the double sum of every kFitSumBuckets of them.  A block looks at eight ranges of so many buckets, far apart (the
+// Bucket sums, and the double sum of every kFitSumBuckets of them.  A block looks at up to eight ranges of so many buckets, far apart (the
 // samples lie in about a hundred groups of 256 buckets; with a block per group those few blocks took 450 us for 16.8 M samples):
 // a warp each, which writes the zeros of a range without samples, most of them, and then all warps take the others, a bucket each.
 // Bound by the latency of the buckets' loads: 16.8 M normal samples 39 us; with a block per range, 32 768 of which nine tenths
@@ -276,22 +278,26 @@ constexpr int kFitSumRanges = 8;
 static_assert(kFitSumBuckets == 32, "a lane per bucket of a range");
 __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__ sorted, const unsigned int* __restrict__ count,
                                                        const unsigned int* __restrict__ offset, int shift, double* __restrict__ sum,
-                                                       double* __restrict__ part, const FitState* __restrict__ state) {
+                                                       double* __restrict__ part, const FitState* __restrict__ state, int ranges) {
     __shared__ double s_warp[8];
     __shared__ int s_some[kFitSumRanges];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned int below = (1u << shift) - 1u;
-    const int mine = (blockIdx.x + warp * gridDim.x) * kFitSumBuckets + lane;
-    const unsigned int c_mine = count[mine];
-    if (state->go_over_all) return;
-    const bool some = __any_sync(0xffffffffu, c_mine != 0u);
-    if (!some) {
-        sum[mine] = 0.0;
-        if (lane == 0) part[mine / kFitSumBuckets] = 0.0;
+    if (warp < ranges) {
+        const int mine = (blockIdx.x + warp * gridDim.x) * kFitSumBuckets + lane;
+        const unsigned int c_mine = count[mine];
+        if (state->go_over_all) return;
+        const bool some = __any_sync(0xffffffffu, c_mine != 0u);
+        if (!some) {
+            sum[mine] = 0.0;
+            if (lane == 0) part[mine / kFitSumBuckets] = 0.0;
+        }
+        if (lane == 0) s_some[warp] = some ? 1 : 0;
+    } else if (state->go_over_all) {
+        return;
     }
-    if (lane == 0) s_some[warp] = some ? 1 : 0;
     __syncthreads();
-    for (int r = 0; r < kFitSumRanges; ++r) {
+    for (int r = 0; r < ranges; ++r) {
         if (s_some[r] == 0) continue;
         const int range = blockIdx.x + r * gridDim.x;
         const unsigned int c_lane = count[range * kFitSumBuckets + lane], at_lane = offset[range * kFitSumBuckets + lane];
@@ -329,8 +335,10 @@ __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__
     }
 }
 // All iterations of a fit in one CTA, a CTA per fit: warp w follows boundary w, the upper one of bin w.  Bound by the latency of a
-// chain of L2 reads, reductions and barriers: 100 iterations over 16.8 M samples take 340 to 600 us, those of a layer's two
-// fits, side by side, 570 (one after the other 890).  (Significands as 64-bit sums of doubles' conversions took 400 to 660 us; the bits
+// chain of L2 reads, reductions and barriers: a bucket's place, its values, the sums around it and between the boundaries are a few
+// hundred to 2000 cycles each.  Long buckets are read 16 values a lane at a time (eight: six such reads one after the other for 1500
+// values; 24 slow those down whose boundaries lie in small buckets), the rest and small buckets eight, which issues less.  100 iterations of a layer's two fits over 16.8 M samples each, side by side,
+// 497 us (eight at a time throughout 555; 24 470).  (Significands as 64-bit sums of doubles' conversions took 400 to 660 us; the bits
 // below a bucket's prefix are 32-bit sums.  Two warps per boundary that keep their bucket's samples in registers: no change.)
 // `group_sum`: filled here from the parts.
 struct FitJob {
@@ -406,17 +414,21 @@ __global__ void __launch_bounds__(1024) fit_iterate_kernel(const __grid_constant
             }
             unsigned int c = 0, t = 0;   // t: 1024 x 2^20 at most
             if (b_count <= kFitMaxBucket) {
-                for (unsigned int i = lane; i < b_count; i += 32 * kFitBatch) {
-                    float x[kFitBatch];
+                const auto look = [&](auto batch, unsigned int i) {
+                    constexpr int B = decltype(batch)::value;
+                    float x[B];
 #pragma unroll
-                    for (int j = 0; j < kFitBatch; ++j) x[j] = i + 32u * j < b_count ? sorted[b_at + i + 32u * j] : INFINITY;
+                    for (int j = 0; j < B; ++j) x[j] = i + 32u * j < b_count ? sorted[b_at + i + 32u * j] : INFINITY;
 #pragma unroll
-                    for (int j = 0; j < kFitBatch; ++j) {
+                    for (int j = 0; j < B; ++j) {
                         const bool le = !(bound < x[j]);   // (the padding is not)
                         c += le ? 1u : 0u;
                         t += le ? __float_as_uint(x[j]) & ((1u << shift) - 1u) : 0u;
                     }
-                }
+                };
+                unsigned int at = 0;
+                for (; at + 32u * (kFitLongBatch - kFitBatch) < b_count; at += 32u * kFitLongBatch) look(std::integral_constant<int, kFitLongBatch>{}, at + lane);
+                for (; at < b_count; at += 32u * kFitBatch) look(std::integral_constant<int, kFitBatch>{}, at + lane);
             }
             c = __reduce_add_sync(0xffffffffu, c);
             const unsigned int t_high = __reduce_add_sync(0xffffffffu, t >> 16), t_low = __reduce_add_sync(0xffffffffu, t & 0xffffu);
@@ -744,7 +756,9 @@ public:
         fit_offsets_kernel<<<n_groups_, 256, 0, stream_>>>(d_count, d_group, d_offset, d_cursor);
         if (windowed_) fit_scatter_window_kernel<<<window_ctas_, 1024, window_bytes(), stream_>>>(r_.data, un, shift_, window_, d_offset, begin_, d_cursor, d_sorted, state());
         else fit_scatter_kernel<<<grid, 256, 0, stream_>>>(r_.data, un, shift_, d_cursor, d_sorted, state());
-        fit_sums_kernel<<<n_parts / kFitSumRanges, 256, 0, stream_>>>(d_sorted, d_count, d_offset, shift_, d_sum, d_part, state());
+        int ranges = kFitSumRanges;   // fewer where the blocks would not fill the device: 1 M samples of all exponents, 2048 ranges, 188 us, 193 with eight
+        while (ranges > 1 && n_parts / ranges < 8 * sms_) ranges /= 2;
+        fit_sums_kernel<<<n_parts / ranges, 256, 0, stream_>>>(d_sorted, d_count, d_offset, shift_, d_sum, d_part, state(), ranges);
         TQ_CUDA(cudaGetLastError());
         job = FitJob{d_sorted, d_count, d_offset, d_sum, d_part, d_group_sum, state(), un, n_groups_, shift_, r_.iterations};
         iterated_ = true;
