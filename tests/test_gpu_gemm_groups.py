@@ -48,3 +48,28 @@ def test_grouped_matrices_of_other_splits(tq, oracle, outs, m, shared):
         lin.check_status()
     for lin in lins:
         lin.close()
+
+
+@pytest.mark.parametrize("m", [128, 256])
+@pytest.mark.parametrize("shared", [True, False])
+def test_weight_tiles_that_wait_for_their_slot(tq, m, shared):
+    """Tall activation tiles: the products are slower than the lookups, so that every weight tile is written as soon as the MMAs have read the
+    one before it in its slot.  Columns of one pipeline stage in 16 have an activation, the others' weights are a hundred times as large: a tile
+    that is read too late or overwritten too early does not go unseen.  Against the dequantised weights; the tolerance of the tile edges."""
+    import torch
+    c = tq.generate_codebook(4)
+    g = torch.Generator(device="cuda").manual_seed(m)
+    cols, rows = 8192, 20000
+    stage = torch.arange(cols, device="cuda") // 128
+    some = (stage % 16 == 5).float()
+    w = torch.randn((rows, cols), device="cuda", generator=g) * (2.0 - 1.98 * some)
+    lin = tq.TurboQuantLinear(cols, rows, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, 128, shared)), c, c, 128)
+    x = (torch.randn((m, cols), device="cuda", generator=g) * some).half()
+    back = lin.dequantize(out=torch.empty((rows, cols), device="cuda", dtype=torch.float16))
+    y = lin.forward(x)
+    want = x.double() @ back.double().T
+    assert rel_l2(y.cpu().numpy(), want.cpu().numpy()) < 4.9e-4 + 2.0 ** -11   # (and the dequantised weights' own rounding)
+    for _ in range(10):
+        assert torch.equal(lin.forward(x), y)
+    lin.check_status()
+    lin.close()

@@ -566,11 +566,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                          : "=r"(ready) : "r"(bar_e), "r"(par) : "memory");
             auto slot_free = [&] {
-                if (__all_sync(0xffffffffu, ready)) return true;
-                if (__all_sync(0xffffffffu, bar_wait(bar_e, par, abort_flag))) return true;
-                raise_status(p.status, 6u);
-                atomicExch(&s_abort, 1u);
-                return false;
+                if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, bar_wait(bar_e, par, abort_flag))) {
+                    raise_status(p.status, 6u);
+                    atomicExch(&s_abort, 1u);
+                    return false;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");   // the MMAs' reads of the slot before the stores to it
+                return true;
             };
             // where the group's next stage is
             f_it += kGroups;
