@@ -239,6 +239,11 @@ int tq_linear_forward_scatter(tq_linear_t lin, const void* x_fp16_device, int ba
 int tq_linear_forward_group(const tq_linear_t* lins, int n, const void* x_fp16_device, int batch, void* const* y_fp16_device,
                             void* stream);
 
+/** CTAs that share an output tile (128 weight rows x 256 activation rows) of a forward of more than eight rows, along K, on a device of `sms`
+ *  multiprocessors; planes: 1, or 2 for a layer with two rotations.  The same alone and in a group, where the sums of the splits
+ *  have to be the same.  Needs no device; -1 for sizes that are none. */
+int tq_linear_k_splits(int out_features, int in_features, long rows, int planes, int sms);
+
 /** Forward whose fp16 result is this layer's rows inside a wider buffer: activation row n goes to
  *  y_fp16_device[n * y_row_stride ...] (y_row_stride >= out_features, in elements).  x and y are
  *  device pointers; any batch size (decode kernel up to 8 rows, tensor-memory kernel above).  A

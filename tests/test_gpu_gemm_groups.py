@@ -32,7 +32,8 @@ def test_stages_and_groups(tq, oracle, cols, rows, m, shared):
 @pytest.mark.parametrize("outs", [(3584, 512, 512), (200, 3000), (64, 130, 9000, 64), (512, 512)])
 @pytest.mark.parametrize("m", [9, 64, 300])
 @pytest.mark.parametrize("shared", [True, False])
-def test_grouped_matrices_of_other_splits(tq, oracle, outs, m, shared):
+@pytest.mark.parametrize("cols", [1536, 4096])
+def test_grouped_matrices_of_other_splits(tq, oracle, outs, m, shared, cols):
     """Matrices whose K is split differently (few weight rows: many splits), in any order, against calls of their own: the same bits."""
     import torch
     rng = np.random.default_rng(m + sum(outs))
@@ -40,9 +41,9 @@ def test_grouped_matrices_of_other_splits(tq, oracle, outs, m, shared):
     c = tq.codebook_from_centroids(cb)
     lins = []
     for o in outs:
-        w = (rng.standard_normal((o, 1536)) * 0.02).astype(np.float32)
-        lins.append(tq.TurboQuantLinear(1536, o, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, 128, shared)), c, c, 128))
-    x = torch.from_numpy(rng.standard_normal((m, 1536)).astype(np.float16)).cuda()
+        w = (rng.standard_normal((o, cols)) * 0.02).astype(np.float32)
+        lins.append(tq.TurboQuantLinear(cols, o, tq.quantize_weight(w, c, c, tq.QuantizerConfig(4, 4, 128, shared)), c, c, 128))
+    x = torch.from_numpy(rng.standard_normal((m, cols)).astype(np.float16)).cuda()
     for lin, y in zip(lins, tq.forward_group(lins, x)):
         assert torch.equal(y, lin.forward(x))
         lin.check_status()

@@ -77,6 +77,7 @@ def load() -> C.CDLL:
     sig("tq_linear_forward_noalloc", i, [vp, vp, i, vp, vp])
     sig("tq_linear_forward_strided", i, [vp, vp, i, vp, C.c_long, vp])
     sig("tq_linear_noalloc_scratch_limit", C.c_size_t, [])
+    sig("tq_linear_k_splits", i, [i, i, C.c_long, i, i])
     sig("tq_linear_forward_group", i, [C.POINTER(C.c_void_p), i, vp, i, C.POINTER(C.c_void_p), vp])
     sig("tq_linear_dequantize", i, [vp, vp, i, vp])
     sig("tq_linear_status", i, [vp])

@@ -619,6 +619,14 @@ int tq_linear_forward_noalloc(tq_linear_t lin, const void* x_fp16_device, int ba
     });
 }
 
+int tq_linear_k_splits(int out_features, int in_features, long rows, int planes, int sms) {
+    return guarded<int>(0, -1, [&]() {
+        TQ_REQUIRE(out_features >= 1 && in_features >= 1 && tq::gemm_supported(in_features) && rows >= 1 && (planes == 1 || planes == 2) && sms >= 1,
+                   "tq_linear_k_splits: bad sizes");
+        return tq::gemm_k_splits(out_features, in_features, rows, planes, sms);
+    });
+}
+
 size_t tq_linear_noalloc_scratch_limit(void) { return tq::gemv_static_scratch_capacity(); }
 
 int tq_linear_dequantize(tq_linear_t lin, void* result, int result_dtype, void* stream) {

@@ -961,13 +961,15 @@ size_t xrot_bytes(int in, long m, int n_planes) {
 }  // namespace
 
 // When the output has too few tiles to occupy the SMs (few activation rows on a matrix with few
-// rows and many columns), K is split over several CTAs per tile: up to eight splits of four K blocks at least, more of eight.  (All of
-// eight: 1024 x 1024 at 32 rows 9.0 us, 8.0 so, 600 x 2048 at 100 rows 11.5 and 10.0, 4096 x 1024 at 20 9.4 and 8.8; up to twelve splits of
-// four: 512 x 8192 at 12 rows 9.8 -> 10.3, whose sums then outweigh what the CTAs gain.)
+// rows and many columns), K is split over several CTAs per tile; every split keeps at least 8 K blocks.  (Splits of four, up to eight of them, are up to
+// 12 % faster for a matrix of up to 2048 columns alone, 1024 x 1024 at 32 rows 8.7 -> 7.9 us.  But a matrix has the same splits in a group, for the same bits,
+// and the CTAs of a group then outnumber the SMs: 2048 -> 2048 + 256 + 256 at 32 rows 9.2 -> 13.6, 2560 -> 2560 + 512 + 512 9.8 -> 15.1.  And of 512 or 768 columns
+// the sums outweigh what the CTAs gain: 512 x 8192 at 128 rows 9.0 -> 14.1.)
 int gemm_k_splits(int out, int in, long m, int n_planes, int sm_count) {
     const long tiles = static_cast<long>((out + kTileRows - 1) / kTileRows) * ((m + kTileTok - 1) / kTileTok);
     const int n_kb = in / kBlockK * n_planes;
-    const long s = std::min<long>(sm_count / (tiles > 0 ? tiles : 1), std::max(n_kb / 8, std::min(8, n_kb / 4)));
+    long s = sm_count / (tiles > 0 ? tiles : 1);
+    if (s > n_kb / 8) s = n_kb / 8;
     return s < 1 ? 1 : static_cast<int>(s);
 }
 
