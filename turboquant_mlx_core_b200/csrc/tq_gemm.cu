@@ -265,11 +265,16 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
 // rows of a K block are 1 KB of the operand tile: they meet in shared memory (slots of a core matrix's rows permuted by its column: no
 // bank conflicts) and leave as contiguous stores; a lane's own 16-byte pieces of a row are 128 bytes apart.
 // Instructions bound it, a third of the time the lane exchanges alone: 286 per 256 columns of a row with the exchanges in a loop, 64-bit places
-// and the signs of the lanes found anew for every row; 218 so, and the signs are made in front of the wait.  2048 x 18944: 53 -> 44 us under the
+// and the signs of the lanes found anew for every row; 218 so.  2048 x 18944: 53 -> 44 us under the
 // profiler, 64 x 18944 with the product behind it 27.5 -> 25.2.  With two columns an instruction (fp32 pairs): 302, the pairs have to be made.
 template <int CHUNKS, int STAGES>
 __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, int rows, int block, uint32_t seed,
                                                       unsigned col_group, unsigned row_group, float inv_sqrt, int row_steps, uint4 (*s_rows)[256 * CHUNKS]) {
+    // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done.  A CTA of few rows waits first, so that the
+    // product's CTAs may come and set themselves up beside it: with the signs in front 8192 x 512, block 512, took 13.6 us at 100 rows instead
+    // of 11.8 (with the older loop 13.0), 1024 x 512, block 64, 10.8 at 128 instead of 10.0.  Many rows' CTAs, wave after wave, have them made by then.
+    const bool wait_first = CHUNKS == 1 || row_steps == 1;
+    if (wait_first) pdl_wait_release();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int col = static_cast<int>(col_group) * 256 * CHUNKS + 8 * lane;
     // in is a multiple of 64 and of the block: whole lanes only, and exchanges stay inside a block.  (A group of several
@@ -302,7 +307,7 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
         return xrot + (static_cast<size_t>(row8 / kTileTok) * kb_per_plane + kb_at) * (kTileTok * kBlockK) + ((row8 % kTileTok >> 3) * 64 + t) * 8;
     };
     __half* dst = place(first);
-    pdl_wait_release();   // x, and the scratch this kernel overwrites, belong to the kernels before it until they are done
+    if (!wait_first) pdl_wait_release();
     // a row's loads are on their way while the one before it is worked on (not of blocks of 1024, which fill the registers)
     constexpr bool kAhead = CHUNKS <= 2;
     uint4 next[CHUNKS];
