@@ -157,16 +157,20 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
     const uint32_t seed = plane ? seed_r : seed_p;
     const __half* const src = x + static_cast<size_t>(row) * in + col;
-    uint4 signs[CHUNKS];   // in front of the wait: 4096 x 4096 at eight rows 9.9 -> 9.6 us with the product
-#pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
+    // The signs of one chunk in front of the wait: 4096 x 4096 at eight rows 9.9 -> 9.6 us with the product.  Those of two or four take longer than
+    // the loads, behind which they are made: in front, 4096 x 4096, block 512, took 8.8 us at one row instead of 8.3, 1024 x 1024 6.4 instead of 5.9.
+    uint4 signs;
+    if (CHUNKS == 1) signs = chunk_signs(seed, static_cast<uint32_t>(col), block);
     grid_dependency_sync();
     uint4 raw[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
     float v[CHUNKS][8];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
+    for (int c = 0; c < CHUNKS; ++c) {
+        if (CHUNKS > 1) signs = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
+        rotate_chunk(v[c], raw[c], signs, block, lane, live);
+    }
 #pragma unroll
     for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll
