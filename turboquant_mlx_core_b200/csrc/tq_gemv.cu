@@ -74,7 +74,7 @@ constexpr uint32_t kLutBytes = 0x10000u;  // 256 entries * 256 B
 // Partial-sum ring: ring * 16 warps * (16 rows * bp + 4) floats.  Eight rows take three slots of 32 KB, which tied the warps to each
 // other's pace: seven of 60 KB, 151936 x 2048 75.4 -> 73.9 us, 37888 x 3584 41.1 -> 40.1.  (Fewer rows have seven to sixteen slots as it is, and
 // gained nothing from more.  With two rotations a unit takes longer, the sums keep up, and those of the last units, three behind instead of one, come at the
-// end: five rows, 4096 x 11008 17.1 us with three slots, 18.5 with seven, 4096 x 14336 21.6 and 22.6, 18944 x 3584 24.7 and 25.3.)
+// end: five rows, 11008 x 4096 17.1 us with three slots, 18.5 with seven, 14336 x 4096 21.6 and 22.6, 18944 x 3584 24.7 and 25.3.)
 __host__ __device__ constexpr int red_bytes(int bp, bool dual) { return bp == 8 && !dual ? 61440 : 32768; }
 constexpr int kMaxRing = 16;
 constexpr int kFlushUnits = 8;             // units a warp finishes between two arrival counts (several slots only)
