@@ -97,3 +97,28 @@ def test_sum_of_slots_and_rmsnorm(tq, n_slots, residual, cols, offset):
     for s in range(n_slots):
         want = want + slots[s].float()
     assert torch.equal(outs[0], want.half()) and torch.equal(outs[2], outs[0]) and torch.equal(outs[3], outs[1])
+
+
+@pytest.mark.parametrize("n_slots,residual", [(1, True), (3, False), (8, True)])
+@pytest.mark.parametrize("cols,offset", [(c, 0) for c in (2040, 2048, 2056, 4088, 4096, 4104, 8184, 8192, 8200)] + [(2046, 0), (8194, 0), (4096, 2)])
+def test_rows_at_the_ends_of_what_stays_in_registers(tq, n_slots, residual, cols, offset):
+    """One, two, four steps of 2048 columns in registers, and more: the norm against 64 bits, the fused form against the norm on its own."""
+    import torch
+    L = tq.load()
+    rng = np.random.default_rng(cols + n_slots)
+    rows, n = 5, 5 * cols
+    slots = _at(torch, rng.standard_normal((n_slots, rows, cols)).astype(np.float16), offset)
+    res = _at(torch, rng.standard_normal((rows, cols)).astype(np.float16), offset) if residual else None
+    w = _at(torch, (1 + 0.1 * rng.standard_normal(cols)).astype(np.float16), offset)
+    outs = [_at(torch, np.zeros((rows, cols), np.float16), offset) for _ in range(4)]
+    r = _p(res) if residual else None
+    assert L.tq_exchange_sum_f16(_p(slots), n_slots, n, n, r, _p(outs[0]), None) == 0
+    assert L.tq_rmsnorm_f16(_p(outs[0]), _p(w), _p(outs[1]), rows, cols, 1e-6, None) == 0
+    assert L.tq_exchange_sum_f16_rmsnorm(_p(slots), n_slots, n, rows, cols, r, _p(outs[2]), _p(w), _p(outs[3]), 1e-6, None) == 0
+    torch.cuda.synchronize()
+    want = res.float() if residual else torch.zeros((rows, cols), device="cuda")
+    for s in range(n_slots):
+        want = want + slots[s].float()
+    assert torch.equal(outs[0], want.half()) and torch.equal(outs[2], outs[0]) and torch.equal(outs[3], outs[1])
+    x = outs[0].double()
+    assert rel_l2(outs[1].cpu().numpy(), (x / torch.sqrt((x ** 2).mean(1, keepdim=True) + 1e-6) * w.double()).cpu().numpy()) < TOL

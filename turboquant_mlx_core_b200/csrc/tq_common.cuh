@@ -294,7 +294,7 @@ __device__ __forceinline__ void rotate_chunk_fixed(float (&v)[8], const uint4& r
 
 // Threads of a CTA that normalises a row (the RMSNorm kernel and the row-wise all-reduce tails: the same count, so the same
 // order of additions).  Eight columns per thread and step: 256 threads take 8192 columns in the four steps that stay in
-// registers, and eight rows run on an SM at a time (with 1024 threads and two columns per step a row's barriers and
+// registers, and four to eight rows run on an SM at a time (with 1024 threads and two columns per step a row's barriers and
 // reduction were most of its time).
 constexpr int kRowNormThreads = 256;
 constexpr int kRowNormKeep = 4;
@@ -310,24 +310,36 @@ __device__ __forceinline__ void store_row8(__half* p, int n, const uint4& v) {
     if constexpr (WIDE) *reinterpret_cast<uint4*>(p) = v;
     else store_halves(p, n, v);
 }
-__device__ __forceinline__ bool rows_wide(int cols, const void* a, const void* b, const void* c) {
+__host__ __device__ __forceinline__ bool rows_wide(int cols, const void* a, const void* b, const void* c) {
     return cols % 8 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
+// KEEP: the steps of a row that stay in registers, as many as its columns need, at most kRowNormKeep; kRowNormMore: so many, and others that are
+// read twice.  Fewer leave room for more CTAs on an SM, which is what many rows are bound by (row_ctas; 0: the plain sum): with registers for
+// four steps whatever the columns, and three CTAs, 512 x 1024 took 2.3 us and the sum of two slots with it 3.5, 1.6 and 2.3 so; 2048 x 3584 6.2 and 11.3, 4.5
+// and 7.4.  Rows that are not whole 16-byte pieces keep four steps and ask for the weights late, as many registers as that takes.
+constexpr int kRowNormMore = kRowNormKeep + 1;
+constexpr int row_ctas(int keep) { return keep == 0 ? 8 : keep == 1 ? 6 : keep == 2 ? 5 : 4; }
+#define TQ_ROW_KERNEL(K, KERNEL, WIDE, COLS)                                                        \
+    K = KERNEL<false, kRowNormMore>;                                                                \
+    if (WIDE) K = (COLS) <= 8 * kRowNormThreads ? KERNEL<true, 1>                                   \
+                  : (COLS) <= 16 * kRowNormThreads ? KERNEL<true, 2>                                \
+                  : (COLS) <= 8 * kRowNormKeep * kRowNormThreads ? KERNEL<true, kRowNormKeep> : KERNEL<true, kRowNormMore>;
 
 // yr[:] = xr[:] * rsqrt(mean(xr[:]^2) + eps) * w for one row, by the whole CTA (kRowNormThreads threads; cols even).  A
-// thread takes the columns 8 (threadIdx.x + k * kRowNormThreads) .. + 7, whatever the alignment, the first kRowNormKeep
-// steps of them in `keep`; the others are read from xr.  Shared by the RMSNorm kernel and the all-reduce tails that
-// normalise the row they have just summed, so the fused and the separate form give the same bits.  The weights are asked for
+// thread takes the columns 8 (threadIdx.x + k * kRowNormThreads) .. + 7, whatever the alignment, the first KEEP
+// steps of them in `keep`; the others (MORE) are read from xr.  Shared by the RMSNorm kernel and the all-reduce tails that
+// normalise the row they have just summed, so the fused and the separate form give the same bits.  WIDE: the weights are asked for
 // in front of the sum of squares, whose barrier they would otherwise be waited for behind.
-template <bool WIDE>
-__device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], const __half* xr, const __half* __restrict__ w, __half* yr, int cols,
-                                             float eps) {
+template <bool WIDE, bool MORE, int KEEP>
+__device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[KEEP], const __half* xr, const __half* __restrict__ w, __half* yr, int cols, float eps) {
     constexpr int kStep = 8 * kRowNormThreads;
     const int c0 = threadIdx.x * 8;
-    uint4 gain[kRowNormKeep];
+    uint4 gain[KEEP];
+    if constexpr (WIDE) {
 #pragma unroll
-    for (int k = 0; k < kRowNormKeep; ++k)
-        gain[k] = c0 + k * kStep < cols ? load_row8<WIDE>(w + c0 + k * kStep, cols - c0 - k * kStep) : make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < KEEP; ++k)
+            gain[k] = c0 + k * kStep < cols ? load_row8<WIDE>(w + c0 + k * kStep, 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
     float ss = 0.f;
     auto add = [&](const uint4& raw) {
         float v[8];
@@ -336,8 +348,9 @@ __device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], 
         for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
     };
 #pragma unroll
-    for (int k = 0; k < kRowNormKeep; ++k) add(keep[k]);   // (zero beyond the row)
-    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) add(load_row8<WIDE>(xr + c, cols - c));
+    for (int k = 0; k < KEEP; ++k) add(keep[k]);   // (zero beyond the row)
+    if constexpr (MORE)
+        for (int c = c0 + KEEP * kStep; c < cols; c += kStep) add(load_row8<WIDE>(xr + c, cols - c));
     __shared__ float s_part[kRowNormThreads / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -356,19 +369,23 @@ __device__ __forceinline__ void rmsnorm_kept(const uint4 (&keep)[kRowNormKeep], 
         store_row8<WIDE>(yr + c, cols - c, pack_halves(v));
     };
 #pragma unroll
-    for (int k = 0; k < kRowNormKeep; ++k)
-        if (c0 + k * kStep < cols) write(c0 + k * kStep, keep[k], gain[k]);
-    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) write(c, load_row8<WIDE>(xr + c, cols - c), load_row8<WIDE>(w + c, cols - c));
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = c0 + k * kStep;
+        if (c < cols) write(c, keep[k], WIDE ? gain[k] : load_row8<WIDE>(w + c, cols - c));
+    }
+    if constexpr (MORE)
+        for (int c = c0 + KEEP * kStep; c < cols; c += kStep) write(c, load_row8<WIDE>(xr + c, cols - c), load_row8<WIDE>(w + c, cols - c));
 }
-template <bool WIDE>
+template <bool WIDE, int KEEP>
 __device__ __forceinline__ void rmsnorm_row(const __half* xr, const __half* __restrict__ w, __half* yr, int cols, float eps) {
-    uint4 keep[kRowNormKeep];
+    constexpr int kKeep = KEEP < kRowNormMore ? KEEP : kRowNormKeep;
+    uint4 keep[kKeep];
 #pragma unroll
-    for (int k = 0; k < kRowNormKeep; ++k) {
+    for (int k = 0; k < kKeep; ++k) {
         const int c = 8 * (threadIdx.x + k * kRowNormThreads);
         keep[k] = c < cols ? load_row8<WIDE>(xr + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
     }
-    rmsnorm_kept<WIDE>(keep, xr, w, yr, cols, eps);
+    rmsnorm_kept<WIDE, KEEP == kRowNormMore>(keep, xr, w, yr, cols, eps);
 }
 
 __device__ __forceinline__ void raise_status(unsigned int* status, unsigned int code) {

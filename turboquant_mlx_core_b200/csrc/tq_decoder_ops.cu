@@ -20,13 +20,11 @@ __device__ __forceinline__ void ops_dependency_sync() {
 }
 
 // y[r, :] = x[r, :] * rsqrt(mean(x[r, :]^2) + eps) * w      one CTA per row
-__global__ void __launch_bounds__(kRowNormThreads) rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
+template <bool WIDE, int KEEP>
+__global__ void __launch_bounds__(kRowNormThreads, row_ctas(KEEP)) rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
                                                       int cols, float eps) {
     ops_dependency_sync();
-    const __half* const xr = x + static_cast<size_t>(blockIdx.x) * cols;
-    __half* const yr = y + static_cast<size_t>(blockIdx.x) * cols;
-    if (rows_wide(cols, x, w, y)) rmsnorm_row<true>(xr, w, yr, cols, eps);
-    else rmsnorm_row<false>(xr, w, yr, cols, eps);
+    rmsnorm_row<WIDE, KEEP>(x + static_cast<size_t>(blockIdx.x) * cols, w, y + static_cast<size_t>(blockIdx.x) * cols, cols, eps);
 }
 
 // Rotary embedding, "rotate half" convention: element i of a head pairs with element i + d/2;
@@ -136,7 +134,9 @@ void launch_rmsnorm_f16(const __half* x, const __half* weight, __half* y, long r
     if (rows == 0) return;
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = ops_config(static_cast<unsigned>(rows), kRowNormThreads, stream, attr);
-    TQ_CUDA(cudaLaunchKernelEx(&cfg, rmsnorm_kernel, x, weight, y, cols, eps));
+    decltype(&rmsnorm_kernel<true, 1>) kernel;
+    TQ_ROW_KERNEL(kernel, rmsnorm_kernel, rows_wide(cols, x, weight, y), cols)
+    TQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, x, weight, y, cols, eps));
 }
 
 // Whether the row kernel took the call: head sizes up to 512 in sixteens, aligned tensors.

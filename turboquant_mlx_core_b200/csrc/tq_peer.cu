@@ -15,6 +15,7 @@
 // nothing in the kernel arguments changes from step to step.  exchange_sum_f16 adds the ranks'
 // slots in rank order (fixed order: every rank computes the same bits), exchange_merge_attention
 // merges softmax parts.  A kernel only ever waits for kernels running on OTHER GPUs.
+#include <algorithm>
 #include <cstdint>
 
 #include "tq_common.cuh"
@@ -102,11 +103,11 @@ __global__ void exchange_wait_kernel(const unsigned int* __restrict__ flags, int
 }
 
 // out[i] = fp16( residual[i] + sum over slots s, in slot order, of fp32(slots[s][i]) )   (residual may be NULL)
-// ROWS (one CTA per row of `cols` elements): the CTA then writes normed[row] = RMSNorm(out[row]) * norm_w, the bits
-// rmsnorm_kernel would give on out.  (A kernel of its own: its registers would leave the plain sum half the warps, 7.4 us instead of 6.0 for
-// 2048 x 3584 in the L2 cache.)
-template <bool ROWS>
-__global__ void __launch_bounds__(kRowNormThreads) exchange_sum_f16_kernel(const __half* __restrict__ slots, int n_slots, long slot_stride,
+// WIDE: whole 16-byte pieces.  KEEP != 0 (one CTA per row of `cols` elements): the CTA then writes normed[row] = RMSNorm(out[row]) * norm_w,
+// the bits rmsnorm_kernel would give on out.  (Kernels of their own: the plain
+// sum, whose blocks are eight to an SM, took 5.9 us for 2048 x 3584 with the registers of the others, 4.2 so.)
+template <bool WIDE, int KEEP>
+__global__ void __launch_bounds__(kRowNormThreads, row_ctas(KEEP)) exchange_sum_f16_kernel(const __half* __restrict__ slots, int n_slots, long slot_stride,
                                                                long count, const __half* __restrict__ residual, __half* __restrict__ out,
                                                                const __half* __restrict__ norm_w, __half* __restrict__ normed, int cols,
                                                                float eps) {
@@ -115,65 +116,66 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_f16_kernel(const
     // the sum of (up to) eight elements from i on, rounded and stored
     auto sum8 = [&](long i, int n) {
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, h[8];
-        if (residual != nullptr) unpack_halves(load_halves(residual + i, n), a);
+        if (residual != nullptr) unpack_halves(load_row8<WIDE>(residual + i, n), a);
+#pragma unroll (KEEP == 0 ? 1 : 4)
         for (int s = 0; s < n_slots; ++s) {   // written by other GPUs: plain loads after the acquire of the wait kernel
-            unpack_halves(load_halves(slots + s * slot_stride + i, n), h);
+            unpack_halves(load_row8<WIDE>(slots + s * slot_stride + i, n), h);
 #pragma unroll
             for (int j = 0; j < 8; ++j) a[j] += h[j];
         }
         const uint4 r = pack_halves(a);
-        store_halves(out + i, n, r);
+        store_row8<WIDE>(out + i, n, r);
         return r;
     };
-    if constexpr (!ROWS) {
+    if constexpr (KEEP == 0) {
         const long step = static_cast<long>(gridDim.x) * blockDim.x * 8;
         for (long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8; i < count; i += step)
             sum8(i, static_cast<int>(min(8L, count - i)));
-        return;
-    }
-    // a row per CTA; a thread sums the columns that it normalises afterwards (rmsnorm_kept's)
-    const long row = static_cast<long>(blockIdx.x) * cols;
-    const int c0 = 8 * threadIdx.x;
-    constexpr int kStep = 8 * kRowNormThreads;
-    uint4 keep[kRowNormKeep];
-    if (rows_wide(cols, slots, residual, out) && rows_wide(cols, norm_w, normed, nullptr) && slot_stride % 8 == 0) {
-        // Whole 16-byte pieces, all of a thread's loads and then the weights on their way together: with a look at the alignment in front
-        // of each load 2048 x 3584 took 11.1 us instead of 8.8, one row of 3584 2.9 instead of 1.9.
-        uint4 res[kRowNormKeep];
+    } else {
+        // a row per CTA; a thread sums the columns that it normalises afterwards (rmsnorm_kept's)
+        const long row = static_cast<long>(blockIdx.x) * cols;
+        const int c0 = 8 * threadIdx.x;
+        constexpr int kStep = 8 * kRowNormThreads;
+        constexpr int kKeep = KEEP < kRowNormMore ? KEEP : kRowNormKeep;
+        uint4 keep[kKeep];
+        if constexpr (WIDE) {
+            // All of a thread's loads and then the weights on their way together: with a look at the alignment in front
+            // of each load 2048 x 3584 took 11.1 us instead of 6.2, one row of 3584 2.9 instead of 1.5.
+            uint4 res[kKeep];
 #pragma unroll
-        for (int k = 0; k < kRowNormKeep; ++k) {
-            const bool in = c0 + k * kStep < cols;
-            res[k] = in && residual != nullptr ? *reinterpret_cast<const uint4*>(residual + row + c0 + k * kStep) : make_uint4(0u, 0u, 0u, 0u);
-            keep[k] = in ? *reinterpret_cast<const uint4*>(slots + row + c0 + k * kStep) : make_uint4(0u, 0u, 0u, 0u);
-        }
+            for (int k = 0; k < kKeep; ++k) {
+                const bool in = c0 + k * kStep < cols;
+                res[k] = in && residual != nullptr ? *reinterpret_cast<const uint4*>(residual + row + c0 + k * kStep) : make_uint4(0u, 0u, 0u, 0u);
+                keep[k] = in ? *reinterpret_cast<const uint4*>(slots + row + c0 + k * kStep) : make_uint4(0u, 0u, 0u, 0u);
+            }
 #pragma unroll
-        for (int k = 0; k < kRowNormKeep; ++k) {
-            const int c = c0 + k * kStep;
-            if (c >= cols) continue;
-            float a[8], h[8];
-            unpack_halves(res[k], a);
-            unpack_halves(keep[k], h);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) a[j] += h[j];
-            for (int s = 1; s < n_slots; ++s) {
-                unpack_halves(*reinterpret_cast<const uint4*>(slots + s * slot_stride + row + c), h);
+            for (int k = 0; k < kKeep; ++k) {
+                const int c = c0 + k * kStep;
+                if (c >= cols) continue;
+                float a[8], h[8];
+                unpack_halves(res[k], a);
+                unpack_halves(keep[k], h);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) a[j] += h[j];
-            }
-            keep[k] = pack_halves(a);
-            *reinterpret_cast<uint4*>(out + row + c) = keep[k];
-        }
-        for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) sum8(row + c, cols - c);
-        rmsnorm_kept<true>(keep, out + row, norm_w, normed + row, cols, eps);
-        return;
-    }
+                for (int s = 1; s < n_slots; ++s) {
+                    unpack_halves(*reinterpret_cast<const uint4*>(slots + s * slot_stride + row + c), h);
 #pragma unroll
-    for (int k = 0; k < kRowNormKeep; ++k) {
-        const int c = c0 + k * kStep;
-        keep[k] = c < cols ? sum8(row + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
+                    for (int j = 0; j < 8; ++j) a[j] += h[j];
+                }
+                keep[k] = pack_halves(a);
+                *reinterpret_cast<uint4*>(out + row + c) = keep[k];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kKeep; ++k) {
+                const int c = c0 + k * kStep;
+                keep[k] = c < cols ? sum8(row + c, cols - c) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+        if constexpr (KEEP == kRowNormMore)
+            for (int c = c0 + kKeep * kStep; c < cols; c += kStep) sum8(row + c, cols - c);
+        rmsnorm_kept<WIDE, KEEP == kRowNormMore>(keep, out + row, norm_w, normed + row, cols, eps);
     }
-    for (int c = c0 + kRowNormKeep * kStep; c < cols; c += kStep) sum8(row + c, cols - c);
-    rmsnorm_kept<false>(keep, out + row, norm_w, normed + row, cols, eps);
 }
 
 // Packets of the flag-in-data exchange {2 halves, epoch, 2 halves, epoch} -> contiguous fp16 (4 per packet).
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_packets_kernel(c
     }
     if (by_row) {
         __syncthreads();   // the row is complete (every thread gets here, also after a timeout)
-        rmsnorm_row<false>(out + static_cast<long>(blockIdx.x) * cols, norm_w, normed + static_cast<long>(blockIdx.x) * cols, cols, eps);
+        rmsnorm_row<false, kRowNormMore>(out + static_cast<long>(blockIdx.x) * cols, norm_w, normed + static_cast<long>(blockIdx.x) * cols, cols, eps);
     }
 }
 
@@ -375,16 +377,22 @@ void launch_exchange_sum_f16(const __half* slots, int n_slots, long slot_stride,
                    reinterpret_cast<uintptr_t>(out) % 4 == 0,
                "exchange sum: even element counts and 4-byte aligned buffers");
     if (count == 0) return;
-    long blocks = (count / 8 + 255) / 256;
-    blocks = blocks < 1 ? 1 : (blocks > 1184 ? 1184 : blocks);
+    long blocks = std::max(1L, (count / 8 + 255) / 256);
+    blocks = std::min<long>(blocks, 148 * row_ctas(0));
     if (norm_w != nullptr) {
         TQ_REQUIRE(normed != nullptr && cols > 0 && cols % 2 == 0 && count % cols == 0, "exchange sum + RMSNorm: whole rows of an even length");
         blocks = count / cols;
     }
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = pdl_config(dim3(static_cast<unsigned>(blocks)), dim3(norm_w ? kRowNormThreads : 256), stream, attr);
-    TQ_CUDA(cudaLaunchKernelEx(&cfg, norm_w != nullptr ? exchange_sum_f16_kernel<true> : exchange_sum_f16_kernel<false>, slots, n_slots, slot_stride, count,
-                               residual, out, norm_w, normed, cols, eps));
+    const bool wide = rows_wide(8, slots, residual, out) && slot_stride % 8 == 0;
+    auto* kernel = exchange_sum_f16_kernel<false, 0>;
+    if (norm_w != nullptr) {
+        TQ_ROW_KERNEL(kernel, exchange_sum_f16_kernel, wide && rows_wide(cols, norm_w, normed, nullptr), cols)
+    } else if (wide && count % 8 == 0) {
+        kernel = exchange_sum_f16_kernel<true, 0>;
+    }
+    TQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, slots, n_slots, slot_stride, count, residual, out, norm_w, normed, cols, eps));
 }
 
 void launch_exchange_unpack_packets(const uint4* packets, long n_packets, __half* out, cudaStream_t stream) {
