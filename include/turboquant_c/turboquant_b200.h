@@ -490,6 +490,11 @@ int tq_kv_attention(const tq_kv_cache_t* caches, int n_seqs, int layer, const vo
 int tq_kv_attention_lse(const tq_kv_cache_t* caches, int n_seqs, int layer, const void* queries, int q_dtype,
                         int q_heads, void* out_fp16, float* lse_out, int start, int end, int use_qjl, void* stream);
 
+/** How tq_kv_attention cuts the work of n_seqs sequences of tokens[i] tokens (from the first on) on a device of `sms` multiprocessors: *ranges pieces for
+ *  a team of warps each, and per job (sequence, KV head, up to 8 of its query heads) *parts of them, or 0: then a range is whole jobs
+ *  (*whole_jobs = 1) or an equal share of all tokens.  Needs no device. */
+int tq_kv_attention_plan(int head_dim, int q_heads, int kv_heads, int n_seqs, const int* tokens, int sms, int* ranges, int* parts, int* whole_jobs);
+
 /* ---- fp16 decode window and hybrid attention -------------------------------------------------
  * The reference keeps these in its C++ layer only (no C symbol): turboquant::DecodeBuffer
  * (include/turboquant/decode_buffer.h:11-47, src/decode_buffer.cpp) and hybrid_attention

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 TOL = 2.1e-3
 CASES = [
     # tokens of each sequence, query heads, KV heads, head size
-    ([6000], 4, 1, 32),                       # hundreds of parts of one job
+    ([6000], 4, 1, 32),                       # many parts of one job
     ([9000], 8, 1, 128),
     ([5000, 17], 2, 1, 64),
     ([1500], 3, 1, 256),

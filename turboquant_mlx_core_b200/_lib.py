@@ -137,6 +137,7 @@ def load() -> C.CDLL:
     sig("tq_kv_append_batch", i, [C.POINTER(C.c_void_p), i, i, vp, vp, i, vp])
     sig("tq_kv_attention", i, [C.POINTER(C.c_void_p), i, i, vp, i, i, vp, i, i, i, vp])
     sig("tq_kv_attention_lse", i, [C.POINTER(C.c_void_p), i, i, vp, i, i, vp, vp, i, i, i, vp])
+    sig("tq_kv_attention_plan", i, [i, i, i, i, C.POINTER(i), i, C.POINTER(i), C.POINTER(i), C.POINTER(i)])
 
     sig("tq_codebook_fit", i, [vp, C.c_long, i, i, vp, vp, C.POINTER(C.c_int), vp])
     sig("tq_fit_layer_codebooks", i, [vp, i, i, u32, i, i, i, vp, vp, vp, vp, vp])

@@ -990,6 +990,28 @@ int tq_kv_attention_lse(const tq_kv_cache_t* caches, int n_seqs, int layer, cons
     });
 }
 
+int tq_kv_attention_plan(int head_dim, int q_heads, int kv_heads, int n_seqs, const int* tokens, int sms, int* ranges, int* parts, int* whole_jobs) {
+    return guarded<int>(0, -1, [&]() {
+        TQ_REQUIRE((head_dim == 32 || head_dim == 64 || head_dim == 128 || head_dim == 256) && kv_heads >= 1 && q_heads >= 1 && q_heads % kv_heads == 0 &&
+                       n_seqs >= 1 && tokens && sms >= 1 && ranges && parts && whole_jobs,
+                   "tq_kv_attention_plan: bad sizes");
+        std::vector<tq::AttnSeq> seqs(static_cast<size_t>(n_seqs));
+        for (int i = 0; i < n_seqs; ++i) {
+            TQ_REQUIRE(tokens[i] >= 0, "tq_kv_attention_plan: negative number of tokens");
+            seqs[i].end = tokens[i];
+        }
+        long longest = 0, shortest = 0;
+        const long tiles = tq::attn_number_tiles(seqs.data(), n_seqs, &longest, &shortest);
+        TQ_REQUIRE(tiles > 0, "tq_kv_attention_plan: no tokens");
+        const long jobs_per_seq = static_cast<long>(kv_heads) * ((q_heads / kv_heads + tq::kAttnJobHeads - 1) / tq::kAttnJobHeads);
+        const tq::AttnPlan plan = tq::attn_plan(head_dim, n_seqs * jobs_per_seq, tiles * jobs_per_seq, longest, shortest, sms);
+        *ranges = plan.ranges;
+        *parts = plan.parts;
+        *whole_jobs = plan.whole_jobs;
+        return 0;
+    });
+}
+
 tq_decode_buffer_t tq_decode_buffer_create(int window_size, int num_heads, int head_dim) {
     return guarded<tq_decode_buffer_t>(nullptr, nullptr, [&]() -> tq_decode_buffer_t {
         auto* b = new turboquant::DecodeBuffer(window_size, num_heads, head_dim);

@@ -45,7 +45,8 @@ __constant__ float kC3[8] = {-2.152176f, -1.344318f, -0.756130f, -0.245379f, 0.2
 
 constexpr uint32_t kTabBytes = 256 * 128;                       // the pair table, at the start of shared memory
 constexpr float kNone = -1e30f;
-constexpr int kGroup = 8;                                       // query heads of a job
+constexpr int kGroup = kAttnJobHeads;
+constexpr int kTeamWarps = 8;
 constexpr int kMaxRanges = 320;                                 // two per SM
 constexpr int kFewParts = 6;                                    // parts of a job that its last team adds in one round trip
 constexpr unsigned long long kWaitLimitNs = 200ull * 1000 * 1000;
@@ -195,7 +196,7 @@ __device__ __forceinline__ float load_f32(uint32_t addr) {
     return v;
 }
 
-template <int D, bool QJL>
+template <int D, bool QJL, bool PARTS>
 __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __grid_constant__ AttnArgs a) {
     using C = AttnCfg<D>;
     using B = KvBlock<D>;
@@ -255,16 +256,16 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         return;
     }
     const int jobs_per_seq = a.kv_heads * a.gchunks, G = a.q_heads / a.kv_heads;
-    // where range r starts: an equal share of the flat tiles, or of the jobs, or of a job's tiles
+    // where range r starts: an equal share of the flat tiles, or of the jobs, or (PARTS) of a job's tiles
     auto range_start = [&](int r) {
-        if (!a.whole_jobs && a.parts == 0) return static_cast<int>(static_cast<long>(a.units) * r / a.ranges);
-        const int job = a.parts != 0 ? r / a.parts : static_cast<int>(static_cast<long>(a.n_seqs) * jobs_per_seq * r / a.ranges);
+        if (!PARTS && !a.whole_jobs) return static_cast<int>(static_cast<long>(a.units) * r / a.ranges);
+        const int job = PARTS ? r / a.parts : static_cast<int>(static_cast<long>(a.n_seqs) * jobs_per_seq * r / a.ranges);
         if (job >= a.n_seqs * jobs_per_seq) return a.units;
         const int seq = job / jobs_per_seq;
         const AttnSeq S = attn_seq(a.seqs, seq);
-        const int tiles = (S.end + kKvTile - 1) / kKvTile - S.start / kKvTile;
-        const int start = (S.tile0 + seq * a.pad) * jobs_per_seq + (job - seq * jobs_per_seq) * (tiles + a.pad);
-        return a.parts != 0 ? start + static_cast<int>(static_cast<long>(tiles) * (r - job * a.parts) / a.parts) : start;   // (parts: no empty tiles)
+        const int start = (S.tile0 + seq * a.pad) * jobs_per_seq + (job - seq * jobs_per_seq) * ((S.end + kKvTile - 1) / kKvTile - S.start / kKvTile + a.pad);
+        if constexpr (PARTS) return start + static_cast<int>(static_cast<long>((S.end + kKvTile - 1) / kKvTile - S.start / kKvTile) * (r - job * a.parts) / a.parts);
+        else return start;
     };
     if (a.seqs.table != nullptr) pdl_wait_release();   // the table may have been uploaded just before
     int u = range_start(range);
@@ -689,9 +690,8 @@ __global__ void __launch_bounds__(AttnCfg<D>::kThreads, 1) attn_kernel(const __g
         const bool whole = done.n_tiles == done.tiles;
         // which ranges share the job: the range of flat tile x is ((x + 1) ranges - 1) / units
         const int job_u0 = u - done.n_tiles - done.tile0;   // the job's first tile
-        const int c_first = whole ? range : a.parts != 0 ? done.job * a.parts : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
-        const int c_last = whole ? range
-                                 : a.parts != 0 ? c_first + a.parts - 1 : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
+        const int c_first = whole ? range : PARTS ? done.job * a.parts : static_cast<int>((static_cast<long>(job_u0 + 1) * a.ranges - 1) / a.units);
+        const int c_last = whole ? range : PARTS ? c_first + a.parts - 1 : static_cast<int>((static_cast<long>(job_u0 + done.tiles) * a.ranges - 1) / a.units);
         float* const my_part = a.part + static_cast<size_t>(2 * range + (done.tile0 == 0 ? 1 : 0)) * C::kPartFloats;
         auto scale_add = [](float4& x, float f0, const float4& y, float f1) {
             x.x = fmaf(x.x, f0, y.x * f1);
@@ -851,11 +851,13 @@ void launch_d(const AttnArgs& args, int grid, cudaStream_t stream) {
     static bool configured[64] = {false};   // the opt-in size is a per-device attribute
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(attn_kernel<D, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {   // both, so that neither is used for the first time in a capture
+        TQ_CUDA(cudaFuncSetAttribute(attn_kernel<D, QJL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        TQ_CUDA(cudaFuncSetAttribute(attn_kernel<D, QJL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    launch_pdl(attn_kernel<D, QJL>, dim3(static_cast<unsigned>(grid)), dim3(C::kThreads), kSmem, stream, args);
+    launch_pdl(args.parts != 0 ? attn_kernel<D, QJL, true> : attn_kernel<D, QJL, false>, dim3(static_cast<unsigned>(grid)), dim3(C::kThreads), kSmem, stream,
+               args);
 }
 
 }  // namespace
@@ -878,6 +880,88 @@ size_t attn_scratch_bytes(int dim, int sm_count) { return static_cast<size_t>(2 
 
 size_t attn_counters(int n_seqs, int q_heads, int kv_heads) {
     return static_cast<size_t>(n_seqs) * kv_heads * ((q_heads / kv_heads + kGroup - 1) / kGroup);
+}
+
+// Or each job is cut into as many parts: a range has one job, so that the parts are as long as each other, end together and are few (an
+// equal share's ranges span two jobs each, and it takes all the ranges there are).  The number of parts, 0 where the plan at hand - `ranges` of
+// jobs_per_range whole jobs, or equal shares (0) - is as good.  Times of a whole call in ns, fitted to 2000 calls of 1 to 64 sequences of 40 to
+// 100 000 tokens, alike and of very different lengths: 5 % off for parts, 9 % for whole jobs, 13 % for shares (more often too low than too high),
+// which is why the parts have to be 5 % better than whole jobs, and than shares of 256 dims.  None of those calls is more than 2 % slower for it; chosen
+// without that margin, and with costs that left out the call itself, 25 were (64 dims, 4 sequences of up to 550 tokens, 8 / 8 heads 7.8 -> 8.3 us; 32
+// dims, 8 of 2400 to 13 000 25.5 -> 29.9).
+// Before and with the parts taken, us: 128 dims, 28 / 4 heads, 1 x 1024 tokens 10.5 / 7.9, 1 x 4096 10.2 / 9.5, 1 x 8192 14.4 / 10.9, 1 x 32768 20.6 / 15.6,
+// 8 x 1024 10.7 / 9.1, 3494 and 5026 beside each other 17.3 / 10.4; 40 / 8 heads, 1 x 8192 14.8 / 11.6, 8 x 4096 23.7 / 18.8; 8 / 1 heads, 1 x 100000
+// 30.7 / 18.6; 64 dims 1 x 16384 15.0 / 12.5, 16 x 4096, 8 / 8 29.4 / 26.1; 32 dims 1 x 16384 11.7 / 9.8; 256 dims 1 x 512 19.9 / 14.6, 4 x 2048 25.2 / 18.6.
+// 16 x 32768, whose 64 jobs would be four parts each of the 4.6 that the SMs have room for, 80.3 in equal shares, 85.5 so.  A part has a tile of its job at
+// least, so a short sequence beside long ones leaves few parts, one of up to 16 tokens none.
+static int attn_parts(int head_dim, long jobs, int ranges, long jobs_per_range, long share, long units, long longest, long shortest, long most, int sm_count) {
+    struct {
+        int tile, tile_beside, second;   // a tile with one team on the SM, with two; the second team's start
+        int part, job;                   // equal shares: a part; the end of a job
+        int merge, each;                 // cut at all; for each part of a job that its last one adds (many cost more each)
+        int call;                        // what every plan has
+    } ns;
+    switch (head_dim) {
+        case 32: ns = {61, 80, 800, 5800, 4200, 2500, 40, 3900}; break;
+        case 64: ns = {98, 141, 1700, 6700, 4200, 2600, 44, 4500}; break;
+        case 256: ns = {387, 387, 0, 9400, 7400, 3000, 80, 8300}; break;
+        default: ns = {99, 147, 2650, 7200, 5000, 2450, 48, 4800}; break;
+    }
+    auto tiles_ns = [&](long tiles, long n) { return n > sm_count ? tiles * ns.tile_beside + ns.second : tiles * ns.tile; };
+    const long at_hand = jobs_per_range != 0 ? tiles_ns(jobs_per_range * longest, ranges) + (jobs_per_range - 1) * ns.job
+                                             : tiles_ns(share, ranges) + ns.part + ns.each * ranges / jobs + ns.job * share * jobs / units;
+    long best = (at_hand + ns.call) * (jobs_per_range != 0 || head_dim == 256 ? 95 : 100) / 100 - ns.call;
+    int parts = 0;
+    // (powers of two, three times them, and as many as there are SMs or ranges: a call's host time is microseconds)
+    const long most_parts = std::min(most / jobs, shortest);
+    auto consider = [&](long p) {
+        if (p < 2 || p > most_parts) return;
+        const long cost = tiles_ns(std::max<long>(kTeamWarps, (longest + p - 1) / p), jobs * p) + ns.merge + (ns.each + p / 4) * p;
+        if (cost >= best) return;
+        best = cost;
+        parts = static_cast<int>(p);
+    };
+    for (long p = 2; p <= most_parts; p *= 2) {
+        consider(p);
+        consider(p + p / 2);
+    }
+    consider(sm_count / jobs);
+    consider(most_parts);
+    return parts;
+}
+
+AttnPlan attn_plan(int head_dim, long jobs, long units, long longest, long shortest, int sm_count) {
+    // Two ranges per SM while every range has a tile per warp; fewer for short jobs, whose time is the merge of the parts.
+    const int team = kTeamWarps, teams = head_dim == 256 ? 1 : 2;
+    const long most = std::min<long>(static_cast<long>(teams) * sm_count, head_dim == 32 ? AttnCfg<32>::kMaxParts : kMaxRanges);
+    AttnPlan plan{};
+    plan.ranges = static_cast<int>(std::min<long>(most, std::max<long>(1, (units + team - 1) / team)));
+    // Or whole jobs per range.  An equal share of the tiles cuts most jobs, and the part of a job costs more than a whole one
+    // (publish, fence, count, read back); against that stand the tiles that the longest range has more, and the end of every
+    // further job of a range.  Costs in ns by head size, from calls forced both ways (28 / 4 heads unless said, cut against
+    // whole, us): 32 dims 1 x 4096 tokens 8.2 / 18.0, 8 x 2000, 32 / 8 heads 10.6 / 11.0, 32 x 1000, 32 / 8 18.3 / 14.6;
+    // 64 dims 4 x 4096, 8 / 8 heads 17.2 / 27.6, 8 x 2000, 32 / 8 17.1 / 15.9, 64 x 1000, 8 / 8 35.0 / 30.5;
+    // 128 dims 1 x 4096 10.0 / 28.5, 8 x 2000, 32 / 8 19.4 / 16.6, 64 x 1000, 8 / 8 38.6 / 33.2, 10 x 10539, 8 / 2 22.4 / 68.3;
+    // 256 dims 16 x 2048, 14 / 2 31.1 / 57.2, 32 x 1000, 32 / 8 67.7 / 64.0, 64 x 1000, 8 / 8 124 / 128.
+    struct { int tile, tile_beside, part, job; } ns;   // a tile with one team on the SM, with two; a part; the end of a job
+    switch (head_dim) {
+        case 32: ns = {66, 143, 4000, 6000}; break;
+        case 64: ns = {100, 165, 7000, 6000}; break;
+        case 256: ns = {400, 400, 9000, 8000}; break;
+        default: ns = {100, 190, 10000, 6000}; break;
+    }
+    const long jobs_per_range = (jobs + most - 1) / most, job_ranges = (jobs + jobs_per_range - 1) / jobs_per_range;
+    auto tile_ns = [&](long ranges) { return static_cast<long>(ranges > sm_count ? ns.tile_beside : ns.tile); };
+    const long share = (units + plan.ranges - 1) / plan.ranges;
+    plan.whole_jobs = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * ns.job <=
+                   share * tile_ns(plan.ranges) + ns.part + ns.job * share * jobs / units;
+    if (plan.whole_jobs) plan.ranges = static_cast<int>(job_ranges);
+    plan.parts = attn_parts(head_dim, jobs, plan.ranges, plan.whole_jobs ? jobs_per_range : 0, share, units, longest, shortest, most, sm_count);
+    if (plan.parts != 0) {
+        plan.whole_jobs = 0;
+        plan.ranges = static_cast<int>(jobs * plan.parts);
+    }
+    return plan;
 }
 
 void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, long shortest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
@@ -910,67 +994,10 @@ void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long long
     a.score_scale = static_cast<float>(1.4426950408889634 / d / kAttnCentroidScale);
     // of the rotated query: the residual's reconstruction, in units of the scaled centroids
     a.qscale = static_cast<float>(std::sqrt(2.0 / (3.14159265358979323846 * d)) * kAttnCentroidScale);
-    // Two ranges per SM while every range has a tile per warp; fewer for short jobs, whose time is the merge of the parts.
-    const int team = 8, teams = head_dim == 256 ? 1 : 2;
-    const long most = std::min<long>(static_cast<long>(teams) * sm_count, head_dim == 32 ? AttnCfg<32>::kMaxParts : kMaxRanges);
-    a.ranges = static_cast<int>(std::min<long>(most, std::max<long>(1, (units + team - 1) / team)));
-    // Or whole jobs per range.  An equal share of the tiles cuts most jobs, and the part of a job costs more than a whole one
-    // (publish, fence, count, read back); against that stand the tiles that the longest range has more, and the end of every
-    // further job of a range.  Costs in ns by head size, from calls forced both ways (28 / 4 heads unless said, cut against
-    // whole, us): 32 dims 1 x 4096 tokens 8.2 / 18.0, 8 x 2000, 32 / 8 heads 10.6 / 11.0, 32 x 1000, 32 / 8 18.3 / 14.6;
-    // 64 dims 4 x 4096, 8 / 8 heads 17.2 / 27.6, 8 x 2000, 32 / 8 17.1 / 15.9, 64 x 1000, 8 / 8 35.0 / 30.5;
-    // 128 dims 1 x 4096 10.0 / 28.5, 8 x 2000, 32 / 8 19.4 / 16.6, 64 x 1000, 8 / 8 38.6 / 33.2, 10 x 10539, 8 / 2 22.4 / 68.3;
-    // 256 dims 16 x 2048, 14 / 2 31.1 / 57.2, 32 x 1000, 32 / 8 67.7 / 64.0, 64 x 1000, 8 / 8 124 / 128.
-    // Or, few jobs, each in as many parts: a range has one job, so that the parts are as long as each other, end together and are few
-    // (an equal share's ranges span two jobs each, and it takes all the ranges there are).  With one team an SM a tile takes half as
-    // long, so one part an SM is often the best.  Equal shares or whole jobs against as many parts as the rule takes, us: 128 dims,
-    // 28 / 4 heads, 1 x 1024 tokens 10.5 / 7.9, 1 x 4096 10.2 / 9.5, 1 x 8192 14.4 / 10.9, 1 x 32768 20.6 / 15.6, 8 x 1024 10.7 / 9.1; 40 / 8
-    // heads, 1 x 8192 14.8 / 11.6, 8 x 4096 23.7 / 18.8; 8 / 1 heads, 1 x 100000 30.7 / 18.6; 64 dims 1 x 16384 15.0 / 12.5, 16 x 4096, 8 / 8
-    // 29.4 / 26.1; 32 dims 1 x 16384 11.7 / 9.8; 256 dims 1 x 512 19.9 / 14.6, 4 x 2048 25.2 / 18.6.  16 x 32768, whose 64 jobs would be four
-    // parts each of the 4.6 that the SMs have room for, 80.3 in equal shares, 85.5 so.
-    struct {
-        int tile, tile_beside;   // a tile with one team on the SM, with two
-        int part, job;           // equal shares: a part; the end of a job
-        int merge, each;         // equal parts: cut at all; for each part of a job that its last one adds (many cost more each)
-    } ns;
-    switch (head_dim) {
-        case 32: ns = {66, 143, 4000, 6000, 2000, 40}; break;
-        case 64: ns = {100, 155, 7000, 6000, 2300, 44}; break;
-        case 256: ns = {400, 400, 9000, 8000, 3500, 75}; break;
-        default: ns = {100, 176, 10000, 6000, 2500, 48}; break;
-    }
-    constexpr long kSecondTeam = 1000;   // the start of a second team beside the first
-    const long jobs = static_cast<long>(n_seqs) * kv_heads * a.gchunks;
-    const long jobs_per_range = (jobs + most - 1) / most, job_ranges = (jobs + jobs_per_range - 1) / jobs_per_range;
-    auto tile_ns = [&](long ranges) { return static_cast<long>(ranges > sm_count ? ns.tile_beside : ns.tile); };
-    const long share = (units + a.ranges - 1) / a.ranges;
-    const long whole_ns = jobs_per_range * longest * tile_ns(job_ranges) + (jobs_per_range - 1) * ns.job;
-    const long share_ns = share * tile_ns(a.ranges) + ns.part + ns.each * a.ranges / jobs + ns.job * share * jobs / units;
-    a.whole_jobs = whole_ns <= share_ns;
-    a.parts = 0;
-    long best = std::min(whole_ns, share_ns);
-    // (powers of two, three times them, and as many as there are SMs or ranges: a call's host time is microseconds)
-    const long most_parts = std::min(most / jobs, shortest);   // (a part has a tile of every job)
-    auto consider = [&](long p) {
-        if (p < 2 || p > most_parts) return;
-        const long ranges = jobs * p, part = std::max<long>(team, (longest + p - 1) / p);
-        const long cost = part * tile_ns(ranges) + ns.merge + (ns.each + p / 4) * p + (ranges > sm_count ? kSecondTeam : 0);
-        if (cost >= best) return;
-        best = cost;
-        a.parts = static_cast<int>(p);
-    };
-    for (long p = 2; p <= most_parts; p *= 2) {
-        consider(p);
-        consider(p + p / 2);
-    }
-    consider(sm_count / jobs);
-    consider(most_parts);
-    if (a.parts != 0) {
-        a.whole_jobs = 0;
-        a.ranges = static_cast<int>(jobs * a.parts);
-    } else if (a.whole_jobs) {
-        a.ranges = static_cast<int>(job_ranges);
-    }
+    const AttnPlan plan = attn_plan(head_dim, static_cast<long>(n_seqs) * kv_heads * a.gchunks, units, longest, shortest, sm_count);
+    a.ranges = plan.ranges;
+    a.parts = plan.parts;
+    a.whole_jobs = plan.whole_jobs;
     // 32: five rounds of the team's warps, about 6 us; less where ranges are short and every job ends in several of them
     a.pad = a.parts != 0 ? 0 : static_cast<int>(std::min<long>(32, units / a.ranges / 8));
     units += static_cast<long>(n_seqs) * kv_heads * a.gchunks * a.pad;

@@ -112,6 +112,13 @@ constexpr float kAttnSoftmaxSlack = 2.0f;
 
 // Sets the descriptors' tile0 and returns the tiles of all sequences; `longest`, `shortest`: of the longest, of the shortest.
 long attn_number_tiles(AttnSeq* seqs, int n_seqs, long* longest, long* shortest);
+// How the work is cut: a team's tiles are a range.  parts != 0: each job (sequence, KV head, 8 query heads) is so many ranges; whole_jobs: a range is
+// whole jobs; otherwise all ranges have an equal share of the tiles.  units: the tiles of all jobs.
+struct AttnPlan {
+    int ranges, parts, whole_jobs;
+};
+AttnPlan attn_plan(int head_dim, long jobs, long units, long longest, long shortest, int sm_count);
+constexpr int kAttnJobHeads = 8;
 size_t attn_scratch_bytes(int dim, int sm_count);
 size_t attn_counters(int n_seqs, int q_heads, int kv_heads);   // zeroed words; every launch leaves them zero
 void launch_kv_attention(const AttnSeqs& seqs, int n_seqs, long tiles, long longest, long shortest, const void* q, bool q_is_f16, int q_heads, int kv_heads, int head_dim,
