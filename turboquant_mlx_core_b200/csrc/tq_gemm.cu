@@ -37,10 +37,10 @@
 //              tile's first MMA waits until this one is read)
 // A CTA per SM walks the output tiles (of a single matrix; a group's matrices have a CTA per tile) and its ring of stages runs on from tile to tile: with a CTA per
 // tile, set-up, first loads and epilogue took 8 to 18 of 47 thousand cycles (5120 x 55296: 89 -> 76 us at
-// 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the shared-memory pipe bounds it: 256 cycles of lookups and 64 of code loads
-// per 128 x 64 weights, 32 to 128 more for the activation tile, of the 400 to 450 that they take; at 16 rows that is 86 % of what the
-// memory delivers.  At 256 it is the same pipe: lookups, code loads, the activation tile's write and its read.  What a call costs besides
-// its stages is some 8 us: the rotation in front and its end, the CTA's set-up, the first codes, the epilogue.
+// 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the producers bound it: some 420 cycles per 128 x 64 weights, of which the shared-memory
+// pipe is taken for 320 (256 of lookups, 64 of code loads) and 32 to 128 more by the activation tile; it is busy for 63 % of a launch at 32 rows.  At
+// 16 rows that is 86 % of what the memory delivers.  At 256 it is that pipe: lookups, code loads, the activation tile's write and its read.  What a call
+// costs besides its stages is some 8 us: the rotation in front and its end, the CTA's set-up, the first codes, the epilogue.
 // The activation tile is as tall as the rows it really has (in steps of 16): a decode batch of 9..64
 // rows costs a short MMA and a short copy, so the codes are streamed once whatever the batch.
 // The dequantised weights never touch HBM; a weight tile is looked up once per 256 activation
@@ -75,7 +75,6 @@ constexpr int kProducerWarps = 8 * kGroups;
 constexpr int kProducerThreads = kProducerWarps * 32;
 constexpr int kMmaWarp = kProducerWarps;       // issues the MMAs, owns the tensor-memory allocation
 constexpr int kCopyWarp = kProducerWarps + 1;  // issues the activation-tile bulk copies
-constexpr int kEpilogueWarp = kProducerWarps + 2;  // first of four warps that drain the accumulators
 constexpr int kEpilogueWarps = 4;
 constexpr int kGemmThreads = kProducerThreads + 64 + 32 * kEpilogueWarps;
 constexpr uint32_t kLutBytes = 256 * 32 * 4;           // 256 entries x 32 lane copies x two fp16
@@ -387,7 +386,7 @@ __device__ __forceinline__ void rotate_rows_wide(const __half* __restrict__ x, _
 }
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
-                                                                   int in, long rows, int n_planes, int block,
+                                                                   int in, long rows, int block,
                                                                    uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
     rotate_rows_wide<CHUNKS>(x, xrot, in, rows, block, seed_p, seed_r, inv_sqrt, row_steps);
 }
@@ -398,7 +397,7 @@ struct RotateGroupArgs {
 };
 template <int CHUNKS>
 __global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
-                                                                         long rows, int n_planes, int block, float inv_sqrt, int row_steps) {
+                                                                         long rows, int block, float inv_sqrt, int row_steps) {
     rotate_rows_wide<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
 }
 
@@ -528,7 +527,6 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         const uint8_t* const code_lane = p.codes + (lane >> 2) * 64 + 16 * (lane & 3);
         const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3) + (DUAL ? 16 * sub : 0)) << 16) + kTmemAColumn +
                                  (DUAL ? 0u : kTmemASubCols * static_cast<uint32_t>(sub));
-        const int n_stages = n_local * n_it;
 
         // The group's next stage to fetch: its place in its tile, where its codes are, stages left.
         const int full_it = n_it - ((!DUAL && sub != 0 && (n_kb & 1)) ? 1 : 0);   // stages of a tile that have a block for this warp
@@ -931,8 +929,8 @@ void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int 
         if (ctas < (1L << 31)) {
             const dim3 grid(static_cast<unsigned int>(ctas), static_cast<unsigned int>(n));
 #define TQ_ROTATE_WIDE(CHUNKS)                                                                                                                         \
-    if (n == 1) launch_pdl(rotate_rows_f16_wide_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot.xrot[0], in, m, n_planes, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
-    else launch_pdl(rotate_rows_f16_wide_group_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot, in, m, n_planes, bs, inv_sqrt, row_steps);
+    if (n == 1) launch_pdl(rotate_rows_f16_wide_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot.xrot[0], in, m, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
+    else launch_pdl(rotate_rows_f16_wide_group_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot, in, m, bs, inv_sqrt, row_steps);
             switch (cols) {
                 case 256: TQ_ROTATE_WIDE(1) break;
                 case 512: TQ_ROTATE_WIDE(2) break;

@@ -68,7 +68,6 @@ namespace {
 constexpr int kWarps = 16;
 constexpr int kThreads = kWarps * 32;
 constexpr int kSlice = 256;               // columns per warp
-constexpr int kChunk = kWarps * kSlice;   // widest chunk: columns one unit covers with all 16 warps on one row tile
 constexpr uint32_t kLutAddr = 0x10000u;   // shared-window address of the table
 constexpr uint32_t kLutBytes = 0x10000u;  // 256 entries * 256 B
 // Partial-sum ring: ring * 16 warps * (16 rows * bp + 4) floats.  Eight rows take three slots of 32 KB, which tied the warps to each
@@ -352,7 +351,6 @@ __device__ __forceinline__ void store_y(const GemvArgs& p, const ScatterArgs& sc
 // streaming read drops from 5.8 to 3.4 TB/s when a CTA holds 216 KB), so the codes are never
 // staged through shared memory: they go from HBM straight into registers.
 constexpr size_t kGemvSmem = kLutAddr + kLutBytes;  // dynamic bytes requested (window end)
-constexpr int kConsumerThreads = kThreads;
 constexpr int kCtaThreads = kThreads;
 constexpr unsigned long long kWaitLimitNs = 200ull * 1000 * 1000;  // bounded waits: give up after 0.2 s and flag it
 
