@@ -337,9 +337,10 @@ __global__ void __launch_bounds__(256) fit_sums_kernel(const float* __restrict__
 // All iterations of a fit in one CTA, a CTA per fit: warp w follows boundary w, the upper one of bin w.  Bound by the latency of a
 // chain of L2 reads, reductions and barriers: a bucket's place, its values, the sums around it and between the boundaries are a few
 // hundred to 2000 cycles each.  Long buckets are read 16 values a lane at a time (eight: six such reads one after the other for 1500
-// values; 24 slow those down whose boundaries lie in small buckets), the rest and small buckets eight, which issues less.  100 iterations of a layer's two fits over 16.8 M samples each, side by side,
-// 497 us (eight at a time throughout 555; 24 470).  (Significands as 64-bit sums of doubles' conversions took 400 to 660 us; the bits
-// below a bucket's prefix are 32-bit sums.  Two warps per boundary that keep their bucket's samples in registers: no change.)
+// values; 24 slow those down whose boundaries lie in small buckets), the rest and small buckets eight, which issues less.  100 iterations of a
+// layer's two fits over 16.8 M samples each, side by side, 497 us (eight at a time throughout 555; 24 470); samples over 60 decades, whose boundaries lie in
+// small buckets, cost 2 % more for it, 4 M of them 453 -> 463 us a fit.  (Significands as 64-bit sums of doubles' conversions took 400 to 660 us;
+// the bits below a bucket's prefix are 32-bit sums.  Two warps per boundary that keep their bucket's samples in registers: no change.)
 // `group_sum`: filled here from the parts.
 struct FitJob {
     const float* sorted;
