@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256) ring_write_kernel(const InT* __restrict__
                                                          long src_token0, int row, int window, long slot0, __half* __restrict__ ring_k,
                                                          __half* __restrict__ ring_v) {
     pdl_wait_release();
+    behind_wait(src_k, src_v);
     // token t of the source (counted from src_token0) goes to slot (slot0 + t) % window; `row` = heads * dim
     const long total = n_tokens * row;
     for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __
                                                                 int n_splits, float scale, float* __restrict__ part_acc,
                                                                 float* __restrict__ part_ml) {
     pdl_wait_release();
+    behind_wait(keys, values, q);
     constexpr int D = 128;
     __shared__ __half s_q[8][D + 8];
     __shared__ float s_m[4][8], s_l[4][8];
@@ -318,13 +320,13 @@ __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __
         uint4 fka[4], fkb[4], fva[4], fvb[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            fka[j] = __ldg(ka + 4 * j);
-            fkb[j] = __ldg(kb + 4 * j);
+            fka[j] = ka[4 * j];
+            fkb[j] = kb[4 * j];
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            fva[j] = __ldg(xa + 4 * j);
-            fvb[j] = __ldg(xb + 4 * j);
+            fva[j] = xa[4 * j];
+            fvb[j] = xb[4 * j];
         }
         float c1[4] = {0.f, 0.f, 0.f, 0.f}, c1b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -427,6 +429,7 @@ __global__ void __launch_bounds__(kCombineThreads) dense_combine_kernel(const fl
     __shared__ float s_m[kCombineThreads / 32], s_l[kCombineThreads / 32];
     __shared__ __align__(16) float4 s_sum[kRows][kLanes];
     pdl_wait_release();
+    behind_wait(part_acc, part_ml);
     const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float2 ml = tid < n_splits ? *reinterpret_cast<const float2*>(part_ml + (static_cast<size_t>(h) * n_splits + tid) * 2)
                                      : make_float2(-INFINITY, 0.f);

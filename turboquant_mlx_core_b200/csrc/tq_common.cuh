@@ -188,6 +188,14 @@ __device__ __forceinline__ void pdl_wait_release() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
 }
+// Pointers to what kernels in front write, taken up behind the wait.  A load through a const __restrict__ pointer, and any __ldg, is one of memory that
+// nothing writes while the kernel runs: the compiler may carry it out in front of the wait, and did (the rotation of blocks of 512 read its
+// activation before the kernel in front had written it).  A pointer that comes out of here is nothing the compiler knows, from a place that it does
+// not move: plain loads through it stay behind.
+template <typename... Pointer>
+__device__ __forceinline__ void behind_wait(Pointer&... p) {
+    (..., [&] { asm volatile("" : "+l"(p)::"memory"); }());
+}
 template <typename Kernel, typename... Args>
 inline void launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchAttribute attr[1];

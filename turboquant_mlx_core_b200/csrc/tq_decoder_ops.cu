@@ -24,6 +24,7 @@ template <bool WIDE, int KEEP>
 __global__ void __launch_bounds__(kRowNormThreads, row_ctas(KEEP)) rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
                                                       int cols, float eps) {
     ops_dependency_sync();
+    behind_wait(x, w);
     rmsnorm_row<WIDE, KEEP>(x + static_cast<size_t>(blockIdx.x) * cols, w, y + static_cast<size_t>(blockIdx.x) * cols, cols, eps);
 }
 
@@ -33,6 +34,7 @@ __global__ void __launch_bounds__(kRowNormThreads, row_ctas(KEEP)) rmsnorm_kerne
 __global__ void __launch_bounds__(128) rope_kernel(__half* __restrict__ x, const int* __restrict__ positions, int heads, int dim,
                                                    float log2_theta, long total_pairs, __half* __restrict__ x2, int heads2, long total_pairs2) {
     ops_dependency_sync();
+    behind_wait(x, positions, x2);
     const int half = dim >> 1;
     for (long i0 = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < total_pairs + total_pairs2;
          i0 += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -60,6 +62,7 @@ constexpr int kRopeThreads = 256, kRopeHalfMax = 256;
 __global__ void __launch_bounds__(kRopeThreads) rope_rows_kernel(__half* __restrict__ x, const int* __restrict__ positions, int heads, int dim,
                                                                  float log2_theta, __half* __restrict__ x2, int heads2) {
     ops_dependency_sync();
+    behind_wait(x, positions, x2);
     __shared__ __align__(16) float s_cos[kRopeHalfMax], s_sin[kRopeHalfMax];
     const int half = dim >> 1, per_head = half / 8, items = (heads + heads2) * per_head;
     const long row = blockIdx.x;
@@ -91,6 +94,7 @@ __device__ __forceinline__ float swiglu(float g, float u) { return g / (1.0f + _
 // two per thread and a 64-bit division for each pair).
 __global__ void __launch_bounds__(256) swiglu_wide_kernel(const __half* __restrict__ gate_up, __half* __restrict__ act, int inter, long rows) {
     ops_dependency_sync();
+    behind_wait(gate_up);
     const int j = (blockIdx.x * 256 + threadIdx.x) * 8;
     if (j >= inter) return;
     for (long r = blockIdx.y; r < rows; r += gridDim.y) {
@@ -105,6 +109,7 @@ __global__ void __launch_bounds__(256) swiglu_wide_kernel(const __half* __restri
 }
 __global__ void __launch_bounds__(256) swiglu_kernel(const __half* __restrict__ gate_up, __half* __restrict__ act, int inter, long rows) {
     ops_dependency_sync();
+    behind_wait(gate_up);
     const long total = rows * inter;
     for (long i = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2; i < total; i += static_cast<long>(gridDim.x) * blockDim.x * 2) {
         const long r = i / inter, j = i - r * inter;

@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
     const long rem = warp - static_cast<long>(plane) * rows * blocks_per_row;
     const long blk = rem / rows, row = rem - blk * rows;
     const uint32_t seed = plane ? seed_r : seed_p;
+    behind_wait(x);
     const __half* src = x + row * in + blk * BS + lane * E;
     float v[E];
 #pragma unroll
@@ -307,12 +308,13 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
     };
     __half* dst = place(first);
     if (!wait_first) pdl_wait_release();
+    behind_wait(src);
     // a row's loads are on their way while the one before it is worked on (not of blocks of 1024, which fill the registers)
     constexpr bool kAhead = CHUNKS <= 2;
     uint4 next[CHUNKS];
     auto load = [&](const __half* from, bool there) {
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) next[c] = there ? __ldg(reinterpret_cast<const uint4*>(from + 256 * c)) : make_uint4(0, 0, 0, 0);
+        for (int c = 0; c < CHUNKS; ++c) next[c] = there ? *reinterpret_cast<const uint4*>(from + 256 * c) : make_uint4(0, 0, 0, 0);
     };
     if (kAhead) load(src, have && first + wib < rows);
     for (int row8 = first; row8 < last; row8 += 8) {

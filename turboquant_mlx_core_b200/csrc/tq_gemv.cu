@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(128) rotate_x_kernel(const __half* __restrict_
     const int rem = warp - plane * batch * blocks_per_row;
     const int row = rem / blocks_per_row, blk = rem - row * blocks_per_row;
     const uint32_t seed = plane ? seed_r : seed_p;
+    behind_wait(x);
     const __half* src = x + static_cast<size_t>(row) * in + blk * BS + lane * E;
     float v[E];
 #pragma unroll
@@ -156,15 +157,16 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     const unsigned live = __ballot_sync(0xffffffffu, col < in);   // the lanes that exchange values
     if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
     const uint32_t seed = plane ? seed_r : seed_p;
-    const __half* const src = x + static_cast<size_t>(row) * in + col;
     // The signs of one chunk in front of the wait: 4096 x 4096 at eight rows 9.9 -> 9.6 us with the product.  Those of two or four take longer than
     // the loads, behind which they are made: in front, 4096 x 4096, block 512, took 8.8 us at one row instead of 8.3, 1024 x 1024 6.4 instead of 5.9.
     uint4 signs;
     if (CHUNKS == 1) signs = chunk_signs(seed, static_cast<uint32_t>(col), block);
     grid_dependency_sync();
+    behind_wait(x);
+    const __half* const src = x + static_cast<size_t>(row) * in + col;
     uint4 raw[CHUNKS];
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
+    for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
     float v[CHUNKS][8];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
@@ -210,18 +212,19 @@ __global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __rest
     const int row = warp / groups_per_row, col = (warp - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
     const unsigned live = __ballot_sync(0xffffffffu, col < in);   // the lanes that exchange values
     if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
+    behind_wait(x);
     const __half* const src = x + static_cast<size_t>(row) * in + col;
     uint4 raw[CHUNKS];
     if (aligned) {
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) raw[c] = __ldg(reinterpret_cast<const uint4*>(src + 256 * c));
+        for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
     } else {
         const unsigned short* const h = reinterpret_cast<const unsigned short*>(src);
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
             uint32_t w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = __ldg(h + 256 * c + 2 * j) | (static_cast<uint32_t>(__ldg(h + 256 * c + 2 * j + 1)) << 16);
+            for (int j = 0; j < 4; ++j) w[j] = h[256 * c + 2 * j] | (static_cast<uint32_t>(h[256 * c + 2 * j + 1]) << 16);
             raw[c] = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
@@ -466,7 +469,7 @@ template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false
 __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk, const __half* row = nullptr) {
     auto load_x = [&](int col) {   // eight columns of the row that is rotated in here
         if constexpr (ROW) return *reinterpret_cast<const uint4*>(row + col);
-        else return __ldg(reinterpret_cast<const uint4*>(p.x + col));
+        else return *reinterpret_cast<const uint4*>(p.x + col);   // (no __ldg: it must stay behind the wait)
     };
     // columns per chunk, derived here: one more field in GemvArgs made ptxas spill within the 128 registers
     const int chunk_cols = p.wpt * kSlice;

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(NW * 32, StagedCfg<NW>::kMinBlocks) tq8_gemv_s
                 }
             } else {
                 uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-                if (col < p.in) raw = __ldg(reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(n) * p.in + col));
+                if (col < p.in) raw = *reinterpret_cast<const uint4*>(p.x + static_cast<size_t>(n) * p.in + col);   // (no __ldg: it must stay behind the wait)
                 const uint32_t xw[4] = {raw.x, raw.y, raw.z, raw.w};
                 float v[8];
 #pragma unroll

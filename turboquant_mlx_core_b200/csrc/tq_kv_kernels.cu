@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 7 : (D == 256 ? 3 : 2)) kv_enc
     }
     __syncthreads();
     pdl_wait_release();
+    behind_wait(keys, values);
 
     const int lane = threadIdx.x & 31, q = lane & 3;
     const bool odd = (lane & 4) != 0;
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 7 : (D == 256 ? 3 : 2)) kv_enc
     for (int i = 0; i < N / kPer; ++i) {
         uint4 raw;
         if (aligned) {
-            raw = __ldg(reinterpret_cast<const uint4*>(src) + i);
+            raw = reinterpret_cast<const uint4*>(src)[i];
         } else {
             InT* const e = reinterpret_cast<InT*>(&raw);
 #pragma unroll
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(64) kv_encode_few_kernel(const InT* __restrict
     const int token = ((first >> 1) + pair) * 2 + (odd ? 1 : 0), tok = token - first;   // absolute, and within the call
     const bool live = in_range && tok >= 0 && tok < tokens;
     const int src_tok = tok < 0 ? 0 : (tok < tokens ? tok : tokens - 1);
-    const InT* const src = (value ? values : keys) + ((static_cast<size_t>(sidx) * tokens + src_tok) * heads + head) * D + l * 8;
+    const InT* src = (value ? values : keys) + ((static_cast<size_t>(sidx) * tokens + src_tok) * heads + head) * D + l * 8;
     uint32_t flips = 0, qflips = 0;   // bit j: dim j's rotation sign, its residual sign (set = +1)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -397,13 +398,14 @@ __global__ void __launch_bounds__(64) kv_encode_few_kernel(const InT* __restrict
         qflips |= qjl_sign_is_positive(qjl_seed, static_cast<uint32_t>(l * 8 + j)) ? 1u << j : 0u;
     }
     pdl_wait_release();
+    behind_wait(src);
 
     float v[8];
     if (aligned) {
         constexpr int kPer = 16 / static_cast<int>(sizeof(InT));
 #pragma unroll
         for (int i = 0; i < 8 / kPer; ++i) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + i);
+            const uint4 raw = reinterpret_cast<const uint4*>(src)[i];
             const InT* e = reinterpret_cast<const InT*>(&raw);
 #pragma unroll
             for (int j = 0; j < kPer; ++j) v[i * kPer + j] = as_f32<InT>(e[j]);
@@ -530,6 +532,7 @@ __global__ void __launch_bounds__(128) kv_decode_kernel(const unsigned char* __r
     }
     __syncthreads();
     pdl_wait_release();
+    behind_wait(base);
     const int lane = threadIdx.x & 31, q = lane & 3;
     const long quad = (static_cast<long>(blockIdx.x) * 128 + threadIdx.x) >> 2;
     const bool live = quad < n_vec;

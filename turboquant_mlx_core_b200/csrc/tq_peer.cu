@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kRowNormThreads, row_ctas(KEEP)) exchange_sum_
                                                                float eps) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    behind_wait(slots, residual, norm_w);
     // the sum of (up to) eight elements from i on, rounded and stored
     auto sum8 = [&](long i, int n) {
         float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, h[8];
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_packets_kernel(c
                                                                    float eps) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    behind_wait(local, residual, norm_w);
     const unsigned int want = *reinterpret_cast<const volatile unsigned int*>(epoch);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wait_epoch, 1u);
     const uint4* const half = base + static_cast<size_t>(want & 1u) * world * packets;
@@ -300,6 +302,7 @@ __global__ void __launch_bounds__(128) exchange_merge_attention_kernel(const __h
                                                                        long part_stride_l, __half* __restrict__ out) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    behind_wait(outs, lses);
     const long row = blockIdx.x;
     if (row >= rows) return;
     float m = -INFINITY;
