@@ -196,19 +196,27 @@ template <typename... Pointer>
 __device__ __forceinline__ void behind_wait(Pointer&... p) {
     (..., [&] { asm volatile("" : "+l"(p)::"memory"); }());
 }
+// `carveout`: how much of the SM's memory is to be shared memory while this kernel runs, in percent (0: the driver's choice).  An SM has one division at a
+// time and changes it only when it is empty: kernels that are to overlap ask for the same one.
 template <typename Kernel, typename... Args>
-inline void launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchAttribute attr[1];
+inline void launch_pdl_carved(Kernel kernel, dim3 grid, dim3 block, size_t smem, int carveout, cudaStream_t stream, Args... args) {
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = static_cast<unsigned int>(carveout);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = carveout > 0 ? 2 : 1;
     TQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+template <typename Kernel, typename... Args>
+inline void launch_pdl(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    launch_pdl_carved(kernel, grid, block, smem, 0, stream, args...);
 }
 
 // Up to 8 halves (n, even, at least 4-byte aligned) from or to memory, 16 bytes at once where they are all there and aligned;

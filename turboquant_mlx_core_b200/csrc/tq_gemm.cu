@@ -16,7 +16,7 @@
 //   D[128 x 256] (TMEM, fp32) += A[128 x 64] (weights, fp16, TMEM) . B[256 x 64]^T (xrot, fp16, smem)
 // per 64-column K block, as four tcgen05.mma (M 128, N 256, K 16) issued by one thread.
 //   A pipeline stage is 128 K columns (two 64-column K blocks), the ring has up to four stages.
-//   warps 0-23 producers in three groups of eight; group g takes the stages g, g + 3, ...: codes HBM ->
+//   warps 0-23 producers in three groups of eight (or two, or one, see gemm_groups); group g takes the stages g, g + 3, ...: codes HBM ->
 //              registers (the group's next stage, as the present one's are used up) -> lookup (lane-private fp16 table in
 //              shared memory) -> weight tile in TENSOR memory (tcgen05.st, 64 columns of fp16 pairs per
 //              stage).  The store's 16x256b shape takes registers in the fragment order (lane / 4 = row,
@@ -32,15 +32,16 @@
 //              elected lane issues its eight MMAs and commits to the stage's "empty" barrier.  This serial
 //              chain (wait, fence, issue, commit) bounds the kernel when the MMAs are short, hence few and
 //              long stages.
-//   warps 26-29 epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
+//   warps 26-29 (three groups) epilogue: tcgen05.ld the accumulator, scale by norm * inv_scale, store fp16, beside the
 //              next tile's products (up to 128 activation rows: two accumulators in turn; above, the next
-//              tile's first MMA waits until this one is read)
+//              tile's first MMA waits until this one is read).  A CTA of one or two groups has one tile: its producers drain it, 32 rows each
 // A CTA per SM walks the output tiles (of a single matrix; a group's matrices have a CTA per tile) and its ring of stages runs on from tile to tile: with a CTA per
 // tile, set-up, first loads and epilogue took 8 to 18 of 47 thousand cycles (5120 x 55296: 89 -> 76 us at
 // 32 rows, 544 -> 464 us at 1024).  Up to 64 rows the producers bound it: some 420 cycles per 128 x 64 weights, of which the shared-memory
 // pipe is taken for 320 (256 of lookups, 64 of code loads) and 32 to 128 more by the activation tile; it is busy for 63 % of a launch at 32 rows.  At
 // 16 rows that is 86 % of what the memory delivers.  At 256 it is that pipe: lookups, code loads, the activation tile's write and its read.  What a call
-// costs besides its stages is some 8 us: the rotation in front and its end, the CTA's set-up, the first codes, the epilogue.
+// costs besides its stages is some 6 us where the next kernel's CTAs are set up beside the last one's (gemm_groups), 8 us otherwise: two or three waits of 1.1 us
+// for the end of the kernel in front, the rotation, the first activation tile, the epilogue, the split sums.
 // The activation tile is as tall as the rows it really has (in steps of 16): a decode batch of 9..64
 // rows costs a short MMA and a short copy, so the codes are streamed once whatever the batch.
 // The dequantised weights never touch HBM; a weight tile is looked up once per 256 activation
@@ -70,24 +71,48 @@ constexpr int kTileTok = 256;   // activation rows per CTA (MMA N)
 constexpr int kBlockK = 64;     // columns of a K block
 constexpr int kSubPerStage = 2; // K blocks per pipeline stage: a stage is 128 K columns
 constexpr int kStagesMax = 4;   // ring of stages: weight tiles in tensor memory (4 x 64 columns), activation tiles in shared memory (as many as fit)
-constexpr int kGroups = 3;      // producer groups of eight warps: group g dequantises the stages g, g + 3, ...
-constexpr int kProducerWarps = 8 * kGroups;
-constexpr int kProducerThreads = kProducerWarps * 32;
-constexpr int kMmaWarp = kProducerWarps;       // issues the MMAs, owns the tensor-memory allocation
-constexpr int kCopyWarp = kProducerWarps + 1;  // issues the activation-tile bulk copies
+constexpr int kGroupsMax = 3;   // producer groups of eight warps: group g dequantises the stages g, g + groups, ...
 constexpr int kEpilogueWarps = 4;
-constexpr int kGemmThreads = kProducerThreads + 64 + 32 * kEpilogueWarps;
+// With three groups four more warps drain the accumulators beside the next tile's products; a CTA of one or two groups has one tile, which its producers
+// drain when they are through with it.
+__host__ __device__ constexpr int gemm_threads(int groups) { return groups * 256 + 64 + (groups == kGroupsMax ? 32 * kEpilogueWarps : 0); }
 constexpr uint32_t kLutBytes = 256 * 32 * 4;           // 256 entries x 32 lane copies x two fp16
 constexpr uint32_t kTmemCols = 512;   // accumulators: columns 0..255 (two of up to 128 columns, or one); weight tiles: 4 stages x 64 columns from 256 on
 constexpr uint32_t kTmemAColumn = 256;
 constexpr uint32_t kTmemASubCols = kBlockK / 2;                    // one K block: two fp16 per 32-bit column
 constexpr uint32_t kTmemAStageCols = kSubPerStage * kTmemASubCols;
+// One group: 256 columns, so that two CTAs share an SM: an accumulator of 64 or 128 columns, the rest weight tiles (three stages or two).
+__host__ __device__ constexpr uint32_t one_group_a_column(uint32_t rows) { return rows <= 64 ? 64 : 128; }
+__host__ __device__ constexpr uint32_t one_group_stages(uint32_t rows) { return (256 - one_group_a_column(rows)) / kTmemAStageCols; }
 constexpr uint32_t kLutWin = 0x800u;  // window address of the lookup tables (an immediate of the lookup's load)
 // Everything an SM can give one CTA: tables at kLutWin, then three 64 KB stages for a 256-row tile.
 constexpr size_t kGemmSmemBytes = 232448 - 512;
 // What a launch of m activation rows needs of it (an SM is set up faster for less: 3584 x 37888 at 16 rows 32.9 us with all of it, 32.4 so).
-size_t gemm_smem_bytes(long m) {
-    return std::min(kGemmSmemBytes, kLutWin + kLutBytes + kStagesMax * kSubPerStage * static_cast<size_t>(std::min<long>(kTileTok, (m + 15) / 16 * 16)) * kBlockK * 2);
+size_t gemm_smem_bytes(long m, int groups) {
+    const int rows = static_cast<int>(std::min<long>(kTileTok, (m + 15) / 16 * 16));
+    const int stages = groups == 1 ? static_cast<int>(one_group_stages(static_cast<uint32_t>(rows))) : kStagesMax;
+    return std::min(kGemmSmemBytes, kLutWin + kLutBytes + static_cast<size_t>(stages) * kSubPerStage * rows * kBlockK * 2);
+}
+// Producer groups of a single product.  Three stream codes fastest (5120 x 55296 at 32 rows 60 us, 66 with two), but 30 warps of 64 registers fill the SM: the
+// CTA is set up, makes its table and fetches its first codes only when the rotation in front is gone, and the kernels around it wait for its end in
+// turn.  18 warps leave room for CTAs of the rotation and of the split sums, and all of a call's kernels are there when the one in
+// front of them ends: what lies between two of them is one wait (1.1 us).  So two groups where a CTA has one tile and few stages, that is less to
+// stream than the set-up costs.  Calls in a graph, three groups (one kernel after the other) -> two: 4096 x 4096 at 16 rows (eight stages) 11.5 -> 9.2 us,
+// 3584 x 3584 at 64 12.7 -> 11.7 (at 256 20.3 -> 17.4), 3072 x 18944 at 64 (24) 19.0 -> 17.7, 3584 x 18944 at 16 (28) 19.8 -> 19.0, 18944 x 3584 at 16 (30)
+// 21.6 -> 20.9; beyond that the other way round, at 64 rows a little earlier: 28672 x 2048 (25) 24.4 -> 25.9, 4096 x 18944 (32) 23.3 -> 24.0.
+int gemm_groups(long n_tiles, int k_blocks, long m, int sm_count) {
+    const int stages = (k_blocks + kSubPerStage - 1) / kSubPerStage;
+    return n_tiles <= sm_count && stages <= (m <= 32 ? 30 : 24) ? 2 : kGroupsMax;
+}
+// Rows up to which one group serves a launch of several matrices (its tensor memory holds an accumulator of so many).
+constexpr long kGroupOneRows = 128;
+// An SM divides its 228 KB between shared memory and first-level cache anew only when it is empty, and small kernels ask for little of it: the product's
+// CTA did not come beside them.  So all three kernels of a call ask for what the product takes and 10 KB, where that is more than 100 KB (7168 x 2048 at 64
+// rows 14.3 -> 12.0 us, 8192 x 1024 12.6 -> 11.5; 4096 x 4096 at 16 rows, whose loads of codes then have less of the cache, 8.5 -> 9.1).  Percent; 0: no wish.
+int gemm_carveout(long m, int groups) {
+    if (m <= 32 || groups == kGroupsMax) return 0;
+    const size_t kb = (gemm_smem_bytes(m, groups) / 1024 + 1) * (groups == 1 ? 2 : 1) + 10;
+    return std::min(100, static_cast<int>(kb * 100 / 228 + 1));
 }
 constexpr unsigned long long kGemmWaitLimitNs = 200ull * 1000 * 1000;
 
@@ -258,6 +283,41 @@ __global__ void __launch_bounds__(128) rotate_rows_f16_kernel(const __half* __re
     }
 }
 
+// The butterfly stages of a block above 128 columns, between a lane's chunks.
+template <int CHUNKS>
+__device__ __forceinline__ void rotate_chunks_above(float (&v)[CHUNKS][8]) {
+#pragma unroll
+    for (int h = 1; h < CHUNKS; h <<= 1)
+#pragma unroll
+        for (int i = 0; i < CHUNKS; i += 2 * h)
+#pragma unroll
+            for (int c = i; c < i + h; ++c)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float a0 = v[c][j], b0 = v[c + h][j];
+                    v[c][j] = __fadd_rn(a0, b0);
+                    v[c + h][j] = __fsub_rn(a0, b0);
+                }
+}
+// A lane's rotated columns of a row to their places among the 8 rows in shared memory.  The lane's two groups of four columns are 16 positions
+// apart; lane ^ 2 holds the ones next to them.  The lanes swap one group each, so that every lane stores a whole core-matrix row of 8.
+template <int CHUNKS>
+__device__ __forceinline__ void rotated_row_out(float (&v)[CHUNKS][8], float inv_sqrt, int lane, int wib, unsigned live, uint4* s_rows) {
+    const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
+    const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
+    const int cc = pos >> 3;
+    uint4* const put = s_rows + (lane >> 3) * 64 + cc * 8 + (wib ^ cc);
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[c][j] *= inv_sqrt;
+        const uint4 h = pack_halves(v[c]);
+        const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
+        const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
+        put[256 * c] = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
+    }
+}
+
 // The same with 16-byte accesses, for any WHT block: a warp takes CHUNKS x 256 columns of a row (one block of 512 or
 // 1024 columns, or the blocks of 256 columns), lane l the 8 columns 8l..8l+7 of each chunk; butterfly stages below 8 stay in
 // the lane, the next are lane exchanges, those above 128 stay in the lane again (the add tree of warp_fwht).  The 8 warps of
@@ -288,12 +348,6 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
 #pragma unroll
     for (int k = 0; k < STAGES; ++k) side[k] = (lane & (1 << k)) != 0 ? -1.0f : 1.0f;
     const int kb_per_plane = in / kBlockK;
-    // A lane's two groups of four columns are 16 positions apart; lane ^ 2 holds the ones next to them.  The lanes swap
-    // one group each, so that every lane stores a whole core-matrix row of 8.
-    const bool odd = (lane & 2) != 0;   // of the pair: the upper four of the row
-    const int pos = 16 * (2 * (lane & 1) + (odd ? 1 : 0)) + 8 * ((lane >> 2) & 1);   // k_position of the row's first column
-    const int cc = pos >> 3;
-    uint4* put = &s_rows[0][(lane >> 3) * 64 + cc * 8 + (wib ^ cc)];
     // in the other direction: thread -> K block (of four per chunk), core column and row
     const int t = threadIdx.x & 63, tc = t >> 3, tr = t & 7;
     const uint4* get = &s_rows[0][(threadIdx.x >> 6) * 64 + tc * 8 + (tr ^ tc)];
@@ -327,27 +381,8 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
             float v[CHUNKS][8];
 #pragma unroll
             for (int c = 0; c < CHUNKS; ++c) rotate_chunk_fixed<STAGES>(v[c], raw[c], signs[c], side, live);
-#pragma unroll
-            for (int h = 1; h < CHUNKS; h <<= 1)
-#pragma unroll
-                for (int i = 0; i < CHUNKS; i += 2 * h)
-#pragma unroll
-                    for (int c = i; c < i + h; ++c)
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float a0 = v[c][j], b0 = v[c + h][j];
-                            v[c][j] = __fadd_rn(a0, b0);
-                            v[c + h][j] = __fsub_rn(a0, b0);
-                        }
-#pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[c][j] *= inv_sqrt;
-                const uint4 h = pack_halves(v[c]);
-                const uint2 keep = odd ? make_uint2(h.z, h.w) : make_uint2(h.x, h.y), give = odd ? make_uint2(h.x, h.y) : make_uint2(h.z, h.w);
-                const uint2 got = make_uint2(__shfl_xor_sync(live, give.x, 2), __shfl_xor_sync(live, give.y, 2));
-                put[256 * c] = odd ? make_uint4(got.x, got.y, keep.x, keep.y) : make_uint4(keep.x, keep.y, got.x, got.y);
-            }
+            rotate_chunks_above<CHUNKS>(v);
+            rotated_row_out<CHUNKS>(v, inv_sqrt, lane, wib, live, &s_rows[flip == kOther ? 0 : 1][0]);
         }
         __syncthreads();   // (the other buffer's readers are past it when it is written again)
         if (row8 + tr < rows) {
@@ -355,7 +390,6 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
             for (int c = 0; c < CHUNKS; ++c)
                 if (kb_at + 4 * c < kb_per_plane) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(4 * c) * (kTileTok * kBlockK)) = get[256 * c];
         }
-        put += flip;
         get += flip;
         flip = -flip;
         src += src_step;
@@ -363,11 +397,53 @@ __device__ __forceinline__ void rotate_rows_wide_body(const __half* __restrict__
         if ((row8 + 8) % kTileTok == 0) dst = place(row8 + 8);
     }
 }
+// The same of one group of 8 rows a CTA, for few rows (FEW): the kernel lies between two others whose ends are waited for, so what counts is the time from one
+// wait to the next.  It lets the product's CTAs come at once - beside it they make their tables and fetch their first codes - and has its signs
+// in hand when its own wait is over.  32 registers (48 and 64 with two and four chunks): three CTAs of it fit beside a product's, where four with 40 kept it
+// away: 8192 x 2048 at 64 rows 14.0 -> 12.4 us, 4096 x 4096 12.8 -> 11.4.
+template <int CHUNKS, int STAGES>
+__device__ __forceinline__ void rotate_rows_few_body(const __half* __restrict__ x, __half* __restrict__ xrot, int in, int rows, int block, uint32_t seed,
+                                                     unsigned col_group, unsigned row_group, float inv_sqrt, uint4* s_rows) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, row8 = 8 * static_cast<int>(row_group);
+    const int col = static_cast<int>(col_group) * 256 * CHUNKS + 8 * lane;
+    const bool have = col < in;   // (see above)
+    const unsigned live = __ballot_sync(0xffffffffu, have);
+    uint4 signs[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block);
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // x, and the scratch that is overwritten, belong to the kernels before until they are done
+    behind_wait(x);
+    if (have && row8 + wib < rows) {
+        const __half* const src = x + static_cast<size_t>(row8 + wib) * in + col;
+        uint4 raw[CHUNKS];
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
+        float side[STAGES];
+#pragma unroll
+        for (int k = 0; k < STAGES; ++k) side[k] = (lane & (1 << k)) != 0 ? -1.0f : 1.0f;
+        float v[CHUNKS][8];
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) rotate_chunk_fixed<STAGES>(v[c], raw[c], signs[c], side, live);
+        rotate_chunks_above<CHUNKS>(v);
+        rotated_row_out<CHUNKS>(v, inv_sqrt, lane, wib, live, s_rows);
+    }
+    __syncthreads();
+    const int t = threadIdx.x & 63, tc = t >> 3, tr = t & 7, kb_per_plane = in / kBlockK;
+    const int kb_at = static_cast<int>(col_group) * 4 * CHUNKS + static_cast<int>(threadIdx.x >> 6);
+    if (row8 + tr < rows) {
+        __half* const dst = xrot + (static_cast<size_t>(row8 / kTileTok) * kb_per_plane + kb_at) * (kTileTok * kBlockK) + ((row8 % kTileTok >> 3) * 64 + t) * 8;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c)
+            if (kb_at + 4 * c < kb_per_plane)
+                *reinterpret_cast<uint4*>(dst + static_cast<size_t>(4 * c) * (kTileTok * kBlockK)) = s_rows[256 * c + (threadIdx.x >> 6) * 64 + tc * 8 + (tr ^ tc)];
+    }
+}
 // The lane exchanges of a block as a constant of the loop over rows.
-template <int CHUNKS>
+template <int CHUNKS, bool FEW>
 __device__ __forceinline__ void rotate_rows_wide(const __half* __restrict__ x, __half* __restrict__ xrot, int in, long rows, int block, uint32_t seed_p,
                                                  uint32_t seed_r, float inv_sqrt, int row_steps) {
-    __shared__ __align__(16) uint4 s_rows[2][256 * CHUNKS];   // [step parity][K block][core column][row slot]
+    __shared__ __align__(16) uint4 s_rows[FEW ? 1 : 2][256 * CHUNKS];   // [step parity][K block][core column][row slot]
     const unsigned groups_per_row = (static_cast<unsigned>(in) + 256 * CHUNKS - 1) / (256 * CHUNKS);
     const unsigned row_groups = static_cast<unsigned>((rows + 8 * row_steps - 1) / (8 * row_steps));
     // blockIdx.x -> (plane, column group, rows); warp -> row inside a group of 8
@@ -375,32 +451,37 @@ __device__ __forceinline__ void rotate_rows_wide(const __half* __restrict__ x, _
     const uint32_t seed = plane ? seed_r : seed_p;
     __half* const to = xrot + plane * ((static_cast<size_t>(rows) + kTileTok - 1) / kTileTok * (in / kBlockK) * (kTileTok * kBlockK));
     const int m = static_cast<int>(rows);
+#define TQ_ROTATE_BODY(STAGES)                                                                                                        \
+    if constexpr (FEW) rotate_rows_few_body<CHUNKS, STAGES>(x, to, in, m, block, seed, cg, rg, inv_sqrt, &s_rows[0][0]);               \
+    else rotate_rows_wide_body<CHUNKS, STAGES>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows)
     if constexpr (CHUNKS > 1) {
-        rotate_rows_wide_body<CHUNKS, 5>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows);
+        TQ_ROTATE_BODY(5);
     } else {
         switch (block) {
-            case 32: rotate_rows_wide_body<1, 2>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
-            case 64: rotate_rows_wide_body<1, 3>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
-            case 128: rotate_rows_wide_body<1, 4>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
-            default: rotate_rows_wide_body<1, 5>(x, to, in, m, block, seed, cg, rg, inv_sqrt, row_steps, s_rows); break;
+            case 32: TQ_ROTATE_BODY(2); break;
+            case 64: TQ_ROTATE_BODY(3); break;
+            case 128: TQ_ROTATE_BODY(4); break;
+            default: TQ_ROTATE_BODY(5); break;
         }
     }
+#undef TQ_ROTATE_BODY
 }
-template <int CHUNKS>
-__global__ void __launch_bounds__(256) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
+__host__ __device__ constexpr int rotate_ctas(int chunks, bool few) { return chunks == 1 ? (few ? 8 : 5) : !few ? 0 : chunks == 2 ? 5 : 4; }
+template <int CHUNKS, bool FEW>
+__global__ void __launch_bounds__(256, rotate_ctas(CHUNKS, FEW)) rotate_rows_f16_wide_kernel(const __half* __restrict__ x, __half* __restrict__ xrot,
                                                                    int in, long rows, int block,
                                                                    uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int row_steps) {
-    rotate_rows_wide<CHUNKS>(x, xrot, in, rows, block, seed_p, seed_r, inv_sqrt, row_steps);
+    rotate_rows_wide<CHUNKS, FEW>(x, xrot, in, rows, block, seed_p, seed_r, inv_sqrt, row_steps);
 }
 // The same rows rotated for several matrices at once (their own seeds and destinations): blockIdx.y = matrix.
 struct RotateGroupArgs {
     __half* xrot[4];
     uint32_t seed_p[4], seed_r[4];
 };
-template <int CHUNKS>
-__global__ void __launch_bounds__(256) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
+template <int CHUNKS, bool FEW>
+__global__ void __launch_bounds__(256, rotate_ctas(CHUNKS, FEW)) rotate_rows_f16_wide_group_kernel(const __half* __restrict__ x, const __grid_constant__ RotateGroupArgs g, int in,
                                                                          long rows, int block, float inv_sqrt, int row_steps) {
-    rotate_rows_wide<CHUNKS>(x, g.xrot[blockIdx.y], in, rows, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
+    rotate_rows_wide<CHUNKS, FEW>(x, g.xrot[blockIdx.y], in, rows, block, g.seed_p[blockIdx.y], g.seed_r[blockIdx.y], inv_sqrt, row_steps);
 }
 
 struct GemmArgs {
@@ -426,8 +507,11 @@ struct GemmArgs {
 // primary seed, its second the residual ones.  A lookup serves both (as two planes one after the other the codes were read and looked up
 // twice: 3584 x 3584, block 512, 20.2 us at 64 rows, 31.6 at 256 and 116 at 2048; 16.7, 24.8 and 93 so.  18944 x 3584 at 64 rows 50.7
 // and 39.6.)
-template <bool DUAL>
+template <bool DUAL, int kGroups>
 __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const int t_step, const int t_end, const int bz) {
+    constexpr int kProducerWarps = 8 * kGroups, kGemmThreads = gemm_threads(kGroups);
+    constexpr int kMmaWarp = kProducerWarps;       // issues the MMAs, owns the tensor-memory allocation
+    constexpr int kCopyWarp = kProducerWarps + 1;  // issues the activation-tile bulk copies
     extern __shared__ __align__(128) uint8_t gemm_smem[];
     __shared__ __align__(8) unsigned long long s_full[kStagesMax], s_empty[kStagesMax], s_accum_full[2], s_accum_empty[2];
     __shared__ uint32_t s_tmem_base;
@@ -439,7 +523,10 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     // the tail of a prefill) costs a short MMA and a short copy.
     auto tile_rows = [&](int t) { return min(kTileTok, ((p.m - (t % n_tok) * kTileTok) + 15) & ~15); };
     const int n_max = min(kTileTok, (p.m + 15) & ~15);
-    const int n_acc = n_max <= kTileTok / 2 ? 2 : 1;   // accumulators: with two, a tile is drained beside the next one's products
+    const uint32_t tmem_cols = kGroups == 1 ? 256u : kTmemCols;
+    const uint32_t a_column = kGroups == 1 ? one_group_a_column(static_cast<uint32_t>(n_max)) : kTmemAColumn;
+    const int max_stages = kGroups == 1 ? static_cast<int>(one_group_stages(static_cast<uint32_t>(n_max))) : kStagesMax;
+    const int n_acc = kGroups == kGroupsMax && n_max <= kTileTok / 2 ? 2 : 1;   // accumulators: with two, a tile is drained beside the next one's products
     const int n_local = t0 < t_end ? (t_end - t0 + t_step - 1) / t_step : 0;
 
     // ---- shared-memory map -------------------------------------------------------------------
@@ -454,8 +541,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     const uint32_t stage_bytes = kSubPerStage * piece_bytes;
     const uint32_t smem_end = raw + dyn_bytes;
     int n_st = smem_end > stage0 ? static_cast<int>((smem_end - stage0) / stage_bytes) : 0;
-    if (n_st > kStagesMax) n_st = kStagesMax;
-    if (raw > kLutWin || n_st < kGroups) {  // layout does not fit: refuse to run (nothing allocated yet)
+    if (n_st > max_stages) n_st = max_stages;
+    if (raw > kLutWin || n_st < kGroups || n_max > (kGroups == 1 ? 128 : kTileTok)) {  // layout does not fit: refuse to run (nothing allocated yet)
         if (tid == 0) raise_status(p.status, 9u);
         return;
     }
@@ -481,9 +568,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem_base)),
-                     "r"(kTmemCols)
+                     "r"(tmem_cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        // The kernels behind may come: what they do in front of their waits reads nothing but weights.  Not before this CTA has its tensor memory,
+        // which a CTA of the next product beside it may hold while that one waits for this kernel's end.  (With three groups there is no room for
+        // them: let go at the end of the copies, small ones go to many SMs; let go here they crowd on the first that are free, 2048 x 37888 at 16 rows 21.3 -> 21.9.)
+        if (kGroups < kGroupsMax) asm volatile("griddepcontrol.launch_dependents;");
     }
     // lookup table: entry e, lane copy l at kLutWin + e * 128 + l * 4, value (t, t) or (primary, residual) as fp16
 #pragma unroll
@@ -508,6 +599,62 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     const int n_kb = static_cast<int>(static_cast<long>(kb_per_plane) * (bz + 1) / p.k_splits) - kb_base;
     const int n_it = (n_kb + kBlocksPerStage - 1) / kBlocksPerStage;
 
+    auto epilogue = [&] {
+        // ---- epilogue: TMEM lanes 32 * (warp & 3) .. + 31 (a lane = a weight row), 32 activation rows at a time ----
+        constexpr int kColStep = kGroups == kGroupsMax ? 32 : 8 * kProducerWarps;   // a quarter of the warps for a quarter of the lanes
+        int acc = 0;
+        uint32_t par = 0u;
+        for (int j = 0; j < n_local; ++j) {
+            const int t = t0 + j * t_step;
+            if (!__all_sync(0xffffffffu, bar_wait(bar_acc_full + 8u * acc, par, abort_flag) && !*abort_flag)) {
+                raise_status(p.status, 8u);
+                atomicExch(&s_abort, 1u);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int r = (t / n_tok) * kTileRows + 32 * (warp & 3) + lane;
+            const int tok0 = (t % n_tok) * kTileTok;
+            const int rows = min(kTileTok, p.m - tok0);
+            const bool r_ok = r < p.out;
+            const float scale = r_ok ? __ldg(p.norms + r) * p.inv_scale : 0.f;
+            const uint32_t d_tmem = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(acc * (kTileTok / 2));
+            const int c_first = kGroups == kGroupsMax ? 0 : 32 * (warp >> 2);
+            __half* y = p.y + static_cast<size_t>(tok0 + c_first) * p.y_stride + r;
+            float* part = p.partial + (static_cast<size_t>(bz) * p.m + tok0 + c_first) * p.out + r;   // (only used with k_splits > 1)
+#pragma unroll 1
+            for (int c0 = c_first; c0 < rows; c0 += kColStep) {
+                uint32_t v[32];
+                tmem_ld32(d_tmem + static_cast<uint32_t>(c0), v);
+                if (kGroups == kGroupsMax && c0 + 32 >= rows) {   // the last read: the accumulator is free
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(bar_acc_empty + 8u * acc);
+                }
+                const int n = r_ok ? min(32, rows - c0) : 0;
+                if (p.k_splits == 1) {
+                    if (n == 32) {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k) {
+                            *y = __float2half_rn(__uint_as_float(v[k]) * scale);
+                            y += p.y_stride;
+                        }
+                        if (kColStep > 32) y += (kColStep - 32) * p.y_stride;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 32; ++k)
+                            if (k < n) y[k * p.y_stride] = __float2half_rn(__uint_as_float(v[k]) * scale);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; ++k)
+                        if (k < n) part[static_cast<size_t>(k) * p.out] = __uint_as_float(v[k]);
+                    part += static_cast<size_t>(kColStep) * p.out;
+                }
+            }
+            if (++acc == n_acc) { acc = 0; par ^= 1u; }
+        }
+    };
+
     if (warp < kProducerWarps) {
         // ---- producers ------------------------------------------------------------------------
         // Weight tile in tensor memory: lane = row of the tile, 64 columns per stage (two fp16 per
@@ -527,7 +674,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
         const int last_tile = (p.out - 1) >> 4;
         const size_t tile_row_bytes = static_cast<size_t>(code_tiles_per_row(p.in)) * kCodeTileBytes;
         const uint8_t* const code_lane = p.codes + (lane >> 2) * 64 + 16 * (lane & 3);
-        const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3) + (DUAL ? 16 * sub : 0)) << 16) + kTmemAColumn +
+        const uint32_t a_taddr = tmem_d + (static_cast<uint32_t>(32 * (warp & 3) + (DUAL ? 16 * sub : 0)) << 16) + a_column +
                                  (DUAL ? 0u : kTmemASubCols * static_cast<uint32_t>(sub));
 
         // The group's next stage to fetch: its place in its tile, where its codes are, stages left.
@@ -649,6 +796,10 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                 par ^= 1u;
             }
         }
+        if constexpr (kGroups < kGroupsMax) {
+            __syncwarp();
+            epilogue();
+        }
     } else if (warp == kCopyWarp) {
         // ---- activation tiles: one bulk copy per K block of the stage, as far ahead as the ring allows ----
         // One thread runs the whole loop; ring slot and phase are kept incrementally (no divisions on
@@ -687,7 +838,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                 }
             }
             // every activation tile of this CTA is on its way: the kernel after this one may start setting up
-            asm volatile("griddepcontrol.launch_dependents;");
+            if (kGroups == kGroupsMax) asm volatile("griddepcontrol.launch_dependents;");
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
@@ -716,7 +867,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const int nsub = DUAL ? kSubPerStage : min(kSubPerStage, n_kb - kSubPerStage * it);
-                    const uint32_t a_tmem = tmem_d + kTmemAColumn + kTmemAStageCols * static_cast<uint32_t>(slot);
+                    const uint32_t a_tmem = tmem_d + a_column + kTmemAStageCols * static_cast<uint32_t>(slot);
                     const uint32_t b_stage = stage0 + static_cast<uint32_t>(slot) * stage_bytes;
                     if (elect_one()) {
 #pragma unroll
@@ -740,71 +891,22 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             }
         }
         __syncwarp();
-    } else {
-        // ---- epilogue: TMEM lanes 32 * (warp & 3) .. + 31 (a lane = a weight row), 32 activation rows at a time ----
-        int acc = 0;
-        uint32_t par = 0u;
-        for (int j = 0; j < n_local; ++j) {
-            const int t = t0 + j * t_step;
-            if (!__all_sync(0xffffffffu, bar_wait(bar_acc_full + 8u * acc, par, abort_flag) && !*abort_flag)) {
-                raise_status(p.status, 8u);
-                atomicExch(&s_abort, 1u);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int r = (t / n_tok) * kTileRows + 32 * (warp & 3) + lane;
-            const int tok0 = (t % n_tok) * kTileTok;
-            const int rows = min(kTileTok, p.m - tok0);
-            const bool r_ok = r < p.out;
-            const float scale = r_ok ? __ldg(p.norms + r) * p.inv_scale : 0.f;
-            const uint32_t d_tmem = tmem_d + (static_cast<uint32_t>(32 * (warp & 3)) << 16) + static_cast<uint32_t>(acc * (kTileTok / 2));
-            __half* y = p.y + static_cast<size_t>(tok0) * p.y_stride + r;
-            float* part = p.partial + (static_cast<size_t>(bz) * p.m + tok0) * p.out + r;   // (only used with k_splits > 1)
-#pragma unroll 1
-            for (int c0 = 0; c0 < rows; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(d_tmem + static_cast<uint32_t>(c0), v);
-                if (c0 + 32 >= rows) {   // the last read: the accumulator is free
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(bar_acc_empty + 8u * acc);
-                }
-                const int n = r_ok ? min(32, rows - c0) : 0;
-                if (p.k_splits == 1) {
-                    if (n == 32) {
-#pragma unroll
-                        for (int k = 0; k < 32; ++k) {
-                            *y = __float2half_rn(__uint_as_float(v[k]) * scale);
-                            y += p.y_stride;
-                        }
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 32; ++k)
-                            if (k < n) y[k * p.y_stride] = __float2half_rn(__uint_as_float(v[k]) * scale);
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 32; ++k)
-                        if (k < n) part[static_cast<size_t>(k) * p.out] = __uint_as_float(v[k]);
-                    part += static_cast<size_t>(32) * p.out;
-                }
-            }
-            if (++acc == n_acc) { acc = 0; par ^= 1u; }
-        }
+    } else if constexpr (kGroups == kGroupsMax) {
+        epilogue();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(tmem_cols) : "memory");
     }
 }
 
 // gridDim.x CTAs walk the output tiles, gridDim.y = K splits.
-template <bool DUAL>
-__global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_kernel(const GemmArgs p) {
+template <bool DUAL, int GROUPS>
+__global__ void __launch_bounds__(gemm_threads(kGroupsMax), 1) tq8_gemm_kernel(const GemmArgs p) {
     const int n_tiles = ((p.out + kTileRows - 1) / kTileRows) * ((p.m + kTileTok - 1) / kTileTok);
-    gemm_body<DUAL>(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
+    gemm_body<DUAL, GROUPS>(p, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), n_tiles, static_cast<int>(blockIdx.y));
 }
 
 // Several matrices that multiply the same activation rows (q / k / v, gate / up) in one launch, a CTA per tile and K split.  Every
@@ -821,8 +923,12 @@ struct GemmGroupArgs {
     int n_tiles[kMaxGemmGroup];     // (flat)
     int n, flat;
 };
-template <bool DUAL>
-__global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const __grid_constant__ GemmGroupArgs grp) {
+// Where the CTAs outnumber the SMs they have one group of producers each and go two to an SM, the second half beside the first instead of behind it
+// (80 registers: a third one would find no tensor memory).  Two or three groups, one CTA to an SM -> one group: 3584 -> 3584 + 512 + 512 at 16 rows 15.1 -> 9.4 us,
+// at 64 17.6 -> 13.4, 5120 -> 5120 + 1024 + 1024 at 32 21.6 -> 19.3, 4096 -> 2 x 11008 at 16 39.1 -> 33.0.  Where they do not, two groups: 2048 -> 2 x 1024 at 32 rows
+// 7.1 -> 6.7, 768 -> 2 x 768 at 100 8.1 -> 6.7 (three 9.6).
+template <bool DUAL, int GROUPS>
+__global__ void __launch_bounds__(GROUPS == 1 ? 384 : gemm_threads(kGroupsMax), GROUPS == 1 ? 2 : 1) tq8_gemm_group_kernel(const __grid_constant__ GemmGroupArgs grp) {
     const int b = static_cast<int>(blockIdx.x);
     int i = 0;
     while (i + 1 < grp.n && b >= grp.start[i + 1]) ++i;
@@ -831,18 +937,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) tq8_gemm_group_kernel(const _
         bz = t / grp.n_tiles[i];
         t -= bz * grp.n_tiles[i];
     }
-    gemm_body<DUAL>(grp.m[i], t, 1, t + 1, bz);
+    gemm_body<DUAL, GROUPS>(grp.m[i], t, 1, t + 1, bz);
 }
 
 // y = fp16(norm * inv_scale * sum over K splits, in split order) - fixed order, run-to-run identical - for the matrices of a call
-// that were split (a group's by blockIdx.z).  Latency counts, it follows every split product of a decode batch: a thread takes four weight
-// rows, requests their norms before the kernel in front has ended, and then up to kBatch splits' sums at once.  (With one
-// element per thread, a 64-bit division for its place and the splits in turn: 7.9 us for 64 x 3584 in five splits under the
-// profiler, 4.7 here; 2048 x 512 twice in four splits 20.8, 15.4 here.)  Calls in a graph, with one element per thread and here:
-// 4096 x 1024 at 16 rows 10.0 and 10.1 us, 2048 x 600 at 100 rows 11.2 and 11.2, 4096 x 4096 at 16 rows 13.35 and 13.35, 3584 x 512 at 64
-// rows 10.5 and 10.1, 8192 x 2048 at 9 rows 13.87 and 13.87.  With the norms' products in front of the wait and eight splits
-// at once the last two were 9.9 and 14.38, 4096 x 4096 13.61; with an early release of the kernel behind and CTAs of 32
-// threads on top of that, up to a microsecond more.
+// that were split (a group's by blockIdx.z).  Latency counts, it follows every split product of a decode batch: a thread takes V weight
+// rows, requests their norms before the kernel in front has ended, and then BATCH splits' sums at once.  Behind products that leave room (early) its
+// CTAs are there before these end, and let those of the next call's rotation come in turn.  64 registers: eight CTAs to an SM, one or two beside a
+// product's.  With 126 (all sums of twelve splits at once) 8192 x 1024 in 16 splits took 11.2 us at 32 rows instead of 8.6, 2048 x 2048 at 512 rows 19.2 instead of 16.2;
+// as few CTAs as SMs, with several rows each, crowd on a few of them (3584 x 3584 at 64 rows 12.2 -> 15.0).  Behind a product that fills the SMs four CTAs to an SM
+// spread better (18944 x 3584 at 64 rows 25.1 us, 25.6 with eight): 126 registers there.
 struct FinishOne {
     const float* partial;
     const float* norms;
@@ -853,64 +957,98 @@ struct FinishOne {
 };
 struct FinishArgs { FinishOne m[kMaxGemmGroup]; };
 constexpr int kFinishThreads = 128;
-__device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m) {
+// V sums side by side in one access.
+template <int V>
+struct Sums {
+    float v[V];
+    __device__ __forceinline__ void load(const float* p) {
+        if constexpr (V == 4) {
+            const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+            const float2 t = __ldcg(reinterpret_cast<const float2*>(p));
+            v[0] = t.x; v[1] = t.y;
+        }
+    }
+};
+// V = 4, or 2 where more than eight splits are to be asked for at once.
+template <int kBatch, int V>
+__device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool early) {
     const int out = f.out, k_splits = f.k_splits;
-    const int c = 4 * static_cast<int>(blockIdx.x * kFinishThreads + threadIdx.x);
+    const int c = V * static_cast<int>(blockIdx.x * kFinishThreads + threadIdx.x);
     if (c >= out) return;
-    float norm[4];   // (used behind the wait only: a product with it in front of the wait would wait for it there)
+    float norm[V];   // (used behind the wait only: a product with it in front of the wait would wait for it there)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) norm[k] = c + k < out ? __ldg(f.norms + c + k) : 0.f;
-    pdl_wait_release();
-    constexpr int kBatch = 12;
+    for (int k = 0; k < V; ++k) norm[k] = c + k < out ? __ldg(f.norms + c + k) : 0.f;
+    if (early) asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!early) asm volatile("griddepcontrol.launch_dependents;");
+    const float* partial = f.partial;
+    behind_wait(partial);
     const size_t split = static_cast<size_t>(m) * out;
     for (int row = blockIdx.y; row < m; row += gridDim.y) {
-        const float* const src = f.partial + static_cast<size_t>(row) * out + c;
+        const float* const src = partial + static_cast<size_t>(row) * out + c;
         __half* const y = f.y + row * f.y_stride + c;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] = 0.f;
         if (f.vec) {
             for (int z0 = 0; z0 < k_splits; z0 += kBatch) {
-                float4 v[kBatch];
+                Sums<V> v[kBatch];
 #pragma unroll
                 for (int z = 0; z < kBatch; ++z)
-                    if (z0 + z < k_splits) v[z] = __ldcg(reinterpret_cast<const float4*>(src + (z0 + z) * split));
+                    if (z0 + z < k_splits) v[z].load(src + (z0 + z) * split);
 #pragma unroll
                 for (int z = 0; z < kBatch; ++z)
                     if (z0 + z < k_splits) {
-                        acc[0] += v[z].x; acc[1] += v[z].y; acc[2] += v[z].z; acc[3] += v[z].w;
+#pragma unroll
+                        for (int k = 0; k < V; ++k) acc[k] += v[z].v[k];
                     }
             }
-            const __half2 lo = __floats2half2_rn(acc[0] * (norm[0] * f.inv_scale), acc[1] * (norm[1] * f.inv_scale));
-            const __half2 hi = __floats2half2_rn(acc[2] * (norm[2] * f.inv_scale), acc[3] * (norm[3] * f.inv_scale));
-            *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            uint32_t h[V / 2];
+#pragma unroll
+            for (int k = 0; k < V; k += 2) {
+                const __half2 h2 = __floats2half2_rn(acc[k] * (norm[k] * f.inv_scale), acc[k + 1] * (norm[k + 1] * f.inv_scale));
+                h[k / 2] = *reinterpret_cast<const uint32_t*>(&h2);
+            }
+            if constexpr (V == 4) *reinterpret_cast<uint2*>(y) = make_uint2(h[0], h[1]);
+            else *reinterpret_cast<uint32_t*>(y) = h[0];
         } else {
             for (int z = 0; z < k_splits; ++z)
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                for (int k = 0; k < V; ++k)
                     if (c + k < out) acc[k] += __ldcg(src + z * split + k);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < V; ++k)
                 if (c + k < out) y[k] = __float2half_rn(acc[k] * (norm[k] * f.inv_scale));
         }
     }
 }
 // (A single matrix as a group of one, its parameters found by an index: 0.2 us more a call.)
-__global__ void __launch_bounds__(kFinishThreads) gemm_finish_kernel(const __grid_constant__ FinishOne f, int m) { gemm_finish_body(f, m); }
-__global__ void __launch_bounds__(kFinishThreads) gemm_finish_group_kernel(const __grid_constant__ FinishArgs f, int m) { gemm_finish_body(f.m[blockIdx.z], m); }
+template <int BATCH, int V>
+__global__ void __launch_bounds__(kFinishThreads, BATCH * V == 32 ? 8 : 0) gemm_finish_kernel(const __grid_constant__ FinishOne f, int m, bool early) { gemm_finish_body<BATCH, V>(f, m, early); }
+template <int BATCH, int V>
+__global__ void __launch_bounds__(kFinishThreads, BATCH * V == 32 ? 8 : 0) gemm_finish_group_kernel(const __grid_constant__ FinishArgs f, int m, bool early) { gemm_finish_body<BATCH, V>(f.m[blockIdx.z], m, early); }
 void finish_add(FinishArgs& f, int& n, const GemmArgs& a) {
     if (a.k_splits <= 1) return;
     f.m[n] = FinishOne{a.partial, a.norms, a.y, a.y_stride, a.out, a.k_splits,
                        a.out % 4 == 0 && a.y_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.y) % 8 == 0 ? 1 : 0, a.inv_scale};
     ++n;
 }
-void launch_finish(const FinishArgs& f, int n, int m, int sm_count, cudaStream_t stream) {
+void launch_finish(const FinishArgs& f, int n, int m, int groups, int sm_count, cudaStream_t stream) {
     if (n == 0) return;
-    int widest = 0;
-    for (int i = 0; i < n; ++i) widest = std::max(widest, f.m[i].out);
-    const int gx = (widest + 4 * kFinishThreads - 1) / (4 * kFinishThreads);
-    const int gy = std::max(1, std::min(m, 16 * sm_count / (gx * n)));   // sixteen CTAs per SM: one wave
+    int widest = 0, most = 0;
+    for (int i = 0; i < n; ++i) {
+        widest = std::max(widest, f.m[i].out);
+        most = std::max(most, f.m[i].k_splits);
+    }
+    const bool few = groups < kGroupsMax;
+    const int v = few && most > 8 ? 2 : 4, carveout = gemm_carveout(m, groups);
+    const int gx = (widest + v * kFinishThreads - 1) / (v * kFinishThreads);
+    const int gy = std::max(1, std::min(m, 16 * sm_count / (gx * n)));   // up to sixteen CTAs per SM
     const dim3 grid(static_cast<unsigned int>(gx), static_cast<unsigned int>(gy), static_cast<unsigned int>(n));
-    if (n == 1) launch_pdl(gemm_finish_kernel, grid, dim3(kFinishThreads), 0, stream, f.m[0], m);
-    else launch_pdl(gemm_finish_group_kernel, grid, dim3(kFinishThreads), 0, stream, f, m);
+    if (n == 1) launch_pdl_carved(!few ? gemm_finish_kernel<12, 4> : v == 4 ? gemm_finish_kernel<8, 4> : gemm_finish_kernel<16, 2>, grid, dim3(kFinishThreads), 0, carveout, stream, f.m[0], m, few);
+    else launch_pdl_carved(v == 4 ? gemm_finish_group_kernel<8, 4> : gemm_finish_group_kernel<16, 2>, grid, dim3(kFinishThreads), 0, carveout, stream, f, m, few);
 }
 
 // Groups of 8 rows that a CTA of the rotation takes one after the other: as many as leave eight CTAs per SM.
@@ -920,7 +1058,7 @@ int rotate_row_steps(long groups, int sm_count) { return static_cast<int>(std::m
 // not aligned.  Both kernels add in the order of warp_fwht, in fp32: the operand does not depend on the alignment.  (With four of the
 // butterflies as products with +-1 on the tensor cores a 7B layer's projections of 2048 rows took 1100 us instead of 1120, of 64 rows
 // 119 instead of 121; but the sums were rounded elsewhere, and the results of the two kernels differed.)
-void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int in, long m, int n_planes, uint32_t block, int sm_count, cudaStream_t stream) {
+void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int in, long m, int n_planes, uint32_t block, int groups_of_product, int carveout, int sm_count, cudaStream_t stream) {
     const float inv_sqrt = 1.0f / std::sqrt(static_cast<float>(block));
     const int bs = static_cast<int>(block);
     if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {
@@ -930,9 +1068,10 @@ void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int 
         const long ctas = groups * ((m + 8L * row_steps - 1) / (8L * row_steps));
         if (ctas < (1L << 31)) {
             const dim3 grid(static_cast<unsigned int>(ctas), static_cast<unsigned int>(n));
+            const bool few = row_steps == 1 && groups_of_product < kGroupsMax;
 #define TQ_ROTATE_WIDE(CHUNKS)                                                                                                                         \
-    if (n == 1) launch_pdl(rotate_rows_f16_wide_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot.xrot[0], in, m, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
-    else launch_pdl(rotate_rows_f16_wide_group_kernel<CHUNKS>, grid, dim3(256), 0, stream, x, rot, in, m, bs, inv_sqrt, row_steps);
+    if (n == 1) launch_pdl_carved(few ? rotate_rows_f16_wide_kernel<CHUNKS, true> : rotate_rows_f16_wide_kernel<CHUNKS, false>, grid, dim3(256), 0, carveout, stream, x, rot.xrot[0], in, m, bs, rot.seed_p[0], rot.seed_r[0], inv_sqrt, row_steps); \
+    else launch_pdl_carved(few ? rotate_rows_f16_wide_group_kernel<CHUNKS, true> : rotate_rows_f16_wide_group_kernel<CHUNKS, false>, grid, dim3(256), 0, carveout, stream, x, rot, in, m, bs, inv_sqrt, row_steps);
             switch (cols) {
                 case 256: TQ_ROTATE_WIDE(1) break;
                 case 512: TQ_ROTATE_WIDE(2) break;
@@ -961,6 +1100,15 @@ void launch_rotate_rows(const __half* x, const RotateGroupArgs& rot, int n, int 
 size_t xrot_bytes(int in, long m, int n_planes) {
     const size_t padded = (static_cast<size_t>(m) + kTileTok - 1) / kTileTok * kTileTok;  // whole operand tiles
     return (static_cast<size_t>(n_planes) * padded * static_cast<size_t>(in) * sizeof(__half) + 255) & ~static_cast<size_t>(255);
+}
+
+auto gemm_kernel_of(int n_planes, int groups) {
+    if (n_planes == 2) return groups == 2 ? tq8_gemm_kernel<true, 2> : tq8_gemm_kernel<true, 3>;
+    return groups == 2 ? tq8_gemm_kernel<false, 2> : tq8_gemm_kernel<false, 3>;
+}
+auto gemm_group_kernel_of(int n_planes, int groups) {
+    if (n_planes == 2) return groups == 1 ? tq8_gemm_group_kernel<true, 1> : groups == 2 ? tq8_gemm_group_kernel<true, 2> : tq8_gemm_group_kernel<true, 3>;
+    return groups == 1 ? tq8_gemm_group_kernel<false, 1> : groups == 2 ? tq8_gemm_group_kernel<false, 2> : tq8_gemm_group_kernel<false, 3>;
 }
 
 }  // namespace
@@ -1000,12 +1148,16 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
     TQ_REQUIRE(scratch != nullptr, "tq8_gemm needs its scratch buffer");
     if (out == 0) return;
     __half* xrot = static_cast<__half*>(scratch);
+    const long n_tiles = static_cast<long>((out + kTileRows - 1) / kTileRows) * ((m + kTileTok - 1) / kTileTok);
+    TQ_REQUIRE(n_tiles < (1L << 31), "tq8_gemm: too many output tiles");
+    const int k_splits = gemm_k_splits(out, in, m, n_planes, sm_count);
+    const int groups = gemm_groups(n_tiles, in / kBlockK * n_planes / k_splits, m, sm_count);
 
     // 1. rotate every activation row
     {
         RotateGroupArgs rot{};
         rot.xrot[0] = xrot; rot.seed_p[0] = seed_p; rot.seed_r[0] = seed_r;
-        launch_rotate_rows(x, rot, 1, in, m, n_planes, block, sm_count, stream);
+        launch_rotate_rows(x, rot, 1, in, m, n_planes, block, groups, gemm_carveout(m, groups), sm_count, stream);
     }
     // 2. the GEMM
     GemmArgs a{};
@@ -1016,27 +1168,24 @@ void launch_tq8_gemm(const uint8_t* codes, const float* norms, const float* tabl
         a.table += 512;   // (the pairs, behind the two tables)
         a.inv_scale *= pair_unit;
     }
-    a.k_splits = gemm_k_splits(out, in, m, n_planes, sm_count);
+    a.k_splits = k_splits;
     a.partial = a.k_splits > 1 ? reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + xrot_bytes(in, m, n_planes)) : nullptr;
-    const size_t smem = gemm_smem_bytes(m);
     static bool configured[64] = {false};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
+        for (auto* const k : {tq8_gemm_kernel<false, 2>, tq8_gemm_kernel<true, 2>, tq8_gemm_kernel<false, 3>, tq8_gemm_kernel<true, 3>})
+            TQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
     // a CTA per SM walks the tiles (with a K split there are fewer tiles x splits than SMs)
-    const long n_tiles = static_cast<long>((out + kTileRows - 1) / kTileRows) * ((m + kTileTok - 1) / kTileTok);
-    TQ_REQUIRE(n_tiles < (1L << 31), "tq8_gemm: too many output tiles");
     const dim3 grid(static_cast<unsigned int>(std::min<long>(n_tiles, sm_count)), static_cast<unsigned int>(a.k_splits));
-    launch_pdl(n_planes == 2 ? tq8_gemm_kernel<true> : tq8_gemm_kernel<false>, grid, dim3(kGemmThreads), smem, stream, a);
+    launch_pdl_carved(gemm_kernel_of(n_planes, groups), grid, dim3(gemm_threads(groups)), gemm_smem_bytes(m, groups), gemm_carveout(m, groups), stream, a);
     TQ_CUDA(cudaGetLastError());
     FinishArgs fin{};
     int n_fin = 0;
     finish_add(fin, n_fin, a);
-    launch_finish(fin, n_fin, static_cast<int>(m), sm_count, stream);
+    launch_finish(fin, n_fin, static_cast<int>(m), groups, sm_count, stream);
 }
 
 void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, long m, int sm_count, cudaStream_t stream) {
@@ -1053,7 +1202,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     FinishArgs fin{};
     int n_fin = 0;
     grp.n = n;
-    long n_ctas = 0;
+    long n_ctas = 0, n_products = 0;
     int order[kMaxGemmGroup], splits[kMaxGemmGroup];
     const long tok_tiles = (m + kTileTok - 1) / kTileTok;
     for (int i = 0; i < n; ++i) {
@@ -1085,27 +1234,29 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         grp.n_tiles[i] = static_cast<int>(n_tiles);
         grp.start[i] = static_cast<int>(n_ctas);
         n_ctas += grp.flat ? n_tiles * a.k_splits : row_tiles;
+        n_products += n_tiles * a.k_splits;
         TQ_REQUIRE(n_tiles < (1L << 31) && n_ctas < (1L << 31), "tq8_gemm group: too many output tiles");
         rot.xrot[i] = static_cast<__half*>(it.scratch);
         rot.seed_p[i] = it.seed_p; rot.seed_r[i] = it.seed_r;
         finish_add(fin, n_fin, a);
     }
     for (int i = n; i <= kMaxGemmGroup; ++i) grp.start[i] = static_cast<int>(n_ctas);
+    const int groups = m <= kGroupOneRows && n_products > sm_count ? 1 : 2;
     // 1. the rotations
-    launch_rotate_rows(x, rot, n, in, m, n_planes, block, sm_count, stream);
+    launch_rotate_rows(x, rot, n, in, m, n_planes, block, groups, gemm_carveout(m, groups), sm_count, stream);
     // 2. the GEMMs
     static bool configured[64] = {false};
     int dev = 0;
     TQ_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !configured[dev]) {
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
-        TQ_CUDA(cudaFuncSetAttribute(tq8_gemm_group_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
+        for (auto* const k : {tq8_gemm_group_kernel<false, 1>, tq8_gemm_group_kernel<true, 1>, tq8_gemm_group_kernel<false, 2>, tq8_gemm_group_kernel<true, 2>, tq8_gemm_group_kernel<false, 3>, tq8_gemm_group_kernel<true, 3>})
+            TQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmemBytes)));
         if (dev < 64) configured[dev] = true;
     }
     const dim3 grid(static_cast<unsigned int>(n_ctas), grp.flat ? 1u : static_cast<unsigned int>(tok_tiles), grp.flat ? 1u : static_cast<unsigned int>(splits[0]));
-    launch_pdl(n_planes == 2 ? tq8_gemm_group_kernel<true> : tq8_gemm_group_kernel<false>, grid, dim3(kGemmThreads), gemm_smem_bytes(m), stream, grp);
+    launch_pdl_carved(gemm_group_kernel_of(n_planes, groups), grid, dim3(gemm_threads(groups)), gemm_smem_bytes(m, groups), gemm_carveout(m, groups), stream, grp);
     // 3. the split-K sums
-    launch_finish(fin, n_fin, static_cast<int>(m), sm_count, stream);
+    launch_finish(fin, n_fin, static_cast<int>(m), groups, sm_count, stream);
 }
 
 }  // namespace tq
