@@ -106,12 +106,25 @@ __device__ __forceinline__ uint32_t lut_addr(uint32_t word, uint32_t lane_const)
 }
 
 // ---- activation rotation ---------------------------------------------------------------------
+// Where word (row, col) of a rotated activation stands when the decode kernel is to read it: in the order of its B fragments.  A load of a
+// warp is 16 bytes of every lane (g = row, q = 16 columns of a 64-column block): blocks of [4 pieces of 4 columns][bp rows][16-column groups q][4], bp the
+// rows rounded up to 1, 2, 4 or 8.  Row after row, those 16 bytes lay in as many lines as there were lanes, and every CTA spent more time on its 128 KB
+// of activations than on a unit of codes: 4096 x 4096 at eight rows 9.6 -> 8.2 us, 3584 x 3584 with two rotations at eight
+// 12.0 -> 9.4, 18944 x 3584 at four 24.5 -> 23.7, 27648 x 5120 at eight 46.2 -> 44.3.  (in is a multiple of 32: a last block of 32 columns has two groups q.)
+__host__ __device__ __forceinline__ int fragment_groups(int in, int col) {
+    const int left = (in - (col & ~63)) >> 4;
+    return left < 4 ? left : 4;
+}
+__host__ __device__ __forceinline__ size_t fragment_place(int in, int bp, int row, int col) {
+    return static_cast<size_t>(col >> 6) * (64 * bp) + static_cast<size_t>(((((col & 15) >> 2) * bp + row) * fragment_groups(in, col) + ((col & 63) >> 4)) * 4 + (col & 3));
+}
+__host__ __device__ __forceinline__ constexpr int padded_rows(int batch) { return batch <= 1 ? 1 : batch <= 2 ? 2 : batch <= 4 ? 4 : 8; }
 // One warp per (plane, batch row, WHT block): xrot = FWHT(sign o x) / sqrt(bs), rounded to
-// TF32 and stored as fp32 [plane][row][in].
+// TF32 and stored as fp32, [plane][row][in] or (fragments: the padded rows; one plane) in the decode kernel's order.
 template <int E>
 __global__ void __launch_bounds__(128) rotate_x_kernel(const __half* __restrict__ x, float* __restrict__ xrot, int in,
                                                        int batch, int n_planes, uint32_t seed_p, uint32_t seed_r,
-                                                       float inv_sqrt) {
+                                                       float inv_sqrt, int fragments) {
     // Let the GEMV that follows start its set-up right away; it waits for this grid to
     // finish before it reads xrot.
     grid_launch_dependents();
@@ -133,9 +146,10 @@ __global__ void __launch_bounds__(128) rotate_x_kernel(const __half* __restrict_
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = __half2float(src[j]) * sign_value(seed, static_cast<uint32_t>(lane * E + j));
     warp_fwht<E>(v, lane);
-    float* dst = xrot + (static_cast<size_t>(plane) * batch + row) * in + blk * BS + lane * E;
+    const int col = blk * BS + lane * E;
+    float* const dst = xrot + (static_cast<size_t>(plane) * batch + row) * in + col;
 #pragma unroll
-    for (int j = 0; j < E; ++j) dst[j] = to_tf32(v[j] * inv_sqrt);
+    for (int j = 0; j < E; ++j) *(fragments ? xrot + fragment_place(in, fragments, row, col + j) : dst + j) = to_tf32(v[j] * inv_sqrt);
 }
 
 // The same with 16-byte accesses: a warp takes CHUNKS x 256 columns of a row (a WHT block of 512 or 1024 columns, or the
@@ -145,7 +159,7 @@ __global__ void __launch_bounds__(128) rotate_x_kernel(const __half* __restrict_
 // same reason the launch asks for shared memory it does not use: four CTAs per SM.
 template <int CHUNKS>
 __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __restrict__ x, float* __restrict__ xrot, int in, int batch,
-                                                            int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt) {
+                                                            int n_planes, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt, int fragments) {
     grid_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
@@ -161,12 +175,25 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     // the loads, behind which they are made: in front, 4096 x 4096, block 512, took 8.8 us at one row instead of 8.3, 1024 x 1024 6.4 instead of 5.9.
     uint4 signs;
     if (CHUNKS == 1) signs = chunk_signs(seed, static_cast<uint32_t>(col), block);
+    // A lane's eight columns are four and four: in the order of the fragments a piece apart, 256 columns on at 256 words a row.  (Their places in front
+    // of the wait, those of several chunks beside the loads, like the signs: 4096 x 4096, block 512, one row 8.2 us, in front 8.5.)
+    float* dst = xrot;
+    int half = 4, chunk = 256;
+    auto find_place = [&] {
+        dst += fragments ? fragment_place(in, fragments, row, col) : (static_cast<size_t>(plane) * batch + row) * in + col;
+        if (fragments) {
+            half = 4 * fragments * fragment_groups(in, col);
+            chunk = 256 * fragments;
+        }
+    };
+    if (CHUNKS == 1) find_place();
     grid_dependency_sync();
     behind_wait(x);
     const __half* const src = x + static_cast<size_t>(row) * in + col;
     uint4 raw[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
+    if (CHUNKS > 1) find_place();
     float v[CHUNKS][8];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
@@ -185,55 +212,61 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
                     v[c][j] = __fadd_rn(a, b);
                     v[c + h][j] = __fsub_rn(a, b);
                 }
-    float* const dst = xrot + (static_cast<size_t>(plane) * batch + row) * in + col;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
         for (int j = 0; j < 8; j += 4)
-            *reinterpret_cast<float4*>(dst + 256 * c + j) = make_float4(to_tf32(v[c][j] * inv_sqrt), to_tf32(v[c][j + 1] * inv_sqrt),
-                                                                        to_tf32(v[c][j + 2] * inv_sqrt), to_tf32(v[c][j + 3] * inv_sqrt));
+            *reinterpret_cast<float4*>(dst + c * chunk + j / 4 * half) =
+                make_float4(to_tf32(v[c][j] * inv_sqrt), to_tf32(v[c][j + 1] * inv_sqrt), to_tf32(v[c][j + 2] * inv_sqrt), to_tf32(v[c][j + 3] * inv_sqrt));
 }
-constexpr size_t kRotateXSmem = 48 * 1024;
+constexpr size_t kRotateXSmem = 48 * 1024, kRotatePairSmem = 38 * 1024;
 
-// The activation of weights with two rotations: a warp rotates CHUNKS x 256 columns of a row with either seed and writes pairs
-// of fp16 (primary, residual), [row][in], each 256 columns times a power of two that brings the largest value of the
+// The activation of weights with two rotations: two warps rotate CHUNKS x 256 columns of a row, each with one of the seeds, and write pairs
+// of fp16 (primary, residual) in the order of the decode kernel's fragments, each 256 columns times a power of two that brings the largest value of the
 // two to [2^14, 2^15), and that power's inverse to xscale[row][columns / 256].  A row that is not 16-byte aligned (`aligned` = 0) is
 // read in halves: 2 KB at most per warp.
+// The decode kernel waits for the end of this one, few warps alone on their SMs: what counts is the instructions of a warp behind its wait.  So the
+// signs are in hand before it, and a warp has one seed, not both: 1.6 us from the wait to the end at four rows of 3584 columns in blocks of 512, 3 to 3.8 with
+// both seeds in a warp and the signs behind the wait (3584 x 3584 8.8 -> 8.4, with the order of the fragments 9.7 -> 8.4; eight rows 12.0 -> 8.7).
 template <int CHUNKS>
 __global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __restrict__ x, uint32_t* __restrict__ pairs, float* __restrict__ xscale,
                                                             int in, int batch, int block, uint32_t seed_p, uint32_t seed_r, float inv_sqrt,
                                                             int aligned) {
     grid_launch_dependents();
-    grid_dependency_sync();
-    const int lane = threadIdx.x & 31;
+    __shared__ __align__(16) float4 s_give[4][CHUNKS][32];   // the half of a lane's columns that the other warp writes
+    __shared__ unsigned int s_top[4][CHUNKS];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, plane = wib & 1;
     const int slices = (in + kSlice - 1) / kSlice, groups_per_row = (in + 256 * CHUNKS - 1) / (256 * CHUNKS);
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= batch * groups_per_row) return;
-    const int row = warp / groups_per_row, col = (warp - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
-    const unsigned live = __ballot_sync(0xffffffffu, col < in);   // the lanes that exchange values
-    if (col >= in) return;   // a trailing group of less than 256 columns: whole WHT blocks, whole lanes
+    const int item = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 6);
+    const int row = item / groups_per_row, col = (item - row * groups_per_row) * 256 * CHUNKS + 8 * lane;
+    const bool have = row < batch && col < in;   // (a trailing group of less than 256 columns: whole WHT blocks, whole lanes)
+    const unsigned live = __ballot_sync(0xffffffffu, have);   // the lanes that exchange values
+    uint4 signs[CHUNKS];
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(plane ? seed_r : seed_p, static_cast<uint32_t>(col + 256 * c), block);
+    uint32_t* const dst = pairs + fragment_place(in, padded_rows(batch), row, col + 4 * plane);
+    const int chunk = 256 * padded_rows(batch);
+    grid_dependency_sync();
     behind_wait(x);
-    const __half* const src = x + static_cast<size_t>(row) * in + col;
-    uint4 raw[CHUNKS];
-    if (aligned) {
+    float v[CHUNKS][8];
+    if (have) {
+        const __half* const src = x + static_cast<size_t>(row) * in + col;
+        uint4 raw[CHUNKS];
+        if (aligned) {
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
-    } else {
-        const unsigned short* const h = reinterpret_cast<const unsigned short*>(src);
+            for (int c = 0; c < CHUNKS; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + 256 * c);
+        } else {
+            const unsigned short* const h = reinterpret_cast<const unsigned short*>(src);
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) {
-            uint32_t w[4];
+            for (int c = 0; c < CHUNKS; ++c) {
+                uint32_t w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = h[256 * c + 2 * j] | (static_cast<uint32_t>(h[256 * c + 2 * j + 1]) << 16);
-            raw[c] = make_uint4(w[0], w[1], w[2], w[3]);
+                for (int j = 0; j < 4; ++j) w[j] = h[256 * c + 2 * j] | (static_cast<uint32_t>(h[256 * c + 2 * j + 1]) << 16);
+                raw[c] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
         }
-    }
-    float v[2][CHUNKS][8];
 #pragma unroll
-    for (int plane = 0; plane < 2; ++plane) {
-        const uint32_t seed = plane ? seed_r : seed_p;
-#pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[plane][c], raw[c], chunk_signs(seed, static_cast<uint32_t>(col + 256 * c), block), block, lane, live);
+        for (int c = 0; c < CHUNKS; ++c) rotate_chunk(v[c], raw[c], signs[c], block, lane, live);
 #pragma unroll
         for (int h = 1; h < CHUNKS; h <<= 1)
 #pragma unroll
@@ -242,35 +275,42 @@ __global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __rest
                 for (int c = i; c < i + h; ++c)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float a = v[plane][c][j], b = v[plane][c + h][j];
-                        v[plane][c][j] = __fadd_rn(a, b);
-                        v[plane][c + h][j] = __fsub_rn(a, b);
+                        const float a = v[c][j], b = v[c + h][j];
+                        v[c][j] = __fadd_rn(a, b);
+                        v[c + h][j] = __fsub_rn(a, b);
                     }
-    }
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c) {
-        unsigned int top = 0;
-#pragma unroll
-        for (int plane = 0; plane < 2; ++plane)
+        for (int c = 0; c < CHUNKS; ++c) {
+            unsigned int top = 0;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                v[plane][c][j] = to_tf32(v[plane][c][j] * inv_sqrt);
-                top = max(top, __float_as_uint(v[plane][c][j]) & 0x7fffffffu);
+                v[c][j] = to_tf32(v[c][j] * inv_sqrt);
+                top = max(top, __float_as_uint(v[c][j]) & 0x7fffffffu);
             }
+            top = __reduce_max_sync(live, top);
+            if (lane == 0) s_top[wib][c] = top;
+            s_give[wib][c][lane] = plane ? make_float4(v[c][0], v[c][1], v[c][2], v[c][3]) : make_float4(v[c][4], v[c][5], v[c][6], v[c][7]);
+        }
+    }
+    __syncthreads();
+    if (!have) return;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
         // 2^(14 - exponent), between 2^-113 and 2^126 (its inverse is a normal number); 1 beside an infinity or a NaN
-        const unsigned int e = __reduce_max_sync(live, top) >> 23;
+        const unsigned int e = max(s_top[wib][c], s_top[wib ^ 1][c]) >> 23;
         const unsigned int f = e == 255u ? 127u : min(268u - e, 253u);
         const float up = __uint_as_float(f << 23);
-        uint32_t w[8];
+        const float4 got = s_give[wib ^ 1][c][lane];
+        const float other[4] = {got.x, got.y, got.z, got.w};
+        uint32_t w[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const __half2 h = __floats2half2_rn(v[0][c][j] * up, v[1][c][j] * up);
+        for (int j = 0; j < 4; ++j) {   // the warp of the primary seed writes the lower four columns, the other the upper four
+            const float mine = plane ? v[c][4 + j] : v[c][j];
+            const __half2 h = plane ? __floats2half2_rn(other[j] * up, mine * up) : __floats2half2_rn(mine * up, other[j] * up);
             w[j] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        uint4* const dst = reinterpret_cast<uint4*>(pairs + static_cast<size_t>(row) * in + col + 256 * c);
-        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        if (lane == 0) xscale[row * slices + col / kSlice + c] = __uint_as_float((254u - f) << 23);
+        *reinterpret_cast<uint4*>(dst + c * chunk) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (lane == 0 && plane == 0) xscale[row * slices + col / kSlice + c] = __uint_as_float((254u - f) << 23);
     }
 }
 
@@ -278,7 +318,7 @@ struct GemvArgs {
     const uint8_t* codes;   // joint bytes in 16 x 64 tiles (code_offset)
     const float* norms;     // [out]
     const float* table;     // [256] fp32; two rotations: [256] pairs of fp16
-    const float* xrot;      // [batch, in] fp32 (TF32-rounded), used when x == nullptr; two rotations: pairs of fp16
+    const float* xrot;      // [batch, in] fp32 (TF32-rounded) in fragment_place order, used when x == nullptr; two rotations: pairs of fp16
     const float* xscale;    // two rotations: [8, ceil(in / 256)] what the pairs of a row's 256 columns are to be multiplied by
     const __half* x;        // [batch, in] fp16: rotate inside the kernel (WHT block <= 256), else nullptr
     __half* y;              // [batch, y_stride]: row r of activation row n at y[n * y_stride + r]
@@ -601,6 +641,13 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
 #pragma unroll
     for (int k = 0; k < 4; ++k) tab_first[k] = __ldg(p.table + (tid >> 3) + 64 * k);
 
+    // The signs of a row that is rotated in here (a slice is a multiple of the block: the same for all).  A kernel of two units and more waits long enough to
+    // have them first (3584 x 3584 7.3 -> 7.15 us, 5120 x 5120 16.0 -> 15.5); one of a unit follows the kernel before it so soon that they are made while the
+    // row's loads are on their way (2048 x 4096 5.5, in front 5.8).
+    uint4 row_signs = make_uint4(0, 0, 0, 0);
+    constexpr bool kMayRotate = ROW || (BP == 1 && !DUAL);
+    if (kMayRotate && n_local > 1) row_signs = chunk_signs(p.seed_p, static_cast<uint32_t>(8 * lane), p.block);
+
     // Everything below reads or writes data the preceding kernels produce or still use.
     grid_dependency_sync();
     if constexpr (SCATTER) {
@@ -633,6 +680,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     if (ROW || (!DUAL && p.x != nullptr)) {
         const int cl0 = (MULTI ? cur.slot * chunk_cols : 0) + slice0 + 8 * lane;
         if (cl0 < p.in) x_first = load_x(cl0);
+        if (n_local <= 1) row_signs = chunk_signs(p.seed_p, static_cast<uint32_t>(8 * lane), p.block);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -766,41 +814,15 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 // exchanges (same add tree as rotate_x_kernel).  A 1 KB strip of shared memory per warp turns the
                 // result into the fragment layout.  Every lane loads the row's fragment, so B columns 1..7 repeat
                 // column 0 and their results are never read: nothing to clear.
-                const uint32_t seed = p.seed_p;
                 const int cl = colw + 8 * lane;
                 uint4 xc = x0;
                 if (!have_x0) {
                     xc = make_uint4(0, 0, 0, 0);
                     if (cl < p.in) xc = load_x(cl);
                 }
-                const uint32_t xw[4] = {xc.x, xc.y, xc.z, xc.w};
                 float v[8];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const __half2 h2 = *reinterpret_cast<const __half2*>(&xw[j]);
-                    const float lo = __low2float(h2), hi = __high2float(h2);
-                    v[2 * j] = sign_is_positive(seed, static_cast<uint32_t>((8 * lane + 2 * j) & (p.block - 1))) ? lo : -lo;
-                    v[2 * j + 1] = sign_is_positive(seed, static_cast<uint32_t>((8 * lane + 2 * j + 1) & (p.block - 1))) ? hi : -hi;
-                }
-#pragma unroll
-                for (int h = 1; h < 8; h <<= 1)
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2 * h)
-#pragma unroll
-                        for (int j = i; j < i + h; ++j) {
-                            const float a = v[j], b = v[j + h];
-                            v[j] = __fadd_rn(a, b);
-                            v[j + h] = __fsub_rn(a, b);
-                        }
-                const int lane_steps = p.block >> 3;  // lanes per WHT block
-                for (int m = 1; m < lane_steps; m <<= 1) {
-                    const bool upper = (lane & m) != 0;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float o = __shfl_xor_sync(0xffffffffu, v[j], m);
-                        v[j] = upper ? __fsub_rn(o, v[j]) : __fadd_rn(v[j], o);
-                    }
-                }
+                const uint4 sg = MULTI && !have_x0 ? chunk_signs(p.seed_p, static_cast<uint32_t>(8 * lane), p.block) : row_signs;
+                rotate_chunk(v, xc, sg, p.block, lane, 0xffffffffu);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) v[j] = to_tf32(v[j] * p.inv_sqrt_block);
                 sts_v4(strip_addr + static_cast<uint32_t>(lane) * 32u, v[0], v[1], v[2], v[3]);
@@ -815,7 +837,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                                      : "r"(strip_addr + static_cast<uint32_t>(64 * s + 16 * q + k) * 4u));
                 __syncwarp();
             } else {
-            const float* xr = p.xrot + static_cast<size_t>(g) * p.in + col0;
+            const float* xr = p.xrot + static_cast<size_t>(colw) * BP + q * 4;
             if constexpr (DUAL) {
                 const int slices = (p.in + kSlice - 1) / kSlice;
 #pragma unroll
@@ -828,9 +850,10 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const bool ok = have_row && (col0 + 64 * s) < p.in;
+                const int groups4 = colw + 64 * s + 64 <= p.in ? 16 : 8;   // 4 fragment_groups
 #pragma unroll
                 for (int k = 0; k < 16; k += 4) {
-                    const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * s + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * BP * s + (k / 4 * BP + g) * groups4) : make_float4(0.f, 0.f, 0.f, 0.f);
                     bfrag[s][k] = __float_as_uint(t.x);
                     bfrag[s][k + 1] = __float_as_uint(t.y);
                     bfrag[s][k + 2] = __float_as_uint(t.z);
@@ -1270,7 +1293,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
         TQ_CUDA(cudaGetLastError());
     }
     if (n_planes == 2) launch_rotate_x_pair(x, xrot, in, batch, block, seed_p, seed_r, stream);
-    else if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, 1, seed_p, seed_r, stream);
+    else if (!fused_rotation) launch_rotate_x(x, xrot, in, batch, block, 1, seed_p, seed_r, stream, true);
     // 2. the GEMV itself
     {
         const int n_units = a.n_row_units * a.n_slots;
@@ -1433,7 +1456,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
         if (!fused[i]) {
             float* const xrot = const_cast<float*>(grp.m[i].xrot);
             if (items[i].n_planes == 2) launch_rotate_x_pair(x, xrot, items[i].in, batch, items[i].block, items[i].seed_p, items[i].seed_r, stream);
-            else launch_rotate_x(x, xrot, items[i].in, batch, items[i].block, 1, items[i].seed_p, items[i].seed_r, stream);
+            else launch_rotate_x(x, xrot, items[i].in, batch, items[i].block, 1, items[i].seed_p, items[i].seed_r, stream, true);
         }
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1467,7 +1490,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
 // The activation rotation alone (the pre-kernel of several rows or WHT blocks above 256 columns), also for the other decode
 // kernels: xrot = [n_planes, batch, in] fp32.
 void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
-                     uint32_t seed_r, cudaStream_t stream) {
+                     uint32_t seed_r, cudaStream_t stream, bool fragments) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1482,14 +1505,14 @@ void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t b
         auto* const wide = wide_cols == 256 ? rotate_x_wide_kernel<1> : (wide_cols == 512 ? rotate_x_wide_kernel<2> : rotate_x_wide_kernel<4>);
         cfg.gridDim = dim3((n_planes * batch * ((in + wide_cols - 1) / wide_cols) + 3) / 4);
         cfg.dynamicSmemBytes = kRotateXSmem;
-        TQ_CUDA(cudaLaunchKernelEx(&cfg, wide, x, xrot, in, batch, n_planes, static_cast<int>(block), seed_p, seed_r, inv_sqrt));
+        TQ_CUDA(cudaLaunchKernelEx(&cfg, wide, x, xrot, in, batch, n_planes, static_cast<int>(block), seed_p, seed_r, inv_sqrt, fragments ? padded_rows(batch) : 0));
         return;
     }
     const int n_warps = n_planes * batch * (in / static_cast<int>(block));
     cfg.gridDim = dim3((n_warps + 3) / 4);
 #define TQ_ROT_CASE(EV)                                                                                            \
     case 32 * EV:                                                                                                  \
-        TQ_CUDA(cudaLaunchKernelEx(&cfg, rotate_x_kernel<EV>, x, xrot, in, batch, n_planes, seed_p, seed_r, inv_sqrt)); \
+        TQ_CUDA(cudaLaunchKernelEx(&cfg, rotate_x_kernel<EV>, x, xrot, in, batch, n_planes, seed_p, seed_r, inv_sqrt, fragments ? padded_rows(batch) : 0)); \
         break;
     switch (block) {
         TQ_ROT_CASE(1) TQ_ROT_CASE(2) TQ_ROT_CASE(4) TQ_ROT_CASE(8) TQ_ROT_CASE(16) TQ_ROT_CASE(32)
@@ -1504,7 +1527,7 @@ static void launch_rotate_x_pair(const __half* x, float* xrot, int in, int batch
                                  cudaStream_t stream) {
     const int wide_cols = block <= 256 ? 256 : static_cast<int>(block);
     auto* const kernel = wide_cols == 256 ? rotate_x_pair_kernel<1> : (wide_cols == 512 ? rotate_x_pair_kernel<2> : rotate_x_pair_kernel<4>);
-    launch_pdl(kernel, dim3((batch * ((in + wide_cols - 1) / wide_cols) + 3) / 4), dim3(128), kRotateXSmem, stream, x,
+    launch_pdl(kernel, dim3((2 * batch * ((in + wide_cols - 1) / wide_cols) + 3) / 4), dim3(128), kRotatePairSmem, stream, x,
                reinterpret_cast<uint32_t*>(xrot), xrot + static_cast<size_t>(8) * in, in, batch, static_cast<int>(block), seed_p, seed_r,
                1.0f / std::sqrt(static_cast<float>(block)), reinterpret_cast<uintptr_t>(x) % 16 == 0 ? 1 : 0);
 }

@@ -757,7 +757,7 @@ void launch_tq8_gemv_staged(const uint8_t* codes, const float* norms, const floa
     a.x = x;
     a.xrot = nullptr;
     if (!fused_rotation) {
-        launch_rotate_x(x, xrot, in, batch, block, n_planes, seed_p, seed_r, stream);
+        launch_rotate_x(x, xrot, in, batch, block, n_planes, seed_p, seed_r, stream, false);
         a.xrot = xrot;
     }
 

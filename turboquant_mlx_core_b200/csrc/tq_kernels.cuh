@@ -107,9 +107,10 @@ void launch_tq8_gemv_staged_static(const uint8_t* codes, const float* norms, con
                                    int out, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p, uint32_t seed_r,
                                    unsigned int* status, int sm_count, cudaStream_t stream);
 void* gemv_static_scratch_address();   // device address of that array on the current device (tq_gemv.cu)
-// The activation rotation of tq_gemv.cu alone: xrot = [n_planes, batch, in] fp32 (TF32-rounded).
+// The activation rotation of tq_gemv.cu alone: xrot = [n_planes, batch, in] fp32 (TF32-rounded).  `fragments` (one plane): in the order
+// in which tq8_gemv_kernel reads it.
 void launch_rotate_x(const __half* x, float* xrot, int in, int batch, uint32_t block, int n_planes, uint32_t seed_p,
-                     uint32_t seed_r, cudaStream_t stream);
+                     uint32_t seed_r, cudaStream_t stream, bool fragments);
 
 // Allocation-free variant: scratch is a fixed array in the library image
 // (gemv_static_scratch_capacity() bytes); throws if the layer needs more.
