@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(GROUPS == 1 ? 384 : gemm_threads(kGroupsMax), 
 // CTAs are there before these end, and let those of the next call's rotation come in turn.  64 registers: eight CTAs to an SM, one or two beside a
 // product's.  With 126 (all sums of twelve splits at once) 8192 x 1024 in 16 splits took 11.2 us at 32 rows instead of 8.6, 2048 x 2048 at 512 rows 19.2 instead of 16.2;
 // as few CTAs as SMs, with several rows each, crowd on a few of them (3584 x 3584 at 64 rows 12.2 -> 15.0).  Behind a product that fills the SMs four CTAs to an SM
-// spread better (18944 x 3584 at 64 rows 25.1 us, 25.6 with eight): 126 registers there.
+// spread better (18944 x 3584 at 64 rows 25.1 us, 25.6 with eight).
 struct FinishOne {
     const float* partial;
     const float* norms;
@@ -970,6 +970,11 @@ struct Sums {
             v[0] = t.x; v[1] = t.y;
         }
     }
+    // Rows that are not whole pieces: the first n of them.
+    __device__ __forceinline__ void load_some(const float* p, int n) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = k < n ? __ldcg(p + k) : 0.f;
+    }
 };
 // V = 4, or 2 where more than eight splits are to be asked for at once.
 template <int kBatch, int V>
@@ -992,19 +997,25 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool
         float acc[V];
 #pragma unroll
         for (int k = 0; k < V; ++k) acc[k] = 0.f;
-        if (f.vec) {
-            for (int z0 = 0; z0 < k_splits; z0 += kBatch) {
-                Sums<V> v[kBatch];
+        for (int z0 = 0; z0 < k_splits; z0 += kBatch) {
+            Sums<V> v[kBatch];
+            if (f.vec) {
 #pragma unroll
                 for (int z = 0; z < kBatch; ++z)
                     if (z0 + z < k_splits) v[z].load(src + (z0 + z) * split);
+            } else {
 #pragma unroll
                 for (int z = 0; z < kBatch; ++z)
-                    if (z0 + z < k_splits) {
-#pragma unroll
-                        for (int k = 0; k < V; ++k) acc[k] += v[z].v[k];
-                    }
+                    if (z0 + z < k_splits) v[z].load_some(src + (z0 + z) * split, out - c);
             }
+#pragma unroll
+            for (int z = 0; z < kBatch; ++z)
+                if (z0 + z < k_splits) {
+#pragma unroll
+                    for (int k = 0; k < V; ++k) acc[k] += v[z].v[k];
+                }
+        }
+        if (f.vec) {
             uint32_t h[V / 2];
 #pragma unroll
             for (int k = 0; k < V; k += 2) {
@@ -1014,10 +1025,6 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool
             if constexpr (V == 4) *reinterpret_cast<uint2*>(y) = make_uint2(h[0], h[1]);
             else *reinterpret_cast<uint32_t*>(y) = h[0];
         } else {
-            for (int z = 0; z < k_splits; ++z)
-#pragma unroll
-                for (int k = 0; k < V; ++k)
-                    if (c + k < out) acc[k] += __ldcg(src + z * split + k);
 #pragma unroll
             for (int k = 0; k < V; ++k)
                 if (c + k < out) y[k] = __float2half_rn(acc[k] * (norm[k] * f.inv_scale));
@@ -1029,6 +1036,7 @@ template <int BATCH, int V>
 __global__ void __launch_bounds__(kFinishThreads, BATCH * V == 32 ? 8 : 0) gemm_finish_kernel(const __grid_constant__ FinishOne f, int m, bool early) { gemm_finish_body<BATCH, V>(f, m, early); }
 template <int BATCH, int V>
 __global__ void __launch_bounds__(kFinishThreads, BATCH * V == 32 ? 8 : 0) gemm_finish_group_kernel(const __grid_constant__ FinishArgs f, int m, bool early) { gemm_finish_body<BATCH, V>(f.m[blockIdx.z], m, early); }
+constexpr size_t kFourCtas = 48 * 1024;   // shared memory that is asked for and not used: so many CTAs to an SM
 void finish_add(FinishArgs& f, int& n, const GemmArgs& a) {
     if (a.k_splits <= 1) return;
     f.m[n] = FinishOne{a.partial, a.norms, a.y, a.y_stride, a.out, a.k_splits,
@@ -1047,7 +1055,7 @@ void launch_finish(const FinishArgs& f, int n, int m, int groups, int sm_count, 
     const int gx = (widest + v * kFinishThreads - 1) / (v * kFinishThreads);
     const int gy = std::max(1, std::min(m, 16 * sm_count / (gx * n)));   // up to sixteen CTAs per SM
     const dim3 grid(static_cast<unsigned int>(gx), static_cast<unsigned int>(gy), static_cast<unsigned int>(n));
-    if (n == 1) launch_pdl_carved(!few ? gemm_finish_kernel<12, 4> : v == 4 ? gemm_finish_kernel<8, 4> : gemm_finish_kernel<16, 2>, grid, dim3(kFinishThreads), 0, carveout, stream, f.m[0], m, few);
+    if (n == 1) launch_pdl_carved(!few ? gemm_finish_kernel<12, 4> : v == 4 ? gemm_finish_kernel<8, 4> : gemm_finish_kernel<16, 2>, grid, dim3(kFinishThreads), few ? 0 : kFourCtas, carveout, stream, f.m[0], m, few);
     else launch_pdl_carved(v == 4 ? gemm_finish_group_kernel<8, 4> : gemm_finish_group_kernel<16, 2>, grid, dim3(kFinishThreads), 0, carveout, stream, f, m, few);
 }
 

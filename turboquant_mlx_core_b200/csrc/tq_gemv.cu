@@ -106,19 +106,24 @@ __device__ __forceinline__ uint32_t lut_addr(uint32_t word, uint32_t lane_const)
 }
 
 // ---- activation rotation ---------------------------------------------------------------------
-// Where word (row, col) of a rotated activation stands when the decode kernel is to read it: in the order of its B fragments.  A load of a
-// warp is 16 bytes of every lane (g = row, q = 16 columns of a 64-column block): blocks of [4 pieces of 4 columns][bp rows][16-column groups q][4], bp the
-// rows rounded up to 1, 2, 4 or 8.  Row after row, those 16 bytes lay in as many lines as there were lanes, and every CTA spent more time on its 128 KB
-// of activations than on a unit of codes: 4096 x 4096 at eight rows 9.6 -> 8.2 us, 3584 x 3584 with two rotations at eight
-// 12.0 -> 9.4, 18944 x 3584 at four 24.5 -> 23.7, 27648 x 5120 at eight 46.2 -> 44.3.  (in is a multiple of 32: a last block of 32 columns has two groups q.)
+// Where word (row, col) of a rotated activation stands when the decode kernel is to read it: in the order of its B fragments, bp the rows rounded
+// up to 1, 4 or 8.  A product takes two columns (2 m and the next) of every 16-column group q of a 64-column block; its eight B columns are
+// the bp rows for 8 / bp products m side by side (m = (8 / bp) jj + m', B column g = m' bp + row).  So lane (g, q) has 2 bp words of a block, words 2 jj and the next, and
+// they come in pieces of four (two with one row), a piece of all lanes side by side.  Row after row, the 16 bytes of every lane lay in a line of their own, and
+// every CTA spent more time on its 128 KB of activations than on a unit of codes: 4096 x 4096 at eight rows 9.6 -> 8.2 us, 3584 x 3584 with two
+// rotations at eight 12.0 -> 9.4, 18944 x 3584 at four 24.5 -> 23.7, 27648 x 5120 at eight 46.2 -> 44.3.  (in is a multiple of 32: a last block of 32 columns has two groups q.)
 __host__ __device__ __forceinline__ int fragment_groups(int in, int col) {
     const int left = (in - (col & ~63)) >> 4;
     return left < 4 ? left : 4;
 }
+__host__ __device__ __forceinline__ int row_bits(int bp) { return bp >= 8 ? 3 : bp >> 1; }   // log2
 __host__ __device__ __forceinline__ size_t fragment_place(int in, int bp, int row, int col) {
-    return static_cast<size_t>(col >> 6) * (64 * bp) + static_cast<size_t>(((((col & 15) >> 2) * bp + row) * fragment_groups(in, col) + ((col & 63) >> 4)) * 4 + (col & 3));
+    const int m = (col & 15) >> 1, jj = m >> (3 - row_bits(bp)), g = ((m & (8 / bp - 1)) << row_bits(bp)) + row, r = 2 * jj + (col & 1);
+    const int groups = fragment_groups(in, col), lane = g * groups + ((col & 63) >> 4);
+    return static_cast<size_t>(col >> 6) * (64 * bp) + static_cast<size_t>(bp == 1 ? 2 * lane + r : ((r >> 2) * 8 * groups + lane) * 4 + (r & 3));
 }
-__host__ __device__ __forceinline__ constexpr int padded_rows(int batch) { return batch <= 1 ? 1 : batch <= 2 ? 2 : batch <= 4 ? 4 : 8; }
+// (Two rows as a kernel of their own, four products side by side: 2048 x 151936 81 us instead of 67.)
+__host__ __device__ __forceinline__ constexpr int padded_rows(int batch) { return batch <= 1 ? 1 : batch <= 4 ? 4 : 8; }
 // One warp per (plane, batch row, WHT block): xrot = FWHT(sign o x) / sqrt(bs), rounded to
 // TF32 and stored as fp32, [plane][row][in] or (fragments: the padded rows; one plane) in the decode kernel's order.
 template <int E>
@@ -175,16 +180,14 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
     // the loads, behind which they are made: in front, 4096 x 4096, block 512, took 8.8 us at one row instead of 8.3, 1024 x 1024 6.4 instead of 5.9.
     uint4 signs;
     if (CHUNKS == 1) signs = chunk_signs(seed, static_cast<uint32_t>(col), block);
-    // A lane's eight columns are four and four: in the order of the fragments a piece apart, 256 columns on at 256 words a row.  (Their places in front
-    // of the wait, those of several chunks beside the loads, like the signs: 4096 x 4096, block 512, one row 8.2 us, in front 8.5.)
-    float* dst = xrot;
-    int half = 4, chunk = 256;
+    // A lane's eight columns go out in pairs, 256 columns on at 256 words a row.  (Their places in front of the wait, those of several chunks beside the
+    // loads, like the signs: 4096 x 4096, block 512, one row 8.2 us, in front 8.5.)
+    float* dst[4];
+    const int chunk = fragments ? 256 * fragments : 256;
     auto find_place = [&] {
-        dst += fragments ? fragment_place(in, fragments, row, col) : (static_cast<size_t>(plane) * batch + row) * in + col;
-        if (fragments) {
-            half = 4 * fragments * fragment_groups(in, col);
-            chunk = 256 * fragments;
-        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            dst[i] = xrot + (fragments ? fragment_place(in, fragments, row, col + 2 * i) : (static_cast<size_t>(plane) * batch + row) * in + col + 2 * i);
     };
     if (CHUNKS == 1) find_place();
     grid_dependency_sync();
@@ -215,9 +218,8 @@ __global__ void __launch_bounds__(128) rotate_x_wide_kernel(const __half* __rest
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c)
 #pragma unroll
-        for (int j = 0; j < 8; j += 4)
-            *reinterpret_cast<float4*>(dst + c * chunk + j / 4 * half) =
-                make_float4(to_tf32(v[c][j] * inv_sqrt), to_tf32(v[c][j + 1] * inv_sqrt), to_tf32(v[c][j + 2] * inv_sqrt), to_tf32(v[c][j + 3] * inv_sqrt));
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float2*>(dst[i] + c * chunk) = make_float2(to_tf32(v[c][2 * i] * inv_sqrt), to_tf32(v[c][2 * i + 1] * inv_sqrt));
 }
 constexpr size_t kRotateXSmem = 48 * 1024, kRotatePairSmem = 38 * 1024;
 
@@ -244,7 +246,9 @@ __global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __rest
     uint4 signs[CHUNKS];
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) signs[c] = chunk_signs(plane ? seed_r : seed_p, static_cast<uint32_t>(col + 256 * c), block);
-    uint32_t* const dst = pairs + fragment_place(in, padded_rows(batch), row, col + 4 * plane);
+    uint32_t* dst[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) dst[i] = pairs + fragment_place(in, padded_rows(batch), row, col + 4 * plane + 2 * i);
     const int chunk = 256 * padded_rows(batch);
     grid_dependency_sync();
     behind_wait(x);
@@ -309,7 +313,8 @@ __global__ void __launch_bounds__(128) rotate_x_pair_kernel(const __half* __rest
             const __half2 h = plane ? __floats2half2_rn(other[j] * up, mine * up) : __floats2half2_rn(mine * up, other[j] * up);
             w[j] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        *reinterpret_cast<uint4*>(dst + c * chunk) = make_uint4(w[0], w[1], w[2], w[3]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<uint2*>(dst[i] + c * chunk) = make_uint2(w[2 * i], w[2 * i + 1]);
         if (lane == 0 && plane == 0) xscale[row * slices + col / kSlice + c] = __uint_as_float((254u - f) << 23);
     }
 }
@@ -499,13 +504,14 @@ __device__ __forceinline__ void ll_send_packets(const ScatterArgs& sc, const __h
     }
 }
 
-// BP = activation rows padded to 1, 2, 4 or 8 (compile time, so that the partial-sum ring
+// BP = activation rows padded to 1, 4 or 8 (compile time, so that the partial-sum ring
 // geometry and the reduction need no runtime arithmetic).
 // MULTI = more than one slot (row units finished through partial sums in scratch); compile time, so that the
 // single-slot kernels carry none of that path's state in their 128 registers.
 // DUAL = weights with two rotations: table words and activation words are pairs of fp16.
 // ROW = the activation row is a kernel parameter, `row` its generic address.
-template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false>
+// DEEP = all four steps of a unit's codes in registers, not two (one activation row, many units a CTA).
+template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false, bool DEEP = false>
 __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk, const __half* row = nullptr) {
     auto load_x = [&](int col) {   // eight columns of the row that is rotated in here
         if constexpr (ROW) return *reinterpret_cast<const uint4*>(row + col);
@@ -522,6 +528,8 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     constexpr int kLag = kRing / 2;                       // how many units behind the sums run
     constexpr uint32_t kSlotBytes = kWarps * kTileFloats * 4;  // one ring slot: [warp][16 rows][BP] floats (+ padding)
     constexpr int kPer = BP >= 2 ? BP / 2 : 1;            // floats a lane adds in the reduction
+    constexpr int kSide = 8 / BP, kAcc = kSide < 2 ? 2 : kSide;   // products side by side in the B columns; accumulators
+    constexpr int kSteps = DEEP ? 4 : 2;                  // steps of codes in registers
 
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ unsigned int s_abort;
@@ -609,12 +617,11 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     };
     Pos cur = make_pos(u_begin);
     Pos nxt = (n_local > 1) ? next_pos(cur) : cur;
-    // Two register buffers (even / odd step): two steps, 32 KB per SM, in flight.  Four buffers
-    // were measured and bought nothing: the kernel is bound by L1 data-pipe wavefronts (table
-    // lookups plus the code loads), not by the depth of the load queue.
-    uint4 blo[2], bhi[2];
+    // Two register buffers (even / odd step): two steps, 32 KB per SM, in flight.  (Four for one row and many units a CTA, see the launch; several rows are
+    // bound by L1 data-pipe wavefronts, table lookups plus the code loads, and gain nothing from more.)
+    uint4 blo[kSteps], bhi[kSteps];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kSteps; ++s) {
         blo[s] = make_uint4(0, 0, 0, 0);
         bhi[s] = make_uint4(0, 0, 0, 0);
         load_step(cur, s, true, blo[s], bhi[s]);
@@ -792,7 +799,10 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             if (pend == kFlushUnits || ru + 1 == p.n_row_units) flush_pending(ru);
         }
     };
-    uint32_t bfrag[4][16];
+    // B fragments.  bp rows fill bp of a product's eight columns: so the columns are 8 / bp products' pieces of the rows side by side (fragment_place), each of
+    // those products has an accumulator, and only its own columns of it count.  With a fragment per product, 64 registers whatever the rows and zero columns for those that
+    // are missing, fewer lookups were in flight: one row, 4096 x 4096 7.5 -> 6.3 us, 1024 x 1024 5.0 -> 4.0, 18944 x 3584 24.0 -> 22.5.
+    uint32_t bfrag[4][2 * BP];
     int staged_slot = -1;
     // ring bookkeeping: slot / parity for the unit being written and the unit being summed
     int ws = 0;             // write slot = i % kRing
@@ -805,15 +815,14 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     // caller has already requested it (have_x0).
     float xs[2];   // two rotations: the scales of activation rows 2q and 2q + 1 in this warp's slice
     auto stage_slot = [&](int slot, const uint4& x0, bool have_x0) {
-            // B fragment of MMA (s, m): k = q -> column 64 s + 16 q + 2 m, k = q+4 -> the next column; n = g.
+            // B fragment of MMA (s, m): k = q -> column 64 s + 16 q + 2 m, k = q+4 -> the next column; n = g: row and product (see bfrag).
             const int colw = (MULTI ? slot * chunk_cols : 0) + slice0;  // first column of this warp's slice
             const int col0 = colw + 16 * q;
             if (ROW || (BP == 1 && !DUAL && p.x != nullptr)) {
                 // One activation row (the launcher rotates in here only then): rotate this warp's 256 columns of it.
                 // Lane l holds columns 8l..8l+7 of the slice, stages below 8 stay in the lane, the rest are lane
                 // exchanges (same add tree as rotate_x_kernel).  A 1 KB strip of shared memory per warp turns the
-                // result into the fragment layout.  Every lane loads the row's fragment, so B columns 1..7 repeat
-                // column 0 and their results are never read: nothing to clear.
+                // result into the fragment layout.
                 const int cl = colw + 8 * lane;
                 uint4 xc = x0;
                 if (!have_x0) {
@@ -830,14 +839,12 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 __syncwarp();
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
-#pragma unroll
-                    for (int k = 0; k < 16; k += 4)
-                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                                     : "=r"(bfrag[s][k]), "=r"(bfrag[s][k + 1]), "=r"(bfrag[s][k + 2]), "=r"(bfrag[s][k + 3])
-                                     : "r"(strip_addr + static_cast<uint32_t>(64 * s + 16 * q + k) * 4u));
+                    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];"
+                                 : "=r"(bfrag[s][0]), "=r"(bfrag[s][1])
+                                 : "r"(strip_addr + static_cast<uint32_t>(64 * s + 16 * q + 2 * g) * 4u));
                 __syncwarp();
             } else {
-            const float* xr = p.xrot + static_cast<size_t>(colw) * BP + q * 4;
+            const float* xr = p.xrot + static_cast<size_t>(colw) * BP;
             if constexpr (DUAL) {
                 const int slices = (p.in + kSlice - 1) / kSlice;
 #pragma unroll
@@ -846,18 +853,24 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                     xs[k] = (n < BP && n < p.batch && colw < p.in) ? p.xscale[n * slices + colw / kSlice] : 0.f;
                 }
             }
-            const bool have_row = g < p.batch;
+            const bool have_row = (g & (BP - 1)) < p.batch;
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const bool ok = have_row && (col0 + 64 * s) < p.in;
-                const int groups4 = colw + 64 * s + 64 <= p.in ? 16 : 8;   // 4 fragment_groups
+                const int groups = colw + 64 * s + 64 <= p.in ? 4 : 2;   // fragment_groups
+                if constexpr (BP == 1) {
+                    const float2 t = ok ? *reinterpret_cast<const float2*>(xr + 64 * s + 2 * (g * groups + q)) : make_float2(0.f, 0.f);
+                    bfrag[s][0] = __float_as_uint(t.x);
+                    bfrag[s][1] = __float_as_uint(t.y);
+                } else {
 #pragma unroll
-                for (int k = 0; k < 16; k += 4) {
-                    const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * BP * s + (k / 4 * BP + g) * groups4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    bfrag[s][k] = __float_as_uint(t.x);
-                    bfrag[s][k + 1] = __float_as_uint(t.y);
-                    bfrag[s][k + 2] = __float_as_uint(t.z);
-                    bfrag[s][k + 3] = __float_as_uint(t.w);
+                    for (int k = 0; k < 2 * BP; k += 4) {
+                        const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * BP * s + (2 * k + g) * groups * 4 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        bfrag[s][k] = __float_as_uint(t.x);
+                        bfrag[s][k + 1] = __float_as_uint(t.y);
+                        bfrag[s][k + 2] = __float_as_uint(t.z);
+                        bfrag[s][k + 3] = __float_as_uint(t.w);
+                    }
                 }
             }
             }
@@ -869,11 +882,17 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         if (cur.slot != staged_slot) stage_slot(cur.slot, make_uint4(0, 0, 0, 0), false);
         const bool has_next = i + 1 < n_local;
 
-        float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[kAcc][4];
+#pragma unroll
+        for (int m = 0; m < kAcc; ++m)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[m][k] = 0.f;
+        float(&acc0)[4] = acc[0];
+        float(&acc1)[4] = acc[1];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            uint4& lo = blo[s & 1];
-            uint4& hi = bhi[s & 1];
+            uint4& lo = blo[s % kSteps];
+            uint4& hi = bhi[s % kSteps];
             // 16 independent lookups, then the 4 MMAs they feed (bytes 0,1 of a word feed one
             // MMA, bytes 2,3 the next); two accumulator chains.  Once the second half's addresses
             // are formed the code registers are free: the step two ahead is loaded into them.
@@ -891,18 +910,17 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 ad[6] = lut_addr<3>(l, lane_const);
                 ad[7] = lut_addr<3>(u, lane_const);
                 if (w == 3) {
-                    if (s < 2) load_step(cur, s + 2, true, lo, hi);
-                    else load_step(nxt, s - 2, has_next, lo, hi);
+                    if (s + kSteps < 4) load_step(cur, (s + kSteps) % 4, true, lo, hi);
+                    else load_step(nxt, (s + kSteps) % 4, has_next, lo, hi);
                 }
                 uint32_t av[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) av[k] = lut_load(ad[k]);
-                if constexpr (DUAL) {
-                    mma_f16(acc0, av[0], av[1], av[2], av[3], bfrag[s][4 * w + 0], bfrag[s][4 * w + 1]);
-                    mma_f16(acc1, av[4], av[5], av[6], av[7], bfrag[s][4 * w + 2], bfrag[s][4 * w + 3]);
-                } else {
-                    mma_tf32(acc0, av[0], av[1], av[2], av[3], bfrag[s][4 * w + 0], bfrag[s][4 * w + 1]);
-                    mma_tf32(acc1, av[4], av[5], av[6], av[7], bfrag[s][4 * w + 2], bfrag[s][4 * w + 3]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int m = 2 * w + h, b = 2 * (m / kSide);
+                    if constexpr (DUAL) mma_f16(acc[m % kAcc], av[4 * h], av[4 * h + 1], av[4 * h + 2], av[4 * h + 3], bfrag[s][b], bfrag[s][b + 1]);
+                    else mma_tf32(acc[m % kAcc], av[4 * h], av[4 * h + 1], av[4 * h + 2], av[4 * h + 3], bfrag[s][b], bfrag[s][b + 1]);
                 }
             }
         }
@@ -926,6 +944,23 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
             // C fragment: (row g, columns 2q, 2q+1) and (row g+8, same columns)
             const uint32_t dst = red_addr + static_cast<uint32_t>(ws) * kSlotBytes + static_cast<uint32_t>(warp * kTileFloats) * 4u;
             const int n = 2 * q;
+            // Lane q has columns 2q and 2q + 1: of accumulator m' those that are rows for product m' count, and the products' sums meet in the lanes of the rows.
+            if constexpr (BP == 1) {
+                float top = q == 0 ? acc[0][0] + acc[1][1] : q == 1 ? acc[2][0] + acc[3][1] : q == 2 ? acc[4][0] + acc[5][1] : acc[6][0] + acc[7][1];
+                float low = q == 0 ? acc[0][2] + acc[1][3] : q == 1 ? acc[2][2] + acc[3][3] : q == 2 ? acc[4][2] + acc[5][3] : acc[6][2] + acc[7][3];
+                top += __shfl_xor_sync(0xffffffffu, top, 1);
+                low += __shfl_xor_sync(0xffffffffu, low, 1);
+                acc0[0] = top + __shfl_xor_sync(0xffffffffu, top, 2);
+                acc0[2] = low + __shfl_xor_sync(0xffffffffu, low, 2);
+                acc1[0] = acc1[2] = 0.f;
+            } else if constexpr (BP == 4) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float v = q < 2 ? acc[0][k] : acc[1][k];
+                    acc0[k] = v + __shfl_xor_sync(0xffffffffu, v, 2);
+                    acc1[k] = 0.f;
+                }
+            }
             if constexpr (DUAL) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -1037,9 +1072,9 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     }
 }
 
-template <int BP, bool MULTI, bool DUAL>
+template <int BP, bool MULTI, bool DUAL, bool DEEP = false>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_kernel(const GemvArgs p) {
-    gemv_body<BP, false, false, MULTI, DUAL>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    gemv_body<BP, false, false, MULTI, DUAL, false, DEEP>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
 }
 // The one activation row of a host caller, which rides in the launch (16 N bytes of fp16): as a kernel of its own in front, which wrote it to
 // device memory, it cost a launch and its end.  4096 x 4096 from and to host memory 31.3 us, 29.7 so, 512 x 14336 39.8 and 33.5.
@@ -1278,7 +1313,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     }
     const bool fused_rotation = fill_gemv_args(a, x, out, in, batch, block, n_planes, pair_unit, seed_p, scratch);
     float* xrot = const_cast<float*>(a.xrot);
-    const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));
+    const int bp = padded_rows(batch);
 
     configure_gemv_kernels();
 
@@ -1304,11 +1339,15 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
         cfg.stream = stream;
         cfg.attrs = attr;
         cfg.numAttrs = n_attr;
+        // One row has the registers for four steps of codes.  They pay from some eight units a CTA on: 2048 x 151936 (32 units) 63.0 -> 61.4 us, 5120 x 55296 70.2 ->
+        // 67.7, 18944 x 3584 (8) 22.6 -> 22.1; before, the first unit comes later: 4096 x 4096 (2) 6.3 -> 6.7, 4096 x 11008 (5) 12.4 -> 12.7.
+        const bool deep = n_units >= 8 * sm_count - sm_count / 2;
         // one destination with the layer's own row stride and no signal: the plain variant
         const bool scatter = sa.n_peer > 0 || sa.n_signal > 0 || sa.ll != 0 || sa.y_stride != a.out;
 #define TQ_GEMV_LAUNCH3(BPV, MV, DV)                                                                  \
     if (sa.ll) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_packets_kernel<BPV, MV, DV>, a, sa));        \
     else if (scatter) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_scatter_kernel<BPV, MV, DV>, a, sa)); \
+    else if (BPV == 1 && deep) TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_kernel<BPV, MV, DV, BPV == 1>, a)); \
     else TQ_CUDA(cudaLaunchKernelEx(&cfg, tq8_gemv_kernel<BPV, MV, DV>, a));
 #define TQ_GEMV_LAUNCH2(BPV, MV)                         \
     if (n_planes == 2) { TQ_GEMV_LAUNCH3(BPV, MV, true) } \
@@ -1318,7 +1357,6 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     else { TQ_GEMV_LAUNCH2(BPV, false) }
         switch (bp) {
             case 1: TQ_GEMV_LAUNCH(1) break;
-            case 2: TQ_GEMV_LAUNCH(2) break;
             case 4: TQ_GEMV_LAUNCH(4) break;
             default: TQ_GEMV_LAUNCH(8) break;
         }
@@ -1397,7 +1435,10 @@ static void configure_gemv_kernels() {
     TQ_GEMV_ATTR2(BPV, false) \
     TQ_GEMV_ATTR2(BPV, true)
     TQ_GEMV_ATTR(1)
-    TQ_GEMV_ATTR(2)
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<1, false, false, true>))
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<1, true, false, true>))
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<1, false, true, true>))
+    TQ_GEMV_ATTR1((tq8_gemv_kernel<1, true, true, true>))
     TQ_GEMV_ATTR(4)
     TQ_GEMV_ATTR(8)
 #undef TQ_GEMV_ATTR
@@ -1468,7 +1509,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));
+    const int bp = padded_rows(batch);
     const bool multi = grp.m[0].n_slots > 1;   // the same for all: same in_features and planes
     const bool dual = items[0].n_planes == 2;
 #define TQ_GROUP_LAUNCH2(BPV, DV)                                                             \
@@ -1479,7 +1520,6 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     else { TQ_GROUP_LAUNCH2(BPV, false) }
     switch (bp) {
         case 1: TQ_GROUP_LAUNCH(1) break;
-        case 2: TQ_GROUP_LAUNCH(2) break;
         case 4: TQ_GROUP_LAUNCH(4) break;
         default: TQ_GROUP_LAUNCH(8) break;
     }
