@@ -260,7 +260,21 @@ __host__ __device__ __forceinline__ int dense_frag_dim(int ks, int c) {
     return 32 * (ks >> 1) + 8 * ((c & 7) >> 1) + 4 * (ks & 1) + 2 * (c >> 3) + (c & 1);
 }
 
-template <typename QT>
+// 16 bytes of the window, which is read once; STREAM: past the first-level cache.  (The pointer comes from behind the wait: the load has nothing else that
+// keeps it there.)  A window that the L2 cache does not hold comes faster without a place made for every line: 131072 tokens of 4 heads
+// 51.7 -> 46.7 us with the combine, 65536 33.4 -> 28.3; one that it may hold does not, 49152 tokens (100 MB) 23.4 and 23.4, 32768 17.8 and 19.0.
+template <bool STREAM>
+__device__ __forceinline__ uint4 load_window(const uint4* p) {
+    if constexpr (STREAM) {
+        uint4 v;
+        asm("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+        return v;
+    } else {
+        return *p;
+    }
+}
+constexpr size_t kStreamBytes = size_t(100) << 20;
+template <typename QT, bool STREAM>
 __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __restrict__ keys, const __half* __restrict__ values,
                                                                 int n_tokens, int kv_heads, int q_heads, const QT* __restrict__ q,
                                                                 int n_splits, float scale, float* __restrict__ part_acc,
@@ -320,13 +334,13 @@ __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __
         uint4 fka[4], fkb[4], fva[4], fvb[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            fka[j] = ka[4 * j];
-            fkb[j] = kb[4 * j];
+            fka[j] = load_window<STREAM>(ka + 4 * j);
+            fkb[j] = load_window<STREAM>(kb + 4 * j);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            fva[j] = xa[4 * j];
-            fvb[j] = xb[4 * j];
+            fva[j] = load_window<STREAM>(xa + 4 * j);
+            fvb[j] = load_window<STREAM>(xb + 4 * j);
         }
         float c1[4] = {0.f, 0.f, 0.f, 0.f}, c1b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -542,12 +556,13 @@ void launch_dense_attention(const __half* keys, const __half* values, int n_toke
                                                                        part_ml);
     static const bool cuda_core_only = std::getenv("TQ_WINDOW_ATTENTION_FMA") != nullptr;   // measurement switch: the fp32-FMA kernel at head_dim 128
     if (head_dim == 128 && !cuda_core_only) {
+        const bool streamed = static_cast<size_t>(n_tokens) * kv_heads * head_dim * 2 * sizeof(__half) > kStreamBytes;
         if (q_is_f16)
-            launch_pdl(dense_attn_mma_kernel<__half>, grid, dim3(128), 0, stream, keys, values, n_tokens, kv_heads, q_heads,
-                       static_cast<const __half*>(q), n_splits, scale, part_acc, part_ml);
+            launch_pdl(streamed ? dense_attn_mma_kernel<__half, true> : dense_attn_mma_kernel<__half, false>, grid, dim3(128), 0, stream, keys, values, n_tokens,
+                       kv_heads, q_heads, static_cast<const __half*>(q), n_splits, scale, part_acc, part_ml);
         else
-            launch_pdl(dense_attn_mma_kernel<float>, grid, dim3(128), 0, stream, keys, values, n_tokens, kv_heads, q_heads,
-                       static_cast<const float*>(q), n_splits, scale, part_acc, part_ml);
+            launch_pdl(streamed ? dense_attn_mma_kernel<float, true> : dense_attn_mma_kernel<float, false>, grid, dim3(128), 0, stream, keys, values, n_tokens,
+                       kv_heads, q_heads, static_cast<const float*>(q), n_splits, scale, part_acc, part_ml);
         launch_pdl(dense_combine_kernel<128>, dim3(q_heads), dim3(kCombineThreads), 0, stream, part_acc, part_ml, n_splits, out);
         TQ_CUDA(cudaGetLastError());
         return;
