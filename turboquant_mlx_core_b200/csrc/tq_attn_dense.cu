@@ -39,8 +39,33 @@ __global__ void __launch_bounds__(256) ring_write_kernel(const InT* __restrict__
         const long t = i / row, e = i - t * row;
         const long slot = (slot0 + t) % window;
         const size_t s = static_cast<size_t>(src_token0 + t) * row + e;
-        ring_k[slot * row + e] = __float2half_rn(static_cast<float>(src_k[s]));
-        ring_v[slot * row + e] = __float2half_rn(static_cast<float>(src_v[s]));
+        const float k = static_cast<float>(src_k[s]), v = static_cast<float>(src_v[s]);   // (both before a store, behind which the second would wait)
+        ring_k[slot * row + e] = __float2half_rn(k);
+        ring_v[slot * row + e] = __float2half_rn(v);
+    }
+}
+// The same eight elements at a time: rows of whole 16-byte pieces, aligned.  Element by element 131072 tokens of 4 heads took 340 us (fp32 265), bound by the
+// 64-bit divisions of every element's place and 2-byte accesses; 74 and 92 so, near what the memory delivers.  A token slid into a window: 0.6 us less.
+template <typename InT>
+__global__ void __launch_bounds__(256) ring_write_wide_kernel(const InT* __restrict__ src_k, const InT* __restrict__ src_v, unsigned int n_pieces, unsigned int row8,
+                                                              long src_token0, unsigned int window, unsigned int slot0, uint4* __restrict__ ring_k,
+                                                              uint4* __restrict__ ring_v) {
+    pdl_wait_release();
+    behind_wait(src_k, src_v);
+    auto piece = [](const InT* p, size_t i) {
+        if constexpr (sizeof(InT) == 2) return reinterpret_cast<const uint4*>(p)[i];
+        else {
+            const float4 a = reinterpret_cast<const float4*>(p)[2 * i], b = reinterpret_cast<const float4*>(p)[2 * i + 1];
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            return pack_halves(v);
+        }
+    };
+    for (unsigned int i = blockIdx.x * 256 + threadIdx.x; i < n_pieces; i += gridDim.x * 256) {
+        const unsigned int t = i / row8, e = i - t * row8, slot = (slot0 + t) % window;
+        const size_t s = static_cast<size_t>(src_token0) * row8 + i, d = static_cast<size_t>(slot) * row8 + e;
+        const uint4 k = piece(src_k, s), v = piece(src_v, s);
+        ring_k[d] = k;
+        ring_v[d] = v;
     }
 }
 
@@ -261,8 +286,9 @@ __host__ __device__ __forceinline__ int dense_frag_dim(int ks, int c) {
 }
 
 // 16 bytes of the window, which is read once; STREAM: past the first-level cache.  (The pointer comes from behind the wait: the load has nothing else that
-// keeps it there.)  A window that the L2 cache does not hold comes faster without a place made for every line: 131072 tokens of 4 heads
-// 51.7 -> 46.7 us with the combine, 65536 33.4 -> 28.3; one that it may hold does not, 49152 tokens (100 MB) 23.4 and 23.4, 32768 17.8 and 19.0.
+// keeps it there.)  A window that comes from memory comes faster without a place made for every line; one that still sits in the L2 cache does not.  Three
+// windows in turn, as a model's layers are, with the combine: 131072 tokens of 4 heads 51.7 -> 49.5 us, 65536 33.7 -> 31.0, 49152 28.1 -> 25.8, 32768 (64 MB) 22.2 ->
+// 21.1, 16384 16.7 and 16.9.  The same window again and again: 131072 51.7 -> 46.7, 65536 33.4 -> 28.3, 49152 23.4 and 23.4, 32768 17.8 and 19.0.
 template <bool STREAM>
 __device__ __forceinline__ uint4 load_window(const uint4* p) {
     if constexpr (STREAM) {
@@ -273,7 +299,7 @@ __device__ __forceinline__ uint4 load_window(const uint4* p) {
         return *p;
     }
 }
-constexpr size_t kStreamBytes = size_t(100) << 20;
+constexpr size_t kStreamBytes = size_t(60) << 20;
 template <typename QT, bool STREAM>
 __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __restrict__ keys, const __half* __restrict__ values,
                                                                 int n_tokens, int kv_heads, int q_heads, const QT* __restrict__ q,
@@ -505,6 +531,21 @@ void launch_ring_write(const void* keys, const void* values, bool is_f16, long n
                        long slot0, __half* ring_k, __half* ring_v, cudaStream_t stream) {
     if (n_tokens <= 0) return;
     const long total = n_tokens * row;
+    const auto at = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+    if (row % 8 == 0 && ((at(keys) | at(values) | at(ring_k) | at(ring_v)) & 15) == 0 && total < (1L << 33) && n_tokens < (1L << 30)) {
+        const unsigned int pieces = static_cast<unsigned int>(total / 8), row8 = static_cast<unsigned int>(row / 8);
+        const dim3 grid(static_cast<unsigned int>(std::min<long>((total / 8 + 255) / 256, 148L * 8)));
+        uint4* const rk = reinterpret_cast<uint4*>(ring_k);
+        uint4* const rv = reinterpret_cast<uint4*>(ring_v);
+        if (is_f16)
+            launch_pdl(ring_write_wide_kernel<__half>, grid, dim3(256), 0, stream, static_cast<const __half*>(keys), static_cast<const __half*>(values), pieces,
+                       row8, src_token0, static_cast<unsigned int>(window), static_cast<unsigned int>(slot0), rk, rv);
+        else
+            launch_pdl(ring_write_wide_kernel<float>, grid, dim3(256), 0, stream, static_cast<const float*>(keys), static_cast<const float*>(values), pieces,
+                       row8, src_token0, static_cast<unsigned int>(window), static_cast<unsigned int>(slot0), rk, rv);
+        TQ_CUDA(cudaGetLastError());
+        return;
+    }
     const int blocks = static_cast<int>(std::min<long>((total + 255) / 256, 148L * 8));
     if (is_f16)
         launch_pdl(ring_write_kernel<__half>, dim3(blocks), dim3(256), 0, stream, static_cast<const __half*>(keys),
