@@ -122,7 +122,7 @@ __host__ __device__ __forceinline__ size_t fragment_place(int in, int bp, int ro
     const int groups = fragment_groups(in, col), lane = g * groups + ((col & 63) >> 4);
     return static_cast<size_t>(col >> 6) * (64 * bp) + static_cast<size_t>(bp == 1 ? 2 * lane + r : ((r >> 2) * 8 * groups + lane) * 4 + (r & 3));
 }
-// (Two rows as a kernel of their own, four products side by side: 2048 x 151936 81 us instead of 67.)
+// Of the fragments; two rows have those of four (with four products side by side 2048 x 151936 took 81 us instead of 67), and sums of their own (BP).
 __host__ __device__ __forceinline__ constexpr int padded_rows(int batch) { return batch <= 1 ? 1 : batch <= 4 ? 4 : 8; }
 // One warp per (plane, batch row, WHT block): xrot = FWHT(sign o x) / sqrt(bs), rounded to
 // TF32 and stored as fp32, [plane][row][in] or (fragments: the padded rows; one plane) in the decode kernel's order.
@@ -504,7 +504,7 @@ __device__ __forceinline__ void ll_send_packets(const ScatterArgs& sc, const __h
     }
 }
 
-// BP = activation rows padded to 1, 4 or 8 (compile time, so that the partial-sum ring
+// BP = activation rows padded to 1, 2, 4 or 8 (compile time, so that the partial-sum ring
 // geometry and the reduction need no runtime arithmetic).
 // MULTI = more than one slot (row units finished through partial sums in scratch); compile time, so that the
 // single-slot kernels carry none of that path's state in their 128 registers.
@@ -528,7 +528,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     constexpr int kLag = kRing / 2;                       // how many units behind the sums run
     constexpr uint32_t kSlotBytes = kWarps * kTileFloats * 4;  // one ring slot: [warp][16 rows][BP] floats (+ padding)
     constexpr int kPer = BP >= 2 ? BP / 2 : 1;            // floats a lane adds in the reduction
-    constexpr int kSide = 8 / BP, kAcc = kSide < 2 ? 2 : kSide;   // products side by side in the B columns; accumulators
+    constexpr int kFrag = padded_rows(BP), kSide = 8 / kFrag, kAcc = kSide < 2 ? 2 : kSide;   // products side by side in the B columns; accumulators
     constexpr int kSteps = DEEP ? 4 : 2;                  // steps of codes in registers
 
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -802,7 +802,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     // B fragments.  bp rows fill bp of a product's eight columns: so the columns are 8 / bp products' pieces of the rows side by side (fragment_place), each of
     // those products has an accumulator, and only its own columns of it count.  With a fragment per product, 64 registers whatever the rows and zero columns for those that
     // are missing, fewer lookups were in flight: one row, 4096 x 4096 7.5 -> 6.3 us, 1024 x 1024 5.0 -> 4.0, 18944 x 3584 24.0 -> 22.5.
-    uint32_t bfrag[4][2 * BP];
+    uint32_t bfrag[4][2 * kFrag];
     int staged_slot = -1;
     // ring bookkeeping: slot / parity for the unit being written and the unit being summed
     int ws = 0;             // write slot = i % kRing
@@ -844,7 +844,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                                  : "r"(strip_addr + static_cast<uint32_t>(64 * s + 16 * q + 2 * g) * 4u));
                 __syncwarp();
             } else {
-            const float* xr = p.xrot + static_cast<size_t>(colw) * BP;
+            const float* xr = p.xrot + static_cast<size_t>(colw) * kFrag;
             if constexpr (DUAL) {
                 const int slices = (p.in + kSlice - 1) / kSlice;
 #pragma unroll
@@ -853,7 +853,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                     xs[k] = (n < BP && n < p.batch && colw < p.in) ? p.xscale[n * slices + colw / kSlice] : 0.f;
                 }
             }
-            const bool have_row = (g & (BP - 1)) < p.batch;
+            const bool have_row = (g & (kFrag - 1)) < p.batch;
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const bool ok = have_row && (col0 + 64 * s) < p.in;
@@ -864,8 +864,8 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                     bfrag[s][1] = __float_as_uint(t.y);
                 } else {
 #pragma unroll
-                    for (int k = 0; k < 2 * BP; k += 4) {
-                        const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * BP * s + (2 * k + g) * groups * 4 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int k = 0; k < 2 * kFrag; k += 4) {
+                        const float4 t = ok ? *reinterpret_cast<const float4*>(xr + 64 * kFrag * s + (2 * k + g) * groups * 4 + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
                         bfrag[s][k] = __float_as_uint(t.x);
                         bfrag[s][k + 1] = __float_as_uint(t.y);
                         bfrag[s][k + 2] = __float_as_uint(t.z);
@@ -953,7 +953,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
                 acc0[0] = top + __shfl_xor_sync(0xffffffffu, top, 2);
                 acc0[2] = low + __shfl_xor_sync(0xffffffffu, low, 2);
                 acc1[0] = acc1[2] = 0.f;
-            } else if constexpr (BP == 4) {
+            } else if constexpr (kFrag == 4) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const float v = q < 2 ? acc[0][k] : acc[1][k];
@@ -1313,7 +1313,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     }
     const bool fused_rotation = fill_gemv_args(a, x, out, in, batch, block, n_planes, pair_unit, seed_p, scratch);
     float* xrot = const_cast<float*>(a.xrot);
-    const int bp = padded_rows(batch);
+    const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));   // (of the ring; fragments: padded_rows)
 
     configure_gemv_kernels();
 
@@ -1357,6 +1357,7 @@ void launch_tq8_gemv_scatter(const uint8_t* codes, const float* norms, const flo
     else { TQ_GEMV_LAUNCH2(BPV, false) }
         switch (bp) {
             case 1: TQ_GEMV_LAUNCH(1) break;
+            case 2: TQ_GEMV_LAUNCH(2) break;
             case 4: TQ_GEMV_LAUNCH(4) break;
             default: TQ_GEMV_LAUNCH(8) break;
         }
@@ -1439,6 +1440,7 @@ static void configure_gemv_kernels() {
     TQ_GEMV_ATTR1((tq8_gemv_kernel<1, true, false, true>))
     TQ_GEMV_ATTR1((tq8_gemv_kernel<1, false, true, true>))
     TQ_GEMV_ATTR1((tq8_gemv_kernel<1, true, true, true>))
+    TQ_GEMV_ATTR(2)
     TQ_GEMV_ATTR(4)
     TQ_GEMV_ATTR(8)
 #undef TQ_GEMV_ATTR
@@ -1509,7 +1511,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int bp = padded_rows(batch);
+    const int bp = batch <= 1 ? 1 : (batch <= 2 ? 2 : (batch <= 4 ? 4 : 8));   // (of the ring; fragments: padded_rows)
     const bool multi = grp.m[0].n_slots > 1;   // the same for all: same in_features and planes
     const bool dual = items[0].n_planes == 2;
 #define TQ_GROUP_LAUNCH2(BPV, DV)                                                             \
@@ -1520,6 +1522,7 @@ void launch_tq8_gemv_group(const GemvGroupItem* items, int n, const __half* x, i
     else { TQ_GROUP_LAUNCH2(BPV, false) }
     switch (bp) {
         case 1: TQ_GROUP_LAUNCH(1) break;
+        case 2: TQ_GROUP_LAUNCH(2) break;
         case 4: TQ_GROUP_LAUNCH(4) break;
         default: TQ_GROUP_LAUNCH(8) break;
     }
