@@ -970,21 +970,23 @@ struct Sums {
             v[0] = t.x; v[1] = t.y;
         }
     }
-    // Rows that are not whole pieces: the first n of them.
-    __device__ __forceinline__ void load_some(const float* p, int n) {
+    // `step` apart, those below n.
+    __device__ __forceinline__ void load_some(const float* p, int n, int step) {
 #pragma unroll
-        for (int k = 0; k < V; ++k) v[k] = k < n ? __ldcg(p + k) : 0.f;
+        for (int k = 0; k < V; ++k) v[k] = k * step < n ? __ldcg(p + k * step) : 0.f;
     }
 };
 // V = 4, or 2 where more than eight splits are to be asked for at once.
 template <int kBatch, int V>
 __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool early) {
     const int out = f.out, k_splits = f.k_splits;
-    const int c = V * static_cast<int>(blockIdx.x * kFinishThreads + threadIdx.x);
+    // a thread's V rows: side by side in whole pieces, otherwise a CTA's width apart, so that a warp's accesses are contiguous all the same
+    const int step = f.vec ? 1 : kFinishThreads;
+    const int c = f.vec ? V * static_cast<int>(blockIdx.x * kFinishThreads + threadIdx.x) : static_cast<int>(V * blockIdx.x * kFinishThreads + threadIdx.x);
     if (c >= out) return;
     float norm[V];   // (used behind the wait only: a product with it in front of the wait would wait for it there)
 #pragma unroll
-    for (int k = 0; k < V; ++k) norm[k] = c + k < out ? __ldg(f.norms + c + k) : 0.f;
+    for (int k = 0; k < V; ++k) norm[k] = c + k * step < out ? __ldg(f.norms + c + k * step) : 0.f;
     if (early) asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!early) asm volatile("griddepcontrol.launch_dependents;");
@@ -1006,7 +1008,7 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool
             } else {
 #pragma unroll
                 for (int z = 0; z < kBatch; ++z)
-                    if (z0 + z < k_splits) v[z].load_some(src + (z0 + z) * split, out - c);
+                    if (z0 + z < k_splits) v[z].load_some(src + (z0 + z) * split, out - c, kFinishThreads);
             }
 #pragma unroll
             for (int z = 0; z < kBatch; ++z)
@@ -1027,7 +1029,7 @@ __device__ __forceinline__ void gemm_finish_body(const FinishOne& f, int m, bool
         } else {
 #pragma unroll
             for (int k = 0; k < V; ++k)
-                if (c + k < out) y[k] = __float2half_rn(acc[k] * (norm[k] * f.inv_scale));
+                if (c + k * kFinishThreads < out) y[k * kFinishThreads] = __float2half_rn(acc[k] * (norm[k] * f.inv_scale));
         }
     }
 }
