@@ -134,8 +134,9 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait; gives up at once when another thread has already flagged a failure.  (Without a time to sleep: with 20 us of it
-// 3584 x 37888 at 16 rows took 35.3 us instead of 34.2.)
+// Bounded wait; gives up at once when another thread has already flagged a failure.  Its time begins when it does not find the phase over: a thread whose phase
+// ends only when kernels in front are done waits for those first (griddepcontrol.wait), with no limit of its own, or their time would count.  (Without
+// a time to sleep: with 20 us of it 3584 x 37888 at 16 rows took 35.3 us instead of 34.2.)
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile unsigned int* abort_flag) {
     unsigned long long t0 = 0;
     for (uint32_t spin = 0;; ++spin) {
@@ -602,6 +603,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     auto epilogue = [&] {
         // ---- epilogue: TMEM lanes 32 * (warp & 3) .. + 31 (a lane = a weight row), 32 activation rows at a time ----
         constexpr int kColStep = kGroups == kGroupsMax ? 32 : 8 * kProducerWarps;   // a quarter of the warps for a quarter of the lanes
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // (see bar_wait)
         int acc = 0;
         uint32_t par = 0u;
         for (int j = 0; j < n_local; ++j) {
@@ -718,10 +720,13 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                          : "=r"(ready) : "r"(bar_e), "r"(par) : "memory");
             auto slot_free = [&] {
-                if (!__all_sync(0xffffffffu, ready) && !__all_sync(0xffffffffu, bar_wait(bar_e, par, abort_flag))) {
-                    raise_status(p.status, 6u);
-                    atomicExch(&s_abort, 1u);
-                    return false;
+                if (!__all_sync(0xffffffffu, ready)) {
+                    asm volatile("griddepcontrol.wait;" ::: "memory");   // (see bar_wait; a full ring in front of the first activation tile)
+                    if (!__all_sync(0xffffffffu, bar_wait(bar_e, par, abort_flag))) {
+                        raise_status(p.status, 6u);
+                        atomicExch(&s_abort, 1u);
+                        return false;
+                    }
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");   // the MMAs' reads of the slot before the stores to it
                 return true;
@@ -847,6 +852,7 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             int slot = 0, acc = 0;
             uint32_t par = 0u, acc_par = 1u;   // acc_par: parity of the "drained" phase to wait for
             bool ok = true;
+            asm volatile("griddepcontrol.wait;" ::: "memory");   // (see bar_wait)
             for (int j = 0; ok && j < n_local; ++j) {
                 const uint32_t idesc = instr_desc(static_cast<uint32_t>(tile_rows(t0 + j * t_step)));
                 const uint32_t d_tmem = tmem_d + static_cast<uint32_t>(acc * (kTileTok / 2));
