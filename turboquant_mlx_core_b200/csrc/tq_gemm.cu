@@ -114,7 +114,7 @@ int gemm_carveout(long m, int groups) {
     const size_t kb = (gemm_smem_bytes(m, groups) / 1024 + 1) * (groups == 1 ? 2 : 1) + 10;
     return std::min(100, static_cast<int>(kb * 100 / 228 + 1));
 }
-constexpr unsigned long long kGemmWaitLimitNs = 200ull * 1000 * 1000;
+constexpr unsigned long long kGemmWaitLimitNs = 200ull * 1000 * 1000, kGemmCopyLandNs = 1000ull * 1000;
 
 // instruction descriptor: D fp32, A and B fp16, both K-major, M = 128, N = n (a multiple of 16 up to 256)
 __host__ __device__ constexpr uint32_t instr_desc(uint32_t n) {
@@ -820,6 +820,8 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
             for (int t = t0; ok && t < t_end; t += t_step) {
                 const uint32_t b_bytes = static_cast<uint32_t>(tile_rows(t)) * (kBlockK * 2);
                 for (int it = 0; it < n_it; ++it) {
+                    ok = !*abort_flag;   // no copy once another thread has given up: it would be on its way when the CTA ends
+                    if (!ok) break;
                     if (filled >= n_st && !bar_wait(bar_empty + 8u * slot, par, abort_flag)) {
                         raise_status(p.status, 6u);
                         atomicExch(&s_abort, 1u);
@@ -902,6 +904,12 @@ __device__ __forceinline__ void gemm_body(const GemmArgs& p, const int t0, const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    // Given up: what the copying lane has started lands before the CTA's shared memory becomes another's.  Its barriers may miss arrivals of warps that are gone
+    // and say nothing, so a time: a copy takes microseconds, and no further one starts.
+    if (*abort_flag && warp == kCopyWarp) {
+        const unsigned long long t0 = timer_ns();
+        while (timer_ns() - t0 < kGemmCopyLandNs) {}
+    }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(tmem_cols) : "memory");
