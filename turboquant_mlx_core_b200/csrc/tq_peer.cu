@@ -81,10 +81,10 @@ __global__ void __launch_bounds__(kBcastThreads) exchange_broadcast_kernel(const
 }
 
 // One warp: lane i waits until flags[i] has reached the epoch of this wait (kept in *epoch, which
-// the kernel advances by one per launch).
+// the kernel advances by one per launch).  Kernels that wait for other ranks let the next one come behind that wait (this one by its end): a kernel that
+// is let come waits on its SMs, with their registers and tensor memory, and a kernel of another stream that this wait's ranks need would not get there.
 __global__ void exchange_wait_kernel(const unsigned int* __restrict__ flags, int n, unsigned int* epoch, unsigned int* status) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
     const int lane = threadIdx.x;
     unsigned int want = 0;
     if (lane == 0) want = atomicAdd(epoch, 1u) + 1u;
@@ -188,13 +188,12 @@ __global__ void __launch_bounds__(256) exchange_unpack_packets_kernel(const uint
 }
 
 // Waits (bounded) for the packets every other rank wrote in the exchange that has just completed on this rank
-// (*epoch is its number) and writes their rows into the gathered result: row block `src` of every activation row.
+// (*epoch is its number) and writes their rows into the gathered result: row block `src` of every activation row.  (Its end lets the next kernel come.)
 __global__ void __launch_bounds__(256) exchange_wait_packets_kernel(const uint4* __restrict__ base, const unsigned int* __restrict__ epoch,
                                                                     unsigned int* __restrict__ wait_epoch, int rank, int world, long per_row,
                                                                     int batch, long rows, __half* __restrict__ out, long out_stride,
                                                                     unsigned int* status) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
     const unsigned int want = *reinterpret_cast<const volatile unsigned int*>(epoch);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wait_epoch, 1u);   // one wait per exchange, like tq_exchange_wait
     const long packets = static_cast<long>(batch) * per_row;
@@ -230,7 +229,6 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_packets_kernel(c
                                                                    const __half* __restrict__ norm_w, __half* __restrict__ normed, int cols,
                                                                    float eps) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
     behind_wait(local, residual, norm_w);
     const unsigned int want = *reinterpret_cast<const volatile unsigned int*>(epoch);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(wait_epoch, 1u);
@@ -290,6 +288,7 @@ __global__ void __launch_bounds__(kRowNormThreads) exchange_sum_packets_kernel(c
     }
     if (by_row) {
         __syncthreads();   // the row is complete (every thread gets here, also after a timeout)
+        asm volatile("griddepcontrol.launch_dependents;");
         rmsnorm_row<false, kRowNormMore>(out + static_cast<long>(blockIdx.x) * cols, norm_w, normed + static_cast<long>(blockIdx.x) * cols, cols, eps);
     }
 }
