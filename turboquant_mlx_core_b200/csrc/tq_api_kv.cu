@@ -635,7 +635,8 @@ public:
     }
     void slide_window(const void* keys, const void* values, int dtype, int num_tokens, cudaStream_t st) {
         TQ_REQUIRE(num_tokens >= 0, "decode buffer: negative token count");
-        write(keys, values, dtype, num_tokens, window_start_, st);
+        const int first = std::max(0, num_tokens - window_);   // those before it are overwritten by the window's worth behind them
+        write(keys, values, dtype, num_tokens - first, static_cast<int>((static_cast<long>(window_start_) + first) % window_), st, first);
         window_start_ = static_cast<int>((static_cast<long>(window_start_) + num_tokens) % window_);
     }
     void read(bool values, int start, int end, void* out, cudaStream_t st) {
@@ -659,13 +660,16 @@ public:
     }
 
 private:
-    void write(const void* keys, const void* values, int dtype, int n, int slot0, cudaStream_t st) {
+    // n <= window_ tokens, from the source's `first` on, to the slots slot0.. (each slot once: the kernel writes them in no order)
+    void write(const void* keys, const void* values, int dtype, int n, int slot0, cudaStream_t st, int first = 0) {
         TQ_REQUIRE(dtype == TQ_F32 || dtype == TQ_F16, "decode buffer: keys and values must be fp32 or fp16");
         if (n == 0) return;
         TQ_REQUIRE(keys != nullptr && values != nullptr, "decode buffer: NULL keys or values");
         tq::ensure_device(device_);
         const int row = heads_ * dim_;
-        const size_t bytes = static_cast<size_t>(n) * row * (dtype == TQ_F32 ? 4 : 2);
+        const size_t row_bytes = static_cast<size_t>(row) * (dtype == TQ_F32 ? 4 : 2), bytes = n * row_bytes;
+        keys = static_cast<const char*>(keys) + first * row_bytes;
+        values = static_cast<const char*>(values) + first * row_bytes;
         const void* dk = keys;
         const void* dv = values;
         if (!tq::is_device_pointer(keys)) {
