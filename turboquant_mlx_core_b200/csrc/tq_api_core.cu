@@ -23,15 +23,22 @@ int current_device() {
     return d;
 }
 
-int sm_count(int device) {
+static int device_attribute(cudaDeviceAttr which, int device, int (&cache)[64]) {
     static std::mutex mu;
-    static int cache[64] = {0};
     std::lock_guard<std::mutex> lock(mu);
     if (device >= 0 && device < 64 && cache[device]) return cache[device];
     int n = 0;
-    TQ_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device));
+    TQ_CUDA(cudaDeviceGetAttribute(&n, which, device));
     if (device >= 0 && device < 64) cache[device] = n;
     return n;
+}
+int sm_count(int device) {
+    static int cache[64] = {0};
+    return device_attribute(cudaDevAttrMultiProcessorCount, device, cache);
+}
+size_t l2_bytes(int device) {
+    static int cache[64] = {0};
+    return static_cast<size_t>(device_attribute(cudaDevAttrL2CacheSize, device, cache));
 }
 
 // N(0,1) Lloyd-Max centroids for 1..5 bits: the values of src/codebook.cpp:16-45.

@@ -734,7 +734,7 @@ void hybrid_attention(TQKVCache* cache, DecodeBuffer* buf, int layer, const void
     const int n_splits = tq::dense_attention_splits(seq_len, heads, q_heads, tq::sm_count(cache->device()));
     buf->scratch().reserve(tq::dense_attention_scratch_bytes(q_heads, dim, n_splits), st);
     tq::launch_dense_attention(buf->key_ring(), buf->value_ring(), seq_len, heads, dim, d_q, q_dtype == TQ_F16, q_heads, n_splits,
-                               buf->scratch().as<void>(), d_out, st);
+                               tq::l2_bytes(cache->device()), buf->scratch().as<void>(), d_out, st);
     if (!out_dev) {
         TQ_CUDA(cudaMemcpyAsync(out, d_out, n_q * sizeof(__half), cudaMemcpyDeviceToHost, st));
         TQ_CUDA(cudaStreamSynchronize(st));

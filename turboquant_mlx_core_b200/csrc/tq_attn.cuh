@@ -133,6 +133,6 @@ void launch_ring_read(const __half* ring, long n_tokens, int row, int window, lo
 int dense_attention_splits(int n_tokens, int kv_heads, int q_heads, int sm_count);
 size_t dense_attention_scratch_bytes(int q_heads, int head_dim, int n_splits);
 void launch_dense_attention(const __half* keys, const __half* values, int n_tokens, int kv_heads, int head_dim, const void* q,
-                            bool q_is_f16, int q_heads, int n_splits, void* scratch, __half* out, cudaStream_t stream);
+                            bool q_is_f16, int q_heads, int n_splits, size_t l2_bytes, void* scratch, __half* out, cudaStream_t stream);
 
 }  // namespace tq

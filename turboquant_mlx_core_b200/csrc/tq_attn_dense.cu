@@ -286,9 +286,10 @@ __host__ __device__ __forceinline__ int dense_frag_dim(int ks, int c) {
 }
 
 // 16 bytes of the window, which is read once; STREAM: past the first-level cache.  (The pointer comes from behind the wait: the load has nothing else that
-// keeps it there.)  A window that comes from memory comes faster without a place made for every line; one that still sits in the L2 cache does not.  Three
-// windows in turn, as a model's layers are, with the combine: 131072 tokens of 4 heads 51.7 -> 49.5 us, 65536 33.7 -> 31.0, 49152 28.1 -> 25.8, 32768 (64 MB) 22.2 ->
-// 21.1, 16384 16.7 and 16.9.  The same window again and again: 131072 51.7 -> 46.7, 65536 33.4 -> 28.3, 49152 23.4 and 23.4, 32768 17.8 and 19.0.
+// keeps it there.)  A window that comes from memory comes faster without a place made for every line; one that still sits in the L2 cache does not.  So from the size
+// on that the L2 cache does not hold from call to call, five sixths of it (105 MB).  Keys and values of 4 heads with the combine, calls in a graph, cached and past the cache: the
+// same window again and again 64 MB 15.5 and 19.2 us, 96 MB 21.1 and 24.0, 104 MB 25.1 and 26.3, 112 MB 27.7 and 26.7, 128 MB 30.7 and 28.8, 256 MB 49.2 and 47.3; three windows
+// in turn, as a model's layers are, 64 MB 19.8 and 19.6, 96 MB 25.7 and 24.7, 104 MB 27.6 and 26.6, 112 MB 28.6 and 27.3, 128 MB 30.6 and 29.5, 256 MB 49.2 and 48.6.
 template <bool STREAM>
 __device__ __forceinline__ uint4 load_window(const uint4* p) {
     if constexpr (STREAM) {
@@ -299,7 +300,6 @@ __device__ __forceinline__ uint4 load_window(const uint4* p) {
         return *p;
     }
 }
-constexpr size_t kStreamBytes = size_t(60) << 20;
 template <typename QT, bool STREAM>
 __global__ void __launch_bounds__(128, 3) dense_attn_mma_kernel(const __half* __restrict__ keys, const __half* __restrict__ values,
                                                                 int n_tokens, int kv_heads, int q_heads, const QT* __restrict__ q,
@@ -578,7 +578,7 @@ size_t dense_attention_scratch_bytes(int q_heads, int head_dim, int n_splits) {
 }
 
 void launch_dense_attention(const __half* keys, const __half* values, int n_tokens, int kv_heads, int head_dim, const void* q,
-                            bool q_is_f16, int q_heads, int n_splits, void* scratch, __half* out, cudaStream_t stream) {
+                            bool q_is_f16, int q_heads, int n_splits, size_t l2_bytes, void* scratch, __half* out, cudaStream_t stream) {
     TQ_REQUIRE(q_heads % kv_heads == 0, "window attention: query heads must be a multiple of KV heads");
     TQ_REQUIRE(n_tokens > 0 && n_splits >= 1 && n_splits <= kMaxSplits, "window attention: empty range");
     const int G = q_heads / kv_heads;
@@ -597,7 +597,7 @@ void launch_dense_attention(const __half* keys, const __half* values, int n_toke
                                                                        part_ml);
     static const bool cuda_core_only = std::getenv("TQ_WINDOW_ATTENTION_FMA") != nullptr;   // measurement switch: the fp32-FMA kernel at head_dim 128
     if (head_dim == 128 && !cuda_core_only) {
-        const bool streamed = static_cast<size_t>(n_tokens) * kv_heads * head_dim * 2 * sizeof(__half) > kStreamBytes;
+        const bool streamed = static_cast<size_t>(n_tokens) * kv_heads * head_dim * 2 * sizeof(__half) > l2_bytes / 6 * 5;   // (see load_window)
         if (q_is_f16)
             launch_pdl(streamed ? dense_attn_mma_kernel<__half, true> : dense_attn_mma_kernel<__half, false>, grid, dim3(128), 0, stream, keys, values, n_tokens,
                        kv_heads, q_heads, static_cast<const __half*>(q), n_splits, scale, part_acc, part_ml);

@@ -36,6 +36,7 @@ R guarded(R ok_unused, R fail, F&& body) {
 // ---- device selection -------------------------------------------------------------------
 int current_device();
 int sm_count(int device);
+size_t l2_bytes(int device);
 // cudaSetDevice only when another device is current (it is not free even as a no-op).
 inline void ensure_device(int device) {
     int cur = -1;
