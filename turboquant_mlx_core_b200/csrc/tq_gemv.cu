@@ -511,7 +511,10 @@ __device__ __forceinline__ void ll_send_packets(const ScatterArgs& sc, const __h
 // DUAL = weights with two rotations: table words and activation words are pairs of fp16.
 // ROW = the activation row is a kernel parameter, `row` its generic address.
 // DEEP = all four steps of a unit's codes in registers, not two (one activation row, many units a CTA).
-template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false, bool DEEP = false>
+// AT_FIRST = a new slot is known by its first row unit, not by a number that is kept: a register less, which eight rows of two rotations in several slots turn into
+// more lookups in flight (5120 x 27648 at eight rows 53.9 -> 51.2 us, 18944 x 3584 30.8 -> 29.7, 14336 x 4096 27.7 -> 26.8).  The other kernels spill with it (the group's of the same
+// rows: twice 5120 x 27648 94 -> 117; one row, four steps: 5120 x 27648 38.6 -> 39.4).
+template <int BP, bool SCATTER, bool LL, bool MULTI, bool DUAL, bool ROW = false, bool DEEP = false, bool AT_FIRST = false>
 __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& sargs, const int bid, const int nblk, const __half* row = nullptr) {
     auto load_x = [&](int col) {   // eight columns of the row that is rotated in here
         if constexpr (ROW) return *reinterpret_cast<const uint4*>(row + col);
@@ -879,7 +882,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
     stage_slot(cur.slot, x_first, ROW || (!DUAL && p.x != nullptr));
 
     for (int i = 0; i < n_local; ++i) {
-        if (cur.slot != staged_slot) stage_slot(cur.slot, make_uint4(0, 0, 0, 0), false);
+        if (AT_FIRST ? i > 0 && cur.ru == 0 : cur.slot != staged_slot) stage_slot(cur.slot, make_uint4(0, 0, 0, 0), false);
         const bool has_next = i + 1 < n_local;
 
         float acc[kAcc][4];
@@ -893,9 +896,8 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
         for (int s = 0; s < 4; ++s) {
             uint4& lo = blo[s % kSteps];
             uint4& hi = bhi[s % kSteps];
-            // 16 independent lookups, then the 4 MMAs they feed (bytes 0,1 of a word feed one
-            // MMA, bytes 2,3 the next); two accumulator chains.  Once the second half's addresses
-            // are formed the code registers are free: the step two ahead is loaded into them.
+            // Eight independent lookups (a word of each row), then the two MMAs they feed (bytes 0, 1 of the words feed one, bytes 2, 3 the next), kAcc
+            // accumulator chains.  Once the last words' addresses are formed the code registers are free: the step kSteps ahead is loaded into them.
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
                 const uint32_t l = w == 0 ? lo.x : (w == 1 ? lo.y : (w == 2 ? lo.z : lo.w));
@@ -1074,7 +1076,7 @@ __device__ __forceinline__ void gemv_body(const GemvArgs& p, const ScatterArgs& 
 
 template <int BP, bool MULTI, bool DUAL, bool DEEP = false>
 __global__ void __launch_bounds__(kCtaThreads, 1) tq8_gemv_kernel(const GemvArgs p) {
-    gemv_body<BP, false, false, MULTI, DUAL, false, DEEP>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
+    gemv_body<BP, false, false, MULTI, DUAL, false, DEEP, BP == 8 && MULTI && DUAL>(p, ScatterArgs{}, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x));
 }
 // The one activation row of a host caller, which rides in the launch (16 N bytes of fp16): as a kernel of its own in front, which wrote it to
 // device memory, it cost a launch and its end.  4096 x 4096 from and to host memory 31.3 us, 29.7 so, 512 x 14336 39.8 and 33.5.
