@@ -104,11 +104,20 @@ int gemm_groups(long n_tiles, int k_blocks, long m, int sm_count) {
     const int stages = (k_blocks + kSubPerStage - 1) / kSubPerStage;
     return n_tiles <= sm_count && stages <= (m <= 32 ? 30 : 24) ? 2 : kGroupsMax;
 }
-// Rows up to which one group serves a launch of several matrices (its tensor memory holds an accumulator of so many).
+// Producer groups of a launch of several matrices; `least` is the smallest count of K splits.  Up to 128 rows (one group's tensor memory holds an accumulator of so many): one, two CTAs to an
+// SM, where the CTAs outnumber the SMs (figures beside the kernel), otherwise two.  Above, a CTA to an SM: two, whose CTAs are set up beside the rotation, but three
+// where matrices of unequal splits leave long CTAs to a matrix that is split itself, beside short ones of the others: the long ones' codes are the launch's time.  Two groups and three, two
+// rotations, weights from memory: 8192 -> 8192 + 1024 + 1024 (64 stages, 7, 7) at 192 rows 86.9 and 82.8 us, 6144 -> 6144 + 1024 + 1024 (32, 5, 5) at 256 77.3 and 73.6, 5120 -> 5120 + 1024 +
+// 1024 (27, 4, 4) at 224 62.4 and 59.3, 4096 -> 4096 + 1024 + 1024 (32, 7, 7) at 384 66.9 and 65.4.  The other way round: 14336 -> 2048 + 512 (25, 6) at 192 46.0 and 47.6, 4096 -> 4096 + 1024 +
+// 1024 (16, 4, 4) at 192 45.4 and 47.5, 4096 -> 8192 + 2048 (32, 6) at 129 38.1 and 39.3 (at 192 47.4 and 46.1); not split, 5120 -> 5120 + 1024 + 1024 (80, 9, 9) at 512 83.3 and 84.7; equal splits, 8192 -> 2 x 4096 (32, 32) at 256 74.7 and 77.3.
 constexpr long kGroupOneRows = 128;
+int group_call_groups(long m, long n_products, bool unequal, int least, int k_blocks, int sm_count) {
+    if (m <= kGroupOneRows) return n_products > sm_count ? 1 : 2;
+    return unequal && least > 1 && (k_blocks / least + kSubPerStage - 1) / kSubPerStage > 26 ? kGroupsMax : 2;
+}
 // An SM divides its 228 KB between shared memory and first-level cache anew only when it is empty, and small kernels ask for little of it: the product's
-// CTA did not come beside them.  So all three kernels of a call ask for what the product takes and 10 KB, where that is more than 100 KB (7168 x 2048 at 64
-// rows 14.3 -> 12.0 us, 8192 x 1024 12.6 -> 11.5; 4096 x 4096 at 16 rows, whose loads of codes then have less of the cache, 8.5 -> 9.1).  Percent; 0: no wish.
+// CTA did not come beside them.  So above 32 rows all three kernels of a call with one or two groups ask for what the product (two CTAs of one group) takes and 10 KB (7168 x 2048 at 64
+// rows 14.3 -> 12.0 us, 8192 x 1024 12.6 -> 11.5).  Up to 32 rows not: 4096 x 4096 at 16, whose loads of codes then have less of the cache, 8.5 -> 9.1.  Percent; 0: no wish.
 int gemm_carveout(long m, int groups) {
     if (m <= 32 || groups == kGroupsMax) return 0;
     const size_t kb = (gemm_smem_bytes(m, groups) / 1024 + 1) * (groups == 1 ? 2 : 1) + 10;
@@ -937,10 +946,11 @@ struct GemmGroupArgs {
     int n_tiles[kMaxGemmGroup];     // (flat)
     int n, flat;
 };
-// Where the CTAs outnumber the SMs they have one group of producers each and go two to an SM, the second half beside the first instead of behind it
+// Up to 128 rows, where the CTAs outnumber the SMs they have one group of producers each and go two to an SM, the second half beside the first instead of behind it
 // (80 registers: a third one would find no tensor memory).  Two or three groups, one CTA to an SM -> one group: 3584 -> 3584 + 512 + 512 at 16 rows 15.1 -> 9.4 us,
 // at 64 17.6 -> 13.4, 5120 -> 5120 + 1024 + 1024 at 32 21.6 -> 19.3, 4096 -> 2 x 11008 at 16 39.1 -> 33.0.  Where they do not, two groups: 2048 -> 2 x 1024 at 32 rows
 // 7.1 -> 6.7, 768 -> 2 x 768 at 100 8.1 -> 6.7 (three 9.6).
+// (The bound of two groups is that of three: 64 registers a thread, so that CTAs of the rotation and of the sums fit beside them.)
 template <bool DUAL, int GROUPS>
 __global__ void __launch_bounds__(GROUPS == 1 ? 384 : gemm_threads(kGroupsMax), GROUPS == 1 ? 2 : 1) tq8_gemm_group_kernel(const __grid_constant__ GemmGroupArgs grp) {
     const int b = static_cast<int>(blockIdx.x);
@@ -1266,7 +1276,7 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         finish_add(fin, n_fin, a);
     }
     for (int i = n; i <= kMaxGemmGroup; ++i) grp.start[i] = static_cast<int>(n_ctas);
-    const int groups = m <= kGroupOneRows && n_products > sm_count ? 1 : 2;
+    const int groups = group_call_groups(m, n_products, grp.flat != 0, splits[order[0]], in / kBlockK * n_planes, sm_count);
     // 1. the rotations
     launch_rotate_rows(x, rot, n, in, m, n_planes, block, groups, gemm_carveout(m, groups), sm_count, stream);
     // 2. the GEMMs
