@@ -104,16 +104,41 @@ int gemm_groups(long n_tiles, int k_blocks, long m, int sm_count) {
     const int stages = (k_blocks + kSubPerStage - 1) / kSubPerStage;
     return n_tiles <= sm_count && stages <= (m <= 32 ? 30 : 24) ? 2 : kGroupsMax;
 }
-// Producer groups of a launch of several matrices; `least` is the smallest count of K splits.  Up to 128 rows (one group's tensor memory holds an accumulator of so many): one, two CTAs to an
-// SM, where the CTAs outnumber the SMs (figures beside the kernel), otherwise two.  Above, a CTA to an SM: two, whose CTAs are set up beside the rotation, but three
+// Producer groups of a launch of several matrices, each of them `ctas` CTAs (tiles x K splits) of `stages` stages.  One group (two CTAs to an SM, up to 128 rows: its tensor memory holds an
+// accumulator of so many) hides a CTA's beginning and end behind the other's stages, but takes nearly twice as long for a stage.  So where the CTAs outnumber the SMs (otherwise: two) it is
+// compared with CTAs that have an SM to themselves, in stages, a CTA's beginning and end as 20 of them: 2 stages + 20 a CTA on 2 x SMs, stages + 20 on the SMs; in waves, or where the matrices' CTAs
+// are not equally long by their sum, but no less than the longest.  Three groups and one, 16 rows, weights from memory: 4096 -> 2 x 14080 (220 CTAs of 32 stages) 39.9 and 34.1 us, 2048 -> 2 x 28160 (440 of 16)
+// 39.4 and 36.5, 4096 -> 2 x 38400 (600 of 32) 94.0 and 88.9, 5120 -> 5120 + 1024 + 1024 (120 of 13, 160 of 4) 21.0 and 16.6; the other way round 8192 -> 2 x 22528 (352 of 64) 98.3 and 110.8, 4096 ->
+// 2 x 28160 (440 of 32) 60.2 and 65.7, two rotations 5120 -> 2 x 22528 (352 of 80) 86.7 and 103.4, 8192 -> 8192 + 1024 + 1024 (128 of 64, 288 of 7) 41.6 and 47.5.
+// Of CTAs alone on an SM, three groups stream codes faster, two are set up beside the rotation.  Up to 64 rows (32 of two rotations) three: two would take 104.3 us for the first of those four, 62.1, 92.7 and
+// 42.6; above that the tensor cores' share grows and two: two rotations 4096 -> 2 x 19200 at 128 rows 98.1 -> 92.9, 2048 -> 2 x 19200 at 64 48.0 -> 46.2.  Above 128 rows two as well, but three
 // where matrices of unequal splits leave long CTAs to a matrix that is split itself, beside short ones of the others: the long ones' codes are the launch's time.  Two groups and three, two
 // rotations, weights from memory: 8192 -> 8192 + 1024 + 1024 (64 stages, 7, 7) at 192 rows 86.9 and 82.8 us, 6144 -> 6144 + 1024 + 1024 (32, 5, 5) at 256 77.3 and 73.6, 5120 -> 5120 + 1024 +
 // 1024 (27, 4, 4) at 224 62.4 and 59.3, 4096 -> 4096 + 1024 + 1024 (32, 7, 7) at 384 66.9 and 65.4.  The other way round: 14336 -> 2048 + 512 (25, 6) at 192 46.0 and 47.6, 4096 -> 4096 + 1024 +
-// 1024 (16, 4, 4) at 192 45.4 and 47.5, 4096 -> 8192 + 2048 (32, 6) at 129 38.1 and 39.3 (at 192 47.4 and 46.1); not split, 5120 -> 5120 + 1024 + 1024 (80, 9, 9) at 512 83.3 and 84.7; equal splits, 8192 -> 2 x 4096 (32, 32) at 256 74.7 and 77.3.
-constexpr long kGroupOneRows = 128;
-int group_call_groups(long m, long n_products, bool unequal, int least, int k_blocks, int sm_count) {
-    if (m <= kGroupOneRows) return n_products > sm_count ? 1 : 2;
-    return unequal && least > 1 && (k_blocks / least + kSubPerStage - 1) / kSubPerStage > 26 ? kGroupsMax : 2;
+// 1024 (16, 4, 4) at 192 45.4 and 47.5, 4096 -> 8192 + 2048 (32, 6) at 129 38.1 and 39.3 (at 192 47.4 and 46.1); not split, 5120 -> 5120 + 1024 + 1024 (80, 9, 9) at 512 83.3 and 84.7; equal
+// splits, 8192 -> 2 x 4096 (32, 32) at 256 74.7 and 77.3.
+constexpr long kGroupOneRows = 128, kCtaEndsInStages = 20;
+struct GroupCallCtas {
+    long ctas[4];
+    int stages[4], n, least;   // least: the smallest count of K splits
+    bool unequal;              // splits
+};
+int group_call_groups(const GroupCallCtas& c, long m, int n_planes, int sm_count) {
+    long all = 0, longest = 0;
+    for (int i = 0; i < c.n; ++i) {
+        all += c.ctas[i];
+        longest = std::max<long>(longest, c.stages[i]);
+    }
+    if (m > kGroupOneRows) return c.unequal && c.least > 1 && longest > 26 ? kGroupsMax : 2;
+    if (all <= sm_count) return 2;
+    auto time = [&](long per_stage, long slots) {
+        if (!c.unequal) return (all + slots - 1) / slots * (per_stage * longest + kCtaEndsInStages);
+        long sum = 0;
+        for (int i = 0; i < c.n; ++i) sum += c.ctas[i] * (per_stage * c.stages[i] + kCtaEndsInStages);
+        return std::max(per_stage * longest + kCtaEndsInStages, sum / slots);
+    };
+    if (time(2, 2 * sm_count) <= time(1, sm_count)) return 1;
+    return m * n_planes <= 64 ? kGroupsMax : 2;
 }
 // An SM divides its 228 KB between shared memory and first-level cache anew only when it is empty, and small kernels ask for little of it: the product's
 // CTA did not come beside them.  So above 32 rows all three kernels of a call with one or two groups ask for what the product (two CTAs of one group) takes and 10 KB (7168 x 2048 at 64
@@ -946,9 +971,9 @@ struct GemmGroupArgs {
     int n_tiles[kMaxGemmGroup];     // (flat)
     int n, flat;
 };
-// Up to 128 rows, where the CTAs outnumber the SMs they have one group of producers each and go two to an SM, the second half beside the first instead of behind it
+// CTAs of one group of producers (group_call_groups) go two to an SM, the second half beside the first instead of behind it
 // (80 registers: a third one would find no tensor memory).  Two or three groups, one CTA to an SM -> one group: 3584 -> 3584 + 512 + 512 at 16 rows 15.1 -> 9.4 us,
-// at 64 17.6 -> 13.4, 5120 -> 5120 + 1024 + 1024 at 32 21.6 -> 19.3, 4096 -> 2 x 11008 at 16 39.1 -> 33.0.  Where they do not, two groups: 2048 -> 2 x 1024 at 32 rows
+// at 64 17.6 -> 13.4, 5120 -> 5120 + 1024 + 1024 at 32 21.6 -> 19.3, 4096 -> 2 x 11008 at 16 39.1 -> 33.0.  Fewer CTAs than SMs, two groups: 2048 -> 2 x 1024 at 32 rows
 // 7.1 -> 6.7, 768 -> 2 x 768 at 100 8.1 -> 6.7 (three 9.6).
 // (The bound of two groups is that of three: 64 registers a thread, so that CTAs of the rotation and of the sums fit beside them.)
 template <bool DUAL, int GROUPS>
@@ -1237,7 +1262,8 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
     FinishArgs fin{};
     int n_fin = 0;
     grp.n = n;
-    long n_ctas = 0, n_products = 0;
+    long n_ctas = 0;
+    GroupCallCtas shape{};
     int order[kMaxGemmGroup], splits[kMaxGemmGroup];
     const long tok_tiles = (m + kTileTok - 1) / kTileTok;
     for (int i = 0; i < n; ++i) {
@@ -1269,14 +1295,18 @@ void launch_tq8_gemm_group(const GemmGroupItem* items, int n, const __half* x, l
         grp.n_tiles[i] = static_cast<int>(n_tiles);
         grp.start[i] = static_cast<int>(n_ctas);
         n_ctas += grp.flat ? n_tiles * a.k_splits : row_tiles;
-        n_products += n_tiles * a.k_splits;
+        shape.ctas[i] = n_tiles * a.k_splits;
+        shape.stages[i] = (in / kBlockK * n_planes / a.k_splits + kSubPerStage - 1) / kSubPerStage;
         TQ_REQUIRE(n_tiles < (1L << 31) && n_ctas < (1L << 31), "tq8_gemm group: too many output tiles");
         rot.xrot[i] = static_cast<__half*>(it.scratch);
         rot.seed_p[i] = it.seed_p; rot.seed_r[i] = it.seed_r;
         finish_add(fin, n_fin, a);
     }
     for (int i = n; i <= kMaxGemmGroup; ++i) grp.start[i] = static_cast<int>(n_ctas);
-    const int groups = group_call_groups(m, n_products, grp.flat != 0, splits[order[0]], in / kBlockK * n_planes, sm_count);
+    shape.n = n;
+    shape.least = splits[order[0]];
+    shape.unequal = grp.flat != 0;
+    const int groups = group_call_groups(shape, m, n_planes, sm_count);
     // 1. the rotations
     launch_rotate_rows(x, rot, n, in, m, n_planes, block, groups, gemm_carveout(m, groups), sm_count, stream);
     // 2. the GEMMs
