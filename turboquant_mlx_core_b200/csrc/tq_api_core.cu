@@ -2,8 +2,8 @@
 // non-tensor handles of turboquant_c.h (model, coordinator, cluster planner).
 #include <sys/stat.h>
 
+#include <atomic>
 #include <cmath>
-#include <mutex>
 
 #include "tq_host.hpp"
 #include "tq_kernels.cuh"
@@ -23,21 +23,21 @@ int current_device() {
     return d;
 }
 
-static int device_attribute(cudaDeviceAttr which, int device, int (&cache)[64]) {
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    if (device >= 0 && device < 64 && cache[device]) return cache[device];
-    int n = 0;
+// (Looked up in every call, so without a lock.)
+static int device_attribute(cudaDeviceAttr which, int device, std::atomic<int> (&cache)[64]) {
+    const bool kept = device >= 0 && device < 64;
+    int n = kept ? cache[device].load(std::memory_order_relaxed) : 0;
+    if (n) return n;
     TQ_CUDA(cudaDeviceGetAttribute(&n, which, device));
-    if (device >= 0 && device < 64) cache[device] = n;
+    if (kept) cache[device].store(n, std::memory_order_relaxed);
     return n;
 }
 int sm_count(int device) {
-    static int cache[64] = {0};
+    static std::atomic<int> cache[64];
     return device_attribute(cudaDevAttrMultiProcessorCount, device, cache);
 }
 size_t l2_bytes(int device) {
-    static int cache[64] = {0};
+    static std::atomic<int> cache[64];
     return static_cast<size_t>(device_attribute(cudaDevAttrL2CacheSize, device, cache));
 }
 
